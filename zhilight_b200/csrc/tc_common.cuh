@@ -69,8 +69,8 @@ __device__ __forceinline__ uint2 tc_ld_tag(const uint2* p) {
     return v;
 }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// true in exactly one lane of a converged warp (elect.sync): ptxas then knows the guarded region is single-threaded and passes
-// the tcgen05 operands through plain R2UR moves instead of a per-instruction ELECT / R2UR.BROADCAST waterfall loop
+// true in exactly one lane of a converged warp (elect.sync): the compiler then knows that the guarded region is single-threaded
+// (measured: 850 cycles per 128-k stage of 8 MMAs behind `if (lane == 0)`, against back-to-back issue behind the election)
 __device__ __forceinline__ bool tc_elect_one() {
     uint32_t pred;
     asm volatile(

@@ -16,9 +16,9 @@
 //
 //   warps 0-3          epilogue     : tcgen05.ld 32x32b of their TMEM lane quadrant; bias / residual / SwiGLU / qkv-RoPE-KV
 //   warps 4 .. 4+4KQ-1 dequant      : quadrant = warp % 4 = 32-row block of the tile, k-slice = (warp - 4) / 4 of KQ;
-//                                     the lane owns ONE weight row: nibbles -> fp16 (PRMT 0x64xx / 0x54xx magic, exact
-//                                     q - z, one HMUL2 by the group scale) in registers, tcgen05.st into the A columns
-//   then               raw producer : tensor-TMA (UTMALDG.4D / .3D) of the 4 ZLW4I records of a stage
+//                                     the lane owns ONE weight row: nibbles -> fp16 (byte permute, 0x64xx / 0x54xx magic, exact
+//                                     q - z, one __hmul2 by the group scale) in registers, tcgen05.st into the A columns
+//   then               raw producer : tensor-TMA (4-D / 3-D boxes) of the 4 ZLW4I records of a stage
 //                      x producer   : cp.async.bulk.tensor.2d, box 64 k x NTOK tokens, SWIZZLE_128B, OOB rows = 0
 //                      MMA issuer   : one thread, 8 x tcgen05.mma 128 x NTOK x 16 per stage (A from TMEM, B from smem),
 //                                     tcgen05.commit frees the stage; also owns the TMEM allocation
