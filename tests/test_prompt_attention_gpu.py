@@ -1,0 +1,88 @@
+"""GPU: attention of several query rows per task (portions of a prompt, tree rows) against the oracle, at the edges of the kernel's
+64-row blocks and 64-key tiles, with masks of any shape, key splits and both cache layouts."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import ops as oops
+from tests.helpers import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+# fp16 / bf16 output rounding (2^-12 / 2^-9 of a value on average) plus as much again for the rounding of the probabilities
+TOL = {torch.float16: ("f16", 1e-3), torch.bfloat16: ("bf16", 6e-3)}
+
+
+def _run(cuda, dtype, lens, len_q, hq, hkv, d, masks, bshd=True, seed=0):
+    from zhilight_b200 import ops
+    g = torch.Generator().manual_seed(seed)
+    q = torch.randn(len(lens), len_q, hq, d, generator=g).to(dtype)
+    shapes = [(n, hkv, d) if bshd else (hkv, n, d) for n in lens]
+    ks = [torch.randn(*s, generator=g).to(dtype) for s in shapes]
+    vs = [torch.randn(*s, generator=g).to(dtype) for s in shapes]
+    flat = None if masks is None else torch.cat([m.reshape(-1) for m in masks]).to(cuda)
+    out = ops.decode_attention(q.to(cuda), torch.tensor(lens, dtype=torch.int32, device=cuda), [k.to(cuda) for k in ks], [v.to(cuda) for v in vs],
+                               flat, d ** -0.5, max(lens), hkv, bshd=bshd).float().cpu().numpy()
+    nat = [[t.float().numpy() if bshd else t.float().permute(1, 0, 2).contiguous().numpy() for t in x] for x in (ks, vs)]
+    ones = [np.ones((len_q, n), np.int8) for n in lens]
+    ref = oops.decode_attention(q.float().numpy(), nat[0], nat[1], lens, ones if masks is None else [m.numpy() for m in masks], d ** -0.5, hq // hkv,
+                                TOL[dtype][0])
+    return out, np.asarray(ref)
+
+
+def _causal(len_q, n):
+    return (torch.arange(n)[None, :] <= torch.arange(n - len_q, n)[:, None]).to(torch.int8)
+
+
+@pytest.mark.parametrize("dtype", list(TOL))
+@pytest.mark.parametrize("hq,hkv,d", [(8, 2, 128), (4, 4, 64), (9, 3, 64), (16, 1, 128)])
+@pytest.mark.parametrize("len_q,ctx", [(16, 16), (17, 63), (64, 65), (160, 160), (321, 321), (330, 515), (1030, 1030)])
+def test_causal_portions(lib, cuda, dtype, hq, hkv, d, len_q, ctx):
+    """Both sides of the dispatch line."""
+    out, ref = _run(cuda, dtype, [ctx], len_q, hq, hkv, d, [_causal(len_q, ctx)])
+    tol = TOL[dtype][1]
+    assert rel_l2(out, ref) <= tol
+    for i in (0, len_q // 2, len_q - 1):                # single rows: a wrong row or head cannot hide in the whole
+        for h in (0, hq - 1):
+            assert rel_l2(out[0, i, h], ref[0, i, h]) <= 4 * tol, (i, h)
+
+
+@pytest.mark.parametrize("bshd", [True, False])
+@pytest.mark.parametrize("masked", [True, False])
+def test_ragged_tasks_and_any_mask(lib, cuda, bshd, masked):
+    lens, len_q = [200, 33, 1, 128], 41
+    g = torch.Generator().manual_seed(4)
+    masks = [(torch.rand(len_q, n, generator=g) < 0.4).to(torch.int8) * 3 for n in lens] if masked else None   # any non-zero byte is visible
+    if masked:
+        masks[0][5] = 0                                 # rows that see nothing give zeros
+        masks[2][:] = 0
+        masks[3][:, :100] = 0                           # whole tiles without a visible key before the visible ones
+    out, ref = _run(cuda, torch.float16, lens, len_q, 8, 2, 128, masks, bshd, seed=1)
+    assert rel_l2(out, ref) <= 1e-3
+    if masked:
+        assert not out[0, 5].any() and not out[2].any()
+
+
+@pytest.mark.parametrize("len_q,ctx", [(33, 1500), (40, 2049)])
+def test_key_splits(lib, cuda, len_q, ctx):
+    """Few row blocks over many keys: the keys are split and merged."""
+    out, ref = _run(cuda, torch.bfloat16, [ctx], len_q, 4, 1, 128, [_causal(len_q, ctx)], seed=2)
+    assert rel_l2(out, ref) <= 6e-3
+
+
+def test_infinities_and_nans_stay_in_their_rows(lib, cuda):
+    from zhilight_b200 import ops
+    g = torch.Generator().manual_seed(3)
+    q, k, v = (torch.randn(*s, generator=g).half() for s in ((1, 320, 4, 128), (384, 1, 128), (384, 1, 128)))
+    q[0, 3, 1, 7] = float("inf")
+    q[0, 9, 2, 0] = float("nan")
+    mask = _causal(320, 384).to(cuda)
+    call = lambda q_: ops.decode_attention(q_.to(cuda), torch.tensor([384], dtype=torch.int32, device=cuda), [k.to(cuda)], [v.to(cuda)],  # noqa: E731
+                                           mask, 0.125, 384, 1)
+    bad = call(q)
+    q[0, 3, 1] = q[0, 9, 2] = 0
+    good = call(q)
+    assert torch.isnan(bad[0, 3, 1]).all() and torch.isnan(bad[0, 9, 2]).all()
+    keep = torch.ones(320, 4, dtype=torch.bool, device=cuda)
+    keep[3, 1] = keep[9, 2] = False
+    assert torch.equal(bad[0][keep], good[0][keep])

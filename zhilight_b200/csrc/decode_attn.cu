@@ -13,6 +13,7 @@
 #include "common.cuh"
 #include "decode_attn_short.cuh"
 #include "decode_attn_warp.cuh"
+#include "prompt_attn.cuh"
 
 #include <cstdlib>
 #include <type_traits>
@@ -368,6 +369,66 @@ extern "C" size_t zl_decode_attention_workspace_bytes(int B, int len_q, int num_
     return (size_t)B * len_q * num_heads * splits * (dim_head + 2) * sizeof(float);
 }
 
+// Workspace of the prompt kernel ahead of the splits' partial results: the mask's bits, then the last visible keys.
+static size_t prompt_head_bytes(int B, int len_q, int max_len_buf, const int8_t* mask) {
+    const size_t q_rows = (size_t)B * len_q;
+    return mask ? (q_rows * cdiv(max_len_buf, kPaKeys) * 8 + 15) / 16 * 16 + (q_rows * 4 + 15) / 16 * 16 : 0;
+}
+// Which kernel serves several query rows.  The decode kernels read K and V once per query row and stay at their latency (12 - 17 us)
+// while these reads fit one wave; the prompt kernel reads them once per 64 (query, head) rows and has a mask pass and a longer
+// chain (14 - 23 us).  Measured in 256-key CTAs of the decode kernels, D = 128: 8 heads on 1, 1100 keys: 120 CTAs 16.7 against
+// 20.9 us, 160 CTAs 23.3 against 20.8; 32 heads on 8, 1100 keys: 160 CTAs 20.9 against 21.9, 240 CTAs 21.1 against 20.1, 20480 CTAs
+// 287 against 45; 16 on 8: 640 CTAs 20.9 against 21.4, 960 CTAs 22.9 against 21.9.  Halving the head's width halves the reads but
+// not the chain: D = 64, 32 on 8, 1100 keys: 1280 CTAs 19.8 against 20.9; 16 on 16: 1280 CTAs 18.9 against 19.9, 2048 CTAs 17.4
+// against 15.4.  The mask's bits live in the workspace, so a masked call without room for them keeps the decode kernels.
+static bool prompt_route(int len_q, int m_query, int dim_head, int B, int num_kv_heads, const int8_t* mask, int max_len_buf, const void* out,
+                         const void* workspace, size_t workspace_bytes) {
+    if (len_q < 2 || num_kv_heads > 65535 || B > 65535 / 16) return false;
+    const long long ctas = (long long)B * len_q * num_kv_heads * cdiv(m_query, 8) * cdiv(max_len_buf, 256);
+    const long long line = dim_head == 64 ? 1536 : m_query >= 4 ? 192 : 768;
+    if (ctas < line) return false;
+    if ((reinterpret_cast<uintptr_t>(out) & 3) || (reinterpret_cast<uintptr_t>(workspace) & 15)) return false;
+    return !mask || (workspace && prompt_head_bytes(B, len_q, max_len_buf, mask) <= workspace_bytes && len_q <= 65535);
+}
+
+template <typename T, int D>
+static int prompt_attention(const void* q, const int32_t* buf_lens, void* const* k_addrs, void* const* v_addrs, const int8_t* mask, float scale,
+                            int max_len_buf, void* out, int B, int len_q, int num_heads, int num_kv_heads, int bshd, void* workspace,
+                            size_t workspace_bytes, int pdl, zl_stream_t stream) {
+    const int m_query = num_heads / num_kv_heads;
+    const int blocks = cdiv(len_q * m_query, kPaRows), tiles = cdiv(max_len_buf, kPaKeys);
+    int splits = workspace ? prompt_attn_splits((long long)blocks * num_kv_heads * B, tiles) : 1;
+    const size_t q_rows = (size_t)B * len_q, vheads = q_rows * num_heads;
+    const size_t head_bytes = prompt_head_bytes(B, len_q, max_len_buf, mask);
+    if (splits > 1 && head_bytes + vheads * splits * (D + 2) * sizeof(float) > workspace_bytes) splits = 1;
+    uint64_t* bits = mask ? static_cast<uint64_t*>(workspace) : nullptr;
+    int32_t* last = mask ? reinterpret_cast<int32_t*>(static_cast<uint8_t*>(workspace) + (q_rows * tiles * 8 + 15) / 16 * 16) : nullptr;
+    float *part_o = nullptr, *part_m = nullptr, *part_l = nullptr;
+    if (splits > 1) {
+        part_o = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + head_bytes);
+        part_m = part_o + vheads * splits * D;
+        part_l = part_m + vheads * splits;
+    }
+    static bool attr_set[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64 || !attr_set[dev]) {
+        ZL_CHECK_CUDA(cudaFuncSetAttribute(k_attn_prompt<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, prompt_attn_smem_bytes<D>()));
+        if (dev >= 0 && dev < 64) attr_set[dev] = true;
+    }
+    if (mask)
+        ZL_CHECK_CUDA(launch(k_mask_bits, dim3(len_q, B), dim3(256), 0, stream, pdl != 0, mask, buf_lens, bits, last, len_q, tiles));
+    ZL_CHECK_CUDA(launch(k_attn_prompt<T, D>, dim3(blocks, num_kv_heads, B * splits), dim3(kPaThreads), (size_t)prompt_attn_smem_bytes<D>(), stream,
+                         pdl != 0, (const T*)q, buf_lens, (T* const*)k_addrs, (T* const*)v_addrs, (const uint64_t*)bits, (const int32_t*)last, tiles,
+                         scale, (T*)out, part_o, part_m, part_l, len_q, num_heads, num_kv_heads, m_query, splits, bshd));
+    if (splits > 1)
+        ZL_CHECK_CUDA(launch(k_attn_combine<T>, dim3((unsigned)vheads), dim3(D), 0, stream, pdl != 0, (const float*)part_o, (const float*)part_m,
+                             (const float*)part_l, (T*)out, splits));
+    g_attn_pf_ptr = nullptr;
+    g_attn_pf_bytes = 0;
+    return ZL_OK;
+}
+
 extern "C" int zl_decode_attention(const void* q, const int32_t* buf_lens, void* const* k_addrs,
                                    void* const* v_addrs, const int8_t* mask, float scale, int max_len_buf,
                                    void* out, int B, int len_q, int num_heads, int num_kv_heads, int dim_head,
@@ -378,6 +439,17 @@ extern "C" int zl_decode_attention(const void* q, const int32_t* buf_lens, void*
     ZL_CHECK_SUPPORTED(dim_head == 64 || dim_head == 128);
     ZL_CHECK_SUPPORTED(dtype == ZL_F16 || dtype == ZL_BF16);
     const int m_query = num_heads / num_kv_heads;
+    if (prompt_route(len_q, m_query, dim_head, B, num_kv_heads, mask, max_len_buf, out, workspace, workspace_bytes)) {
+        if (dtype == ZL_F16)
+            return dim_head == 128 ? prompt_attention<__half, 128>(q, buf_lens, k_addrs, v_addrs, mask, scale, max_len_buf, out, B, len_q, num_heads,
+                                                                   num_kv_heads, bshd, workspace, workspace_bytes, pdl, stream)
+                                   : prompt_attention<__half, 64>(q, buf_lens, k_addrs, v_addrs, mask, scale, max_len_buf, out, B, len_q, num_heads,
+                                                                  num_kv_heads, bshd, workspace, workspace_bytes, pdl, stream);
+        return dim_head == 128 ? prompt_attention<__nv_bfloat16, 128>(q, buf_lens, k_addrs, v_addrs, mask, scale, max_len_buf, out, B, len_q,
+                                                                      num_heads, num_kv_heads, bshd, workspace, workspace_bytes, pdl, stream)
+                               : prompt_attention<__nv_bfloat16, 64>(q, buf_lens, k_addrs, v_addrs, mask, scale, max_len_buf, out, B, len_q,
+                                                                     num_heads, num_kv_heads, bshd, workspace, workspace_bytes, pdl, stream);
+    }
     int splits = attn_num_splits(B, len_q, num_kv_heads, m_query, max_len_buf);
     // latency regime: few CTAs of work -> 256-key CTAs that issue all their loads up front
     const int hg0 = (m_query + 7) / 8;
