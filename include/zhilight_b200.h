@@ -147,6 +147,8 @@ int zl_w4_int_layout_route(int M, int N, int K);
 /* last watchdog code published by a tcgen05 kernel on the current device (0 = none); a bounded mbarrier wait that expires
  * records which pipeline barrier starved and traps instead of hanging the GPU. */
 unsigned zl_w4_tc_watchdog(void);
+/* the same of the general tensor-core GEMM (zl_gemm_nt*, zl_dense_gemm_skinny* with prompt-sized M) */
+unsigned zl_gemm_tc_watchdog(void);
 /* debug / tests: at least `splits` pieces per weight-row tile in the tcgen05 kernel's stream-k schedule (0 = automatic; also
  * ZL_TC_SPLITS). */
 int zl_w4_tc_set_splits(int splits);

@@ -1,0 +1,124 @@
+"""GPU: the general GEMM on the tensor cores (prompt-sized M) against the same products in 64 bits: edges of its 256-row and 32-row tiles
+and of the 64-k stages, every epilogue, batches, and grouped rows with empty, one-row and more-than-one-tile groups."""
+import numpy as np
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+BF, HF = torch.bfloat16, torch.float16
+
+
+def _rand(g, *shape, dtype):
+    return torch.randn(*shape, generator=g).to(dtype).cuda()
+
+
+def _close(y, ref, mag, k, out_dtype):
+    """mag: the sums of the products' magnitudes.  Every 16 products are added to an fp32 accumulator that may drop up to a unit in its last
+    place, so the sum is off by at most (k / 16 + 2) 2^-23 of it; 16-bit outputs round by half a unit of theirs."""
+    y, ref = y.double(), ref.double()
+    lim = (k / 16 + 2) * 2.0 ** -23 * mag + (0 if out_dtype == torch.float32 else 2.0 ** (-8 if out_dtype == BF else -11)) * ref.abs()
+    bad = (y - ref).abs() > lim
+    assert not bad.any(), (int(bad.sum()), float((y - ref).abs().max()))
+
+
+@pytest.fixture(autouse=True)
+def no_wait_gave_up(lib, cuda):
+    yield
+    torch.cuda.synchronize()
+    assert lib.zl_gemm_tc_watchdog() == 0
+
+
+@pytest.mark.parametrize("dtype,out", [(BF, BF), (BF, torch.float32), (HF, HF), (HF, torch.float32)])
+@pytest.mark.parametrize("m,n,k", [(33, 128, 64), (64, 136, 72), (65, 250, 136), (256, 256, 128), (257, 513, 448), (300, 520, 1000), (40, 4096, 512),
+                                   (777, 2048, 328)])
+def test_plain(lib, cuda, dtype, out, m, n, k):
+    from zhilight_b200 import ops
+    g = torch.Generator().manual_seed(m + n)
+    x, w, b = _rand(g, m, k, dtype=dtype), _rand(g, n, k, dtype=dtype), torch.randn(n, generator=g).cuda()
+    ref, mag = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    _close(ops.gemm_nt(x, w, out_dtype=out), ref, mag, k, out)
+    _close(ops.gemm_nt_bias(x, w, b, out_dtype=out), ref + b.double(), mag + b.double().abs(), k, out)
+
+
+@pytest.mark.parametrize("dtype", [BF, HF])
+@pytest.mark.parametrize("m,n,k", [(65, 128, 64), (95, 1000, 96), (512, 264, 2048)])
+def test_skinny_entry_with_bias_and_activations(lib, cuda, dtype, m, n, k):
+    """zl_dense_gemm_skinny's bias is of the input type; its activations; more rows than one of its 32-row passes."""
+    from zhilight_b200 import ops
+    g = torch.Generator().manual_seed(k)
+    x, w, b = _rand(g, m, k, dtype=dtype) / 8, _rand(g, n, k, dtype=dtype), _rand(g, n, dtype=dtype)
+    mul = torch.randn(m, n, generator=g).cuda()
+    ref, mag = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    _close(ops.dense_gemm_skinny(x, w, b), ref + b.double(), mag + b.double().abs(), k, dtype)
+    for act, want in ((1, F.relu(ref) ** 2), (2, torch.tanh(ref)), (3, F.gelu(ref, approximate="tanh") * mul.double())):
+        y = ops.dense_gemm_skinny_mul(x, w, act, mul if act == 3 else None, out_dtype=torch.float32)
+        assert float((y.double() - want).norm() / want.norm()) < 1e-5, act
+
+
+@pytest.mark.parametrize("m,n,k", [(40, 130, 64), (257, 512, 200)])
+def test_epilogues(lib, cuda, m, n, k):
+    from zhilight_b200 import ops
+    g = torch.Generator().manual_seed(n)
+    x, w, mul = _rand(g, m, k, dtype=BF) / 8, _rand(g, n, k, dtype=BF), torch.randn(m, n, generator=g).cuda()
+    ref = x.double() @ w.double().T
+    a, u = ref[:, 0::2], ref[:, 1::2]
+    ga, cu = a.clamp(max=1.5), u.clamp(-1.5, 1.5)
+    rel = lambda y, want: float((y.double() - want).norm() / want.norm())  # noqa: E731
+    f32 = torch.float32
+    assert rel(ops.gemm_nt(x, w, f32, ops.GEMM_EPI_RELU2), F.relu(ref) ** 2) < 1e-5
+    assert rel(ops.gemm_nt(x, w, f32, ops.GEMM_EPI_SIGMOID_GATE, mul), ref * torch.sigmoid(mul.double())) < 1e-5
+    assert rel(ops.gemm_nt_bias(x, w, None, f32, ops.GEMM_EPI_TANH), torch.tanh(ref)) < 1e-5
+    assert rel(ops.gemm_nt_fused(x, w, None, f32, ops.GEMM_EPI_GELU_TANH_MUL, mul), F.gelu(ref, approximate="tanh") * mul.double()) < 1e-5
+    assert rel(ops.gemm_nt_fused(x, w, None, f32, ops.GEMM_EPI_SOFTCAP, limit=2.0), 2 * torch.tanh(ref / 2)) < 1e-5
+    assert rel(ops.gemm_nt_fused(x, w, None, f32, ops.GEMM_EPI_GEGLU_TANH), F.gelu(a, approximate="tanh") * u) < 1e-5
+    assert rel(ops.gemm_nt_glu_clamp(x, w, None, f32, 1.5, 1.7, 0.5), ga * torch.sigmoid(1.7 * ga) * (cu + 0.5)) < 1e-5
+
+
+@pytest.mark.parametrize("b,m,n,k", [(3, 70, 128, 64), (5, 33, 300, 128), (90, 40, 512, 64)])
+def test_batches(lib, cuda, b, m, n, k):
+    from zhilight_b200 import ops
+    g = torch.Generator().manual_seed(b)
+    x, w = _rand(g, b, m, k, dtype=BF), _rand(g, b, n, k, dtype=BF)
+    prod = lambda a, c: torch.einsum("bmk,bnk->bmn", a, c)  # noqa: E731
+    _close(ops.gemm_nt(x, w, out_dtype=torch.float32), prod(x.double(), w.double()), prod(x.double().abs(), w.double().abs()), k, torch.float32)
+
+
+@pytest.mark.parametrize("dtype", [BF, HF])
+@pytest.mark.parametrize("sizes", [[0, 9, 1, 0, 31], [32, 33, 0, 64, 1], [1] * 150, [256, 0, 257, 3], [700, 12]])
+@pytest.mark.parametrize("n,k", [(128, 64), (300, 200), (512, 520)])
+def test_grouped(lib, cuda, dtype, sizes, n, k):
+    from zhilight_b200 import ops
+    rng = np.random.default_rng(sum(sizes) + n)
+    g = torch.Generator().manual_seed(n)
+    total, groups = sum(sizes), len(sizes)
+    t = total // 2 + 1                                  # rows of x: several list entries share one
+    x, w = _rand(g, t, k, dtype=dtype) / 8, _rand(g, groups, n, k, dtype=dtype)
+    off = torch.tensor(np.concatenate([[0], np.cumsum(sizes)]), dtype=torch.int32, device="cuda")
+    rows = torch.tensor(rng.integers(0, t, total), dtype=torch.int32, device="cuda")
+    back = torch.tensor(rng.permutation(total), dtype=torch.int32, device="cuda")
+    owner = torch.repeat_interleave(torch.arange(groups), torch.tensor(sizes)).cuda()
+    prod = lambda a, c: torch.einsum("rk,rnk->rn", a[rows.long()], c[owner])  # noqa: E731
+    ref, mag = prod(x.double(), w.double()), prod(x.double().abs(), w.double().abs())
+    a, u = ref[:, 0::2].clamp(max=1.0), ref[:, 1::2].clamp(-1.0, 1.0)
+    y = ops.gemm_nt_grouped(x, w, off, total, x_rows=rows, out_dtype=torch.float32, epilogue=ops.GEMM_EPI_GLU_CLAMP, limit=1.0, alpha=1.7, beta=1.0)
+    want = a * torch.sigmoid(1.7 * a) * (u + 1)
+    assert float((y.double() - want).norm() / want.norm()) < 1e-5
+    xs = x[rows.long()].contiguous()
+    y = ops.gemm_nt_grouped(xs, w, off, total, y_rows=back, out_dtype=torch.float32)
+    _close(y[back.long()], ref, mag, k, torch.float32)
+    _close(ops.gemm_nt_grouped(x, w, off, total, x_rows=rows), ref, mag, k, dtype)
+
+
+def test_infinities_stay_in_their_rows_and_columns(lib, cuda):
+    from zhilight_b200 import ops
+    g = torch.Generator().manual_seed(1)
+    x, w = _rand(g, 70, 128, dtype=BF), _rand(g, 256, 128, dtype=BF)
+    good = ops.gemm_nt(x, w, out_dtype=torch.float32)
+    x[69, 3], w[17, 5] = float("inf"), float("nan")
+    bad = ops.gemm_nt(x, w, out_dtype=torch.float32)
+    assert not torch.isfinite(bad[69]).any() and torch.isnan(bad[:, 17]).all()
+    keep = torch.ones_like(bad, dtype=torch.bool)
+    keep[69], keep[:, 17] = False, False
+    assert torch.equal(bad[keep], good[keep])

@@ -30,7 +30,7 @@ NVCC_FLAGS = [
 
 
 # sources of the families whose drivers stand on their own (names without .cu)
-_FP32_RESIDUAL_COMMON = ["misc", "dense_gemm", "gemm_tiled", "group_norm_conv"]
+_FP32_RESIDUAL_COMMON = ["misc", "dense_gemm", "gemm_tiled", "gemm_tc", "group_norm_conv"]
 FAMILY_SOURCES = {
     "kodupel": _FP32_RESIDUAL_COMMON + ["mixer_rows", "moe_route", "delta_rule", "sink_attn", "kodupel_runner"],
     "dekipel": _FP32_RESIDUAL_COMMON + ["latent_attn", "dekipel_runner"],

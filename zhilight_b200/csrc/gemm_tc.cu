@@ -1,0 +1,425 @@
+// General GEMM y[b](M, N) = epi(x[b](M, K) @ w[b](N, K)^T + bias) of 16-bit inputs on the 5th-generation tensor cores, for prompt-sized
+// M: the counterpart of gemm_tiled.cu's mma.sync kernel and of dense_gemm.cu's 32-row passes, same epilogues, same fp32
+// accumulation, and the grouped form of a mixture of experts.
+//
+// A tile is 256 rows of w (tcgen05.mma's A operand, 128 per CTA of the pair) by up to 256 rows of x (the B operand, half per CTA):
+// per 64-k stage each SM loads 16 KB of w and 16 KB of x for 512 cycles of MMA, where 64 x 64 tiles on mma.sync load 16 KB for 64
+// cycles' worth.  Operands through tensor-TMA in six stages of 128-byte swizzled rows, two accumulators in TMEM so that a tile's
+// epilogue runs under the next tile's MMAs, persistent pairs of CTAs that take the tiles in turn.  bf16, 14336 x 4096: M = 2048
+// 970 -> 171 us (1410 TFLOP/s), M = 512 268 -> 55 us, M = 64 69 -> 30 us; 8192 x 2048, M = 1024: 154 -> 34 us.  Bound by the tensor
+// cores from about 1000 rows on, below by the loads of w (and by too few tiles: 4096 x 14336 keeps 16 of 74 pairs busy at M <= 256,
+// 52 us against 200).
+//
+//   warp 0       producer  : w and x boxes
+//   warp 1       MMA       : of the leader, one elected lane, 4 x 256 x ntok x 16 per stage
+//   warp 2       TMEM allocation
+//   warps 4-11   epilogue  : quadrant = warp % 4, 16-row chunks of x in turns; lane = row of w = column of y
+//   warps 12-15  grouped   : rows of x through their index lists, by 16-byte cp.async into the swizzled layout that the boxes have;
+//                            a stage's barrier counts the copies as they land, warp 3 hands the stage to the MMAs
+#include "gemm_common.cuh"
+#include "tc2_common.cuh"
+
+#include <type_traits>
+
+namespace zl {
+
+constexpr int kGtThreads = 12 * 32, kGtRowWarps = 4, kGtGroupThreads = kGtThreads + kGtRowWarps * 32, kGtEpiWarps = 8;
+constexpr int kGtStages = 6, kGtAStage = 128 * 128, kGtBStage = 128 * 128;
+constexpr int kGtBarOff = kGtStages * (kGtAStage + kGtBStage);
+constexpr int kGtMiscOff = kGtBarOff + (3 * kGtStages + 4) * 8;
+constexpr int kGtMaxGroups = 1024;
+constexpr int kGtCumOff = kGtMiscOff + 16;                       // grouped: tiles before each group
+constexpr int kGtBytes = kGtCumOff + (kGtMaxGroups + 1) * 4 + 1024;   // + slack for the manual 1024-byte alignment
+static_assert(kGtBytes <= 232448, "shared memory");
+
+struct alignas(64) GemmTcP {
+    CUtensorMap wmap;           // w (K, N, batch), box 64 x 128
+    CUtensorMap xmap;           // x (K, rows, batch), box 64 x box_rows; not grouped
+    GemmP g;
+    int epi, groups;            // groups: batch, or the number of groups
+    int row_tiles, tok_tiles;   // tok_tiles: not grouped
+    int ntok, box_rows;         // not grouped: rows of x of a tile, and of a box (a CTA's half of them)
+    int wide;                   // two neighbouring values of y may be stored together
+};
+
+// code of the last wait that gave up (0: none)
+__device__ unsigned g_gemm_tc_err;
+
+struct GtTile {
+    int b, n0, t0, ntok, M, first;
+};
+
+// tile `i` of the launch; false behind the last one.  Row tiles of a group follow each other with the rows of x innermost, so that
+// the pairs working at one time share their rows of w
+template <bool GROUPED>
+__device__ __forceinline__ bool gt_tile(const GemmTcP& p, const int* s_cum, int i, int& hint, GtTile& t) {
+    if constexpr (GROUPED) {
+        if (i >= s_cum[p.groups]) return false;
+        while (i >= s_cum[hint + 1]) ++hint;
+        t.b = hint;
+        t.first = p.g.grp_off[hint];
+        t.M = p.g.grp_off[hint + 1] - t.first;
+        const int tt = (t.M + 255) >> 8, j = i - s_cum[hint];
+        t.n0 = (j / tt) * kTc2Rows;
+        t.t0 = (j % tt) * 256;
+        t.ntok = min(256, (t.M - t.t0 + 31) & ~31);
+    } else {
+        const int per = p.row_tiles * p.tok_tiles;
+        if (i >= per * p.groups) return false;
+        t.b = i / per;
+        const int j = i - t.b * per;
+        t.n0 = (j / p.tok_tiles) * kTc2Rows;
+        t.t0 = (j % p.tok_tiles) * p.ntok;
+        t.M = p.g.M;
+        t.first = 0;
+        t.ntok = min(p.ntok, (t.M - t.t0 + 31) & ~31);
+    }
+    return true;
+}
+
+template <typename T, typename TO, int EPI>
+__device__ __forceinline__ void gt_store16(const GemmTcP& p, const GtTile& t, int n, int c0, float (&v)[16], float bias, int lane) {
+    const GemmP& g = p.g;
+    TO* y = static_cast<TO*>(g.y) + (size_t)t.b * (g.grp_off ? 0 : g.yb);
+    int mine = 0;   // row of y of token c0 + lane
+    if (g.grp_off) {
+        const int m = t.t0 + c0 + (lane & 15);
+        mine = m < t.M ? (g.y_rows ? g.y_rows[t.first + m] : t.first + m) : 0;
+    }
+    const int odd = lane & 1;
+    if constexpr (epi_pairs(EPI)) {
+        // gate and up of an output sit in neighbouring lanes: the even lane takes the tokens 0, 2, ..., the odd one 1, 3, ...
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float a0 = v[2 * j] + bias, a1 = v[2 * j + 1] + bias;
+            const float other = __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, 1);
+            v[j] = pair_unit<EPI>(odd ? other : a0, odd ? a1 : other, g);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int m = t.t0 + c0 + 2 * j + odd;
+            const int row = g.grp_off ? __shfl_sync(0xffffffffu, mine, 2 * j + odd) : m;
+            if ((n | 1) < g.N && m < t.M) y[(size_t)row * g.ldy + (n >> 1)] = from_f32<TO>(v[j]);
+        }
+    } else {
+        // results first, stores behind them: the compiler cannot tell y from the gate's values
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int m = t.t0 + c0 + i;
+            v[i] = m < t.M && n < g.N ? gemm_epilogue<EPI>(v[i] + bias, g, t.b, m, n) : 0.f;
+        }
+        if (p.wide) {   // two columns of every other token per lane: half the stores, twice as wide
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float other = __shfl_xor_sync(0xffffffffu, odd ? v[2 * j] : v[2 * j + 1], 1);
+                const int m = t.t0 + c0 + 2 * j + odd;
+                const int row = g.grp_off ? __shfl_sync(0xffffffffu, mine, 2 * j + odd) : m;
+                struct alignas(2 * sizeof(TO)) Two {
+                    TO a, b;
+                } two = {from_f32<TO>(odd ? other : v[2 * j]), from_f32<TO>(odd ? v[2 * j + 1] : other)};
+                if (n < g.N && m < t.M) *reinterpret_cast<Two*>(y + (size_t)row * g.ldy + (n & ~1)) = two;   // N is even
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const int m = t.t0 + c0 + i;
+                const int row = g.grp_off ? __shfl_sync(0xffffffffu, mine, i) : m;
+                if (n < g.N && m < t.M) y[(size_t)row * g.ldy + n] = from_f32<TO>(v[i]);
+            }
+        }
+    }
+}
+
+template <typename T, typename TO, bool GROUPED>
+__global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_gemm_tc(const __grid_constant__ GemmTcP p) {
+    extern __shared__ uint8_t smem_dyn[];
+    uint8_t* smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + kGtBarOff);
+    uint64_t* empty = full + kGtStages;
+    uint64_t* acc_full = empty + kGtStages;
+    uint64_t* acc_empty = acc_full + 2;
+    uint64_t* rows_full = acc_empty + 2;       // grouped: this CTA's rows of a stage have landed
+    uint32_t* s_tmem = reinterpret_cast<uint32_t*>(smem + kGtMiscOff);
+    volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
+    int* s_cum = reinterpret_cast<int*>(smem + kGtCumOff);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank();
+    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const int ks = (p.g.K + 63) / 64;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kGtStages; ++i) {
+            mbar_init(&full[i], GROUPED ? 3 : 1);
+            mbar_init(&empty[i], 1);
+            mbar_init(&rows_full[i], kGtRowWarps * 32);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&acc_full[i], 1);
+            mbar_init(&acc_empty[i], 2 * kGtEpiWarps);
+        }
+        *s_abort = 0;
+        mbar_fence_init();
+    }
+    if (warp == 2) tc2_alloc(s_tmem);
+    pdl_trigger();
+    pdl_wait();
+    if (GROUPED && warp == 3) {   // tiles before each group: a running sum over the groups' sizes
+        int base = 0;
+        for (int g0 = 0; g0 < p.groups; g0 += 32) {
+            const int g = g0 + lane;
+            int c = 0;
+            if (g < p.groups) c = ((p.g.grp_off[g + 1] - p.g.grp_off[g] + 255) >> 8) * p.row_tiles;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, c, o);
+                if (lane >= o) c += u;
+            }
+            if (g < p.groups) s_cum[g + 1] = base + c;
+            base += __shfl_sync(0xffffffffu, c, 31);
+        }
+        if (lane == 0) s_cum[0] = 0;
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();   // both CTAs' barriers and allocations are in place
+    tc_fence_after();
+    const uint32_t tmem = *s_tmem;
+
+    if (warp == 0) {
+        int st = 0, hint = 0;
+        uint32_t ph = 0;
+        GtTile t;
+        bool ok = true;
+        for (int i = pair; ok && gt_tile<GROUPED>(p, s_cum, i, hint, t); i += pairs) {
+            const int tb = t.t0 + (int)rank * (t.ntok >> 1);
+            const uint32_t bytes = 2u * (kGtAStage + (GROUPED ? 0 : p.box_rows * 128));
+            for (int k = 0; k < ks; ++k) {
+                if (!(ok = tc2_wait(&empty[st], ph ^ 1u, s_abort, &g_gemm_tc_err, 0x2100 + st))) break;
+                if (tc_elect_one()) {
+                    const uint32_t bar = cluster_map(smem_u32(&full[st]), 0);
+                    uint8_t* sa = smem + st * (kGtAStage + kGtBStage);
+                    if (rank == 0) mbar_expect_tx(&full[st], bytes);
+                    tma2_load_3d(sa, &p.wmap, k * 64, t.n0 + (int)rank * 128, t.b, bar);
+                    if (!GROUPED) tma2_load_3d(sa + kGtAStage, &p.xmap, k * 64, tb, t.b, bar);
+                }
+                __syncwarp();
+                if (++st == kGtStages) {
+                    st = 0;
+                    ph ^= 1u;
+                }
+            }
+        }
+    } else if (warp == 1 && rank == 0) {
+        int st = 0, acc = 0, hint = 0;
+        uint32_t ph = 0, acc_ph = 0;
+        GtTile t;
+        bool ok = true;
+        for (int i = pair; ok && gt_tile<GROUPED>(p, s_cum, i, hint, t); i += pairs) {
+            if (!(ok = tc2_wait(&acc_empty[acc], acc_ph ^ 1u, s_abort, &g_gemm_tc_err, 0x2300 + acc))) break;
+            tc_fence_after();
+            const uint32_t d = tmem + (uint32_t)(acc * 256);
+            const uint32_t idesc = tc2_idesc(std::is_same<T, __nv_bfloat16>::value, t.ntok);
+            for (int k = 0; k < ks; ++k) {
+                if (!(ok = tc2_wait(&full[st], ph, s_abort, &g_gemm_tc_err, 0x2400 + st))) break;
+                tc_fence_after();
+                if (tc_elect_one()) {
+                    const uint64_t ad = tc_desc_sw128(smem_u32(smem + st * (kGtAStage + kGtBStage)));
+                    const uint64_t bd = tc_desc_sw128(smem_u32(smem + st * (kGtAStage + kGtBStage) + kGtAStage));
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) tc2_mma_ss(d, ad + (uint64_t)(j * 2), bd + (uint64_t)(j * 2), idesc, (k > 0 || j > 0) ? 1u : 0u);
+                    tc2_commit(&empty[st]);
+                    if (k == ks - 1) tc2_commit(&acc_full[acc]);
+                }
+                __syncwarp();
+                if (++st == kGtStages) {
+                    st = 0;
+                    ph ^= 1u;
+                }
+            }
+            if (++acc == 2) {
+                acc = 0;
+                acc_ph ^= 1u;
+            }
+        }
+    } else if (GROUPED && warp == 3) {
+        // rows that have landed become visible to the proxy the MMAs read through, then count as arrived at the leader
+        int st = 0, hint = 0;
+        uint32_t ph = 0;
+        GtTile t;
+        bool ok = true;
+        for (int i = pair; ok && gt_tile<GROUPED>(p, s_cum, i, hint, t); i += pairs)
+            for (int k = 0; k < ks; ++k) {
+                if (!(ok = tc2_wait(&rows_full[st], ph, s_abort, &g_gemm_tc_err, 0x2500 + st))) break;
+                if (lane == 0) {
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    mbar_arrive_at(cluster_map(smem_u32(&full[st]), 0));
+                }
+                if (++st == kGtStages) {
+                    st = 0;
+                    ph ^= 1u;
+                }
+            }
+    } else if (GROUPED && warp >= 12) {
+        // thread: 16-byte chunk c of rows j, j + 16, ... of the CTA's half
+        const int tid = threadIdx.x - 12 * 32, c = tid & 7, j = tid >> 3;
+        const uint32_t sm = smem_u32(smem) + kGtAStage + (uint32_t)(j * 128 + ((c ^ (j & 7)) << 4));
+        int st = 0, hint = 0;
+        uint32_t ph = 0;
+        GtTile t;
+        bool ok = true;
+        for (int i = pair; ok && gt_tile<GROUPED>(p, s_cum, i, hint, t); i += pairs) {
+            const int half = t.ntok >> 1, tb = t.t0 + (int)rank * half;
+            const T* row[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {   // rows behind the group's end load its first row and are not stored
+                const int m = tb + j + u * 16, e = t.first + (m < t.M ? m : 0);
+                row[u] = static_cast<const T*>(p.g.x) + (size_t)(p.g.x_rows ? p.g.x_rows[e] : e) * p.g.ldx + c * 8;
+            }
+            for (int k = 0; k < ks; ++k) {
+                if (!(ok = tc2_wait(&empty[st], ph ^ 1u, s_abort, &g_gemm_tc_err, 0x2200 + st))) break;
+                const bool in = k * 64 + c * 8 < p.g.K;
+                const int bytes = in ? 16 : 0;   // 0: zeros, nothing is read
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (u * 16 < half)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sm + (uint32_t)(st * (kGtAStage + kGtBStage) + u * 2048)),
+                                     "l"(in ? row[u] + k * 64 : row[u] - c * 8), "r"(bytes)
+                                     : "memory");
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&rows_full[st])) : "memory");
+                if (++st == kGtStages) {
+                    st = 0;
+                    ph ^= 1u;
+                }
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else if (warp >= 4) {
+        const int q = warp & 3, set = (warp - 4) >> 2;
+        int acc = 0, hint = 0;
+        uint32_t acc_ph = 0;
+        GtTile t;
+        for (int i = pair; gt_tile<GROUPED>(p, s_cum, i, hint, t); i += pairs) {
+            if (!tc2_wait(&acc_full[acc], acc_ph, s_abort, &g_gemm_tc_err, 0x2800 + acc)) break;
+            tc_fence_after();
+            const int n = t.n0 + (int)rank * 128 + q * 32 + lane;
+            float bias = 0.f;
+            if (n < p.g.N) {
+                if (p.g.bias) bias = p.g.bias[(size_t)t.b * p.g.bb + n];
+                else if (p.g.bias_t) bias = to_f32<T>(static_cast<const T*>(p.g.bias_t)[n]);
+            }
+            const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * 256);
+            for (int c0 = set * 16; c0 < t.ntok && t.t0 + c0 < t.M; c0 += 32) {
+                float v[16];
+                tc_ld16(taddr + (uint32_t)c0, v);
+                switch (p.epi) {
+#define ZL_GT_EPI(E) case E: gt_store16<T, TO, E>(p, t, n, c0, v, bias, lane); break;
+                    ZL_GT_EPI(ZL_GEMM_EPI_RELU2)
+                    ZL_GT_EPI(ZL_GEMM_EPI_SIGMOID_GATE)
+                    ZL_GT_EPI(ZL_GEMM_EPI_TANH)
+                    ZL_GT_EPI(ZL_GEMM_EPI_GLU_CLAMP)
+                    ZL_GT_EPI(ZL_GEMM_EPI_GEGLU_TANH)
+                    ZL_GT_EPI(ZL_GEMM_EPI_GELU_TANH_MUL)
+                    ZL_GT_EPI(ZL_GEMM_EPI_SOFTCAP)
+                    ZL_GT_EPI(ZL_GEMM_EPI_REGLU)
+                    default: gt_store16<T, TO, ZL_GEMM_EPI_NONE>(p, t, n, c0, v, bias, lane);
+#undef ZL_GT_EPI
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_at(cluster_map(smem_u32(&acc_empty[acc]), 0));
+            if (++acc == 2) {
+                acc = 0;
+                acc_ph ^= 1u;
+            }
+        }
+    }
+    __syncwarp();
+    tc2_drain(s_abort);
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();   // nobody's shared memory or TMEM goes while the other CTA may still use it
+    if (warp == 2) {
+        tc_fence_after();
+        tc2_dealloc(tmem);
+    }
+}
+
+// Rows of x per tile for M rows, `rows` row tiles (times the batch) and `pairs` pairs of CTAs: the waves times a tile's cost per
+// 64-k stage, which is its loads (16 KB of w and 64 B per row of x, about 50 B a cycle) rather than its MMAs (2 cycles per row)
+static int gt_pick_ntok(int M, long long rows, int pairs) {
+    int best = 32;
+    double best_cost = 1e30;
+    for (int n = 32; n <= 256; n += 32) {
+        const long long tiles = rows * cdiv(M, n), waves = (tiles + pairs - 1) / pairs;
+        const double cost = (double)waves * (330.0 + 1.3 * n);
+        if (cost < best_cost - 1e-9) {
+            best_cost = cost;
+            best = n;
+        }
+        if (n >= M) break;
+    }
+    return best;
+}
+
+bool gemm_tc_route(const GemmP& p, int batch, int in_dtype) {
+    if (in_dtype != ZL_F16 && in_dtype != ZL_BF16) return false;
+    // 16-byte aligned bases and pitches (tensor-TMA, cp.async), extents below 2^31
+    if ((reinterpret_cast<uintptr_t>(p.x) & 15) || (reinterpret_cast<uintptr_t>(p.w) & 15) || p.ldx % 8 || p.ldw % 8) return false;
+    // a batch whose matrices share one x or w (pitch 0) stays with the tile kernel: a tensor map has no zero pitch
+    if (batch > 1 && (p.wb % 8 || p.wb <= 0 || (!p.grp_off && (p.xb % 8 || p.xb <= 0)))) return false;
+    if (p.N < 128 || p.K < 64) return false;
+    // groups: few rows through small matrices are the tile kernel's (32 groups of 1024 x 768: 36 list entries 22 against 27 us, 256
+    // entries 30 against 28; 16 of 4096 x 2048: 36 entries 75 against 69 us, 2048 entries 202 against 86)
+    if (p.grp_off) return batch <= kGtMaxGroups && p.K % 8 == 0 && (p.M >= 128 || (p.M > 8 && (long long)batch * p.N * p.K >= (64ll << 20)));
+    return p.M > 32 && (long long)cdiv(p.N, kTc2Rows) * cdiv(p.M, 32) * batch < (1ll << 30);
+}
+
+template <typename T, typename TO>
+static cudaError_t launch_gt(const GemmTcP& q, bool grouped, int pairs, bool pdl, cudaStream_t stream) {
+    static bool set[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64 || !set[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<T, TO, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGtBytes);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gemm_tc<T, TO, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGtBytes);
+        if (e != cudaSuccess) return e;
+        if (dev >= 0 && dev < 64) set[dev] = true;
+    }
+    return grouped ? launch_pairs(k_gemm_tc<T, TO, true>, pairs, dim3(kGtGroupThreads), (size_t)kGtBytes, stream, pdl, q)
+                   : launch_pairs(k_gemm_tc<T, TO, false>, pairs, dim3(kGtThreads), (size_t)kGtBytes, stream, pdl, q);
+}
+
+cudaError_t launch_gemm_tc(const GemmP& p, int batch, int in_dtype, int out_dtype, int epilogue, bool pdl, cudaStream_t stream) {
+    const bool bf16 = in_dtype == ZL_BF16, grouped = p.grp_off != nullptr;
+    const int max_pairs = device_sm_count() / 2;
+    GemmTcP q;
+    q.g = p;
+    q.epi = epilogue;
+    q.groups = batch;
+    q.row_tiles = cdiv(p.N, kTc2Rows);
+    q.tok_tiles = q.ntok = q.box_rows = 0;
+    const int elem = out_dtype == ZL_F32 ? 4 : 2;
+    q.wide = p.N % 2 == 0 && p.ldy % 2 == 0 && p.yb % 2 == 0 && reinterpret_cast<uintptr_t>(p.y) % (2 * elem) == 0;
+    int pairs = max_pairs;
+    if (!tc2_map_3d(&q.wmap, p.w, bf16, p.K, p.N, batch, p.ldw, p.wb, 128)) return cudaErrorInvalidValue;
+    if (!grouped) {
+        q.ntok = gt_pick_ntok(p.M, (long long)q.row_tiles * batch, max_pairs);
+        q.box_rows = q.ntok / 2;
+        q.tok_tiles = cdiv(p.M, q.ntok);
+        const long long tiles = (long long)q.row_tiles * q.tok_tiles * batch;
+        if (tiles < pairs) pairs = (int)tiles;
+        if (!tc2_map_3d(&q.xmap, p.x, bf16, p.K, p.M, batch, p.ldx, p.xb, q.box_rows)) return cudaErrorInvalidValue;
+    }
+    if (bf16) return out_dtype == ZL_F32 ? launch_gt<__nv_bfloat16, float>(q, grouped, pairs, pdl, stream)
+                                         : launch_gt<__nv_bfloat16, __nv_bfloat16>(q, grouped, pairs, pdl, stream);
+    return out_dtype == ZL_F32 ? launch_gt<__half, float>(q, grouped, pairs, pdl, stream) : launch_gt<__half, __half>(q, grouped, pairs, pdl, stream);
+}
+
+}  // namespace zl
+
+extern "C" unsigned zl_gemm_tc_watchdog(void) {
+    unsigned v = 0;
+    cudaMemcpyFromSymbol(&v, zl::g_gemm_tc_err, sizeof v);
+    return v;
+}

@@ -1,0 +1,129 @@
+// Building blocks of the kernels that run one tcgen05.mma over a pair of SMs (cta_group::2): a cluster of two CTAs, of which rank 0
+// (the leader) issues the MMAs for both.  Each CTA holds 128 of the 256 A rows and half of the B rows in its own shared memory, and
+// the accumulators of its own 128 rows in its own TMEM.  Waits give up after about a second (an error word is set, every role
+// leaves its loop, TMEM is freed and the kernel returns): a fault in the protocol must not hang the GPU.
+#pragma once
+#include "tc_common.cuh"
+
+namespace zl {
+
+constexpr int kTc2Rows = 256;                 // A rows of a tile (both CTAs)
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// address of this CTA's shared-memory word `addr` in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+// Arrives on a barrier of any CTA of the cluster.  What it hands over lies in TMEM or has been read from there (ordered by
+// tcgen05.fence), was written by the async proxy, or was made visible to it by fence.proxy.async: no thread of the other CTA reads it
+// (a release at cluster scope, which that would take, costs the handing-over warp about a microsecond)
+__device__ __forceinline__ void mbar_arrive_at(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// For a whole warp, one lane polls; false: gave up (this wait or another one of the CTA's) and the caller leaves its loop.
+__device__ __forceinline__ bool tc2_wait(uint64_t* bar, uint32_t parity, volatile int* s_abort, unsigned* err, unsigned code) {
+    bool ok = true;
+    if ((threadIdx.x & 31) == 0) {
+        ok = mbar_try_wait(bar, parity);
+        if (!ok) {
+            const long long t0 = clock64();
+            unsigned spins = 0;
+            while (!(ok = mbar_try_wait(bar, parity))) {
+                if ((++spins & 1023u) == 0 && (*s_abort || clock64() - t0 > 2000000000ll)) {
+                    if (!*s_abort && err) atomicExch(err, code);
+                    *s_abort = 1;
+                    break;
+                }
+            }
+        }
+    }
+    return __all_sync(0xffffffffu, ok);
+}
+// after an abort: give copies and MMAs in flight time to land before shared memory and TMEM go away
+__device__ __forceinline__ void tc2_drain(volatile int* s_abort) {
+    if (!*s_abort) return;
+    const long long t0 = clock64();
+    while (clock64() - t0 < 4000000ll) {}
+}
+
+// loads whose completion is counted on a barrier of the leader: `bar` is a cluster address
+__device__ __forceinline__ void tma2_load_3d(void* smem_dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+            smem_u32(smem_dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ void tc2_alloc(uint32_t* s_tmem) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "n"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+}
+__device__ __forceinline__ void tc2_dealloc(uint32_t tmem) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512));
+}
+// arrives on the barrier at this offset in both CTAs once the MMAs issued so far have completed
+__device__ __forceinline__ void tc2_commit(uint64_t* bar) {
+    const uint16_t both = 3;
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+                 "h"(both)
+                 : "memory");
+}
+// kind::f16, fp32 accumulators, 256 x n x 16; bf16 or fp16 operands, both K-major
+__host__ __device__ constexpr uint32_t tc2_idesc(bool bf16, int n) {
+    return (1u << 4) | (bf16 ? (1u << 7) | (1u << 10) : 0u) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTc2Rows >> 4) << 24);
+}
+__device__ __forceinline__ void tc2_mma_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum)
+        : "memory");
+}
+__device__ __forceinline__ void tc2_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accum)
+        : "memory");
+}
+
+// launch of a grid of CTA pairs
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pairs(void (*kernel)(KArgs...), int pairs, dim3 block, size_t smem, cudaStream_t stream, bool pdl, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * pairs);
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 2 : 1;
+    zl_count_launch();
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+// (K, rows, batch) tensor of 16-bit values, row pitch ld and batch pitch in elements; box = 64 k x box_rows rows, 128-byte swizzle
+inline bool tc2_map_3d(CUtensorMap* map, const void* base, bool bf16, uint64_t k, uint64_t rows, uint64_t batch, uint64_t ld, uint64_t batch_ld,
+                       uint32_t box_rows) {
+    const uint64_t dims[3] = {k, rows, batch}, strides[2] = {ld * 2, (batch > 1 ? batch_ld : ld * rows) * 2};
+    const uint32_t box[3] = {64, box_rows, 1};
+    return tc_make_map_nd(map, base, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, dims, strides, box,
+                          CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+}  // namespace zl
