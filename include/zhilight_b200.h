@@ -149,6 +149,8 @@ int zl_w4_int_layout_route(int M, int N, int K);
 unsigned zl_w4_tc_watchdog(void);
 /* the same of the general tensor-core GEMM (zl_gemm_nt*, zl_dense_gemm_skinny* with prompt-sized M) */
 unsigned zl_gemm_tc_watchdog(void);
+/* ... and of the 4-bit kernel over pairs of SMs (prompt-sized M) */
+unsigned zl_w4_tc2_watchdog(void);
 /* debug / tests: at least `splits` pieces per weight-row tile in the tcgen05 kernel's stream-k schedule (0 = automatic; also
  * ZL_TC_SPLITS). */
 int zl_w4_tc_set_splits(int splits);

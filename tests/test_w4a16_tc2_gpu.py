@@ -1,0 +1,97 @@
+"""GPU: the 4-bit GEMM over pairs of SMs (prompt-sized M) against the oracle: edges of its 256-row and 32-token tiles, odd numbers of 128-row
+tiles, every epilogue.  Tolerance as in test_w4a16_tc_gpu.py: relative L2 <= 1e-3 for fp16 outputs."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import gptq, ops as oops
+from tests.helpers import rel_l2
+from tests.test_w4a16_tc_gpu import TOL, _setup
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def no_wait_gave_up(lib, cuda):
+    yield
+    torch.cuda.synchronize()
+    assert lib.zl_w4_tc2_watchdog() == 0
+
+
+def _x(m, k, seed):
+    return torch.randn(m, k, generator=torch.Generator().manual_seed(seed)).half()
+
+
+@pytest.mark.parametrize("m", [129, 160, 161, 255, 256, 257, 300, 513, 1000])
+@pytest.mark.parametrize("k,n", [(128, 128), (1024, 384), (640, 512)])
+def test_token_counts_and_row_tiles(lib, cuda, m, k, n):
+    from zhilight_b200 import ops
+    w, packed = _setup(cuda, k, n, False, 5)
+    x = _x(m, k, m)
+    y = ops.w4a16_gemm_fused(x.to(cuda), packed, n, k, variant=1).float().cpu().numpy()
+    ref = gptq.gemm_f32(x.numpy(), w)
+    assert rel_l2(y, ref) <= TOL
+    for i in (0, 31, 32, 127, 128, m - 1):
+        assert rel_l2(y[i], ref[i]) <= 2 * TOL, i
+
+
+@pytest.mark.parametrize("k,n,m,sym", [(4096, 6144, 200, False), (4096, 4096, 520, True), (14336, 4096, 257, False), (4096, 28672, 300, False),
+                                       (14336, 512, 200, False), (14336, 512, 100, True), (4096, 6144, 70, False)])
+def test_model_shapes(lib, cuda, k, n, m, sym):
+    """Also shapes below 257 tokens that stay with w4a16_tc.cu, or leave it for less than 129."""
+    from zhilight_b200 import ops
+    w, packed = _setup(cuda, k, n, sym, 3)
+    x = _x(m, k, 1)
+    y = ops.w4a16_gemm_fused(x.to(cuda), packed, n, k, variant=1)
+    assert torch.equal(y, ops.w4a16_gemm_fused(x.to(cuda), packed, n, k, variant=1))
+    assert rel_l2(y.float().cpu().numpy(), gptq.gemm_f32(x.numpy(), w)) <= TOL
+
+
+@pytest.mark.parametrize("m", [150, 400])
+def test_bias_residual_swiglu(lib, cuda, m):
+    from zhilight_b200 import ops
+    k, f, n = 1024, 1344, 384
+    w, packed = _setup(cuda, k, 2 * f, False, 7, ops.swiglu_row_map(f, cuda))
+    x = _x(m, k, 9)
+    y = ops.w4a16_gemm_fused(x.to(cuda), packed, 2 * f, k, epilogue=ops.EPI_SWIGLU, variant=1).float().cpu().numpy()
+    gu = oops._t(gptq.gemm_f32(x.numpy(), w), "f16")
+    assert rel_l2(y, gu[:, :f] / (1.0 + np.exp(-gu[:, :f])) * gu[:, f:]) <= 2e-3
+    w2, packed2 = _setup(cuda, k, n, True, 4)
+    g = torch.Generator().manual_seed(2)
+    bias, res = (torch.randn(n, generator=g) * 0.5).half(), torch.randn(m, n, generator=g).half()
+    y2 = ops.w4a16_gemm_fused(x.to(cuda), packed2, n, k, bias=bias.to(cuda), residual=res.to(cuda), epilogue=ops.EPI_RESIDUAL, variant=1)
+    lin = oops._t(gptq.gemm_f32(x.numpy(), w2) + bias.float().numpy(), "f16")
+    assert rel_l2(y2.float().cpu().numpy(), oops._t(lin + res.float().numpy(), "f16")) <= TOL
+    h = res.to(cuda)                                    # the residual stream is updated in place
+    ops.w4a16_gemm_fused(x.to(cuda), packed2, n, k, bias=bias.to(cuda), residual=h, epilogue=ops.EPI_RESIDUAL, variant=1, out=h)
+    assert torch.equal(h, y2)
+
+
+@pytest.mark.parametrize("d,hq,hkv,k,t", [(128, 4, 2, 512, 140), (64, 4, 2, 256, 300), (128, 8, 1, 1024, 257)])
+def test_qkv_rope_epilogue(lib, cuda, d, hq, hkv, k, t):
+    from zhilight_b200 import ops
+    n = (hq + 2 * hkv) * d
+    _, packed = _setup(cuda, k, n, False, 14, ops.qkv_rope_row_map(hq + 2 * hkv, d, cuda))
+    _, plain = _setup(cuda, k, n, False, 14)
+    x = _x(t, k, 8).to(cuda)
+    pos = torch.tensor([(5 * i) % 61 for i in range(t)], dtype=torch.int32, device=cuda)
+    cos, sin = ops.rope_cos_sin(pos, d, 10000.0)
+    tb = torch.tensor([i % 3 for i in range(t)], dtype=torch.int32, device=cuda)
+    pl = torch.tensor([-1 if i == 7 else i // 3 for i in range(t)], dtype=torch.int32, device=cuda)   # a token that is not cached
+    bufs = [[torch.zeros(t // 3 + 2, hkv, d, dtype=torch.float16, device=cuda) for _ in range(3)] for _ in range(4)]
+    q = ops.w4a16_gemm_fused(x, packed, n, k, epilogue=ops.EPI_QKV_ROPE, variant=1,
+                             rope=dict(cos=cos, sin=sin, token_batch=tb, placement=pl, k_bufs=bufs[0], v_bufs=bufs[1], num_heads=hq,
+                                       num_kv_heads=hkv, dim_head=d))
+    q2 = ops.qkv_rope_append(cos, sin, ops.w4a16_gemm_fused(x, plain, n, k, variant=1), tb, pl, bufs[2], bufs[3], hq, hkv, d)
+    torch.testing.assert_close(q, q2, rtol=2 ** -9, atol=3e-3)
+    for a, b in zip(bufs[0] + bufs[1], bufs[2] + bufs[3]):
+        torch.testing.assert_close(a, b, rtol=2 ** -9, atol=3e-3)
+    assert float(bufs[0][0].abs().max()) > 0
+
+
+def test_strided_activations(lib, cuda):
+    from zhilight_b200 import ops
+    w, packed = _setup(cuda, 512, 256, False, 21)
+    x = torch.randn(200, 576, generator=torch.Generator().manual_seed(3)).half().to(cuda)[:, :512]
+    y = ops.w4a16_gemm_fused(x, packed, 256, 512, variant=1).float().cpu().numpy()
+    assert rel_l2(y, gptq.gemm_f32(x.cpu().numpy(), w)) <= TOL

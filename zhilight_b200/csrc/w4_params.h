@@ -52,6 +52,10 @@ cudaError_t prepare_w4_v3();
 cudaError_t launch_w4_tc(const W4Params& p, bool pdl, cudaStream_t stream);
 bool w4_tc_supports(int mc, int N, int K);
 cudaError_t prepare_w4_tc();
+// the same over pairs of SMs for prompt-sized M, all rows in one launch (w4a16_tc2.cu)
+cudaError_t launch_w4_tc2(const W4Params& p, bool pdl, cudaStream_t stream);
+bool w4_tc2_route(int M, int N, int K);
+cudaError_t prepare_w4_tc2();
 cudaError_t prepare_w8_tc();   // w8_tc.cu
 
 }  // namespace zl

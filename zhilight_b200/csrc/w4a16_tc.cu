@@ -33,10 +33,7 @@
 // quarter-warp read 16-byte chunks 64 B apart -- a 4-way bank conflict in the plain record layout -- so the nibble words
 // arrive through a tensor map with 64-byte swizzle (chunk ^= (row >> 1) & 3): conflict-free, the HBM format is unchanged.
 // The 80-byte scale / zero trailers of the four records of a stage come through a second (unswizzled) map.
-#include "common.cuh"
-#include "w4_layout.cuh"
-#include "w4_params.h"
-#include "tc_common.cuh"
+#include "w4a16_tc.cuh"
 
 #include <cstdlib>
 #include <map>
@@ -44,30 +41,6 @@
 #include <tuple>
 
 namespace zl {
-
-struct alignas(64) W4TcParams {
-    CUtensorMap xmap;           // x (M, K) fp16 row-major, box {64, NTOK}, 128-byte swizzle
-    CUtensorMap wmap;           // ZLW4I nibble words as [N/32][G][32 rows][64 B], box {64 B, 32, 1, 4}, 64-byte swizzle
-    CUtensorMap tmap;           // the 80-byte scale / zero trailers as [N/32][G][80 B], box {80 B, 1, 4}
-    const uint8_t* packed;      // ZLW4I
-    const __half* bias;         // indexed by PACKED row
-    const __half* residual;
-    __half* y;
-    int M, N, K, epi;
-    int dbg;                    // ZL_TC_DBG timing ablations (results are wrong): 1 no x loads, 2 no dequant, 4 no MMA, 8 no weight loads
-    uint2* ws;                  // [2 * CTA + slot][M][128] tagged words {fp32 partial sum, tag}: all zero between launches
-    float* ws_f32;              // plain scratch (its last MB carries the ZL_TC_DBG trace)
-    unsigned* err;              // watchdog code
-    long long* trace;           // ZL_TC_DBG & 16: clock64 stamps of CTA 0, [role][64 stages][8]
-    const float* cos;
-    const float* sin;
-    __half* q_out;
-    const int32_t* token_batch;
-    const int32_t* placement;
-    __half* const* k_addrs;
-    __half* const* v_addrs;
-    int num_heads, num_kv_heads, dim_head;
-};
 
 // instruction descriptor, kind::f16: D f32 (bits 4-5 = 1), A/B f16 (0), both K-major, N >> 3 at bit 17, M >> 4 at bit 24
 __host__ __device__ constexpr uint32_t tc_idesc_f16(int n) {
@@ -80,80 +53,6 @@ __device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, 
         "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accum)
         : "memory");
 }
-
-// ---- epilogue of 16 tokens (c0 .. c0+15) for the weight row owned by this lane -----------------------------------------
-// Packed row p = tile * 128 + 32 * quadrant + lane.  Inside a 32-row block, rows (16 tt + g) and (16 tt + g + 8) are
-// partners (gate / up, RoPE low / high half): lane and lane + 8.
-// the epilogue warps share their schedulers with the dequant warps, which are issue-bound: SiLU through the fast exp / divide
-// (2 ulp of fp32, invisible after the fp16 rounding of the product)
-__device__ __forceinline__ float tc_silu(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
-
-__device__ __forceinline__ void tc_epilogue16(const W4TcParams& p, int prow, int lane, int c0, float (&v)[16],
-                                              const uint32_t* rpre = nullptr) {   // rpre: 16 residual halves, packed in pairs
-    const float b = p.bias ? __half2float(p.bias[prow]) : 0.f;
-    if (p.epi == ZL_EPI_SWIGLU) {
-        const int n_out = p.N / 2;
-        const int col = (prow >> 5) * 16 + ((lane >> 4) << 3) + (lane & 7);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const float mine = __half2float(__float2half_rn(v[i] + b));
-            const float up = __shfl_down_sync(0xffffffffu, mine, 8);
-            const int tok = c0 + i;
-            if (!(lane & 8) && tok < p.M) p.y[(size_t)tok * n_out + col] = __float2half_rn(tc_silu(mine) * up);
-        }
-    } else if (p.epi == ZL_EPI_QKV_ROPE) {
-        const int d = p.dim_head, half_dim = d / 2, tiles_per_head = d / 32;
-        const int st = prow >> 5, head = st / tiles_per_head, jt = st % tiles_per_head;
-        const int c = jt * 16 + ((lane >> 4) << 3) + (lane & 7);
-        const bool is_v = head >= p.num_heads + p.num_kv_heads;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const float lo = __half2float(__float2half_rn(v[i] + b));
-            const float hi = __shfl_down_sync(0xffffffffu, lo, 8);
-            const int tok = c0 + i;
-            if ((lane & 8) || tok >= p.M) continue;
-            __half olo, ohi;
-            if (is_v) {
-                olo = __float2half_rn(lo);
-                ohi = __float2half_rn(hi);
-            } else {
-                const float* cs = p.cos + (size_t)tok * d;
-                const float* sn = p.sin + (size_t)tok * d;
-                olo = __float2half_rn(lo * cs[c] - hi * sn[c]);
-                ohi = __float2half_rn(hi * cs[c + half_dim] + lo * sn[c + half_dim]);
-            }
-            if (head < p.num_heads) {
-                __half* dst = p.q_out + ((size_t)tok * p.num_heads + head) * d;
-                dst[c] = olo;
-                dst[c + half_dim] = ohi;
-            } else {
-                const int pl = p.placement[tok];
-                if (pl >= 0) {
-                    const bool is_k = !is_v;
-                    const int hk = is_k ? head - p.num_heads : head - p.num_heads - p.num_kv_heads;
-                    __half* base = (is_k ? p.k_addrs : p.v_addrs)[p.token_batch[tok]];
-                    __half* dst = base + ((size_t)pl * p.num_kv_heads + hk) * d;
-                    dst[c] = olo;
-                    dst[c + half_dim] = ohi;
-                }
-            }
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const int tok = c0 + i;
-            if (tok >= p.M) continue;
-            __half h = __float2half_rn(v[i] + b);
-            if (p.epi == ZL_EPI_RESIDUAL) {
-                const __half r = rpre ? __ushort_as_half((unsigned short)(rpre[i >> 1] >> ((i & 1) * 16)))
-                                      : p.residual[(size_t)tok * p.N + prow];
-                h = __float2half_rn(__half2float(h) + __half2float(r));
-            }
-            p.y[(size_t)tok * p.N + prow] = h;
-        }
-    }
-}
-
 
 template <int NTOK>
 struct TsCfg {
@@ -500,18 +399,9 @@ __global__ void __launch_bounds__(TsCfg<NTOK>::kThreads, 1) k_w4a16_ts(const __g
             tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * NTOK);
             uint2* wsp = whole ? nullptr : p.ws + ((size_t)sch.slot((int)blockIdx.x, tile) * p.M) * kTcRows + m;
-            // residual rows are one L2 round trip per 16-token chunk away: fetch the next chunk's while this one is processed
-            const bool pre = whole && p.epi == ZL_EPI_RESIDUAL;
+            const bool pre = whole && p.epi == ZL_EPI_RESIDUAL && p.wide;
             uint32_t rnext[8];
-            auto fetch_res = [&](int c0) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const uint32_t lo = (c0 + 2 * i < p.M) ? __half_as_ushort(p.residual[(size_t)(c0 + 2 * i) * p.N + prow]) : 0u;
-                    const uint32_t hi = (c0 + 2 * i + 1 < p.M) ? __half_as_ushort(p.residual[(size_t)(c0 + 2 * i + 1) * p.N + prow]) : 0u;
-                    rnext[i] = lo | (hi << 16);
-                }
-            };
-            if (pre) fetch_res(0);
+            if (pre) tc_fetch_residual(p, prow, lane, 0, rnext);
 #pragma unroll 1
             for (int c0 = 0; c0 < NTOK; c0 += 16) {
                 if (c0 >= p.M) break;
@@ -526,7 +416,7 @@ __global__ void __launch_bounds__(TsCfg<NTOK>::kThreads, 1) k_w4a16_ts(const __g
                     uint32_t rcur[8];
 #pragma unroll
                     for (int i = 0; i < 8; ++i) rcur[i] = rnext[i];
-                    if (c0 + 16 < NTOK && c0 + 16 < p.M) fetch_res(c0 + 16);
+                    if (c0 + 16 < NTOK && c0 + 16 < p.M) tc_fetch_residual(p, prow, lane, c0 + 16, rnext);
                     tc_epilogue16(p, prow, lane, c0, v, rcur);
                 } else {
                     tc_epilogue16(p, prow, lane, c0, v);
@@ -715,15 +605,7 @@ static int tc_pick_ctas(int n_tiles, int G) {
     return (int)P;
 }
 
-cudaError_t launch_w4_tc(const W4Params& p, bool pdl, cudaStream_t stream) {
-    TcDeviceState* st = tc_state();
-    if (!st || !st->ws) return cudaErrorNotSupported;
-    const int ntok = p.mc <= 32 ? 32 : p.mc <= 64 ? 64 : p.mc <= 128 ? 128 : 256;
-    const int n_tiles = p.N / kTcRows, G = p.K / kW4GroupK;
-    W4TcParams q;
-    if (!tc_make_map_2d(&q.xmap, p.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)p.mc, (uint64_t)p.K, (uint64_t)p.ldx * 2,
-                        (uint32_t)ntok))
-        return cudaErrorInvalidValue;
+bool w4_tc_params(W4TcParams& q, const W4Params& p) {
     {
         // the weight maps depend only on (address, N, K): encode once per weight matrix (cuTensorMapEncodeTiled costs
         // microseconds of host time per call)
@@ -736,16 +618,16 @@ cudaError_t launch_w4_tc(const W4Params& p, bool pdl, cudaStream_t stream) {
         const auto key = std::make_tuple((const void*)p.packed, p.N, p.K);
         auto it = cache.find(key);
         if (it == cache.end()) {
-            const uint64_t nb = (uint64_t)p.N / 32;
-            const uint64_t wd[4] = {16, 32, (uint64_t)G, nb}, wstr[3] = {64, (uint64_t)kW4BlockBytes, (uint64_t)G * kW4BlockBytes};
+            const uint64_t G = (uint64_t)(p.K / kW4GroupK), nb = (uint64_t)p.N / 32;
+            const uint64_t wd[4] = {16, 32, G, nb}, wstr[3] = {64, (uint64_t)kW4BlockBytes, G * kW4BlockBytes};
             const uint32_t wbox[4] = {16, 32, 1, 4};
-            const uint64_t td[3] = {20, (uint64_t)G, nb}, tstr[2] = {(uint64_t)kW4BlockBytes, (uint64_t)G * kW4BlockBytes};
+            const uint64_t td[3] = {20, G, nb}, tstr[2] = {(uint64_t)kW4BlockBytes, G * kW4BlockBytes};
             const uint32_t tbox[3] = {20, 1, 4};
             WMaps m;
             if (!tc_make_map_nd(&m.w, p.packed, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, wd, wstr, wbox, CU_TENSOR_MAP_SWIZZLE_64B) ||
                 !tc_make_map_nd(&m.t, p.packed + kW4ScaleOff, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, td, tstr, tbox,
                                 CU_TENSOR_MAP_SWIZZLE_NONE))
-                return cudaErrorInvalidValue;
+                return false;
             if (cache.size() > 4096) cache.clear();
             it = cache.emplace(key, m).first;
         }
@@ -760,14 +642,6 @@ cudaError_t launch_w4_tc(const W4Params& p, bool pdl, cudaStream_t stream) {
     q.N = p.N;
     q.K = p.K;
     q.epi = p.epi;
-    {
-        static const int tc_dbg = getenv("ZL_TC_DBG") ? atoi(getenv("ZL_TC_DBG")) : 0;
-        q.dbg = tc_dbg;
-    }
-    q.ws = st->ws_ll;
-    q.ws_f32 = st->ws;
-    q.err = st->err;
-    q.trace = reinterpret_cast<long long*>(reinterpret_cast<uint8_t*>(st->ws) + st->ws_bytes - (1 << 20));   // last MB of the workspace
     q.cos = p.cos;
     q.sin = p.sin;
     q.q_out = p.q_out;
@@ -778,6 +652,34 @@ cudaError_t launch_w4_tc(const W4Params& p, bool pdl, cudaStream_t stream) {
     q.num_heads = p.num_heads;
     q.num_kv_heads = p.num_kv_heads;
     q.dim_head = p.dim_head;
+    q.dbg = 0;
+    q.ws = nullptr;
+    q.ws_f32 = nullptr;
+    q.trace = nullptr;
+    q.err = nullptr;
+    q.ntok = q.tok_tiles = 0;
+    q.wide = ((reinterpret_cast<uintptr_t>(p.y) | reinterpret_cast<uintptr_t>(p.residual)) & 3) == 0;
+    return true;
+}
+
+cudaError_t launch_w4_tc(const W4Params& p, bool pdl, cudaStream_t stream) {
+    TcDeviceState* st = tc_state();
+    if (!st || !st->ws) return cudaErrorNotSupported;
+    const int ntok = p.mc <= 32 ? 32 : p.mc <= 64 ? 64 : p.mc <= 128 ? 128 : 256;
+    const int n_tiles = p.N / kTcRows, G = p.K / kW4GroupK;
+    W4TcParams q;
+    if (!tc_make_map_2d(&q.xmap, p.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)p.mc, (uint64_t)p.K, (uint64_t)p.ldx * 2,
+                        (uint32_t)ntok))
+        return cudaErrorInvalidValue;
+    if (!w4_tc_params(q, p)) return cudaErrorInvalidValue;
+    {
+        static const int tc_dbg = getenv("ZL_TC_DBG") ? atoi(getenv("ZL_TC_DBG")) : 0;
+        q.dbg = tc_dbg;
+    }
+    q.ws = st->ws_ll;
+    q.ws_f32 = st->ws;
+    q.err = st->err;
+    q.trace = reinterpret_cast<long long*>(reinterpret_cast<uint8_t*>(st->ws) + st->ws_bytes - (1 << 20));   // last MB of the workspace
     const int ctas = tc_pick_ctas(n_tiles, G);
     if ((size_t)2 * ctas * p.mc * kTcRows * 8 > st->ws_ll_bytes) return cudaErrorInvalidValue;
     const dim3 grid(ctas);

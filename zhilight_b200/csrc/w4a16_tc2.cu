@@ -1,0 +1,351 @@
+// W4A16 GEMM for prompt-sized M: tcgen05.mma over pairs of SMs (cta_group::2), the dequantised weights as the A operand in tensor
+// memory.  Same arithmetic contract as w4a16_tc.cu (w = (q - z) * s rounded to fp16 once, fp16 x fp16 products, fp32 accumulation
+// over all of K) and the same packed weights, maps, conversion and epilogues.
+//
+// What bounded w4a16_tc.cu at 256 tokens (28672 x 4096: 115 us, 523 TFLOP/s): one accumulator leaves no MMA under an epilogue, and
+// cutting the tiles into one range per CTA makes two of a CTA's two or three pieces partial ones that travel through L2 as tagged
+// words.  Here
+//   * a tile is 256 rows of w by up to 256 tokens over two SMs: each converts its own 128 rows and loads half of the tokens;
+//   * tiles are whole, taken in turn by persistent pairs; the token tile's size is chosen so that the last wave is full;
+//   * up to 128 tokens there are two accumulators; with one, eight epilogue warps shorten the gap.
+// 28672 x 4096 with SwiGLU: 1000 tokens 499 -> 197 us, 256 tokens 128 -> 61; 4096 x 14336 with the residual: 1000 tokens 408 -> 91 us
+// (1290 TFLOP/s).  Bound by the tensor cores at 256 tokens (1030 cycles per 128-k group for 1024 of MMA, at the clock that the power limit
+// leaves); below 200 tokens by the hand-over of a group (830 cycles; two groups per stage were slower, 2380 per stage: too few slots).
+//
+//   warps 0-7    epilogue : quadrant = warp % 4, 16-token chunks in turns
+//   warps 8-23   dequant  : four groups of four take the stages (one 128-k group each) in turn, one group per stage slot; lane =
+//                           weight row, quadrant = warp % 4; their arrivals of both CTAs meet on the leader's barrier
+//   warp 24      weights  : tensor-TMA of the 4 ZLW4I records of a stage and their trailers, this CTA's 128 rows
+//   warp 25      x        : this CTA's half of the tokens, counted on the leader's barrier
+//   warp 26      MMA      : of the leader, 8 x 256 x ntok x 16 per stage; TMEM allocation
+#include "tc2_common.cuh"
+#include "w4a16_tc.cuh"
+
+namespace zl {
+
+struct T2Cfg {
+    static constexpr int kEpiWarps = 8, kDqWarps = 16, kGroupWarps = 4;
+    static constexpr int kWarpDq0 = kEpiWarps, kWarpRaw = kWarpDq0 + kDqWarps, kWarpX = kWarpRaw + 1, kWarpMma = kWarpRaw + 2;
+    static constexpr int kThreads = (kWarpMma + 1) * 32;
+    static constexpr int AS = 4;                                       // stages of A (TMEM, 64 columns each) and x (shared memory)
+    static constexpr int RS = 8;                                       // stages of packed weights
+    static constexpr int kACol0 = 256;                                 // accumulators: columns 0 .. 255
+    static constexpr int kXStage = 2 * 128 * 128;                      // [64-k atom][up to 128 tokens][128 B]
+    static constexpr int kNib = 4 * 2048, kTr = 384;                   // four records' nibbles; their 80-byte trailers, padded
+    static constexpr int kNibOff = AS * kXStage;
+    static constexpr int kTrOff = kNibOff + RS * kNib;
+    static constexpr int kBarOff = kTrOff + RS * kTr;
+    static constexpr int kMiscOff = kBarOff + (2 * RS + 2 * AS + 4) * 8;
+    static constexpr int kBytes = kMiscOff + 16 + 1024;                // + slack for the manual 1024-byte alignment
+    static_assert(kACol0 + AS * 64 <= 512, "TMEM columns");
+    static_assert(kBytes <= 232448, "shared memory");
+};
+
+// code of the last wait that gave up (0: none)
+__device__ unsigned g_w4_tc2_err;
+
+struct T2Tile {
+    int n0, t0, ntok;   // first row of w of the pair, first token, tokens (a multiple of 32)
+};
+__device__ __forceinline__ bool t2_tile(const W4TcParams& p, int i, T2Tile& t) {
+    const int rt = i / p.tok_tiles;
+    t.n0 = rt * kTc2Rows;
+    t.t0 = (i - rt * p.tok_tiles) * p.ntok;
+    t.ntok = min(p.ntok, (p.M - t.t0 + 31) & ~31);
+    return t.n0 < p.N;
+}
+
+__global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_constant__ W4TcParams p) {
+    using C = T2Cfg;
+    extern __shared__ uint8_t smem_dyn[];
+    uint8_t* smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
+    uint64_t* raw_full = reinterpret_cast<uint64_t*>(smem + C::kBarOff);
+    uint64_t* raw_empty = raw_full + C::RS;
+    uint64_t* a_full = raw_empty + C::RS;      // leader's: a dequant group of each CTA, and the x bytes of both
+    uint64_t* ax_empty = a_full + C::AS;
+    uint64_t* acc_full = ax_empty + C::AS;
+    uint64_t* acc_empty = acc_full + 2;        // leader's: the epilogue warps of both CTAs
+    uint32_t* s_tmem = reinterpret_cast<uint32_t*>(smem + C::kMiscOff);
+    volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank();
+    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const int G = p.K / kW4GroupK;
+    const int nacc = p.ntok <= 128 ? 2 : 1;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < C::RS; ++i) {
+            mbar_init(&raw_full[i], 1);
+            mbar_init(&raw_empty[i], C::kGroupWarps);
+        }
+        for (int i = 0; i < C::AS; ++i) {
+            mbar_init(&a_full[i], 2 * C::kGroupWarps + 1);
+            mbar_init(&ax_empty[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&acc_full[i], 1);
+            mbar_init(&acc_empty[i], 2 * C::kEpiWarps);
+        }
+        *s_abort = 0;
+        mbar_fence_init();
+    }
+    if (warp == C::kWarpMma) tc2_alloc(s_tmem);
+    pdl_trigger();
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();   // both CTAs' barriers and allocations are in place
+    tc_fence_after();
+    const uint32_t tmem = *s_tmem;
+    T2Tile t;
+
+    if (warp == C::kWarpRaw) {
+        // constants: may run ahead of the predecessor kernel (PDL).  The row tiles of one wave are read by several pairs and again
+        // by the next token tiles: no evict-first hint here
+        int rs = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int i = pair; ok && t2_tile(p, i, t); i += pairs) {
+            const int rec = (t.n0 + (int)rank * 128) / 32;
+            for (int g = 0; g < G; ++g) {
+                if (!(ok = tc2_wait(&raw_empty[rs], ph ^ 1u, s_abort, &g_w4_tc2_err, 0x3100 + rs))) break;
+                if (tc_elect_one()) {
+                    mbar_expect_tx(&raw_full[rs], C::kNib + 4 * 80);
+                    asm volatile(
+                        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(
+                            smem_u32(smem + C::kNibOff + rs * C::kNib)),
+                        "l"(reinterpret_cast<uint64_t>(&p.wmap)), "r"(0), "r"(0), "r"(g), "r"(rec), "r"(smem_u32(&raw_full[rs]))
+                        : "memory");
+                    asm volatile(
+                        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+                            smem_u32(smem + C::kTrOff + rs * C::kTr)),
+                        "l"(reinterpret_cast<uint64_t>(&p.tmap)), "r"(0), "r"(g), "r"(rec), "r"(smem_u32(&raw_full[rs]))
+                        : "memory");
+                }
+                __syncwarp();
+                if (++rs == C::RS) {
+                    rs = 0;
+                    ph ^= 1u;
+                }
+            }
+        }
+    } else if (warp == C::kWarpX) {
+        pdl_wait();   // activations: produced by the predecessor kernel
+        int as = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        const int box = p.ntok >> 1;   // rows of a load; a shorter last tile loads rows it does not use
+        for (int i = pair; ok && t2_tile(p, i, t); i += pairs) {
+            const int tb = t.t0 + (int)rank * (t.ntok >> 1);
+            for (int g = 0; g < G; ++g) {
+                if (!(ok = tc2_wait(&ax_empty[as], ph ^ 1u, s_abort, &g_w4_tc2_err, 0x3200 + as))) break;
+                if (tc_elect_one()) {
+                    if (rank == 0) mbar_expect_tx(&a_full[as], (uint32_t)(4 * box * 128));
+                    const uint32_t bar = cluster_map(smem_u32(&a_full[as]), 0);
+                    uint8_t* dst = smem + as * C::kXStage;
+                    tma2_load_3d(dst, &p.xmap, g * kW4GroupK, tb, 0, bar);
+                    tma2_load_3d(dst + box * 128, &p.xmap, g * kW4GroupK + 64, tb, 0, bar);
+                }
+                __syncwarp();
+                if (++as == C::AS) {
+                    as = 0;
+                    ph ^= 1u;
+                }
+            }
+        }
+    } else if (warp == C::kWarpMma) {
+        if (rank == 0) {
+            int as = 0, acc = 0;
+            uint32_t ph = 0, acc_ph = 0;
+            bool ok = true;
+            const uint64_t atom = (uint64_t)(((p.ntok >> 1) * 128) >> 4);   // descriptor step from k 0..63 to k 64..127 of a stage
+            for (int i = pair; ok && t2_tile(p, i, t); i += pairs) {
+                if (!(ok = tc2_wait(&acc_empty[acc], acc_ph ^ 1u, s_abort, &g_w4_tc2_err, 0x3300 + acc))) break;
+                tc_fence_after();
+                const uint32_t d = tmem + (uint32_t)(acc * 128), idesc = tc2_idesc(false, t.ntok);
+                for (int g = 0; g < G; ++g) {
+                    if (!(ok = tc2_wait(&a_full[as], ph, s_abort, &g_w4_tc2_err, 0x3400 + as))) break;
+                    tc_fence_after();
+                    if (tc_elect_one()) {
+                        const uint32_t a = tmem + (uint32_t)(C::kACol0 + as * 64);
+                        const uint64_t xd = tc_desc_sw128(smem_u32(smem + as * C::kXStage));
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            tc2_mma_ts(d, a + (uint32_t)(j * 8), xd + (j >> 2) * atom + (uint64_t)((j & 3) * 2), idesc, (g > 0 || j > 0) ? 1u : 0u);
+                        tc2_commit(&ax_empty[as]);
+                        if (g == G - 1) tc2_commit(&acc_full[acc]);
+                    }
+                    __syncwarp();
+                    if (++as == C::AS) {
+                        as = 0;
+                        ph ^= 1u;
+                    }
+                }
+                if (++acc == nacc) {
+                    acc = 0;
+                    acc_ph ^= 1u;
+                }
+            }
+        }
+    } else if (warp >= C::kWarpDq0) {
+        const int as = (warp - C::kWarpDq0) >> 2, q = warp & 3;   // the group's stage slot
+        const int tt = lane >> 4, hi = (lane >> 3) & 1, g8 = lane & 7;
+        const uint32_t mask = hi ? 0xf0f0f0f0u : 0x0f0f0f0fu;
+        const uint32_t magic = hi ? 0x54545454u : 0x64646464u;   // 64 + n / 16 for a high nibble n, 1024 + n for a low one
+        const uint32_t sw = (uint32_t)(g8 >> 1) & 3u;            // the map's 64-byte swizzle: chunk ^= (row >> 1) & 3
+        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(C::kACol0 + as * 64);
+        const uint32_t full = cluster_map(smem_u32(&a_full[as]), 0);
+        int st = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int i = pair; ok && t2_tile(p, i, t); i += pairs) {
+            for (int g = 0; g < G; ++g, ++st) {
+                if (st % C::AS != as) continue;
+                const int rs = st % C::RS;
+                if (!(ok = tc2_wait(&raw_full[rs], (uint32_t)(st / C::RS) & 1u, s_abort, &g_w4_tc2_err, 0x3600 + rs))) break;
+                const uint8_t* nib = smem + C::kNibOff + rs * C::kNib + q * 2048;
+                const uint8_t* tr = smem + C::kTrOff + rs * C::kTr + q * 80;
+                const __half2 sc2 = *reinterpret_cast<const __half2*>(tr + (tt * 8 + g8) * 4);
+                const int zz = tr[64 + tt * 8 + g8];
+                const __half2 cz = __float2half2_rn(hi ? (float)(64 + (zz >> 4)) : (float)(1024 + (zz & 0xF)));
+                const __half2 s2 = hi ? __half2half2(__high2half(sc2)) : __half2half2(__low2half(sc2));
+#pragma unroll
+                for (int ks = 0; ks < 2; ++ks) {    // 64 k at a time: 32 columns
+                    uint4 wv[4];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        // 16-k chunk kc of the group: k = 32 t + 16 hh + ..., record row (2 tt + hh) * 8 + g, chunk t
+                        const int kc = ks * 4 + c, tq = kc >> 1, hh = kc & 1;
+                        wv[c] = *reinterpret_cast<const uint4*>(nib + ((tt * 2 + hh) * 8 + g8) * 64 + (((uint32_t)tq ^ sw) << 4));
+                    }
+                    if (ks == 1) {
+                        __syncwarp();               // every lane's shared-memory reads of the stage have returned
+                        if (lane == 0) mbar_arrive(&raw_empty[rs]);
+                    }
+                    uint32_t r[2][16];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const uint32_t words[4] = {wv[c].x, wv[c].y, wv[c].z, wv[c].w};
+#pragma unroll
+                        for (int wq = 0; wq < 4; ++wq) {
+                            const uint32_t wm = words[wq] & mask;
+                            uint32_t a0 = __byte_perm(wm, magic, 0x4140), a1 = __byte_perm(wm, magic, 0x4342);
+                            __half2 v0 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&a0), cz), s2);
+                            __half2 v1 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&a1), cz), s2);
+                            r[c >> 1][(c & 1) * 8 + wq * 2] = *reinterpret_cast<uint32_t*>(&v0);
+                            r[c >> 1][(c & 1) * 8 + wq * 2 + 1] = *reinterpret_cast<uint32_t*>(&v1);
+                        }
+                    }
+                    if (ks == 0) {
+                        if (!(ok = tc2_wait(&ax_empty[as], ph ^ 1u, s_abort, &g_w4_tc2_err, 0x3700 + as))) break;
+                        tc_fence_after();
+                    }
+                    tc_st16(taddr + (uint32_t)(ks * 32), r[0]);
+                    tc_st16(taddr + (uint32_t)(ks * 32 + 16), r[1]);
+                }
+                if (!ok) break;
+                ph ^= 1u;
+                tc_wait_st();
+                tc_fence_before();
+                __syncwarp();                       // one arrival per warp
+                if (lane == 0) mbar_arrive_at(full);
+            }
+        }
+    } else {
+        const int q = warp & 3, set = warp >> 2;
+        int acc = 0;
+        uint32_t acc_ph = 0;
+        pdl_wait();
+        for (int i = pair; t2_tile(p, i, t); i += pairs) {
+            const int prow = t.n0 + (int)rank * 128 + q * 32 + lane;
+            const bool res = p.epi == ZL_EPI_RESIDUAL && p.wide && prow < p.N;
+            uint32_t rnext[8];
+            if (res) tc_fetch_residual(p, prow, lane, t.t0 + set * 16, rnext);
+            if (!tc2_wait(&acc_full[acc], acc_ph, s_abort, &g_w4_tc2_err, 0x3800 + acc)) break;
+            tc_fence_after();
+            const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * 128);
+            if (prow < p.N) {               // N % 128 == 0: all of the CTA's rows or none
+                for (int c0 = set * 16; c0 < t.ntok && t.t0 + c0 < p.M; c0 += 32) {
+                    float v[16];
+                    tc_ld16(taddr + (uint32_t)c0, v);
+                    if (res) {
+                        uint32_t rcur[8];
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) rcur[u] = rnext[u];
+                        if (c0 + 32 < t.ntok) tc_fetch_residual(p, prow, lane, t.t0 + c0 + 32, rnext);
+                        tc_epilogue16(p, prow, lane, t.t0 + c0, v, rcur);
+                    } else {
+                        tc_epilogue16(p, prow, lane, t.t0 + c0, v);
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_at(cluster_map(smem_u32(&acc_empty[acc]), 0));
+            if (++acc == nacc) {
+                acc = 0;
+                acc_ph ^= 1u;
+            }
+        }
+    }
+    __syncwarp();
+    tc2_drain(s_abort);
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();   // nobody's shared memory or TMEM goes while the other CTA may still use it
+    if (warp == C::kWarpMma) {
+        tc_fence_after();
+        tc2_dealloc(tmem);
+    }
+}
+
+// ---- host side --------------------------------------------------------------------------------------------------------
+cudaError_t prepare_w4_tc2() {
+    return cudaFuncSetAttribute(k_w4a16_tc2, cudaFuncAttributeMaxDynamicSharedMemorySize, T2Cfg::kBytes);
+}
+
+// Tokens per tile: the waves of the launch times a tile's cost.  A 128-k group costs its MMAs (4 cycles per token) or the conversion and
+// hand-over of its weights (830 cycles), whichever is longer; with one accumulator the epilogue comes on top.
+static double t2_cost(int n, long long tiles, int G, int pairs) {
+    const double group = 4.0 * n > 830.0 ? 4.0 * n : 830.0;
+    return (double)((tiles + pairs - 1) / pairs) * (G * group + (n > 128 ? 16.0 * n : 500.0));
+}
+static int t2_pick_ntok(int M, int row_tiles, int G, int pairs) {
+    int best = 32;
+    for (int n = 32; n <= 256; n += 32) {
+        if (t2_cost(n, (long long)row_tiles * cdiv(M, n), G, pairs) < t2_cost(best, (long long)row_tiles * cdiv(M, best), G, pairs)) best = n;
+        if (n >= M) break;
+    }
+    return best;
+}
+
+// Whether M tokens are this kernel's.  Beyond 256 w4a16_tc.cu would need several passes; below, whole tiles on few pairs stand against
+// its ranges over all SMs and their exchange: 10 us + 4.2 ns per token and million weights.  Measured, this kernel against that one:
+// 28672 x 4096 at M = 32 / 64 / 128: 34 / 35 / 39 against 34 / 41 / 60 us; 4096 x 14336 at M = 128 / 192 / 256: 51 / 52 / 54 against
+// 39 / 56 / 64; 6144 x 4096 at M = 64 / 128: 22 / 23 against 21 / 32; 4096 x 4096 at M = 128 / 192: 22 / 23 against 21 / 27.
+bool w4_tc2_route(int M, int N, int K) {
+    if (M <= 16 || N % kTcRows || K % kW4GroupK) return false;
+    if (M > 256) return true;
+    const int row_tiles = cdiv(N, kTc2Rows), G = K / kW4GroupK, pairs = device_sm_count() / 2, n = t2_pick_ntok(M, row_tiles, G, pairs);
+    const double here = 5.0 + t2_cost(n, (long long)row_tiles * cdiv(M, n), G, pairs) / 1900.0;
+    return here < 10.0 + 4.2e-9 * M * (double)N * K;
+}
+
+// all M tokens in one launch
+cudaError_t launch_w4_tc2(const W4Params& p, bool pdl, cudaStream_t stream) {
+    const int row_tiles = cdiv(p.N, kTc2Rows), G = p.K / kW4GroupK, max_pairs = device_sm_count() / 2;
+    W4TcParams q;
+    if (!w4_tc_params(q, p)) return cudaErrorInvalidValue;
+    q.ntok = t2_pick_ntok(p.mc, row_tiles, G, max_pairs);
+    q.tok_tiles = cdiv(p.mc, q.ntok);
+    if (!tc2_map_3d(&q.xmap, p.x, false, p.K, p.mc, 1, p.ldx, 0, q.ntok / 2)) return cudaErrorInvalidValue;
+    const int tiles = row_tiles * q.tok_tiles;
+    return launch_pairs(k_w4a16_tc2, tiles < max_pairs ? tiles : max_pairs, dim3(T2Cfg::kThreads), (size_t)T2Cfg::kBytes, stream, pdl, q);
+}
+
+}  // namespace zl
+
+extern "C" unsigned zl_w4_tc2_watchdog(void) {
+    unsigned v = 0;
+    cudaMemcpyFromSymbol(&v, zl::g_w4_tc2_err, sizeof v);
+    return v;
+}
