@@ -131,3 +131,28 @@ def test_fp8_quant_one_and_two_launches_bit_exact(lib, cuda, tag, n):
         ov, os_ = oracle.fp8_quant_per_tensor(x, dtype=tag)
         assert s.item() == os_
         np.testing.assert_array_equal(oracle.e4m3_decode(q.cpu().numpy()), ov)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,n,k", [(1, 33000, 4160), (9, 16384, 3136), (25, 4100, 12352), (33, 130, 64), (65, 1000, 192), (300, 257, 1088)])
+def test_products_on_pairs_of_sms(lib, cuda, dtype, m, n, k):
+    """The dispatch lines and the edges of the 256-row, 32-row and 128-byte tiles; odd row counts, K a multiple of 64 only."""
+    from zhilight_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(m)
+    r = lambda *s: torch.rand(*s, generator=g, device="cuda")  # noqa: E731
+    xq, w = (torch.randint(-127, 128, s, generator=g, device="cuda", dtype=torch.int8) for s in ((m, k), (n, k)))
+    sx, sw, b = r(m) * 0.01, r(n) * 0.01, (r(n) - 0.5).to(dtype)
+    acc = (xq.double() @ w.double().T).float()          # below 2^24 in magnitude or rounded as the kernel rounds its s32 sums
+    want = ((acc * sx[:, None]) * sw).to(dtype)
+    assert torch.equal(ops.w8a8_gemm(xq, sx, w, sw, dtype), want)
+    assert torch.equal(ops.w8a8_gemm(xq, sx, w, sw, dtype, bias=b), (want.float() + b.float()).to(dtype))
+    assert torch.equal(ops.w8a8_gemm(xq, sx, w, sw.to(dtype), dtype), ((acc * sx[:, None]) * sw.to(dtype).float()).to(dtype))
+    x8, w8 = (torch.randn(*s, generator=g, device="cuda").to(torch.float8_e4m3fn) for s in ((m, k), (n, k)))
+    one = r(1)
+    y = ops.w8a8_gemm(x8.view(torch.uint8), one, w8.view(torch.uint8), sw, dtype, ops.W8_FP8 if n == 1 else 2, bias=b)
+    ref = (x8.double() @ w8.double().T) * one.double() * sw.double() + b.double()
+    mag = (x8.double().abs() @ w8.double().abs().T) * one.double() * sw.double()
+    # an fp32 accumulator that may drop a unit in its last place per 32 products, and the output's rounding
+    lim = (k / 32 + 4) * 2.0 ** -23 * mag + 2.0 ** (-11 if dtype == torch.float16 else -8) * ref.abs() + 2.0 ** -24
+    assert not ((y.double() - ref).abs() > lim).any()
+    assert lib.zl_gemm_tc_watchdog() == 0

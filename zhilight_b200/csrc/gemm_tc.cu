@@ -16,6 +16,9 @@
 //   warps 4-11   epilogue  : quadrant = warp % 4, 16-row chunks of x in turns; lane = row of w = column of y
 //   warps 12-15  grouped   : rows of x through their index lists, by 16-byte cp.async into the swizzled layout that the boxes have;
 //                            a stage's barrier counts the copies as they land, warp 3 hands the stage to the MMAs
+//
+// The 8-bit Linears (zl_w8a8_gemm: Int8Linear, Fp8Linear) run on the same kernel: a stage is 128 bytes of k whatever the type, only the MMA
+// (kind::i8 with s32 accumulators, kind::f8f6f4) and the epilogue (scale-back, bias) are theirs.
 #include "gemm_common.cuh"
 #include "tc2_common.cuh"
 
@@ -24,13 +27,15 @@
 namespace zl {
 
 constexpr int kGtThreads = 12 * 32, kGtRowWarps = 4, kGtGroupThreads = kGtThreads + kGtRowWarps * 32, kGtEpiWarps = 8;
-constexpr int kGtStages = 6, kGtAStage = 128 * 128, kGtBStage = 128 * 128;
-constexpr int kGtBarOff = kGtStages * (kGtAStage + kGtBStage);
-constexpr int kGtMiscOff = kGtBarOff + (3 * kGtStages + 4) * 8;
+// The ring is cut into as many stages as fit, of blocks of 16 KB of w and 128 bytes per row of a CTA's half tile of x.
+constexpr int kGtRing = 204800, kGtMaxStages = 12, kGtAStage = 128 * 128;
+constexpr int kGtBarOff = kGtRing;
+constexpr int kGtMiscOff = kGtBarOff + (3 * kGtMaxStages + 4) * 8;
 constexpr int kGtMaxGroups = 1024;
 constexpr int kGtCumOff = kGtMiscOff + 16;                       // grouped: tiles before each group
 constexpr int kGtBytes = kGtCumOff + (kGtMaxGroups + 1) * 4 + 1024;   // + slack for the manual 1024-byte alignment
 static_assert(kGtBytes <= 232448, "shared memory");
+enum { kGt16 = 0, kGtInt8 = 1, kGtFp8 = 2 };
 
 struct alignas(64) GemmTcP {
     CUtensorMap wmap;           // w (K, N, batch), box 64 x 128
@@ -40,6 +45,11 @@ struct alignas(64) GemmTcP {
     int row_tiles, tok_tiles;   // tok_tiles: not grouped
     int ntok, box_rows;         // not grouped: rows of x of a tile, and of a box (a CTA's half of them)
     int wide;                   // two neighbouring values of y may be stored together
+    int stages, sub;            // stages of `sub` blocks: 128 bytes of k of w (16 KB) and of x
+    int block_bytes;
+    const float* sx;            // 8-bit: scales of the rows of x (int8) or one (fp8)
+    const void* sw;             // 8-bit: scales of the rows of w, or one
+    int sw_mode;                // 0: per row in y's type, 1 / 2: per row fp32, 3: one fp32
 };
 
 // code of the last wait that gave up (0: none)
@@ -77,6 +87,32 @@ __device__ __forceinline__ bool gt_tile(const GemmTcP& p, const int* s_cum, int 
     return true;
 }
 
+// 16 rows of y, column n of this lane; mine: row of y of token c0 + lane (grouped)
+template <typename TO>
+__device__ __forceinline__ void gt_put16(const GemmTcP& p, const GtTile& t, TO* y, int mine, int n, int c0, const float (&v)[16], int lane) {
+    const GemmP& g = p.g;
+    const int odd = lane & 1;
+    if (p.wide) {   // two columns of every other token per lane: half the stores, twice as wide
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float other = __shfl_xor_sync(0xffffffffu, odd ? v[2 * j] : v[2 * j + 1], 1);
+            const int m = t.t0 + c0 + 2 * j + odd;
+            const int row = g.grp_off ? __shfl_sync(0xffffffffu, mine, 2 * j + odd) : m;
+            struct alignas(2 * sizeof(TO)) Two {
+                TO a, b;
+            } two = {from_f32<TO>(odd ? other : v[2 * j]), from_f32<TO>(odd ? v[2 * j + 1] : other)};
+            if (n < g.N && m < t.M) *reinterpret_cast<Two*>(y + (size_t)row * g.ldy + (n & ~1)) = two;   // N is even
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int m = t.t0 + c0 + i;
+            const int row = g.grp_off ? __shfl_sync(0xffffffffu, mine, i) : m;
+            if (n < g.N && m < t.M) y[(size_t)row * g.ldy + n] = from_f32<TO>(v[i]);
+        }
+    }
+}
+
 template <typename T, typename TO, int EPI>
 __device__ __forceinline__ void gt_store16(const GemmTcP& p, const GtTile& t, int n, int c0, float (&v)[16], float bias, int lane) {
     const GemmP& g = p.g;
@@ -108,35 +144,37 @@ __device__ __forceinline__ void gt_store16(const GemmTcP& p, const GtTile& t, in
             const int m = t.t0 + c0 + i;
             v[i] = m < t.M && n < g.N ? gemm_epilogue<EPI>(v[i] + bias, g, t.b, m, n) : 0.f;
         }
-        if (p.wide) {   // two columns of every other token per lane: half the stores, twice as wide
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float other = __shfl_xor_sync(0xffffffffu, odd ? v[2 * j] : v[2 * j + 1], 1);
-                const int m = t.t0 + c0 + 2 * j + odd;
-                const int row = g.grp_off ? __shfl_sync(0xffffffffu, mine, 2 * j + odd) : m;
-                struct alignas(2 * sizeof(TO)) Two {
-                    TO a, b;
-                } two = {from_f32<TO>(odd ? other : v[2 * j]), from_f32<TO>(odd ? v[2 * j + 1] : other)};
-                if (n < g.N && m < t.M) *reinterpret_cast<Two*>(y + (size_t)row * g.ldy + (n & ~1)) = two;   // N is even
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int m = t.t0 + c0 + i;
-                const int row = g.grp_off ? __shfl_sync(0xffffffffu, mine, i) : m;
-                if (n < g.N && m < t.M) y[(size_t)row * g.ldy + n] = from_f32<TO>(v[i]);
-            }
-        }
+        gt_put16<TO>(p, t, y, mine, n, c0, v, lane);
     }
 }
 
-template <typename T, typename TO, bool GROUPED>
+// 8-bit: v are the raw accumulators (s32 bits or f32)
+template <typename TO, int KIND>
+__device__ __forceinline__ void gt_store16_8bit(const GemmTcP& p, const GtTile& t, int n, int c0, float (&v)[16], float s_w, float bias, bool has_bias,
+                                                int lane) {
+    const int mt = t.t0 + c0 + (lane & 15);
+    const float scales = KIND == kGtFp8 ? p.sx[0] * s_w : (mt < t.M ? p.sx[mt] : 0.f);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        if constexpr (KIND == kGtFp8) {
+            v[i] *= scales;                                       // cuBLASLt fp8: D = (scaleA * scaleB) * acc (+ bias)
+            if (has_bias) v[i] += bias;
+        } else {
+            // quant_scale_back (quant_kernel.cu:231-246): T(float(acc) * sx[m] * sw[n]), then add_bias in T
+            v[i] = __fmul_rn(__fmul_rn((float)__float_as_int(v[i]), __shfl_sync(0xffffffffu, scales, i)), s_w);
+            if (has_bias) v[i] = to_f32<TO>(from_f32<TO>(v[i])) + bias;
+        }
+    }
+    gt_put16<TO>(p, t, static_cast<TO*>(p.g.y), 0, n, c0, v, lane);
+}
+
+template <typename T, typename TO, bool GROUPED, int KIND, int SUB>
 __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_gemm_tc(const __grid_constant__ GemmTcP p) {
     extern __shared__ uint8_t smem_dyn[];
     uint8_t* smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + kGtBarOff);
-    uint64_t* empty = full + kGtStages;
-    uint64_t* acc_full = empty + kGtStages;
+    uint64_t* empty = full + kGtMaxStages;
+    uint64_t* acc_full = empty + kGtMaxStages;
     uint64_t* acc_empty = acc_full + 2;
     uint64_t* rows_full = acc_empty + 2;       // grouped: this CTA's rows of a stage have landed
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(smem + kGtMiscOff);
@@ -145,10 +183,13 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-    const int ks = (p.g.K + 63) / 64;
+    constexpr int kBlockK = KIND == kGt16 ? 64 : 128;   // 128 bytes
+    constexpr int sub = SUB;
+    const int stages = p.stages, block_bytes = p.block_bytes, stage_bytes = sub * block_bytes;
+    const int ks = (p.g.K + kBlockK * sub - 1) / (kBlockK * sub);
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < kGtStages; ++i) {
+        for (int i = 0; i < stages; ++i) {
             mbar_init(&full[i], GROUPED ? 3 : 1);
             mbar_init(&empty[i], 1);
             mbar_init(&rows_full[i], kGtRowWarps * 32);
@@ -192,18 +233,21 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
         bool ok = true;
         for (int i = pair; ok && gt_tile<GROUPED>(p, s_cum, i, hint, t); i += pairs) {
             const int tb = t.t0 + (int)rank * (t.ntok >> 1);
-            const uint32_t bytes = 2u * (kGtAStage + (GROUPED ? 0 : p.box_rows * 128));
+            const uint32_t bytes = 2u * sub * (kGtAStage + (GROUPED ? 0 : p.box_rows * 128));
             for (int k = 0; k < ks; ++k) {
                 if (!(ok = tc2_wait(&empty[st], ph ^ 1u, s_abort, &g_gemm_tc_err, 0x2100 + st))) break;
                 if (tc_elect_one()) {
                     const uint32_t bar = cluster_map(smem_u32(&full[st]), 0);
-                    uint8_t* sa = smem + st * (kGtAStage + kGtBStage);
                     if (rank == 0) mbar_expect_tx(&full[st], bytes);
-                    tma2_load_3d(sa, &p.wmap, k * 64, t.n0 + (int)rank * 128, t.b, bar);
-                    if (!GROUPED) tma2_load_3d(sa + kGtAStage, &p.xmap, k * 64, tb, t.b, bar);
+#pragma unroll
+                    for (int u = 0; u < sub; ++u) {   // a block behind K arrives as zeros
+                        uint8_t* sa = smem + st * stage_bytes + u * block_bytes;
+                        tma2_load_3d(sa, &p.wmap, (k * sub + u) * kBlockK, t.n0 + (int)rank * 128, t.b, bar);
+                        if (!GROUPED) tma2_load_3d(sa + kGtAStage, &p.xmap, (k * sub + u) * kBlockK, tb, t.b, bar);
+                    }
                 }
                 __syncwarp();
-                if (++st == kGtStages) {
+                if (++st == stages) {
                     st = 0;
                     ph ^= 1u;
                 }
@@ -218,20 +262,28 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
             if (!(ok = tc2_wait(&acc_empty[acc], acc_ph ^ 1u, s_abort, &g_gemm_tc_err, 0x2300 + acc))) break;
             tc_fence_after();
             const uint32_t d = tmem + (uint32_t)(acc * 256);
-            const uint32_t idesc = tc2_idesc(std::is_same<T, __nv_bfloat16>::value, t.ntok);
+            const uint32_t idesc = KIND == kGt16 ? tc2_idesc(std::is_same<T, __nv_bfloat16>::value, t.ntok) : tc2_idesc8(KIND == kGtFp8, t.ntok);
             for (int k = 0; k < ks; ++k) {
                 if (!(ok = tc2_wait(&full[st], ph, s_abort, &g_gemm_tc_err, 0x2400 + st))) break;
                 tc_fence_after();
                 if (tc_elect_one()) {
-                    const uint64_t ad = tc_desc_sw128(smem_u32(smem + st * (kGtAStage + kGtBStage)));
-                    const uint64_t bd = tc_desc_sw128(smem_u32(smem + st * (kGtAStage + kGtBStage) + kGtAStage));
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) tc2_mma_ss(d, ad + (uint64_t)(j * 2), bd + (uint64_t)(j * 2), idesc, (k > 0 || j > 0) ? 1u : 0u);
+                    for (int u = 0; u < sub; ++u) {
+                        const uint32_t at = smem_u32(smem + st * stage_bytes + u * block_bytes);
+                        const uint64_t ad = tc_desc_sw128(at), bd = tc_desc_sw128(at + kGtAStage);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {   // 32 bytes of k per MMA
+                            const uint64_t a = ad + (uint64_t)(j * 2), b = bd + (uint64_t)(j * 2);
+                            const uint32_t accum = (k > 0 || u > 0 || j > 0) ? 1u : 0u;
+                            if constexpr (KIND == kGt16) tc2_mma_ss(d, a, b, idesc, accum);
+                            else tc2_mma_ss8<KIND == kGtFp8>(d, a, b, idesc, accum);
+                        }
+                    }
                     tc2_commit(&empty[st]);
                     if (k == ks - 1) tc2_commit(&acc_full[acc]);
                 }
                 __syncwarp();
-                if (++st == kGtStages) {
+                if (++st == stages) {
                     st = 0;
                     ph ^= 1u;
                 }
@@ -254,7 +306,7 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     mbar_arrive_at(cluster_map(smem_u32(&full[st]), 0));
                 }
-                if (++st == kGtStages) {
+                if (++st == stages) {
                     st = 0;
                     ph ^= 1u;
                 }
@@ -277,16 +329,21 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
             }
             for (int k = 0; k < ks; ++k) {
                 if (!(ok = tc2_wait(&empty[st], ph ^ 1u, s_abort, &g_gemm_tc_err, 0x2200 + st))) break;
-                const bool in = k * 64 + c * 8 < p.g.K;
-                const int bytes = in ? 16 : 0;   // 0: zeros, nothing is read
 #pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    if (u * 16 < half)
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sm + (uint32_t)(st * (kGtAStage + kGtBStage) + u * 2048)),
-                                     "l"(in ? row[u] + k * 64 : row[u] - c * 8), "r"(bytes)
-                                     : "memory");
+                for (int u2 = 0; u2 < sub; ++u2) {
+                    const int k0 = (k * sub + u2) * 64;
+                    const bool in = k0 + c * 8 < p.g.K;
+                    const int bytes = in ? 16 : 0;   // 0: zeros, nothing is read
+                    const uint32_t dst = sm + (uint32_t)(st * stage_bytes + u2 * block_bytes);
+#pragma unroll
+                    for (int u = 0; u < 8; ++u)
+                        if (u * 16 < half)
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (uint32_t)(u * 2048)),
+                                         "l"(in ? row[u] + k0 : row[u] - c * 8), "r"(bytes)
+                                         : "memory");
+                }
                 asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&rows_full[st])) : "memory");
-                if (++st == kGtStages) {
+                if (++st == stages) {
                     st = 0;
                     ph ^= 1u;
                 }
@@ -302,8 +359,11 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
             if (!tc2_wait(&acc_full[acc], acc_ph, s_abort, &g_gemm_tc_err, 0x2800 + acc)) break;
             tc_fence_after();
             const int n = t.n0 + (int)rank * 128 + q * 32 + lane;
-            float bias = 0.f;
+            float bias = 0.f, s_w = 0.f;
             if (n < p.g.N) {
+                if (KIND != kGt16)
+                    s_w = p.sw_mode == 0 ? to_f32<T>(static_cast<const T*>(p.sw)[n])
+                                         : static_cast<const float*>(p.sw)[p.sw_mode == 3 ? 0 : n];
                 if (p.g.bias) bias = p.g.bias[(size_t)t.b * p.g.bb + n];
                 else if (p.g.bias_t) bias = to_f32<T>(static_cast<const T*>(p.g.bias_t)[n]);
             }
@@ -311,7 +371,9 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
             for (int c0 = set * 16; c0 < t.ntok && t.t0 + c0 < t.M; c0 += 32) {
                 float v[16];
                 tc_ld16(taddr + (uint32_t)c0, v);
-                switch (p.epi) {
+                if constexpr (KIND != kGt16) {
+                    gt_store16_8bit<TO, KIND>(p, t, n, c0, v, s_w, bias, p.g.bias_t != nullptr, lane);
+                } else switch (p.epi) {
 #define ZL_GT_EPI(E) case E: gt_store16<T, TO, E>(p, t, n, c0, v, bias, lane); break;
                     ZL_GT_EPI(ZL_GEMM_EPI_RELU2)
                     ZL_GT_EPI(ZL_GEMM_EPI_SIGMOID_GATE)
@@ -375,46 +437,90 @@ bool gemm_tc_route(const GemmP& p, int batch, int in_dtype) {
     return p.M > 32 && (long long)cdiv(p.N, kTc2Rows) * cdiv(p.M, 32) * batch < (1ll << 30);
 }
 
-template <typename T, typename TO>
-static cudaError_t launch_gt(const GemmTcP& q, bool grouped, int pairs, bool pdl, cudaStream_t stream) {
+template <typename T, typename TO, bool GROUPED, int KIND, int SUB>
+static cudaError_t launch_gt_sub(const GemmTcP& q, int pairs, bool pdl, cudaStream_t stream) {
     static bool set[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<T, TO, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGtBytes);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gemm_tc<T, TO, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGtBytes);
+        const cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<T, TO, GROUPED, KIND, SUB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGtBytes);
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) set[dev] = true;
     }
-    return grouped ? launch_pairs(k_gemm_tc<T, TO, true>, pairs, dim3(kGtGroupThreads), (size_t)kGtBytes, stream, pdl, q)
-                   : launch_pairs(k_gemm_tc<T, TO, false>, pairs, dim3(kGtThreads), (size_t)kGtBytes, stream, pdl, q);
+    return launch_pairs(k_gemm_tc<T, TO, GROUPED, KIND, SUB>, pairs, dim3(GROUPED ? kGtGroupThreads : kGtThreads), (size_t)kGtBytes, stream, pdl, q);
+}
+template <typename T, typename TO, bool GROUPED, int KIND>
+static cudaError_t launch_gt(const GemmTcP& q, int pairs, bool pdl, cudaStream_t stream) {
+    if constexpr (!GROUPED)
+        if (q.sub == 2) return launch_gt_sub<T, TO, GROUPED, KIND, 2>(q, pairs, pdl, stream);
+    return launch_gt_sub<T, TO, GROUPED, KIND, 1>(q, pairs, pdl, stream);
+}
+template <typename T, typename TO>
+static cudaError_t launch_gt16(const GemmTcP& q, bool grouped, int pairs, bool pdl, cudaStream_t stream) {
+    return grouped ? launch_gt<T, TO, true, kGt16>(q, pairs, pdl, stream) : launch_gt<T, TO, false, kGt16>(q, pairs, pdl, stream);
+}
+
+// tiles, maps and stages of a call; returns the number of pairs, 0 on failure
+static int gt_plan(GemmTcP& q, CUtensorMapDataType dt, int batch, int out_bytes) {
+    const GemmP& p = q.g;
+    const bool grouped = p.grp_off != nullptr;
+    int pairs = device_sm_count() / 2;
+    q.groups = batch;
+    q.row_tiles = cdiv(p.N, kTc2Rows);
+    q.tok_tiles = 0;
+    q.ntok = 256;
+    q.wide = p.N % 2 == 0 && p.ldy % 2 == 0 && p.yb % 2 == 0 && reinterpret_cast<uintptr_t>(p.y) % (2 * out_bytes) == 0;
+    if (!tc2_map_3d(&q.wmap, p.w, dt, p.K, p.N, batch, p.ldw, p.wb, 128)) return 0;
+    if (!grouped) {
+        q.ntok = gt_pick_ntok(p.M, (long long)q.row_tiles * batch, pairs);
+        q.tok_tiles = cdiv(p.M, q.ntok);
+        const long long tiles = (long long)q.row_tiles * q.tok_tiles * batch;
+        if (tiles < pairs) pairs = (int)tiles;
+        if (!tc2_map_3d(&q.xmap, p.x, dt, p.K, p.M, batch, p.ldx, p.xb, q.ntok / 2)) return 0;
+    }
+    q.box_rows = q.ntok / 2;
+    q.block_bytes = kGtAStage + q.box_rows * 128;
+    // handing a stage over costs the MMA warp about 450 cycles, a block's MMAs 2 per row of x: small tiles take two blocks per stage
+    // (not grouped rows, whose copies come to too few stages then: 87 -> 95 us)
+    q.sub = q.ntok <= 128 && !grouped ? 2 : 1;
+    const int fit = kGtRing / (q.sub * q.block_bytes);
+    q.stages = fit < kGtMaxStages ? fit : kGtMaxStages;
+    return pairs;
 }
 
 cudaError_t launch_gemm_tc(const GemmP& p, int batch, int in_dtype, int out_dtype, int epilogue, bool pdl, cudaStream_t stream) {
     const bool bf16 = in_dtype == ZL_BF16, grouped = p.grp_off != nullptr;
-    const int max_pairs = device_sm_count() / 2;
-    GemmTcP q;
+    GemmTcP q{};
     q.g = p;
     q.epi = epilogue;
-    q.groups = batch;
-    q.row_tiles = cdiv(p.N, kTc2Rows);
-    q.tok_tiles = q.ntok = q.box_rows = 0;
-    const int elem = out_dtype == ZL_F32 ? 4 : 2;
-    q.wide = p.N % 2 == 0 && p.ldy % 2 == 0 && p.yb % 2 == 0 && reinterpret_cast<uintptr_t>(p.y) % (2 * elem) == 0;
-    int pairs = max_pairs;
-    if (!tc2_map_3d(&q.wmap, p.w, bf16, p.K, p.N, batch, p.ldw, p.wb, 128)) return cudaErrorInvalidValue;
-    if (!grouped) {
-        q.ntok = gt_pick_ntok(p.M, (long long)q.row_tiles * batch, max_pairs);
-        q.box_rows = q.ntok / 2;
-        q.tok_tiles = cdiv(p.M, q.ntok);
-        const long long tiles = (long long)q.row_tiles * q.tok_tiles * batch;
-        if (tiles < pairs) pairs = (int)tiles;
-        if (!tc2_map_3d(&q.xmap, p.x, bf16, p.K, p.M, batch, p.ldx, p.xb, q.box_rows)) return cudaErrorInvalidValue;
-    }
-    if (bf16) return out_dtype == ZL_F32 ? launch_gt<__nv_bfloat16, float>(q, grouped, pairs, pdl, stream)
-                                         : launch_gt<__nv_bfloat16, __nv_bfloat16>(q, grouped, pairs, pdl, stream);
-    return out_dtype == ZL_F32 ? launch_gt<__half, float>(q, grouped, pairs, pdl, stream) : launch_gt<__half, __half>(q, grouped, pairs, pdl, stream);
+    const int pairs = gt_plan(q, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, batch, out_dtype == ZL_F32 ? 4 : 2);
+    if (pairs <= 0) return cudaErrorInvalidValue;
+    if (bf16) return out_dtype == ZL_F32 ? launch_gt16<__nv_bfloat16, float>(q, grouped, pairs, pdl, stream)
+                                         : launch_gt16<__nv_bfloat16, __nv_bfloat16>(q, grouped, pairs, pdl, stream);
+    return out_dtype == ZL_F32 ? launch_gt16<__half, float>(q, grouped, pairs, pdl, stream) : launch_gt16<__half, __half>(q, grouped, pairs, pdl, stream);
 }
+
+template <typename T, bool FP8>
+cudaError_t launch_w8_gemm_tc(const uint8_t* xq, const float* sx, const uint8_t* w, const void* sw, int sw_mode, const T* bias, T* y, int M, int N, int K,
+                              bool pdl, cudaStream_t stream) {
+    GemmTcP q{};
+    q.g = GemmP{xq, w, y, nullptr, K, 0, K, 0, N, 0, 0, 0, M, N, K};
+    q.g.bias_t = bias;
+    q.sx = sx;
+    q.sw = sw;
+    q.sw_mode = sw_mode;
+    const int pairs = gt_plan(q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, 2);
+    if (pairs <= 0) return cudaErrorInvalidValue;
+    return launch_gt<T, T, false, FP8 ? kGtFp8 : kGtInt8>(q, pairs, pdl, stream);
+}
+#define ZL_W8_TC(T, F8)                                                                                                                    \
+    template cudaError_t launch_w8_gemm_tc<T, F8>(const uint8_t*, const float*, const uint8_t*, const void*, int, const T*, T*, int, int, int, bool, \
+                                                  cudaStream_t);
+ZL_W8_TC(__half, false)
+ZL_W8_TC(__half, true)
+ZL_W8_TC(__nv_bfloat16, false)
+ZL_W8_TC(__nv_bfloat16, true)
+#undef ZL_W8_TC
 
 }  // namespace zl
 

@@ -89,6 +89,25 @@ __device__ __forceinline__ void tc2_mma_ss(uint32_t d_tmem, uint64_t adesc, uint
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum)
         : "memory");
 }
+// 8-bit operands, 256 x n x 32: kind::i8 (s8 x s8 -> s32) or kind::f8f6f4 (e4m3 x e4m3 -> f32)
+__host__ __device__ constexpr uint32_t tc2_idesc8(bool fp8, int n) {
+    return (fp8 ? (1u << 4) : ((2u << 4) | (1u << 7) | (1u << 10))) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTc2Rows >> 4) << 24);
+}
+template <bool FP8>
+__device__ __forceinline__ void tc2_mma_ss8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
+    if constexpr (FP8)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+            "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+            "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum)
+            : "memory");
+}
 __device__ __forceinline__ void tc2_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -117,13 +136,13 @@ inline cudaError_t launch_pairs(void (*kernel)(KArgs...), int pairs, dim3 block,
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-// (K, rows, batch) tensor of 16-bit values, row pitch ld and batch pitch in elements; box = 64 k x box_rows rows, 128-byte swizzle
-inline bool tc2_map_3d(CUtensorMap* map, const void* base, bool bf16, uint64_t k, uint64_t rows, uint64_t batch, uint64_t ld, uint64_t batch_ld,
-                       uint32_t box_rows) {
-    const uint64_t dims[3] = {k, rows, batch}, strides[2] = {ld * 2, (batch > 1 ? batch_ld : ld * rows) * 2};
-    const uint32_t box[3] = {64, box_rows, 1};
-    return tc_make_map_nd(map, base, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, dims, strides, box,
-                          CU_TENSOR_MAP_SWIZZLE_128B);
+// (K, rows, batch) tensor, row pitch ld and batch pitch in elements; box = 128 bytes of k x box_rows rows, 128-byte swizzle
+inline bool tc2_map_3d(CUtensorMap* map, const void* base, CUtensorMapDataType dt, uint64_t k, uint64_t rows, uint64_t batch, uint64_t ld,
+                       uint64_t batch_ld, uint32_t box_rows) {
+    const uint64_t elem = dt == CU_TENSOR_MAP_DATA_TYPE_UINT8 ? 1 : 2;
+    const uint64_t dims[3] = {k, rows, batch}, strides[2] = {ld * elem, (batch > 1 ? batch_ld : ld * rows) * elem};
+    const uint32_t box[3] = {(uint32_t)(128 / elem), box_rows, 1};
+    return tc_make_map_nd(map, base, dt, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 }  // namespace zl

@@ -1,4 +1,4 @@
-// tcgen05 / TMEM / TMA building blocks shared by the tensor-core kernels (w4a16_tc.cu, w8_tc.cu): bounded mbarrier waits,
+// tcgen05 / TMEM / TMA building blocks shared by the tensor-core kernels (w4a16_tc.cu, tc2_common.cuh): bounded mbarrier waits,
 // tensor-TMA loads, shared-memory matrix descriptors, TMEM loads, and the host-side tensor-map encoder.
 #pragma once
 #include "common.cuh"

@@ -56,6 +56,5 @@ cudaError_t prepare_w4_tc();
 cudaError_t launch_w4_tc2(const W4Params& p, bool pdl, cudaStream_t stream);
 bool w4_tc2_route(int M, int N, int K);
 cudaError_t prepare_w4_tc2();
-cudaError_t prepare_w8_tc();   // w8_tc.cu
 
 }  // namespace zl

@@ -337,7 +337,7 @@ cudaError_t launch_w4_tc2(const W4Params& p, bool pdl, cudaStream_t stream) {
     if (!w4_tc_params(q, p)) return cudaErrorInvalidValue;
     q.ntok = t2_pick_ntok(p.mc, row_tiles, G, max_pairs);
     q.tok_tiles = cdiv(p.mc, q.ntok);
-    if (!tc2_map_3d(&q.xmap, p.x, false, p.K, p.mc, 1, p.ldx, 0, q.ntok / 2)) return cudaErrorInvalidValue;
+    if (!tc2_map_3d(&q.xmap, p.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, p.K, p.mc, 1, p.ldx, 0, q.ntok / 2)) return cudaErrorInvalidValue;
     const int tiles = row_tiles * q.tok_tiles;
     return launch_pairs(k_w4a16_tc2, tiles < max_pairs ? tiles : max_pairs, dim3(T2Cfg::kThreads), (size_t)T2Cfg::kBytes, stream, pdl, q);
 }

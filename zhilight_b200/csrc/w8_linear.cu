@@ -18,11 +18,10 @@
 #include <cstdlib>
 
 namespace zl {
-// tcgen05 W8A8 kernel (w8_tc.cu)
-bool w8_tc_supports(int N, int K);
+// the same products on pairs of SMs (gemm_tc.cu)
 template <typename T, bool FP8>
-cudaError_t launch_w8_tc(const uint8_t* xq, const float* sx, const uint8_t* w, const void* sw, int sw_mode, const T* bias, T* y,
-                         int mc, int N, int K, bool pdl, cudaStream_t stream);
+cudaError_t launch_w8_gemm_tc(const uint8_t* xq, const float* sx, const uint8_t* w, const void* sw, int sw_mode, const T* bias, T* y, int M, int N, int K,
+                              bool pdl, cudaStream_t stream);
 }  // namespace zl
 
 #include <cuda_fp8.h>
@@ -473,6 +472,19 @@ extern "C" int zl_int8_scale_back(const int32_t* acc, const float* x_scale, cons
     return ZL_OK;
 }
 
+// Whether M rows go to the kernel on pairs of SMs (gemm_tc.cu), which costs the same from 1 row to 128; the mma.sync kernel reads the
+// weights once per 32 rows and its activations once per 16 weight rows.  us, here against mma.sync (int8 / fp8):
+//   M = 64      4096 x 4096 19 against 24; 4096 x 14336 26 / 31
+//   M = 32      8192 x 8192 23 against 34 / 46; 14336 x 4096 19 / 33 / 44; 4096 x 14336 27 / 29 / 37; 4096 x 4096 19 / 15 / 17
+//   M = 16      8192 x 8192 23 / 25 / 35; 14336 x 4096 19 / 25 / 33; 4096 x 14336 27 / 21 / 29
+//   M = 8       8192 x 8192 23 / 20 / 21; 28672 x 8192 48 / 60 / 62
+static bool w8_tc_route(int M, int N, int K) {
+    if (M > 32) return true;
+    const long long weights = (long long)N * K;
+    if (weights < (48ll << 20)) return false;
+    return weights >= (128ll << 20) || M > (N >= 8192 ? 8 : 24);
+}
+
 extern "C" int zl_w8a8_gemm(const void* xq, const float* x_scale, const void* w, const void* w_scale,
                             int w_scale_dtype, const void* bias, void* y, int M, int N, int K, int kind, int dtype,
                             int pdl, zl_stream_t stream) {
@@ -486,42 +498,22 @@ extern "C" int zl_w8a8_gemm(const void* xq, const float* x_scale, const void* w,
     const uint8_t* xq8 = static_cast<const uint8_t*>(xq);
     const uint8_t* w8 = static_cast<const uint8_t*>(w);
     const int sw_f32 = kind == ZL_W8_FP8_ROWS ? 2 : (w_scale_dtype == ZL_F32 ? 1 : 0);
-    // measured on B200 (tools/w8_bench.py): with the reference's row-major (N, K) layout every 128-byte row segment of a TMA
-    // box comes from a different DRAM page, and the mma.sync kernel's 16-byte row-contiguous loads stream faster at decode
-    // sizes; the tcgen05 kernel takes over where the mma.sync kernel would re-stream the weights (M > 32: prefill chunks)
-    static const int tc_min_m = getenv("ZL_W8_TC_MIN_M") ? atoi(getenv("ZL_W8_TC_MIN_M")) : 33;
-    if (M >= tc_min_m && w8_tc_supports(N, K)) {
-        // tcgen05 path (w8_tc.cu): both operands through the TMA engine, s32 / f32 accumulators in TMEM
-        {
-            static bool prepared[64] = {};
-            int dev = 0;
-            cudaGetDevice(&dev);
-            if (dev < 0 || dev >= 64 || !prepared[dev]) {
-                int rc = zl_prepare();
-                if (rc != ZL_OK) return rc;
-                if (dev >= 0 && dev < 64) prepared[dev] = true;
-            }
-        }
+    if (w8_tc_route(M, N, K)) {
         const bool fp8 = kind != ZL_W8_INT8;
         const int sw_mode = fp8 ? (kind == ZL_W8_FP8_ROWS ? 2 : 3) : sw_f32;
-        for (int m0 = 0; m0 < M; m0 += 256) {
-            const int mc = (M - m0) < 256 ? (M - m0) : 256;
-            const bool p = pdl != 0 && m0 == 0;
-            const float* sx = kind == ZL_W8_INT8 ? x_scale + m0 : x_scale;
-            cudaError_t e;
-            if (dtype == ZL_F16) {
-                const __half* b = static_cast<const __half*>(bias);
-                __half* yo = static_cast<__half*>(y) + (size_t)m0 * N;
-                e = fp8 ? launch_w8_tc<__half, true>(xq8 + (size_t)m0 * K, sx, w8, w_scale, sw_mode, b, yo, mc, N, K, p, stream)
-                        : launch_w8_tc<__half, false>(xq8 + (size_t)m0 * K, sx, w8, w_scale, sw_mode, b, yo, mc, N, K, p, stream);
-            } else {
-                const __nv_bfloat16* b = static_cast<const __nv_bfloat16*>(bias);
-                __nv_bfloat16* yo = static_cast<__nv_bfloat16*>(y) + (size_t)m0 * N;
-                e = fp8 ? launch_w8_tc<__nv_bfloat16, true>(xq8 + (size_t)m0 * K, sx, w8, w_scale, sw_mode, b, yo, mc, N, K, p, stream)
-                        : launch_w8_tc<__nv_bfloat16, false>(xq8 + (size_t)m0 * K, sx, w8, w_scale, sw_mode, b, yo, mc, N, K, p, stream);
-            }
-            ZL_CHECK_CUDA(e);
+        cudaError_t e;
+#define ZL_W8_TC(TT, F8)                                                                                                              \
+    e = launch_w8_gemm_tc<TT, F8>(xq8, x_scale, w8, w_scale, sw_mode, static_cast<const TT*>(bias), static_cast<TT*>(y), M, N, K, pdl != 0, \
+                                  stream)
+        if (dtype == ZL_F16) {
+            if (fp8) ZL_W8_TC(__half, true);
+            else ZL_W8_TC(__half, false);
+        } else {
+            if (fp8) ZL_W8_TC(__nv_bfloat16, true);
+            else ZL_W8_TC(__nv_bfloat16, false);
         }
+#undef ZL_W8_TC
+        ZL_CHECK_CUDA(e);
         return ZL_OK;
     }
     for (int m0 = 0; m0 < M; m0 += 32) {
