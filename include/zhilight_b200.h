@@ -288,6 +288,8 @@ int zl_kv_int8_quant_append(const void* k_src, const void* v_src, const int32_t*
  * Decode-step helpers around the layers
  * ------------------------------------------------------------------------------------------ */
 /* nn::Embedding lookup (src/nn/embedding/embedding.cu:20-60): out[t,:] = table[ids[t],:]. */
+/* n host words (buffer addresses) -> a device table, in stream order; the host array may go when the call returns */
+int zl_write_pointers(void* dst, const void* pointers, int n, zl_stream_t stream);
 int zl_embedding(const int32_t* ids, const void* table, void* out, int T, int D, int vocab, int dtype, int pdl,
                  zl_stream_t stream);
 /* greedy pick (generator/batch_generator.cpp:1762-1884 with beam 1): argmax over fp32 logits (T, V). */

@@ -170,4 +170,6 @@ def check(rc):
 
 def call(name, *args):
     """Call an int-returning entry point and raise ZLError on failure."""
-    check(getattr(load(), name)(*args))
+    rc = getattr(_lib or load(), name)(*args)
+    if rc != 0:
+        check(rc)

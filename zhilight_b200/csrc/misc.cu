@@ -42,6 +42,14 @@ __global__ void k_embedding(const int32_t* __restrict__ ids, const T* __restrict
     for (int i = threadIdx.x; i < D / 8; i += blockDim.x) dst[i] = src[i];
 }
 
+// 256 words that travel as kernel parameters: a table of pointers written in stream order, without a copy from host memory to wait for
+struct Words256 {
+    unsigned long long w[256];
+};
+__global__ void k_write_words(const __grid_constant__ Words256 words, unsigned long long* dst, int n) {
+    if (threadIdx.x < n) dst[threadIdx.x] = words.w[threadIdx.x];
+}
+
 // stage 1: per (token, chunk) partial argmax; stage 2: merge.  Ties -> lowest index.
 __global__ void k_argmax_partial(const float* __restrict__ logits, int V, int chunks, float* __restrict__ pval,
                                  int* __restrict__ pidx) {
@@ -182,6 +190,18 @@ __global__ void k_fill_uniform(T* __restrict__ p, size_t n, float lo, float hi, 
 }  // namespace zl
 
 using namespace zl;
+
+extern "C" int zl_write_pointers(void* dst, const void* pointers, int n, zl_stream_t stream) {
+    ZL_CHECK_ARG(dst && pointers && n > 0 && (reinterpret_cast<uintptr_t>(dst) & 7) == 0);
+    for (int i = 0; i < n; i += 256) {
+        const int c = n - i < 256 ? n - i : 256;
+        Words256 w;
+        memcpy(w.w, static_cast<const unsigned long long*>(pointers) + i, (size_t)c * 8);
+        memset(w.w + c, 0, (size_t)(256 - c) * 8);
+        ZL_CHECK_CUDA(launch(k_write_words, dim3(1), dim3(256), 0, stream, false, w, static_cast<unsigned long long*>(dst) + i, c));
+    }
+    return ZL_OK;
+}
 
 extern "C" int zl_embedding(const int32_t* ids, const void* table, void* out, int T, int D, int vocab, int dtype,
                             int pdl, zl_stream_t stream) {

@@ -3,6 +3,7 @@
 Every function takes CUDA tensors, passes raw pointers to libzhilight_b200.so on the current stream and
 returns torch tensors.  Names / argument meaning mirror the reference operator each one replaces.
 """
+import array
 import ctypes
 
 import torch
@@ -30,11 +31,12 @@ def _p(t):
         raise _lib.ZLError(-1, "zhilight_b200 ops need CUDA tensors (no CPU fallback)")
     if not t.is_contiguous():
         raise _lib.ZLError(-1, "tensor must be contiguous")
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """Handle of the current stream of the current device, without the Stream object around it."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 # ------------------------------------------------------------------ load-time transforms
@@ -169,20 +171,19 @@ def w4a16_gemm_fused(x, packed, n, k, group_size=128, bias=None, residual=None, 
     if x.dtype != torch.float16:
         raise _lib.ZLError(-2, "A must be half")
     m = x.shape[0]
-    a = _lib.W4FusedArgs()
-    a.x, a.ldx, a.packed, a.bias, a.residual = x.data_ptr(), x.stride(0), packed.data_ptr(), _dp(bias), _dp(residual)
-    a.M, a.N, a.K, a.group_size, a.epilogue, a.pdl = m, n, k, group_size, epilogue, int(pdl)
-    a.ln_weight, a.eps = _dp(ln_weight), eps
-    a.variant = int(variant)
-    keep = []
+    # in the structure's order: one call, not an assignment for each of its members
+    a = _lib.W4FusedArgs(x.data_ptr(), x.stride(0), packed.data_ptr(), _dp(bias), _dp(residual), None, m, n, k, group_size, epilogue,
+                         int(pdl), _dp(ln_weight), eps)
+    if variant:
+        a.variant = int(variant)
+    table = None
     if epilogue == EPI_QKV_ROPE:
         r = rope
         q = torch.empty((m, r["num_heads"] * r["dim_head"]), dtype=torch.float16, device=x.device)
-        ka, va = _ptr_table(r["k_bufs"], x.device), _ptr_table(r["v_bufs"], x.device)
-        keep += [ka, va]
+        (ka, va), table = _ptr_tables(x.device, r["k_bufs"], r["v_bufs"])
         a.cos, a.sin, a.q_out = r["cos"].data_ptr(), r["sin"].data_ptr(), q.data_ptr()
         a.token_batch, a.placement = r["token_batch"].data_ptr(), r["placement"].data_ptr()
-        a.k_addrs, a.v_addrs = ka.data_ptr(), va.data_ptr()
+        a.k_addrs, a.v_addrs = ka, va
         a.num_heads, a.num_kv_heads, a.dim_head = r["num_heads"], r["num_kv_heads"], r["dim_head"]
         ret = q
     else:
@@ -192,8 +193,8 @@ def w4a16_gemm_fused(x, packed, n, k, group_size=128, bias=None, residual=None, 
         a.y = out.data_ptr()
         ret = out
     _lib.call("zl_w4a16_gemm_fused", ctypes.byref(a), _stream())
-    if keep:
-        torch.cuda.current_stream().synchronize()
+    if table is not None:
+        _in_use(x, packed, bias, residual, ln_weight, r["cos"], r["sin"], r["token_batch"], r["placement"], *r["k_bufs"], *r["v_bufs"])
     return ret
 
 
@@ -318,25 +319,53 @@ def rope_qk_cache(cos, sin, qkv, num_heads, num_kv_heads, dim_head, neox=True):
 
 
 def _ptr_table(tensors, device):
-    return torch.tensor([t.data_ptr() for t in tensors], dtype=torch.int64, device=device)
+    """int64 tensor of the tensors' addresses, written in stream order (no copy from host memory to wait for)."""
+    out = torch.empty(len(tensors), dtype=torch.int64, device=device)
+    if len(tensors) > 0:
+        words = array.array("Q", [t.data_ptr() for t in tensors])
+        _lib.call("zl_write_pointers", _p(out), words.buffer_info()[0], len(tensors), _stream())
+    return out
+
+
+def _ptr_tables(device, *lists):
+    """One table after the other: the address of each, and the tensor that holds them."""
+    table = _ptr_table([t for x in lists for t in x], device)
+    at, out = table.data_ptr(), []
+    for x in lists:
+        out.append(at)
+        at += 8 * len(x)
+    return out, table
+
+
+def _in_use(*tensors):
+    """The call goes on after this function returns.  Memory that belongs to another stream is not given away before it ends;
+    what the allocator does not watch (mapped host memory) is waited for."""
+    s = torch.cuda.current_stream()
+    for t in tensors:
+        if t is None:
+            continue
+        if t.is_cuda:
+            t.record_stream(s)
+        else:
+            s.synchronize()
 
 
 def copy_to_rag_buffer2(placement, buf_lens, k_src, v_src, k_bufs, v_bufs, bshd=True):
     b, len_q, hkv, d = k_src.shape
-    ka, va = _ptr_table(k_bufs, k_src.device), _ptr_table(v_bufs, k_src.device)
-    _lib.call("zl_copy_to_rag_buffer2", _p(placement), _p(buf_lens), _p(k_src), _p(v_src), _p(ka), _p(va), b, len_q,
+    (ka, va), _table = _ptr_tables(k_src.device, k_bufs, v_bufs)
+    _lib.call("zl_copy_to_rag_buffer2", _p(placement), _p(buf_lens), _p(k_src), _p(v_src), ka, va, b, len_q,
               hkv, d, int(bshd), _dt(k_src), _stream())
-    torch.cuda.current_stream().synchronize()      # keep the pointer tables alive until the copy ran
+    _in_use(placement, buf_lens, k_src, v_src, *k_bufs, *v_bufs)
 
 
 def qkv_rope_append(cos, sin, qkv, token_batch, placement, k_bufs, v_bufs, num_heads, num_kv_heads, dim_head,
                     buf_lens=None, neox=True, bshd=True, pdl=False):
     t = qkv.shape[0]
     q = torch.empty((t, num_heads * dim_head), dtype=qkv.dtype, device=qkv.device)
-    ka, va = _ptr_table(k_bufs, qkv.device), _ptr_table(v_bufs, qkv.device)
-    _lib.call("zl_qkv_rope_append", _p(cos), _p(sin), _p(qkv), _p(q), _p(token_batch), _p(placement), _p(ka), _p(va),
+    (ka, va), _table = _ptr_tables(qkv.device, k_bufs, v_bufs)
+    _lib.call("zl_qkv_rope_append", _p(cos), _p(sin), _p(qkv), _p(q), _p(token_batch), _p(placement), ka, va,
               t, num_heads, num_kv_heads, dim_head, int(neox), int(bshd), _p(buf_lens), _dt(qkv), int(pdl), _stream())
-    torch.cuda.current_stream().synchronize()
+    _in_use(cos, sin, qkv, token_batch, placement, buf_lens, *k_bufs, *v_bufs)
     return q
 
 
@@ -346,10 +375,10 @@ def decode_attention(q, buf_lens, k_bufs, v_bufs, mask, scale, max_len_buf, num_
     out = torch.empty_like(q)
     ws_bytes = _lib.load().zl_decode_attention_workspace_bytes(b, len_q, hq, d, max_len_buf)
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-    ka, va = _ptr_table(k_bufs, q.device), _ptr_table(v_bufs, q.device)
-    _lib.call("zl_decode_attention", _p(q), _p(buf_lens), _p(ka), _p(va), _p(mask), float(scale), max_len_buf,
+    (ka, va), _table = _ptr_tables(q.device, k_bufs, v_bufs)
+    _lib.call("zl_decode_attention", _p(q), _p(buf_lens), ka, va, _p(mask), float(scale), max_len_buf,
               _p(out), b, len_q, hq, num_kv_heads, d, int(bshd), _p(ws), ws_bytes, _dt(q), int(pdl), _stream())
-    torch.cuda.current_stream().synchronize()
+    _in_use(q, buf_lens, mask, *k_bufs, *v_bufs)
     return out
 
 
@@ -361,21 +390,21 @@ def decode_attention_kv8(q, buf_lens, k_bufs, v_bufs, sk_bufs, sv_bufs, mask, sc
     out = torch.empty(q.shape, dtype=out_dtype or q.dtype, device=q.device)
     ws_bytes = _lib.load().zl_decode_attention_workspace_bytes(b, len_q, hq, d, max_len_buf)
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-    tabs = [_ptr_table(x, q.device) for x in (k_bufs, v_bufs, sk_bufs, sv_bufs)]
-    _lib.call("zl_decode_attention_kv8", _p(q), _p(buf_lens), _p(tabs[0]), _p(tabs[1]), _p(tabs[2]), _p(tabs[3]), _p(mask),
+    tabs, _table = _ptr_tables(q.device, k_bufs, v_bufs, sk_bufs, sv_bufs)
+    _lib.call("zl_decode_attention_kv8", _p(q), _p(buf_lens), *tabs, _p(mask),
               float(scale), max_len_buf, _p(out), b, len_q, hq, num_kv_heads, d, _p(ws), ws_bytes, _dt(out), int(pdl),
               _stream())
-    torch.cuda.current_stream().synchronize()
+    _in_use(q, buf_lens, mask, *k_bufs, *v_bufs, *sk_bufs, *sv_bufs)
     return out
 
 
 def kv_int8_quant_append(k_src, v_src, token_batch, placement, k_bufs, v_bufs, sk_bufs, sv_bufs):
     """k_src / v_src (T, H_kv, d) -> uint8 codes + fp32 scales scattered into the per-task caches."""
     t, hkv, d = k_src.shape
-    tabs = [_ptr_table(x, k_src.device) for x in (k_bufs, v_bufs, sk_bufs, sv_bufs)]
-    _lib.call("zl_kv_int8_quant_append", _p(k_src), _p(v_src), _p(token_batch), _p(placement), _p(tabs[0]), _p(tabs[1]),
-              _p(tabs[2]), _p(tabs[3]), t, hkv, d, _dt(k_src), 0, _stream())
-    torch.cuda.current_stream().synchronize()
+    tabs, _table = _ptr_tables(k_src.device, k_bufs, v_bufs, sk_bufs, sv_bufs)
+    _lib.call("zl_kv_int8_quant_append", _p(k_src), _p(v_src), _p(token_batch), _p(placement), *tabs, t, hkv, d, _dt(k_src), 0,
+              _stream())
+    _in_use(k_src, v_src, token_batch, placement, *k_bufs, *v_bufs, *sk_bufs, *sv_bufs)
 
 
 def embedding(ids, table):
