@@ -181,3 +181,50 @@ def test_qkv_rope_epilogue_int(lib, cuda, d, hq, hkv, k, t):
     torch.testing.assert_close(q, q2, rtol=2 ** -9, atol=3e-3)
     for a, b in zip(kb + vb, kb2 + vb2):
         torch.testing.assert_close(a, b, rtol=2 ** -9, atol=3e-3)
+
+
+@pytest.mark.parametrize("m,k,n", [(3, 9728 + 128, 512), (4, 7424, 512), (4, 8192, 128 * 40), (3, 14336, 4096), (4, 14336, 4096), (4, 14336 + 256, 256), (2, 16384, 256)])
+@pytest.mark.parametrize("epilogue", ["none", "residual", "swiglu"])
+def test_wide_k_of_few_rows(lib, cuda, m, k, n, epilogue):
+    """3-stage rings: what the 4-stage ones leave no room for.  Each output is exact but for the activations' 15-bit groups
+    (2^-15 of a group's maximum each) and its own rounding to fp16, 2^-11."""
+    from zhilight_b200 import ops
+    w, packed_i, _, _ = _setup(cuda, k, n, False, 8)
+    assert lib.zl_w4_int_layout_route(m, n, k) == 4          # (what callers choose a fused RMSNorm by: refused at these sizes)
+    with pytest.raises(Exception):
+        ops.w4a16_gemm_fused(torch.zeros(m, k, dtype=torch.float16, device=cuda), packed_i, n, k, variant=1,
+                             ln_weight=torch.ones(k, dtype=torch.float16, device=cuda))
+    g = torch.Generator().manual_seed(m + k)
+    x = (torch.randn(m, k, generator=g) * torch.logspace(-2, 1, k)[torch.randperm(k, generator=g)]).half()
+    ref = gptq.gemm_f32(x.numpy(), w)
+    args, limit = {}, 4e-4
+    if epilogue == "residual":
+        res = torch.randn(m, n, generator=g).half()
+        args = dict(epilogue=ops.EPI_RESIDUAL, residual=res.to(cuda))
+        ref = ref + res.float().numpy()
+    elif epilogue == "swiglu":      # rows in tiles of 8 gate, 8 up (the packed order is the test's own, the map only names it)
+        args, limit = dict(epilogue=ops.EPI_SWIGLU), 1.2e-3
+        t = ref.reshape(m, n // 16, 2, 8)
+        gate, up = (np.float16(t[:, :, i]).astype(np.float32) for i in (0, 1))
+        ref = (gate / (1 + np.exp(-gate)) * up).reshape(m, n // 2)
+    y = ops.w4a16_gemm_fused(x.to(cuda), packed_i, n, k, variant=1, **args).float().cpu().numpy()
+    ref = ref if epilogue != "swiglu" else np.clip(ref, -65504, 65504)
+    assert rel_l2(y, ref) <= limit
+
+
+def test_wide_k_nonfinite_activations(lib, cuda):
+    """a single Inf gives +-Inf by the weight's sign (NaN where the weight is zero), a NaN gives NaN; other rows keep their values"""
+    from zhilight_b200 import ops
+    k, n = 8192, 256
+    w, packed_i, _, _ = _setup(cuda, k, n, False, 9)
+    x = torch.randn(4, k, generator=torch.Generator().manual_seed(1)).half()
+    clean = ops.w4a16_gemm_fused(x.to(cuda), packed_i, n, k, variant=1)
+    x[1, 700] = float("inf")
+    x[2, 8191] = float("nan")
+    y = ops.w4a16_gemm_fused(x.to(cuda), packed_i, n, k, variant=1)
+    assert torch.equal(y[0], clean[0]) and torch.equal(y[3], clean[3]) and bool(torch.isnan(y[2]).all())
+    col = torch.from_numpy(np.ascontiguousarray(w)).float()
+    col = (col if col.shape[0] == n else col.T)[:, 700].numpy()
+    got = y[1].float().cpu().numpy()
+    assert np.array_equal(np.isnan(got), col == 0) and np.array_equal(np.sign(got[col != 0]), np.sign(col[col != 0]))
+    assert np.isinf(got[col != 0]).all()

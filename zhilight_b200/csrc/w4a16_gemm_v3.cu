@@ -42,13 +42,16 @@ __device__ __forceinline__ void imma_u8u8(int (&d)[4], const uint32_t (&a)[4], u
 // reduction), while the integer decomposition of the activations is staged ONCE per CTA by all warps together:
 //   wide : SUBS=2 x 8 warps, 5-stage rings  (N/32 > #SMs: qkv, gate/up)  -- two tile pipelines per SM
 //   tall : SUBS=1 x 16 warps, 4-stage rings (N/32 <= #SMs: o_proj, down) -- k split 16 ways
+//   deep : 3-stage rings, one reduction buffer of 4 token rows -- what leaves room for 4 staged rows of K up to 14.6 k.
 // RT = token rows kept in the split-k reduction buffers (even, >= mc): small batches shrink them to make room for
 // deeper rings -- the tile loop is latency-bound on ring depth (4 -> 5 stages is worth ~25 %).
+constexpr int kV3DeepRows = 4;
+
 template <int NT, int WARPS, int SUBS, int STAGES, int RT = NT * 8>
 struct V3Smem {
     static constexpr int kWarpsTotal = WARPS * SUBS;
     static constexpr int kRingBytes = kWarpsTotal * STAGES * kW4BlockBytes;
-    static constexpr int kRedBufs = (NT == 1) ? 2 : 1;
+    static constexpr int kRedBufs = (NT == 1 && RT != kV3DeepRows) ? 2 : 1;
     static constexpr int kRedFloats = WARPS * RT * 32;                     // per sub-CTA, per buffer
     static constexpr int kBarOff = kRingBytes;
     static constexpr int kRedOff = kBarOff + kWarpsTotal * STAGES * 8;
@@ -65,6 +68,31 @@ __host__ __device__ inline int v3_stage_bytes(int mc, int K) {
 
 __device__ __forceinline__ void sub_barrier(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
+
+// sum over the groups of a token that hold an Inf or NaN (the staging left them out of the integer sums) of w * x, the weight
+// rounded to fp16: +-Inf or NaN as in the fp16 kernels.  Plain loops over global memory, for such tokens only.
+__device__ __noinline__ float v3_nonfinite_sum(const uint8_t* packed, const __half* x, int K, int tile, int row) {
+    const int G = K / kW4GroupK;
+    const int tt = row >> 4, g = row & 7, up = (row >> 3) & 1;
+    float sum = 0.f;
+    for (int gi = 0; gi < G; ++gi) {
+        const __half* xg = x + gi * kW4GroupK;
+        bool finite = true;
+        for (int k = 0; k < kW4GroupK; ++k) finite &= (__half_as_ushort(xg[k]) & 0x7c00u) != 0x7c00u;
+        if (finite) continue;
+        const uint8_t* blk = packed + ((size_t)tile * G + gi) * kW4BlockBytes;
+        const __half2 s2 = reinterpret_cast<const __half2*>(blk + kW4ScaleOff)[tt * 8 + g];
+        const float s = up ? __high2float(s2) : __low2float(s2);
+        const int z = (blk[kW4ZeroOff + tt * 8 + g] >> (4 * up)) & 15;
+        for (int k = 0; k < kW4GroupK; ++k) {   // the word of (row, k): see ZLW4I in w4_layout.cuh
+            const int j = ((k >> 3) & 3) * 2 + ((k >> 2) & 1);
+            const uint32_t word = reinterpret_cast<const uint32_t*>(blk)[((tt * 2 + (j >> 2)) * 32 + g * 4 + (k >> 5)) * 4 + (j & 3)];
+            const int q = (word >> (8 * (k & 3) + 4 * up)) & 15;
+            sum = fmaf(__half2float(__float2half_rn((float)(q - z) * s)), __half2float(xg[k]), sum);
+        }
+    }
+    return sum;
 }
 
 // PACK block math for NB blocks of one warp at once (NB = 2: two independent dependency chains interleave).
@@ -232,11 +260,12 @@ __global__ void __launch_bounds__(WARPS * SUBS * 32, 1) k_w4a16_v3(const W4Param
         l2_prefetch_lines(p.pf_ptr, (size_t)p.pf_bytes, (int)blockIdx.x * WT + warp, (int)gridDim.x * WT, lane);
     // staging assignment: group gi -> warp gi % WT.  RMSNorm weights are constants: fetch them before the wait.
     constexpr int kMaxNg = 8;   // groups per warp kept in registers during staging (K <= 8*WT*128)
-    uint2 lnw[kMaxNg];
-    if (NORM) {
+    uint2 lnw[NORM ? kMaxNg : 1];
+    if constexpr (NORM) {
 #pragma unroll
         for (int gl = 0; gl < kMaxNg; ++gl) {
             const int gi = warp + gl * WT;
+            lnw[gl] = make_uint2(0u, 0u);
             if (gi < G)
                 lnw[gl] = (p.dbg & 16) ? make_uint2(0x3c003c00u, 0x3c003c00u)   // timing probe: 1.0h (results are wrong)
                                        : *reinterpret_cast<const uint2*>(p.ln_w + gi * kW4GroupK + lane * 4);
@@ -270,23 +299,34 @@ __global__ void __launch_bounds__(WARPS * SUBS * 32, 1) k_w4a16_v3(const W4Param
         tp_slots = tp->inbox[tp->rank] + comm_ll_offset(tp_ws, tp->slot_bytes) + (size_t)tp_parity * tp_ws * tp_slot_bytes;
 
     // ---- stage the activations as block-floating-point integers, once per CTA ----
+    // Every CTA stages all rows, so a row's K values cost each SM the instructions below (K = 14336: 112 groups); they, not the
+    // loads, are the time.  Two groups at a time without a branch between them, so that their reductions overlap; a group's
+    // registers are refilled for the next token as soon as they are read.  One group after the other, with the conversions and float
+    // maxima this replaces: 28672 x 4096 with the norm, 4 rows 20.3 us -> 18.5; 4096 x 4096, 3 rows 9.4 -> 8.3.
+    uint2 raw[kMaxNg];
+    const __half* x_own = p.x + warp * kW4GroupK + lane * 4;
+#pragma unroll
+    for (int gl = 0; gl < kMaxNg; ++gl) {
+        raw[gl] = make_uint2(0u, 0u);
+        if (warp + gl * WT < G) raw[gl] = ld_cg_u2(x_own + gl * (WT * kW4GroupK));
+    }
     for (int tok = 0; tok < p.mc; ++tok) {
-        uint2 raw[kMaxNg];
+        float sq = 0.f;
+        bool bad = false;
+        x_own += p.ldx;
 #pragma unroll
-        for (int gl = 0; gl < kMaxNg; ++gl) {
-            const int gi = warp + gl * WT;
-            if (gi < G) raw[gl] = ld_cg_u2(p.x + (size_t)tok * p.ldx + gi * kW4GroupK + lane * 4);
-        }
-        if (tp_mode == 1) {
-            // x := T(T(sum_r partial_r) + x): fp32 sum in rank order (identical on every rank and CTA), the reference's
-            // reduce_sum + element_add_scale rounding points (model_context.cpp:203-243, block_kernel.cu:7-17).  One group
-            // at a time: the accumulators of all groups at once cost the 512-thread CTA its register budget.
-            // element i of token tok lives in word (tok * K + i) / 2 of the source's slot; this lane needs 4 elements = 2 words
-            const uint8_t* src0 = tp_slots + ((size_t)tok * p.K + lane * 4) * 4;
+        for (int gl0 = 0; gl0 < kMaxNg; gl0 += 2) {
+            if (warp + gl0 * WT >= G) break;
+            if (tp_mode == 1) {
+                // x := T(T(sum_r partial_r) + x): fp32 sum in rank order (identical on every rank and CTA), the reference's
+                // reduce_sum + element_add_scale rounding points (model_context.cpp:203-243, block_kernel.cu:7-17).  One group
+                // at a time: the accumulators of all groups at once cost the 512-thread CTA its register budget.
+                // element i of token tok lives in word (tok * K + i) / 2 of the source's slot; this lane needs 4 elements = 2 words
+                const uint8_t* src0 = tp_slots + ((size_t)tok * p.K + lane * 4) * 4;
 #pragma unroll
-            for (int gl = 0; gl < kMaxNg; ++gl) {
-                const int gi = warp + gl * WT;
-                if (gi < G) {
+                for (int u = 0; u < 2; ++u) {
+                    const int gi = warp + (gl0 + u) * WT;
+                    if (gi >= G) continue;
                     float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
                     for (int r = 0; r < tp_ws; ++r) {
                         const uint8_t* src = src0 + (size_t)r * tp_slot_bytes + (size_t)gi * kW4GroupK * 4;
@@ -305,58 +345,71 @@ __global__ void __launch_bounds__(WARPS * SUBS * 32, 1) k_w4a16_v3(const W4Param
                         a2 += b.x;
                         a3 += b.y;
                     }
-                    const __half2 h01 = __hadd2(__floats2half2_rn(a0, a1), *reinterpret_cast<__half2*>(&raw[gl].x));
-                    const __half2 h23 = __hadd2(__floats2half2_rn(a2, a3), *reinterpret_cast<__half2*>(&raw[gl].y));
-                    raw[gl].x = *reinterpret_cast<const uint32_t*>(&h01);
-                    raw[gl].y = *reinterpret_cast<const uint32_t*>(&h23);
+                    const __half2 h01 = __hadd2(__floats2half2_rn(a0, a1), *reinterpret_cast<__half2*>(&raw[gl0 + u].x));
+                    const __half2 h23 = __hadd2(__floats2half2_rn(a2, a3), *reinterpret_cast<__half2*>(&raw[gl0 + u].y));
+                    raw[gl0 + u].x = *reinterpret_cast<const uint32_t*>(&h01);
+                    raw[gl0 + u].y = *reinterpret_cast<const uint32_t*>(&h23);
                     if (blockIdx.x == 0)
-                        *reinterpret_cast<uint2*>(p.tp_h_out + (size_t)tok * p.K + gi * kW4GroupK + lane * 4) = raw[gl];
+                        *reinterpret_cast<uint2*>(p.tp_h_out + (size_t)tok * p.K + gi * kW4GroupK + lane * 4) = raw[gl0 + u];
                 }
             }
-        }
-        float sq = 0.f;
-        bool bad = false;
+            uint32_t w01[2], w23[2], sum[2];
+            float sg[2];
 #pragma unroll
-        for (int gl = 0; gl < kMaxNg; ++gl) {
-            const int gi = warp + gl * WT;
-            if (gi < G) {
-                __half2 h01 = *reinterpret_cast<__half2*>(&raw[gl].x), h23 = *reinterpret_cast<__half2*>(&raw[gl].y);
-                if (NORM) {
+            for (int u = 0; u < 2; ++u) {
+                __half2 h01 = *reinterpret_cast<__half2*>(&raw[gl0 + u].x), h23 = *reinterpret_cast<__half2*>(&raw[gl0 + u].y);
+                if constexpr (NORM) {
                     const float2 f01 = __half22float2(h01), f23 = __half22float2(h23);
                     sq = fmaf(f01.x, f01.x, sq);
                     sq = fmaf(f01.y, f01.y, sq);
                     sq = fmaf(f23.x, f23.x, sq);
                     sq = fmaf(f23.y, f23.y, sq);
-                    h01 = __hmul2(h01, *reinterpret_cast<const __half2*>(&lnw[gl].x));
-                    h23 = __hmul2(h23, *reinterpret_cast<const __half2*>(&lnw[gl].y));
+                    h01 = __hmul2(h01, *reinterpret_cast<const __half2*>(&lnw[gl0 + u].x));
+                    h23 = __hmul2(h23, *reinterpret_cast<const __half2*>(&lnw[gl0 + u].y));
                 }
-                const float2 a = __half22float2(h01), b = __half22float2(h23);
-                // non-negative floats order like their bit patterns (and NaN patterns sort above Inf, which fmaxf would
-                // drop): integer maxima, then one REDUX instead of a shuffle tree
-                const uint32_t amax_l = max(max(__float_as_uint(fabsf(a.x)), __float_as_uint(fabsf(a.y))),
-                                            max(__float_as_uint(fabsf(b.x)), __float_as_uint(fabsf(b.y))));
-                const uint32_t amax_bits = __reduce_max_sync(0xffffffffu, amax_l);
+                w01[u] = *reinterpret_cast<const uint32_t*>(&h01);
+                w23[u] = *reinterpret_cast<const uint32_t*>(&h23);
+            }
+            if (tok + 1 < p.mc) {
+                raw[gl0] = ld_cg_u2(x_own + gl0 * (WT * kW4GroupK));
+                if (warp + (gl0 + 1) * WT < G) raw[gl0 + 1] = ld_cg_u2(x_own + (gl0 + 1) * (WT * kW4GroupK));
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                // magnitudes order like their bit patterns (NaN patterns above Inf's): integer maxima, then one REDUX
+                const uint32_t m2 = __vmaxu2(w01[u] & 0x7fff7fffu, w23[u] & 0x7fff7fffu);
+                const uint32_t amax = __reduce_max_sync(0xffffffffu, max(m2 & 0xffffu, m2 >> 16));
                 // 2^e with m = x * 2^-e in (-2^15, 2^15): e = floor(log2 amax) - 14
-                const uint32_t ex = (amax_bits >> 23) & 0xffu;
-                const bool zero = ex < 20u || ex == 0xffu;   // all-zero group -> 0; non-finite group -> poisons the token
-                bad |= ex == 0xffu;                          // (a NaN's bit pattern is above Inf's: REDUX max keeps it)
+                const uint32_t ex = __float_as_uint(__half2float(__ushort_as_half((unsigned short)amax))) >> 23;
+                const bool inf = amax >= 0x7c00u;            // non-finite group -> poisons the token
+                const bool zero = amax == 0u || inf;         // all-zero group -> 0
+                bad |= inf;
                 // PACK keeps one bit of headroom (|m| <= 2^14) so that the rounded-up high digit still fits int8
                 constexpr uint32_t kE = PACK ? 13u : 14u;
-                const float sg = zero ? 1.0f : __uint_as_float((ex - kE) << 23);
+                sg[u] = zero ? 1.0f : __uint_as_float((ex - kE) << 23);
                 const float inv = zero ? 0.0f : __uint_as_float((254u + kE - ex) << 23);
-                const int m0 = __float2int_rn(a.x * inv), m1 = __float2int_rn(a.y * inv);
-                const int m2 = __float2int_rn(b.x * inv), m3 = __float2int_rn(b.y * inv);
+                const uint32_t v01 = inf ? 0u : w01[u], v23 = inf ? 0u : w23[u];
+                const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&v01));
+                const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&v23));
+                // rounded to the nearest integer by an addition: 1.5 * 2^23 + m, whose low 16 bits are m's (x * inv is exact).
                 // byte 0 of each m -> lo, byte 1 -> hi (two's complement high byte == floor(m / 256)): 6 PRMTs.
                 // PACK: lo is read as SIGNED, so hi = floor((m + 128) / 256) = byte 1 of m + 128.
-                constexpr int kR = PACK ? 128 : 0;
-                const uint32_t lo = __byte_perm(__byte_perm((uint32_t)m0, (uint32_t)m1, 0x0040),
-                                                __byte_perm((uint32_t)m2, (uint32_t)m3, 0x0040), 0x5410);
-                const uint32_t hi = __byte_perm(__byte_perm((uint32_t)(m0 + kR), (uint32_t)(m1 + kR), 0x0051),
-                                                __byte_perm((uint32_t)(m2 + kR), (uint32_t)(m3 + kR), 0x0051), 0x5410);
-                *reinterpret_cast<uint32_t*>(xs_hi + tok * row_b + gi * 128 + lane * 4) = hi;
-                *reinterpret_cast<uint32_t*>(xs_lo + tok * row_b + gi * 128 + lane * 4) = lo;
-                const int sm = __reduce_add_sync(0xffffffffu, m0 + m1 + m2 + m3);
-                if (lane == 0) xs_tab[gi * p.mc + tok] = make_int2(sm, (int)__float_as_uint(sg));
+                constexpr float kMagic = 12582912.0f;
+                constexpr uint32_t kR = PACK ? 128u : 0u;
+                const uint32_t m0 = __float_as_uint(fmaf(a.x, inv, kMagic)), m1 = __float_as_uint(fmaf(a.y, inv, kMagic));
+                const uint32_t m4 = __float_as_uint(fmaf(b.x, inv, kMagic)), m3 = __float_as_uint(fmaf(b.y, inv, kMagic));
+                w01[u] = __byte_perm(__byte_perm(m0, m1, 0x0040), __byte_perm(m4, m3, 0x0040), 0x5410);             // lo
+                w23[u] = __byte_perm(__byte_perm(m0 + kR, m1 + kR, 0x0051), __byte_perm(m4 + kR, m3 + kR, 0x0051), 0x5410);   // hi
+                sum[u] = __reduce_add_sync(0xffffffffu, m0 + m1 + m4 + m3 - 4u * 0x4b400000u);
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int gi = warp + (gl0 + u) * WT;
+                if (gi < G) {
+                    *reinterpret_cast<uint32_t*>(xs_hi + tok * row_b + gi * 128 + lane * 4) = w23[u];
+                    *reinterpret_cast<uint32_t*>(xs_lo + tok * row_b + gi * 128 + lane * 4) = w01[u];
+                    if (lane == 0) xs_tab[gi * p.mc + tok] = make_int2((int)sum[u], (int)__float_as_uint(sg[u]));
+                }
             }
         }
         if (NORM) {
@@ -387,6 +440,14 @@ __global__ void __launch_bounds__(WARPS * SUBS * 32, 1) k_w4a16_v3(const W4Param
     size_t tp_my_slot = 0;
     if (tp_mode == 2)
         tp_my_slot = comm_ll_offset(tp_ws, tp->slot_bytes) + ((size_t)tp_parity * tp_ws + tp->rank) * tp_slot_bytes;
+
+    auto poison = [&](int tok, int tile, int row) {
+        const float po = s_poison[tok];
+        if constexpr (RT == kV3DeepRows) {
+            if (po != po) return v3_nonfinite_sum(p.packed, p.x + (size_t)tok * p.ldx, p.K, tile, row);
+        }
+        return po;
+    };
 
     int c_slot = 0;
     uint32_t c_parity = 0;
@@ -565,8 +626,8 @@ __global__ void __launch_bounds__(WARPS * SUBS * 32, 1) k_w4a16_v3(const W4Param
                     gate *= s_rstd[tok];
                     up *= s_rstd[tok];
                 }
-                gate += s_poison[tok];
-                up += s_poison[tok];
+                gate += poison(tok, st, rg);
+                up += poison(tok, st, rg + 8);
                 if (p.bias) {
                     gate += __half2float(p.bias[n0 + rg]);
                     up += __half2float(p.bias[n0 + rg + 8]);
@@ -588,8 +649,8 @@ __global__ void __launch_bounds__(WARPS * SUBS * 32, 1) k_w4a16_v3(const W4Param
                     lo *= s_rstd[tok];
                     hi *= s_rstd[tok];
                 }
-                lo += s_poison[tok];
-                hi += s_poison[tok];
+                lo += poison(tok, st, rlo);
+                hi += poison(tok, st, rlo + 8);
                 if (p.bias) {
                     lo += __half2float(p.bias[n0 + rlo]);
                     hi += __half2float(p.bias[n0 + rlo + 8]);
@@ -650,7 +711,7 @@ __global__ void __launch_bounds__(WARPS * SUBS * 32, 1) k_w4a16_v3(const W4Param
                     const int tok = e >> 5, row = e & 31;
                     float v = sum_red(tok * 32 + row);
                     if (NORM) v *= s_rstd[tok];
-                    v += s_poison[tok];
+                    v += poison(tok, st, row);
                     if (p.bias) v += __half2float(p.bias[n0 + row]);
                     __half h = __float2half_rn(v);
                     if (p.epi == ZL_EPI_RESIDUAL)
@@ -762,6 +823,24 @@ bool launch_w4_v3(const W4Params& p, bool pdl, cudaStream_t stream, cudaError_t*
     return false;
 }
 
+// Three or four rows of a K too wide for the 4-stage rings, no fused RMSNorm (the kernel that served these calls has none, so
+// what was refused stays refused).  Shared memory bounds the form: 4 x 14336 staged values take 118 KB of the 227, and three
+// ring stages per warp the rest.  The tcgen05 kernel pays its exchange of partial tiles at any M; N x K, 4 rows, it -> this kernel,
+// us: 4096 x 14336 21.4 -> 16.4, 8192 x 8192 22.3 -> 14.2, 28672 x 8192 47.7 -> 30.6, 512 x 8192 15.5 -> 10.3.
+bool w4_v3_deep_fits(int mc, int N, int K) {
+    (void)N;
+    return mc <= kV3DeepRows && K / kW4GroupK <= 8 * 16 &&
+           V3Smem<1, 16, 1, 3, kV3DeepRows>::kBytes + v3_stage_bytes(mc, K) <= kV3Budget &&
+           V3Smem<1, 8, 2, 3, kV3DeepRows>::kBytes + v3_stage_bytes(mc, K) <= kV3Budget;
+}
+
+cudaError_t launch_w4_v3_deep(const W4Params& p, bool pdl, cudaStream_t stream) {
+    const int smem = v3_stage_bytes(p.mc, p.K);
+    if (v3_is_tall(p))
+        return launch_v3_t<1, false, 16, 1, 3, kV3DeepRows, true>(p, V3Smem<1, 16, 1, 3, kV3DeepRows>::kBytes + smem, pdl, stream);
+    return launch_v3_t<1, false, 8, 2, 3, kV3DeepRows, true>(p, V3Smem<1, 8, 2, 3, kV3DeepRows>::kBytes + smem, pdl, stream);
+}
+
 bool w4_v3_fits(int mc, int N, int K) {
     const int G = K / kW4GroupK;
     if (G > 8 * 16) return false;
@@ -785,6 +864,10 @@ cudaError_t prepare_w4_v3() {
     ZL_SET1(false, 8, 2, 5) ZL_SET1(true, 8, 2, 5) ZL_SET1(false, 8, 2, 4) ZL_SET1(true, 8, 2, 4)
     ZL_SET1(false, 16, 1, 4) ZL_SET1(true, 16, 1, 4)
 #undef ZL_SET1
+    e = cudaFuncSetAttribute(k_w4a16_v3<1, false, 16, 1, 3, kV3DeepRows, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kV3Budget);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(k_w4a16_v3<1, false, 8, 2, 3, kV3DeepRows, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kV3Budget);
+    if (e != cudaSuccess) return e;
 #define ZL_SET2(NORM, W, SB, ST)                                                                               \
     e = cudaFuncSetAttribute(k_w4a16_v3<1, NORM, W, SB, ST, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
                              kV3Budget);                                                                        \
