@@ -128,3 +128,23 @@ def test_embedding_and_argmax(lib, cuda):
     assert out[3].item() == 77
     for i in (0, 1, 2, 4, 5, 6):
         assert out[i].item() == ref[i].item()
+
+
+@pytest.mark.parametrize("d", [8, 2048, 2056, 4096, 4104, 8192, 8200, 16384])
+@pytest.mark.parametrize("scale", [1.0, 2.5])
+def test_add_rmsnorm_row_lengths(lib, cuda, d, scale):
+    """each number of chunks a thread holds, in place as well, against float64: one rounding to bf16 (7 stored bits: half a unit is at most 2^-8 of the value)"""
+    from zhilight_b200 import ops
+    g = torch.Generator().manual_seed(d)
+    a, b, w = (torch.randn(*s, generator=g).bfloat16() for s in ((3, d), (3, d), (d,)))
+    for mode in (0, 1):
+        total = a.double() + b.double()
+        v = total.bfloat16().double() if mode == 0 else total
+        ref = v * torch.rsqrt((v * v).mean(1, keepdim=True) + 1e-5) * w.double() / scale
+        s, y = ops.add_rmsnorm(a.to(cuda), b.to(cuda), w.to(cuda), 1e-5, scale, mode=mode)
+        assert torch.equal(s.cpu(), total.bfloat16())
+        assert bool(((y.cpu().double() - ref).abs() <= 1.01 * 2.0 ** -8 * ref.abs() + 1e-30).all())
+    v = a.double()
+    ref = v * torch.rsqrt((v * v).mean(1, keepdim=True) + 1e-5) * w.double() / scale
+    y = ops.rmsnorm(a.to(cuda), w.to(cuda), 1e-5, scale)
+    assert bool(((y.cpu().double() - ref).abs() <= 1.01 * 2.0 ** -8 * ref.abs() + 1e-30).all())

@@ -156,3 +156,35 @@ def test_products_on_pairs_of_sms(lib, cuda, dtype, m, n, k):
     lim = (k / 32 + 4) * 2.0 ** -23 * mag + 2.0 ** (-11 if dtype == torch.float16 else -8) * ref.abs() + 2.0 ** -24
     assert not ((y.double() - ref).abs() > lim).any()
     assert lib.zl_gemm_tc_watchdog() == 0
+
+
+@pytest.mark.parametrize("tag", ["f16", "bf16"])
+@pytest.mark.parametrize("m,k", [(2, 8), (3, 2048), (3, 2056), (3, 4096), (2, 4104), (2, 8192), (2, 8200), (2, 16384), (3, 16392), (1, 40000)])
+def test_int8_quant_row_lengths_bit_exact(lib, cuda, tag, m, k):
+    """each number of chunks that a thread holds in registers, its first and last row length, and the form that reads rows twice"""
+    from zhilight_b200 import ops
+    x = _x(m, k, tag, seed=k)
+    q, s = ops.int8_quant_per_token(_dev(x, tag, cuda))
+    oq, os_ = oracle.int8_quant_per_token(x)
+    np.testing.assert_array_equal(q.cpu().numpy(), oq)
+    np.testing.assert_array_equal(s.cpu().numpy(), os_)
+
+
+@pytest.mark.parametrize("m,n,k", [(24, 8192, 8192), (40, 256, 128), (40, 300, 4096), (300, 4096, 1024)])
+def test_gemm_that_starts_during_the_quantisation(lib, cuda, m, n, k):
+    """the GEMM's weights are fetched while the rows are still being quantised: the same bytes as one launch after the other"""
+    from zhilight_b200 import ops
+    w = torch.randint(-127, 128, (n, k), dtype=torch.int8, device=cuda)
+    sw = torch.rand(n, device=cuda) * 0.01
+    for seed in range(6):
+        x = torch.randn(m, k, device=cuda, generator=torch.Generator(device=cuda).manual_seed(seed)).half()
+        got = ops.int8_linear(x, w, sw)
+        q, s = ops.int8_quant_per_token(x)
+        torch.cuda.synchronize()
+        assert torch.equal(got, ops.w8a8_gemm(q, s, w, sw, torch.float16, ops.W8_INT8))
+        w8 = w.view(torch.uint8) & 0x77                  # finite fp8 codes
+        one = torch.ones(1, device=cuda)
+        got = ops.fp8_linear(x, w8, one)
+        q, s = ops.fp8_quant_per_tensor(x)
+        torch.cuda.synchronize()
+        assert torch.equal(got, ops.w8a8_gemm(q, s, w8, one, torch.float16, ops.W8_FP8))

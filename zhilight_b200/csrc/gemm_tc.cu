@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
     }
     if (warp == 2) tc2_alloc(s_tmem);
     pdl_trigger();
-    pdl_wait();
+    if (KIND == kGt16) pdl_wait();   // 8-bit: below; the weights do not wait for the rows' quantisation (8192 x 8192, 24 rows: 1 us)
     if (GROUPED && warp == 3) {   // tiles before each group: a running sum over the groups' sizes
         int base = 0;
         for (int g0 = 0; g0 < p.groups; g0 += 32) {
@@ -231,21 +231,36 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
         uint32_t ph = 0;
         GtTile t;
         bool ok = true;
+        const uint32_t bytes = 2u * sub * (kGtAStage + (GROUPED ? 0 : p.box_rows * 128));
+        auto weights = [&](int at, int k) {   // one lane: the stage's bytes and this CTA's half of its weight rows
+            const uint32_t bar = cluster_map(smem_u32(&full[at]), 0);
+            if (rank == 0) mbar_expect_tx(&full[at], bytes);
+#pragma unroll
+            for (int u = 0; u < sub; ++u)     // a block behind K arrives as zeros
+                tma2_load_3d(smem + at * stage_bytes + u * block_bytes, &p.wmap, (k * sub + u) * kBlockK, t.n0 + (int)rank * 128, t.b, bar);
+        };
+        int ahead = 0;                        // stages of the first tile whose weights are on their way already
+        if (KIND != kGt16) {
+            if (gt_tile<GROUPED>(p, s_cum, pair, hint, t)) ahead = min(stages, ks);
+            if (tc_elect_one())
+                for (int k = 0; k < ahead; ++k) weights(k, k);
+            __syncwarp();
+            pdl_wait();
+        }
         for (int i = pair; ok && gt_tile<GROUPED>(p, s_cum, i, hint, t); i += pairs) {
             const int tb = t.t0 + (int)rank * (t.ntok >> 1);
-            const uint32_t bytes = 2u * sub * (kGtAStage + (GROUPED ? 0 : p.box_rows * 128));
             for (int k = 0; k < ks; ++k) {
                 if (!(ok = tc2_wait(&empty[st], ph ^ 1u, s_abort, &g_gemm_tc_err, 0x2100 + st))) break;
                 if (tc_elect_one()) {
-                    const uint32_t bar = cluster_map(smem_u32(&full[st]), 0);
-                    if (rank == 0) mbar_expect_tx(&full[st], bytes);
+                    if (KIND == kGt16 || ahead <= 0) weights(st, k);
+                    if (!GROUPED) {
+                        const uint32_t bar = cluster_map(smem_u32(&full[st]), 0);
 #pragma unroll
-                    for (int u = 0; u < sub; ++u) {   // a block behind K arrives as zeros
-                        uint8_t* sa = smem + st * stage_bytes + u * block_bytes;
-                        tma2_load_3d(sa, &p.wmap, (k * sub + u) * kBlockK, t.n0 + (int)rank * 128, t.b, bar);
-                        if (!GROUPED) tma2_load_3d(sa + kGtAStage, &p.xmap, (k * sub + u) * kBlockK, tb, t.b, bar);
+                        for (int u = 0; u < sub; ++u)
+                            tma2_load_3d(smem + st * stage_bytes + u * block_bytes + kGtAStage, &p.xmap, (k * sub + u) * kBlockK, tb, t.b, bar);
                     }
                 }
+                --ahead;
                 __syncwarp();
                 if (++st == stages) {
                     st = 0;
@@ -254,6 +269,7 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
             }
         }
     } else if (warp == 1 && rank == 0) {
+        if (KIND != kGt16) pdl_wait();       // nothing of use arrives before, and the bounded waits start here
         int st = 0, acc = 0, hint = 0;
         uint32_t ph = 0, acc_ph = 0;
         GtTile t;
@@ -351,6 +367,7 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
     } else if (warp >= 4) {
+        if (KIND != kGt16) pdl_wait();
         const int q = warp & 3, set = (warp - 4) >> 2;
         int acc = 0, hint = 0;
         uint32_t acc_ph = 0;

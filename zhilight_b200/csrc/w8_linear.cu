@@ -67,7 +67,10 @@ __device__ __forceinline__ V block_reduce(V v, V* sh, bool is_max) {
 }
 
 // quant_calc_scale (quant_kernel.cu:15-47): scale = absmax/127, q = int8(nearbyint(x * (127/absmax))).
-template <typename T>
+// Bound by latency (24 x 8192: 0.6 MB): with NC > 0 a thread holds its NC chunks of 8 values in registers, all loads on their way at
+// once and the row read one time; rows longer than 8 chunks per thread (K > 16384) are read twice, chunk after chunk.
+// 24 x 8192 fp16: 6.2 -> 3.8 us.
+template <typename T, int NC>
 __global__ void __launch_bounds__(256) k_int8_quant_per_token(const T* __restrict__ x, int ldx, int8_t* __restrict__ q,
                                                               float* __restrict__ scale, int K) {
     __shared__ float sh[8];
@@ -75,17 +78,29 @@ __global__ void __launch_bounds__(256) k_int8_quant_per_token(const T* __restric
     pdl_wait();
     const T* row = x + (size_t)blockIdx.x * ldx;
     float amax = 0.f;
-    for (int i = threadIdx.x * 8; i < K; i += blockDim.x * 8) {
+    auto take_max = [&](const uint4& raw) {
         float v[8];
-        unpack8<T>(ld_cg_u4(row + i), v);
+        unpack8<T>(raw, v);
 #pragma unroll
         for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));
+    };
+    uint4 held[NC > 0 ? NC : 1];
+    if constexpr (NC > 0) {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const int i = (threadIdx.x + c * 256) * 8;
+            held[c] = i < K ? ld_cg_u4(row + i) : make_uint4(0, 0, 0, 0);   // zeros leave the maximum as it is
+        }
+#pragma unroll
+        for (int c = 0; c < NC; ++c) take_max(held[c]);
+    } else {
+        for (int i = threadIdx.x * 8; i < K; i += 256 * 8) take_max(ld_cg_u4(row + i));
     }
     amax = block_reduce(amax, sh, true);
     const float bs = __fdiv_rn(127.f, amax);
-    for (int i = threadIdx.x * 8; i < K; i += blockDim.x * 8) {
+    auto convert = [&](const uint4& raw, int i) {
         float v[8];
-        unpack8<T>(ld_cg_u4(row + i), v);
+        unpack8<T>(raw, v);
         uint32_t w[2] = {0, 0};
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -95,6 +110,15 @@ __global__ void __launch_bounds__(256) k_int8_quant_per_token(const T* __restric
             w[j >> 2] |= (uint32_t)(qi & 0xff) << (8 * (j & 3));
         }
         *reinterpret_cast<uint2*>(q + (size_t)blockIdx.x * K + i) = make_uint2(w[0], w[1]);
+    };
+    if constexpr (NC > 0) {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const int i = (threadIdx.x + c * 256) * 8;
+            if (i < K) convert(held[c], i);
+        }
+    } else {
+        for (int i = threadIdx.x * 8; i < K; i += 256 * 8) convert(ld_cg_u4(row + i), i);
     }
     if (threadIdx.x == 0) scale[blockIdx.x] = __fdiv_rn(amax, 127.f);
 }
@@ -405,6 +429,14 @@ static cudaError_t launch_w8(const uint8_t* xq, const float* sx, const uint8_t* 
     return launch_w8_ks<T, FP8, 4>(xq, sx, w, sw, sw_f32, bias, y, mc, N, K, pdl, st);
 }
 
+template <typename T>
+static cudaError_t launch_int8_quant(const T* x, int ldx, int8_t* q, float* scale, int M, int K, bool pdl, cudaStream_t stream) {
+    const int chunks = cdiv(K, 256 * 8);
+    auto kernel = chunks <= 1 ? k_int8_quant_per_token<T, 1> : chunks <= 2 ? k_int8_quant_per_token<T, 2>
+                  : chunks <= 4 ? k_int8_quant_per_token<T, 4> : chunks <= 8 ? k_int8_quant_per_token<T, 8> : k_int8_quant_per_token<T, 0>;
+    return launch(kernel, dim3(M), dim3(256), 0, stream, pdl, x, ldx, q, scale, K);
+}
+
 }  // namespace zl
 
 using namespace zl;
@@ -415,13 +447,8 @@ extern "C" int zl_int8_quant_per_token(const void* x, int ldx, void* q, float* s
     ZL_CHECK_ARG(dtype == ZL_F16 || dtype == ZL_BF16);
     ZL_CHECK_SUPPORTED(K % 8 == 0 && ldx % 8 == 0 && ldx >= K);
     ZL_CHECK_ARG((reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(q) & 7) == 0);
-    cudaError_t e;
-    if (dtype == ZL_F16)
-        e = launch(k_int8_quant_per_token<__half>, dim3(M), dim3(256), 0, stream, pdl != 0,
-                   static_cast<const __half*>(x), ldx, static_cast<int8_t*>(q), scale, K);
-    else
-        e = launch(k_int8_quant_per_token<__nv_bfloat16>, dim3(M), dim3(256), 0, stream, pdl != 0,
-                   static_cast<const __nv_bfloat16*>(x), ldx, static_cast<int8_t*>(q), scale, K);
+    const cudaError_t e = dtype == ZL_F16 ? launch_int8_quant(static_cast<const __half*>(x), ldx, static_cast<int8_t*>(q), scale, M, K, pdl != 0, stream)
+                                          : launch_int8_quant(static_cast<const __nv_bfloat16*>(x), ldx, static_cast<int8_t*>(q), scale, M, K, pdl != 0, stream);
     ZL_CHECK_CUDA(e);
     return ZL_OK;
 }

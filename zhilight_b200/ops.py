@@ -252,13 +252,14 @@ def w8a8_gemm(xq, x_scale, w, w_scale, out_dtype, kind=W8_INT8, bias=None, pdl=F
 def int8_linear(x, w_q, w_scale, bias=None, pdl=False):
     """Int8Linear::forward (linear.cpp:560-636) in two launches instead of three."""
     q, s = int8_quant_per_token(x, pdl)
-    return w8a8_gemm(q, s, w_q, w_scale, x.dtype, W8_INT8, bias, pdl)
+    # the launch before is the quantisation, itself behind everything earlier: the GEMM may start on its weights during it
+    return w8a8_gemm(q, s, w_q, w_scale, x.dtype, W8_INT8, bias, True)
 
 
 def fp8_linear(x, w_fp8, w_scale, bias=None, pdl=False):
     """Fp8Linear::forward (linear.cpp:1660-1695)."""
     q, s = fp8_quant_per_tensor(x, pdl)
-    return w8a8_gemm(q, s, w_fp8, w_scale, x.dtype, W8_FP8, bias, pdl)
+    return w8a8_gemm(q, s, w_fp8, w_scale, x.dtype, W8_FP8, bias, True)
 
 
 def rmsnorm(x, weight, eps, scale=1.0, pdl=False):
