@@ -107,7 +107,6 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
-__device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 // ---- host: cuTensorMapEncodeTiled through the runtime's driver entry point (no -lcuda) ----
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -157,17 +156,15 @@ inline bool tc_make_map_nd(CUtensorMap* map, const void* base, CUtensorMapDataTy
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// per-device scratch of the split-k reductions: fp32 / int32 partial tiles, arrival counters, watchdog word
+// per-device scratch of the stream-k kernel: partial tiles, watchdog word, hand-over trace
 struct TcDeviceState {
-    float* ws = nullptr;
+    long long* trace = nullptr;        // ZL_TC_DBG & 16
     uint2* ws_ll = nullptr;            // W4 kernel: tagged partial-tile words {fp32 bits, tag}, all zero between launches
     size_t ws_ll_bytes = 0;
-    unsigned* counters = nullptr;
     unsigned* err = nullptr;
-    size_t ws_bytes = 0;
 };
 constexpr size_t kTcWsLlBytes = 80ull << 20;   // >= 2 slots x 148 CTAs x 256 tokens x 128 rows x 8 B
-constexpr size_t kTcWsBytes = 64ull << 20;   // >= 2 x 148 items x 256 tokens x 128 rows x 4 B
+constexpr size_t kTcTraceBytes = 1 << 20;
 constexpr int kTcMaxTiles = 8192;
 TcDeviceState* tc_state();                   // w4a16_tc.cu; nullptr before prepare_w4_tc() ran on the current device
 

@@ -1,6 +1,6 @@
 // W4A16 GEMM on the 5th-generation tensor cores: tcgen05.mma (kind::f16) with the dequantised weights as the A operand in
-// TENSOR MEMORY, activations through tensor-TMA, TMEM accumulators.  Serves every M the exact-integer mma.sync kernel
-// (w4a16_gemm_v3.cu) cannot stage: batch 17..256 decode and chunked prefill.
+// TENSOR MEMORY, activations through tensor-TMA, TMEM accumulators.  Serves the M <= 256 that neither the exact-integer
+// mma.sync kernel (w4a16_gemm_v3.cu) can stage nor whole tiles on pairs of SMs (w4a16_tc2.cu) serve faster.
 //
 // Replaces the reference's Marlin kernel (src/nn/quant/marlin/gptq_marlin.cu:425-1620), the M <= 40 GEMV tiles of
 // KERNEL_gemm_warp_reduce (src/nn/quant/gptq/q_gemm_k_major.cu:176-237, 580-686: the weight matrix is streamed
@@ -505,12 +505,10 @@ cudaError_t prepare_w4_tc() {
     TcDeviceState* st = tc_state();
     if (!st) return cudaErrorInvalidDevice;
     cudaError_t e;
-    if (!st->ws) {
-        if ((e = cudaMalloc((void**)&st->ws, kTcWsBytes)) != cudaSuccess) return e;
-        if ((e = cudaMalloc((void**)&st->counters, (kTcMaxTiles + 16) * sizeof(unsigned))) != cudaSuccess) return e;
-        if ((e = cudaMemset(st->counters, 0, (kTcMaxTiles + 16) * sizeof(unsigned))) != cudaSuccess) return e;
-        st->err = st->counters + kTcMaxTiles;
-        st->ws_bytes = kTcWsBytes;
+    if (!st->trace) {
+        if ((e = cudaMalloc((void**)&st->trace, kTcTraceBytes)) != cudaSuccess) return e;
+        if ((e = cudaMalloc((void**)&st->err, sizeof(unsigned))) != cudaSuccess) return e;
+        if ((e = cudaMemset(st->err, 0, sizeof(unsigned))) != cudaSuccess) return e;
         if ((e = cudaMalloc((void**)&st->ws_ll, kTcWsLlBytes)) != cudaSuccess) return e;
         if ((e = cudaMemset(st->ws_ll, 0, kTcWsLlBytes)) != cudaSuccess) return e;
         st->ws_ll_bytes = kTcWsLlBytes;
@@ -539,9 +537,9 @@ extern "C" unsigned zl_w4_tc_watchdog(void) {
 // copies the ZL_TC_DBG & 16 stamps of the last launch ([11 roles][64 stages][4] clock64 values) to the host; debugging aid
 extern "C" int zl_w4_tc_read_trace(long long* out, int n) {
     TcDeviceState* st = tc_state();
-    if (!st || !st->ws || n > (1 << 17)) return ZL_ERR_INVALID_ARG;
+    if (!st || !st->trace || n > (1 << 17)) return ZL_ERR_INVALID_ARG;
     cudaDeviceSynchronize();
-    return cudaMemcpy(out, reinterpret_cast<uint8_t*>(st->ws) + st->ws_bytes - (1 << 20), (size_t)n * 8, cudaMemcpyDeviceToHost) ==
+    return cudaMemcpy(out, st->trace, (size_t)n * 8, cudaMemcpyDeviceToHost) ==
                    cudaSuccess
                ? ZL_OK
                : ZL_ERR_CUDA;
@@ -654,7 +652,6 @@ bool w4_tc_params(W4TcParams& q, const W4Params& p) {
     q.dim_head = p.dim_head;
     q.dbg = 0;
     q.ws = nullptr;
-    q.ws_f32 = nullptr;
     q.trace = nullptr;
     q.err = nullptr;
     q.ntok = q.tok_tiles = 0;
@@ -664,7 +661,7 @@ bool w4_tc_params(W4TcParams& q, const W4Params& p) {
 
 cudaError_t launch_w4_tc(const W4Params& p, bool pdl, cudaStream_t stream) {
     TcDeviceState* st = tc_state();
-    if (!st || !st->ws) return cudaErrorNotSupported;
+    if (!st || !st->ws_ll) return cudaErrorNotSupported;
     const int ntok = p.mc <= 32 ? 32 : p.mc <= 64 ? 64 : p.mc <= 128 ? 128 : 256;
     const int n_tiles = p.N / kTcRows, G = p.K / kW4GroupK;
     W4TcParams q;
@@ -677,9 +674,8 @@ cudaError_t launch_w4_tc(const W4Params& p, bool pdl, cudaStream_t stream) {
         q.dbg = tc_dbg;
     }
     q.ws = st->ws_ll;
-    q.ws_f32 = st->ws;
     q.err = st->err;
-    q.trace = reinterpret_cast<long long*>(reinterpret_cast<uint8_t*>(st->ws) + st->ws_bytes - (1 << 20));   // last MB of the workspace
+    q.trace = st->trace;
     const int ctas = tc_pick_ctas(n_tiles, G);
     if ((size_t)2 * ctas * p.mc * kTcRows * 8 > st->ws_ll_bytes) return cudaErrorInvalidValue;
     const dim3 grid(ctas);

@@ -18,7 +18,6 @@ struct alignas(64) W4TcParams {
     int M, N, K, epi;
     int dbg;                    // ZL_TC_DBG timing ablations (results are wrong): 1 no x loads, 2 no dequant, 4 no MMA, 8 no weight loads
     uint2* ws;                  // [2 * CTA + slot][M][128] tagged words {fp32 partial sum, tag}: all zero between launches
-    float* ws_f32;              // plain scratch (its last MB carries the ZL_TC_DBG trace)
     unsigned* err;              // watchdog code
     long long* trace;           // ZL_TC_DBG & 16: clock64 stamps of CTA 0, [role][64 stages][8]
     const float* cos;
