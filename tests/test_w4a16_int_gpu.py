@@ -186,8 +186,8 @@ def test_qkv_rope_epilogue_int(lib, cuda, d, hq, hkv, k, t):
 @pytest.mark.parametrize("m,k,n", [(3, 9728 + 128, 512), (4, 7424, 512), (4, 8192, 128 * 40), (3, 14336, 4096), (4, 14336, 4096), (4, 14336 + 256, 256), (2, 16384, 256)])
 @pytest.mark.parametrize("epilogue", ["none", "residual", "swiglu"])
 def test_wide_k_of_few_rows(lib, cuda, m, k, n, epilogue):
-    """3-stage rings: what the 4-stage ones leave no room for.  Each output is exact but for the activations' 15-bit groups
-    (2^-15 of a group's maximum each) and its own rounding to fp16, 2^-11."""
+    """What the integer kernel's rings leave no room for goes to the tcgen05 kernel, which takes the activations as they are: weights and
+    outputs round to fp16, half a unit 2^-11 of a value at most, so 2^-11 / sqrt(3) each on average, 4e-4 together."""
     from zhilight_b200 import ops
     w, packed_i, _, _ = _setup(cuda, k, n, False, 8)
     assert lib.zl_w4_int_layout_route(m, n, k) == 4          # (what callers choose a fused RMSNorm by: refused at these sizes)
@@ -228,3 +228,33 @@ def test_wide_k_nonfinite_activations(lib, cuda):
     got = y[1].float().cpu().numpy()
     assert np.array_equal(np.isnan(got), col == 0) and np.array_equal(np.sign(got[col != 0]), np.sign(col[col != 0]))
     assert np.isinf(got[col != 0]).all()
+
+
+@pytest.mark.parametrize("m,k", [(3, 14336), (4, 14336), (4, 8192)])
+@pytest.mark.parametrize("peak,every", [(400.0, False), (4000.0, False), (30000.0, False), (1000.0, True)])
+def test_wide_k_keeps_small_values_beside_a_large_one(lib, cuda, m, k, peak, every):
+    """One activation far above the rest of its group (or one in every group): the outputs whose weight there is zero see only the small
+    ones, with the fp16 kernels' error (4e-4, see above), not a share of the large one's."""
+    from zhilight_b200 import ops
+    n = 512 if every else 4096
+    groups = np.arange(k // 128) if every else np.array([k // 256])
+    places = groups * 128 + 37
+    w, packed_i, _, (o_qw, o_qz, o_sc) = _setup(cuda, k, n, True, 5)
+    if every:                                            # no output has zeros at all of these places by chance
+        qw, qz, sc, gi = gptq.make_gptq_checkpoint(k, n, 128, True, seed=5)
+        for p in places:                                 # words of eight rows, four bits each; 8 is the symmetric zero
+            shift = np.uint32(4 * (p % 8))
+            qw.view(np.uint32)[p // 8] = (qw.view(np.uint32)[p // 8] & ~(np.uint32(15) << shift)) | (np.uint32(8) << shift)
+        o_qw, o_qz, o_sc, _ = gptq.to_k_major(qw, qz, sc, gi, 128)
+        w = gptq.dequant_k_major_f32(o_qw, o_qz, o_sc, True)
+        packed_i = ops.w4_pack(_dev(o_qw.view(np.int32), cuda), _dev(o_qz, cuda), _dev(o_sc, cuda), 128, True, None, variant=1)
+    w = w if w.shape[0] == n else w.T
+    blind = np.flatnonzero((w[:, places] == 0).all(1))
+    assert blind.size >= 64
+    x = torch.randn(m, k, generator=torch.Generator().manual_seed(k))
+    x[:, places] = peak
+    x = x.half()
+    y = ops.w4a16_gemm_fused(x.to(cuda), packed_i, n, k, variant=1).double().cpu().numpy()[:, blind]
+    ref = x.double().numpy() @ w[blind].T.astype(np.float64)
+    for i in range(m):
+        assert rel_l2(y[i], ref[i]) <= 4e-4, i

@@ -46,8 +46,6 @@ cudaError_t prepare_w4_v2();
 // exact-integer kernel on the ZLW4I layout; false = staged activations do not fit shared memory
 bool launch_w4_v3(const W4Params& p, bool pdl, cudaStream_t stream, cudaError_t* err);
 bool w4_v3_fits(int mc, int N, int K);
-bool w4_v3_deep_fits(int mc, int N, int K);
-cudaError_t launch_w4_v3_deep(const W4Params& p, bool pdl, cudaStream_t stream);
 cudaError_t prepare_w4_v3();
 // tcgen05 / TMEM / TMA kernel on the ZLW4I layout (w4a16_tc.cu): up to 256 tokens per launch, N % 128 == 0, no fused
 // RMSNorm prologue (ln_w is ignored)

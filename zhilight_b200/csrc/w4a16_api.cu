@@ -139,8 +139,6 @@ extern "C" int zl_w4a16_gemm_fused(const zl_w4_fused_args_t* a, zl_stream_t stre
     ZL_CHECK_SUPPORTED(route != 0 && "ZLW4I layout: M > 16 (or staged activations too large) and N % 128 != 0: use variant 0");
     ZL_CHECK_SUPPORTED(!(route == 4 && a->ln_weight) && "the tcgen05 kernel has no fused RMSNorm prologue: run zl_rmsnorm first");
     const bool pairs = route == 4 && w4_tc2_route(a->M, a->N, a->K);
-    // up to 4 rows of a wide K: the integer kernel with shorter rings (both sides measured at w4_v3_deep_fits)
-    const bool deep = route == 4 && w4_v3_deep_fits(a->M, a->N, a->K);
     const int step = pairs ? a->M : route == 4 ? 256 : 32;
     for (int m0 = 0; m0 < a->M; m0 += step) {
         W4Params p;
@@ -182,9 +180,7 @@ extern "C" int zl_w4a16_gemm_fused(const zl_w4_fused_args_t* a, zl_stream_t stre
         p.tp_h_out = static_cast<__half*>(a->tp_h_out);
         p.pf_ptr = static_cast<const uint8_t*>(a->prefetch_ptr);
         p.pf_bytes = a->prefetch_bytes;
-        if (deep) {
-            ZL_CHECK_CUDA(launch_w4_v3_deep(p, a->pdl != 0, stream));
-        } else if (pairs) {
+        if (pairs) {
             ZL_CHECK_CUDA(launch_w4_tc2(p, a->pdl != 0, stream));
         } else if (route == 4) {
             ZL_CHECK_CUDA(launch_w4_tc(p, a->pdl != 0 && m0 == 0, stream));

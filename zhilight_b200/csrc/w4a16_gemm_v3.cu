@@ -42,16 +42,13 @@ __device__ __forceinline__ void imma_u8u8(int (&d)[4], const uint32_t (&a)[4], u
 // reduction), while the integer decomposition of the activations is staged ONCE per CTA by all warps together:
 //   wide : SUBS=2 x 8 warps, 5-stage rings  (N/32 > #SMs: qkv, gate/up)  -- two tile pipelines per SM
 //   tall : SUBS=1 x 16 warps, 4-stage rings (N/32 <= #SMs: o_proj, down) -- k split 16 ways
-//   deep : 3-stage rings, one reduction buffer of 4 token rows -- what leaves room for 4 staged rows of K up to 14.6 k.
 // RT = token rows kept in the split-k reduction buffers (even, >= mc): small batches shrink them to make room for
 // deeper rings -- the tile loop is latency-bound on ring depth (4 -> 5 stages is worth ~25 %).
-constexpr int kV3DeepRows = 4;
-
 template <int NT, int WARPS, int SUBS, int STAGES, int RT = NT * 8>
 struct V3Smem {
     static constexpr int kWarpsTotal = WARPS * SUBS;
     static constexpr int kRingBytes = kWarpsTotal * STAGES * kW4BlockBytes;
-    static constexpr int kRedBufs = (NT == 1 && RT != kV3DeepRows) ? 2 : 1;
+    static constexpr int kRedBufs = (NT == 1) ? 2 : 1;
     static constexpr int kRedFloats = WARPS * RT * 32;                     // per sub-CTA, per buffer
     static constexpr int kBarOff = kRingBytes;
     static constexpr int kRedOff = kBarOff + kWarpsTotal * STAGES * 8;
@@ -68,31 +65,6 @@ __host__ __device__ inline int v3_stage_bytes(int mc, int K) {
 
 __device__ __forceinline__ void sub_barrier(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-
-// sum over the groups of a token that hold an Inf or NaN (the staging left them out of the integer sums) of w * x, the weight
-// rounded to fp16: +-Inf or NaN as in the fp16 kernels.  Plain loops over global memory, for such tokens only.
-__device__ __noinline__ float v3_nonfinite_sum(const uint8_t* packed, const __half* x, int K, int tile, int row) {
-    const int G = K / kW4GroupK;
-    const int tt = row >> 4, g = row & 7, up = (row >> 3) & 1;
-    float sum = 0.f;
-    for (int gi = 0; gi < G; ++gi) {
-        const __half* xg = x + gi * kW4GroupK;
-        bool finite = true;
-        for (int k = 0; k < kW4GroupK; ++k) finite &= (__half_as_ushort(xg[k]) & 0x7c00u) != 0x7c00u;
-        if (finite) continue;
-        const uint8_t* blk = packed + ((size_t)tile * G + gi) * kW4BlockBytes;
-        const __half2 s2 = reinterpret_cast<const __half2*>(blk + kW4ScaleOff)[tt * 8 + g];
-        const float s = up ? __high2float(s2) : __low2float(s2);
-        const int z = (blk[kW4ZeroOff + tt * 8 + g] >> (4 * up)) & 15;
-        for (int k = 0; k < kW4GroupK; ++k) {   // the word of (row, k): see ZLW4I in w4_layout.cuh
-            const int j = ((k >> 3) & 3) * 2 + ((k >> 2) & 1);
-            const uint32_t word = reinterpret_cast<const uint32_t*>(blk)[((tt * 2 + (j >> 2)) * 32 + g * 4 + (k >> 5)) * 4 + (j & 3)];
-            const int q = (word >> (8 * (k & 3) + 4 * up)) & 15;
-            sum = fmaf(__half2float(__float2half_rn((float)(q - z) * s)), __half2float(xg[k]), sum);
-        }
-    }
-    return sum;
 }
 
 // PACK block math for NB blocks of one warp at once (NB = 2: two independent dependency chains interleave).
@@ -441,14 +413,6 @@ __global__ void __launch_bounds__(WARPS * SUBS * 32, 1) k_w4a16_v3(const W4Param
     if (tp_mode == 2)
         tp_my_slot = comm_ll_offset(tp_ws, tp->slot_bytes) + ((size_t)tp_parity * tp_ws + tp->rank) * tp_slot_bytes;
 
-    auto poison = [&](int tok, int tile, int row) {
-        const float po = s_poison[tok];
-        if constexpr (RT == kV3DeepRows) {
-            if (po != po) return v3_nonfinite_sum(p.packed, p.x + (size_t)tok * p.ldx, p.K, tile, row);
-        }
-        return po;
-    };
-
     int c_slot = 0;
     uint32_t c_parity = 0;
     for (int ti = 0; ti < my_tiles; ++ti) {
@@ -626,8 +590,8 @@ __global__ void __launch_bounds__(WARPS * SUBS * 32, 1) k_w4a16_v3(const W4Param
                     gate *= s_rstd[tok];
                     up *= s_rstd[tok];
                 }
-                gate += poison(tok, st, rg);
-                up += poison(tok, st, rg + 8);
+                gate += s_poison[tok];
+                up += s_poison[tok];
                 if (p.bias) {
                     gate += __half2float(p.bias[n0 + rg]);
                     up += __half2float(p.bias[n0 + rg + 8]);
@@ -649,8 +613,8 @@ __global__ void __launch_bounds__(WARPS * SUBS * 32, 1) k_w4a16_v3(const W4Param
                     lo *= s_rstd[tok];
                     hi *= s_rstd[tok];
                 }
-                lo += poison(tok, st, rlo);
-                hi += poison(tok, st, rlo + 8);
+                lo += s_poison[tok];
+                hi += s_poison[tok];
                 if (p.bias) {
                     lo += __half2float(p.bias[n0 + rlo]);
                     hi += __half2float(p.bias[n0 + rlo + 8]);
@@ -711,7 +675,7 @@ __global__ void __launch_bounds__(WARPS * SUBS * 32, 1) k_w4a16_v3(const W4Param
                     const int tok = e >> 5, row = e & 31;
                     float v = sum_red(tok * 32 + row);
                     if (NORM) v *= s_rstd[tok];
-                    v += poison(tok, st, row);
+                    v += s_poison[tok];
                     if (p.bias) v += __half2float(p.bias[n0 + row]);
                     __half h = __float2half_rn(v);
                     if (p.epi == ZL_EPI_RESIDUAL)
@@ -823,24 +787,6 @@ bool launch_w4_v3(const W4Params& p, bool pdl, cudaStream_t stream, cudaError_t*
     return false;
 }
 
-// Three or four rows of a K too wide for the 4-stage rings, no fused RMSNorm (the kernel that served these calls has none, so
-// what was refused stays refused).  Shared memory bounds the form: 4 x 14336 staged values take 118 KB of the 227, and three
-// ring stages per warp the rest.  The tcgen05 kernel pays its exchange of partial tiles at any M; N x K, 4 rows, it -> this kernel,
-// us: 4096 x 14336 21.4 -> 16.4, 8192 x 8192 22.3 -> 14.2, 28672 x 8192 47.7 -> 30.6, 512 x 8192 15.5 -> 10.3.
-bool w4_v3_deep_fits(int mc, int N, int K) {
-    (void)N;
-    return mc <= kV3DeepRows && K / kW4GroupK <= 8 * 16 &&
-           V3Smem<1, 16, 1, 3, kV3DeepRows>::kBytes + v3_stage_bytes(mc, K) <= kV3Budget &&
-           V3Smem<1, 8, 2, 3, kV3DeepRows>::kBytes + v3_stage_bytes(mc, K) <= kV3Budget;
-}
-
-cudaError_t launch_w4_v3_deep(const W4Params& p, bool pdl, cudaStream_t stream) {
-    const int smem = v3_stage_bytes(p.mc, p.K);
-    if (v3_is_tall(p))
-        return launch_v3_t<1, false, 16, 1, 3, kV3DeepRows, true>(p, V3Smem<1, 16, 1, 3, kV3DeepRows>::kBytes + smem, pdl, stream);
-    return launch_v3_t<1, false, 8, 2, 3, kV3DeepRows, true>(p, V3Smem<1, 8, 2, 3, kV3DeepRows>::kBytes + smem, pdl, stream);
-}
-
 bool w4_v3_fits(int mc, int N, int K) {
     const int G = K / kW4GroupK;
     if (G > 8 * 16) return false;
@@ -864,10 +810,6 @@ cudaError_t prepare_w4_v3() {
     ZL_SET1(false, 8, 2, 5) ZL_SET1(true, 8, 2, 5) ZL_SET1(false, 8, 2, 4) ZL_SET1(true, 8, 2, 4)
     ZL_SET1(false, 16, 1, 4) ZL_SET1(true, 16, 1, 4)
 #undef ZL_SET1
-    e = cudaFuncSetAttribute(k_w4a16_v3<1, false, 16, 1, 3, kV3DeepRows, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kV3Budget);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_w4a16_v3<1, false, 8, 2, 3, kV3DeepRows, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kV3Budget);
-    if (e != cudaSuccess) return e;
 #define ZL_SET2(NORM, W, SB, ST)                                                                               \
     e = cudaFuncSetAttribute(k_w4a16_v3<1, NORM, W, SB, ST, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
                              kV3Budget);                                                                        \
