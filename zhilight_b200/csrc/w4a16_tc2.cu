@@ -18,6 +18,10 @@
 //   warp 24      weights  : tensor-TMA of the 4 ZLW4I records of a stage and their trailers, this CTA's 128 rows
 //   warp 25      x        : this CTA's half of the tokens, counted on the leader's barrier
 //   warp 26      MMA      : of the leader, 8 x 256 x ntok x 16 per stage; TMEM allocation
+//
+// The launch may start while its predecessor still runs, for as long as that takes (an all-reduce waits for its slowest rank).  A wait
+// that ends only after x has come would count that time, so no warp enters one before griddepcontrol.wait: the weights of the first RS
+// stages are fetched and each group's first stage is converted ahead of it, neither of which waits for anything but the weights.
 #include "tc2_common.cuh"
 #include "w4a16_tc.cuh"
 
@@ -101,12 +105,13 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
     if (warp == C::kWarpRaw) {
         // constants: may run ahead of the predecessor kernel (PDL).  The row tiles of one wave are read by several pairs and again
         // by the next token tiles: no evict-first hint here
-        int rs = 0;
+        int rs = 0, st = 0;
         uint32_t ph = 0;
         bool ok = true;
         for (int i = pair; ok && t2_tile(p, i, t); i += pairs) {
             const int rec = (t.n0 + (int)rank * 128) / 32;
-            for (int g = 0; g < G; ++g) {
+            for (int g = 0; g < G; ++g, ++st) {
+                if (st == C::RS) pdl_wait();
                 if (!(ok = tc2_wait(&raw_empty[rs], ph ^ 1u, s_abort, &g_w4_tc2_err, 0x3100 + rs))) break;
                 if (tc_elect_one()) {
                     mbar_expect_tx(&raw_full[rs], C::kNib + 4 * 80);
@@ -154,6 +159,7 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
         }
     } else if (warp == C::kWarpMma) {
         if (rank == 0) {
+            pdl_wait();
             int as = 0, acc = 0;
             uint32_t ph = 0, acc_ph = 0;
             bool ok = true;
@@ -200,6 +206,7 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
         for (int i = pair; ok && t2_tile(p, i, t); i += pairs) {
             for (int g = 0; g < G; ++g, ++st) {
                 if (st % C::AS != as) continue;
+                if (st == as + C::AS) pdl_wait();
                 const int rs = st % C::RS;
                 if (!(ok = tc2_wait(&raw_full[rs], (uint32_t)(st / C::RS) & 1u, s_abort, &g_w4_tc2_err, 0x3600 + rs))) break;
                 const uint8_t* nib = smem + C::kNibOff + rs * C::kNib + q * 2048;
