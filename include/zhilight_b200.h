@@ -144,13 +144,19 @@ int zl_w4_int_kernel_fits(int M, int N, int K);
 /* which kernel serves (M, N, K) on the ZLW4I layout (variant 1): 3 = exact-integer mma.sync kernel, 4 = tcgen05 / TMEM /
  * TMA kernel (any M, N % 128 == 0, no fused RMSNorm prologue), 0 = neither (pack variant 0 and use the fp16 mma.sync kernel). */
 int zl_w4_int_layout_route(int M, int N, int K);
-/* last watchdog code published by a tcgen05 kernel on the current device (0 = none); a bounded mbarrier wait that expires
+/* last watchdog code published by the 4-bit stream-k kernel on the current device (0 = none); a bounded mbarrier wait that expires
  * records which pipeline barrier starved and traps instead of hanging the GPU. */
 unsigned zl_w4_tc_watchdog(void);
-/* the same of the general tensor-core GEMM (zl_gemm_nt*, zl_dense_gemm_skinny* with prompt-sized M) */
+/* The kernels over pairs of SMs do not trap: a wait that expires leaves a code in host memory and the kernel returns with its output
+ * incomplete.  zl_check_waits, called after a synchronisation, is ZL_OK, or ZL_ERR_CUDA once for each kernel (of this process) that has
+ * left a code since it was last reported; zl_last_error names it.  The decoders ask at the end of every step, the GEMMs at each call. */
+int zl_check_waits(void);
+/* the unreported code of the general tensor-core GEMM (zl_gemm_nt*, zl_dense_gemm_skinny* and zl_w8a8_gemm with prompt-sized M) and of
+ * the 4-bit GEMM over pairs of SMs, after a synchronisation of the device; 0 = none */
 unsigned zl_gemm_tc_watchdog(void);
-/* ... and of the 4-bit kernel over pairs of SMs (prompt-sized M) */
 unsigned zl_w4_tc2_watchdog(void);
+/* tests: the two codes, in this order (host memory; NULL: none could be had) */
+void* zl_wait_words(void);
 /* debug / tests: at least `splits` pieces per weight-row tile in the tcgen05 kernel's stream-k schedule (0 = automatic; also
  * ZL_TC_SPLITS). */
 int zl_w4_tc_set_splits(int splits);

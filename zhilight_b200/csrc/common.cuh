@@ -34,12 +34,30 @@
 
 #define ZL_CHECK_LAUNCH() ZL_CHECK_CUDA(cudaGetLastError())
 
+// a bounded wait inside a kernel has given up since the last check: its launch left its output incomplete
+#define ZL_CHECK_WAITS()                                                               \
+    do {                                                                               \
+        if (zl_check_waits() != ZL_OK) return ZL_ERR_CUDA;                             \
+    } while (0)
+
+// the end of a step: results may be read, and are known to be complete
+#define ZL_SYNC(stream)                                                                \
+    do {                                                                               \
+        ZL_CHECK_CUDA(cudaStreamSynchronize(stream));                                  \
+        ZL_CHECK_WAITS();                                                              \
+    } while (0)
+
 extern "C" void zl_set_last_error(const char* file, int line, const char* msg);
 extern "C" void zl_count_launch(void);
 
 namespace zl {
 
 constexpr int kWarp = 32;
+
+// The words that kernels write when a bounded wait gives up, one for each kernel that returns then instead of trapping: pinned host memory,
+// so that a host thread which has synchronised anyway reads them without a copy.  nullptr: no memory.
+enum { kWaitGemmTc = 0, kWaitW4Pairs = 1, kWaitWords = 2 };
+unsigned* wait_words();   // misc.cu
 
 __host__ __device__ inline int cdiv(int a, int b) { return (a + b - 1) / b; }
 

@@ -294,7 +294,7 @@ int alloc_runtime(zl_dekalorn* m) {
     RCHECK(dmalloc(&m->attn_ws, m->attn_ws_bytes));
     RCHECK(dmalloc(&m->argmax_ws, zl_argmax_workspace_bytes(T)));
     ZL_CHECK_CUDA(cudaMallocHost((void**)&m->h_stage, sizeof(int32_t) * 7 * (size_t)T));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -645,7 +645,7 @@ extern "C" int zl_dekalorn_step(zl_dekalorn_t* m, const int32_t* tokens_host, co
     if (n_want && next_host) ZL_CHECK_CUDA(cudaMemcpyAsync(hs + 4 * T, m->d_next, (size_t)n_want * 4, cudaMemcpyDeviceToHost, st));
     if (n_want && logits_host)
         ZL_CHECK_CUDA(cudaMemcpyAsync(logits_host, m->logits, (size_t)n_want * c.vocab * 4, cudaMemcpyDeviceToHost, st));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(st));
+    ZL_SYNC(st);
     if (n_want && next_host)
         for (int i = 0; i < n_want; ++i) next_host[i] = hs[4 * T + i];
     if (max_len > m->cur_max_len) m->cur_max_len = max_len;
@@ -655,7 +655,7 @@ extern "C" int zl_dekalorn_step(zl_dekalorn_t* m, const int32_t* tokens_host, co
 extern "C" int zl_dekalorn_set_state(zl_dekalorn_t* m, const int32_t* tokens_host, const int32_t* positions_host, int B) {
     ZL_CHECK_ARG(m && tokens_host && positions_host && B > 0 && B <= m->cfg.max_batch);
     if (!m->finalized) return fail(__LINE__, "model not finalized");
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));   // the staging buffer is free again
+    ZL_SYNC(m->stream);   // the staging buffer is free again
     int32_t* hs = m->h_stage;
     const int T = m->tcap;
     int mx = 0;
@@ -674,7 +674,7 @@ extern "C" int zl_dekalorn_set_state(zl_dekalorn_t* m, const int32_t* tokens_hos
     k_iota_i32<<<cdiv(B, 256), 256, 0, m->stream>>>(m->d_slots, m->d_want, B);
     k_iota_i32<<<cdiv(B, 256), 256, 0, m->stream>>>(m->d_run0, m->d_want, B);
     ZL_CHECK_LAUNCH();
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -690,7 +690,7 @@ extern "C" int zl_dekalorn_step_device(zl_dekalorn_t* m, int B) {
 
 extern "C" int zl_dekalorn_sync(zl_dekalorn_t* m) {
     ZL_CHECK_ARG(m);
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -711,7 +711,7 @@ extern "C" int zl_dekalorn_read_layers(zl_dekalorn_t* m, float* out_host, int T)
     const size_t row = (size_t)m->cfg.width * 4;
     ZL_CHECK_CUDA(cudaMemcpy2DAsync(out_host, (size_t)T * row, m->layer_dump, (size_t)m->tcap * row, (size_t)T * row,
                                     m->runs.size(), cudaMemcpyDeviceToHost, m->stream));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -723,7 +723,7 @@ extern "C" int zl_dekalorn_read_cache(zl_dekalorn_t* m, int run, int slot, int n
     const KLayer& L = m->layers[U.layer];
     const auto& lc = L.c;
     const bool latent = lc.type == ZL_DEKALORN_LATENT;
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     const size_t kw = (size_t)lc.kv_heads * lc.dim * (lc.type == ZL_DEKALORN_DIFF ? 2 : 1), vw = (size_t)lc.kv_heads * lc.vdim;
     // per output: the cache, elements per cached row, first element, elements wanted
     const SlotCache* caches[2] = {&U.a, latent ? &U.a : &U.b};

@@ -124,7 +124,7 @@ int finalize_layer(zl_dekipel* m, int l) {
                                                                          static_cast<__nv_bfloat16*>(L.uk_t), H, lc.dim, R);
         }
         ZL_CHECK_LAUNCH();
-        ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+        ZL_SYNC(m->stream);
         staged_drop(m->staged, p + "mix.uk");
         m->weight_bytes += (double)n * m->esz;
     }
@@ -200,7 +200,7 @@ int alloc_runtime(zl_dekipel* m) {
     RCHECK(dmalloc(&m->attn_ws, m->attn_ws_bytes));
     RCHECK(dmalloc(&m->argmax_ws, zl_argmax_workspace_bytes(T)));
     ZL_CHECK_CUDA(cudaMallocHost((void**)&m->h_stage, sizeof(int32_t) * 5 * (size_t)T));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -477,7 +477,7 @@ extern "C" int zl_dekipel_step(zl_dekipel_t* m, const int32_t* tokens_host, cons
     if (n_want && next_host) ZL_CHECK_CUDA(cudaMemcpyAsync(hs + 4 * T, m->d_next, (size_t)n_want * 4, cudaMemcpyDeviceToHost, st));
     if (n_want && logits_host)
         ZL_CHECK_CUDA(cudaMemcpyAsync(logits_host, m->logits, (size_t)n_want * c.vocab * 4, cudaMemcpyDeviceToHost, st));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(st));
+    ZL_SYNC(st);
     if (n_want && next_host)
         for (int i = 0; i < n_want; ++i) next_host[i] = hs[4 * T + i];
     if (max_len > m->cur_max_len) m->cur_max_len = max_len;
@@ -487,7 +487,7 @@ extern "C" int zl_dekipel_step(zl_dekipel_t* m, const int32_t* tokens_host, cons
 extern "C" int zl_dekipel_set_state(zl_dekipel_t* m, const int32_t* tokens_host, const int32_t* positions_host, int B) {
     ZL_CHECK_ARG(m && tokens_host && positions_host && B > 0 && B <= m->cfg.max_batch);
     if (!m->finalized) return fail(__LINE__, "model not finalized");
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));   // the staging buffer is free again
+    ZL_SYNC(m->stream);   // the staging buffer is free again
     int32_t* hs = m->h_stage;
     int mx = 0;
     for (int i = 0; i < B; ++i) {
@@ -502,7 +502,7 @@ extern "C" int zl_dekipel_set_state(zl_dekipel_t* m, const int32_t* tokens_host,
     ZL_CHECK_CUDA(cudaMemcpyAsync(m->d_pos, hs + B, (size_t)B * 4, cudaMemcpyHostToDevice, m->stream));
     k_iota_i32<<<cdiv(B, 256), 256, 0, m->stream>>>(m->d_slots, m->d_want, B);
     ZL_CHECK_LAUNCH();
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -518,7 +518,7 @@ extern "C" int zl_dekipel_step_device(zl_dekipel_t* m, int B) {
 
 extern "C" int zl_dekipel_sync(zl_dekipel_t* m) {
     ZL_CHECK_ARG(m);
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -539,7 +539,7 @@ extern "C" int zl_dekipel_read_layers(zl_dekipel_t* m, float* out_host, int T) {
     const size_t row = (size_t)m->cfg.width * 4;
     ZL_CHECK_CUDA(cudaMemcpy2DAsync(out_host, (size_t)T * row, m->layer_dump, (size_t)m->tcap * row, (size_t)T * row,
                                     m->cfg.num_layers, cudaMemcpyDeviceToHost, m->stream));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 

@@ -238,6 +238,7 @@ extern "C" int zl_dense_gemm_skinny_act(const void* x, int ldx, const void* w, c
 extern "C" int zl_dense_gemm_skinny_mul(const void* x, int ldx, const void* w, const void* bias, void* y, int M, int N,
                                         int K, int dtype, int out_dtype, int act, const float* mul_all, int ld_mul, int pdl,
                                         zl_stream_t stream) {
+    ZL_CHECK_WAITS();
     ZL_CHECK_ARG(x && w && y && M > 0 && N > 0 && K > 0 && act >= 0 && act <= 3);
     ZL_CHECK_ARG(act != 3 || (mul_all && ld_mul >= N));
     ZL_CHECK_ARG(dtype == ZL_F16 || dtype == ZL_BF16);

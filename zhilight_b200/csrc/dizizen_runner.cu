@@ -227,7 +227,7 @@ int finalize_layer(zl_dizizen* m, int l) {
     RCHECK(take_weight(m, mx + "o", D, H * vd, &L.o));
     RCHECK(take_f32(m, mx + "o.b", 1, D, &L.o_b));
     RCHECK(bias_copy_act(m, L.o_b, D, &L.o_b_act));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     RCHECK(bias_copy_act(m, L.b_in, L.n_in, &L.b_in_act));
     if (ff) RCHECK(finalize_ff(m, l));
     L.qk_rot = lc.rot_dims > 0 ? rot_index(m, lc.rot_base, lc.rot_dims) : -1;
@@ -307,7 +307,7 @@ int alloc_runtime(zl_dizizen* m) {
     RCHECK(dmalloc(&m->attn_ws, m->attn_ws_bytes));
     RCHECK(dmalloc(&m->argmax_ws, zl_argmax_workspace_bytes(T)));
     ZL_CHECK_CUDA(cudaMallocHost((void**)&m->h_stage, sizeof(int32_t) * 7 * (size_t)T));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -659,7 +659,7 @@ extern "C" int zl_dizizen_step(zl_dizizen_t* m, const int32_t* tokens_host, cons
     if (n_want && next_host) ZL_CHECK_CUDA(cudaMemcpyAsync(hs + 4 * T, m->d_next, (size_t)n_want * 4, cudaMemcpyDeviceToHost, st));
     if (n_want && logits_host)
         ZL_CHECK_CUDA(cudaMemcpyAsync(logits_host, m->logits, (size_t)n_want * c.vocab * 4, cudaMemcpyDeviceToHost, st));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(st));
+    ZL_SYNC(st);
     if (n_want && next_host)
         for (int i = 0; i < n_want; ++i) next_host[i] = hs[4 * T + i];
     if (max_len > m->cur_max_len) m->cur_max_len = max_len;
@@ -669,7 +669,7 @@ extern "C" int zl_dizizen_step(zl_dizizen_t* m, const int32_t* tokens_host, cons
 extern "C" int zl_dizizen_set_state(zl_dizizen_t* m, const int32_t* tokens_host, const int32_t* positions_host, int B) {
     ZL_CHECK_ARG(m && tokens_host && positions_host && B > 0 && B <= m->cfg.max_batch);
     if (!m->finalized) return fail(__LINE__, "model not finalized");
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));   // the staging buffer is free again
+    ZL_SYNC(m->stream);   // the staging buffer is free again
     int32_t* hs = m->h_stage;
     const int T = m->tcap;
     int mx = 0;
@@ -688,7 +688,7 @@ extern "C" int zl_dizizen_set_state(zl_dizizen_t* m, const int32_t* tokens_host,
     k_iota_i32<<<cdiv(B, 256), 256, 0, m->stream>>>(m->d_slots, m->d_want, B);
     k_iota_i32<<<cdiv(B, 256), 256, 0, m->stream>>>(m->d_run0, m->d_want, B);
     ZL_CHECK_LAUNCH();
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -704,7 +704,7 @@ extern "C" int zl_dizizen_step_device(zl_dizizen_t* m, int B) {
 
 extern "C" int zl_dizizen_sync(zl_dizizen_t* m) {
     ZL_CHECK_ARG(m);
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -725,7 +725,7 @@ extern "C" int zl_dizizen_read_layers(zl_dizizen_t* m, float* out_host, int T) {
     const size_t row = (size_t)m->cfg.width * 4;
     ZL_CHECK_CUDA(cudaMemcpy2DAsync(out_host, (size_t)T * row, m->layer_dump, (size_t)m->tcap * row, (size_t)T * row,
                                     m->cfg.num_layers, cudaMemcpyDeviceToHost, m->stream));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -735,7 +735,7 @@ extern "C" int zl_dizizen_read_cache(zl_dizizen_t* m, int layer, int slot, int n
     if (!m->finalized) return fail(__LINE__, "model not finalized");
     const DLayer& L = m->layers[layer];
     ZL_CHECK_ARG(L.c.kv_from < 0);
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     const SlotCache* cs[2] = {&L.kcache, &L.vcache};
     float* outs[2] = {keys_host, values_host};
     const size_t ns[2] = {(size_t)n_rows * L.c.kv_heads * L.c.dim, (size_t)n_rows * L.c.kv_heads * L.c.vdim};

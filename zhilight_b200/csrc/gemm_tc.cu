@@ -50,10 +50,8 @@ struct alignas(64) GemmTcP {
     const float* sx;            // 8-bit: scales of the rows of x (int8) or one (fp8)
     const void* sw;             // 8-bit: scales of the rows of w, or one
     int sw_mode;                // 0: per row in y's type, 1 / 2: per row fp32, 3: one fp32
+    unsigned* err;              // wait_words()[kWaitGemmTc]
 };
-
-// code of the last wait that gave up (0: none)
-__device__ unsigned g_gemm_tc_err;
 
 struct GtTile {
     int b, n0, t0, ntok, M, first;
@@ -250,7 +248,7 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
         for (int i = pair; ok && gt_tile<GROUPED>(p, s_cum, i, hint, t); i += pairs) {
             const int tb = t.t0 + (int)rank * (t.ntok >> 1);
             for (int k = 0; k < ks; ++k) {
-                if (!(ok = tc2_wait(&empty[st], ph ^ 1u, s_abort, &g_gemm_tc_err, 0x2100 + st))) break;
+                if (!(ok = tc2_wait(&empty[st], ph ^ 1u, s_abort, p.err, 0x2100 + st))) break;
                 if (tc_elect_one()) {
                     if (KIND == kGt16 || ahead <= 0) weights(st, k);
                     if (!GROUPED) {
@@ -275,12 +273,12 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
         GtTile t;
         bool ok = true;
         for (int i = pair; ok && gt_tile<GROUPED>(p, s_cum, i, hint, t); i += pairs) {
-            if (!(ok = tc2_wait(&acc_empty[acc], acc_ph ^ 1u, s_abort, &g_gemm_tc_err, 0x2300 + acc))) break;
+            if (!(ok = tc2_wait(&acc_empty[acc], acc_ph ^ 1u, s_abort, p.err, 0x2300 + acc))) break;
             tc_fence_after();
             const uint32_t d = tmem + (uint32_t)(acc * 256);
             const uint32_t idesc = KIND == kGt16 ? tc2_idesc(std::is_same<T, __nv_bfloat16>::value, t.ntok) : tc2_idesc8(KIND == kGtFp8, t.ntok);
             for (int k = 0; k < ks; ++k) {
-                if (!(ok = tc2_wait(&full[st], ph, s_abort, &g_gemm_tc_err, 0x2400 + st))) break;
+                if (!(ok = tc2_wait(&full[st], ph, s_abort, p.err, 0x2400 + st))) break;
                 tc_fence_after();
                 if (tc_elect_one()) {
 #pragma unroll
@@ -317,7 +315,7 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
         bool ok = true;
         for (int i = pair; ok && gt_tile<GROUPED>(p, s_cum, i, hint, t); i += pairs)
             for (int k = 0; k < ks; ++k) {
-                if (!(ok = tc2_wait(&rows_full[st], ph, s_abort, &g_gemm_tc_err, 0x2500 + st))) break;
+                if (!(ok = tc2_wait(&rows_full[st], ph, s_abort, p.err, 0x2500 + st))) break;
                 if (lane == 0) {
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     mbar_arrive_at(cluster_map(smem_u32(&full[st]), 0));
@@ -344,7 +342,7 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
                 row[u] = static_cast<const T*>(p.g.x) + (size_t)(p.g.x_rows ? p.g.x_rows[e] : e) * p.g.ldx + c * 8;
             }
             for (int k = 0; k < ks; ++k) {
-                if (!(ok = tc2_wait(&empty[st], ph ^ 1u, s_abort, &g_gemm_tc_err, 0x2200 + st))) break;
+                if (!(ok = tc2_wait(&empty[st], ph ^ 1u, s_abort, p.err, 0x2200 + st))) break;
 #pragma unroll
                 for (int u2 = 0; u2 < sub; ++u2) {
                     const int k0 = (k * sub + u2) * 64;
@@ -373,7 +371,7 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
         uint32_t acc_ph = 0;
         GtTile t;
         for (int i = pair; gt_tile<GROUPED>(p, s_cum, i, hint, t); i += pairs) {
-            if (!tc2_wait(&acc_full[acc], acc_ph, s_abort, &g_gemm_tc_err, 0x2800 + acc)) break;
+            if (!tc2_wait(&acc_full[acc], acc_ph, s_abort, p.err, 0x2800 + acc)) break;
             tc_fence_after();
             const int n = t.n0 + (int)rank * 128 + q * 32 + lane;
             float bias = 0.f, s_w = 0.f;
@@ -482,6 +480,9 @@ static int gt_plan(GemmTcP& q, CUtensorMapDataType dt, int batch, int out_bytes)
     const GemmP& p = q.g;
     const bool grouped = p.grp_off != nullptr;
     int pairs = device_sm_count() / 2;
+    unsigned* words = wait_words();
+    if (!words) return 0;
+    q.err = words + kWaitGemmTc;
     q.groups = batch;
     q.row_tiles = cdiv(p.N, kTc2Rows);
     q.tok_tiles = 0;
@@ -542,7 +543,7 @@ ZL_W8_TC(__nv_bfloat16, true)
 }  // namespace zl
 
 extern "C" unsigned zl_gemm_tc_watchdog(void) {
-    unsigned v = 0;
-    cudaMemcpyFromSymbol(&v, zl::g_gemm_tc_err, sizeof v);
-    return v;
+    cudaDeviceSynchronize();
+    const unsigned* words = zl::wait_words();
+    return words ? words[zl::kWaitGemmTc] : 0u;
 }

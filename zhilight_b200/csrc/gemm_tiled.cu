@@ -484,6 +484,7 @@ static int grouped_small_max() {
 }
 
 static int gemm_dispatch(GemmP p, int batch, int in_dtype, int out_dtype, int epilogue, int pdl, cudaStream_t stream) {
+    ZL_CHECK_WAITS();
     const int M = p.M, N = p.N, K = p.K;
     const bool grouped = p.grp_off != nullptr, pairs = epi_pairs(epilogue);
     ZL_CHECK_ARG(p.x && p.w && p.y && M > 0 && N > 0 && K > 0 && batch > 0 && batch <= 65535);

@@ -125,7 +125,7 @@ int take_norm(zl_kodupel* m, const std::string& name, int n, float** out) {
     RCHECK(take_f32(m, name, 1, n, out));
     k_add_one<<<cdiv(n, 256), 256, 0, m->stream>>>(*out, n);
     ZL_CHECK_LAUNCH();
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -134,7 +134,7 @@ int put_bias(zl_kodupel* m, const std::string& name, int n, float* dst, int off)
     const Staged* s = need(m, name, 1, n);
     if (!s) return ZL_ERR_STATE;
     RCHECK(convert_to<float>(m, s, dst + off, (size_t)n));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     staged_drop(m->staged, name);
     return ZL_OK;
 }
@@ -145,7 +145,7 @@ int bias_act_copy(zl_kodupel* m, const float* src, int n, void** out) {
     RCHECK(dmalloc(out, (size_t)n * 2));
     k_convert<float, __nv_bfloat16><<<cdiv(n, 256), 256, 0, m->stream>>>(src, static_cast<__nv_bfloat16*>(*out), (size_t)n);
     ZL_CHECK_LAUNCH();
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -181,7 +181,7 @@ int finalize_experts(zl_kodupel* m, int l) {
                                                                  (__nv_bfloat16*)L.w_gu + off, F, D);
         }
         ZL_CHECK_LAUNCH();
-        ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+        ZL_SYNC(m->stream);
         staged_drop(m->staged, pe + "gate");
         staged_drop(m->staged, pe + "up");
         m->weight_bytes += 2.0 * n * m->esz;
@@ -252,7 +252,7 @@ int finalize_layer(zl_kodupel* m, int l) {
         RCHECK(take_f32(m, mx + "norm", 1, hd, &L.out_norm));
         RCHECK(take_weight(m, mx + "o", D, hd, &L.o));
     }
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     RCHECK(bias_act_copy(m, L.b_in, L.n_in, &L.b_in_act));
     if (lc.experts > 0) {
         RCHECK(take_norm(m, p + "norm2", D, &L.norm2));
@@ -331,7 +331,7 @@ int alloc_runtime(zl_kodupel* m) {
     RCHECK(dmalloc(&m->delta_ws, m->delta_ws_bytes));
     RCHECK(dmalloc(&m->argmax_ws, zl_argmax_workspace_bytes(T)));
     ZL_CHECK_CUDA(cudaMallocHost((void**)&m->h_stage, sizeof(int32_t) * 7 * (size_t)T));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -642,7 +642,7 @@ extern "C" int zl_kodupel_step(zl_kodupel_t* m, const int32_t* tokens_host, cons
     if (n_want && next_host) ZL_CHECK_CUDA(cudaMemcpyAsync(hs + 4 * T, m->d_next, (size_t)n_want * 4, cudaMemcpyDeviceToHost, st));
     if (n_want && logits_host)
         ZL_CHECK_CUDA(cudaMemcpyAsync(logits_host, m->logits, (size_t)n_want * c.vocab * 4, cudaMemcpyDeviceToHost, st));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(st));
+    ZL_SYNC(st);
     if (n_want && next_host)
         for (int i = 0; i < n_want; ++i) next_host[i] = hs[4 * T + i];
     if (max_len > m->cur_max_len) m->cur_max_len = max_len;
@@ -652,7 +652,7 @@ extern "C" int zl_kodupel_step(zl_kodupel_t* m, const int32_t* tokens_host, cons
 extern "C" int zl_kodupel_set_state(zl_kodupel_t* m, const int32_t* tokens_host, const int32_t* positions_host, int B) {
     ZL_CHECK_ARG(m && tokens_host && positions_host && B > 0 && B <= m->cfg.max_batch);
     if (!m->finalized) return fail(__LINE__, "model not finalized");
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));   // the staging buffer is free again
+    ZL_SYNC(m->stream);   // the staging buffer is free again
     int32_t* hs = m->h_stage;
     const int T = m->tcap;
     int mx = 0;
@@ -671,7 +671,7 @@ extern "C" int zl_kodupel_set_state(zl_kodupel_t* m, const int32_t* tokens_host,
     k_iota_i32<<<cdiv(B, 256), 256, 0, m->stream>>>(m->d_slots, m->d_want, B);
     k_iota_i32<<<cdiv(B, 256), 256, 0, m->stream>>>(m->d_run0, m->d_want, B);
     ZL_CHECK_LAUNCH();
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -687,7 +687,7 @@ extern "C" int zl_kodupel_step_device(zl_kodupel_t* m, int B) {
 
 extern "C" int zl_kodupel_sync(zl_kodupel_t* m) {
     ZL_CHECK_ARG(m);
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -708,7 +708,7 @@ extern "C" int zl_kodupel_read_layers(zl_kodupel_t* m, float* out_host, int T) {
     const size_t row = (size_t)m->cfg.width * 4;
     ZL_CHECK_CUDA(cudaMemcpy2DAsync(out_host, (size_t)T * row, m->layer_dump, (size_t)m->tcap * row, (size_t)T * row,
                                     m->cfg.num_layers, cudaMemcpyDeviceToHost, m->stream));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -717,7 +717,7 @@ extern "C" int zl_kodupel_read_state(zl_kodupel_t* m, int layer, int slot, float
     if (!m->finalized) return fail(__LINE__, "model not finalized");
     const KLayer& L = m->layers[layer];
     ZL_CHECK_ARG(L.c.type == ZL_MIXER_GENERAL_DELTA);
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     ZL_CHECK_CUDA(cudaMemcpy(out_host, (const char*)L.state.buf + (size_t)slot * L.state.slot_bytes, L.state.slot_bytes,
                              cudaMemcpyDeviceToHost));
     return ZL_OK;

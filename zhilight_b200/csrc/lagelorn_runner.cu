@@ -138,7 +138,7 @@ int put_f32(zl_lagelorn* m, const std::string& name, int n, float* dst, size_t o
     const Staged* s = need(m, name, 1, n);
     if (!s) return ZL_ERR_STATE;
     RCHECK(convert_to<float>(m, s, dst + off, (size_t)n));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     staged_drop(m->staged, name);
     return ZL_OK;
 }
@@ -147,7 +147,7 @@ int put_f32_2d(zl_lagelorn* m, const std::string& name, int rows, int cols, floa
     const Staged* s = need(m, name, rows, cols);
     if (!s) return ZL_ERR_STATE;
     RCHECK(convert_to<float>(m, s, dst + off, (size_t)rows * cols));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     staged_drop(m->staged, name);
     return ZL_OK;
 }
@@ -158,7 +158,7 @@ int bias_act_copy(zl_lagelorn* m, const float* src, int n, void** out) {
     RCHECK(dmalloc(out, (size_t)n * 2));
     k_convert<float, __nv_bfloat16><<<cdiv(n, 256), 256, 0, m->stream>>>(src, static_cast<__nv_bfloat16*>(*out), (size_t)n);
     ZL_CHECK_LAUNCH();
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -186,7 +186,7 @@ int finalize_ff(zl_lagelorn* m, int l) {
             k_interleave_rows2<<<blocks, 256, 0, m->stream>>>((const float*)g->ptr, (const float*)u->ptr, (__nv_bfloat16*)L.w_gu, F, D);
     }
     ZL_CHECK_LAUNCH();
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     staged_drop(m->staged, p + "gate");
     staged_drop(m->staged, p + "up");
     m->weight_bytes += 2.0 * n * m->esz;
@@ -201,7 +201,7 @@ int finalize_ff(zl_lagelorn* m, int l) {
     else
         k_interleave_rows2<<<cdiv(F, 256), 256, 0, m->stream>>>((const float*)gb->ptr, (const float*)ub->ptr, L.b_gu, F, 1);
     ZL_CHECK_LAUNCH();
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     staged_drop(m->staged, p + "gate.b");
     staged_drop(m->staged, p + "up.b");
     RCHECK(take_weight(m, p + "down", D, F, &L.w_down));
@@ -292,7 +292,7 @@ int finalize_layer(zl_lagelorn* m, int l) {
     RCHECK(take_weight(m, p + "side.gate", c.side_dim, D, &L.s_gate));
     RCHECK(take_weight(m, p + "side.proj", D, c.side_dim, &L.s_proj));
     RCHECK(take_f32(m, p + "side.norm", 1, D, &L.s_norm));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     L.ready = true;
     return ZL_OK;
 }
@@ -362,7 +362,7 @@ int alloc_runtime(zl_lagelorn* m) {
     RCHECK(dmalloc(&m->delta_ws, m->delta_ws_bytes));
     RCHECK(dmalloc(&m->argmax_ws, zl_argmax_workspace_bytes(T)));
     ZL_CHECK_CUDA(cudaMallocHost((void**)&m->h_stage, sizeof(int32_t) * 7 * (size_t)T));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -722,7 +722,7 @@ extern "C" int zl_lagelorn_step(zl_lagelorn_t* m, const int32_t* tokens_host, co
     if (n_want && next_host) ZL_CHECK_CUDA(cudaMemcpyAsync(hs + 4 * T, m->d_next, (size_t)n_want * 4, cudaMemcpyDeviceToHost, st));
     if (n_want && logits_host)
         ZL_CHECK_CUDA(cudaMemcpyAsync(logits_host, m->logits, (size_t)n_want * c.vocab * 4, cudaMemcpyDeviceToHost, st));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(st));
+    ZL_SYNC(st);
     if (n_want && next_host)
         for (int i = 0; i < n_want; ++i) next_host[i] = hs[4 * T + i];
     if (max_len > m->cur_max_len) m->cur_max_len = max_len;
@@ -732,7 +732,7 @@ extern "C" int zl_lagelorn_step(zl_lagelorn_t* m, const int32_t* tokens_host, co
 extern "C" int zl_lagelorn_set_state(zl_lagelorn_t* m, const int32_t* tokens_host, const int32_t* positions_host, int B) {
     ZL_CHECK_ARG(m && tokens_host && positions_host && B > 0 && B <= m->cfg.max_batch);
     if (!m->finalized) return fail(__LINE__, "model not finalized");
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));   // the staging buffer is free again
+    ZL_SYNC(m->stream);   // the staging buffer is free again
     int32_t* hs = m->h_stage;
     const int T = m->tcap;
     int mx = 0;
@@ -751,7 +751,7 @@ extern "C" int zl_lagelorn_set_state(zl_lagelorn_t* m, const int32_t* tokens_hos
     k_iota_i32<<<cdiv(B, 256), 256, 0, m->stream>>>(m->d_slots, m->d_want, B);
     k_iota_i32<<<cdiv(B, 256), 256, 0, m->stream>>>(m->d_run0, m->d_want, B);
     ZL_CHECK_LAUNCH();
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -767,7 +767,7 @@ extern "C" int zl_lagelorn_step_device(zl_lagelorn_t* m, int B) {
 
 extern "C" int zl_lagelorn_sync(zl_lagelorn_t* m) {
     ZL_CHECK_ARG(m);
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -788,7 +788,7 @@ extern "C" int zl_lagelorn_read_layers(zl_lagelorn_t* m, float* out_host, int T)
     const size_t row = (size_t)m->cfg.width * 4;
     ZL_CHECK_CUDA(cudaMemcpy2DAsync(out_host, (size_t)T * row, m->layer_dump, (size_t)m->tcap * row, (size_t)T * row,
                                     m->cfg.num_layers, cudaMemcpyDeviceToHost, m->stream));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -797,7 +797,7 @@ extern "C" int zl_lagelorn_read_state(zl_lagelorn_t* m, int layer, int slot, flo
     if (!m->finalized) return fail(__LINE__, "model not finalized");
     const GLayer& L = m->layers[layer];
     const SlotCache& sc = L.c.type == ZL_LAYER_DELTA ? L.state : L.r_state;
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     ZL_CHECK_CUDA(cudaMemcpy(out_host, (const char*)sc.buf + (size_t)slot * sc.slot_bytes, sc.slot_bytes, cudaMemcpyDeviceToHost));
     return ZL_OK;
 }

@@ -206,7 +206,7 @@ int check_g_idx_sequential(zl_llama* m, const std::string& prefix, int K) {
         return fail_state(__LINE__, "ill-shaped g_idx for " + prefix + " (expected K int32)");
     std::vector<int32_t> host(K);
     ZL_CHECK_CUDA(cudaMemcpyAsync(host.data(), gi->ptr, (size_t)K * 4, cudaMemcpyDeviceToHost, m->stream));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     for (int k = 0; k < K; ++k)
         if (host[k] != k / m->cfg.group_size)
             return fail_state(__LINE__, "act-order (desc_act) GPTQ checkpoint: " + prefix +
@@ -252,7 +252,7 @@ int to_k_major(zl_llama* m, const std::string& prefix, int K, int N, uint32_t* q
     RCHECK(zl_transpose_2d(w_kn, qw_km + (size_t)n_off * (K / 8), K / 8, N, 4, st));
     RCHECK(zl_transpose_2d(z8, qz_km + (size_t)n_off * G, G, N, 1, st));
     RCHECK(zl_transpose_2d(sc->ptr, sc_km + (size_t)n_off * G, G, N, 2, st));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(st));
+    ZL_SYNC(st);
     (void)n_total;
     return ZL_OK;
 }
@@ -319,12 +319,12 @@ int build_w4(zl_llama* m, const std::vector<std::string>& prefixes, const std::v
             void* pb = nullptr;
             RCHECK(dmalloc(&pb, (size_t)N * 2));
             RCHECK(zl_gather_rows_16(out->bias, row_map, pb, N, m->stream));
-            ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+            ZL_SYNC(m->stream);
             cudaFree(out->bias);
             out->bias = pb;
         }
     }
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     for (auto& p : prefixes) {
         drop(m, p + ".qweight");
         drop(m, p + ".qzeros");
@@ -368,7 +368,7 @@ int build_dense(zl_llama* m, const std::vector<std::string>& prefixes, const std
             off += ns[i];
         }
     }
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     for (auto& p : prefixes) {
         drop(m, p + ".weight");
         drop(m, p + ".bias");
@@ -393,7 +393,7 @@ int dense_to_int8(zl_llama* m, DenseLin* d) {
     else
         k_f32_to_t<__nv_bfloat16><<<cdiv(d->N, 256), 256, 0, m->stream>>>(sf, static_cast<__nv_bfloat16*>(d->w_scale), d->N);
     ZL_CHECK_LAUNCH();
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     cudaFree(sf);
     cudaFree(d->w);
     d->w = nullptr;
@@ -438,7 +438,7 @@ int build_fp8(zl_llama* m, const std::vector<std::string>& prefixes, const std::
             off += ns[i];
         }
     }
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     for (auto& p : prefixes) {
         drop(m, p + ".weight");
         drop(m, p + ".weight_scale");
@@ -565,7 +565,7 @@ int alloc_runtime(zl_llama* m) {
     ZL_CHECK_CUDA(cudaMallocHost((void**)&m->h_ring, sizeof(int32_t) * zl_llama::kStageSlots * 2 * B));
     for (int i = 0; i < zl_llama::kStageSlots; ++i)
         ZL_CHECK_CUDA(cudaEventCreateWithFlags(&m->ring_ev[i], cudaEventDisableTiming));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -1273,7 +1273,7 @@ extern "C" int zl_llama_decode(zl_llama_t* m, const int32_t* tokens_host, const 
     if (logits_host)   // (B, vocab/tp) of this rank's shard
         ZL_CHECK_CUDA(cudaMemcpyAsync(logits_host, m->logits, (size_t)B * m->vshard * 4, cudaMemcpyDeviceToHost,
                                       m->stream));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     for (int i = 0; i < B; ++i) next_tokens_host[i] = m->h_stage[3 * B + i];
     return ZL_OK;
 }
@@ -1282,7 +1282,7 @@ extern "C" int zl_llama_get_state(zl_llama_t* m, int32_t* tokens_host, int32_t* 
     ZL_CHECK_ARG(m && tokens_host && positions_host && B > 0 && B <= m->cfg.max_batch);
     ZL_CHECK_CUDA(cudaMemcpyAsync(m->h_stage, m->d_tokens, B * 4, cudaMemcpyDeviceToHost, m->stream));
     ZL_CHECK_CUDA(cudaMemcpyAsync(m->h_stage + B, m->d_pos, B * 4, cudaMemcpyDeviceToHost, m->stream));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     for (int i = 0; i < B; ++i) {
         tokens_host[i] = m->h_stage[i];
         positions_host[i] = m->h_stage[B + i];
@@ -1346,6 +1346,7 @@ extern "C" int zl_llama_bench_gemms(zl_llama_t* m, int B, int iters, float* ms, 
     }
     ZL_CHECK_CUDA(cudaEventRecord(e1, st));
     ZL_CHECK_CUDA(cudaEventSynchronize(e1));
+    ZL_CHECK_WAITS();
     ZL_CHECK_CUDA(cudaEventElapsedTime(ms, e0, e1));
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -1356,7 +1357,7 @@ extern "C" int zl_llama_bench_gemms(zl_llama_t* m, int B, int iters, float* ms, 
 
 extern "C" int zl_llama_sync(zl_llama_t* m) {
     ZL_CHECK_ARG(m);
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -1376,7 +1377,7 @@ extern "C" int zl_llama_prefill(zl_llama_t* m, int task, const int32_t* tokens_h
     int32_t* h_tok = m->h_stage + 4 * m->cfg.max_batch + 4;   // pinned staging for one chunk of token ids
     for (int c0 = 0; c0 < n; c0 += chunk) {
         const int cn = (n - c0) < chunk ? (n - c0) : chunk;
-        if (c0 > 0) ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));   // staging buffer reuse
+        if (c0 > 0) ZL_SYNC(m->stream);   // staging buffer reuse
         for (int i = 0; i < cn; ++i) {
             ZL_CHECK_ARG(tokens_host[c0 + i] >= 0 && tokens_host[c0 + i] < m->cfg.vocab_size);
             h_tok[i] = tokens_host[c0 + i];
@@ -1388,7 +1389,7 @@ extern "C" int zl_llama_prefill(zl_llama_t* m, int task, const int32_t* tokens_h
     ZL_CHECK_CUDA(cudaMemcpyAsync(m->h_stage + 3 * m->cfg.max_batch, m->d_next, 4, cudaMemcpyDeviceToHost, m->stream));
     if (logits_host)
         ZL_CHECK_CUDA(cudaMemcpyAsync(logits_host, m->logits, (size_t)m->vshard * 4, cudaMemcpyDeviceToHost, m->stream));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     *next_token_host = m->h_stage[3 * m->cfg.max_batch];
     if (pos0 + n > m->cur_max_len) m->cur_max_len = pos0 + n;
     return ZL_OK;

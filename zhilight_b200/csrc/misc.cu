@@ -6,6 +6,7 @@
 #include <atomic>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 
 static thread_local char g_last_error[512] = "";
 static std::atomic<long long> g_launches{0};
@@ -16,6 +17,41 @@ extern "C" void zl_set_last_error(const char* file, int line, const char* msg) {
 }
 extern "C" const char* zl_last_error(void) { return g_last_error; }
 extern "C" int zl_version(void) { return 100; }
+
+// One allocation for the process, visible to every device; it may first be needed inside a stream capture, where an allocation has to
+// be declared as no part of it.
+unsigned* zl::wait_words() {
+    static std::mutex mu;
+    static unsigned* words = nullptr;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!words) {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        void* p = nullptr;
+        if (cudaHostAlloc(&p, zl::kWaitWords * sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+            memset(p, 0, zl::kWaitWords * sizeof(unsigned));
+            words = static_cast<unsigned*>(p);
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    return words;
+}
+extern "C" void* zl_wait_words(void) { return zl::wait_words(); }
+extern "C" int zl_check_waits(void) {
+    static const char* const names[zl::kWaitWords] = {"general tensor-core GEMM", "4-bit GEMM over pairs of SMs"};
+    unsigned* words = zl::wait_words();
+    if (!words) return ZL_OK;   // no kernel that would write them has been launched
+    for (int i = 0; i < zl::kWaitWords; ++i) {
+        if (__atomic_load_n(&words[i], __ATOMIC_ACQUIRE) == 0) continue;
+        const unsigned code = __atomic_exchange_n(&words[i], 0u, __ATOMIC_ACQ_REL);   // reported once
+        if (code == 0) continue;
+        char msg[160];
+        snprintf(msg, sizeof msg, "a wait inside the %s gave up (code %#x): the output of that launch is incomplete", names[i], code);
+        zl_set_last_error(__FILE__, __LINE__, msg);
+        return ZL_ERR_CUDA;
+    }
+    return ZL_OK;
+}
 extern "C" void zl_count_launch(void) { g_launches.fetch_add(1, std::memory_order_relaxed); }
 extern "C" long long zl_launch_count(int reset) {
     long long v = g_launches.load();

@@ -51,7 +51,7 @@ inline int staged_load(StagedMap& m, const char* name, const void* data_host, in
     const size_t bytes = (size_t)rows * cols * elem_bytes;
     RCHECK(dmalloc(&s.ptr, bytes));
     ZL_CHECK_CUDA(cudaMemcpyAsync(s.ptr, data_host, bytes, cudaMemcpyHostToDevice, stream));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(stream));
+    ZL_SYNC(stream);
     staged_drop(m, name);
     m[name] = s;
     return ZL_OK;
@@ -169,7 +169,7 @@ int take_f32(M* m, const std::string& name, int rows, int cols, float** out) {
     const size_t n = (size_t)rows * cols;
     RCHECK(dmalloc((void**)out, n * 4));
     RCHECK(convert_to<float>(m, s, *out, n));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     staged_drop(m->staged, name);
     m->weight_bytes += (double)n * 4;
     return ZL_OK;
@@ -185,7 +185,7 @@ int put_weight(M* m, const std::string& name, int rows, int cols, void* dst, siz
         RCHECK(convert_to<float>(m, s, static_cast<float*>(dst) + off, n));
     else
         RCHECK(convert_to<__nv_bfloat16>(m, s, static_cast<__nv_bfloat16*>(dst) + off, n));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     staged_drop(m->staged, name);
     m->weight_bytes += (double)n * m->esz;
     return ZL_OK;
@@ -235,7 +235,7 @@ int take_norm_plus_one(M* m, const std::string& name, int n, float** out) {
     RCHECK(take_f32(m, name, 1, n, out));
     k_add_const<<<cdiv(n, 256), 256, 0, m->stream>>>(*out, n, 1.0f);
     ZL_CHECK_LAUNCH();
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -245,7 +245,7 @@ int put_bias_f32(M* m, const std::string& name, int n, float* dst, int off) {
     const Staged* s = need(m, name, 1, n);
     if (!s) return ZL_ERR_STATE;
     RCHECK(convert_to<float>(m, s, dst + off, (size_t)n));
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     staged_drop(m->staged, name);
     return ZL_OK;
 }
@@ -257,7 +257,7 @@ int bias_copy_act(M* m, const float* src, int n, void** out) {
     RCHECK(dmalloc(out, (size_t)n * 2));
     k_convert<float, __nv_bfloat16><<<cdiv(n, 256), 256, 0, m->stream>>>(src, static_cast<__nv_bfloat16*>(*out), (size_t)n);
     ZL_CHECK_LAUNCH();
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     return ZL_OK;
 }
 
@@ -290,7 +290,7 @@ int put_interleaved(M* m, const std::string& a, const std::string& b, int rows, 
                                                                   (__nv_bfloat16*)dst + off, rows, cols);
     }
     ZL_CHECK_LAUNCH();
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     staged_drop(m->staged, a);
     staged_drop(m->staged, b);
     if (!dst_f32) m->weight_bytes += 2.0 * n * m->esz;
@@ -338,7 +338,7 @@ int take_latent(M* m, const std::string& name, bool uk, int H, int n, int R, int
         else launch_uk_uv<float, __nv_bfloat16>(uk, s->ptr, *out, H, n, R, RC, m->stream);
     }
     ZL_CHECK_LAUNCH();
-    ZL_CHECK_CUDA(cudaStreamSynchronize(m->stream));
+    ZL_SYNC(m->stream);
     staged_drop(m->staged, name);
     m->weight_bytes += (double)H * n * RC * m->esz;
     return ZL_OK;

@@ -1,7 +1,8 @@
 // Building blocks of the kernels that run one tcgen05.mma over a pair of SMs (cta_group::2): a cluster of two CTAs, of which rank 0
 // (the leader) issues the MMAs for both.  Each CTA holds 128 of the 256 A rows and half of the B rows in its own shared memory, and
-// the accumulators of its own 128 rows in its own TMEM.  Waits give up after about a second (an error word is set, every role
-// leaves its loop, TMEM is freed and the kernel returns): a fault in the protocol must not hang the GPU.
+// the accumulators of its own 128 rows in its own TMEM.  Waits give up after about a second (a word in host memory is set, every role
+// leaves its loop, TMEM is freed and the kernel returns): a fault in the protocol must not hang the GPU.  What is left of the output is
+// unwritten then; zl_check_waits() makes it an error of the next synchronisation of a decoder, or of the next call of these GEMMs.
 #pragma once
 #include "tc_common.cuh"
 
@@ -40,7 +41,10 @@ __device__ __forceinline__ bool tc2_wait(uint64_t* bar, uint32_t parity, volatil
             unsigned spins = 0;
             while (!(ok = mbar_try_wait(bar, parity))) {
                 if ((++spins & 1023u) == 0 && (*s_abort || clock64() - t0 > 2000000000ll)) {
-                    if (!*s_abort && err) atomicExch(err, code);
+                    if (!*s_abort) {
+                        *reinterpret_cast<volatile unsigned*>(err) = code;   // host memory
+                        __threadfence_system();
+                    }
                     *s_abort = 1;
                     break;
                 }

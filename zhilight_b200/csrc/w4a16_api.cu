@@ -98,6 +98,7 @@ extern "C" int zl_w4a16_gemm_fused(const zl_w4_fused_args_t* a, zl_stream_t stre
             if (dev >= 0 && dev < 64) prepared[dev] = true;
         }
     }
+    ZL_CHECK_WAITS();
     ZL_CHECK_ARG(a && a->x && a->packed && a->M > 0 && a->N > 0 && a->K > 0);
     ZL_CHECK_SUPPORTED(a->group_size == kW4GroupK);
     ZL_CHECK_SUPPORTED(a->N % 32 == 0 && a->K % kW4GroupK == 0);

@@ -18,7 +18,7 @@ struct alignas(64) W4TcParams {
     int M, N, K, epi;
     int dbg;                    // ZL_TC_DBG timing ablations (results are wrong): 1 no x loads, 2 no dequant, 4 no MMA, 8 no weight loads
     uint2* ws;                  // [2 * CTA + slot][M][128] tagged words {fp32 partial sum, tag}: all zero between launches
-    unsigned* err;              // watchdog code
+    unsigned* err;              // where a wait that gives up leaves its code
     long long* trace;           // ZL_TC_DBG & 16: clock64 stamps of CTA 0, [role][64 stages][8]
     const float* cos;
     const float* sin;

@@ -45,9 +45,6 @@ struct T2Cfg {
     static_assert(kBytes <= 232448, "shared memory");
 };
 
-// code of the last wait that gave up (0: none)
-__device__ unsigned g_w4_tc2_err;
-
 struct T2Tile {
     int n0, t0, ntok;   // first row of w of the pair, first token, tokens (a multiple of 32)
 };
@@ -112,7 +109,7 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
             const int rec = (t.n0 + (int)rank * 128) / 32;
             for (int g = 0; g < G; ++g, ++st) {
                 if (st == C::RS) pdl_wait();
-                if (!(ok = tc2_wait(&raw_empty[rs], ph ^ 1u, s_abort, &g_w4_tc2_err, 0x3100 + rs))) break;
+                if (!(ok = tc2_wait(&raw_empty[rs], ph ^ 1u, s_abort, p.err, 0x3100 + rs))) break;
                 if (tc_elect_one()) {
                     mbar_expect_tx(&raw_full[rs], C::kNib + 4 * 80);
                     asm volatile(
@@ -142,7 +139,7 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
         for (int i = pair; ok && t2_tile(p, i, t); i += pairs) {
             const int tb = t.t0 + (int)rank * (t.ntok >> 1);
             for (int g = 0; g < G; ++g) {
-                if (!(ok = tc2_wait(&ax_empty[as], ph ^ 1u, s_abort, &g_w4_tc2_err, 0x3200 + as))) break;
+                if (!(ok = tc2_wait(&ax_empty[as], ph ^ 1u, s_abort, p.err, 0x3200 + as))) break;
                 if (tc_elect_one()) {
                     if (rank == 0) mbar_expect_tx(&a_full[as], (uint32_t)(4 * box * 128));
                     const uint32_t bar = cluster_map(smem_u32(&a_full[as]), 0);
@@ -165,11 +162,11 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
             bool ok = true;
             const uint64_t atom = (uint64_t)(((p.ntok >> 1) * 128) >> 4);   // descriptor step from k 0..63 to k 64..127 of a stage
             for (int i = pair; ok && t2_tile(p, i, t); i += pairs) {
-                if (!(ok = tc2_wait(&acc_empty[acc], acc_ph ^ 1u, s_abort, &g_w4_tc2_err, 0x3300 + acc))) break;
+                if (!(ok = tc2_wait(&acc_empty[acc], acc_ph ^ 1u, s_abort, p.err, 0x3300 + acc))) break;
                 tc_fence_after();
                 const uint32_t d = tmem + (uint32_t)(acc * 128), idesc = tc2_idesc(false, t.ntok);
                 for (int g = 0; g < G; ++g) {
-                    if (!(ok = tc2_wait(&a_full[as], ph, s_abort, &g_w4_tc2_err, 0x3400 + as))) break;
+                    if (!(ok = tc2_wait(&a_full[as], ph, s_abort, p.err, 0x3400 + as))) break;
                     tc_fence_after();
                     if (tc_elect_one()) {
                         const uint32_t a = tmem + (uint32_t)(C::kACol0 + as * 64);
@@ -208,7 +205,7 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
                 if (st % C::AS != as) continue;
                 if (st == as + C::AS) pdl_wait();
                 const int rs = st % C::RS;
-                if (!(ok = tc2_wait(&raw_full[rs], (uint32_t)(st / C::RS) & 1u, s_abort, &g_w4_tc2_err, 0x3600 + rs))) break;
+                if (!(ok = tc2_wait(&raw_full[rs], (uint32_t)(st / C::RS) & 1u, s_abort, p.err, 0x3600 + rs))) break;
                 const uint8_t* nib = smem + C::kNibOff + rs * C::kNib + q * 2048;
                 const uint8_t* tr = smem + C::kTrOff + rs * C::kTr + q * 80;
                 const __half2 sc2 = *reinterpret_cast<const __half2*>(tr + (tt * 8 + g8) * 4);
@@ -243,7 +240,7 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
                         }
                     }
                     if (ks == 0) {
-                        if (!(ok = tc2_wait(&ax_empty[as], ph ^ 1u, s_abort, &g_w4_tc2_err, 0x3700 + as))) break;
+                        if (!(ok = tc2_wait(&ax_empty[as], ph ^ 1u, s_abort, p.err, 0x3700 + as))) break;
                         tc_fence_after();
                     }
                     tc_st16(taddr + (uint32_t)(ks * 32), r[0]);
@@ -267,7 +264,7 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
             const bool res = p.epi == ZL_EPI_RESIDUAL && p.wide && prow < p.N;
             uint32_t rnext[8];
             if (res) tc_fetch_residual(p, prow, lane, t.t0 + set * 16, rnext);
-            if (!tc2_wait(&acc_full[acc], acc_ph, s_abort, &g_w4_tc2_err, 0x3800 + acc)) break;
+            if (!tc2_wait(&acc_full[acc], acc_ph, s_abort, p.err, 0x3800 + acc)) break;
             tc_fence_after();
             const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * 128);
             if (prow < p.N) {               // N % 128 == 0: all of the CTA's rows or none
@@ -341,7 +338,10 @@ bool w4_tc2_route(int M, int N, int K) {
 cudaError_t launch_w4_tc2(const W4Params& p, bool pdl, cudaStream_t stream) {
     const int row_tiles = cdiv(p.N, kTc2Rows), G = p.K / kW4GroupK, max_pairs = device_sm_count() / 2;
     W4TcParams q;
+    unsigned* words = wait_words();
+    if (!words) return cudaErrorMemoryAllocation;
     if (!w4_tc_params(q, p)) return cudaErrorInvalidValue;
+    q.err = words + kWaitW4Pairs;
     q.ntok = t2_pick_ntok(p.mc, row_tiles, G, max_pairs);
     q.tok_tiles = cdiv(p.mc, q.ntok);
     if (!tc2_map_3d(&q.xmap, p.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, p.K, p.mc, 1, p.ldx, 0, q.ntok / 2)) return cudaErrorInvalidValue;
@@ -352,7 +352,7 @@ cudaError_t launch_w4_tc2(const W4Params& p, bool pdl, cudaStream_t stream) {
 }  // namespace zl
 
 extern "C" unsigned zl_w4_tc2_watchdog(void) {
-    unsigned v = 0;
-    cudaMemcpyFromSymbol(&v, zl::g_w4_tc2_err, sizeof v);
-    return v;
+    cudaDeviceSynchronize();
+    const unsigned* words = zl::wait_words();
+    return words ? words[zl::kWaitW4Pairs] : 0u;
 }

@@ -515,6 +515,7 @@ static bool w8_tc_route(int M, int N, int K) {
 extern "C" int zl_w8a8_gemm(const void* xq, const float* x_scale, const void* w, const void* w_scale,
                             int w_scale_dtype, const void* bias, void* y, int M, int N, int K, int kind, int dtype,
                             int pdl, zl_stream_t stream) {
+    ZL_CHECK_WAITS();
     ZL_CHECK_ARG(xq && x_scale && w && w_scale && y && M > 0 && N > 0 && K > 0);
     ZL_CHECK_ARG(dtype == ZL_F16 || dtype == ZL_BF16);
     ZL_CHECK_ARG(kind == ZL_W8_INT8 || kind == ZL_W8_FP8 || kind == ZL_W8_FP8_ROWS);

@@ -39,6 +39,12 @@ def _stream():
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
+def check_waits():
+    """After a synchronisation: raises if a bounded wait inside a GEMM over pairs of SMs has given up, its output being incomplete.
+    The decoders and the next call of such a GEMM raise by themselves."""
+    _lib.call("zl_check_waits")
+
+
 # ------------------------------------------------------------------ load-time transforms
 def gptq_shuffle(qweight, q_perm=None):
     """nn::gptq::gptq_shuffle -- in place on (K/8, N) int32."""
