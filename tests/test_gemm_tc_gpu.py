@@ -122,3 +122,54 @@ def test_infinities_stay_in_their_rows_and_columns(lib, cuda):
     keep = torch.ones_like(bad, dtype=torch.bool)
     keep[69], keep[:, 17] = False, False
     assert torch.equal(bad[keep], good[keep])
+
+
+def _nt(lib, x, xb, ldx, w, wb, ldw, y, yb, ldy, m, n, k, batch, epilogue=0, gate=None, gb=0, ldg=0):
+    """zl_gemm_nt on tensors of any pitches (elements)."""
+    from zhilight_b200 import _lib, ops
+    _lib.call("zl_gemm_nt", x.data_ptr(), ldx, xb, w.data_ptr(), ldw, wb, y.data_ptr(), ldy, yb, m, n, k, batch, ops._dt(x), ops._dt(y),
+              epilogue, gate.data_ptr() if gate is not None else None, ldg, gb, 0, torch.cuda.current_stream().cuda_stream)
+
+
+@pytest.mark.parametrize("dtype", [BF, HF])
+@pytest.mark.parametrize("t", [33, 64, 300])
+@pytest.mark.parametrize("h,d,r,rs", [(16, 128, 512, 512), (5, 128, 512, 576), (3, 192, 136, 140)])
+def test_heads_as_the_batch(lib, cuda, dtype, t, h, d, r, rs):
+    """The latent layers' products: pitch between heads smaller than the row pitch, for x and y; y's rows longer than its columns; the
+    way back with a gate that is part of a wider row."""
+    from zhilight_b200 import ops
+    g = torch.Generator().manual_seed(t + r)
+    q, uk = _rand(g, t, h, d, dtype=dtype), _rand(g, h, r, d, dtype=dtype)
+    y = torch.full((t, h, rs), -7.0, device=cuda)
+    _nt(lib, q, d, h * d, uk, r * d, d, y, rs, h * rs, t, r, d, h)
+    prod = lambda a, c: torch.einsum("thd,hrd->thr", a.double(), c.double())  # noqa: E731
+    _close(y[:, :, :r], prod(q, uk), prod(q.abs(), uk.abs()), d, torch.float32)
+    assert bool((y[:, :, r:] == -7.0).all())
+    lat, uv = _rand(g, t, h, r, dtype=dtype) / 8, _rand(g, h, d, r, dtype=dtype)
+    wide = torch.randn(t, 24 + h * d, generator=g).cuda()
+    gate = wide[:, 24:]
+    for epilogue in (ops.GEMM_EPI_NONE, ops.GEMM_EPI_SIGMOID_GATE):
+        out = torch.zeros(t, h, d, dtype=dtype, device=cuda)
+        _nt(lib, lat, r, h * r, uv, d * r, r, out, d, h * d, t, d, r, h, epilogue, gate, d, wide.shape[1])
+        s = torch.sigmoid(gate.double()).reshape(t, h, d) if epilogue else torch.ones(t, h, d, dtype=torch.float64, device=cuda)
+        _close(out, prod(lat, uv) * s, prod(lat.abs(), uv.abs()) * s * 1.01, r + 64, dtype)   # + 64: a few units of fp32 for the sigmoid
+
+
+@pytest.mark.parametrize("ldx,ldw,ldy,pad", [(136, 128, 200, 0), (1024, 520, 130, 1), (128, 128, 129, 3)])
+def test_row_pitches_and_odd_distances(lib, cuda, ldx, ldw, ldy, pad):
+    """Rows apart from each other; an output whose rows, matrices and base are no multiples of two values (narrow stores)."""
+    g = torch.Generator().manual_seed(ldx)
+    b, m, n, k = 3, 45, 128, 128
+    x, w = _rand(g, b, m, ldx, dtype=BF), _rand(g, b, n, ldw, dtype=BF)
+    flat = torch.full((pad + b * (m * ldy + pad),), -7.0, dtype=BF, device=cuda)
+    y = flat[pad:]
+    yb = m * ldy + pad
+    _nt(lib, x, m * ldx, ldx, w, n * ldw, ldw, y, yb, ldy, m, n, k, b)
+    xs, ws = x[:, :, :k].double(), w[:, :, :k].double()
+    ref, mag = torch.einsum("bmk,bnk->bmn", xs, ws), torch.einsum("bmk,bnk->bmn", xs.abs(), ws.abs())
+    for i in range(b):
+        _close(y[i * yb:i * yb + m * ldy].reshape(m, ldy)[:, :n], ref[i], mag[i], k, BF)
+    touched = torch.zeros_like(flat, dtype=torch.bool)
+    for i in range(b):
+        touched[pad + i * yb:pad + i * yb + m * ldy].reshape(m, ldy)[:, :n] = True
+    assert bool((flat[~touched] == -7.0).all())

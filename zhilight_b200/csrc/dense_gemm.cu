@@ -255,8 +255,9 @@ extern "C" int zl_dense_gemm_skinny_mul(const void* x, int ldx, const void* w, c
         GemmP p{x, w, y, mul_all, ldx, 0, K, 0, N, 0, ld_mul, 0, M, N, K};
         p.bias_t = bias;
         const int epi = act == 1 ? ZL_GEMM_EPI_RELU2 : act == 2 ? ZL_GEMM_EPI_TANH : act == 3 ? ZL_GEMM_EPI_GELU_TANH_MUL : ZL_GEMM_EPI_NONE;
-        if (gemm_tc_route(p, 1, dtype)) {
-            ZL_CHECK_CUDA(launch_gemm_tc(p, 1, dtype, out_dtype, epi, pdl != 0, stream));
+        const cudaError_t e = gemm_tc_route(p, 1, dtype) ? launch_gemm_tc(p, 1, dtype, out_dtype, epi, pdl != 0, stream) : cudaErrorNotSupported;
+        if (e != cudaErrorNotSupported) {
+            ZL_CHECK_CUDA(e);
             return ZL_OK;
         }
     }

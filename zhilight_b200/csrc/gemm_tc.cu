@@ -475,7 +475,7 @@ static cudaError_t launch_gt16(const GemmTcP& q, bool grouped, int pairs, bool p
     return grouped ? launch_gt<T, TO, true, kGt16>(q, pairs, pdl, stream) : launch_gt<T, TO, false, kGt16>(q, pairs, pdl, stream);
 }
 
-// tiles, maps and stages of a call; returns the number of pairs, 0 on failure
+// tiles, maps and stages of a call; returns the number of pairs, 0 without a map
 static int gt_plan(GemmTcP& q, CUtensorMapDataType dt, int batch, int out_bytes) {
     const GemmP& p = q.g;
     const bool grouped = p.grp_off != nullptr;
@@ -512,7 +512,7 @@ cudaError_t launch_gemm_tc(const GemmP& p, int batch, int in_dtype, int out_dtyp
     q.g = p;
     q.epi = epilogue;
     const int pairs = gt_plan(q, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, batch, out_dtype == ZL_F32 ? 4 : 2);
-    if (pairs <= 0) return cudaErrorInvalidValue;
+    if (pairs <= 0) return cudaErrorNotSupported;
     if (bf16) return out_dtype == ZL_F32 ? launch_gt16<__nv_bfloat16, float>(q, grouped, pairs, pdl, stream)
                                          : launch_gt16<__nv_bfloat16, __nv_bfloat16>(q, grouped, pairs, pdl, stream);
     return out_dtype == ZL_F32 ? launch_gt16<__half, float>(q, grouped, pairs, pdl, stream) : launch_gt16<__half, __half>(q, grouped, pairs, pdl, stream);
@@ -528,7 +528,7 @@ cudaError_t launch_w8_gemm_tc(const uint8_t* xq, const float* sx, const uint8_t*
     q.sw = sw;
     q.sw_mode = sw_mode;
     const int pairs = gt_plan(q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, 2);
-    if (pairs <= 0) return cudaErrorInvalidValue;
+    if (pairs <= 0) return cudaErrorNotSupported;
     return launch_gt<T, T, false, FP8 ? kGtFp8 : kGtInt8>(q, pairs, pdl, stream);
 }
 #define ZL_W8_TC(T, F8)                                                                                                                    \

@@ -501,10 +501,13 @@ static int gemm_dispatch(GemmP p, int batch, int in_dtype, int out_dtype, int ep
     const int elem = in_dtype == ZL_F32 ? 4 : 2;
     // gathered rows start at any multiple of ldx: the batch stride plays no part in their alignment
     const bool vx = aligned_for(p.x, p.ldx, p.xb, K, elem, batch), vw = aligned_for(p.w, p.ldw, p.wb, K, elem, batch);
-    cudaError_t e;
-    if (gemm_tc_route(p, batch, in_dtype)) {
-        e = launch_gemm_tc(p, batch, in_dtype, out_dtype, epilogue, pdl != 0, stream);
-    } else if (in_dtype == ZL_F32) {
+    cudaError_t e = gemm_tc_route(p, batch, in_dtype) ? launch_gemm_tc(p, batch, in_dtype, out_dtype, epilogue, pdl != 0, stream)
+                                                      : cudaErrorNotSupported;
+    if (e != cudaErrorNotSupported) {
+        ZL_CHECK_CUDA(e);
+        return ZL_OK;
+    }
+    if (in_dtype == ZL_F32) {
         const dim3 grid(cdiv(N, kGB), cdiv(M, kGB), batch), block(256);
         if (epilogue == ZL_GEMM_EPI_RELU2)
             e = launch(k_gemm_f32<ZL_GEMM_EPI_RELU2>, grid, block, 0, stream, pdl != 0, p, (int)vx, (int)vw);

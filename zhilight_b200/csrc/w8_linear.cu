@@ -541,8 +541,10 @@ extern "C" int zl_w8a8_gemm(const void* xq, const float* x_scale, const void* w,
             else ZL_W8_TC(__nv_bfloat16, false);
         }
 #undef ZL_W8_TC
-        ZL_CHECK_CUDA(e);
-        return ZL_OK;
+        if (e != cudaErrorNotSupported) {   // else: nothing launched, no tensor map could be made
+            ZL_CHECK_CUDA(e);
+            return ZL_OK;
+        }
     }
     for (int m0 = 0; m0 < M; m0 += 32) {
         const int mc = (M - m0) < 32 ? (M - m0) : 32;
