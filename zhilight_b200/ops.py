@@ -345,16 +345,22 @@ def _ptr_tables(device, *lists):
 
 
 def _in_use(*tensors):
-    """The call goes on after this function returns.  Memory that belongs to another stream is not given away before it ends;
-    what the allocator does not watch (mapped host memory) is waited for."""
+    """The call goes on after this function returns.  Memory of torch's allocator that belongs to another stream is not given away
+    before it ends.  Memory of another owner (DLPack, IPC: torch cannot resize it; mapped host memory) goes with its tensor, so the
+    call is waited for, except while it is only being captured."""
     s = torch.cuda.current_stream()
+    wait = False
     for t in tensors:
         if t is None:
             continue
-        if t.is_cuda:
+        if not t.is_cuda:
+            wait = True
+        elif t.untyped_storage().resizable():
             t.record_stream(s)
         else:
-            s.synchronize()
+            wait = wait or not torch.cuda.is_current_stream_capturing()
+    if wait:
+        s.synchronize()
 
 
 def copy_to_rag_buffer2(placement, buf_lens, k_src, v_src, k_bufs, v_bufs, bshd=True):
