@@ -173,3 +173,36 @@ def test_row_pitches_and_odd_distances(lib, cuda, ldx, ldw, ldy, pad):
     for i in range(b):
         touched[pad + i * yb:pad + i * yb + m * ldy].reshape(m, ldy)[:, :n] = True
     assert bool((flat[~touched] == -7.0).all())
+
+
+_FEW_ROWS = """
+import sys, torch
+sys.path.insert(0, sys.argv[1])
+from zhilight_b200 import ops
+g = torch.Generator(device="cuda").manual_seed(1)
+groups, n, k, m = 8, 2048, 4096, 20                      # large enough for the tensor-core kernel from 9 rows on
+x = torch.randn(m, k, generator=g, device="cuda").bfloat16()
+w = torch.randn(groups, n, k, generator=g, device="cuda").bfloat16()
+owner = torch.arange(m, device="cuda") * groups // m
+def call(lo, hi):
+    off = torch.zeros(groups + 1, dtype=torch.int32, device="cuda")
+    off[1:] = torch.bincount(owner[lo:hi], minlength=groups).cumsum(0)
+    return ops.gemm_nt_grouped(x[lo:hi].contiguous(), w, off, hi - lo, out_dtype=torch.float32)
+whole, parts = call(0, m), torch.cat([call(i, min(i + 8, m)) for i in range(0, m, 8)])
+print("SAME" if torch.equal(whole, parts) else "OTHER")
+"""
+
+
+@pytest.mark.parametrize("limit,want", [("32", "SAME"), (None, "OTHER")])
+def test_row_limit_of_the_few_rows_kernel(cuda, limit, want):
+    """ZL_GEMM_GROUPED_SMALL_MAX keeps the rows of a step up to that count with the few-rows kernel, whose sums do not depend on how many rows there
+    are; without it 20 rows of large matrices take the tensor-core kernel, which adds in another order."""
+    import os
+    import subprocess
+    import sys
+    env = {k: v for k, v in os.environ.items() if k != "ZL_GEMM_GROUPED_SMALL_MAX"}
+    if limit:
+        env["ZL_GEMM_GROUPED_SMALL_MAX"] = limit
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _FEW_ROWS, root], env=env, capture_output=True, text=True, timeout=300)
+    assert r.stdout.split() == [want], r.stdout + r.stderr

@@ -501,7 +501,10 @@ static int gemm_dispatch(GemmP p, int batch, int in_dtype, int out_dtype, int ep
     const int elem = in_dtype == ZL_F32 ? 4 : 2;
     // gathered rows start at any multiple of ldx: the batch stride plays no part in their alignment
     const bool vx = aligned_for(p.x, p.ldx, p.xb, K, elem, batch), vw = aligned_for(p.w, p.ldw, p.wb, K, elem, batch);
-    cudaError_t e = gemm_tc_route(p, batch, in_dtype) ? launch_gemm_tc(p, batch, in_dtype, out_dtype, epilogue, pdl != 0, stream)
+    // a decode step's experts: a handful of rows per group
+    const bool few_rows = grouped && in_dtype != ZL_F32 && M <= grouped_small_max() && vx && vw && K % 8 == 0 && (size_t)8 * K * 2 <= 160 * 1024 &&
+                          (epilogue == ZL_GEMM_EPI_NONE || epilogue == ZL_GEMM_EPI_RELU2 || pairs);
+    cudaError_t e = !few_rows && gemm_tc_route(p, batch, in_dtype) ? launch_gemm_tc(p, batch, in_dtype, out_dtype, epilogue, pdl != 0, stream)
                                                       : cudaErrorNotSupported;
     if (e != cudaErrorNotSupported) {
         ZL_CHECK_CUDA(e);
@@ -527,8 +530,7 @@ static int gemm_dispatch(GemmP p, int batch, int in_dtype, int out_dtype, int ep
             e = launch(k_gemm_f32<ZL_GEMM_EPI_SOFTCAP>, grid, block, 0, stream, pdl != 0, p, (int)vx, (int)vw);
         else
             e = launch(k_gemm_f32<ZL_GEMM_EPI_NONE>, grid, block, 0, stream, pdl != 0, p, (int)vx, (int)vw);
-    } else if (grouped && M <= grouped_small_max() && vx && vw && K % 8 == 0 && (size_t)8 * K * 2 <= 160 * 1024 &&
-               (epilogue == ZL_GEMM_EPI_NONE || epilogue == ZL_GEMM_EPI_RELU2 || pairs)) {   // a decode step's experts: a handful of rows per group
+    } else if (few_rows) {
         p.act_relu2 = epilogue == ZL_GEMM_EPI_RELU2;
         if (in_dtype == ZL_BF16)
             e = out_dtype == ZL_F32 ? launch_grouped_small<__nv_bfloat16, float>(p, batch, pairs, pdl != 0, stream)
