@@ -144,6 +144,8 @@ int zl_w4_int_kernel_fits(int M, int N, int K);
 /* which kernel serves (M, N, K) on the ZLW4I layout (variant 1): 3 = exact-integer mma.sync kernel, 4 = tcgen05 / TMEM /
  * TMA kernel (any M, N % 128 == 0, no fused RMSNorm prologue), 0 = neither (pack variant 0 and use the fp16 mma.sync kernel). */
 int zl_w4_int_layout_route(int M, int N, int K);
+/* whether, of the two kernels behind answer 4, the one over pairs of SMs serves the shape (1) or the stream-k kernel (0) */
+int zl_w4_pairs_route(int M, int N, int K);
 /* last watchdog code published by the 4-bit stream-k kernel on the current device (0 = none); a bounded mbarrier wait that expires
  * records which pipeline barrier starved and traps instead of hanging the GPU. */
 unsigned zl_w4_tc_watchdog(void);

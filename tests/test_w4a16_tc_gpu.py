@@ -1,6 +1,7 @@
-"""GPU parity: the tcgen05 W4A16 kernel (k_w4a16_ts: A operand in TMEM, ZLW4I layout) vs the CPU oracle.
+"""GPU parity: the tcgen05 W4A16 kernels of the ZLW4I layout vs the CPU oracle: stream-k (k_w4a16_ts) and pairs of SMs (k_w4a16_tc2).  Which one serves
+a shape is zl_w4_pairs_route's answer; the tests named stream_k assert that it is the first.
 
-The kernel rounds w = (q - z) * s to fp16 once (what the reference's M > 40 dequant + cuBLASLt route does,
+Each rounds w = (q - z) * s to fp16 once (what the reference's M > 40 dequant + cuBLASLt route does,
 q_gemm_k_major.cu:843-905, 1083-1100), multiplies fp16 x fp16 exactly and accumulates all of K in fp32 in TMEM.
 Tolerance (north_star): relative L2 <= 1e-3 against the fp32 oracle for fp16 outputs."""
 import numpy as np
@@ -35,7 +36,7 @@ def splits(lib):
 
 
 def _check_watchdog(lib):
-    assert lib.zl_w4_tc_watchdog() == 0
+    assert lib.zl_w4_tc_watchdog() == 0 and lib.zl_w4_tc2_watchdog() == 0
 
 
 def test_route_selects_tcgen05(lib):
@@ -52,7 +53,7 @@ def test_route_selects_tcgen05(lib):
 
 @pytest.mark.parametrize("m", [17, 32, 33, 64, 65, 128, 200, 256, 300])
 def test_token_counts(lib, cuda, m):
-    """every NTOK instantiation (32 / 64 / 128 / 256), ragged last 16-token chunk, and a second pass beyond 256"""
+    """ragged last 16-token chunks on both sides of 256 rows (a small matrix: pairs of SMs)"""
     from zhilight_b200 import ops
     k, n = 1024, 512
     w, packed = _setup(cuda, k, n, False, 5)
@@ -166,3 +167,58 @@ def test_strided_activations_and_fused_norm_is_rejected(lib, cuda):
     assert rel_l2(y, gptq.gemm_f32(x.cpu().numpy(), w)) <= TOL
     with pytest.raises(_lib.ZLError):
         ops.w4a16_gemm_fused(x, packed, n, k, variant=1, ln_weight=torch.ones(k, dtype=torch.float16, device=cuda))
+
+
+@pytest.mark.parametrize("m", [17, 32, 33, 64, 65, 128, 129, 200, 256])
+@pytest.mark.parametrize("k,n", [(8192, 384), (14336, 512)])
+def test_stream_k_token_counts(lib, cuda, m, k, n):
+    """every NTOK instantiation (32 / 64 / 128 / 256), ragged last 16-token chunk; every tile is cut"""
+    from zhilight_b200 import ops
+    assert lib.zl_w4_int_layout_route(m, n, k) == 4 and lib.zl_w4_pairs_route(m, n, k) == 0
+    w, packed = _setup(cuda, k, n, False, 5)
+    x = torch.randn(m, k, generator=torch.Generator().manual_seed(m)).half()
+    y = ops.w4a16_gemm_fused(x.to(cuda), packed, n, k, variant=1)
+    assert torch.equal(y, ops.w4a16_gemm_fused(x.to(cuda), packed, n, k, variant=1))   # the exchanged words are empty again
+    _check_watchdog(lib)
+    y, ref = y.float().cpu().numpy(), gptq.gemm_f32(x.numpy(), w)
+    assert rel_l2(y, ref) <= TOL
+    for i in range(m):
+        assert rel_l2(y[i], ref[i]) <= 2 * TOL, i
+
+
+@pytest.mark.parametrize("m,k,f,n", [(20, 4096, 1280, 640), (40, 4096, 1344, 640), (100, 4096, 1280, 512), (33, 4096, 14336, 28672)])
+def test_stream_k_bias_residual_swiglu(lib, cuda, m, k, f, n):
+    """Epilogues behind the exchange of partial tiles, and (the last shape, more tiles than blocks) of whole tiles with the residual
+    fetched ahead; the residual's stores of two columns and, from an odd address, of one."""
+    from zhilight_b200 import ops
+    assert [lib.zl_w4_pairs_route(m, i, k) for i in (2 * f, n)] == [0, 0]
+    g = torch.Generator().manual_seed(9)
+    x = torch.randn(m, k, generator=g).half()
+    w, packed = _setup(cuda, k, 2 * f, False, 7, ops.swiglu_row_map(f, cuda))
+    y = ops.w4a16_gemm_fused(x.to(cuda), packed, 2 * f, k, epilogue=ops.EPI_SWIGLU, variant=1).float().cpu().numpy()
+    gu = oops._t(gptq.gemm_f32(x.numpy(), w), "f16")
+    assert rel_l2(y, gu[:, :f] / (1.0 + np.exp(-gu[:, :f])) * gu[:, f:]) <= 2e-3
+    del w, packed
+    w2, packed2 = _setup(cuda, k, n, True, 4)
+    bias, res = (torch.randn(n, generator=g) * 0.5).half(), torch.randn(m, n, generator=g).half()
+    call = lambda r, out=None: ops.w4a16_gemm_fused(x.to(cuda), packed2, n, k, bias=bias.to(cuda), residual=r,  # noqa: E731
+                                                    epilogue=ops.EPI_RESIDUAL, variant=1, out=out)
+    y2 = call(res.to(cuda))
+    lin = oops._t(gptq.gemm_f32(x.numpy(), w2) + bias.float().numpy(), "f16")
+    assert rel_l2(y2.float().cpu().numpy(), oops._t(lin + res.float().numpy(), "f16")) <= TOL
+    h = res.to(cuda)                                    # in place
+    call(h, out=h)
+    assert torch.equal(h, y2)
+    odd = torch.empty(m * n + 1, dtype=torch.float16, device=cuda)[1:].view(m, n)
+    odd.copy_(res)
+    call(odd, out=odd)
+    assert torch.equal(odd, y2)
+    _check_watchdog(lib)
+
+
+@pytest.mark.parametrize("t", [32, 64])
+def test_stream_k_qkv_rope_epilogue(lib, cuda, t):
+    from zhilight_b200 import ops
+    hq, hkv, d, k = 32, 8, 128, 4096
+    assert lib.zl_w4_pairs_route(t, (hq + 2 * hkv) * d, k) == 0
+    test_qkv_rope_epilogue(lib, cuda, lib.zl_w4_tc_set_splits, d, hq, hkv, k, t, 0)

@@ -3,7 +3,9 @@
 // Stands in for nn::gptq::gptq_gemm_k_major's router (reference src/nn/quant/gptq/q_gemm_k_major.cu:957-1116:
 // M <= 40 GEMV, else dequant + cuBLASLt) and for GPTQMarlin::forward (src/nn/linear/linear.cpp:1247-1451):
 //   M <= 16 and the staged activations fit shared memory -> k_w4a16_v3  (exact-integer mma.sync kernel, ZLW4I layout)
-//   otherwise, N % 128 == 0                              -> k_w4a16_ts  (tcgen05 kernel, A operand in TMEM, ZLW4I layout)
+//   otherwise, N % 128 == 0                              -> k_w4a16_tc2 (tcgen05 over pairs of SMs, ZLW4I layout) where w4_tc2_route has it
+//                                                           faster, always above 256 rows; else
+//                                                           k_w4a16_ts  (tcgen05 kernel, stream-k, A operand in TMEM, ZLW4I layout)
 //   otherwise                                            -> k_w4a16_v2  (fp16 mma.sync kernel, ZLW4 layout, 32-row passes)
 #include "common.cuh"
 #include "w4_layout.cuh"
@@ -69,6 +71,10 @@ extern "C" int zl_w4_int_kernel_fits(int M, int N, int K) {
 extern "C" int zl_w4_int_layout_route(int M, int N, int K) {
     if (M <= 0 || N <= 0 || K <= 0 || N % 32 || K % kW4GroupK) return 0;
     return int_layout_route(M, N, K);
+}
+
+extern "C" int zl_w4_pairs_route(int M, int N, int K) {
+    return zl_w4_int_layout_route(M, N, K) == 4 && w4_tc2_route(M, N, K) ? 1 : 0;
 }
 
 extern "C" int zl_qkv_rope_row_map(int32_t* row_map, int n_heads_total, int dim_head, zl_stream_t stream) {
