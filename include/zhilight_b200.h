@@ -165,6 +165,7 @@ int zl_w4_tc_set_splits(int splits);
 /* tests: host view of the tcgen05 kernel's stream-k schedule (the kernel's own scheduling code): pieces of CTA `cta` of `ctas`
  * for n_tiles x G (tile, group) units; out[5 i ..] = tile, g0, g1, pieces of that tile, workspace slot (-1: whole tile);
  * returns the number of pieces. */
+int zl_w4_tc_pipeline(int ntok, int* out); /* tests: {conversion groups, A stages, raw weight stages} for ntok = 32, 64, 128, 256 */
 int zl_w4_tc_schedule(int n_tiles, int G, int ctas, int cta, int* out, int max_pieces);
 /* debug: with ZL_TC_DBG & 16, CTA 0 of the tcgen05 kernel stamps its pipeline hand-overs with clock64; copies
  * [11 roles][64 stages][4 events] of the last launch to `out` (n <= 2816 values). */

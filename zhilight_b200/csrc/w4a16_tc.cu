@@ -67,7 +67,11 @@ struct TsCfg {
     // against 128 cycles of tensor work per group at 32 tokens -- two groups per stage halve that overhead per byte.
     static constexpr int KG = NTOK <= 128 ? 2 : 1;
     static constexpr int AS = NTOK <= 64 ? 3 : (NTOK <= 128 ? 2 : 3);   // A (TMEM) / x (smem) stages
-    static constexpr int RS = NTOK <= 64 ? 4 : 3;                       // raw weight stages
+    // Raw weight stages.  A slot must always be the same group's: a wait by parity cannot tell "landed" from "the landing before last", and
+    // a group whose own stages have landed may stand a stage ahead of the other.  With three slots for two groups (up to 256 tokens
+    // once) it would then take a slot whose bytes for the other group are still on their way, read them too early and free the slot.
+    static constexpr int RS = 4;
+    static_assert(RS % NG == 0, "a raw slot belongs to one group");
     static constexpr int NACC = NTOK <= 128 ? 2 : 1;                    // accumulator buffers in TMEM
     static constexpr int kACol0 = NACC * NTOK;                          // first A column; 64 columns per group
     static constexpr int kXGroup = 2 * NTOK * 128;                      // [k atom (64 k)][token][128 B]
@@ -563,6 +567,19 @@ extern "C" int zl_w4_tc_schedule(int n_tiles, int G, int ctas, int cta, int* out
         out[5 * i + 4] = whole ? -1 : sch.slot(cta, tile);
     }
     return sch.n_segs;
+}
+
+// tests: conversion groups, A stages and raw weight stages of the instantiation that serves up to `ntok` tokens
+template <int NTOK>
+static int ts_pipeline(int* out) {
+    out[0] = TsCfg<NTOK>::NG;
+    out[1] = TsCfg<NTOK>::AS;
+    out[2] = TsCfg<NTOK>::RS;
+    return ZL_OK;
+}
+extern "C" int zl_w4_tc_pipeline(int ntok, int* out) {
+    ZL_CHECK_ARG(out && (ntok == 32 || ntok == 64 || ntok == 128 || ntok == 256));
+    return ntok == 32 ? ts_pipeline<32>(out) : ntok == 64 ? ts_pipeline<64>(out) : ntok == 128 ? ts_pipeline<128>(out) : ts_pipeline<256>(out);
 }
 
 // grid override: ZL_TC_CTAS in the environment, or zl_w4_tc_set_splits(n) = "at least n pieces per tile" (tests exercise
