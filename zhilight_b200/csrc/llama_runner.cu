@@ -616,7 +616,7 @@ static void prefetch_target(zl_llama* m, int l, int slot, int B, const void** pt
 // ZL_NO_PDL_MASK (experiments): launch these kernels with a full dependency instead of a programmatic one.
 // 1 qkv GEMM, 2 attention, 4 o GEMM, 8 gate_up GEMM, 16 down GEMM, 32 final norm, 64 lm_head, 128 argmax.
 // Default 70 = lm_head + o GEMM + attention: a PDL-launched lm_head measured 128 us slower per step than a normally
-// launched one (tools/gpu_tail.sh); early-launched o GEMM / attention CTAs cost another ~1 % each.
+// launched one; early-launched o GEMM / attention CTAs cost another ~1 % each.
 static int no_pdl_mask(bool tensor_parallel = false) {
     static int v = -2;
     if (v == -2) {
@@ -624,8 +624,8 @@ static int no_pdl_mask(bool tensor_parallel = false) {
         v = e ? atoi(e) : -1;
     }
     if (v >= 0) return v;
-    // single GPU: lm_head, o GEMM, attention with full dependencies measured best (tools/gpu_pdlmask.sh: 640 -> 710 tok/s);
-    // tensor parallel (exchange inside the GEMMs): a PDL-launched attention kernel wins (N = 2: 783 vs 754 tok/s, r2s)
+    // single GPU: lm_head, o GEMM, attention with full dependencies measured best (640 -> 710 tok/s);
+    // tensor parallel (exchange inside the GEMMs): a PDL-launched attention kernel wins (N = 2: 783 vs 754 tok/s)
     return tensor_parallel ? 68 : 70;
 }
 
