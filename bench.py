@@ -1305,7 +1305,7 @@ def main():
     out["roofline"] = {
         "bound": "hbm",
         "kernel": ("k_w8a8_skinny (+ activation quant)" if args.quant != "default" else "k_dense_skinny") if dense
-        else ("k_w4a16_v3 (integer IMMA, fused norm / RoPE / SwiGLU / residual variants as in the step)" if B <= 7
+        else ("k_w4a16_v3 (integer, fused norm / RoPE / SwiGLU / residual variants as in the step)" if B <= 7
               else "k_w4a16_ts (tcgen05, A operand in TMEM, tensor-TMA)"),
         "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind,
         "bytes_per_launch": g_bytes / g_launches, "us_per_launch": g_ms * 1e3 / iters / g_launches,

@@ -88,7 +88,7 @@ size_t zl_w4_packed_bytes(int N, int K, int group_size);
 int zl_w4_pack(const uint32_t* qweight_km, const uint8_t* qzeros_km, const void* scales_km,
                const int32_t* row_map, void* packed, int N, int K, int group_size, int sym,
                zl_stream_t stream);
-/* variant 0: ZLW4 (fp16 HMMA kernels); variant 1: ZLW4I (exact-integer IMMA kernel, zl_w4a16_gemm_fused with
+/* variant 0: ZLW4 (fp16 MMA kernels); variant 1: ZLW4I (exact-integer kernel, zl_w4a16_gemm_fused with
  * args.variant = 1).  zl_w4_pack == variant 0. */
 int zl_w4_pack_v(const uint32_t* qweight_km, const uint8_t* qzeros_km, const void* scales_km,
                  const int32_t* row_map, void* packed, int N, int K, int group_size, int sym, int variant,
@@ -296,9 +296,9 @@ int zl_kv_int8_quant_append(const void* k_src, const void* v_src, const int32_t*
 /* ------------------------------------------------------------------------------------------ *
  * Decode-step helpers around the layers
  * ------------------------------------------------------------------------------------------ */
-/* nn::Embedding lookup (src/nn/embedding/embedding.cu:20-60): out[t,:] = table[ids[t],:]. */
 /* n host words (buffer addresses) -> a device table, in stream order; the host array may go when the call returns */
 int zl_write_pointers(void* dst, const void* pointers, int n, zl_stream_t stream);
+/* nn::Embedding lookup (src/nn/embedding/embedding.cu:20-60): out[t,:] = table[ids[t],:]. */
 int zl_embedding(const int32_t* ids, const void* table, void* out, int T, int D, int vocab, int dtype, int pdl,
                  zl_stream_t stream);
 /* greedy pick (generator/batch_generator.cpp:1762-1884 with beam 1): argmax over fp32 logits (T, V). */

@@ -270,7 +270,7 @@ def test_activation_digit_decomposition_identities():
         if not packed:      # two IMMAs: signed high byte (floor), unsigned low byte
             hi, lo = m >> 8, m & 0xFF
             assert hi.min() >= -128 and hi.max() <= 127 and lo.min() >= 0
-        else:               # one IMMA, both digits signed: lo' = int8(m & 0xff), hi' = (m + 128) >> 8
+        else:               # one integer MMA, both digits signed: lo' = int8(m & 0xff), hi' = (m + 128) >> 8
             lo = ((m & 0xFF) ^ 0x80) - 0x80
             hi = (m + 128) >> 8
             assert hi.min() >= -128 and hi.max() <= 127 and lo.min() >= -128 and lo.max() <= 127

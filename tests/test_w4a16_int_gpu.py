@@ -1,4 +1,4 @@
-"""GPU parity: the exact-integer W4A16 kernel (ZLW4I layout, IMMA) vs the CPU oracle.
+"""GPU parity: the exact-integer W4A16 kernel (ZLW4I layout, integer MMA) vs the CPU oracle.
 
 The kernel decomposes activations into 16-bit block-floating-point integers per 128-group and accumulates
 q*m exactly in int32, so it must be at least as close to the fp32 oracle as the fp16-MMA path."""

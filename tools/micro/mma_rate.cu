@@ -1,4 +1,4 @@
-// Micro-benchmark: issue rate / latency of legacy mma.sync HMMA.16816 and IMMA.16832 on sm_100a.
+// Micro-benchmark: issue rate / latency of legacy mma.sync fp16 m16n8k16 and integer m16n8k32 on sm_100a.
 // nvcc -gencode arch=compute_100a,code=sm_100a -O3 -o mma_rate mma_rate.cu && ./mma_rate
 #include <cstdio>
 #include <cstdint>
@@ -44,7 +44,7 @@ void run(const char* name, int warps) {
 }
 
 int main() {
-    run<0, 1>("HMMA.16816", 1); run<0, 8>("HMMA.16816", 1); run<0, 4>("HMMA.16816", 4); run<0, 4>("HMMA.16816", 16);
-    run<1, 1>("IMMA.16832", 1); run<1, 8>("IMMA.16832", 1); run<1, 4>("IMMA.16832", 4); run<1, 4>("IMMA.16832", 16);
+    run<0, 1>("fp16 m16n8k16", 1); run<0, 8>("fp16 m16n8k16", 1); run<0, 4>("fp16 m16n8k16", 4); run<0, 4>("fp16 m16n8k16", 16);
+    run<1, 1>("integer m16n8k32", 1); run<1, 8>("integer m16n8k32", 1); run<1, 4>("integer m16n8k32", 4); run<1, 4>("integer m16n8k32", 16);
     return 0;
 }

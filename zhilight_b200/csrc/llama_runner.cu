@@ -25,8 +25,8 @@ using zl::Staged;
 using zl::SlotCache;
 
 struct W4Lin {
-    void* packed = nullptr;     // ZLW4  (fp16 HMMA kernels) -- only kept when some batch size needs it
-    void* packed_i = nullptr;   // ZLW4I (exact-integer IMMA kernel, small M)
+    void* packed = nullptr;     // ZLW4  (fp16 MMA kernels) -- only kept when some batch size needs it
+    void* packed_i = nullptr;   // ZLW4I (exact-integer kernel, small M)
     void* bias = nullptr;
     int N = 0, K = 0;
 };

@@ -39,7 +39,7 @@ struct V2Smem {
 // largest dynamic smem that still lets two CTAs share an SM (227 KB usable, 1 KB reserved per CTA) / one CTA
 constexpr int kV2TwoCtaBudget = 115000;
 constexpr int kV2OneCtaBudget = 231000;
-__host__ __device__ inline int x_row_bytes(int K) { return K * 2 + 64; }   // +64 B: conflict-free LDS.128 across tokens
+__host__ __device__ inline int x_row_bytes(int K) { return K * 2 + 64; }   // +64 B: conflict-free 16-byte shared loads across tokens
 
 template <int NT, bool NORM>
 __device__ __forceinline__ void load_bfrag_v2(uint4 (&b)[NT][4], const W4Params& p, int kbase, int g, int t,

@@ -1,14 +1,14 @@
 // W4A16 skinny GEMM, exact-integer variant (ZLW4I layout): the default for small M.
 //
 // Why: on B200 a decode GEMM must consume ~23 weight bytes per cycle per SM to keep up with HBM.  The classic
-// "dequantise int4 -> fp16 on the CUDA cores, then HMMA" recipe (our v1/v2 kernels, Marlin, the reference's
+// "dequantise int4 -> fp16 on the CUDA cores, then fp16 MMA" recipe (our v1/v2 kernels, Marlin, the reference's
 // GEMV) costs ~10 issue slots per packed word, which makes the kernel ISSUE-bound before it is HBM-bound
 // (profiles/r01b_w4a16_v2.txt: 48 % issue utilisation at 32 % of HBM peak).  Here the int4 weights never
 // become floating point:
 //   * activations are decomposed once per CTA into a block-floating-point integer  x_k = 2^e_g * m_k,
 //     m_k a 16-bit integer per 128-group (error <= 2^-16 of the group maximum, far below fp16's own 2^-11),
 //     split into a signed high byte and an unsigned low byte;
-//   * a packed weight word turns into two IMMA A registers with two LOP3s (w & 0x0f0f0f0f, w & 0xf0f0f0f0 --
+//   * a packed weight word turns into two A registers of an integer MMA with two masks (w & 0x0f0f0f0f, w & 0xf0f0f0f0 --
 //     the odd nibbles stay multiplied by 16 and the factor is folded into that row's scale);
 //   * sum_k q_k * m_k is accumulated EXACTLY in int32 by mma.sync.m16n8k32 (u8 x s8 and u8 x u8), the zero
 //     point is removed with the exact group sum of m, and only then one fp32 multiply by
@@ -58,7 +58,7 @@ struct V3Smem {
     static constexpr int kBytes = kXOff;
 };
 // staged activations (whole K): mc rows of hi bytes, mc rows of lo bytes, then the group table
-__host__ __device__ inline int v3_row_bytes(int K) { return K + 16; }   // +16: conflict-free LDS.128 across tokens
+__host__ __device__ inline int v3_row_bytes(int K) { return K + 16; }   // +16: conflict-free 16-byte shared loads across tokens
 __host__ __device__ inline int v3_stage_bytes(int mc, int K) {
     return 2 * mc * v3_row_bytes(K) + (K / kW4GroupK) * mc * 8;
 }
@@ -144,7 +144,7 @@ __device__ __forceinline__ void pack_blocks(const W4Params& p, const uint8_t* ri
 }
 
 // PACK (mc <= 4): the MMA N dimension (8 columns) is mostly padding at tiny batch, so the two 8-bit digits of the
-// 16-bit activation mantissas share ONE IMMA: column 2i carries token i's high digit, column 2i+1 its low digit, both
+// 16-bit activation mantissas share ONE integer MMA: column 2i carries token i's high digit, column 2i+1 its low digit, both
 // signed (m = 256*hi' + lo', lo' = int8(m & 0xff), hi' = (m + 128) >> 8, |m| <= 2^14).  Half the IMMAs, half the B
 // loads, and the per-group int->float epilogue only touches real tokens.
 template <int NT, bool NORM, int WARPS, int SUBS, int STAGES, int RT = NT * 8, bool PACK = false, int TPX = 0>
@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(WARPS * SUBS * 32, 1) k_w4a16_v3(const W4Param
 
         int i = 0;
         if constexpr (PACK) {
-            // two blocks in flight per warp: their smem loads, IMMA chains and epilogues interleave (the per-block
+            // two blocks in flight per warp: their smem loads, integer MMA chains and epilogues interleave (the per-block
             // dependency chain, not issue slots or HBM, is what a single block per warp leaves exposed)
             for (; i + 2 <= ng; i += 2) {
                 int ss[2], gg[2];

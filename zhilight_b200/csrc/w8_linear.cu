@@ -6,7 +6,7 @@
 // int32 (M,N) round trip through HBM, and three per FP8 Linear (segmented_max_reduction + T_KERNEL_cvt_half_fp8 +
 // cuBLASLt fp8, fp8/fp8_util.cu:58-228).  Here: one activation-quant kernel (per token / per tensor, optionally
 // fused with RMSNorm like layernorm_quant, quant_kernel.cu:106-227) and ONE GEMM kernel that streams the 8-bit
-// weights once from HBM straight into mma.sync fragments (IMMA.16832 s8*s8->s32 / QMMA e4m3->f32) and applies the
+// weights once from HBM straight into mma.sync fragments (m16n8k32, s8*s8->s32 or e4m3*e4m3->f32) and applies the
 // scale-back (+bias) in its epilogue.  HBM-bound: N*K bytes per call.
 //
 // Layout trick (same as dense_gemm.cu): the sum over k is order-free, so lane (g,t) loads 16 CONTIGUOUS bytes of
