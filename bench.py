@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""bench.py -- decode tokens/s of Llama-3.1-8B GPTQ-int4 (g128) on B200, the BASELINE.json metric.
+"""bench.py -- decode tokens/s of Llama-3.1-8B GPTQ-int4 (g128) on B200.
 
     python bench.py --gpus N --steps K --warmup W [--batch B] [--prompt P] [--impl reference] [--model NAME]
 
@@ -17,7 +17,7 @@ architecture in HF-GPTQ layout, synthetic prompt token ids ("data": "synthetic")
           a reported baseline, not a target.
 
 --impl reference times that CPU path as the whole arm (the reference has no CPU implementation of its own;
-SURVEY.md section 8d names this torch dequant path as the side-by-side baseline).
+this torch dequant path is the side-by-side baseline).
 
 N > 1: tensor parallel over the N GPUs of one node (the reference's row/column split), one process per GPU; the
 partial sums of the row-parallel Linears are exchanged with the one-shot NVLink peer-memory all-reduce
@@ -129,7 +129,7 @@ def gptq_shift(kk):
 
 
 class CpuReference:
-    """The CPU baseline (SURVEY.md 8d "reference side-by-side (ii)"): dequantise W4 -> bf16 on every call (what a
+    """The CPU baseline: dequantise W4 -> bf16 on every call (what a
     dequant-to-bf16 path pays), then x @ W^T in torch on the host cores.  One layer's seven linears are materialised; a
     full decode step runs them num_layers times (the packed weights of a layer, 109 MB, do not stay in the CPU caches)
     and the lm_head once.  Inputs are generated outside the timed region."""
@@ -1260,7 +1260,7 @@ def main():
     if tp_parity is not None:
         out["tp_parity"] = tp_parity
 
-    # ---- latency view of the same path (SURVEY 8d): TTFT = chunked prefill of a fresh prompt + first token,
+    # ---- latency view of the same path: TTFT = chunked prefill of a fresh prompt + first token,
     # TPOT = (t_total - TTFT) / (n_out - 1), both wall clock through the host API, p50 over --requests requests ----
     if world == 1 and args.requests > 0:
         n_out = 16

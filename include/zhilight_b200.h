@@ -2,7 +2,7 @@
  * zhilight_b200 -- C-ABI of the B200-native (sm_100a) quantized-decode hot path of ZhiLight.
  *
  * Every entry point replaces one reference operator (cited as file:line under /root/reference).
- * Conventions (SURVEY.md section 8b):
+ * Conventions:
  *   - plain pointers + sizes, no C++/torch types; all data pointers are DEVICE pointers unless
  *     the name ends in _host;
  *   - stream-ordered on `stream`, no allocation, no host sync inside (except zl_llama_* which
@@ -78,7 +78,7 @@ int zl_gptq_dequant_k_major(const uint32_t* qweight_km, const uint8_t* qzeros_km
                             void* out_f16, int N, int K, int group_size, zl_stream_t stream);
 
 /* ------------------------------------------------------------------------------------------ *
- * ZLW4: the B200 tile-packed W4 layout consumed by zl_w4a16_gemm (DESIGN.md section 3).
+ * ZLW4: the B200 tile-packed W4 layout consumed by zl_w4a16_gemm.
  * Built once at load from the reference k-major tensors
  * (Int4GPTQ::preprocess_weight, src/nn/linear/linear.cpp:1139-1160).
  * ------------------------------------------------------------------------------------------ */
@@ -107,7 +107,7 @@ int zl_w4_unpack(const void* packed, uint32_t* qweight_km, uint8_t* qzeros_km, v
 int zl_w4a16_gemm(const void* x, int ldx, const void* packed, const void* bias, const void* residual,
                   void* y, int M, int N, int K, int group_size, int epilogue, int pdl, zl_stream_t stream);
 
-/* The same GEMM with the neighbouring operators of the decode layer folded in (DESIGN.md section 4.1):
+/* The same GEMM with the neighbouring operators of the decode layer folded in:
  *   ln_weight != NULL : nn::LayerNorm (rms, layernorm.cu:9-42) of x is fused into the prologue:
  *                       y = rsqrt(mean(x^2)+eps) * (W . (x*ln_weight)) (+bias);
  *   epilogue ZL_EPI_QKV_ROPE: W is the fused qkv weight packed with zl_qkv_rope_row_map; the epilogue applies

@@ -1,9 +1,9 @@
 #!/usr/bin/env python
 """Run the REFERENCE's own kernels (oracle/_ref/libzl_ref.so, built by oracle/Makefile.ref from /root/reference
 sources, recompiled for sm_100) on the seeded inputs of oracle/golden_cases.py and store their outputs as
-tests/golden/ref_<case>.npz.  TEST INFRASTRUCTURE; needs a GPU (run through gpurun):
+tests/golden/ref_<case>.npz.  TEST INFRASTRUCTURE; needs a GPU:
 
-    python -m oracle.gen_ref_golden gpurun_out/golden      # then copy *.npz into tests/golden/
+    python -m oracle.gen_ref_golden /tmp/golden      # then copy *.npz into tests/golden/
 
 The fixtures are small (a few hundred KB) and are committed together with this script.
 """
@@ -40,7 +40,7 @@ class Ref:
     def p(t):
         return ctypes.c_void_p(t.data_ptr()) if t is not None else None
 
-    # ---- rope tables, Marlin, native AWQ (round 2) ----
+    # ---- rope tables, Marlin, native AWQ ----
     def rope_cos_sin(self, pos, d, theta, llama3=None):
         t = pos.numel()
         cos = torch.empty((t, d), dtype=torch.float32, device=self.dev)
@@ -398,7 +398,7 @@ def main(out_dir, lib_path=None):
 if __name__ == "__main__":
     # usage: gen_ref_golden.py [out_dir] [shim library]   (default: the reference's own kernels, oracle/_ref/libzl_ref.so;
     # oracle/_ref/libzl_dropin.so runs the same calls through integration/zl_nn_dropin.cpp -> libzhilight_b200.so)
-    main(sys.argv[1] if len(sys.argv) > 1 else os.path.join(HERE, "..", "gpurun_out", "golden"),
+    main(sys.argv[1] if len(sys.argv) > 1 else os.path.join(HERE, "_ref", "golden"),
          sys.argv[2] if len(sys.argv) > 2 else None)
     sys.stdout.flush()
     os._exit(0)      # bmengine statics are torn down after the CUDA driver at interpreter exit

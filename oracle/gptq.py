@@ -291,7 +291,7 @@ def gemv_ref_numerics(x, qweight_km, qzeros_km, scales_km, sym=False, bias=None)
 
 
 # ----------------------------------------------------------------------------
-# Synthetic checkpoints (SURVEY.md section 8d config 1 / 3 generators)
+# Synthetic checkpoints (single projections and whole models)
 # ----------------------------------------------------------------------------
 def make_gptq_checkpoint(k, n, group_size=128, sym=False, seed=0, scale_lo=0.005, scale_hi=0.02):
     """HF-GPTQ tensors with uniform random nibbles.  sym=True stores zeros == 7 (-> 8 after +1)."""

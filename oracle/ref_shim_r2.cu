@@ -1,4 +1,4 @@
-// TEST INFRASTRUCTURE (oracle/_ref), round-2 additions to the shim over the REFERENCE's own kernels: RopePreparer,
+// TEST INFRASTRUCTURE (oracle/_ref), further additions to the shim over the REFERENCE's own kernels: RopePreparer,
 // Marlin (repack + gemm), the native AWQ GEMM, the int8-KV cache path, and a timed chain of the reference's default decode
 // kernels for one layer.  Only linked into oracle/_ref/libzl_ref.so (the drop-in library has no counterpart for these).
 #include <bmengine/core/core.h>
@@ -135,7 +135,7 @@ int zlref_awq_gemm(const void* a, const void* qweight /* (K, N/8) */, const void
               Tensor r = nn::awq::awq_gemm(*g_ctx, A, w, s, z, 32); copy_out(r, out))
 }
 
-// ---- the reference's default decode chain for ONE Llama-class GPTQ layer at len_q = 1 (SURVEY.md 9.8 row 2:
+// ---- the reference's default decode chain for ONE Llama-class GPTQ layer at len_q = 1 (
 // no qkv / ff fusion): RMSNorm, 3 GEMVs (q, k, v written into one fused buffer), rope_qk_cache, copy_to_rag_buffer2,
 // multi_query_attention_rag_buffer, o GEMV, element_add_scale, RMSNorm, 2 GEMVs (gate, up), gate_mul_inplace (SiLU), down
 // GEMV, element_add_scale.  (The default build rotates q and k with two KERNEL_rope_with_cache launches instead of the

@@ -7,8 +7,8 @@ oracle/golden_cases.py) are executed twice on the B200:
                                     libzhilight_b200.so (none of the reference's hot-path kernel files is linked),
 
 each in its own process, and the outputs are compared: integer / index work bit-exact, fp16 within the tolerances of
-north_star (1e-3 rel; 2e-3 where the reference itself accumulates 8 products in fp16).  Skipped when the two
-libraries were not built (they need /root/reference at build time; the built files travel to the GPU box)."""
+required tolerance (1e-3 rel; 2e-3 where the reference itself accumulates 8 products in fp16).  Skipped when the two
+libraries were not built (they need /root/reference at build time; the built files serve elsewhere)."""
 import os
 import subprocess
 import sys

@@ -1,6 +1,6 @@
 """`zhilight_b200.layers.Linear` used the way the reference's tests use `zhilight.internals_.layers.Linear`
 (tests/test_linear.py:48-86: same constructor arguments, load_state_dict / named_parameters / forward, same
-tolerances fp16 rtol 1e-3 atol 3e-3, bf16 rtol 1e-2), extended over the quantised QuantTypes of SURVEY 8-a1."""
+tolerances fp16 rtol 1e-3 atol 3e-3, bf16 rtol 1e-2), extended over the quantised QuantTypes."""
 import numpy as np
 import pytest
 import torch

@@ -45,7 +45,7 @@ def _run(cfg, quant, dtype, sym=False, use_pdl=True, use_graph=True, steps=6, ti
 @pytest.mark.parametrize("fuse", [0, 1, 2, 3])
 def test_gptq_decode_matches_oracle(lib, cuda, cfg, sym, fuse):
     for nxt, logits, ref in _run(cfg, 5, "f16", sym=sym, fuse=fuse):
-        # north_star: logits within 1e-3 rel for fp16 -- measured as relative L2 over the vocabulary
+        # required: logits within 1e-3 rel for fp16 -- measured as relative L2 over the vocabulary
         assert rel_l2(logits, ref) <= 2e-3
         for b in range(len(nxt)):
             order = np.argsort(ref[b])
@@ -185,7 +185,7 @@ def test_w8a8_decode_matches_oracle(lib, cuda, quant, dtype, tol):
 
 @pytest.mark.parametrize("cfg", [TINY128, TINY], ids=["d128", "d64-2kvheads"])
 def test_dual_stream_prefill_matches_single_stream(lib, cuda, monkeypatch, cfg):
-    """the two-half / two-stream prefill pipeline (compute stream + reduce stream, events) must produce
+    """The two-half / two-stream prefill pipeline (compute stream + reduce stream, events) must produce
     the same KV state and logits as the single-stream chunked prefill; on one GPU the 'reduce' is the residual add."""
     from zhilight_b200.llama import LlamaDecoder
     sd = omodel.make_state_dict(cfg, 5, 128, False, seed=13)

@@ -1,4 +1,4 @@
-"""Multi-GPU parity (needs >= 2 GPUs on the box; skipped otherwise -- run with `gpurun --gpus 2`):
+"""Multi-GPU parity (needs >= 2 GPUs on the box; skipped otherwise):
 the NVLink one-shot all-reduce / all-gather against exact sums, and a TP=2 decode against the single-GPU oracle."""
 import os
 import socket
@@ -102,7 +102,7 @@ def _worker(rank, ws, port, q):
             dec.close()
             c2.close()
         os.environ.pop("ZL_TP_UNFUSED", None)
-        # TP chunked prefill: with tp_size > 1 the two-half / two-stream pipeline (SURVEY 8-a16) is on by default --
+        # TP chunked prefill: with tp_size > 1 the two-half / two-stream pipeline is on by default --
         # the reduce stream all-reduces one half's partial sums while the compute stream runs the other half
         sd = omodel.make_state_dict(TINY, 5, 128, False, seed=4)
         dec = LlamaDecoder(quant_type=5, max_batch=1, max_seq=96, tp_rank=rank, tp_size=ws, prefill_chunk=32, **TINY)

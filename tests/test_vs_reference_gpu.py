@@ -1,5 +1,5 @@
 """GPU parity against the REFERENCE's own kernels (oracle/_ref/libzl_ref.so: the reference's hot-path .cu files
-recompiled for sm_100 behind a thin shim) on identical device inputs -- north_star: "outputs match the
+recompiled for sm_100 behind a thin shim) on identical device inputs: "outputs match the
 reference's own kernels on identical inputs (bit-exact for GPTQ unpack/index, within 1e-3 rel for fp16)".
 Skipped when the shim library was not built (it needs /root/reference at build time)."""
 import os
@@ -181,7 +181,7 @@ def test_fp8_linear_vs_reference(lib, ref, cuda, dt):
     assert rel_l2(y, y_ref) < (1e-3 if dt == torch.float16 else 4e-3)
 
 
-# ---- round 2: rope tables, Marlin, native AWQ against the reference's own kernels ----
+# ---- rope tables, Marlin, native AWQ against the reference's own kernels ----
 LLAMA3_8 = dict(factor=8.0, low=1.0, high=4.0, orig=8192)
 LLAMA3_32 = dict(factor=32.0, low=1.0, high=4.0, orig=8192)
 

@@ -1,6 +1,6 @@
-"""GPU parity: W4A16 GEMM on the ZLW4 layout vs the CPU oracle (BASELINE.json config 1 shape and others).
+"""GPU parity: W4A16 GEMM on the ZLW4 layout vs the CPU oracle (1 x 4096 x 4096 and other shapes).
 
-Tolerance (north_star): relative L2 error <= 1e-3 against the fp32 oracle for fp16 outputs."""
+Tolerance: relative L2 error <= 1e-3 against the fp32 oracle for fp16 outputs."""
 import numpy as np
 import pytest
 import torch
@@ -27,7 +27,7 @@ def _setup(cuda, k, n, sym, seed, row_map=None):
 
 @pytest.mark.parametrize("sym", [False, True])
 def test_config1_1x4096x4096(lib, cuda, sym):
-    """SURVEY.md 8d config 1: M=1, K=N=4096, g128, seed 0; unpack bit-exact (test_layout) and y rel-err <= 1e-3."""
+    """M=1, K=N=4096, g128, seed 0; unpack bit-exact (test_layout) and y rel-err <= 1e-3."""
     from zhilight_b200 import ops
     k = n = 4096
     w, packed, km = _setup(cuda, k, n, sym, 0)

@@ -3,7 +3,7 @@ a shape is zl_w4_pairs_route's answer; the tests named stream_k assert that it i
 
 Each rounds w = (q - z) * s to fp16 once (what the reference's M > 40 dequant + cuBLASLt route does,
 q_gemm_k_major.cu:843-905, 1083-1100), multiplies fp16 x fp16 exactly and accumulates all of K in fp32 in TMEM.
-Tolerance (north_star): relative L2 <= 1e-3 against the fp32 oracle for fp16 outputs."""
+Tolerance: relative L2 <= 1e-3 against the fp32 oracle for fp16 outputs."""
 import numpy as np
 import pytest
 import torch

@@ -1,4 +1,4 @@
-"""W8A8 Linear through the C-ABI against the oracle.
+"""W8A8 Linear (Int8Linear, Fp8Linear) through the C-ABI against the oracle.
 
 INT8 is integer work with a two-multiply fp32 epilogue: bit-exact.  FP8 quantisation codes are bit-exact; the fp8
 GEMM accumulates in fp32 in a different order than cuBLASLt: <= 1e-3 rel (fp16) like the reference's own Linear

@@ -1,6 +1,6 @@
 #!/usr/bin/env python
 """Isolated timing of the W8A8 Linear kernels (quant + fused GEMM) on Llama-3.1-8B layer shapes, weights rotated
-through > L2 worth of copies; prints JSON lines with GB/s against the W8 algorithmic bytes (SURVEY 8d)."""
+through > L2 worth of copies; prints JSON lines with GB/s against the W8 algorithmic bytes."""
 import json
 import os
 import sys

@@ -74,7 +74,7 @@ def _digest(paths):
 
 
 def build(force=False, verbose=False, family=None):
-    # fast path: the shipped .so already matches the sources (e.g. on the GPU box, where build/ is not shipped)
+    # fast path: the shipped .so already matches the sources (e.g. where only the built library was copied, without build/)
     all_digest = _digest(_sources() + _headers())
     dig_path = LIB_PATH + ".digest"
     if not force and os.path.exists(LIB_PATH) and os.path.exists(dig_path) and open(dig_path).read() == all_digest:

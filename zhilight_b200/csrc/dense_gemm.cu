@@ -4,7 +4,7 @@
 // (src/nn/linear/linear.cpp:150-430 NormalLinear, src/nn/embedding/embedding.cu:353-392).
 // HBM-bound: W is streamed once, straight from global memory into mma.sync A fragments
 // (16-byte non-allocating loads, 4 k-steps in flight per warp); a k-permutation shared by the A and
-// B fragments makes every load a contiguous 16 bytes (see DESIGN.md section 4.2).
+// B fragments makes every load a contiguous 16 bytes.
 #include "gemm_common.cuh"
 
 #include <cstdlib>

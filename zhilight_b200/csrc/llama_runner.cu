@@ -1163,7 +1163,7 @@ int stage_random_linear(zl_llama* m, const std::string& prefix, int K, int N, ui
             ZL_CHECK_LAUNCH();
         }
         RCHECK(stage_random(m, prefix + ".qzeros", G, N / 8, 4, c.sym ? 1 : 0, 0, 0, seed));
-        RCHECK(stage_random(m, prefix + ".scales", G, N, 2, 2, 0.002f, 0.006f, seed));
+        RCHECK(stage_random(m, prefix + ".scales", G, N, 2, 2, 0.002f, 0.006f, seed));   // small scales: activations stay finite
     } else if (c.quant_type == 6) {
         const int G = K / c.group_size;
         RCHECK(stage_random(m, prefix + ".qweight", K, N / 8, 4, 0, 0, 0, seed));
@@ -1335,7 +1335,7 @@ extern "C" int zl_llama_bench_gemms(zl_llama_t* m, int B, int iters, float* ms, 
                 RCHECK(dense_or_w8(m, m->xn, L.d_gu, m->gu, B, pdl));
                 RCHECK(dense_or_w8(m, m->act, L.d_down, m->pend, B, pdl));
                 if (it == 0) {
-                    // weight bytes: 2 per element dense, 1 (+ per-row scale) for W8A8 (SURVEY 8d)
+                    // weight bytes: 2 per element dense, 1 (+ per-row scale) for W8A8
                     const double wb = L.d_qkv.w8 ? 1.0 : 2.0;
                     nbytes += wb * ((double)L.d_qkv.N * D + (double)D * m->hq * d + 2.0 * m->ff * D + (double)D * m->ff) +
                               2.0 * B * (D + L.d_qkv.N + m->hq * d + D + D + 2 * m->ff + m->ff + D);

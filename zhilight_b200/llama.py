@@ -12,14 +12,14 @@ import numpy as np
 from . import _lib
 
 MODEL_PRESETS = {
-    # shapes of the BASELINE.json configs
+    # shapes of the published models
     "llama-3.1-8b": dict(num_layers=32, dim_model=4096, num_heads=32, num_kv_heads=8, dim_head=128, dim_ff=14336,
                          vocab_size=128256, eps=1e-5, rope_theta=500000.0,
                          rope_llama3=dict(factor=8.0, low=1.0, high=4.0, orig=8192.0)),
     "llama-3.2-1b": dict(num_layers=16, dim_model=2048, num_heads=32, num_kv_heads=8, dim_head=64, dim_ff=8192,
                          vocab_size=128256, eps=1e-5, rope_theta=500000.0,
                          rope_llama3=dict(factor=32.0, low=1.0, high=4.0, orig=8192.0)),
-    # north_star TP=8 target and BASELINE config 4 (Qwen2-72B GPTQ: FF padded to 29696 in the GPTQ build,
+    # models for eight GPUs (Qwen2-72B GPTQ: FF padded to 29696 in the GPTQ build,
     # zhilight/config/qwen2_adapter.py:27-28; q/k/v bias, attention.cpp:105-109)
     "llama-3.1-70b": dict(num_layers=80, dim_model=8192, num_heads=64, num_kv_heads=8, dim_head=128, dim_ff=28672,
                           vocab_size=128256, eps=1e-5, rope_theta=500000.0,
