@@ -61,3 +61,32 @@ def test_decoder_raises_at_the_end_of_its_step(lib, cuda, words):
     words[1] = 0x3403
     with pytest.raises(_lib.ZLError, match="0x3403"):
         dec.prefill(0, np.arange(5, dtype=np.int32), 0)
+
+
+_CAPTURE_FIRST = """
+import sys, torch
+sys.path.insert(0, sys.argv[1])
+from zhilight_b200 import ops
+g = torch.Generator(device="cuda").manual_seed(1)
+x, w = (torch.randn(64, 512, generator=g, device="cuda").half(), torch.randn(1024, 512, generator=g, device="cuda").half())
+x8, w8 = x.clamp(-1, 1).mul(127).to(torch.int8), w.clamp(-1, 1).mul(127).to(torch.int8)
+sx, sw = torch.rand(64, generator=g, device="cuda"), torch.rand(1024, generator=g, device="cuda")
+call = lambda: (ops.gemm_nt(x, w), ops.w8a8_gemm(x8, sx, w8, sw, torch.float16))
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    got = call()
+graph.replay()
+torch.cuda.synchronize()
+print(all(torch.equal(a, b) for a, b in zip(got, call())))
+"""
+
+
+def test_first_call_of_a_process_may_be_captured(cuda):
+    """The words are had at the first call; inside a capture that allocation is no part of it."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _CAPTURE_FIRST, root], capture_output=True, text=True, timeout=300)
+    assert r.stdout.split() == ["True"], r.stdout + r.stderr

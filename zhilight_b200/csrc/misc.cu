@@ -21,20 +21,21 @@ extern "C" int zl_version(void) { return 100; }
 // One allocation for the process, visible to every device; it may first be needed inside a stream capture, where an allocation has to
 // be declared as no part of it.
 unsigned* zl::wait_words() {
+    static std::atomic<unsigned*> words{nullptr};
     static std::mutex mu;
-    static unsigned* words = nullptr;
+    if (unsigned* w = words.load(std::memory_order_acquire)) return w;
     std::lock_guard<std::mutex> lock(mu);
-    if (!words) {
+    if (!words.load(std::memory_order_relaxed)) {
         cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
         cudaThreadExchangeStreamCaptureMode(&mode);
         void* p = nullptr;
         if (cudaHostAlloc(&p, zl::kWaitWords * sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
             memset(p, 0, zl::kWaitWords * sizeof(unsigned));
-            words = static_cast<unsigned*>(p);
+            words.store(static_cast<unsigned*>(p), std::memory_order_release);
         }
         cudaThreadExchangeStreamCaptureMode(&mode);
     }
-    return words;
+    return words.load(std::memory_order_relaxed);
 }
 extern "C" void* zl_wait_words(void) { return zl::wait_words(); }
 extern "C" int zl_check_waits(void) {
