@@ -10,6 +10,14 @@ pytestmark = pytest.mark.gpu
 BF, HF = torch.bfloat16, torch.float16
 
 
+def test_which_kernel(lib):
+    """What the sizes below rely on: short sums of few tiles stay with the tile kernel, both sides of the line are tested."""
+    route = lib.zl_gemm_nt_pairs_route
+    assert [route(*s, 1) for s in ((32, 4096, 4096), (33, 128, 64), (257, 512, 200), (64, 100, 4096))] == [0, 0, 0, 0]
+    assert [route(*s, 1) for s in ((33, 128, 576), (64, 136, 584), (257, 513, 576), (777, 2048, 328), (40, 4096, 512))] == [1, 1, 1, 1, 1]
+    assert [route(33, 512, 128, 16), route(300, 512, 128, 16), route(33, 520, 640, 3), route(64, 640, 128, 64)] == [0, 1, 1, 1]
+
+
 def _rand(g, *shape, dtype):
     return torch.randn(*shape, generator=g).to(dtype).cuda()
 
@@ -32,7 +40,7 @@ def no_wait_gave_up(lib, cuda):
 
 @pytest.mark.parametrize("dtype,out", [(BF, BF), (BF, torch.float32), (HF, HF), (HF, torch.float32)])
 @pytest.mark.parametrize("m,n,k", [(33, 128, 64), (64, 136, 72), (65, 250, 136), (256, 256, 128), (257, 513, 448), (300, 520, 1000), (40, 4096, 512),
-                                   (777, 2048, 328)])
+                                   (777, 2048, 328), (33, 128, 576), (64, 136, 584), (65, 250, 648), (256, 256, 640), (257, 513, 576)])
 def test_plain(lib, cuda, dtype, out, m, n, k):
     from zhilight_b200 import ops
     g = torch.Generator().manual_seed(m + n)
@@ -57,7 +65,7 @@ def test_skinny_entry_with_bias_and_activations(lib, cuda, dtype, m, n, k):
         assert float((y.double() - want).norm() / want.norm()) < 1e-5, act
 
 
-@pytest.mark.parametrize("m,n,k", [(40, 130, 64), (257, 512, 200)])
+@pytest.mark.parametrize("m,n,k", [(40, 130, 64), (257, 512, 200), (40, 130, 576), (257, 512, 648)])
 def test_epilogues(lib, cuda, m, n, k):
     from zhilight_b200 import ops
     g = torch.Generator().manual_seed(n)
@@ -76,7 +84,7 @@ def test_epilogues(lib, cuda, m, n, k):
     assert rel(ops.gemm_nt_glu_clamp(x, w, None, f32, 1.5, 1.7, 0.5), ga * torch.sigmoid(1.7 * ga) * (cu + 0.5)) < 1e-5
 
 
-@pytest.mark.parametrize("b,m,n,k", [(3, 70, 128, 64), (5, 33, 300, 128), (90, 40, 512, 64)])
+@pytest.mark.parametrize("b,m,n,k", [(3, 70, 128, 64), (5, 33, 300, 128), (90, 40, 512, 64), (3, 70, 128, 576), (5, 33, 300, 640)])
 def test_batches(lib, cuda, b, m, n, k):
     from zhilight_b200 import ops
     g = torch.Generator().manual_seed(b)
@@ -111,10 +119,11 @@ def test_grouped(lib, cuda, dtype, sizes, n, k):
     _close(ops.gemm_nt_grouped(x, w, off, total, x_rows=rows), ref, mag, k, dtype)
 
 
-def test_infinities_stay_in_their_rows_and_columns(lib, cuda):
+@pytest.mark.parametrize("k", [128, 640])
+def test_infinities_stay_in_their_rows_and_columns(lib, cuda, k):
     from zhilight_b200 import ops
     g = torch.Generator().manual_seed(1)
-    x, w = _rand(g, 70, 128, dtype=BF), _rand(g, 256, 128, dtype=BF)
+    x, w = _rand(g, 70, k, dtype=BF), _rand(g, 256, k, dtype=BF)
     good = ops.gemm_nt(x, w, out_dtype=torch.float32)
     x[69, 3], w[17, 5] = float("inf"), float("nan")
     bad = ops.gemm_nt(x, w, out_dtype=torch.float32)
@@ -133,7 +142,7 @@ def _nt(lib, x, xb, ldx, w, wb, ldw, y, yb, ldy, m, n, k, batch, epilogue=0, gat
 
 @pytest.mark.parametrize("dtype", [BF, HF])
 @pytest.mark.parametrize("t", [33, 64, 300])
-@pytest.mark.parametrize("h,d,r,rs", [(16, 128, 512, 512), (5, 128, 512, 576), (3, 192, 136, 140)])
+@pytest.mark.parametrize("h,d,r,rs", [(16, 128, 512, 512), (5, 128, 512, 576), (3, 192, 136, 140), (3, 640, 520, 576), (64, 128, 640, 640)])
 def test_heads_as_the_batch(lib, cuda, dtype, t, h, d, r, rs):
     """The latent layers' products: pitch between heads smaller than the row pitch, for x and y; y's rows longer than its columns; the
     way back with a gate that is part of a wider row."""
@@ -155,11 +164,12 @@ def test_heads_as_the_batch(lib, cuda, dtype, t, h, d, r, rs):
         _close(out, prod(lat, uv) * s, prod(lat.abs(), uv.abs()) * s * 1.01, r + 64, dtype)   # + 64: a few units of fp32 for the sigmoid
 
 
-@pytest.mark.parametrize("ldx,ldw,ldy,pad", [(136, 128, 200, 0), (1024, 520, 130, 1), (128, 128, 129, 3)])
-def test_row_pitches_and_odd_distances(lib, cuda, ldx, ldw, ldy, pad):
+@pytest.mark.parametrize("k", [128, 576])
+@pytest.mark.parametrize("ldx,ldw,ldy,pad", [(8, 0, 200, 0), (896, 392, 130, 1), (0, 0, 129, 3)])
+def test_row_pitches_and_odd_distances(lib, cuda, k, ldx, ldw, ldy, pad):
     """Rows apart from each other; an output whose rows, matrices and base are no multiples of two values (narrow stores)."""
     g = torch.Generator().manual_seed(ldx)
-    b, m, n, k = 3, 45, 128, 128
+    b, m, n, ldx, ldw = 3, 45, 128, k + ldx, k + ldw
     x, w = _rand(g, b, m, ldx, dtype=BF), _rand(g, b, n, ldw, dtype=BF)
     flat = torch.full((pad + b * (m * ldy + pad),), -7.0, dtype=BF, device=cuda)
     y = flat[pad:]

@@ -72,6 +72,8 @@ __device__ __forceinline__ float gemm_epilogue(float v, const GemmP& p, int b, i
 // tcgen05 kernel for 16-bit inputs (gemm_tc.cu): whether it is the faster one for the call, and its launch.  cudaErrorNotSupported:
 // nothing was launched, since no tensor map of these pitches could be made; the kernels it stands beside take any.
 bool gemm_tc_route(const GemmP& p, int batch, int in_dtype);
+// whether gemm_tiled.cu's tile kernel is faster at that
+bool gemm_tile_faster(int M, int N, int K, int batch);
 cudaError_t launch_gemm_tc(const GemmP& p, int batch, int in_dtype, int out_dtype, int epilogue, bool pdl, cudaStream_t stream);
 
 }  // namespace zl

@@ -439,6 +439,24 @@ static int gt_pick_ntok(int M, long long rows, int pairs) {
     return best;
 }
 
+// A short K and few tiles are the tile kernel's: a launch of it costs 2.9 us and 1 us per 100 of k, here the pair's allocation, barriers and
+// hand-overs cost 5 us and k a quarter of that.  Both times in us, fitted to 566 measured shapes (M = 33 .. 512, N = 128 .. 4096, K = 64 .. 8192,
+// 1 .. 64 matrices; above K = 512 this kernel was the faster one at all of them): the tile kernel's first wave of 64 x 64 blocks and what
+// each further block's rows cost; here the tile's rows and what a further wave of pairs costs.  Measured, tile kernel / here, M x N x K: 33 x 128 x 64
+// 2.7 / 5.3; 256 x 2048 x 256 5.7 / 6.5; 128 x 512 x 384 7.0 / 6.5; 16 matrices of 33 x 512 x 128 3.8 / 6.0, of 300 x 512 x 128 11.1 / 9.1; 48 of
+// 64 x 1024 x 128 12.7 / 10.7, of 33 x 1024 x 128 9.2 / 9.9.  At no measured shape does the choice cost more than 3 % of the tile kernel's time.
+bool gemm_tile_faster(int M, int N, int K, int batch) {
+    if (K > 512) return false;
+    const int sms = device_sm_count(), pairs = sms / 2;
+    const long long blocks = (long long)batch * cdiv(M, 64) * cdiv(N, 64), rows = (long long)batch * cdiv(N, kTc2Rows);
+    const double further = blocks > sms ? (double)(blocks - sms) * M / (64.0 * cdiv(M, 64)) : 0.0;
+    const int n = gt_pick_ntok(M, rows, pairs);
+    const double waves = (double)((rows * cdiv(M, n) + pairs - 1) / pairs - 1);
+    const double tile = 2.93 + 0.01046 * K + further * (0.00902 + 2.84e-5 * K);
+    const double here = 4.84 + 0.00246 * K + 0.025 * n + waves * (0.205 + 0.0232 * n + 0.001 * K);
+    return tile < here;
+}
+
 bool gemm_tc_route(const GemmP& p, int batch, int in_dtype) {
     if (in_dtype != ZL_F16 && in_dtype != ZL_BF16) return false;
     // 16-byte aligned bases and pitches (tensor-TMA, cp.async), extents below 2^31

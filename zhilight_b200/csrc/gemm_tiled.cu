@@ -504,8 +504,10 @@ static int gemm_dispatch(GemmP p, int batch, int in_dtype, int out_dtype, int ep
     // a decode step's experts: a handful of rows per group
     const bool few_rows = grouped && in_dtype != ZL_F32 && M <= grouped_small_max() && vx && vw && K % 8 == 0 && (size_t)8 * K * 2 <= 160 * 1024 &&
                           (epilogue == ZL_GEMM_EPI_NONE || epilogue == ZL_GEMM_EPI_RELU2 || pairs);
-    cudaError_t e = !few_rows && gemm_tc_route(p, batch, in_dtype) ? launch_gemm_tc(p, batch, in_dtype, out_dtype, epilogue, pdl != 0, stream)
-                                                      : cudaErrorNotSupported;
+    // (the estimate is of aligned rows: others cost the tile kernel more)
+    const bool tiles = few_rows || (!grouped && vx && vw && K % 8 == 0 && gemm_tile_faster(M, N, K, batch));
+    cudaError_t e = !tiles && gemm_tc_route(p, batch, in_dtype) ? launch_gemm_tc(p, batch, in_dtype, out_dtype, epilogue, pdl != 0, stream)
+                                                                : cudaErrorNotSupported;
     if (e != cudaErrorNotSupported) {
         ZL_CHECK_CUDA(e);
         return ZL_OK;
@@ -575,6 +577,16 @@ static int gemm_dispatch(GemmP p, int batch, int in_dtype, int out_dtype, int ep
     }
     ZL_CHECK_CUDA(e);
     return ZL_OK;
+}
+
+extern "C" int zl_gemm_nt_pairs_route(int M, int N, int K, int batch) {
+    GemmP p{};
+    p.M = M;
+    p.N = N;
+    p.K = K;
+    p.ldx = p.ldw = cdiv(K, 8) * 8;
+    p.xb = p.wb = 8;
+    return M > 0 && N > 0 && K > 0 && batch > 0 && !(K % 8 == 0 && gemm_tile_faster(M, N, K, batch)) && gemm_tc_route(p, batch, ZL_BF16) ? 1 : 0;
 }
 
 extern "C" int zl_gemm_nt(const void* x, long long ldx, long long x_batch_stride, const void* w, long long ldw,
