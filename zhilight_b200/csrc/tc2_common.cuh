@@ -41,10 +41,7 @@ __device__ __forceinline__ bool tc2_wait(uint64_t* bar, uint32_t parity, volatil
             unsigned spins = 0;
             while (!(ok = mbar_try_wait(bar, parity))) {
                 if ((++spins & 1023u) == 0 && (*s_abort || clock64() - t0 > 2000000000ll)) {
-                    if (!*s_abort) {
-                        *reinterpret_cast<volatile unsigned*>(err) = code;   // host memory
-                        __threadfence_system();
-                    }
+                    if (!*s_abort) *reinterpret_cast<volatile unsigned*>(err) = code;   // host memory: there when the kernel has ended
                     *s_abort = 1;
                     break;
                 }
