@@ -97,15 +97,11 @@ def test_strided_activations(lib, cuda):
     assert rel_l2(y, gptq.gemm_f32(x.cpu().numpy(), w)) <= TOL
 
 
-def test_predecessor_that_takes_longer_than_a_wait_may(lib, cuda):
-    """Launched behind kernels that let their dependents start at once and then run for 1.6 s, more than the 2e9 cycles after which a
-    wait inside the GEMM gives up: its waits begin when they have ended.  (One block reads a long row, as often as that takes; each of the launches
-    is resident and waits for the one before.)"""
+def behind_slow_predecessors(cuda, ms, call):
+    """Runs `call` behind kernels that let their dependents start at once and take `ms` together: one block reads a long row, as often as
+    that takes; each of the launches is resident and waits for the one before."""
     from zhilight_b200 import _lib, ops
-    k, n, m, long_row = 4096, 512, 300, 1 << 30
-    w, packed = _setup(cuda, k, n, False, 5)
-    x = _x(m, k, 1).to(cuda)
-    want = ops.w4a16_gemm_fused(x, packed, n, k, variant=1)
+    long_row = 1 << 30
     row = torch.full((1, long_row), 0.5, dtype=torch.float16, device=cuda)
     q, scale = torch.empty(long_row, dtype=torch.int8, device=cuda), torch.empty(1, device=cuda)
     stream = torch.cuda.current_stream().cuda_stream
@@ -117,14 +113,25 @@ def test_predecessor_that_takes_longer_than_a_wait_may(lib, cuda):
     slow()
     end.record()
     torch.cuda.synchronize()
-    times = int(1600 / begin.elapsed_time(end)) + 1
+    times = int(ms / begin.elapsed_time(end)) + 1
     assert times <= 100                                 # resident at one time: the hardware's limit is 128
-    got = torch.full_like(want, float("nan"))
     begin.record()
     for _ in range(times):
         slow()
-    ops.w4a16_gemm_fused(x, packed, n, k, variant=1, out=got, pdl=True)
+    call()
     end.record()
     torch.cuda.synchronize()
-    assert begin.elapsed_time(end) > 1400
+    return begin.elapsed_time(end)
+
+
+def test_predecessor_that_takes_longer_than_a_wait_may(lib, cuda):
+    """Longer than the 2e9 cycles after which a wait inside the GEMM gives up: its waits begin when the predecessor has ended."""
+    from zhilight_b200 import ops
+    k, n, m = 4096, 512, 300
+    w, packed = _setup(cuda, k, n, False, 5)
+    x = _x(m, k, 1).to(cuda)
+    want = ops.w4a16_gemm_fused(x, packed, n, k, variant=1)
+    got = torch.full_like(want, float("nan"))
+    took = behind_slow_predecessors(cuda, 1600, lambda: ops.w4a16_gemm_fused(x, packed, n, k, variant=1, out=got, pdl=True))
+    assert took > 1400
     assert torch.equal(got, want)

@@ -222,3 +222,18 @@ def test_stream_k_qkv_rope_epilogue(lib, cuda, t):
     hq, hkv, d, k = 32, 8, 128, 4096
     assert lib.zl_w4_pairs_route(t, (hq + 2 * hkv) * d, k) == 0
     test_qkv_rope_epilogue(lib, cuda, lib.zl_w4_tc_set_splits, d, hq, hkv, k, t, 0)
+
+
+@pytest.mark.parametrize("m,k,n", [(4, 14336, 512), (32, 4096, 6144), (100, 8192, 384), (200, 8192, 384)])
+def test_stream_k_starts_ahead_of_its_predecessor(lib, cuda, m, k, n):
+    """Weights are fetched and converted while the predecessor still runs; the result is that of a launch behind it."""
+    from tests.test_w4a16_tc2_gpu import behind_slow_predecessors
+    from zhilight_b200 import ops
+    assert lib.zl_w4_int_layout_route(m, n, k) == 4 and lib.zl_w4_pairs_route(m, n, k) == 0
+    _, packed = _setup(cuda, k, n, False, 5)
+    x = torch.randn(m, k, generator=torch.Generator().manual_seed(m)).half().to(cuda)
+    want = ops.w4a16_gemm_fused(x, packed, n, k, variant=1)
+    got = torch.full_like(want, float("nan"))
+    behind_slow_predecessors(cuda, 100, lambda: ops.w4a16_gemm_fused(x, packed, n, k, variant=1, out=got, pdl=True))
+    assert torch.equal(got, want)
+    _check_watchdog(lib)

@@ -33,6 +33,9 @@
 // quarter-warp read 16-byte chunks 64 B apart -- a 4-way bank conflict in the plain record layout -- so the nibble words
 // arrive through a tensor map with 64-byte swizzle (chunk ^= (row >> 1) & 3): conflict-free, the HBM format is unchanged.
 // The 80-byte scale / zero trailers of the four records of a stage come through a second (unswizzled) map.
+//
+// Ahead of the launch dependency the producer fetches RS + AS stages and the groups convert the first AS, which wait for weights alone; every
+// bounded wait that ends only after x has come begins behind it, however long the predecessor (an all-reduce with a late rank) takes.
 #include "w4a16_tc.cuh"
 
 #include <cstdlib>
@@ -198,6 +201,7 @@ __global__ void __launch_bounds__(TsCfg<NTOK>::kThreads, 1) k_w4a16_ts(const __g
             sch.seg(si, tile, g0, g1);
             for (int gi = g0; gi < g1; gi += KG, ++st_i) {
                 const int ng = min(KG, g1 - gi);
+                if (st_i == C::RS + C::AS) pdl_wait();   // the groups free the first AS slots whether x has come or not
                 mbar_wait_wd(&raw_empty[rs], ph ^ 1u, p.err, 0x100 + rs);
                 if (lane == 0) stamp(0, st_i, 1);
                 if (tc_elect_one()) {
@@ -258,6 +262,7 @@ __global__ void __launch_bounds__(TsCfg<NTOK>::kThreads, 1) k_w4a16_ts(const __g
     } else if (warp == C::kWarpMma) {
         // ---------------- MMA issue: the warp stays converged (uniform operands), one elected lane issues ----------------
         constexpr uint32_t idesc = tc_idesc_f16(NTOK);
+        pdl_wait();
         int as = 0, acc = 0, st_i = 0;
         uint32_t ph = 0, acc_ph = 0;
         for (int si = 0; si < sch.n_segs; ++si) {
@@ -318,6 +323,7 @@ __global__ void __launch_bounds__(TsCfg<NTOK>::kThreads, 1) k_w4a16_ts(const __g
             sch.seg(si, tile, g0, g1);
             for (int gi = g0; gi < g1; gi += KG, ++st_i) {
                 if (st_i % NG != grp) continue;
+                if (st_i >= C::AS && st_i < C::AS + NG) pdl_wait();
                 const int ng = min(KG, g1 - gi);
                 const int rs = st_i % C::RS, as = st_i % C::AS;
                 const uint32_t rph = (uint32_t)(st_i / C::RS) & 1u, aph = (uint32_t)(st_i / C::AS) & 1u;
