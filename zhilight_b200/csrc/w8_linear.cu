@@ -476,7 +476,7 @@ extern "C" int zl_fp8_quant_per_tensor(const void* x, void* q, float* scale, siz
     ZL_CHECK_ARG(x && q && scale && n > 0);
     ZL_CHECK_ARG(dtype == ZL_F16 || dtype == ZL_BF16);
     ZL_CHECK_SUPPORTED(n % 8 == 0);
-    ZL_CHECK_SUPPORTED(n <= ((size_t)1 << 22));
+    ZL_CHECK_SUPPORTED(n <= ((size_t)1 << 22));   // the range this entry point has always had; the kernels below know no such limit
     const cudaError_t e = dtype == ZL_F16 ? launch_fp8_quant(static_cast<const __half*>(x), static_cast<uint8_t*>(q), scale, n, pdl != 0, stream)
                                           : launch_fp8_quant(static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), scale, n, pdl != 0, stream);
     ZL_CHECK_CUDA(e);
@@ -502,6 +502,8 @@ extern "C" int zl_int8_scale_back(const int32_t* acc, const float* x_scale, cons
 // Whether M rows go to the kernel on pairs of SMs (gemm_tc.cu), which costs the same from 1 row to 128; the mma.sync kernel reads the
 // weights once per 32 rows and its activations once per 16 weight rows.  us, here against mma.sync (int8 / fp8):
 //   M = 64      4096 x 4096 19 against 24; 4096 x 14336 26 / 31
+//   M = 33      no slower than the split-k kernel that served it before, from 1088 x 512 (6.0 against 6.7 / 6.0) and 256 x 1024 (6.7
+//               against 7.9 / 7.0) up to 14336 x 1024 (9.5 / 9.0 against 9.7 / 9.0)
 //   M = 32      8192 x 8192 23 against 34 / 46; 14336 x 4096 19 / 33 / 44; 4096 x 14336 27 / 29 / 37; 4096 x 4096 19 / 15 / 17
 //   M = 16      8192 x 8192 23 / 25 / 35; 14336 x 4096 19 / 25 / 33; 4096 x 14336 27 / 21 / 29
 //   M = 8       8192 x 8192 23 / 20 / 21; 28672 x 8192 48 / 60 / 62
