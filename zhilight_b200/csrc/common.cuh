@@ -55,7 +55,7 @@ namespace zl {
 constexpr int kWarp = 32;
 
 // The words that kernels write when a bounded wait gives up, one for each kernel that returns then instead of trapping: pinned host memory,
-// so that a host thread which has synchronised anyway reads them without a copy.  nullptr: no memory.
+// so that a host thread which has synchronised anyway reads them without a copy; those of the current device.  nullptr: no memory.
 enum { kWaitGemmTc = 0, kWaitW4Pairs = 1, kWaitWords = 2 };
 unsigned* wait_words();   // misc.cu
 

@@ -18,9 +18,11 @@ extern "C" void zl_set_last_error(const char* file, int line, const char* msg) {
 extern "C" const char* zl_last_error(void) { return g_last_error; }
 extern "C" int zl_version(void) { return 100; }
 
-// One allocation for the process, visible to every device; it may first be needed inside a stream capture, where an allocation has to
-// be declared as no part of it.
-unsigned* zl::wait_words() {
+// One allocation for the process, visible to every device, with words of its own for each: a host thread per device hears of its own.  It
+// may first be needed inside a stream capture, where an allocation has to be declared as no part of it.
+constexpr int kWaitDevices = 64;
+static unsigned* all_wait_words() {
+    constexpr size_t kWaitBytes = kWaitDevices * zl::kWaitWords * sizeof(unsigned);
     static std::atomic<unsigned*> words{nullptr};
     static std::mutex mu;
     if (unsigned* w = words.load(std::memory_order_acquire)) return w;
@@ -29,13 +31,21 @@ unsigned* zl::wait_words() {
         cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
         cudaThreadExchangeStreamCaptureMode(&mode);
         void* p = nullptr;
-        if (cudaHostAlloc(&p, zl::kWaitWords * sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
-            memset(p, 0, zl::kWaitWords * sizeof(unsigned));
+        if (cudaHostAlloc(&p, kWaitBytes, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+            memset(p, 0, kWaitBytes);
             words.store(static_cast<unsigned*>(p), std::memory_order_release);
+        } else {
+            cudaGetLastError();   // the caller says what it lacks
         }
         cudaThreadExchangeStreamCaptureMode(&mode);
     }
     return words.load(std::memory_order_relaxed);
+}
+unsigned* zl::wait_words() {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    unsigned* all = all_wait_words();
+    return all ? all + (dev >= 0 && dev < kWaitDevices ? dev : 0) * zl::kWaitWords : nullptr;
 }
 extern "C" void* zl_wait_words(void) { return zl::wait_words(); }
 extern "C" int zl_check_waits(void) {
