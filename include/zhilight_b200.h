@@ -149,15 +149,16 @@ int zl_w4_pairs_route(int M, int N, int K);
 /* last watchdog code published by the 4-bit stream-k kernel on the current device (0 = none); a bounded mbarrier wait that expires
  * records which pipeline barrier starved and traps instead of hanging the GPU. */
 unsigned zl_w4_tc_watchdog(void);
-/* The kernels over pairs of SMs do not trap: a wait that expires leaves a code in host memory and the kernel returns with its output
+/* The kernels over pairs of SMs and the attention of prompt portions do not trap: a wait that expires leaves a code in host memory and the kernel returns with its output
  * incomplete.  zl_check_waits, called after a synchronisation, is ZL_OK, or ZL_ERR_CUDA once for each kernel that has left a code on
- * the current device since it was last reported; zl_last_error names it.  The decoders ask at the end of every step, the GEMMs at each call. */
+ * the current device since it was last reported; zl_last_error names it.  The decoders ask at the end of every step, the GEMMs
+ * and zl_decode_attention with prompt portions at each call. */
 int zl_check_waits(void);
 /* the unreported code of the general tensor-core GEMM (zl_gemm_nt*, zl_dense_gemm_skinny* and zl_w8a8_gemm with prompt-sized M) and of
  * the 4-bit GEMM over pairs of SMs, after a synchronisation of the device; 0 = none */
 unsigned zl_gemm_tc_watchdog(void);
 unsigned zl_w4_tc2_watchdog(void);
-/* tests: the two codes of the current device, in this order (host memory; NULL: none could be had) */
+/* tests: the codes of the current device, these two and that of the attention (host memory; NULL: none could be had) */
 void* zl_wait_words(void);
 /* debug / tests: at least `splits` pieces per weight-row tile in the tcgen05 kernel's stream-k schedule (0 = automatic; also
  * ZL_TC_SPLITS). */

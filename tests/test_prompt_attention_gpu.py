@@ -1,5 +1,5 @@
 """GPU: attention of several query rows per task (portions of a prompt, tree rows) against the oracle, at the edges of the kernel's
-64-row blocks and 64-key tiles, with masks of any shape, key splits and both cache layouts."""
+128-row blocks and 64-key tiles, with masks of any shape, key splits and both cache layouts."""
 import numpy as np
 import pytest
 import torch
@@ -86,3 +86,47 @@ def test_infinities_and_nans_stay_in_their_rows(lib, cuda):
     keep = torch.ones(320, 4, dtype=torch.bool, device=cuda)
     keep[3, 1] = keep[9, 2] = False
     assert torch.equal(bad[0][keep], good[0][keep])
+
+
+def _exact(q, k, v, visible, scale):
+    """q (m, h, d), k and v (n, hk, d), visible (m, n) in 64 bits on the CPU"""
+    m, h, d = q.shape
+    g = h // k.shape[1]
+    s = torch.einsum("mhd,nhd->hmn", q.double(), k.double().repeat_interleave(g, 1)) * scale
+    s = s.masked_fill(visible[None] == 0, -torch.inf)
+    return torch.einsum("hmn,nhd->mhd", torch.softmax(s, -1), v.double().repeat_interleave(g, 1))
+
+
+@pytest.mark.parametrize("dtype", list(TOL))
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("rise", [0.02, 0.5])
+def test_maxima_that_grow_along_the_keys(lib, cuda, dtype, d, rise):
+    """Scores that rise by rise / ln 2 bits a key (the output is a mean over the last keys a row sees): a row's reference maximum has to follow,
+    now by less than the kernel lets it stay behind, now in every tile."""
+    from zhilight_b200 import ops
+    g = torch.Generator().manual_seed(5)
+    m, n, h = 192, 640, 8
+    q, k, v = (torch.randn(*s, generator=g) for s in ((m, h, d), (n, 2, d), (n, 2, d)))
+    q[:, :, 0], k[:, :, 0] = 4.0, (torch.arange(n) * (rise * d ** 0.5 / 4)).round(decimals=2)[:, None]
+    q, k, v = q.to(dtype), k.to(dtype), v.to(dtype)
+    mask = _causal(m, n)
+    out = ops.decode_attention(q[None].to(cuda), torch.tensor([n], dtype=torch.int32, device=cuda), [k.to(cuda)], [v.to(cuda)], mask.to(cuda), d ** -0.5,
+                               n, 2)[0]
+    assert rel_l2(out.double().cpu().numpy(), _exact(q, k, v, mask, d ** -0.5).numpy()) <= TOL[dtype][1]
+
+
+@pytest.mark.parametrize("hq,hkv,d,len_q,ctx", [(1, 1, 128, 127, 513), (1, 1, 128, 128, 512), (1, 1, 128, 129, 511), (3, 1, 64, 341, 1025),
+                                                (8, 8, 128, 130, 130), (16, 2, 128, 50, 2100), (64, 8, 128, 33, 700), (32, 8, 64, 257, 1400)])
+def test_blocks_of_rows_and_clusters_of_splits(lib, cuda, hq, hkv, d, len_q, ctx):
+    """A row more or less than a block, keys in one to eight parts, q on 4 bytes, a negative scale and one of zero."""
+    from zhilight_b200 import ops
+    g = torch.Generator().manual_seed(6)
+    q, k, v = (torch.randn(*s, generator=g).bfloat16() for s in ((len_q, hq, d), (ctx, hkv, d), (ctx, hkv, d)))
+    room = torch.empty(q.numel() + 2, dtype=q.dtype, device=cuda)
+    shifted = room[2:].view(1, len_q, hq, d)
+    shifted.copy_(q)
+    mask, lens = _causal(len_q, ctx), torch.tensor([ctx], dtype=torch.int32, device=cuda)
+    for qd in (q[None].to(cuda), shifted):
+        for scale in (d ** -0.5, -d ** -0.5, 0.0):
+            out = ops.decode_attention(qd, lens, [k.to(cuda)], [v.to(cuda)], mask.to(cuda), scale, ctx, hkv)[0]
+            assert rel_l2(out.double().cpu().numpy(), _exact(q, k, v, mask, scale).numpy()) <= TOL[torch.bfloat16][1], (qd is shifted, scale)

@@ -56,7 +56,7 @@ constexpr int kWarp = 32;
 
 // The words that kernels write when a bounded wait gives up, one for each kernel that returns then instead of trapping: pinned host memory,
 // so that a host thread which has synchronised anyway reads them without a copy; those of the current device.  nullptr: no memory.
-enum { kWaitGemmTc = 0, kWaitW4Pairs = 1, kWaitWords = 2 };
+enum { kWaitGemmTc = 0, kWaitW4Pairs = 1, kWaitAttnPrompt = 2, kWaitWords = 3 };
 unsigned* wait_words();   // misc.cu
 
 __host__ __device__ inline int cdiv(int a, int b) { return (a + b - 1) / b; }

@@ -374,18 +374,19 @@ static size_t prompt_head_bytes(int B, int len_q, int max_len_buf, const int8_t*
     const size_t q_rows = (size_t)B * len_q;
     return mask ? (q_rows * cdiv(max_len_buf, kPaKeys) * 8 + 15) / 16 * 16 + (q_rows * 4 + 15) / 16 * 16 : 0;
 }
-// Which kernel serves several query rows.  The decode kernels read K and V once per query row and stay at their latency (12 - 17 us)
-// while these reads fit one wave; the prompt kernel reads them once per 64 (query, head) rows and has a mask pass and a longer
-// chain (14 - 23 us).  Measured in 256-key CTAs of the decode kernels, D = 128: 8 heads on 1, 1100 keys: 120 CTAs 16.7 against
-// 20.9 us, 160 CTAs 23.3 against 20.8; 32 heads on 8, 1100 keys: 160 CTAs 20.9 against 21.9, 240 CTAs 21.1 against 20.1, 20480 CTAs
-// 287 against 45; 16 on 8: 640 CTAs 20.9 against 21.4, 960 CTAs 22.9 against 21.9.  Halving the head's width halves the reads but
-// not the chain: D = 64, 32 on 8, 1100 keys: 1280 CTAs 19.8 against 20.9; 16 on 16: 1280 CTAs 18.9 against 19.9, 2048 CTAs 17.4
-// against 15.4.  The mask's bits live in the workspace, so a masked call without room for them keeps the decode kernels.
+// Which kernel serves several query rows.  The decode kernels read K and V once per query row and stay at their latency while these reads
+// fit one wave; the prompt kernel reads them once per 128 (query, head) rows and has a mask pass and a longer chain.  Measured in 256-key
+// CTAs of the decode kernels, all launches of a call, decode against prompt kernel in us, D = 128, 1100 keys: 32 heads on 8, 80 CTAs 12.1
+// against 15.3, 160 CTAs 18.0 against 15.6; 64 on 8, 160 CTAs 21.4 against 15.6; 16 on 8, 160 CTAs 17.0 against 15.6; 8 on 8, 360 CTAs
+// 22.7 against 15.6; 300 keys, 144 CTAs 11.6 against 14.8.  D = 64 halves the reads but not the chain: 32 on 8, 160 CTAs 12.3
+// against 12.6, 256 CTAs (32 rows alone) 6.0 against 8.0, 360 CTAs 16.2 against 12.8; 12 on 4, 320 CTAs 15.6 against 12.7; one head per
+// kv head: 16 on 16, 720 CTAs 13.7 against 15.0, 1024 CTAs 8.2 against 8.4, 1280 CTAs 17.4 against 15.2.  The mask's bits live in the
+// workspace, so a masked call without room for them keeps the decode kernels.
 static bool prompt_route(int len_q, int m_query, int dim_head, int B, int num_kv_heads, const int8_t* mask, int max_len_buf, const void* out,
                          const void* workspace, size_t workspace_bytes) {
     if (len_q < 2 || num_kv_heads > 65535 || B > 65535 / 16) return false;
     const long long ctas = (long long)B * len_q * num_kv_heads * cdiv(m_query, 8) * cdiv(max_len_buf, 256);
-    const long long line = dim_head == 64 ? 1536 : m_query >= 4 ? 192 : 768;
+    const long long line = dim_head == 128 ? 150 : m_query > 1 ? 300 : 1000;
     if (ctas < line) return false;
     if ((reinterpret_cast<uintptr_t>(out) & 3) || (reinterpret_cast<uintptr_t>(workspace) & 15)) return false;
     return !mask || (workspace && prompt_head_bytes(B, len_q, max_len_buf, mask) <= workspace_bytes && len_q <= 65535);
@@ -397,33 +398,27 @@ static int prompt_attention(const void* q, const int32_t* buf_lens, void* const*
                             size_t workspace_bytes, int pdl, zl_stream_t stream) {
     const int m_query = num_heads / num_kv_heads;
     const int blocks = cdiv(len_q * m_query, kPaRows), tiles = cdiv(max_len_buf, kPaKeys);
-    int splits = workspace ? prompt_attn_splits((long long)blocks * num_kv_heads * B, tiles) : 1;
-    const size_t q_rows = (size_t)B * len_q, vheads = q_rows * num_heads;
-    const size_t head_bytes = prompt_head_bytes(B, len_q, max_len_buf, mask);
-    if (splits > 1 && head_bytes + vheads * splits * (D + 2) * sizeof(float) > workspace_bytes) splits = 1;
+    const int splits = prompt_attn_splits((long long)blocks * num_kv_heads * B, tiles);
+    const size_t q_rows = (size_t)B * len_q;
     uint64_t* bits = mask ? static_cast<uint64_t*>(workspace) : nullptr;
     int32_t* last = mask ? reinterpret_cast<int32_t*>(static_cast<uint8_t*>(workspace) + (q_rows * tiles * 8 + 15) / 16 * 16) : nullptr;
-    float *part_o = nullptr, *part_m = nullptr, *part_l = nullptr;
-    if (splits > 1) {
-        part_o = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + head_bytes);
-        part_m = part_o + vheads * splits * D;
-        part_l = part_m + vheads * splits;
-    }
+    ZL_CHECK_WAITS();
+    unsigned* words = wait_words();
+    ZL_CHECK_CUDA(words ? cudaSuccess : cudaErrorMemoryAllocation);
     static bool attr_set[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-        ZL_CHECK_CUDA(cudaFuncSetAttribute(k_attn_prompt<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, prompt_attn_smem_bytes<D>()));
+        ZL_CHECK_CUDA(cudaFuncSetAttribute(k_attn_prompt<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, PaCfg<D>::kBytes));
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
     if (mask)
         ZL_CHECK_CUDA(launch(k_mask_bits, dim3(len_q, B), dim3(256), 0, stream, pdl != 0, mask, buf_lens, bits, last, len_q, tiles));
-    ZL_CHECK_CUDA(launch(k_attn_prompt<T, D>, dim3(blocks, num_kv_heads, B * splits), dim3(kPaThreads), (size_t)prompt_attn_smem_bytes<D>(), stream,
-                         pdl != 0, (const T*)q, buf_lens, (T* const*)k_addrs, (T* const*)v_addrs, (const uint64_t*)bits, (const int32_t*)last, tiles,
-                         scale, (T*)out, part_o, part_m, part_l, len_q, num_heads, num_kv_heads, m_query, splits, bshd));
-    if (splits > 1)
-        ZL_CHECK_CUDA(launch(k_attn_combine<T>, dim3((unsigned)vheads), dim3(D), 0, stream, pdl != 0, (const float*)part_o, (const float*)part_m,
-                             (const float*)part_l, (T*)out, splits));
+    const int aligned = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+    // behind the mask's kernel the attention may start early whatever the caller's chain allows: it waits for that kernel to end
+    ZL_CHECK_CUDA((launch_attn_prompt<T, D>(dim3(blocks, num_kv_heads, B * splits), splits, stream, pdl != 0 || mask, (const T*)q, buf_lens,
+                                            (T* const*)k_addrs, (T* const*)v_addrs, (const uint64_t*)bits, (const int32_t*)last, tiles, scale,
+                                            (T*)out, len_q, num_heads, num_kv_heads, m_query, splits, bshd, aligned, words + kWaitAttnPrompt)));
     g_attn_pf_ptr = nullptr;
     g_attn_pf_bytes = 0;
     return ZL_OK;

@@ -49,7 +49,8 @@ unsigned* zl::wait_words() {
 }
 extern "C" void* zl_wait_words(void) { return zl::wait_words(); }
 extern "C" int zl_check_waits(void) {
-    static const char* const names[zl::kWaitWords] = {"general tensor-core GEMM", "4-bit GEMM over pairs of SMs"};
+    static const char* const names[zl::kWaitWords] = {"general tensor-core GEMM", "4-bit GEMM over pairs of SMs",
+                                                      "attention of prompt portions"};
     unsigned* words = zl::wait_words();
     if (!words) return ZL_OK;   // no kernel that would write them has been launched
     for (int i = 0; i < zl::kWaitWords; ++i) {

@@ -3,26 +3,35 @@
 // (reference src/nn/attention/attention_kernel.cu:1252-1457), same softmax: mask ? scale * s : -inf, maximum from -1e20, sum
 // from 1e-20, so a row that sees nothing gives zeros.
 //
-// The decode kernels give every query row a CTA of its own, which reads the task's whole K and V again: 512 rows behind 588
-// bf16 positions, 32 heads on 8, take 306 us so and 58 us here (fp16: 287 and 45).  A CTA owns 64 (query, head) rows of one kv
-// head -- all heads of the group share the tile -- and walks the keys 64 at a time with running maxima: 16 rows per warp,
-// S = Q K^T and O += P V on mma.sync, K and V tiles double-buffered in shared memory through cp.async.  fp16 models carry
-// p * 2^10 in fp16, bf16 models p as bf16 hi + lo (two MMAs), as the decode kernels do.  Bound by the mma.sync rate (64-key tile
-// and warp: 64 MMAs for S, 64 or 128 for O, one per 8 cycles and scheduler).
+// The decode kernels give every query row a CTA of its own, which reads the task's whole K and V again: 512 rows behind 588 bf16 positions,
+// 32 heads on 8, took 306 us so.  A CTA owns 128 (query, head) rows of one kv head -- all heads of the group share the tile -- and walks the
+// keys 64 at a time:
 //
-// An int8 mask is turned into bits first (k_mask_bits), once for all kv heads, together with each row's last visible key: tiles
-// behind the last key any row of the block sees are never loaded, which halves a causal prompt's work.
+//   warps 0-3  softmax : thread = row = lane of tensor memory; running maximum and sum in fp32; the probabilities go back over the scores
+//   warp 4     S = Q K^T by tcgen05.mma, Q and K in shared memory (128-byte swizzle); two buffers of scores in tensor memory
+//   warp 5     O += P V, P from tensor memory, V as it lies (rows of keys: the B operand along n), O in tensor memory; TMEM allocation
+//   warps 6-7  K and V tiles by 16-byte cp.async into the swizzled layout (the buffers' addresses are known to the device only), K a tile ahead
+//
+// fp16 models carry p * 2^10 in fp16, bf16 models p as bf16 hi + lo (two MMAs), as the decode kernels do.  A row's reference maximum only
+// follows the true one once that has grown by 2^5 (fp16) or 2^8, so that O is seldom rescaled.  Two CTAs share an SM (256 columns each): one's
+// MMAs run under the other's softmax.  Bound by the MMAs (bf16, a tile: 450 cycles of S, whose operands come at 128 bytes a cycle, and 580 of
+// P V) and, for short prompts, by a chain of about 10 us (launch, mask, first loads, merge).  500 rows behind 1000 positions, bf16, 32 heads on
+// 8: 62 us on mma.sync with 64-row blocks (65 us of kernel time), 29 here; 512 x 1500 with 64 heads on 8, all launches of the call: 120 -> 50.
+//
+// An int8 mask is turned into bits first (k_mask_bits), once for all kv heads, together with each row's last visible key: tiles behind the last
+// key any row of the block sees are never loaded, which halves a causal prompt's work.  Few blocks are cut along their keys: the CTAs of a
+// cluster take a range each and push their rows' O, maximum and sum into the shared memory of the CTA that finishes the row.
+//
+// Nothing waits for ever: see tc2_common.cuh.  The waits begin behind the launch dependency.
 #pragma once
-#include "common.cuh"
+#include "tc2_common.cuh"
 
 #include <type_traits>
 
 namespace zl {
 
-constexpr int kPaRows = 64, kPaKeys = 64, kPaThreads = 128;
-
-template <int D>
-constexpr int prompt_attn_smem_bytes() { return 2 * 2 * kPaKeys * D * 2; }   // two stages of K and V
+constexpr int kPaRows = 128, kPaKeys = 64;
+constexpr int kPaWarpS = 4, kPaWarpO = 5, kPaWarpLoad = 6, kPaLoaders = 64, kPaThreads = kPaWarpLoad * 32 + kPaLoaders;
 
 // mask rows -> bits.  grid (len_q, B), 256 threads; bits [B][len_q][pitch64] with zero words behind len_buf, last [B][len_q]: index
 // of the last visible key, -1 for none
@@ -61,250 +70,481 @@ __global__ void __launch_bounds__(256) k_mask_bits(const int8_t* __restrict__ ma
     }
 }
 
-template <typename T>
-__device__ __forceinline__ void pa_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    if constexpr (std::is_same<T, __half>::value) mma_16816_f16(d, a, b0, b1, d);
-    else mma_16816_bf16(d, a, b0, b1, d);
+// ---- PTX wrappers (one CTA, cta_group::1) ---------------------------------------------------------------------------------------
+__device__ __forceinline__ void pa_alloc(uint32_t* s_tmem) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "n"(256));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
 }
-// 16-byte chunk c of row r of a tile with D / 8 chunks per row: xor by the row keeps ldmatrix free of bank conflicts
-template <int D>
-__device__ __forceinline__ uint32_t pa_off(int r, int c) { return (uint32_t)(r * (D * 2) + ((c ^ (r & 7)) << 4)); }
+__device__ __forceinline__ void pa_dealloc(uint32_t tmem) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(256));
+}
+__device__ __forceinline__ void pa_mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accum)
+        : "memory");
+}
+__device__ __forceinline__ void pa_mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accum) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accum)
+        : "memory");
+}
+// fp32 accumulators, 128 x n x 16; b_mn: B's rows run along n (V), not along k
+__host__ __device__ constexpr uint32_t pa_idesc(bool bf16, int n, bool b_mn) {
+    return (1u << 4) | (bf16 ? (1u << 7) | (1u << 10) : 0u) | (b_mn ? 1u << 16 : 0u) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kPaRows >> 4) << 24);
+}
+// B as [64 columns of n][k][128 bytes], 128-byte swizzle: 1024 bytes from 8 rows of k to the next, `block` bytes from 64 columns to the next
+__device__ __forceinline__ uint64_t pa_desc_mn(uint32_t saddr, uint32_t block) {
+    return (uint64_t)((saddr >> 4) & 0x3FFF) | (uint64_t)(block >> 4) << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
+}
+__device__ __forceinline__ void pa_ld32(uint32_t taddr, uint32_t* r) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,"
+        "%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+          "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
+          "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
+          "=r"(r[31])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void pa_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// two fp32 lanes of a 64-bit register pair at a time: half the instructions of the scalar forms
+__device__ __forceinline__ uint64_t pa_two(float x, float y) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ void pa_split(uint64_t v, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v)); }
+__device__ __forceinline__ uint64_t pa_fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t pa_add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float pa_max3(float x, float y, float z) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(x), "f"(y), "f"(z));
+    return r;
+}
+__device__ __forceinline__ float pa_exp2(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
 __device__ __forceinline__ void pa_cp16(uint32_t dst, const void* src, bool in) {
     const int bytes = in ? 16 : 0;   // 0: zero fill, nothing is read
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void pa_ldm4(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+__device__ __forceinline__ void pa_landed(uint64_t* bar) {   // one arrival once this thread's copies so far are there
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ void pa_ldm4t(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+__device__ __forceinline__ void pa_fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void pa_st_cluster4(uint32_t addr, uint4 v) {
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
-template <typename T>
-__device__ __forceinline__ void pa_pack(float x, float y, uint32_t& hi, uint32_t& lo) {
-    if constexpr (std::is_same<T, __half>::value) {
-        const __half2 h = __floats2half2_rn(x * 1024.f, y * 1024.f);
-        hi = *reinterpret_cast<const uint32_t*>(&h);
-    } else {
-        const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-        const float2 f = __bfloat1622float2(h);
-        const __nv_bfloat162 l = __floats2bfloat162_rn(x - f.x, y - f.y);
-        hi = *reinterpret_cast<const uint32_t*>(&h);
-        lo = *reinterpret_cast<const uint32_t*>(&l);
-    }
+__device__ __forceinline__ void pa_st_cluster2(uint32_t addr, float2 v) {
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.x), "f"(v.y) : "memory");
 }
 
-// grid (row blocks, kv heads, B * splits); the last row blocks, which see the most keys of a causal prompt, start first
+template <int D>
+struct PaCfg {
+    static constexpr int kAtoms = D / 64;                        // 128-byte columns of a row
+    static constexpr int kQ = kAtoms * kPaRows * 128;            // [64 of d][128 rows][128 B]
+    static constexpr int kTile = kAtoms * kPaKeys * 128;         // K or V: [64 of d][64 keys][128 B]
+    static constexpr int kKOff = kQ, kVOff = kQ + 2 * kTile;
+    static constexpr int kStaged = kQ + 4 * kTile;
+    static constexpr int kRow = D + 4;                           // merge: floats per row, 16-byte chunks of eight lanes on eight bank groups
+    static constexpr int kMl = kPaRows * kRow * 4;               // {maximum, sum} of a row behind the accumulators
+    static constexpr int kMerge = kMl + kPaRows * 8;
+    static constexpr int kBytes = (kStaged > kMerge ? kStaged : kMerge) + 1024;   // + slack for the manual 1024-byte alignment
+    static constexpr int kS = 128;                               // TMEM columns: O 0 .. D - 1, S / P 128 .. 255 (two buffers of 64)
+};
+
+// grid (row blocks, kv heads, B * splits), clusters of `splits` CTAs along z; the last row blocks, which see the most keys of a causal
+// prompt, start first
 template <typename T, int D>
 __global__ void __launch_bounds__(kPaThreads, 2)
 k_attn_prompt(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* const* __restrict__ k_addrs, T* const* __restrict__ v_addrs,
-              const uint64_t* __restrict__ bits, const int32_t* __restrict__ last, int pitch64, float scale, T* __restrict__ out,
-              float* __restrict__ part_o, float* __restrict__ part_m, float* __restrict__ part_l, int len_q, int num_heads, int num_kv_heads,
-              int m_query, int splits, int bshd) {
-    constexpr int KS = D / 16, NJ = D / 8, CH = D / 8;   // k-steps of S, n-tiles of O, 16-byte chunks per row
+              const uint64_t* __restrict__ bits, const int32_t* __restrict__ last, int pitch64, float scale, T* __restrict__ out, int len_q,
+              int num_heads, int num_kv_heads, int m_query, int splits, int bshd, int aligned, unsigned* err) {
+    using C = PaCfg<D>;
     constexpr bool kHalf = std::is_same<T, __half>::value;
-    extern __shared__ __align__(128) uint8_t pa_smem[];
-    __shared__ int s_last;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    constexpr int CH = D / 8;                                    // 16-byte chunks per row
+    extern __shared__ uint8_t pa_smem[];
+    uint8_t* smem = pa_smem + ((1024u - (smem_u32(pa_smem) & 1023u)) & 1023u);
+    __shared__ uint64_t k_full[2], v_full[2];
+    __shared__ uint64_t s_full[2];    // scores of a tile are there, and its K is done with
+    __shared__ uint64_t p_full[2];
+    __shared__ uint64_t o_done[2];    // P V of a tile has been added: its V and its scores' columns are done with
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_gave_up;
+    volatile int* s_abort = &s_gave_up;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rb = (int)gridDim.x - 1 - (int)blockIdx.x, hk = blockIdx.y, b = blockIdx.z / splits, split = blockIdx.z % splits;
     const int rows = len_q * m_query, row0 = rb * kPaRows;
-    pdl_trigger();
+    if (tid == 0) {
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&k_full[i], kPaLoaders);
+            mbar_init(&v_full[i], kPaLoaders);
+            mbar_init(&s_full[i], 1);
+            mbar_init(&p_full[i], 4);
+            mbar_init(&o_done[i], 1);
+        }
+        s_gave_up = 0;
+        mbar_fence_init();
+    }
+    if (warp == kPaWarpO) pa_alloc(&s_tmem);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    pdl_trigger();   // behind the allocation: a dependent that takes all of TMEM cannot keep this block waiting for it
     pdl_wait();
+    const uint32_t tmem = s_tmem;
     const int len_buf = buf_lens[b];
-    const size_t stride = bshd ? (size_t)num_kv_heads * D : (size_t)D;
-    const size_t base = bshd ? (size_t)hk * D : (size_t)hk * len_buf * D;
-    const T* kbase = k_addrs[b] + base;
-    const T* vbase = v_addrs[b] + base;
+    const T *kp = k_addrs[b], *vp = v_addrs[b];
 
-    // keys this block can see
+    // keys this block can see; every warp finds out by itself, the loaders go ahead of the rows of q
     int n = len_buf;
     if (bits) {
-        if (tid == 0) s_last = -1;
-        __syncthreads();
         const int q_lo = row0 / m_query, q_hi = (min(row0 + kPaRows, rows) - 1) / m_query;
-        for (int i = q_lo + tid; i <= q_hi; i += kPaThreads) atomicMax(&s_last, last[(size_t)b * len_q + i]);
-        __syncthreads();
-        n = s_last + 1;
+        int mine = -1;
+        for (int i = q_lo + lane; i <= q_hi; i += 32) mine = max(mine, last[(size_t)b * len_q + i]);
+        asm volatile("" ::"l"(kp), "l"(vp));   // fetched by now, beside the line above: the loaders' next step
+        n = __reduce_max_sync(0xffffffffu, mine) + 1;
+    }
+    if (warp < kPaWarpLoad) {
+        // rows of q: [64 of d][row][128 B], chunks xor the row; rows behind the last one are zeros and are not stored
+        constexpr int kStep = kPaWarpLoad * 32 / CH;
+        const int c = tid % CH, dq = kStep / m_query, dh = kStep % m_query;
+        int r = tid / CH, h = row0 + r;
+        unsigned at = (unsigned)h / (unsigned)m_query;           // its query, then the place of its (query, head) row
+        h -= at * m_query;
+        at = at * num_heads + h;
+        const T* q0 = q + ((size_t)b * len_q * num_heads + hk * m_query) * D + c * 8;
+        const uint32_t dst0 = smem_u32(smem) + (uint32_t)((c >> 3) * (kPaRows * 128));
+#pragma unroll
+        for (int i = 0; i < (kPaRows + kStep - 1) / kStep; ++i, r += kStep) {
+            const bool in = row0 + r < rows;
+            const T* src = q0 + (size_t)(in ? at : 0u) * D;
+            const uint32_t dst = dst0 + (uint32_t)(r * 128 + (((c & 7) ^ (r & 7)) << 4));
+            if (r < kPaRows) {
+                if (aligned) {
+                    pa_cp16(dst, src, in);
+                } else {
+                    const uint32_t* w = reinterpret_cast<const uint32_t*>(src);
+                    *reinterpret_cast<uint4*>(smem + (dst - smem_u32(smem))) = in ? make_uint4(w[0], w[1], w[2], w[3]) : make_uint4(0, 0, 0, 0);
+                }
+            }
+            h += dh;
+            at += dq * num_heads + dh;
+            if (h >= m_query) h -= m_query, at += num_heads - m_query;
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        pa_fence_async();
+        asm volatile("bar.sync 1, %0;" ::"n"(kPaWarpLoad * 32) : "memory");
     }
     const int tiles = cdiv(n, kPaKeys);
-    const int t0 = (int)((long long)tiles * split / splits), t1 = (int)((long long)tiles * (split + 1) / splits);
+    const int t0 = (int)((long long)tiles * split / splits), t1 = (int)((long long)tiles * (split + 1) / splits), count = t1 - t0;
 
-    // this lane's two rows (g and g + 8 of the warp's 16): out of range rows compute on row 0's query and are not stored
-    int qi[2], hd[2];
-    bool live[2];
+    float l = 0.f, m_ref = -1.4426950e20f;                       // of this thread's row; base-2 logarithms
+    if (warp == kPaWarpS) {
+        const uint32_t id = pa_idesc(!kHalf, kPaKeys, false);
+        const uint64_t qd = tc_desc_sw128(smem_u32(smem));
+        for (int j = 0; j < count; ++j) {
+            const int st = j & 1;
+            const uint32_t ph = (uint32_t)(j >> 1) & 1u;
+            if (!tc2_wait(&k_full[st], ph, s_abort, err, 0x4100 + st)) break;
+            pa_fence_async();
+            if (j > 1 && !tc2_wait(&o_done[st], ph ^ 1u, s_abort, err, 0x4180 + st)) break;
+            tc_fence_after();
+            if (tc_elect_one()) {
+                const uint64_t kd = tc_desc_sw128(smem_u32(smem + C::kKOff + st * C::kTile));
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int r = row0 + warp * 16 + g + i * 8;
-        live[i] = r < rows;
-        qi[i] = live[i] ? r / m_query : 0;
-        hd[i] = hk * m_query + (live[i] ? r % m_query : 0);
-    }
-    uint32_t qf[KS][4];
-    {
-        const T* q0 = q + (((size_t)b * len_q + qi[0]) * num_heads + hd[0]) * D + 2 * t;
-        const T* q1 = q + (((size_t)b * len_q + qi[1]) * num_heads + hd[1]) * D + 2 * t;
-#pragma unroll
-        for (int k = 0; k < KS; ++k) {
-            qf[k][0] = *reinterpret_cast<const uint32_t*>(q0 + k * 16);
-            qf[k][1] = *reinterpret_cast<const uint32_t*>(q1 + k * 16);
-            qf[k][2] = *reinterpret_cast<const uint32_t*>(q0 + k * 16 + 8);
-            qf[k][3] = *reinterpret_cast<const uint32_t*>(q1 + k * 16 + 8);
+                for (int k = 0; k < D / 16; ++k)
+                    pa_mma_ss(tmem + (uint32_t)(C::kS + st * 64), qd + (uint64_t)((k >> 2) * (kPaRows * 128 / 16) + (k & 3) * 2),
+                              kd + (uint64_t)((k >> 2) * (kPaKeys * 128 / 16) + (k & 3) * 2), id, k > 0 ? 1u : 0u);
+                tc_commit(&s_full[st]);
+            }
+            __syncwarp();
         }
-    }
-    const uint64_t* brow[2] = {nullptr, nullptr};
-    if (bits) {
+    } else if (warp == kPaWarpO) {
+        const uint32_t id = pa_idesc(!kHalf, D, true);
+        for (int j = 0; j < count; ++j) {
+            const int st = j & 1;
+            const uint32_t ph = (uint32_t)(j >> 1) & 1u;
+            if (!tc2_wait(&v_full[st], ph, s_abort, err, 0x4200 + st)) break;
+            pa_fence_async();
+            if (!tc2_wait(&p_full[st], ph, s_abort, err, 0x4300 + st)) break;
+            tc_fence_after();
+            if (tc_elect_one()) {
+                const uint64_t vd = pa_desc_mn(smem_u32(smem + C::kVOff + st * C::kTile), kPaKeys * 128);
+                const uint32_t p = tmem + (uint32_t)(C::kS + st * 64);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) brow[i] = bits + ((size_t)b * len_q + qi[i]) * pitch64;
-    }
-
-    const uint32_t sm = smem_u32(pa_smem);
-    constexpr uint32_t kTile = kPaKeys * D * 2;
-    auto load_tile = [&](int tile, int st) {
-        const int k0 = tile * kPaKeys;
+                for (int h = 0; h < (kHalf ? 1 : 2); ++h)        // bf16: the probabilities' upper halves, then the lower ones
 #pragma unroll
-        for (int i = 0; i < kPaKeys * CH / kPaThreads; ++i) {
-            const int e = tid + i * kPaThreads, r = e / CH, c = e % CH;
-            const bool in = k0 + r < n;
-            const size_t src = (size_t)(in ? k0 + r : 0) * stride + c * 8;
-            pa_cp16(sm + st * 2 * kTile + pa_off<D>(r, c), kbase + src, in);
-            pa_cp16(sm + st * 2 * kTile + kTile + pa_off<D>(r, c), vbase + src, in);
+                    for (int k = 0; k < kPaKeys / 16; ++k)
+                        pa_mma_ts(tmem, p + (uint32_t)(h * 32 + k * 8), vd + (uint64_t)(k * (16 * 128 / 16)), id, (j > 0 || h > 0 || k > 0) ? 1u : 0u);
+                tc_commit(&o_done[st]);
+            }
+            __syncwarp();
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-
-    float o[NJ][4], mx[2] = {-1e20f, -1e20f}, sum[2] = {0.f, 0.f};
+    } else if (warp >= kPaWarpLoad) {
+        const int t = tid - kPaWarpLoad * 32, c = t % CH;
+        const size_t stride = bshd ? (size_t)num_kv_heads * D : (size_t)D;
+        const size_t base = (bshd ? (size_t)hk * D : (size_t)hk * len_buf * D) + c * 8;
+        const T* kbase = kp + base;
+        const T* vbase = vp + base;
+        const uint32_t at = smem_u32(smem) + (uint32_t)((c >> 3) * (kPaKeys * 128));
+        auto load = [&](const T* from, uint32_t to, int k0) {
 #pragma unroll
-    for (int j = 0; j < NJ; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
-    uint64_t vis_next[2] = {~0ull, ~0ull};
-    if (t0 < t1) {
-        load_tile(t0, 0);
-        if (bits) vis_next[0] = brow[0][t0], vis_next[1] = brow[1][t0];
-    }
-    for (int tile = t0; tile < t1; ++tile) {
-        const int st = (tile - t0) & 1;
-        uint64_t vis[2] = {vis_next[0], vis_next[1]};
-        if (tile + 1 < t1) {
-            load_tile(tile + 1, st ^ 1);
-            if (bits) vis_next[0] = brow[0][tile + 1], vis_next[1] = brow[1][tile + 1];
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            for (int i = 0; i < kPaKeys * CH / kPaLoaders; ++i) {
+                const int r = t / CH + i * (kPaLoaders / CH);
+                const bool in = k0 + r < n;
+                pa_cp16(to + (uint32_t)(r * 128 + (((c & 7) ^ (r & 7)) << 4)), from + (size_t)(in ? k0 + r : 0) * stride, in);
+            }
+        };
+        // K runs a tile ahead of V
+        for (int i = 0; i < 2 * count; ++i) {
+            const int is_v = i > 0 && (i == 2 * count - 1 || !(i & 1)), j = is_v ? (i - 1) >> 1 : (i + 1) >> 1, st = j & 1;
+            if (j > 1 && !tc2_wait(is_v ? &o_done[st] : &s_full[st], ((uint32_t)(j >> 1) & 1u) ^ 1u, s_abort, err, 0x4400 + 2 * is_v + st)) break;
+            load(is_v ? vbase : kbase, at + (uint32_t)((is_v ? C::kVOff : C::kKOff) + st * C::kTile), (t0 + j) * kPaKeys);
+            pa_landed(is_v ? &v_full[st] : &k_full[st]);
         }
-        __syncthreads();
-        const int left = n - tile * kPaKeys;
-        if (left < kPaKeys) {
-            const uint64_t keep = (1ull << left) - 1;
-            vis[0] &= keep, vis[1] &= keep;
-        }
-        // a tile none of the warp's rows sees (the diagonal of a causal prompt) costs nothing
-        if (__any_sync(0xffffffffu, (live[0] && vis[0]) || (live[1] && vis[1]))) {
-            const uint32_t sk = sm + st * 2 * kTile, sv = sk + kTile;
-            float s[8][4];
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else {
+        // warp = quadrant of TMEM lanes, thread = row
+        const int r = row0 + tid;
+        const uint64_t* vis_row = bits ? bits + ((size_t)b * len_q + (r < rows ? r / m_query : 0)) * pitch64 : nullptr;
+        const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
+        constexpr float kLog2e = 1.4426950408889634f;
+        constexpr float kTau = kHalf ? 5.f : 8.f;                // p * 2^10 of fp16 stays below 2^15
+        constexpr float kUp = kHalf ? 10.f : 0.f;
+        uint64_t vis_next = bits && count > 0 ? vis_row[t0] : ~0ull;
+        for (int j = 0; j < count; ++j) {
+            const int st = j & 1;
+            uint64_t vis = vis_next;
+            if (bits && j + 1 < count) vis_next = vis_row[t0 + j + 1];
+            const int left = n - (t0 + j) * kPaKeys;
+            if (left < kPaKeys) vis &= (1ull << left) - 1;
+            if (!tc2_wait(&s_full[st], (uint32_t)(j >> 1) & 1u, s_abort, err, 0x4600 + st)) break;
+            tc_fence_after();
+            const uint32_t ts = taddr + (uint32_t)(C::kS + st * 64);
+            uint32_t raw[64];
+            pa_ld32(ts, raw);
+            pa_ld32(ts + 32, raw + 32);
+            pa_wait_ld();
+            float c = scale * kLog2e;
+            if (!(scale > 0.f) || !__all_sync(0xffffffffu, vis == ~0ull)) {   // some keys are hidden from some row
+                const uint32_t lo = (uint32_t)vis, hi = (uint32_t)(vis >> 32);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+                for (int i = 0; i < 64; ++i) raw[i] = __float_as_uint(((i < 32 ? lo : hi) >> (i & 31) & 1) ? __uint_as_float(raw[i]) * c : -INFINITY);
+                c = 1.f;
+            }
+            float mx[4];
 #pragma unroll
-            for (int k = 0; k < KS; ++k)
+            for (int i = 0; i < 4; ++i) mx[i] = __uint_as_float(raw[i]);
 #pragma unroll
-                for (int jj = 0; jj < 4; ++jj) {
-                    uint32_t kb[4];
-                    pa_ldm4(kb, sk + pa_off<D>(jj * 16 + (lane & 7) + (lane >> 4) * 8, k * 2 + ((lane >> 3) & 1)));
-                    pa_mma<T>(s[2 * jj], qf[k], kb[0], kb[1]);
-                    pa_mma<T>(s[2 * jj + 1], qf[k], kb[2], kb[3]);
+            for (int i = 4; i < 60; i += 8)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) mx[u] = pa_max3(mx[u], __uint_as_float(raw[i + 2 * u]), __uint_as_float(raw[i + 2 * u + 1]));
+            mx[0] = pa_max3(mx[0], __uint_as_float(raw[60]), __uint_as_float(raw[61]));
+            mx[1] = pa_max3(mx[1], __uint_as_float(raw[62]), __uint_as_float(raw[63]));
+            const float m_tile = pa_max3(fmaxf(mx[0], mx[1]), mx[2], mx[3]) * c;
+            // The reference maximum of a row only follows where the true one has left it by a factor of 2^kTau: any reference gives the
+            // same quotient, and rescaling O costs a round trip through the registers.
+            const bool up = m_tile > m_ref + kTau;
+            if (__any_sync(0xffffffffu, up)) {
+                const float f = up ? pa_exp2(m_ref - m_tile) : 1.f;
+                if (up) m_ref = m_tile;
+                l *= f;
+                if (j > 0) {
+                    if (!tc2_wait(&o_done[st ^ 1], (uint32_t)((j - 1) >> 1) & 1u, s_abort, err, 0x4700)) break;
+                    tc_fence_after();
+#pragma unroll 1
+                    for (int d0 = 0; d0 < D; d0 += 16) {
+                        float v[16];
+                        uint32_t w[16];
+                        tc_ld16(taddr + (uint32_t)d0, v);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) w[i] = __float_as_uint(v[i] * f);
+                        tc_st16(taddr + (uint32_t)d0, w);
+                    }
                 }
-            const uint32_t v0[2] = {(uint32_t)vis[0], (uint32_t)(vis[0] >> 32)}, v1[2] = {(uint32_t)vis[1], (uint32_t)(vis[1] >> 32)};
-            float m0 = mx[0], m1 = mx[1];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int sh = (j & 3) * 8 + 2 * t;
-                const uint32_t w0 = v0[j >> 2] >> sh, w1 = v1[j >> 2] >> sh;
-                s[j][0] = (w0 & 1) ? s[j][0] * scale : -INFINITY;
-                s[j][1] = (w0 & 2) ? s[j][1] * scale : -INFINITY;
-                s[j][2] = (w1 & 1) ? s[j][2] * scale : -INFINITY;
-                s[j][3] = (w1 & 2) ? s[j][3] * scale : -INFINITY;
-                m0 = fmaxf(m0, fmaxf(s[j][0], s[j][1]));
-                m1 = fmaxf(m1, fmaxf(s[j][2], s[j][3]));
             }
+            const uint64_t c2 = pa_two(c, c), m2 = pa_two(kUp - m_ref, kUp - m_ref);
+            const uint64_t minus = pa_two(-1.f, -1.f);
+            uint64_t sum = 0;
 #pragma unroll
-            for (int x = 1; x < 4; x <<= 1) {
-                m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, x));
-                m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, x));
+            for (int half = 0; half < 2; ++half) {
+                uint32_t hi[16], lo[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    float x, y;
+                    pa_split(pa_fma2(pa_two(__uint_as_float(raw[half * 32 + 2 * i]), __uint_as_float(raw[half * 32 + 2 * i + 1])), c2, m2), x, y);
+                    x = pa_exp2(x);
+                    y = pa_exp2(y);
+                    sum = pa_add2(sum, pa_two(x, y));
+                    if constexpr (kHalf) {
+                        const __half2 h = __floats2half2_rn(x, y);
+                        hi[i] = *reinterpret_cast<const uint32_t*>(&h);
+                    } else {
+                        const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+                        hi[i] = *reinterpret_cast<const uint32_t*>(&h);
+                        pa_split(pa_fma2(pa_two(__uint_as_float(hi[i] << 16), __uint_as_float(hi[i] & 0xffff0000u)), minus, pa_two(x, y)), x, y);
+                        const __nv_bfloat162 e = __floats2bfloat162_rn(x, y);
+                        lo[i] = *reinterpret_cast<const uint32_t*>(&e);
+                    }
+                }
+                tc_st16(ts + (uint32_t)(half * 16), hi);
+                if constexpr (!kHalf) tc_st16(ts + (uint32_t)(32 + half * 16), lo);
             }
-            constexpr float kLog2e = 1.4426950408889634f;
-            const float c0 = exp2f((mx[0] - m0) * kLog2e), c1 = exp2f((mx[1] - m1) * kLog2e);
-            mx[0] = m0, mx[1] = m1;
-            float l0 = 0.f, l1 = 0.f;
+            float s0, s1;
+            pa_split(sum, s0, s1);
+            l += s0 + s1;
+            tc_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&p_full[st]);
+        }
+        if (count > 0) tc2_wait(&o_done[(count - 1) & 1], (uint32_t)((count - 1) >> 1) & 1u, s_abort, err, 0x4800);
+        tc_fence_after();
+        l += kHalf ? 1024.f * 1e-20f : 1e-20f;
+        if (splits == 1) {
+            T* dst = out + (((size_t)b * len_q + r / m_query) * num_heads + hk * m_query + r % m_query) * D;
+            const float inv = 1.f / l;
+#pragma unroll 1
+            for (int d0 = 0; d0 < D; d0 += 16) {
+                float v[16];
+                tc_ld16(taddr + (uint32_t)d0, v);
+                if (r < rows) {
+                    uint32_t w[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                s[j][0] = exp2f((s[j][0] - m0) * kLog2e);
-                s[j][1] = exp2f((s[j][1] - m0) * kLog2e);
-                s[j][2] = exp2f((s[j][2] - m1) * kLog2e);
-                s[j][3] = exp2f((s[j][3] - m1) * kLog2e);
-                l0 += s[j][0] + s[j][1];
-                l1 += s[j][2] + s[j][3];
-            }
-            sum[0] = fmaf(sum[0], c0, l0);
-            sum[1] = fmaf(sum[1], c1, l1);
+                    for (int i = 0; i < 8; ++i) {
+                        T two[2] = {from_f32<T>(count > 0 ? v[2 * i] * inv : 0.f), from_f32<T>(count > 0 ? v[2 * i + 1] * inv : 0.f)};
+                        w[i] = *reinterpret_cast<const uint32_t*>(two);
+                    }
+                    if (aligned) {
+                        *reinterpret_cast<uint4*>(dst + d0) = make_uint4(w[0], w[1], w[2], w[3]);
+                        *reinterpret_cast<uint4*>(dst + d0 + 8) = make_uint4(w[4], w[5], w[6], w[7]);
+                    } else {
 #pragma unroll
-            for (int j = 0; j < NJ; ++j) o[j][0] *= c0, o[j][1] *= c0, o[j][2] *= c1, o[j][3] *= c1;
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-                uint32_t ah[4], al[4];
-                pa_pack<T>(s[2 * kk][0], s[2 * kk][1], ah[0], al[0]);
-                pa_pack<T>(s[2 * kk][2], s[2 * kk][3], ah[1], al[1]);
-                pa_pack<T>(s[2 * kk + 1][0], s[2 * kk + 1][1], ah[2], al[2]);
-                pa_pack<T>(s[2 * kk + 1][2], s[2 * kk + 1][3], ah[3], al[3]);
-#pragma unroll
-                for (int jj = 0; jj < NJ / 2; ++jj) {
-                    uint32_t vb[4];
-                    pa_ldm4t(vb, sv + pa_off<D>(kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, jj * 2 + (lane >> 4)));
-                    pa_mma<T>(o[2 * jj], ah, vb[0], vb[1]);
-                    pa_mma<T>(o[2 * jj + 1], ah, vb[2], vb[3]);
-                    if constexpr (!kHalf) {
-                        pa_mma<T>(o[2 * jj], al, vb[0], vb[1]);
-                        pa_mma<T>(o[2 * jj + 1], al, vb[2], vb[3]);
+                        for (int i = 0; i < 8; ++i) reinterpret_cast<uint32_t*>(dst + d0)[i] = w[i];
                     }
                 }
             }
         }
-        __syncthreads();   // everyone is done with this stage: the next iteration refills it
     }
-
+    __syncwarp();
+    tc2_drain(s_abort);
+    const int share = kPaRows / splits;   // rows that each CTA of the cluster finishes
+    if (splits > 1) {
+        cluster_sync_all();               // nobody's Q, K and V are needed any more: their place takes the rows' results
+        if (warp < kPaWarpS) {
+            const uint32_t at = smem_u32(smem) + (uint32_t)((split * share + tid % share) * C::kRow * 4);
+            const uint32_t dst = cluster_map(at, tid / share);
+            const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
+            tc_fence_after();
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        float l = sum[i];
-        l += __shfl_xor_sync(0xffffffffu, l, 1);
-        l += __shfl_xor_sync(0xffffffffu, l, 2);
-        l += 1e-20f;
-        if (!live[i]) continue;
-        const float inv = (kHalf ? 1.f / 1024.f : 1.f) / l;
-        const size_t vh = ((size_t)b * len_q + qi[i]) * num_heads + hd[i];
-        if (splits == 1) {
-            T* dst = out + vh * D + 2 * t;
+            for (int d0 = 0; d0 < D; d0 += 64) {
+                uint32_t v[64];
+                pa_ld32(taddr + (uint32_t)d0, v);
+                pa_ld32(taddr + (uint32_t)(d0 + 32), v + 32);
+                pa_wait_ld();
 #pragma unroll
-            for (int j = 0; j < NJ; ++j) {
-                T pr[2] = {from_f32<T>(o[j][2 * i] * inv), from_f32<T>(o[j][2 * i + 1] * inv)};
-                *reinterpret_cast<uint32_t*>(dst + j * 8) = *reinterpret_cast<const uint32_t*>(pr);
+                for (int i = 0; i < 64; i += 4)
+                    pa_st_cluster4(dst + (d0 + i) * 4, count > 0 ? make_uint4(v[i], v[i + 1], v[i + 2], v[i + 3]) : make_uint4(0u, 0u, 0u, 0u));
             }
-        } else {
-            float* dst = part_o + (vh * splits + split) * D + 2 * t;
-#pragma unroll
-            for (int j = 0; j < NJ; ++j) *reinterpret_cast<float2*>(dst + j * 8) = make_float2(o[j][2 * i] * inv, o[j][2 * i + 1] * inv);
-            if (t == 0) {
-                part_m[vh * splits + split] = mx[i];
-                part_l[vh * splits + split] = l;
+            pa_st_cluster2(cluster_map(smem_u32(smem) + C::kMl + (split * share + tid % share) * 8, tid / share), make_float2(m_ref, l));
+        }
+        tc_fence_before();
+        cluster_sync_all();
+    } else {
+        tc_fence_before();
+        __syncthreads();
+    }
+    if (warp == kPaWarpO) {
+        tc_fence_after();
+        pa_dealloc(tmem);
+    }
+    if (splits > 1) {
+        if (tid < share) {                // weights of a row's parts, in place of their maxima and sums
+            float2* ml = reinterpret_cast<float2*>(smem + C::kMl) + tid;
+            float m = -INFINITY, sum = 0.f;
+            for (int s = 0; s < splits; ++s) m = fmaxf(m, ml[s * share].x);
+            for (int s = 0; s < splits; ++s) {
+                const float f = pa_exp2(ml[s * share].x - m);
+                sum = fmaf(ml[s * share].y, f, sum);
+                ml[s * share].x = f;
+            }
+            const float inv = 1.f / sum;
+            for (int s = 0; s < splits; ++s) ml[s * share].x *= inv;
+        }
+        __syncthreads();
+        constexpr int kLanes = D / 4, kPer = kPaThreads / kLanes;   // threads of a row, rows at a time
+        const int d0 = (tid % kLanes) * 4;
+        const unsigned first = row0 + split * share;
+#pragma unroll 4
+        for (int rr = tid / kLanes; rr < share; rr += kPer) {
+            float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int s = 0; s < splits; ++s) {
+                const float4 v = *reinterpret_cast<const float4*>(smem + ((s * share + rr) * C::kRow + d0) * 4);
+                const float f = *reinterpret_cast<const float*>(smem + C::kMl + (s * share + rr) * 8);
+                o.x = fmaf(v.x, f, o.x), o.y = fmaf(v.y, f, o.y), o.z = fmaf(v.z, f, o.z), o.w = fmaf(v.w, f, o.w);
+            }
+            const unsigned r = first + rr, qi = r / (unsigned)m_query;
+            if (r >= (unsigned)rows) continue;
+            T w[4] = {from_f32<T>(o.x), from_f32<T>(o.y), from_f32<T>(o.z), from_f32<T>(o.w)};
+            T* dst = out + (((size_t)b * len_q + qi) * num_heads + hk * m_query + (r - qi * m_query)) * D + d0;
+            const uint2 two = make_uint2(reinterpret_cast<const uint32_t*>(w)[0], reinterpret_cast<const uint32_t*>(w)[1]);
+            if (aligned) {
+                *reinterpret_cast<uint2*>(dst) = two;
+            } else {
+                reinterpret_cast<uint32_t*>(dst)[0] = two.x;
+                reinterpret_cast<uint32_t*>(dst)[1] = two.y;
             }
         }
     }
 }
 
-// Key splits of a launch of `ctas` row blocks over up to `tiles` key tiles: a tile costs a CTA about 0.8 us, the merge of the splits
-// 5 us, so keys are only split where that shortens the longest chain.
+// Key splits (CTAs of a cluster) of a launch of `ctas` row blocks over up to `tiles` key tiles.  A tile is about 1 us of a CTA's chain, being a
+// cluster 3 us, so four tiles stay whole (256 x 256, 32 heads on 8: 12.6 against 14.5 us in two) and further ones are cut down to two a CTA:
+// 32 x 1100 15.8 us in eight, 18.2 in four.  Two CTAs share an SM, but larger clusters then wait for room: beyond one CTA per SM only pairs
+// (256 x 1300, 16 heads on 4: 19.9 us in four, 23.9 in eight; 128 x 600, 64 on 8: 19.0 in two, 21.0 in four).
 inline int prompt_attn_splits(long long ctas, int tiles) {
-    const long long slots = 2ll * device_sm_count();
-    int s = (int)(slots / (ctas > 0 ? ctas : 1));
-    if (s > tiles / 4) s = tiles / 4;
-    if (s > 16) s = 16;
-    if (s < 2 || (tiles - tiles / s) * 8 < 60) return 1;
+    const int sms = device_sm_count();
+    int s = 1;
+    if (tiles >= 8 && ctas * 2 <= 2ll * sms) s = 2;
+    while (s > 1 && s < 8 && tiles >= 4 * s && ctas * s * 2 <= sms) s *= 2;
     return s;
+}
+
+template <typename T, int D, typename... Args>
+inline cudaError_t launch_attn_prompt(dim3 grid, int splits, cudaStream_t stream, bool pdl, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kPaThreads);
+    cfg.dynamicSmemBytes = PaCfg<D>::kBytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (splits > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = splits;
+    }
+    if (pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    zl_count_launch();
+    return cudaLaunchKernelEx(&cfg, k_attn_prompt<T, D>, args...);
 }
 
 }  // namespace zl

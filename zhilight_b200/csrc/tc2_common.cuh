@@ -2,7 +2,7 @@
 // (the leader) issues the MMAs for both.  Each CTA holds 128 of the 256 A rows and half of the B rows in its own shared memory, and
 // the accumulators of its own 128 rows in its own TMEM.  Waits give up after about a second (a word in host memory is set, every role
 // leaves its loop, TMEM is freed and the kernel returns): a fault in the protocol must not hang the GPU.  What is left of the output is
-// unwritten then; zl_check_waits() makes it an error of the next synchronisation of a decoder, or of the next call of these GEMMs.
+// unwritten then; zl_check_waits() makes it an error of the next synchronisation of a decoder, or of the next call of one of these kernels.
 #pragma once
 #include "tc_common.cuh"
 
