@@ -39,9 +39,12 @@ struct W4Params {
     int tp_mode = 0;
     int tp_index = 0;              // exchange index within the step (< 512): parity of the slot + part of the word tag
     __half* tp_h_out = nullptr;
+    int x32 = 0;                   // rows of x start on 32 bytes (set by launch_w4_v2_int_layout)
 };
 
 cudaError_t launch_w4_v2(const W4Params& p, bool pdl, cudaStream_t stream);
+// the same on the ZLW4I layout, up to 16 rows, no fused RMSNorm prologue
+cudaError_t launch_w4_v2_int_layout(const W4Params& p, bool pdl, cudaStream_t stream);
 cudaError_t prepare_w4_v2();
 // exact-integer kernel on the ZLW4I layout; false = staged activations do not fit shared memory
 bool launch_w4_v3(const W4Params& p, bool pdl, cudaStream_t stream, cudaError_t* err);

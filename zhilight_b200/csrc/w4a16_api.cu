@@ -3,6 +3,7 @@
 // Stands in for nn::gptq::gptq_gemm_k_major's router (reference src/nn/quant/gptq/q_gemm_k_major.cu:957-1116:
 // M <= 40 GEMV, else dequant + cuBLASLt) and for GPTQMarlin::forward (src/nn/linear/linear.cpp:1247-1451):
 //   M <= 16 and the staged activations fit shared memory -> k_w4a16_v3  (exact-integer mma.sync kernel, ZLW4I layout)
+//   M <= 16 otherwise, N % 128 == 0                      -> k_w4a16_v2  (fp16 mma.sync kernel, on the ZLW4I layout)
 //   otherwise, N % 128 == 0                              -> k_w4a16_tc2 (tcgen05 over pairs of SMs, ZLW4I layout) where w4_tc2_route has it
 //                                                           faster, always above 256 rows; else
 //                                                           k_w4a16_ts  (tcgen05 kernel, stream-k, A operand in TMEM, ZLW4I layout)
@@ -146,6 +147,11 @@ extern "C" int zl_w4a16_gemm_fused(const zl_w4_fused_args_t* a, zl_stream_t stre
     ZL_CHECK_SUPPORTED(route != 0 && "ZLW4I layout: M > 16 (or staged activations too large) and N % 128 != 0: use variant 0");
     ZL_CHECK_SUPPORTED(!(route == 4 && a->ln_weight) && "the tcgen05 kernel has no fused RMSNorm prologue: run zl_rmsnorm first");
     const bool pairs = route == 4 && w4_tc2_route(a->M, a->N, a->K);
+    // Up to 16 rows that the integer kernel has no room for, and 9 to 16 rows that are its to choose (not the norm's or the exchange's): the fp16
+    // mma.sync kernel.  Against the tcgen05 kernel, us: 4096 x 14336 17.6 -> 10.7 (4 rows), 18.8 -> 13.5 (16); 28672 x 4096 26.1 -> 19.2 (8),
+    // 26.3 -> 24.4 (16); 8192 x 3584 12.8 -> 9.0.  Against the integer kernel: 16384 x 2048, 12 rows 13.8 -> 9.3; up to 8 rows that one is the
+    // faster (28672 x 4096, 5 rows: 16.8 against 19.2).
+    const bool few = a->M <= 16 && (route == 4 || (route == 3 && a->M > 8 && !a->ln_weight && !a->tp_mode));
     const int step = pairs ? a->M : route == 4 ? 256 : 32;
     for (int m0 = 0; m0 < a->M; m0 += step) {
         W4Params p;
@@ -189,6 +195,8 @@ extern "C" int zl_w4a16_gemm_fused(const zl_w4_fused_args_t* a, zl_stream_t stre
         p.pf_bytes = a->prefetch_bytes;
         if (pairs) {
             ZL_CHECK_CUDA(launch_w4_tc2(p, a->pdl != 0, stream));
+        } else if (few) {
+            ZL_CHECK_CUDA(launch_w4_v2_int_layout(p, a->pdl != 0, stream));
         } else if (route == 4) {
             ZL_CHECK_CUDA(launch_w4_tc(p, a->pdl != 0 && m0 == 0, stream));
         } else if (route == 3) {

@@ -12,6 +12,11 @@
 //     per tile);
 //   * 2 CTAs per SM leave room for the next kernel's CTAs to become resident under programmatic dependent
 //     launch and pre-fill their rings.
+//
+// INTL: the same kernel on the ZLW4I layout (w4_layout.cuh), for up to 16 rows that the integer kernel has no room for.  A word there is four
+// consecutive k of rows g and g + 8, which is one MMA's A fragment once the order of k within the group is the layout's; a lane's x then is 64
+// consecutive bytes.  10 instructions per word where ZLW4 takes 9, and no second copy of the weights.  Bound by these conversions and by x, which
+// every CTA reads whole.
 #include "common.cuh"
 #include "w4_layout.cuh"
 #include "w4_params.h"
@@ -41,23 +46,41 @@ constexpr int kV2TwoCtaBudget = 115000;
 constexpr int kV2OneCtaBudget = 231000;
 __host__ __device__ inline int x_row_bytes(int K) { return K * 2 + 64; }   // +64 B: conflict-free 16-byte shared loads across tokens
 
-template <int NT, bool NORM>
+// chunk of 8 k that load ii of lane t covers within a group: what the lane's weight words stand for in the two layouts (w4_layout.cuh)
+template <bool INTL>
+__device__ __forceinline__ int v2_k(int ii, int t) { return INTL ? t * 32 + ii * 8 : ii * 32 + t * 8; }
+// 32 bytes of x at once: two of a lane's neighbouring chunks are one sector
+__device__ __forceinline__ void ld_cg_u8(const void* p, uint4& a, uint4& b) {
+    asm volatile("ld.global.cg.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+                 : "l"(p));
+}
+
+template <int NT, bool NORM, bool INTL>
 __device__ __forceinline__ void load_bfrag_v2(uint4 (&b)[NT][4], const W4Params& p, int kbase, int g, int t,
                                               float (&ss)[NT]) {
     uint4 wl[4];
     if (NORM) {
 #pragma unroll
         for (int ii = 0; ii < 4; ++ii)
-            wl[ii] = *reinterpret_cast<const uint4*>(p.ln_w + kbase + ii * 32 + t * 8);
+            wl[ii] = *reinterpret_cast<const uint4*>(p.ln_w + kbase + v2_k<INTL>(ii, t));
     }
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
         const int tok = nt * 8 + g;
         if (tok < p.mc) {
-            const __half* src = p.x + (size_t)tok * p.ldx + kbase + t * 8;
+            const __half* src = p.x + (size_t)tok * p.ldx + kbase;
+            uint4 in[4];
+            if (INTL && p.x32) {
+                ld_cg_u8(src + t * 32, in[0], in[1]);
+                ld_cg_u8(src + t * 32 + 16, in[2], in[3]);
+            } else {
+#pragma unroll
+                for (int ii = 0; ii < 4; ++ii) in[ii] = ld_cg_u4(src + v2_k<INTL>(ii, t));
+            }
 #pragma unroll
             for (int ii = 0; ii < 4; ++ii) {
-                uint4 v = ld_cg_u4(src + ii * 32);
+                uint4 v = in[ii];
                 if (NORM) {
                     __half2* hv = reinterpret_cast<__half2*>(&v);
                     const __half2* hw = reinterpret_cast<const __half2*>(&wl[ii]);
@@ -78,7 +101,7 @@ __device__ __forceinline__ void load_bfrag_v2(uint4 (&b)[NT][4], const W4Params&
     }
 }
 
-template <int NT, bool NORM, bool XC, int WARPS, int STAGES>
+template <int NT, bool NORM, bool XC, int WARPS, int STAGES, bool INTL>
 __global__ void __launch_bounds__(WARPS * 32, ((NT <= 2 && WARPS == 8) ? 2 : 1)) k_w4a16_v2(const W4Params p) {
     using S = V2Smem<NT, WARPS, STAGES>;
     constexpr int kV2Warps = WARPS;
@@ -143,7 +166,9 @@ __global__ void __launch_bounds__(WARPS * 32, ((NT <= 2 && WARPS == 8) ? 2 : 1))
                         hv[e] = __hmul2(hv[e], hw[e]);
                     }
                 }
-                *reinterpret_cast<uint4*>(xs + (size_t)tok * xrow + ch * 16) = v;
+                // a lane's four chunks of a group lie 64 bytes apart: the reads below are free of bank conflicts
+                const int at = INTL ? (ch & ~15) | ((ch & 3) << 2) | ((ch >> 2) & 3) : ch;
+                *reinterpret_cast<uint4*>(xs + (size_t)tok * xrow + at * 16) = v;
             }
             if (NORM) {
                 sq = warp_sum(sq);
@@ -199,9 +224,9 @@ __global__ void __launch_bounds__(WARPS * 32, ((NT <= 2 && WARPS == 8) ? 2 : 1))
                 }
             } else if (NORM && ti == 0) {
                 // sum(x^2) only needs one pass over K: take it from the first tile
-                load_bfrag_v2<NT, NORM>(bcur, p, (g_begin + i) * kW4GroupK, g, t, ss);
+                load_bfrag_v2<NT, NORM, INTL>(bcur, p, (g_begin + i) * kW4GroupK, g, t, ss);
             } else {
-                load_bfrag_v2<NT, NORM>(bcur, p, (g_begin + i) * kW4GroupK, g, t, ss_dummy);
+                load_bfrag_v2<NT, NORM, INTL>(bcur, p, (g_begin + i) * kW4GroupK, g, t, ss_dummy);
             }
 
             mbar_wait(&bars[s], parity);
@@ -225,6 +250,17 @@ __global__ void __launch_bounds__(WARPS * 32, ((NT <= 2 && WARPS == 8) ? 2 : 1))
                         const int j = hh * 4 + jj;
                         uint32_t w = wj[jj];
                         uint32_t a[4];
+                        if constexpr (INTL) {
+                            // bytes = four consecutive k, the low nibbles row g, the high ones row g + 8: exact q - z by the same magic numbers
+                            const uint32_t lo = w & 0x0f0f0f0fu, hi = w & 0xf0f0f0f0u;
+                            const uint32_t q[4] = {__byte_perm(lo, 0x64646464u, 0x4140), __byte_perm(hi, 0x54545454u, 0x4140),
+                                                   __byte_perm(lo, 0x64646464u, 0x4342), __byte_perm(hi, 0x54545454u, 0x4342)};
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                const __half2 h = __hadd2(*reinterpret_cast<const __half2*>(&q[i]), (i & 1) ? z16 : z1);
+                                a[i] = *reinterpret_cast<const uint32_t*>(&h);
+                            }
+                        } else {
                         uint32_t p0 = lop3_and_or<0x000f000fu, 0x64006400u>(w);
                         uint32_t p1 = lop3_and_or<0x00f000f0u, 0x64006400u>(w);
                         w >>= 8;
@@ -238,6 +274,7 @@ __global__ void __launch_bounds__(WARPS * 32, ((NT <= 2 && WARPS == 8) ? 2 : 1))
                         a[1] = *reinterpret_cast<uint32_t*>(&h1);
                         a[2] = *reinterpret_cast<uint32_t*>(&h2);
                         a[3] = *reinterpret_cast<uint32_t*>(&h3);
+                        }
 #pragma unroll
                         for (int nt = 0; nt < NT; ++nt) {
                             const uint4 bv = bcur[nt][j >> 1];
@@ -392,50 +429,62 @@ __global__ void __launch_bounds__(WARPS * 32, ((NT <= 2 && WARPS == 8) ? 2 : 1))
 
 static int v2_num_sms() { return device_sm_count(); }
 
-template <int NT, bool NORM, bool XC, int WARPS, int STAGES>
+template <int NT, bool NORM, bool XC, int WARPS, int STAGES, bool INTL>
 static cudaError_t launch_v2_t(const W4Params& p, bool pdl, cudaStream_t stream) {
     using S = V2Smem<NT, WARPS, STAGES>;
     const int smem = S::kBytes + (XC ? p.mc * x_row_bytes(p.K) : 0);
     const int tiles = p.N / 32;
     const int max_ctas = v2_num_sms() * (WARPS == 8 ? 2 : 1);
     const int grid = tiles < max_ctas ? tiles : max_ctas;
-    return launch(k_w4a16_v2<NT, NORM, XC, WARPS, STAGES>, dim3(grid), dim3(WARPS * 32), (size_t)smem, stream, pdl, p);
+    return launch(k_w4a16_v2<NT, NORM, XC, WARPS, STAGES, INTL>, dim3(grid), dim3(WARPS * 32), (size_t)smem, stream, pdl, p);
 }
 
-template <int NT, int WARPS, int STAGES>
+template <int NT, int WARPS, int STAGES, bool INTL>
 static cudaError_t launch_v2_shape(const W4Params& p, bool pdl, cudaStream_t stream) {
-    const bool norm = p.ln_w != nullptr;
     // stage x in shared memory when the CTA budget allows (always true for M = 1 at the Llama shapes)
     const int budget = WARPS == 8 ? kV2TwoCtaBudget : kV2OneCtaBudget;
     const bool xc = V2Smem<NT, WARPS, STAGES>::kBytes + p.mc * x_row_bytes(p.K) <= budget;
-    if (xc)
-        return norm ? launch_v2_t<NT, true, true, WARPS, STAGES>(p, pdl, stream)
-                    : launch_v2_t<NT, false, true, WARPS, STAGES>(p, pdl, stream);
-    return norm ? launch_v2_t<NT, true, false, WARPS, STAGES>(p, pdl, stream)
-                : launch_v2_t<NT, false, false, WARPS, STAGES>(p, pdl, stream);
+    if constexpr (!INTL) {
+        if (p.ln_w != nullptr)
+            return xc ? launch_v2_t<NT, true, true, WARPS, STAGES, false>(p, pdl, stream)
+                      : launch_v2_t<NT, true, false, WARPS, STAGES, false>(p, pdl, stream);
+    }
+    return xc ? launch_v2_t<NT, false, true, WARPS, STAGES, INTL>(p, pdl, stream)
+              : launch_v2_t<NT, false, false, WARPS, STAGES, INTL>(p, pdl, stream);
 }
 
-template <int NT>
+template <int NT, bool INTL>
 static cudaError_t launch_v2_nt(const W4Params& p, bool pdl, cudaStream_t stream) {
     const bool tall = NT <= 2 && p.N / 32 <= v2_num_sms() && p.K / kW4GroupK >= 32;
-    if (tall) return launch_v2_shape<(NT <= 2 ? NT : 1), 16, 4>(p, pdl, stream);
-    return launch_v2_shape<NT, 8, (NT == 1 ? 5 : 4)>(p, pdl, stream);
+    if (tall) return launch_v2_shape<(NT <= 2 ? NT : 1), 16, 4, INTL>(p, pdl, stream);
+    return launch_v2_shape<NT, 8, (NT == 1 ? 5 : 4), INTL>(p, pdl, stream);
 }
 
 cudaError_t launch_w4_v2(const W4Params& p, bool pdl, cudaStream_t stream) {
-    if (p.mc <= 8) return launch_v2_nt<1>(p, pdl, stream);
-    if (p.mc <= 16) return launch_v2_nt<2>(p, pdl, stream);
-    return launch_v2_nt<4>(p, pdl, stream);
+    if (p.mc <= 8) return launch_v2_nt<1, false>(p, pdl, stream);
+    if (p.mc <= 16) return launch_v2_nt<2, false>(p, pdl, stream);
+    return launch_v2_nt<4, false>(p, pdl, stream);
+}
+
+cudaError_t launch_w4_v2_int_layout(const W4Params& p, bool pdl, cudaStream_t stream) {
+    W4Params q = p;
+    q.x32 = ((reinterpret_cast<uintptr_t>(p.x) | (size_t)p.ldx * 2) & 31) == 0;
+    return q.mc <= 8 ? launch_v2_nt<1, true>(q, pdl, stream) : launch_v2_nt<2, true>(q, pdl, stream);
 }
 
 cudaError_t prepare_w4_v2() {
     cudaError_t e;
-#define ZL_SET(NT, NORM, XC, W, ST)                                                                                \
-    e = cudaFuncSetAttribute(k_w4a16_v2<NT, NORM, XC, W, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize,         \
+#define ZL_SET(NT, NORM, XC, W, ST, INTL)                                                                          \
+    e = cudaFuncSetAttribute(k_w4a16_v2<NT, NORM, XC, W, ST, INTL>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
                              XC ? (W == 8 ? kV2TwoCtaBudget : kV2OneCtaBudget) : V2Smem<NT, W, ST>::kBytes);        \
     if (e != cudaSuccess) return e;
-#define ZL_SET4(NT, W, ST) ZL_SET(NT, false, false, W, ST) ZL_SET(NT, true, false, W, ST) ZL_SET(NT, false, true, W, ST) ZL_SET(NT, true, true, W, ST)
+#define ZL_SET4(NT, W, ST)                                                                                          \
+    ZL_SET(NT, false, false, W, ST, false) ZL_SET(NT, true, false, W, ST, false)                                    \
+    ZL_SET(NT, false, true, W, ST, false) ZL_SET(NT, true, true, W, ST, false)
+#define ZL_SETI(NT, W, ST) ZL_SET(NT, false, false, W, ST, true) ZL_SET(NT, false, true, W, ST, true)
     ZL_SET4(1, 8, 5) ZL_SET4(2, 8, 4) ZL_SET4(4, 8, 4) ZL_SET4(1, 16, 4) ZL_SET4(2, 16, 4)
+    ZL_SETI(1, 8, 5) ZL_SETI(2, 8, 4) ZL_SETI(1, 16, 4) ZL_SETI(2, 16, 4)
+#undef ZL_SETI
 #undef ZL_SET4
 #undef ZL_SET
     return cudaSuccess;
