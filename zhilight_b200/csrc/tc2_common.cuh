@@ -50,6 +50,32 @@ __device__ __forceinline__ bool tc2_wait(uint64_t* bar, uint32_t parity, volatil
     }
     return __all_sync(0xffffffffu, ok);
 }
+// The same for one thread (an elected lane that runs its warp's whole loop).
+__device__ __forceinline__ bool tc2_wait1(uint64_t* bar, uint32_t parity, volatile int* s_abort, unsigned* err, unsigned code) {
+    if (mbar_try_wait(bar, parity)) return true;
+    const long long t0 = clock64();
+    unsigned spins = 0;
+    while (!mbar_try_wait(bar, parity)) {
+        if ((++spins & 1023u) == 0 && (*s_abort || clock64() - t0 > 2000000000ll)) {
+            if (!*s_abort) *reinterpret_cast<volatile unsigned*>(err) = code;
+            *s_abort = 1;
+            return false;
+        }
+    }
+    return true;
+}
+// whether a phase has ended, without waiting for it
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 // after an abort: give copies and MMAs in flight time to land before shared memory and TMEM go away
 __device__ __forceinline__ void tc2_drain(volatile int* s_abort) {
     if (!*s_abort) return;

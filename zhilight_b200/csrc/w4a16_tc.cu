@@ -631,7 +631,7 @@ bool w4_tc_params(W4TcParams& q, const W4Params& p) {
         // the weight maps depend only on (address, N, K): encode once per weight matrix (cuTensorMapEncodeTiled costs
         // microseconds of host time per call)
         struct WMaps {
-            CUtensorMap w, t;
+            CUtensorMap w, w2, t;
         };
         static std::map<std::tuple<const void*, int, int>, WMaps> cache;
         static std::mutex mu;
@@ -642,10 +642,13 @@ bool w4_tc_params(W4TcParams& q, const W4Params& p) {
             const uint64_t G = (uint64_t)(p.K / kW4GroupK), nb = (uint64_t)p.N / 32;
             const uint64_t wd[4] = {16, 32, G, nb}, wstr[3] = {64, (uint64_t)kW4BlockBytes, G * kW4BlockBytes};
             const uint32_t wbox[4] = {16, 32, 1, 4};
+            const uint64_t w2d[4] = {32, 16, G, nb}, w2str[3] = {128, (uint64_t)kW4BlockBytes, G * kW4BlockBytes};
+            const uint32_t w2box[4] = {32, 16, 1, 4};
             const uint64_t td[3] = {20, G, nb}, tstr[2] = {(uint64_t)kW4BlockBytes, G * kW4BlockBytes};
             const uint32_t tbox[3] = {20, 1, 4};
             WMaps m;
             if (!tc_make_map_nd(&m.w, p.packed, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, wd, wstr, wbox, CU_TENSOR_MAP_SWIZZLE_64B) ||
+                !tc_make_map_nd(&m.w2, p.packed, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, w2d, w2str, w2box, CU_TENSOR_MAP_SWIZZLE_128B) ||
                 !tc_make_map_nd(&m.t, p.packed + kW4ScaleOff, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, td, tstr, tbox,
                                 CU_TENSOR_MAP_SWIZZLE_NONE))
                 return false;
@@ -653,6 +656,7 @@ bool w4_tc_params(W4TcParams& q, const W4Params& p) {
             it = cache.emplace(key, m).first;
         }
         q.wmap = it->second.w;
+        q.wmap2 = it->second.w2;
         q.tmap = it->second.t;
     }
     q.packed = p.packed;

@@ -8,8 +8,9 @@
 namespace zl {
 
 struct alignas(64) W4TcParams {
-    CUtensorMap xmap;           // x (M, K) fp16 row-major, box {64, rows of x per load}, 128-byte swizzle
+    CUtensorMap xmap;           // x (M, K) fp16 row-major, box {64, rows of x per load}, 128-byte swizzle; w4a16_tc2.cu: as [K / 64][M][64]
     CUtensorMap wmap;           // ZLW4I nibble words as [N/32][G][32 rows][64 B], box {64 B, 32, 1, 4}, 64-byte swizzle
+    CUtensorMap wmap2;          // the same as [N/32][G][16 pairs of rows][128 B], box {128 B, 16, 1, 4}, 128-byte swizzle (w4a16_tc2.cu)
     CUtensorMap tmap;           // the 80-byte scale / zero trailers as [N/32][G][80 B], box {80 B, 1, 4}
     const uint8_t* packed;      // ZLW4I
     const __half* bias;         // indexed by PACKED row

@@ -7,41 +7,50 @@
 // words.  Here
 //   * a tile is 256 rows of w by up to 256 tokens over two SMs: each converts its own 128 rows and loads half of the tokens;
 //   * tiles are whole, taken in turn by persistent pairs; the token tile's size is chosen so that the last wave is full;
-//   * up to 128 tokens there are two accumulators; with one, eight epilogue warps shorten the gap.
-// 28672 x 4096 with SwiGLU: 1000 tokens 499 -> 197 us, 256 tokens 128 -> 61; 4096 x 14336 with the residual: 1000 tokens 408 -> 91 us
-// (1290 TFLOP/s).  Bound by the tensor cores at 256 tokens (1030 cycles per 128-k group for 1024 of MMA, at the clock that the power limit
-// leaves); below 200 tokens by the hand-over of a group (830 cycles; two groups per stage were slower, 2380 per stage: too few slots).
+//   * up to 64 tokens there are two accumulators; with one, eight epilogue warps shorten the gap.
+// 28672 x 4096 with SwiGLU: 1000 tokens 499 -> 190 us, 256 tokens 128 -> 60; 4096 x 14336 with the residual: 1000 tokens 408 -> 88 us
+// (1360 TFLOP/s).  Bound by the tensor cores at 256 tokens (1084 cycles per 128-k group, at the clock that the power limit leaves); below 130
+// tokens by the conversion (650 cycles of a group, 340 of them when nothing else runs on the SM).
+//
+// What a stage costs one thread is what bounded small tiles before that (830 cycles): looking at a barrier takes it 120 - 200 cycles even when the
+// phase has ended, two TMA instructions and their votes 400.  So the issuing threads are single lanes that run their warp's loop alone and look at
+// the next barrier while this stage's work is on its way, a stage's x is one box, its weights are two and are issued by two warps in turn, the
+// weight boxes have rows of 128 bytes, the ring of weights takes what room there is, and six slots of A fit beside up to 128 tokens' accumulators.
+// 4096 x 14336, 256 rows 53.9 -> 45.4 us, 512 rows 55.9 -> 49.2; 28672 x 4096, 64 rows 36 -> 32; 6144 x 4096, 96 rows 22.4 -> 18.9.
 //
 //   warps 0-7    epilogue : quadrant = warp % 4, 16-token chunks in turns
 //   warps 8-23   dequant  : four groups of four take the stages (one 128-k group each) in turn, one group per stage slot; lane =
 //                           weight row, quadrant = warp % 4; their arrivals of both CTAs meet on the leader's barrier
-//   warp 24      weights  : tensor-TMA of the 4 ZLW4I records of a stage and their trailers, this CTA's 128 rows
-//   warp 25      x        : this CTA's half of the tokens, counted on the leader's barrier
-//   warp 26      MMA      : of the leader, 8 x 256 x ntok x 16 per stage; TMEM allocation
+//   warps 24, 25 weights  : tensor-TMA of the 4 ZLW4I records of a stage and their trailers, this CTA's 128 rows, stages in turn
+//   warp 26      x        : this CTA's half of the tokens, counted on the leader's barrier
+//   warp 27      MMA      : of the leader, 8 x 256 x ntok x 16 per stage; TMEM allocation
 //
 // The launch may start while its predecessor still runs, for as long as that takes (an all-reduce waits for its slowest rank).  A wait
-// that ends only after x has come would count that time, so no warp enters one before griddepcontrol.wait: the weights of the first RS
+// that ends only after x has come would count that time, so no warp enters one before griddepcontrol.wait: the weights of the ring's first
 // stages are fetched and each group's first stage is converted ahead of it, neither of which waits for anything but the weights.
 #include "tc2_common.cuh"
 #include "w4a16_tc.cuh"
 
 namespace zl {
 
+// What tensor memory leaves beside the accumulators: a slot takes 64 columns, an accumulator one per token.
+__host__ __device__ constexpr int t2_slots(int ntok) { return ntok > 128 ? 4 : 6; }
+__host__ __device__ constexpr int t2_accs(int ntok) { return ntok > 64 ? 1 : 2; }
+__host__ __device__ constexpr int t2_x_bytes(int ntok) { return ntok * 128; }   // of a slot and CTA: [64-k atom][ntok / 2 tokens][128 B]
+
 struct T2Cfg {
     static constexpr int kEpiWarps = 8, kDqWarps = 16, kGroupWarps = 4;
-    static constexpr int kWarpDq0 = kEpiWarps, kWarpRaw = kWarpDq0 + kDqWarps, kWarpX = kWarpRaw + 1, kWarpMma = kWarpRaw + 2;
+    static constexpr int kWarpDq0 = kEpiWarps, kWarpRaw = kWarpDq0 + kDqWarps, kRawWarps = 2, kWarpX = kWarpRaw + kRawWarps, kWarpMma = kWarpX + 1;
     static constexpr int kThreads = (kWarpMma + 1) * 32;
-    static constexpr int AS = 4;                                       // stages of A (TMEM, 64 columns each) and x (shared memory)
-    static constexpr int RS = 8;                                       // stages of packed weights
-    static constexpr int kACol0 = 256;                                 // accumulators: columns 0 .. 255
-    static constexpr int kXStage = 2 * 128 * 128;                      // [64-k atom][up to 128 tokens][128 B]
+    static constexpr int kGroups = kDqWarps / kGroupWarps;
+    static constexpr int kMaxSlots = 6;                                // of A (TMEM, 64 columns each) and x (shared memory)
+    static constexpr int kMaxRaw = 16;                                 // stages of packed weights
     static constexpr int kNib = 4 * 2048, kTr = 384;                   // four records' nibbles; their 80-byte trailers, padded
-    static constexpr int kNibOff = AS * kXStage;
-    static constexpr int kTrOff = kNibOff + RS * kNib;
-    static constexpr int kBarOff = kTrOff + RS * kTr;
-    static constexpr int kMiscOff = kBarOff + (2 * RS + 2 * AS + 4) * 8;
+    static constexpr int kRing = 230400;                               // slots of x, then as many of the weights as fit
+    static constexpr int kBarOff = kRing;
+    static constexpr int kMiscOff = kBarOff + (2 * kMaxRaw + 2 * kMaxSlots + 4) * 8;
     static constexpr int kBytes = kMiscOff + 16 + 1024;                // + slack for the manual 1024-byte alignment
-    static_assert(kACol0 + AS * 64 <= 512, "TMEM columns");
+    static_assert(t2_slots(256) * 64 + 256 <= 512 && t2_slots(128) * 64 + 128 <= 512, "TMEM columns");
     static_assert(kBytes <= 232448, "shared memory");
 };
 
@@ -61,10 +70,10 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
     extern __shared__ uint8_t smem_dyn[];
     uint8_t* smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
     uint64_t* raw_full = reinterpret_cast<uint64_t*>(smem + C::kBarOff);
-    uint64_t* raw_empty = raw_full + C::RS;
-    uint64_t* a_full = raw_empty + C::RS;      // leader's: a dequant group of each CTA, and the x bytes of both
-    uint64_t* ax_empty = a_full + C::AS;
-    uint64_t* acc_full = ax_empty + C::AS;
+    uint64_t* raw_empty = raw_full + C::kMaxRaw;
+    uint64_t* a_full = raw_empty + C::kMaxRaw;      // leader's: a dequant group of each CTA, and the x bytes of both
+    uint64_t* ax_empty = a_full + C::kMaxSlots;
+    uint64_t* acc_full = ax_empty + C::kMaxSlots;
     uint64_t* acc_empty = acc_full + 2;        // leader's: the epilogue warps of both CTAs
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(smem + C::kMiscOff);
     volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
@@ -72,14 +81,18 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
     const uint32_t rank = cluster_rank();
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     const int G = p.K / kW4GroupK;
-    const int nacc = p.ntok <= 128 ? 2 : 1;
+    const int slots = t2_slots(p.ntok), nacc = t2_accs(p.ntok), xstage = t2_x_bytes(p.ntok), acol0 = 512 - slots * 64;
+    // a weight slot is held while its group converts and is then a round trip to L2 from being full again: more than two per group
+    const int rslots = min(C::kMaxRaw, (C::kRing - slots * xstage) / (C::kNib + C::kTr));
+    uint8_t* const nibs = smem + slots * xstage;
+    uint8_t* const trs = nibs + rslots * C::kNib;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < C::RS; ++i) {
+        for (int i = 0; i < rslots; ++i) {
             mbar_init(&raw_full[i], 1);
             mbar_init(&raw_empty[i], C::kGroupWarps);
         }
-        for (int i = 0; i < C::AS; ++i) {
+        for (int i = 0; i < slots; ++i) {
             mbar_init(&a_full[i], 2 * C::kGroupWarps + 1);
             mbar_init(&ax_empty[i], 1);
         }
@@ -99,89 +112,94 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
     const uint32_t tmem = *s_tmem;
     T2Tile t;
 
-    if (warp == C::kWarpRaw) {
+    if (warp >= C::kWarpRaw && warp < C::kWarpX) {
         // constants: may run ahead of the predecessor kernel (PDL).  The row tiles of one wave are read by several pairs and again
         // by the next token tiles: no evict-first hint here
-        int rs = 0, st = 0;
-        uint32_t ph = 0;
-        bool ok = true;
-        for (int i = pair; ok && t2_tile(p, i, t); i += pairs) {
-            const int rec = (t.n0 + (int)rank * 128) / 32;
-            for (int g = 0; g < G; ++g, ++st) {
-                if (st == C::RS) pdl_wait();
-                if (!(ok = tc2_wait(&raw_empty[rs], ph ^ 1u, s_abort, p.err, 0x3100 + rs))) break;
-                if (tc_elect_one()) {
-                    mbar_expect_tx(&raw_full[rs], C::kNib + 4 * 80);
+        if (tc_elect_one()) {
+            // the two warps take the stages in turn: issuing the copies of one takes a thread 400 cycles
+            int g = warp - C::kWarpRaw, rs = g, st = g;
+            uint32_t ph = 0;
+            bool ok = true, free = false, early = true;
+            for (int i = pair; ok && t2_tile(p, i, t); i += pairs, g -= G) {
+                const int rec = (t.n0 + (int)rank * 128) / 32;
+                for (; g < G; g += C::kRawWarps, st += C::kRawWarps) {
+                    if (early && st >= rslots) {
+                        pdl_wait();
+                        early = false;
+                    }
+                    if (!free && !(ok = tc2_wait1(&raw_empty[rs], ph ^ 1u, s_abort, p.err, 0x3100 + rs))) break;
+                    uint64_t* const full = &raw_full[rs];
+                    const uint32_t nib = smem_u32(nibs + rs * C::kNib), tr = smem_u32(trs + rs * C::kTr), bar = smem_u32(full);
+                    rs += C::kRawWarps;
+                    if (rs >= rslots) {
+                        rs -= rslots;
+                        ph ^= 1u;
+                    }
+                    free = mbar_test(&raw_empty[rs], ph ^ 1u);
+                    mbar_expect_tx(full, C::kNib + 4 * 80);
                     asm volatile(
-                        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(
-                            smem_u32(smem + C::kNibOff + rs * C::kNib)),
-                        "l"(reinterpret_cast<uint64_t>(&p.wmap)), "r"(0), "r"(0), "r"(g), "r"(rec), "r"(smem_u32(&raw_full[rs]))
+                        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(nib),
+                        "l"(reinterpret_cast<uint64_t>(&p.wmap2)), "r"(0), "r"(0), "r"(g), "r"(rec), "r"(bar)
                         : "memory");
                     asm volatile(
-                        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
-                            smem_u32(smem + C::kTrOff + rs * C::kTr)),
-                        "l"(reinterpret_cast<uint64_t>(&p.tmap)), "r"(0), "r"(g), "r"(rec), "r"(smem_u32(&raw_full[rs]))
+                        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(tr),
+                        "l"(reinterpret_cast<uint64_t>(&p.tmap)), "r"(0), "r"(g), "r"(rec), "r"(bar)
                         : "memory");
-                }
-                __syncwarp();
-                if (++rs == C::RS) {
-                    rs = 0;
-                    ph ^= 1u;
                 }
             }
         }
+        __syncwarp();
     } else if (warp == C::kWarpX) {
         pdl_wait();   // activations: produced by the predecessor kernel
-        int as = 0;
-        uint32_t ph = 0;
-        bool ok = true;
-        const int box = p.ntok >> 1;   // rows of a load; a shorter last tile loads rows it does not use
-        for (int i = pair; ok && t2_tile(p, i, t); i += pairs) {
-            const int tb = t.t0 + (int)rank * (t.ntok >> 1);
-            for (int g = 0; g < G; ++g) {
-                if (!(ok = tc2_wait(&ax_empty[as], ph ^ 1u, s_abort, p.err, 0x3200 + as))) break;
-                if (tc_elect_one()) {
-                    if (rank == 0) mbar_expect_tx(&a_full[as], (uint32_t)(4 * box * 128));
-                    const uint32_t bar = cluster_map(smem_u32(&a_full[as]), 0);
-                    uint8_t* dst = smem + as * C::kXStage;
-                    tma2_load_3d(dst, &p.xmap, g * kW4GroupK, tb, 0, bar);
-                    tma2_load_3d(dst + box * 128, &p.xmap, g * kW4GroupK + 64, tb, 0, bar);
-                }
-                __syncwarp();
-                if (++as == C::AS) {
-                    as = 0;
-                    ph ^= 1u;
-                }
-            }
-        }
-    } else if (warp == C::kWarpMma) {
-        if (rank == 0) {
-            pdl_wait();
-            int as = 0, acc = 0;
-            uint32_t ph = 0, acc_ph = 0;
-            bool ok = true;
-            const uint64_t atom = (uint64_t)(((p.ntok >> 1) * 128) >> 4);   // descriptor step from k 0..63 to k 64..127 of a stage
+        if (tc_elect_one()) {
+            int as = 0;
+            uint32_t ph = 0;
+            bool ok = true, free = false;
+            const int box = p.ntok >> 1;   // rows of a load; a shorter last tile loads rows it does not use
             for (int i = pair; ok && t2_tile(p, i, t); i += pairs) {
-                if (!(ok = tc2_wait(&acc_empty[acc], acc_ph ^ 1u, s_abort, p.err, 0x3300 + acc))) break;
-                tc_fence_after();
-                const uint32_t d = tmem + (uint32_t)(acc * 128), idesc = tc2_idesc(false, t.ntok);
+                const int tb = t.t0 + (int)rank * (t.ntok >> 1);
                 for (int g = 0; g < G; ++g) {
-                    if (!(ok = tc2_wait(&a_full[as], ph, s_abort, p.err, 0x3400 + as))) break;
-                    tc_fence_after();
-                    if (tc_elect_one()) {
-                        const uint32_t a = tmem + (uint32_t)(C::kACol0 + as * 64);
-                        const uint64_t xd = tc_desc_sw128(smem_u32(smem + as * C::kXStage));
-#pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            tc2_mma_ts(d, a + (uint32_t)(j * 8), xd + (j >> 2) * atom + (uint64_t)((j & 3) * 2), idesc, (g > 0 || j > 0) ? 1u : 0u);
-                        tc2_commit(&ax_empty[as]);
-                        if (g == G - 1) tc2_commit(&acc_full[acc]);
-                    }
-                    __syncwarp();
-                    if (++as == C::AS) {
+                    if (!free && !(ok = tc2_wait1(&ax_empty[as], ph ^ 1u, s_abort, p.err, 0x3200 + as))) break;
+                    uint64_t* const full = &a_full[as];
+                    uint8_t* dst = smem + as * xstage;
+                    if (++as == slots) {
                         as = 0;
                         ph ^= 1u;
                     }
+                    free = mbar_test(&ax_empty[as], ph ^ 1u);
+                    if (rank == 0) mbar_expect_tx(full, (uint32_t)(4 * box * 128));
+                    const uint32_t bar = cluster_map(smem_u32(full), 0);
+                    tma2_load_3d(dst, &p.xmap, 0, tb, g * 2, bar);   // two 64-k atoms
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == C::kWarpMma) {
+        pdl_wait();
+        if (rank == 0 && tc_elect_one()) {
+            int as = 0, acc = 0;
+            uint32_t ph = 0, acc_ph = 0;
+            bool ok = true, ready = false;
+            const uint64_t atom = (uint64_t)(((p.ntok >> 1) * 128) >> 4);   // descriptor step from k 0..63 to k 64..127 of a stage
+            for (int i = pair; ok && t2_tile(p, i, t); i += pairs) {
+                if (!(ok = tc2_wait1(&acc_empty[acc], acc_ph ^ 1u, s_abort, p.err, 0x3300 + acc))) break;
+                const uint32_t d = tmem + (uint32_t)(acc * 64), idesc = tc2_idesc(false, t.ntok);
+                for (int g = 0; g < G; ++g) {
+                    if (!ready && !(ok = tc2_wait1(&a_full[as], ph, s_abort, p.err, 0x3400 + as))) break;
+                    const uint32_t a = tmem + (uint32_t)(acol0 + as * 64);
+                    const uint64_t xd = tc_desc_sw128(smem_u32(smem + as * xstage));
+                    uint64_t* const used = &ax_empty[as];
+                    if (++as == slots) {
+                        as = 0;
+                        ph ^= 1u;
+                    }
+                    ready = mbar_test(&a_full[as], ph);   // looking at a barrier takes 200 cycles: they pass under this stage's MMAs
+                    tc_fence_after();
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        tc2_mma_ts(d, a + (uint32_t)(j * 8), xd + (j >> 2) * atom + (uint64_t)((j & 3) * 2), idesc, (g > 0 || j > 0) ? 1u : 0u);
+                    tc2_commit(used);
+                    if (g == G - 1) tc2_commit(&acc_full[acc]);
                 }
                 if (++acc == nacc) {
                     acc = 0;
@@ -189,69 +207,82 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
                 }
             }
         }
+        __syncwarp();
     } else if (warp >= C::kWarpDq0) {
-        const int as = (warp - C::kWarpDq0) >> 2, q = warp & 3;   // the group's stage slot
+        const int group = (warp - C::kWarpDq0) >> 2, q = warp & 3;
         const int tt = lane >> 4, hi = (lane >> 3) & 1, g8 = lane & 7;
         const uint32_t mask = hi ? 0xf0f0f0f0u : 0x0f0f0f0fu;
         const uint32_t magic = hi ? 0x54545454u : 0x64646464u;   // 64 + n / 16 for a high nibble n, 1024 + n for a low one
-        const uint32_t sw = (uint32_t)(g8 >> 1) & 3u;            // the map's 64-byte swizzle: chunk ^= (row >> 1) & 3
-        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(C::kACol0 + as * 64);
-        const uint32_t full = cluster_map(smem_u32(&a_full[as]), 0);
-        int st = 0;
-        uint32_t ph = 0;
-        bool ok = true;
-        for (int i = pair; ok && t2_tile(p, i, t); i += pairs) {
-            for (int g = 0; g < G; ++g, ++st) {
-                if (st % C::AS != as) continue;
-                if (st == as + C::AS) pdl_wait();
-                const int rs = st % C::RS;
-                if (!(ok = tc2_wait(&raw_full[rs], (uint32_t)(st / C::RS) & 1u, s_abort, p.err, 0x3600 + rs))) break;
-                const uint8_t* nib = smem + C::kNibOff + rs * C::kNib + q * 2048;
-                const uint8_t* tr = smem + C::kTrOff + rs * C::kTr + q * 80;
-                const __half2 sc2 = *reinterpret_cast<const __half2*>(tr + (tt * 8 + g8) * 4);
-                const int zz = tr[64 + tt * 8 + g8];
-                const __half2 cz = __float2half2_rn(hi ? (float)(64 + (zz >> 4)) : (float)(1024 + (zz & 0xF)));
-                const __half2 s2 = hi ? __half2half2(__high2half(sc2)) : __half2half2(__low2half(sc2));
+        const uint32_t sw = (uint32_t)(g8 >> 1);                 // the map's 128-byte swizzle: chunk ^= pair of rows & 7
+        const uint32_t tlane = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)acol0;
+        int stages = 0;
+        for (int i = pair; t2_tile(p, i, t); i += pairs) stages += G;
+        int as = group, rs = group;
+        uint32_t ph = 0, rph = 0;
+        bool raw_ready = false;
+        for (int st = group; st < stages; st += C::kGroups) {
+            if (st >= slots && st < slots + C::kGroups) pdl_wait();
+            if (!raw_ready && !tc2_wait(&raw_full[rs], rph, s_abort, p.err, 0x3600 + rs)) break;
+            // looking at a barrier takes 200 cycles: they pass under the conversion
+            const bool free = mbar_test(&ax_empty[as], ph ^ 1u);
+            const uint8_t* nib = nibs + rs * C::kNib + q * 2048 + (g8 >> 1) * 128;
+            const uint8_t* tr = trs + rs * C::kTr + q * 80;
+            uint64_t* const used = &raw_empty[rs];
+            rs += C::kGroups;
+            if (rs >= rslots) {
+                rs -= rslots;
+                rph ^= 1u;
+            }
+            const bool next = mbar_test(&raw_full[rs], rph);
+            const __half2 sc2 = *reinterpret_cast<const __half2*>(tr + (tt * 8 + g8) * 4);
+            const int zz = tr[64 + tt * 8 + g8];
+            const __half2 cz = __float2half2_rn(hi ? (float)(64 + (zz >> 4)) : (float)(1024 + (zz & 0xF)));
+            const __half2 s2 = hi ? __half2half2(__high2half(sc2)) : __half2half2(__low2half(sc2));
+            const uint32_t taddr = tlane + (uint32_t)(as * 64);
+            bool ok = true;
 #pragma unroll
-                for (int ks = 0; ks < 2; ++ks) {    // 64 k at a time: 32 columns
-                    uint4 wv[4];
+            for (int ks = 0; ks < 2; ++ks) {    // 64 k at a time: 32 columns
+                uint4 wv[4];
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        // 16-k chunk kc of the group: k = 32 t + 16 hh + ..., record row (2 tt + hh) * 8 + g, chunk t
-                        const int kc = ks * 4 + c, tq = kc >> 1, hh = kc & 1;
-                        wv[c] = *reinterpret_cast<const uint4*>(nib + ((tt * 2 + hh) * 8 + g8) * 64 + (((uint32_t)tq ^ sw) << 4));
-                    }
-                    if (ks == 1) {
-                        __syncwarp();               // every lane's shared-memory reads of the stage have returned
-                        if (lane == 0) mbar_arrive(&raw_empty[rs]);
-                    }
-                    uint32_t r[2][16];
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        const uint32_t words[4] = {wv[c].x, wv[c].y, wv[c].z, wv[c].w};
-#pragma unroll
-                        for (int wq = 0; wq < 4; ++wq) {
-                            const uint32_t wm = words[wq] & mask;
-                            uint32_t a0 = __byte_perm(wm, magic, 0x4140), a1 = __byte_perm(wm, magic, 0x4342);
-                            __half2 v0 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&a0), cz), s2);
-                            __half2 v1 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&a1), cz), s2);
-                            r[c >> 1][(c & 1) * 8 + wq * 2] = *reinterpret_cast<uint32_t*>(&v0);
-                            r[c >> 1][(c & 1) * 8 + wq * 2 + 1] = *reinterpret_cast<uint32_t*>(&v1);
-                        }
-                    }
-                    if (ks == 0) {
-                        if (!(ok = tc2_wait(&ax_empty[as], ph ^ 1u, s_abort, p.err, 0x3700 + as))) break;
-                        tc_fence_after();
-                    }
-                    tc_st16(taddr + (uint32_t)(ks * 32), r[0]);
-                    tc_st16(taddr + (uint32_t)(ks * 32 + 16), r[1]);
+                for (int c = 0; c < 4; ++c) {
+                    // 16-k chunk kc of the group: k = 32 t + 16 hh + ..., record row (2 tt + hh) * 8 + g, chunk t
+                    const int kc = ks * 4 + c, tq = kc >> 1, hh = kc & 1;
+                    wv[c] = *reinterpret_cast<const uint4*>(nib + (tt * 2 + hh) * 512 + (((((uint32_t)g8 ^ hh) & 1) << 6) | ((tq ^ sw) << 4)));
                 }
-                if (!ok) break;
+                if (ks == 1) {
+                    __syncwarp();               // every lane's shared-memory reads of the stage have returned
+                    if (lane == 0) mbar_arrive(used);
+                }
+                uint32_t r[2][16];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const uint32_t words[4] = {wv[c].x, wv[c].y, wv[c].z, wv[c].w};
+#pragma unroll
+                    for (int wq = 0; wq < 4; ++wq) {
+                        const uint32_t wm = words[wq] & mask;
+                        uint32_t a0 = __byte_perm(wm, magic, 0x4140), a1 = __byte_perm(wm, magic, 0x4342);
+                        __half2 v0 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&a0), cz), s2);
+                        __half2 v1 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&a1), cz), s2);
+                        r[c >> 1][(c & 1) * 8 + wq * 2] = *reinterpret_cast<uint32_t*>(&v0);
+                        r[c >> 1][(c & 1) * 8 + wq * 2 + 1] = *reinterpret_cast<uint32_t*>(&v1);
+                    }
+                }
+                if (ks == 0) {
+                    if (!__all_sync(0xffffffffu, free) && !(ok = tc2_wait(&ax_empty[as], ph ^ 1u, s_abort, p.err, 0x3700 + as))) break;
+                    tc_fence_after();
+                }
+                tc_st16(taddr + (uint32_t)(ks * 32), r[0]);
+                tc_st16(taddr + (uint32_t)(ks * 32 + 16), r[1]);
+            }
+            if (!ok) break;
+            tc_wait_st();
+            tc_fence_before();
+            raw_ready = __all_sync(0xffffffffu, next);   // one arrival per warp
+            if (lane == 0) mbar_arrive_at(cluster_map(smem_u32(&a_full[as]), 0));
+            as += C::kGroups;
+            if (as >= slots) {
+                as -= slots;
                 ph ^= 1u;
-                tc_wait_st();
-                tc_fence_before();
-                __syncwarp();                       // one arrival per warp
-                if (lane == 0) mbar_arrive_at(full);
             }
         }
     } else {
@@ -266,7 +297,7 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
             if (res) tc_fetch_residual(p, prow, lane, t.t0 + set * 16, rnext);
             if (!tc2_wait(&acc_full[acc], acc_ph, s_abort, p.err, 0x3800 + acc)) break;
             tc_fence_after();
-            const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * 128);
+            const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * 64);
             if (prow < p.N) {               // N % 128 == 0: all of the CTA's rows or none
                 for (int c0 = set * 16; c0 < t.ntok && t.t0 + c0 < p.M; c0 += 32) {
                     float v[16];
@@ -307,11 +338,12 @@ cudaError_t prepare_w4_tc2() {
     return cudaFuncSetAttribute(k_w4a16_tc2, cudaFuncAttributeMaxDynamicSharedMemorySize, T2Cfg::kBytes);
 }
 
-// Tokens per tile: the waves of the launch times a tile's cost.  A 128-k group costs its MMAs (4 cycles per token) or the conversion and
-// hand-over of its weights (830 cycles), whichever is longer; with one accumulator the epilogue comes on top.
+// Tokens per tile: the waves of the launch times a tile's cost.  A 128-k group costs its MMAs (4.24 cycles per token) or the conversion and
+// hand-over of its weights (650 cycles, and from about 100 tokens on both get into each other's way: 400 + 2.6 per token), whichever is
+// longer; with one accumulator the epilogue comes on top.
 static double t2_cost(int n, long long tiles, int G, int pairs) {
-    const double group = 4.0 * n > 830.0 ? 4.0 * n : 830.0;
-    return (double)((tiles + pairs - 1) / pairs) * (G * group + (n > 128 ? 16.0 * n : 500.0));
+    const double group = fmax(650.0, fmax(4.24 * n, 400.0 + 2.6 * n));
+    return (double)((tiles + pairs - 1) / pairs) * (G * group + (n > 64 ? 14.0 * n : 300.0));
 }
 static int t2_pick_ntok(int M, int row_tiles, int G, int pairs) {
     int best = 32;
@@ -324,13 +356,13 @@ static int t2_pick_ntok(int M, int row_tiles, int G, int pairs) {
 
 // Whether M tokens are this kernel's.  Beyond 256 w4a16_tc.cu would need several passes; below, whole tiles on few pairs stand against
 // its ranges over all SMs and their exchange: 10 us + 4.2 ns per token and million weights.  Measured, this kernel against that one:
-// 28672 x 4096 at M = 32 / 64 / 128: 34 / 35 / 39 against 34 / 41 / 60 us; 4096 x 14336 at M = 128 / 192 / 256: 51 / 52 / 54 against
-// 39 / 56 / 64; 6144 x 4096 at M = 64 / 128: 22 / 23 against 21 / 32; 4096 x 4096 at M = 128 / 192: 22 / 23 against 21 / 27.
+// 28672 x 4096 at M = 48 / 64 / 128: 32 / 32 / 38 against 37 / 41 / 60 us; 4096 x 14336 at M = 128 / 144 / 192: 45 / 45 / 44 against
+// 39 / 46 / 56; 6144 x 4096 at M = 64 / 96: 19 / 19 against 21 / 26; 4096 x 4096 at M = 112 / 144: 20 / 20 against 21 / 24.
 bool w4_tc2_route(int M, int N, int K) {
     if (M <= 16 || N % kTcRows || K % kW4GroupK) return false;
     if (M > 256) return true;
     const int row_tiles = cdiv(N, kTc2Rows), G = K / kW4GroupK, pairs = device_sm_count() / 2, n = t2_pick_ntok(M, row_tiles, G, pairs);
-    const double here = 5.0 + t2_cost(n, (long long)row_tiles * cdiv(M, n), G, pairs) / 1900.0;
+    const double here = 7.0 + t2_cost(n, (long long)row_tiles * cdiv(M, n), G, pairs) / 1900.0;
     return here < 10.0 + 4.2e-9 * M * (double)N * K;
 }
 
@@ -344,7 +376,11 @@ cudaError_t launch_w4_tc2(const W4Params& p, bool pdl, cudaStream_t stream) {
     q.err = words + kWaitW4Pairs;
     q.ntok = t2_pick_ntok(p.mc, row_tiles, G, max_pairs);
     q.tok_tiles = cdiv(p.mc, q.ntok);
-    if (!tc2_map_3d(&q.xmap, p.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, p.K, p.mc, 1, p.ldx, 0, q.ntok / 2)) return cudaErrorInvalidValue;
+    {   // x as [K / 64][M][64]: a stage's two atoms of half the tokens are one box
+        const uint64_t dims[3] = {64, (uint64_t)p.mc, (uint64_t)p.K / 64}, strides[2] = {(uint64_t)p.ldx * 2, 128};
+        const uint32_t box[3] = {64, (uint32_t)q.ntok / 2, 2};
+        if (!tc_make_map_nd(&q.xmap, p.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B)) return cudaErrorInvalidValue;
+    }
     const int tiles = row_tiles * q.tok_tiles;
     return launch_pairs(k_w4a16_tc2, tiles < max_pairs ? tiles : max_pairs, dim3(T2Cfg::kThreads), (size_t)T2Cfg::kBytes, stream, pdl, q);
 }
