@@ -12,11 +12,13 @@
 //   warp 5     O += P V, P from tensor memory, V as it lies (rows of keys: the B operand along n), O in tensor memory; TMEM allocation
 //   warps 6-7  K and V tiles by 16-byte cp.async into the swizzled layout (the buffers' addresses are known to the device only), K a tile ahead
 //
-// fp16 models carry p * 2^10 in fp16, bf16 models p as bf16 hi + lo (two MMAs), as the decode kernels do.  A row's reference maximum only
-// follows the true one once that has grown by 2^5 (fp16) or 2^8, so that O is seldom rescaled.  Two CTAs share an SM (256 columns each): one's
-// MMAs run under the other's softmax.  Bound by the MMAs (bf16, a tile: 450 cycles of S, whose operands come at 128 bytes a cycle, and 580 of
-// P V) and, for short prompts, by a chain of about 10 us (launch, mask, first loads, merge).  500 rows behind 1000 positions, bf16, 32 heads on
-// 8: 62 us on mma.sync with 64-row blocks (65 us of kernel time), 29 here; 512 x 1500 with 64 heads on 8, all launches of the call: 120 -> 50.
+// Probabilities are carried as a 16-bit value and the rest of it as another (two MMAs), fp16 models' times 2^10.  A row's reference maximum only
+// follows the true one once that has grown by 2^5 (fp16) or 2^8, so that O is seldom rescaled; with one fp16 value that would cost precision (the
+// largest probability is no power of two any more: 2.8e-4 from 64 bits against 2.55e-4), with two it is 2.1e-4, all of it the output's rounding.  Two
+// CTAs share an SM (256 columns each): one's MMAs run under the other's softmax.  Bound by the MMAs (a tile: 450 cycles of S, whose operands
+// come at 128 bytes a cycle, and 580 of P V) and, for short prompts, by a chain of about 10 us (launch, mask, first loads, merge).  500 rows
+// behind 1000 positions, bf16, 32 heads on 8: 65 us on mma.sync with 64-row blocks, 29 here; 512 x 1500 with 64 heads on 8, all launches of the
+// call: 120 -> 50.
 //
 // An int8 mask is turned into bits first (k_mask_bits), once for all kv heads, together with each row's last visible key: tiles behind the last
 // key any row of the block sees are never loaded, which halves a causal prompt's work.  Few blocks are cut along their keys: the CTAs of a
@@ -285,7 +287,7 @@ k_attn_prompt(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* 
                 const uint64_t vd = pa_desc_mn(smem_u32(smem + C::kVOff + st * C::kTile), kPaKeys * 128);
                 const uint32_t p = tmem + (uint32_t)(C::kS + st * 64);
 #pragma unroll
-                for (int h = 0; h < (kHalf ? 1 : 2); ++h)        // bf16: the probabilities' upper halves, then the lower ones
+                for (int h = 0; h < 2; ++h)                      // the probabilities' upper halves, then the lower ones
 #pragma unroll
                     for (int k = 0; k < kPaKeys / 16; ++k)
                         pa_mma_ts(tmem, p + (uint32_t)(h * 32 + k * 8), vd + (uint64_t)(k * (16 * 128 / 16)), id, (j > 0 || h > 0 || k > 0) ? 1u : 0u);
@@ -392,6 +394,10 @@ k_attn_prompt(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* 
                     if constexpr (kHalf) {
                         const __half2 h = __floats2half2_rn(x, y);
                         hi[i] = *reinterpret_cast<const uint32_t*>(&h);
+                        const float2 f = __half22float2(h);
+                        pa_split(pa_fma2(pa_two(f.x, f.y), minus, pa_two(x, y)), x, y);
+                        const __half2 e = __floats2half2_rn(x, y);
+                        lo[i] = *reinterpret_cast<const uint32_t*>(&e);
                     } else {
                         const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
                         hi[i] = *reinterpret_cast<const uint32_t*>(&h);
@@ -401,7 +407,7 @@ k_attn_prompt(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* 
                     }
                 }
                 tc_st16(ts + (uint32_t)(half * 16), hi);
-                if constexpr (!kHalf) tc_st16(ts + (uint32_t)(32 + half * 16), lo);
+                tc_st16(ts + (uint32_t)(32 + half * 16), lo);
             }
             float s0, s1;
             pa_split(sum, s0, s1);
