@@ -440,6 +440,7 @@ enum {
  * ZL_F16 / ZL_BF16 (tensor cores, fp32 accumulation) or ZL_F32 (plain fp32 FMAs, no reduced-precision mode);
  * out_dtype = in_dtype or ZL_F32; gate (fp32, same indexing as y with ldg / gate_batch_stride) for the gate epilogue. */
 int zl_gemm_nt_pairs_route(int M, int N, int K, int batch); /* 1: 16-bit inputs with aligned rows run on pairs of SMs, 0: on the tile kernels */
+int zl_gemm_pairs_splits(int M, int N, int K, int batch, int elem_bytes); /* how many pairs share the K of a tile there (inputs of 1 or 2 bytes): 1, 2 or 4 */
 int zl_gemm_nt(const void* x, long long ldx, long long x_batch_stride, const void* w, long long ldw,
                long long w_batch_stride, void* y, long long ldy, long long y_batch_stride, int M, int N, int K, int batch,
                int in_dtype, int out_dtype, int epilogue, const float* gate, long long ldg, long long gate_batch_stride,

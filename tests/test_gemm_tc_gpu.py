@@ -93,6 +93,27 @@ def test_batches(lib, cuda, b, m, n, k):
     _close(ops.gemm_nt(x, w, out_dtype=torch.float32), prod(x.double(), w.double()), prod(x.double().abs(), w.double().abs()), k, torch.float32)
 
 
+@pytest.mark.parametrize("dtype,out", [(BF, torch.float32), (HF, HF)])
+@pytest.mark.parametrize("m,n,k,splits", [(33, 512, 8192, 4), (65, 250, 8200, 4), (47, 4096, 6152, 2), (200, 1000, 8192, 4), (256, 3000, 10240, 4), (100, 130, 2056, 4)])
+def test_long_sums_of_few_tiles(lib, cuda, dtype, out, m, n, k, splits):
+    """The pairs of a cluster share a tile's K: chunks of 16 rows that go round between two and four owners, the last one of 1 to 16, parts of unequal
+    length, epilogues behind the exchange, the same result each time."""
+    from zhilight_b200 import ops
+    assert lib.zl_gemm_pairs_splits(m, n, k, 1, 2) == splits
+    g = torch.Generator().manual_seed(m + n)
+    x, w, b = _rand(g, m, k, dtype=dtype), _rand(g, n, k, dtype=dtype), torch.randn(n, generator=g).cuda()
+    ref, mag = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    y = ops.gemm_nt_bias(x, w, b, out_dtype=out)
+    _close(y, ref + b.double(), mag + b.double().abs(), k, out)
+    assert torch.equal(y, ops.gemm_nt_bias(x, w, b, out_dtype=out))
+    y = ops.gemm_nt(x, w, torch.float32, ops.GEMM_EPI_RELU2)
+    assert float((y.double() - F.relu(ref) ** 2).norm() / (F.relu(ref) ** 2).norm()) < 1e-5
+    xb, wb = _rand(g, 2, 40, k, dtype=dtype), _rand(g, 2, 300, k, dtype=dtype)
+    assert lib.zl_gemm_pairs_splits(40, 300, k, 2, 2) > 1
+    prod = lambda a, c: torch.einsum("bmk,bnk->bmn", a, c)  # noqa: E731
+    _close(ops.gemm_nt(xb, wb, out_dtype=out), prod(xb.double(), wb.double()), prod(xb.double().abs(), wb.double().abs()), k, out)
+
+
 @pytest.mark.parametrize("dtype", [BF, HF])
 @pytest.mark.parametrize("sizes", [[0, 9, 1, 0, 31], [32, 33, 0, 64, 1], [1] * 150, [256, 0, 257, 3], [700, 12]])
 @pytest.mark.parametrize("n,k", [(128, 64), (300, 200), (512, 520)])

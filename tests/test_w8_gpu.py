@@ -188,3 +188,22 @@ def test_gemm_that_starts_during_the_quantisation(lib, cuda, m, n, k):
         q, s = ops.fp8_quant_per_tensor(x)
         torch.cuda.synchronize()
         assert torch.equal(got, ops.w8a8_gemm(q, s, w8, one, torch.float16, ops.W8_FP8))
+
+
+@pytest.mark.parametrize("m,n,k,splits", [(40, 8192, 8192, 2), (129, 1000, 16384, 4), (36, 2056, 8256, 4), (64, 5000, 12352, 2)])
+def test_long_sums_of_few_tiles(lib, cuda, m, n, k, splits):
+    """The pairs of a cluster share a tile's K: s32 sums stay exact through the exchange, e4m3 ones as near as those of one pair."""
+    from zhilight_b200 import ops
+    assert lib.zl_gemm_pairs_splits(m, n, k, 1, 1) == splits
+    g = torch.Generator().manual_seed(m)
+    x = torch.randint(-128, 128, (m, k), generator=g, dtype=torch.int8).cuda()
+    w = torch.randint(-128, 128, (n, k), generator=g, dtype=torch.int8).cuda()
+    sx, sw = torch.rand(m, generator=g).cuda(), torch.rand(n, generator=g).cuda()
+    acc = (x.double() @ w.double().T).float()              # below 2^53, then one rounding as from s32
+    y = ops.w8a8_gemm(x, sx, w, sw, torch.float16, ops.W8_INT8)
+    assert torch.equal(y, (acc * sx[:, None] * sw[None]).half())
+    xf, wf = (torch.randn(*s, generator=g).mul(2).to(torch.float8_e4m3fn).cuda() for s in ((m, k), (n, k)))
+    one = torch.tensor([0.25], device=cuda)
+    y = ops.w8a8_gemm(xf.view(torch.uint8), one, wf.view(torch.uint8), one, torch.bfloat16, ops.W8_FP8)
+    ref = xf.double() @ wf.double().T / 16
+    assert float((y.double() - ref).norm() / ref.norm()) <= 2.0 ** -8

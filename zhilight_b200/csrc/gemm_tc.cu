@@ -10,18 +10,23 @@
 // cores from about 1000 rows on, below by the loads of w (and by too few tiles: 4096 x 14336 keeps 16 of 74 pairs busy at M <= 256,
 // 52 us against 200).
 //
-//   warp 0       producer  : w and x boxes
-//   warp 1       MMA       : of the leader, one elected lane, 4 x 256 x ntok x 16 per stage
+//   warp 0       producer  : w and x boxes, one lane
+//   warp 1       MMA       : of the leader, one lane, 4 x 256 x ntok x 16 per 64-k block
 //   warp 2       TMEM allocation
 //   warps 4-11   epilogue  : quadrant = warp % 4, 16-row chunks of x in turns; lane = row of w = column of y
 //   warps 12-15  grouped   : rows of x through their index lists, by 16-byte cp.async into the swizzled layout that the boxes have;
 //                            a stage's barrier counts the copies as they land, warp 3 hands the stage to the MMAs
+//
+// The issuing lanes look at their next barrier while this stage's work is on its way (a look costs 120 - 200 cycles, a warp's vote with it
+// more): bf16 4096 x 4096, 512 rows 27.0 -> 21.8 us; 14336 x 4096, 777 rows 85 -> 75; int8 8192 x 8192, 24 rows 22.8 -> 19.4; 16 experts of 2048 x 2048,
+// 2048 rows 85.6 + 49.6 -> 79 + 47.  Few tiles over a long K: the pairs of a cluster share a tile's K (gt_pick).
 //
 // The 8-bit Linears (zl_w8a8_gemm: Int8Linear, Fp8Linear) run on the same kernel: a stage is 128 bytes of k whatever the type, only the MMA
 // (kind::i8 with s32 accumulators, kind::f8f6f4) and the epilogue (scale-back, bias) are theirs.
 #include "gemm_common.cuh"
 #include "tc2_common.cuh"
 
+#include <atomic>
 #include <type_traits>
 
 namespace zl {
@@ -43,6 +48,7 @@ struct alignas(64) GemmTcP {
     GemmP g;
     int epi, groups;            // groups: batch, or the number of groups
     int row_tiles, tok_tiles;   // tok_tiles: not grouped
+    int splits;                 // pairs of a cluster that share a tile's K (then a tile per cluster); not grouped
     int ntok, box_rows;         // not grouped: rows of x of a tile, and of a box (a CTA's half of them)
     int wide;                   // two neighbouring values of y may be stored together
     int stages, sub;            // stages of `sub` blocks: 128 bytes of k of w (16 KB) and of x
@@ -179,12 +185,15 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
     volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
     int* s_cum = reinterpret_cast<int*>(smem + kGtCumOff);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t rank = cluster_rank();
-    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const int splits = GROUPED ? 1 : p.splits;
+    const uint32_t in_cluster = cluster_rank(), rank = in_cluster & 1, lead = in_cluster & ~1u;   // lead: the pair's leader
+    const int part = (int)(in_cluster >> 1);
+    const int pair = (int)(blockIdx.x >> 1) / splits, pairs = (int)(gridDim.x >> 1) / splits;
     constexpr int kBlockK = KIND == kGt16 ? 64 : 128;   // 128 bytes
     constexpr int sub = SUB;
     const int stages = p.stages, block_bytes = p.block_bytes, stage_bytes = sub * block_bytes;
-    const int ks = (p.g.K + kBlockK * sub - 1) / (kBlockK * sub);
+    const int ks_all = (p.g.K + kBlockK * sub - 1) / (kBlockK * sub);
+    const int k_first = (int)((long long)ks_all * part / splits), ks = (int)((long long)ks_all * (part + 1) / splits) - k_first;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < stages; ++i) {
@@ -224,67 +233,74 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
     tc_fence_after();
     const uint32_t tmem = *s_tmem;
 
+    // The three loops below are one lane's each: a vote or a look at a barrier costs the warp 100 - 200 cycles a stage, so each looks at its next
+    // barrier while this stage's copies or MMAs are on their way
     if (warp == 0) {
-        int st = 0, hint = 0;
-        uint32_t ph = 0;
-        GtTile t;
-        bool ok = true;
-        const uint32_t bytes = 2u * sub * (kGtAStage + (GROUPED ? 0 : p.box_rows * 128));
-        auto weights = [&](int at, int k) {   // one lane: the stage's bytes and this CTA's half of its weight rows
-            const uint32_t bar = cluster_map(smem_u32(&full[at]), 0);
-            if (rank == 0) mbar_expect_tx(&full[at], bytes);
+        if (tc_elect_one()) {
+            int st = 0, hint = 0;
+            uint32_t ph = 0;
+            GtTile t;
+            bool ok = true, free = false;
+            const uint32_t bytes = 2u * sub * (kGtAStage + (GROUPED ? 0 : p.box_rows * 128));
+            auto weights = [&](int at, int k) {   // the stage's bytes and this CTA's half of its weight rows
+                const uint32_t bar = cluster_map(smem_u32(&full[at]), lead);
+                if (rank == 0) mbar_expect_tx(&full[at], bytes);
 #pragma unroll
-            for (int u = 0; u < sub; ++u)     // a block behind K arrives as zeros
-                tma2_load_3d(smem + at * stage_bytes + u * block_bytes, &p.wmap, (k * sub + u) * kBlockK, t.n0 + (int)rank * 128, t.b, bar);
-        };
-        int ahead = 0;                        // stages of the first tile whose weights are on their way already
-        if (KIND != kGt16) {
-            if (gt_tile<GROUPED>(p, s_cum, pair, hint, t)) ahead = min(stages, ks);
-            if (tc_elect_one())
+                for (int u = 0; u < sub; ++u)     // a block behind K arrives as zeros
+                    tma2_load_3d(smem + at * stage_bytes + u * block_bytes, &p.wmap, ((k_first + k) * sub + u) * kBlockK, t.n0 + (int)rank * 128, t.b, bar);
+            };
+            int ahead = 0;                        // stages of the first tile whose weights are on their way already
+            if (KIND != kGt16) {
+                if (gt_tile<GROUPED>(p, s_cum, pair, hint, t)) ahead = min(stages, ks);
                 for (int k = 0; k < ahead; ++k) weights(k, k);
-            __syncwarp();
-            pdl_wait();
-        }
-        for (int i = pair; ok && gt_tile<GROUPED>(p, s_cum, i, hint, t); i += pairs) {
-            const int tb = t.t0 + (int)rank * (t.ntok >> 1);
-            for (int k = 0; k < ks; ++k) {
-                if (!(ok = tc2_wait(&empty[st], ph ^ 1u, s_abort, p.err, 0x2100 + st))) break;
-                if (tc_elect_one()) {
-                    if (KIND == kGt16 || ahead <= 0) weights(st, k);
+                pdl_wait();
+            }
+            for (int i = pair; ok && gt_tile<GROUPED>(p, s_cum, i, hint, t); i += pairs) {
+                const int tb = t.t0 + (int)rank * (t.ntok >> 1);
+                for (int k = 0; k < ks; ++k) {
+                    if (!free && !(ok = tc2_wait1(&empty[st], ph ^ 1u, s_abort, p.err, 0x2100 + st))) break;
+                    const int at = st;
+                    if (++st == stages) {
+                        st = 0;
+                        ph ^= 1u;
+                    }
+                    free = mbar_test(&empty[st], ph ^ 1u);
+                    if (KIND == kGt16 || ahead <= 0) weights(at, k);
                     if (!GROUPED) {
-                        const uint32_t bar = cluster_map(smem_u32(&full[st]), 0);
+                        const uint32_t bar = cluster_map(smem_u32(&full[at]), lead);
 #pragma unroll
                         for (int u = 0; u < sub; ++u)
-                            tma2_load_3d(smem + st * stage_bytes + u * block_bytes + kGtAStage, &p.xmap, (k * sub + u) * kBlockK, tb, t.b, bar);
+                            tma2_load_3d(smem + at * stage_bytes + u * block_bytes + kGtAStage, &p.xmap, ((k_first + k) * sub + u) * kBlockK, tb, t.b, bar);
                     }
-                }
-                --ahead;
-                __syncwarp();
-                if (++st == stages) {
-                    st = 0;
-                    ph ^= 1u;
+                    --ahead;
                 }
             }
         }
+        __syncwarp();
     } else if (warp == 1 && rank == 0) {
         if (KIND != kGt16) pdl_wait();       // nothing of use arrives before, and the bounded waits start here
-        int st = 0, acc = 0, hint = 0;
-        uint32_t ph = 0, acc_ph = 0;
-        GtTile t;
-        bool ok = true;
-        for (int i = pair; ok && gt_tile<GROUPED>(p, s_cum, i, hint, t); i += pairs) {
-            if (!(ok = tc2_wait(&acc_empty[acc], acc_ph ^ 1u, s_abort, p.err, 0x2300 + acc))) break;
-            tc_fence_after();
-            const uint32_t d = tmem + (uint32_t)(acc * 256);
-            const uint32_t idesc = KIND == kGt16 ? tc2_idesc(std::is_same<T, __nv_bfloat16>::value, t.ntok) : tc2_idesc8(KIND == kGtFp8, t.ntok);
-            for (int k = 0; k < ks; ++k) {
-                if (!(ok = tc2_wait(&full[st], ph, s_abort, p.err, 0x2400 + st))) break;
-                tc_fence_after();
-                if (tc_elect_one()) {
+        if (tc_elect_one()) {
+            int st = 0, acc = 0, hint = 0;
+            uint32_t ph = 0, acc_ph = 0;
+            GtTile t;
+            bool ok = true, ready = false;
+            for (int i = pair; ok && gt_tile<GROUPED>(p, s_cum, i, hint, t); i += pairs) {
+                if (!(ok = tc2_wait1(&acc_empty[acc], acc_ph ^ 1u, s_abort, p.err, 0x2300 + acc))) break;
+                const uint32_t d = tmem + (uint32_t)(acc * 256);
+                const uint32_t idesc = KIND == kGt16 ? tc2_idesc(std::is_same<T, __nv_bfloat16>::value, t.ntok) : tc2_idesc8(KIND == kGtFp8, t.ntok);
+                for (int k = 0; k < ks; ++k) {
+                    if (!ready && !(ok = tc2_wait1(&full[st], ph, s_abort, p.err, 0x2400 + st))) break;
+                    const uint32_t base = smem_u32(smem + st * stage_bytes);
+                    uint64_t* const used = &empty[st];
+                    if (++st == stages) {
+                        st = 0;
+                        ph ^= 1u;
+                    }
+                    ready = mbar_test(&full[st], ph);
+                    tc_fence_after();
 #pragma unroll
                     for (int u = 0; u < sub; ++u) {
-                        const uint32_t at = smem_u32(smem + st * stage_bytes + u * block_bytes);
-                        const uint64_t ad = tc_desc_sw128(at), bd = tc_desc_sw128(at + kGtAStage);
+                        const uint64_t ad = tc_desc_sw128(base + u * block_bytes), bd = tc_desc_sw128(base + u * block_bytes + kGtAStage);
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {   // 32 bytes of k per MMA
                             const uint64_t a = ad + (uint64_t)(j * 2), b = bd + (uint64_t)(j * 2);
@@ -293,38 +309,37 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
                             else tc2_mma_ss8<KIND == kGtFp8>(d, a, b, idesc, accum);
                         }
                     }
-                    tc2_commit(&empty[st]);
-                    if (k == ks - 1) tc2_commit(&acc_full[acc]);
+                    tc2_commit(used, lead);
+                    if (k == ks - 1) tc2_commit(&acc_full[acc], lead);
                 }
-                __syncwarp();
-                if (++st == stages) {
-                    st = 0;
-                    ph ^= 1u;
+                if (++acc == 2) {
+                    acc = 0;
+                    acc_ph ^= 1u;
                 }
-            }
-            if (++acc == 2) {
-                acc = 0;
-                acc_ph ^= 1u;
             }
         }
+        __syncwarp();
     } else if (GROUPED && warp == 3) {
         // rows that have landed become visible to the proxy the MMAs read through, then count as arrived at the leader
-        int st = 0, hint = 0;
-        uint32_t ph = 0;
-        GtTile t;
-        bool ok = true;
-        for (int i = pair; ok && gt_tile<GROUPED>(p, s_cum, i, hint, t); i += pairs)
-            for (int k = 0; k < ks; ++k) {
-                if (!(ok = tc2_wait(&rows_full[st], ph, s_abort, p.err, 0x2500 + st))) break;
-                if (lane == 0) {
+        if (tc_elect_one()) {
+            int st = 0, hint = 0;
+            uint32_t ph = 0;
+            GtTile t;
+            bool ok = true, ready = false;
+            for (int i = pair; ok && gt_tile<GROUPED>(p, s_cum, i, hint, t); i += pairs)
+                for (int k = 0; k < ks; ++k) {
+                    if (!ready && !(ok = tc2_wait1(&rows_full[st], ph, s_abort, p.err, 0x2500 + st))) break;
+                    const uint32_t to = cluster_map(smem_u32(&full[st]), lead);
+                    if (++st == stages) {
+                        st = 0;
+                        ph ^= 1u;
+                    }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    mbar_arrive_at(cluster_map(smem_u32(&full[st]), 0));
+                    mbar_arrive_at(to);
+                    ready = mbar_test(&rows_full[st], ph);
                 }
-                if (++st == stages) {
-                    st = 0;
-                    ph ^= 1u;
-                }
-            }
+        }
+        __syncwarp();
     } else if (GROUPED && warp >= 12) {
         // thread: 16-byte chunk c of rows j, j + 16, ... of the CTA's half
         const int tid = threadIdx.x - 12 * 32, c = tid & 7, j = tid >> 3;
@@ -332,7 +347,7 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
         int st = 0, hint = 0;
         uint32_t ph = 0;
         GtTile t;
-        bool ok = true;
+        bool ok = true, free = false;
         for (int i = pair; ok && gt_tile<GROUPED>(p, s_cum, i, hint, t); i += pairs) {
             const int half = t.ntok >> 1, tb = t.t0 + (int)rank * half;
             const T* row[8];
@@ -342,7 +357,8 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
                 row[u] = static_cast<const T*>(p.g.x) + (size_t)(p.g.x_rows ? p.g.x_rows[e] : e) * p.g.ldx + c * 8;
             }
             for (int k = 0; k < ks; ++k) {
-                if (!(ok = tc2_wait(&empty[st], ph ^ 1u, s_abort, p.err, 0x2200 + st))) break;
+                if (!__all_sync(0xffffffffu, free) && !(ok = tc2_wait(&empty[st], ph ^ 1u, s_abort, p.err, 0x2200 + st))) break;
+                free = st + 1 < stages ? mbar_test(&empty[st + 1], ph ^ 1u) : mbar_test(&empty[0], ph);
 #pragma unroll
                 for (int u2 = 0; u2 < sub; ++u2) {
                     const int k0 = (k * sub + u2) * 64;
@@ -364,47 +380,59 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
             }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
-    } else if (warp >= 4) {
+    }
+    // epilogue warps; with K split a tile's only chunks come behind the exchange below
+    const int q = warp & 3, set = (warp - 4) >> 2;
+    float bias = 0.f, s_w = 0.f;
+    auto row_values = [&](const GtTile& t, int n) {
+        bias = s_w = 0.f;
+        if (n < p.g.N) {
+            if (KIND != kGt16)
+                s_w = p.sw_mode == 0 ? to_f32<T>(static_cast<const T*>(p.sw)[n]) : static_cast<const float*>(p.sw)[p.sw_mode == 3 ? 0 : n];
+            if (p.g.bias) bias = p.g.bias[(size_t)t.b * p.g.bb + n];
+            else if (p.g.bias_t) bias = to_f32<T>(static_cast<const T*>(p.g.bias_t)[n]);
+        }
+    };
+    auto put = [&](const GtTile& t, int n, int c0, float (&v)[16]) {
+        if constexpr (KIND != kGt16) {
+            gt_store16_8bit<TO, KIND>(p, t, n, c0, v, s_w, bias, p.g.bias_t != nullptr, lane);
+        } else {
+            switch (p.epi) {
+#define ZL_GT_EPI(E) case E: gt_store16<T, TO, E>(p, t, n, c0, v, bias, lane); break;
+                ZL_GT_EPI(ZL_GEMM_EPI_RELU2)
+                ZL_GT_EPI(ZL_GEMM_EPI_SIGMOID_GATE)
+                ZL_GT_EPI(ZL_GEMM_EPI_TANH)
+                ZL_GT_EPI(ZL_GEMM_EPI_GLU_CLAMP)
+                ZL_GT_EPI(ZL_GEMM_EPI_GEGLU_TANH)
+                ZL_GT_EPI(ZL_GEMM_EPI_GELU_TANH_MUL)
+                ZL_GT_EPI(ZL_GEMM_EPI_SOFTCAP)
+                ZL_GT_EPI(ZL_GEMM_EPI_REGLU)
+                default: gt_store16<T, TO, ZL_GEMM_EPI_NONE>(p, t, n, c0, v, bias, lane);
+#undef ZL_GT_EPI
+            }
+        }
+    };
+    const bool epilogue = warp >= 4 && warp < 4 + kGtEpiWarps;
+    if (epilogue) {
         if (KIND != kGt16) pdl_wait();
-        const int q = warp & 3, set = (warp - 4) >> 2;
         int acc = 0, hint = 0;
         uint32_t acc_ph = 0;
         GtTile t;
         for (int i = pair; gt_tile<GROUPED>(p, s_cum, i, hint, t); i += pairs) {
             if (!tc2_wait(&acc_full[acc], acc_ph, s_abort, p.err, 0x2800 + acc)) break;
             tc_fence_after();
+            if (splits > 1) break;
             const int n = t.n0 + (int)rank * 128 + q * 32 + lane;
-            float bias = 0.f, s_w = 0.f;
-            if (n < p.g.N) {
-                if (KIND != kGt16)
-                    s_w = p.sw_mode == 0 ? to_f32<T>(static_cast<const T*>(p.sw)[n])
-                                         : static_cast<const float*>(p.sw)[p.sw_mode == 3 ? 0 : n];
-                if (p.g.bias) bias = p.g.bias[(size_t)t.b * p.g.bb + n];
-                else if (p.g.bias_t) bias = to_f32<T>(static_cast<const T*>(p.g.bias_t)[n]);
-            }
+            row_values(t, n);
             const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * 256);
             for (int c0 = set * 16; c0 < t.ntok && t.t0 + c0 < t.M; c0 += 32) {
                 float v[16];
                 tc_ld16(taddr + (uint32_t)c0, v);
-                if constexpr (KIND != kGt16) {
-                    gt_store16_8bit<TO, KIND>(p, t, n, c0, v, s_w, bias, p.g.bias_t != nullptr, lane);
-                } else switch (p.epi) {
-#define ZL_GT_EPI(E) case E: gt_store16<T, TO, E>(p, t, n, c0, v, bias, lane); break;
-                    ZL_GT_EPI(ZL_GEMM_EPI_RELU2)
-                    ZL_GT_EPI(ZL_GEMM_EPI_SIGMOID_GATE)
-                    ZL_GT_EPI(ZL_GEMM_EPI_TANH)
-                    ZL_GT_EPI(ZL_GEMM_EPI_GLU_CLAMP)
-                    ZL_GT_EPI(ZL_GEMM_EPI_GEGLU_TANH)
-                    ZL_GT_EPI(ZL_GEMM_EPI_GELU_TANH_MUL)
-                    ZL_GT_EPI(ZL_GEMM_EPI_SOFTCAP)
-                    ZL_GT_EPI(ZL_GEMM_EPI_REGLU)
-                    default: gt_store16<T, TO, ZL_GEMM_EPI_NONE>(p, t, n, c0, v, bias, lane);
-#undef ZL_GT_EPI
-                }
+                put(t, n, c0, v);
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_at(cluster_map(smem_u32(&acc_empty[acc]), 0));
+            if (lane == 0) mbar_arrive_at(cluster_map(smem_u32(&acc_empty[acc]), lead));
             if (++acc == 2) {
                 acc = 0;
                 acc_ph ^= 1u;
@@ -415,7 +443,35 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
     tc2_drain(s_abort);
     tc_fence_before();
     __syncthreads();
-    cluster_sync_all();   // nobody's shared memory or TMEM goes while the other CTA may still use it
+    cluster_sync_all();   // nobody's shared memory or TMEM goes, or takes sums, while another CTA may still use it
+    if (!GROUPED && splits > 1) {
+        tc_fence_after();
+        int hint = 0;
+        GtTile t;
+        const bool any = gt_tile<GROUPED>(p, s_cum, pair, hint, t);
+        const int row = q * 32 + lane, n = t.n0 + (int)rank * 128 + row;
+        const int chunks = any ? min(t.ntok, t.M - t.t0 + 15) / 16 : 0;
+        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16);
+        if (epilogue)
+            for (int c = set; c < chunks; c += 2) {
+                if (c % splits == part) continue;
+                float v[16];
+                tc_ld16(taddr + (uint32_t)(c * 16), v);
+                tc2_split_push(smem_u32(smem), (int)rank, part, c, splits, chunks, row, v);
+            }
+        cluster_sync_all();
+        if (epilogue) {
+            row_values(t, n);
+            for (int c = part + set * splits; c < chunks; c += 2 * splits) {
+                float v[16];
+                tc_ld16(taddr + (uint32_t)(c * 16), v);
+                tc2_split_sum<KIND == kGtInt8>(smem, part, c, splits, chunks, row, v);
+                put(t, n, c * 16, v);
+            }
+        }
+        tc_fence_before();
+        __syncthreads();
+    }
     if (warp == 2) {
         tc_fence_after();
         tc2_dealloc(tmem);
@@ -433,6 +489,32 @@ static int gt_pick_ntok(int M, long long rows, int pairs) {
         if (cost < best_cost - 1e-9) {
             best_cost = cost;
             best = n;
+        }
+        if (n >= M) break;
+    }
+    return best;
+}
+
+// Rows of x per tile, and how many pairs share a tile's K, for `blocks` 128-byte blocks of k: with few tiles the pairs of a cluster (the device holds
+// fit[0] clusters of two pairs at a time, fit[1] of four) take a part each and exchange their sums.  In cycles, fitted to the times below: a block
+// 190 + 1.4 per row of x, the exchange 2850 + 42 per row.  Measured, one pair / two, us, N x K: bf16 4096 x 14336, 65 rows 39.3 / 31.2, 256 rows
+// 42.6 / 37.2; 1024 x 8192, 65 rows 23.3 / 17.2 and 14.9 with four; int8 8192 x 8192, 24 rows 20.3 / 18.9; against it bf16 4096 x 4096, 512 rows
+// 22.5 / 25.4; 8192 x 2048, 256 rows 16.9 / 20.9.
+struct GtPick {
+    int ntok, splits;
+};
+static GtPick gt_pick(int M, long long rows, int pairs, int blocks, const int (&fit)[2]) {
+    GtPick best{32, 1};
+    double best_cost = 1e30;
+    for (int n = 32; n <= 256; n += 32) {
+        const long long tiles = rows * cdiv(M, n), waves = (tiles + pairs - 1) / pairs;
+        for (int s = 1; s <= 4; s *= 2) {
+            if (s > 1 && (tiles > fit[s / 4] || blocks < 8 * s)) continue;
+            const double cost = (double)waves * cdiv(blocks, s) * (190.0 + 1.4 * n) + (s > 1 ? 2850.0 + 42.0 * n : 0.0);
+            if (cost < best_cost - 1e-9) {
+                best_cost = cost;
+                best = GtPick{n, s};
+            }
         }
         if (n >= M) break;
     }
@@ -480,7 +562,7 @@ static cudaError_t launch_gt_sub(const GemmTcP& q, int pairs, bool pdl, cudaStre
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) set[dev] = true;
     }
-    return launch_pairs(k_gemm_tc<T, TO, GROUPED, KIND, SUB>, pairs, dim3(GROUPED ? kGtGroupThreads : kGtThreads), (size_t)kGtBytes, stream, pdl, q);
+    return launch_pairs(k_gemm_tc<T, TO, GROUPED, KIND, SUB>, pairs, q.splits, dim3(GROUPED ? kGtGroupThreads : kGtThreads), (size_t)kGtBytes, stream, pdl, q);
 }
 template <typename T, typename TO, bool GROUPED, int KIND>
 static cudaError_t launch_gt(const GemmTcP& q, int pairs, bool pdl, cudaStream_t stream) {
@@ -491,6 +573,38 @@ static cudaError_t launch_gt(const GemmTcP& q, int pairs, bool pdl, cudaStream_t
 template <typename T, typename TO>
 static cudaError_t launch_gt16(const GemmTcP& q, bool grouped, int pairs, bool pdl, cudaStream_t stream) {
     return grouped ? launch_gt<T, TO, true, kGt16>(q, pairs, pdl, stream) : launch_gt<T, TO, false, kGt16>(q, pairs, pdl, stream);
+}
+
+// clusters of two and of four pairs that the current device holds at a time; 0: none
+static void gt_clusters(int (&fit)[2]) {
+    static std::atomic<int> cache[64][2];       // count + 1
+    int dev = 0;
+    cudaGetDevice(&dev);
+    for (int i = 0; i < 2; ++i) {
+        const bool known = dev >= 0 && dev < 64;
+        int n = known ? cache[dev][i].load(std::memory_order_relaxed) - 1 : -1;
+        if (n < 0) {
+            auto kernel = k_gemm_tc<__half, __half, false, kGt16, 1>;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((device_sm_count() + 7) / 8 * 8);
+            cfg.blockDim = dim3(kGtThreads);
+            cfg.dynamicSmemBytes = kGtBytes;
+            cudaLaunchAttribute attr;
+            attr.id = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim.x = 4u << i;
+            attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+            cfg.attrs = &attr;
+            cfg.numAttrs = 1;
+            n = 0;
+            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGtBytes) != cudaSuccess ||
+                cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+                cudaGetLastError();
+                n = 0;
+            }
+            if (known) cache[dev][i].store(n + 1, std::memory_order_relaxed);
+        }
+        fit[i] = n;
+    }
 }
 
 // tiles, maps and stages of a call; returns the number of pairs, 0 without a map
@@ -505,18 +619,24 @@ static int gt_plan(GemmTcP& q, CUtensorMapDataType dt, int batch, int out_bytes)
     q.row_tiles = cdiv(p.N, kTc2Rows);
     q.tok_tiles = 0;
     q.ntok = 256;
+    q.splits = 1;
     q.wide = p.N % 2 == 0 && p.ldy % 2 == 0 && p.yb % 2 == 0 && reinterpret_cast<uintptr_t>(p.y) % (2 * out_bytes) == 0;
     if (!tc2_map_3d(&q.wmap, p.w, dt, p.K, p.N, batch, p.ldw, p.wb, 128)) return 0;
     if (!grouped) {
-        q.ntok = gt_pick_ntok(p.M, (long long)q.row_tiles * batch, pairs);
+        int fit[2];
+        gt_clusters(fit);
+        const int block_k = dt == CU_TENSOR_MAP_DATA_TYPE_UINT8 ? 128 : 64;
+        const GtPick pick = gt_pick(p.M, (long long)q.row_tiles * batch, pairs, cdiv(p.K, block_k), fit);
+        q.ntok = pick.ntok;
+        q.splits = pick.splits;
         q.tok_tiles = cdiv(p.M, q.ntok);
-        const long long tiles = (long long)q.row_tiles * q.tok_tiles * batch;
+        const long long tiles = (long long)q.row_tiles * q.tok_tiles * batch * q.splits;
         if (tiles < pairs) pairs = (int)tiles;
         if (!tc2_map_3d(&q.xmap, p.x, dt, p.K, p.M, batch, p.ldx, p.xb, q.ntok / 2)) return 0;
     }
     q.box_rows = q.ntok / 2;
     q.block_bytes = kGtAStage + q.box_rows * 128;
-    // handing a stage over costs the MMA warp about 450 cycles, a block's MMAs 2 per row of x: small tiles take two blocks per stage
+    // handing a stage over costs the MMA warp more than a small block's MMAs (2 cycles per row of x): small tiles take two blocks per stage
     // (not grouped rows, whose copies come to too few stages then: 87 -> 95 us)
     q.sub = q.ntok <= 128 && !grouped ? 2 : 1;
     const int fit = kGtRing / (q.sub * q.block_bytes);
@@ -559,6 +679,13 @@ ZL_W8_TC(__nv_bfloat16, true)
 #undef ZL_W8_TC
 
 }  // namespace zl
+
+extern "C" int zl_gemm_pairs_splits(int M, int N, int K, int batch, int elem_bytes) {
+    if (M <= 0 || N <= 0 || K <= 0 || batch <= 0 || (elem_bytes != 1 && elem_bytes != 2)) return 0;
+    int fit[2];
+    zl::gt_clusters(fit);
+    return zl::gt_pick(M, (long long)zl::cdiv(N, zl::kTc2Rows) * batch, zl::device_sm_count() / 2, zl::cdiv(K, 128 / elem_bytes), fit).splits;
+}
 
 extern "C" unsigned zl_gemm_tc_watchdog(void) {
     cudaDeviceSynchronize();

@@ -98,9 +98,9 @@ __device__ __forceinline__ void tc2_alloc(uint32_t* s_tmem) {
 __device__ __forceinline__ void tc2_dealloc(uint32_t tmem) {
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512));
 }
-// arrives on the barrier at this offset in both CTAs once the MMAs issued so far have completed
-__device__ __forceinline__ void tc2_commit(uint64_t* bar) {
-    const uint16_t both = 3;
+// arrives on the barrier at this offset in both CTAs of the pair (lead: the leader's rank in its cluster) once the MMAs issued so far have completed
+__device__ __forceinline__ void tc2_commit(uint64_t* bar, uint32_t lead = 0) {
+    const uint16_t both = (uint16_t)(3u << lead);
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
                  "h"(both)
                  : "memory");
@@ -143,9 +143,41 @@ __device__ __forceinline__ void tc2_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uin
         : "memory");
 }
 
-// launch of a grid of CTA pairs
+// ---- a tile whose K is split over the pairs of one cluster ------------------------------------------------------------------------------
+// A few tiles leave most pairs idle.  So `splits` pairs (a cluster of 2 x splits CTAs) take a range of k each, and each finishes every
+// splits-th chunk of 16 tokens: the others push their sums of it into its shared memory, where the ring was.
+__device__ __forceinline__ void tc2_st_cluster4(uint32_t addr, float a, float b, float c, float d) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+// place of the sums that pair `from` has of 16-token chunk `c` (of the owner's rows): [from][c / splits][4 tokens][128 rows] float4
+__device__ __forceinline__ uint32_t tc2_split_at(int from, int c, int splits, int chunks, int row) {
+    return (uint32_t)((((from * ((chunks + splits - 1) / splits) + c / splits) * 4) * 128 + row) * 16);
+}
+__device__ __forceinline__ void tc2_split_push(uint32_t smem, int rank, int mine, int c, int splits, int chunks, int row, const float (&v)[16]) {
+    const uint32_t dst = cluster_map(smem + tc2_split_at(mine, c, splits, chunks, row), (uint32_t)(2 * (c % splits) + rank));
+#pragma unroll
+    for (int u = 0; u < 4; ++u) tc2_st_cluster4(dst + u * 2048, v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
+}
+// adds the other pairs' sums to this one's, in the order of k; INT: v are the bits of s32 sums
+template <bool INT>
+__device__ __forceinline__ void tc2_split_sum(const uint8_t* smem, int mine, int c, int splits, int chunks, int row, float (&v)[16]) {
+    float own[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) own[i] = v[i], v[i] = 0.f;
+    auto add = [](float& a, float b) { a = INT ? __int_as_float(__float_as_int(a) + __float_as_int(b)) : a + b; };
+    for (int s = 0; s < splits; ++s) {
+        const float4* part = reinterpret_cast<const float4*>(smem + tc2_split_at(s, c, splits, chunks, row));
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const float4 w = s == mine ? make_float4(own[4 * u], own[4 * u + 1], own[4 * u + 2], own[4 * u + 3]) : part[u * 128];
+            add(v[4 * u], w.x), add(v[4 * u + 1], w.y), add(v[4 * u + 2], w.z), add(v[4 * u + 3], w.w);
+        }
+    }
+}
+
+// launch of a grid of CTA pairs, `splits` of them in a cluster
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pairs(void (*kernel)(KArgs...), int pairs, dim3 block, size_t smem, cudaStream_t stream, bool pdl, Args... args) {
+inline cudaError_t launch_pairs(void (*kernel)(KArgs...), int pairs, int splits, dim3 block, size_t smem, cudaStream_t stream, bool pdl, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * pairs);
     cfg.blockDim = block;
@@ -153,7 +185,7 @@ inline cudaError_t launch_pairs(void (*kernel)(KArgs...), int pairs, dim3 block,
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.x = 2 * splits;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;

@@ -382,7 +382,7 @@ cudaError_t launch_w4_tc2(const W4Params& p, bool pdl, cudaStream_t stream) {
         if (!tc_make_map_nd(&q.xmap, p.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B)) return cudaErrorInvalidValue;
     }
     const int tiles = row_tiles * q.tok_tiles;
-    return launch_pairs(k_w4a16_tc2, tiles < max_pairs ? tiles : max_pairs, dim3(T2Cfg::kThreads), (size_t)T2Cfg::kBytes, stream, pdl, q);
+    return launch_pairs(k_w4a16_tc2, tiles < max_pairs ? tiles : max_pairs, 1, dim3(T2Cfg::kThreads), (size_t)T2Cfg::kBytes, stream, pdl, q);
 }
 
 }  // namespace zl
