@@ -142,7 +142,7 @@ int zl_w4a16_gemm_fused(const zl_w4_fused_args_t* args, zl_stream_t stream);
 /* 1 if the exact-integer kernel (variant 1, M <= 16) can run this shape: its staged activations must fit shared memory. */
 int zl_w4_int_kernel_fits(int M, int N, int K);
 /* which kernel serves (M, N, K) on the ZLW4I layout (variant 1): 3 = exact-integer mma.sync kernel (from 9 rows on only with the fused
- * RMSNorm or the exchange, else the fp16 mma.sync kernel), 4 = tcgen05 / TMEM / TMA kernels, up to 16 rows the fp16 mma.sync kernel (any M,
+ * RMSNorm or the exchange, else the fp16 mma.sync kernel), 4 = tcgen05 / TMEM / TMA kernels, up to 16 rows (32 of small matrices) the fp16 mma.sync kernel (any M,
  * N % 128 == 0, no fused RMSNorm prologue), 0 = neither (pack variant 0 and use the fp16 mma.sync kernel). */
 int zl_w4_int_layout_route(int M, int N, int K);
 /* whether, of the two kernels behind answer 4, the one over pairs of SMs serves the shape (1) or the stream-k kernel (0) */

@@ -45,3 +45,20 @@ def test_nine_to_sixteen_rows_keep_small_values_beside_large_ones(lib, cuda, m):
     assert len(blind) > 8
     y = ops.w4a16_gemm_fused(x.to(cuda), packed, n, k, variant=1).float().cpu().numpy()
     assert rel_l2(y[:, blind], ref[:, blind]) <= 2.8e-4
+
+
+@pytest.mark.parametrize("k,n", [(128, 128), (1152, 2304), (8192, 512), (4096, 4096 + 640), (2048, 9472), (1024, 4736 + 128)])
+@pytest.mark.parametrize("m", [17, 24, 25, 32])
+def test_up_to_32_rows_of_small_matrices(lib, cuda, k, n, m):
+    """The edges of its range: K = 8192 of one wave of super-tiles, K = 2048 of two.  Tolerances as above, which the tcgen05 kernels' weights, rounded to
+    fp16, would not keep."""
+    from zhilight_b200 import ops
+    w, packed, _, _ = _setup(cuda, k, n, False, 4)
+    g = torch.Generator().manual_seed(m)
+    x = torch.randn(m, k, generator=g).half()
+    res, bias = torch.randn(m, n, generator=g).half(), torch.randn(n, generator=g).half()
+    ref = gptq.gemm_f32(x.numpy(), w)
+    y = ops.w4a16_gemm_fused(x.to(cuda), packed, n, k, variant=1).float().cpu().numpy()
+    assert max(rel_l2(y[i], ref[i]) for i in range(m)) <= 2.8e-4
+    y = ops.w4a16_gemm_fused(x.to(cuda), packed, n, k, variant=1, bias=bias.to(cuda), residual=res.to(cuda), epilogue=ops.EPI_RESIDUAL).float().cpu().numpy()
+    assert max(rel_l2(y[i], ref[i] + bias.float().numpy() + res[i].float().numpy()) for i in range(m)) <= 5.6e-4

@@ -469,7 +469,8 @@ cudaError_t launch_w4_v2(const W4Params& p, bool pdl, cudaStream_t stream) {
 cudaError_t launch_w4_v2_int_layout(const W4Params& p, bool pdl, cudaStream_t stream) {
     W4Params q = p;
     q.x32 = ((reinterpret_cast<uintptr_t>(p.x) | (size_t)p.ldx * 2) & 31) == 0;
-    return q.mc <= 8 ? launch_v2_nt<1, true>(q, pdl, stream) : launch_v2_nt<2, true>(q, pdl, stream);
+    if (q.mc <= 8) return launch_v2_nt<1, true>(q, pdl, stream);
+    return q.mc <= 16 ? launch_v2_nt<2, true>(q, pdl, stream) : launch_v2_nt<4, true>(q, pdl, stream);
 }
 
 cudaError_t prepare_w4_v2() {
@@ -483,7 +484,7 @@ cudaError_t prepare_w4_v2() {
     ZL_SET(NT, false, true, W, ST, false) ZL_SET(NT, true, true, W, ST, false)
 #define ZL_SETI(NT, W, ST) ZL_SET(NT, false, false, W, ST, true) ZL_SET(NT, false, true, W, ST, true)
     ZL_SET4(1, 8, 5) ZL_SET4(2, 8, 4) ZL_SET4(4, 8, 4) ZL_SET4(1, 16, 4) ZL_SET4(2, 16, 4)
-    ZL_SETI(1, 8, 5) ZL_SETI(2, 8, 4) ZL_SETI(1, 16, 4) ZL_SETI(2, 16, 4)
+    ZL_SETI(1, 8, 5) ZL_SETI(2, 8, 4) ZL_SETI(1, 16, 4) ZL_SETI(2, 16, 4) ZL_SETI(4, 8, 4)
 #undef ZL_SETI
 #undef ZL_SET4
 #undef ZL_SET
