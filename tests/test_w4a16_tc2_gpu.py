@@ -135,3 +135,38 @@ def test_predecessor_that_takes_longer_than_a_wait_may(lib, cuda):
     took = behind_slow_predecessors(cuda, 1600, lambda: ops.w4a16_gemm_fused(x, packed, n, k, variant=1, out=got, pdl=True))
     assert took > 1400
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("m,k,n,splits", [(65, 2304, 1152, 3), (40, 3968, 1280, 4), (97, 2304, 2304, 3), (128, 4096, 4096, 2), (45, 2944, 1280, 4), (256, 3200, 1152, 3),
+                                          (33, 3840, 2304, 3)])
+def test_pairs_that_share_a_tile(lib, cuda, m, k, n, splits):
+    """Two, three and four pairs per tile; K of an odd number of 128-k groups, parts of different lengths, an odd number of 128-row tiles, chunks of
+    16 tokens that do not divide by the pairs.  Every row; with the residual updated in place; twice the same."""
+    from zhilight_b200 import ops
+    assert lib.zl_w4_pairs_splits(m, n, k) == splits
+    w, packed = _setup(cuda, k, n, False, 6)
+    x = _x(m, k, m)
+    ref = gptq.gemm_f32(x.numpy(), w)
+    y = ops.w4a16_gemm_fused(x.to(cuda), packed, n, k, variant=1).float().cpu().numpy()
+    assert max(rel_l2(y[i], ref[i]) for i in range(m)) <= TOL
+    g = torch.Generator().manual_seed(3)
+    bias, res = (torch.randn(n, generator=g) * 0.5).half().to(cuda), torch.randn(m, n, generator=g).half()
+    outs = []
+    for _ in range(2):
+        h = res.to(cuda)
+        ops.w4a16_gemm_fused(x.to(cuda), packed, n, k, bias=bias, residual=h, epilogue=ops.EPI_RESIDUAL, variant=1, out=h)
+        outs.append(h)
+    assert torch.equal(*outs)
+    want = oops._t(oops._t(ref + bias.float().cpu().numpy(), "f16") + res.float().numpy(), "f16")
+    assert rel_l2(outs[0].float().cpu().numpy(), want) <= TOL
+
+
+def test_shared_tiles_with_swiglu(lib, cuda):
+    from zhilight_b200 import ops
+    m, k, f = 72, 3968, 640
+    assert lib.zl_w4_pairs_splits(m, 2 * f, k) > 1
+    w, packed = _setup(cuda, k, 2 * f, False, 7, ops.swiglu_row_map(f, cuda))
+    x = _x(m, k, 9)
+    y = ops.w4a16_gemm_fused(x.to(cuda), packed, 2 * f, k, epilogue=ops.EPI_SWIGLU, variant=1).float().cpu().numpy()
+    gu = oops._t(gptq.gemm_f32(x.numpy(), w), "f16")
+    assert rel_l2(y, gu[:, :f] / (1.0 + np.exp(-gu[:, :f])) * gu[:, f:]) <= 2e-3

@@ -26,7 +26,6 @@
 #include "gemm_common.cuh"
 #include "tc2_common.cuh"
 
-#include <atomic>
 #include <type_traits>
 
 namespace zl {
@@ -577,34 +576,8 @@ static cudaError_t launch_gt16(const GemmTcP& q, bool grouped, int pairs, bool p
 
 // clusters of two and of four pairs that the current device holds at a time; 0: none
 static void gt_clusters(int (&fit)[2]) {
-    static std::atomic<int> cache[64][2];       // count + 1
-    int dev = 0;
-    cudaGetDevice(&dev);
-    for (int i = 0; i < 2; ++i) {
-        const bool known = dev >= 0 && dev < 64;
-        int n = known ? cache[dev][i].load(std::memory_order_relaxed) - 1 : -1;
-        if (n < 0) {
-            auto kernel = k_gemm_tc<__half, __half, false, kGt16, 1>;
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((device_sm_count() + 7) / 8 * 8);
-            cfg.blockDim = dim3(kGtThreads);
-            cfg.dynamicSmemBytes = kGtBytes;
-            cudaLaunchAttribute attr;
-            attr.id = cudaLaunchAttributeClusterDimension;
-            attr.val.clusterDim.x = 4u << i;
-            attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-            cfg.attrs = &attr;
-            cfg.numAttrs = 1;
-            n = 0;
-            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGtBytes) != cudaSuccess ||
-                cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
-                cudaGetLastError();
-                n = 0;
-            }
-            if (known) cache[dev][i].store(n + 1, std::memory_order_relaxed);
-        }
-        fit[i] = n;
-    }
+    static PairsFit known;
+    for (int i = 0; i < 2; ++i) fit[i] = pairs_clusters(k_gemm_tc<__half, __half, false, kGt16, 1>, kGtThreads, kGtBytes, 2 << i, known);
 }
 
 // tiles, maps and stages of a call; returns the number of pairs, 0 without a map

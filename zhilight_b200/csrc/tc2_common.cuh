@@ -6,6 +6,8 @@
 #pragma once
 #include "tc_common.cuh"
 
+#include <atomic>
+
 namespace zl {
 
 constexpr int kTc2Rows = 256;                 // A rows of a tile (both CTAs)
@@ -193,6 +195,36 @@ inline cudaError_t launch_pairs(void (*kernel)(KArgs...), int pairs, int splits,
     cfg.numAttrs = pdl ? 2 : 1;
     zl_count_launch();
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+// clusters of `splits` pairs of a kernel (one CTA per SM) that the current device holds at a time, 0: none; the caller keeps what was asked before
+struct PairsFit {
+    std::atomic<int> known[64][5] = {};   // count + 1
+};
+template <typename... KArgs>
+inline int pairs_clusters(void (*kernel)(KArgs...), int threads, int smem, int splits, PairsFit& fit) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const bool cached = dev >= 0 && dev < 64 && splits < 5;
+    int n = cached ? fit.known[dev][splits].load(std::memory_order_relaxed) - 1 : -1;
+    if (n >= 0) return n;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((device_sm_count() / (2 * splits) + 1) * 2 * splits);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 2 * splits;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    if (cached) fit.known[dev][splits].store(n + 1, std::memory_order_relaxed);
+    return n;
 }
 
 // (K, rows, batch) tensor, row pitch ld and batch pitch in elements; box = 128 bytes of k x box_rows rows, 128-byte swizzle

@@ -682,6 +682,7 @@ bool w4_tc_params(W4TcParams& q, const W4Params& p) {
     q.trace = nullptr;
     q.err = nullptr;
     q.ntok = q.tok_tiles = 0;
+    q.splits = 1;
     q.wide = ((reinterpret_cast<uintptr_t>(p.y) | reinterpret_cast<uintptr_t>(p.residual)) & 3) == 0;
     return true;
 }

@@ -6,7 +6,7 @@
 // cutting the tiles into one range per CTA makes two of a CTA's two or three pieces partial ones that travel through L2 as tagged
 // words.  Here
 //   * a tile is 256 rows of w by up to 256 tokens over two SMs: each converts its own 128 rows and loads half of the tokens;
-//   * tiles are whole, taken in turn by persistent pairs; the token tile's size is chosen so that the last wave is full;
+//   * tiles are taken whole, in turn by persistent pairs; the token tile's size is chosen so that the last wave is full;
 //   * up to 64 tokens there are two accumulators; with one, eight epilogue warps shorten the gap.
 // 28672 x 4096 with SwiGLU: 1000 tokens 499 -> 190 us, 256 tokens 128 -> 60; 4096 x 14336 with the residual: 1000 tokens 408 -> 88 us
 // (1360 TFLOP/s).  Bound by the tensor cores at 256 tokens (1084 cycles per 128-k group, at the clock that the power limit leaves); below 130
@@ -14,16 +14,17 @@
 //
 // What a stage costs one thread is what bounded small tiles before that (830 cycles): looking at a barrier takes it 120 - 200 cycles even when the
 // phase has ended, two TMA instructions and their votes 400.  So the issuing threads are single lanes that run their warp's loop alone and look at
-// the next barrier while this stage's work is on its way, a stage's x is one box, its weights are two and are issued by two warps in turn, the
+// the next barrier while this stage's work is on its way, a stage is two 128-k groups up to 128 tokens, its x is one box, its weights are two and are issued by two warps in turn, the
 // weight boxes have rows of 128 bytes, the ring of weights takes what room there is, and six slots of A fit beside up to 128 tokens' accumulators.
 // 4096 x 14336, 256 rows 53.9 -> 45.4 us, 512 rows 55.9 -> 49.2; 28672 x 4096, 64 rows 36 -> 32; 6144 x 4096, 96 rows 22.4 -> 18.9.
+// Few tiles: the pairs of a cluster share a tile's K (t2_pick).
 //
 //   warps 0-7    epilogue : quadrant = warp % 4, 16-token chunks in turns
-//   warps 8-23   dequant  : four groups of four take the stages (one 128-k group each) in turn, one group per stage slot; lane =
-//                           weight row, quadrant = warp % 4; their arrivals of both CTAs meet on the leader's barrier
+//   warps 8-23   dequant  : four groups of four warps take the 128-k groups in turn, one per slot of A; lane = weight row, quadrant =
+//                           warp % 4; their arrivals of both CTAs for a stage meet on the leader's barrier
 //   warps 24, 25 weights  : tensor-TMA of the 4 ZLW4I records of a stage and their trailers, this CTA's 128 rows, stages in turn
 //   warp 26      x        : this CTA's half of the tokens, counted on the leader's barrier
-//   warp 27      MMA      : of the leader, 8 x 256 x ntok x 16 per stage; TMEM allocation
+//   warp 27      MMA      : of the leader, 8 x 256 x ntok x 16 per 128-k group; TMEM allocation
 //
 // The launch may start while its predecessor still runs, for as long as that takes (an all-reduce waits for its slowest rank).  A wait
 // that ends only after x has come would count that time, so no warp enters one before griddepcontrol.wait: the weights of the ring's first
@@ -65,6 +66,7 @@ __device__ __forceinline__ bool t2_tile(const W4TcParams& p, int i, T2Tile& t) {
     return t.n0 < p.N;
 }
 
+template <int SUB>
 __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_constant__ W4TcParams p) {
     using C = T2Cfg;
     extern __shared__ uint8_t smem_dyn[];
@@ -78,9 +80,12 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(smem + C::kMiscOff);
     volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t rank = cluster_rank();
-    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-    const int G = p.K / kW4GroupK;
+    const int splits = p.splits;
+    const uint32_t in_cluster = cluster_rank(), rank = in_cluster & 1, lead = in_cluster & ~1u;   // lead: the pair's leader
+    const int part = (int)(in_cluster >> 1), pair = (int)(blockIdx.x >> 1) / splits, pairs = (int)(gridDim.x >> 1) / splits;
+    // this pair's 128-k groups of a tile; a group behind K arrives as zeros, as its x does
+    const int stages_all = (p.K / kW4GroupK + SUB - 1) / SUB, g_first = stages_all * part / splits * SUB;
+    const int G = stages_all * (part + 1) / splits * SUB - g_first;
     const int slots = t2_slots(p.ntok), nacc = t2_accs(p.ntok), xstage = t2_x_bytes(p.ntok), acol0 = 512 - slots * 64;
     // a weight slot is held while its group converts and is then a round trip to L2 from being full again: more than two per group
     const int rslots = min(C::kMaxRaw, (C::kRing - slots * xstage) / (C::kNib + C::kTr));
@@ -92,8 +97,8 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
             mbar_init(&raw_full[i], 1);
             mbar_init(&raw_empty[i], C::kGroupWarps);
         }
-        for (int i = 0; i < slots; ++i) {
-            mbar_init(&a_full[i], 2 * C::kGroupWarps + 1);
+        for (int i = 0; i < slots / SUB; ++i) {
+            mbar_init(&a_full[i], 2 * SUB * C::kGroupWarps + 1);
             mbar_init(&ax_empty[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
@@ -110,6 +115,7 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
     cluster_sync_all();   // both CTAs' barriers and allocations are in place
     tc_fence_after();
     const uint32_t tmem = *s_tmem;
+    const int q = warp & 3, set = warp >> 2;   // epilogue warps; with K split a tile's only chunks come behind the exchange below
     T2Tile t;
 
     if (warp >= C::kWarpRaw && warp < C::kWarpX) {
@@ -139,11 +145,11 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
                     mbar_expect_tx(full, C::kNib + 4 * 80);
                     asm volatile(
                         "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(nib),
-                        "l"(reinterpret_cast<uint64_t>(&p.wmap2)), "r"(0), "r"(0), "r"(g), "r"(rec), "r"(bar)
+                        "l"(reinterpret_cast<uint64_t>(&p.wmap2)), "r"(0), "r"(0), "r"(g_first + g), "r"(rec), "r"(bar)
                         : "memory");
                     asm volatile(
                         "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(tr),
-                        "l"(reinterpret_cast<uint64_t>(&p.tmap)), "r"(0), "r"(g), "r"(rec), "r"(bar)
+                        "l"(reinterpret_cast<uint64_t>(&p.tmap)), "r"(0), "r"(g_first + g), "r"(rec), "r"(bar)
                         : "memory");
                 }
             }
@@ -158,18 +164,18 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
             const int box = p.ntok >> 1;   // rows of a load; a shorter last tile loads rows it does not use
             for (int i = pair; ok && t2_tile(p, i, t); i += pairs) {
                 const int tb = t.t0 + (int)rank * (t.ntok >> 1);
-                for (int g = 0; g < G; ++g) {
+                for (int g = 0; g < G; g += SUB) {
                     if (!free && !(ok = tc2_wait1(&ax_empty[as], ph ^ 1u, s_abort, p.err, 0x3200 + as))) break;
                     uint64_t* const full = &a_full[as];
-                    uint8_t* dst = smem + as * xstage;
-                    if (++as == slots) {
+                    uint8_t* dst = smem + as * (SUB * xstage);
+                    if (++as == slots / SUB) {
                         as = 0;
                         ph ^= 1u;
                     }
                     free = mbar_test(&ax_empty[as], ph ^ 1u);
-                    if (rank == 0) mbar_expect_tx(full, (uint32_t)(4 * box * 128));
-                    const uint32_t bar = cluster_map(smem_u32(full), 0);
-                    tma2_load_3d(dst, &p.xmap, 0, tb, g * 2, bar);   // two 64-k atoms
+                    if (rank == 0) mbar_expect_tx(full, (uint32_t)(4 * SUB * box * 128));
+                    const uint32_t bar = cluster_map(smem_u32(full), lead);
+                    tma2_load_3d(dst, &p.xmap, 0, tb, (g_first + g) * 2, bar);   // 2 SUB 64-k atoms
                 }
             }
         }
@@ -184,22 +190,22 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
             for (int i = pair; ok && t2_tile(p, i, t); i += pairs) {
                 if (!(ok = tc2_wait1(&acc_empty[acc], acc_ph ^ 1u, s_abort, p.err, 0x3300 + acc))) break;
                 const uint32_t d = tmem + (uint32_t)(acc * 64), idesc = tc2_idesc(false, t.ntok);
-                for (int g = 0; g < G; ++g) {
+                for (int g = 0; g < G; g += SUB) {
                     if (!ready && !(ok = tc2_wait1(&a_full[as], ph, s_abort, p.err, 0x3400 + as))) break;
-                    const uint32_t a = tmem + (uint32_t)(acol0 + as * 64);
-                    const uint64_t xd = tc_desc_sw128(smem_u32(smem + as * xstage));
+                    const uint32_t a = tmem + (uint32_t)(acol0 + as * (64 * SUB));
+                    const uint64_t xd = tc_desc_sw128(smem_u32(smem + as * (SUB * xstage)));
                     uint64_t* const used = &ax_empty[as];
-                    if (++as == slots) {
+                    if (++as == slots / SUB) {
                         as = 0;
                         ph ^= 1u;
                     }
                     ready = mbar_test(&a_full[as], ph);   // looking at a barrier takes 200 cycles: they pass under this stage's MMAs
                     tc_fence_after();
 #pragma unroll
-                    for (int j = 0; j < 8; ++j)
+                    for (int j = 0; j < 8 * SUB; ++j)
                         tc2_mma_ts(d, a + (uint32_t)(j * 8), xd + (j >> 2) * atom + (uint64_t)((j & 3) * 2), idesc, (g > 0 || j > 0) ? 1u : 0u);
-                    tc2_commit(used);
-                    if (g == G - 1) tc2_commit(&acc_full[acc]);
+                    tc2_commit(used, lead);
+                    if (g == G - SUB) tc2_commit(&acc_full[acc], lead);
                 }
                 if (++acc == nacc) {
                     acc = 0;
@@ -209,7 +215,7 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
         }
         __syncwarp();
     } else if (warp >= C::kWarpDq0) {
-        const int group = (warp - C::kWarpDq0) >> 2, q = warp & 3;
+        const int group = (warp - C::kWarpDq0) >> 2;
         const int tt = lane >> 4, hi = (lane >> 3) & 1, g8 = lane & 7;
         const uint32_t mask = hi ? 0xf0f0f0f0u : 0x0f0f0f0fu;
         const uint32_t magic = hi ? 0x54545454u : 0x64646464u;   // 64 + n / 16 for a high nibble n, 1024 + n for a low one
@@ -224,7 +230,7 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
             if (st >= slots && st < slots + C::kGroups) pdl_wait();
             if (!raw_ready && !tc2_wait(&raw_full[rs], rph, s_abort, p.err, 0x3600 + rs)) break;
             // looking at a barrier takes 200 cycles: they pass under the conversion
-            const bool free = mbar_test(&ax_empty[as], ph ^ 1u);
+            const bool free = mbar_test(&ax_empty[as / SUB], ph ^ 1u);
             const uint8_t* nib = nibs + rs * C::kNib + q * 2048 + (g8 >> 1) * 128;
             const uint8_t* tr = trs + rs * C::kTr + q * 80;
             uint64_t* const used = &raw_empty[rs];
@@ -268,7 +274,7 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
                     }
                 }
                 if (ks == 0) {
-                    if (!__all_sync(0xffffffffu, free) && !(ok = tc2_wait(&ax_empty[as], ph ^ 1u, s_abort, p.err, 0x3700 + as))) break;
+                    if (!__all_sync(0xffffffffu, free) && !(ok = tc2_wait(&ax_empty[as / SUB], ph ^ 1u, s_abort, p.err, 0x3700 + as))) break;
                     tc_fence_after();
                 }
                 tc_st16(taddr + (uint32_t)(ks * 32), r[0]);
@@ -278,7 +284,7 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
             tc_wait_st();
             tc_fence_before();
             raw_ready = __all_sync(0xffffffffu, next);   // one arrival per warp
-            if (lane == 0) mbar_arrive_at(cluster_map(smem_u32(&a_full[as]), 0));
+            if (lane == 0) mbar_arrive_at(cluster_map(smem_u32(&a_full[as / SUB]), lead));
             as += C::kGroups;
             if (as >= slots) {
                 as -= slots;
@@ -286,17 +292,17 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
             }
         }
     } else {
-        const int q = warp & 3, set = warp >> 2;
         int acc = 0;
         uint32_t acc_ph = 0;
         pdl_wait();
         for (int i = pair; t2_tile(p, i, t); i += pairs) {
             const int prow = t.n0 + (int)rank * 128 + q * 32 + lane;
-            const bool res = p.epi == ZL_EPI_RESIDUAL && p.wide && prow < p.N;
+            const bool res = p.epi == ZL_EPI_RESIDUAL && p.wide && prow < p.N && splits == 1;
             uint32_t rnext[8];
             if (res) tc_fetch_residual(p, prow, lane, t.t0 + set * 16, rnext);
             if (!tc2_wait(&acc_full[acc], acc_ph, s_abort, p.err, 0x3800 + acc)) break;
             tc_fence_after();
+            if (splits > 1) break;
             const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * 64);
             if (prow < p.N) {               // N % 128 == 0: all of the CTA's rows or none
                 for (int c0 = set * 16; c0 < t.ntok && t.t0 + c0 < p.M; c0 += 32) {
@@ -315,7 +321,7 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_at(cluster_map(smem_u32(&acc_empty[acc]), 0));
+            if (lane == 0) mbar_arrive_at(cluster_map(smem_u32(&acc_empty[acc]), lead));
             if (++acc == nacc) {
                 acc = 0;
                 acc_ph ^= 1u;
@@ -326,7 +332,32 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
     tc2_drain(s_abort);
     tc_fence_before();
     __syncthreads();
-    cluster_sync_all();   // nobody's shared memory or TMEM goes while the other CTA may still use it
+    cluster_sync_all();   // nobody's shared memory or TMEM goes, or takes sums, while another CTA may still use it
+    if (splits > 1) {
+        tc_fence_after();
+        const bool any = t2_tile(p, pair, t);
+        const int row = q * 32 + lane, prow = t.n0 + (int)rank * 128 + row;
+        const bool epilogue = warp < C::kEpiWarps && any && prow < p.N;
+        const int chunks = min(t.ntok, p.M - t.t0 + 15) / 16;
+        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16);
+        if (epilogue)
+            for (int c = set; c < chunks; c += 2) {
+                if (c % splits == part) continue;
+                float v[16];
+                tc_ld16(taddr + (uint32_t)(c * 16), v);
+                tc2_split_push(smem_u32(smem), (int)rank, part, c, splits, chunks, row, v);
+            }
+        cluster_sync_all();
+        if (epilogue)
+            for (int c = part + set * splits; c < chunks; c += 2 * splits) {
+                float v[16];
+                tc_ld16(taddr + (uint32_t)(c * 16), v);
+                tc2_split_sum<false>(smem, part, c, splits, chunks, row, v);
+                tc_epilogue16(p, prow, lane, t.t0 + c * 16, v);
+            }
+        tc_fence_before();
+        __syncthreads();
+    }
     if (warp == C::kWarpMma) {
         tc_fence_after();
         tc2_dealloc(tmem);
@@ -335,35 +366,61 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
 
 // ---- host side --------------------------------------------------------------------------------------------------------
 cudaError_t prepare_w4_tc2() {
-    return cudaFuncSetAttribute(k_w4a16_tc2, cudaFuncAttributeMaxDynamicSharedMemorySize, T2Cfg::kBytes);
+    const cudaError_t e = cudaFuncSetAttribute(k_w4a16_tc2<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, T2Cfg::kBytes);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(k_w4a16_tc2<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, T2Cfg::kBytes);
 }
 
-// Tokens per tile: the waves of the launch times a tile's cost.  A 128-k group costs its MMAs (4.24 cycles per token) or the conversion and
-// hand-over of its weights (650 cycles, and from about 100 tokens on both get into each other's way: 400 + 2.6 per token), whichever is
-// longer; with one accumulator the epilogue comes on top.
-static double t2_cost(int n, long long tiles, int G, int pairs) {
-    const double group = fmax(650.0, fmax(4.24 * n, 400.0 + 2.6 * n));
-    return (double)((tiles + pairs - 1) / pairs) * (G * group + (n > 64 ? 14.0 * n : 300.0));
+// 128-k groups of a stage.  Handing a stage over costs the MMA warp 460 cycles whatever is in it, which is what bounded up to 128 tokens; of
+// two groups per stage 300 a group are left beside the conversion (28672 x 4096, 32 tokens: 33 -> 30.4 us; 4096 x 14336 45 -> 43).  Above,
+// the MMAs are the longer and four slots of A are too few to pair.
+static int t2_sub(int ntok) { return ntok <= 128 ? 2 : 1; }
+
+// Tokens per tile, and how many pairs share a tile's K: with few tiles the pairs of a cluster (the device holds t2_clusters(s) clusters of s pairs
+// at a time: 33, 22, 15 of 2, 3, 4) take a part each and exchange their sums.  Microseconds, fitted to the times below: a 128-k group costs its
+// conversion (0.31) or its MMAs (0.0022 per token; above 128 tokens the two get into each other's way), a tile's start and end 8.8 + 0.03 per
+// token, a further wave less than that, since two accumulators (up to 64 tokens) or only the next tile's first groups hide the epilogue.
+// Measured, one pair / two / three, N x K, us: 4096 x 14336, 32 tokens 43 / 27 / 22.7, 96 tokens 45 / 31 / 24.7, 256 tokens 46.5 / 33 / -;
+// 4096 x 4096, 96 tokens 18.8 / 16.5 / 16.5, 128 tokens 19.7 / 16.5 / 18.2; 6144 x 4096, 64 tokens 19.0 / 16.5 / -; 8192 x 3584, 128 tokens
+// 19.7 / 18.6 / -.
+struct T2Pick {
+    int ntok, splits;
+    double us;
+};
+static int t2_clusters(int splits) {
+    static PairsFit fit;
+    return pairs_clusters(k_w4a16_tc2<1>, T2Cfg::kThreads, T2Cfg::kBytes, splits, fit);
 }
-static int t2_pick_ntok(int M, int row_tiles, int G, int pairs) {
-    int best = 32;
+static T2Pick t2_pick(int M, int row_tiles, int G) {
+    const int pairs = device_sm_count() / 2;
+    T2Pick best{32, 1, 1e30};
     for (int n = 32; n <= 256; n += 32) {
-        if (t2_cost(n, (long long)row_tiles * cdiv(M, n), G, pairs) < t2_cost(best, (long long)row_tiles * cdiv(M, best), G, pairs)) best = n;
+        const long long tiles = (long long)row_tiles * cdiv(M, n), waves = (tiles + pairs - 1) / pairs;
+        const double group = n <= 128 ? fmax(0.31, 0.0022 * n) : fmax(0.00223 * n, 0.21 + 0.00137 * n);
+        const double further = (double)(waves - 1) * (n <= 64 ? 0.3 : n <= 128 ? 3.0 + 0.03 * n : 0.0074 * n);
+        for (int s = 1; s <= 4; ++s) {
+            const int sub = t2_sub(n), mine = cdiv(cdiv(G, sub), s) * sub;
+            if (s > 1 && (cdiv(G, sub) < 2 * s || tiles * s > pairs || tiles > t2_clusters(s))) break;
+            const double us = 8.8 + 0.03 * n + (double)waves * mine * group + further + (s > 1 ? 1.2 + 0.01 * n : 0.0);
+            if (us < best.us - 1e-9) best = T2Pick{n, s, us};
+        }
         if (n >= M) break;
     }
     return best;
 }
 
-// Whether M tokens are this kernel's.  Beyond 256 w4a16_tc.cu would need several passes; below, whole tiles on few pairs stand against
-// its ranges over all SMs and their exchange: 10 us + 4.2 ns per token and million weights.  Measured, this kernel against that one:
-// 28672 x 4096 at M = 48 / 64 / 128: 32 / 32 / 38 against 37 / 41 / 60 us; 4096 x 14336 at M = 128 / 144 / 192: 45 / 45 / 44 against
-// 39 / 46 / 56; 6144 x 4096 at M = 64 / 96: 19 / 19 against 21 / 26; 4096 x 4096 at M = 112 / 144: 20 / 20 against 21 / 24.
+// Whether M tokens are this kernel's.  Beyond 256 w4a16_tc.cu would need several passes; below, tiles on few pairs stand against its ranges
+// over all SMs and their exchange: 10 us + 4.2 ns per token and million weights.  Measured, N x K, there / here, us: 4096 x 14336 at M = 64 / 96 /
+// 128 / 256 24.7 / 36 / 39 / 55 and 24.2 / 24.7 / 26.7 / 33; 6144 x 4096 at M = 96 / 256 22.3 / 24.7 and 18.4 / 22.6; 28672 x 4096 at M = 32 / 64
+// 32.9 / 36.7 and 30.4 / 31.2, of which a pair of feed-forward calls at M = 32 keeps nothing (54.0 and 54.9); 512 x 14336 at M = 32 13 and 23.
+// Where its ranges are down to eight groups every tile is cut, and what is exchanged grows with M (2304 x 1152 at M = 40 / 256: 18 / 51 there,
+// 12 / 12.4 here; 1664 x 2176: 17 / 50 and 12.4 / 14.5; 3328 x 5248 at M = 128: 31 and 17.5).
 bool w4_tc2_route(int M, int N, int K) {
     if (M <= 16 || N % kTcRows || K % kW4GroupK) return false;
     if (M > 256) return true;
-    const int row_tiles = cdiv(N, kTc2Rows), G = K / kW4GroupK, pairs = device_sm_count() / 2, n = t2_pick_ntok(M, row_tiles, G, pairs);
-    const double here = 7.0 + t2_cost(n, (long long)row_tiles * cdiv(M, n), G, pairs) / 1900.0;
-    return here < 10.0 + 4.2e-9 * M * (double)N * K;
+    const int G = K / kW4GroupK;
+    const double there = 10.0 + 4.2e-9 * M * (double)N * K;
+    const bool cut = M > 32 && (long long)(N / kTcRows) * G < 8 * device_sm_count();
+    return t2_pick(M, cdiv(N, kTc2Rows), G).us < there + (!cut ? 0.0 : K < 4096 ? 0.1 * M : N >= 1024 ? 0.015 * M : 0.0);
 }
 
 // all M tokens in one launch
@@ -374,18 +431,26 @@ cudaError_t launch_w4_tc2(const W4Params& p, bool pdl, cudaStream_t stream) {
     if (!words) return cudaErrorMemoryAllocation;
     if (!w4_tc_params(q, p)) return cudaErrorInvalidValue;
     q.err = words + kWaitW4Pairs;
-    q.ntok = t2_pick_ntok(p.mc, row_tiles, G, max_pairs);
+    const T2Pick pick = t2_pick(p.mc, row_tiles, G);
+    const int sub = t2_sub(pick.ntok);
+    q.ntok = pick.ntok;
+    q.splits = pick.splits;
     q.tok_tiles = cdiv(p.mc, q.ntok);
-    {   // x as [K / 64][M][64]: a stage's two atoms of half the tokens are one box
+    {   // x as [K / 64][M][64]: a stage's atoms of half the tokens are one box
         const uint64_t dims[3] = {64, (uint64_t)p.mc, (uint64_t)p.K / 64}, strides[2] = {(uint64_t)p.ldx * 2, 128};
-        const uint32_t box[3] = {64, (uint32_t)q.ntok / 2, 2};
+        const uint32_t box[3] = {64, (uint32_t)q.ntok / 2, (uint32_t)(2 * sub)};
         if (!tc_make_map_nd(&q.xmap, p.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B)) return cudaErrorInvalidValue;
     }
     const int tiles = row_tiles * q.tok_tiles;
-    return launch_pairs(k_w4a16_tc2, tiles < max_pairs ? tiles : max_pairs, 1, dim3(T2Cfg::kThreads), (size_t)T2Cfg::kBytes, stream, pdl, q);
+    return launch_pairs(sub == 2 ? k_w4a16_tc2<2> : k_w4a16_tc2<1>, (tiles < max_pairs ? tiles : max_pairs) * q.splits, q.splits, dim3(T2Cfg::kThreads),
+                        (size_t)T2Cfg::kBytes, stream, pdl, q);
 }
 
 }  // namespace zl
+
+extern "C" int zl_w4_pairs_splits(int M, int N, int K) {
+    return zl_w4_pairs_route(M, N, K) ? zl::t2_pick(M, zl::cdiv(N, zl::kTc2Rows), K / zl::kW4GroupK).splits : 0;
+}
 
 extern "C" unsigned zl_w4_tc2_watchdog(void) {
     cudaDeviceSynchronize();
