@@ -1,0 +1,115 @@
+"""GPU: the calls that go through the native host module give what the general path of ops.py gives, in every form of their arguments, and refuse the
+same.  The same kernels run on the same inputs: results are equal bit for bit."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _both(monkeypatch, f):
+    """f() through the native module (which has to serve it unless it says otherwise) and through the general path."""
+    from zhilight_b200 import ZLError, _lib
+    outs = []
+    for host in (_lib.host, None):
+        with monkeypatch.context() as m:
+            m.setattr(_lib, "host", host)
+            try:
+                outs.append(f())
+            except (ZLError, RuntimeError, ValueError, IndexError, TypeError) as e:
+                outs.append((type(e), getattr(e, "code", None)))
+    return outs
+
+
+def _same(outs):
+    a, b = outs
+    if isinstance(a, tuple) or isinstance(b, tuple):
+        assert a == b
+    else:
+        assert a.dtype == b.dtype and a.shape == b.shape and a.stride() == b.stride() and torch.equal(a, b)
+
+
+class _Own(torch.Tensor):
+    pass
+
+
+FORMS = {"plain": lambda t: t, "strided": lambda t: torch.cat([t, t], 1)[:, :t.shape[1]], "parameter": lambda t: torch.nn.Parameter(t, requires_grad=False),
+         "subclass": lambda t: t.as_subclass(_Own), "flat": lambda t: t[0], "float": lambda t: t.float(), "narrow": lambda t: t[:, :64]}
+
+
+@pytest.mark.parametrize("form", sorted(FORMS))
+@pytest.mark.parametrize("m", [1, 40])
+def test_linears(lib, cuda, monkeypatch, form, m):
+    from zhilight_b200 import layers
+    g = torch.Generator(device="cuda").manual_seed(m)
+    k, n = 512, 384
+    for quant, dtype in ((0, "bfloat"), (0, "half"), (1, "half"), (7, "bfloat"), (5, "half")):
+        w = torch.randn(n, k, generator=g, device=cuda)
+        sd = {"bias": torch.randn(n, generator=g, device=cuda)}
+        if quant == 1:
+            sd.update(weight=torch.randint(-127, 128, (n, k), generator=g, device=cuda, dtype=torch.int8), weight_scale=torch.rand(n, generator=g, device=cuda) * 0.01)
+        elif quant == 7:
+            sd.update(weight=w.clamp(-4, 4).to(torch.float8_e4m3fn).view(torch.uint8), weight_scale=torch.tensor([0.1], device=cuda))
+        elif quant == 5:
+            sd.update(qweight=torch.randint(-2 ** 31, 2 ** 31 - 1, (k // 8, n), generator=g, device=cuda, dtype=torch.int64).int(),
+                      qzeros=torch.full((k // 128, n // 8), 0x77777777, dtype=torch.int32, device=cuda), scales=torch.rand(k // 128, n, generator=g, device=cuda).half() * 0.01)
+        else:
+            sd["weight"] = w * 0.05
+        lin = layers.Linear(k, n, "", quant, dtype)
+        lin.load_state_dict(sd)
+        x = torch.randn(m, k, generator=g, device=cuda).to(lin.dtype)
+        _same(_both(monkeypatch, lambda: lin(FORMS[form](x))))
+        _same(_both(monkeypatch, lambda: lin(x[None])))
+
+
+def test_entry_points(lib, cuda, monkeypatch):
+    from zhilight_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(0)
+    x, w = torch.randn(3, 256, generator=g, device=cuda).half(), torch.randn(512, 256, generator=g, device=cuda).half()
+    for f in (lambda: ops.dense_gemm_skinny(x, w, out_dtype=torch.float32), lambda: ops.dense_gemm_skinny(x, w, out_dtype=torch.float64),
+              lambda: ops.dense_gemm_skinny(x, w.t()), lambda: ops.dense_gemm_skinny(x[:, :7].contiguous(), w[:, :7].contiguous()), lambda: ops.dense_gemm_skinny(x.cpu(), w),
+              lambda: ops.int8_linear(x, w.to(torch.int8), torch.rand(512, device=cuda, generator=torch.Generator(device="cuda").manual_seed(1))),
+              lambda: ops.int8_linear(x[:0], w.to(torch.int8), torch.ones(512, device=cuda)), lambda: ops.fp8_linear(x, w.to(torch.int8), torch.ones(1, device=cuda).double())):
+        _same(_both(monkeypatch, f))
+
+
+@pytest.mark.parametrize("b,len_q", [(1, 1), (5, 1), (1, 40)])
+def test_attention(lib, cuda, monkeypatch, b, len_q):
+    from zhilight_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(b)
+    lens = [300 - 17 * i for i in range(b)]
+    q = torch.randn(b, len_q, 8, 128, generator=g, device=cuda).half()
+    ks, vs = ([torch.randn(n, 2, 128, generator=g, device=cuda).half() for n in lens] for _ in range(2))
+    length = torch.tensor(lens, dtype=torch.int32, device=cuda)
+    mask = torch.ones(len_q, lens[0], device=cuda).tril(lens[0] - len_q).to(torch.int8) if len_q > 1 else None
+
+    def call(k=ks, v=vs, m=mask, scale=0.09, query=q):
+        return ops.decode_attention(query, length, k, v, m, scale, max(lens), 2)
+    for f in (call, lambda: call(tuple(ks), tuple(vs)), lambda: call(iter(ks), list(vs)), lambda: call(scale=1), lambda: call(query=torch.cat([q, q], 3)[..., :128]),
+              lambda: call([t.as_subclass(_Own) for t in ks]), lambda: call([torch.from_dlpack(t) for t in ks]), lambda: call(query=q.double()),
+              lambda: call(query=q[0])):
+        _same(_both(monkeypatch, f))
+
+
+def test_memory_of_another_stream_outlives_its_tensors(lib, cuda):
+    """A cache that was allocated on another stream and dropped at once is not given away before the call has read it."""
+    from zhilight_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(0)
+    n = 4096
+    q = torch.randn(1, 1, 8, 128, generator=g, device=cuda).half()
+    k, v = (torch.randn(n, 2, 128, generator=g, device=cuda).half() for _ in range(2))
+    length = torch.tensor([n], dtype=torch.int32, device=cuda)
+    ref = ops.decode_attention(q, length, [k], [v], None, 0.09, n, 2)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        k2, v2 = k.clone(), v.clone()
+    torch.cuda.current_stream().wait_stream(side)
+    torch.cuda._sleep(20_000_000)
+    out = ops.decode_attention(q, length, [k2], [v2], None, 0.09, n, 2)
+    at = {k2.data_ptr(), v2.data_ptr()}
+    del k2, v2
+    with torch.cuda.stream(side):
+        new = [torch.full_like(k, 7.0) for _ in range(4)]
+    assert not at & {t.data_ptr() for t in new}
+    torch.cuda.synchronize()
+    assert torch.equal(out, ref)

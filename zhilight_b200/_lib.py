@@ -116,6 +116,7 @@ def parse_header(path=HEADER):
 
 _lib = None
 _protos = None
+host = None   # once loaded: the native module of the calls that are made per layer and token (csrc/host/torch_calls.cpp)
 
 
 _path = None
@@ -132,7 +133,7 @@ def use(path):
 
 def load():
     """Load the library (building nothing).  Raises if the .so is absent."""
-    global _lib, _protos
+    global _lib, _protos, host
     if _lib is not None:
         return _lib
     path = _path or LIB_PATH
@@ -149,7 +150,9 @@ def load():
         fn = getattr(lib, name)          # AttributeError if the symbol is missing
         fn.restype = ctypes.c_char_p if ret.replace("const", "").strip() == "char*" else _ctype(ret)
         fn.argtypes = [_ctype(t) for t, _ in params]
-    _lib = lib
+    from . import _host              # built with the library; ImportError if it is missing
+    _host.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in _protos})
+    _lib, host = lib, _host
     return lib
 
 

@@ -81,7 +81,7 @@ class Linear:
             raise _lib.ZLError(-1, "Input size mismatch")
         if x.dtype != self.dtype:
             raise _lib.ZLError(-1, "Input data type mismatch")
-        x2 = x.reshape(-1, self.dim_in).contiguous()
+        x2 = (x if x.dim() == 2 else x.reshape(-1, self.dim_in)).contiguous()
         q, n, k = self.quant, self.dim_out, self.dim_in
         if q == QUANT_NONE:
             y = ops.dense_gemm_skinny(x2, self._p["weight"], self.bias)
@@ -93,6 +93,6 @@ class Linear:
             y = ops.w4a16_gemm_fused(x2, self._packed, n, k, self.group_size, bias=self.bias, variant=self._variant)
         if self.activation:
             y = ops.activation(y, self.activation)
-        return y.reshape(*x.shape[:-1], n)
+        return y if x.dim() == 2 else y.reshape(*x.shape[:-1], n)
 
     __call__ = forward

@@ -39,6 +39,16 @@ def _stream():
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
+def _done(y):
+    """What a function of the native module returned, other than None: the result, or the library's error code."""
+    if y.__class__ is int:
+        _lib.check(y)
+    return y
+
+
+_CODES = {None: None, torch.float16: F16, torch.bfloat16: BF16, torch.float32: F32}
+
+
 def check_waits():
     """After a synchronisation: raises if a bounded wait inside a GEMM over pairs of SMs has given up, its output being incomplete.
     The decoders and the next call of such a GEMM raise by themselves."""
@@ -174,6 +184,10 @@ def w4a16_gemm_fused(x, packed, n, k, group_size=128, bias=None, residual=None, 
                      ln_weight=None, eps=1e-5, rope=None, variant=0):
     """zl_w4a16_gemm_fused.  rope = dict(cos, sin, token_batch, placement, k_bufs, v_bufs, num_heads, num_kv_heads,
     dim_head) for EPI_QKV_ROPE (returns q); bias must be in packed-row order."""
+    if _lib.host is not None and ln_weight is None and rope is None:
+        y = _lib.host.w4a16_gemm_fused(x, packed, n, k, group_size, bias, residual, epilogue, pdl, out, variant)
+        if y is not None:
+            return _done(y)
     if x.dtype != torch.float16:
         raise _lib.ZLError(-2, "A must be half")
     m = x.shape[0]
@@ -205,6 +219,10 @@ def w4a16_gemm_fused(x, packed, n, k, group_size=128, bias=None, residual=None, 
 
 
 def dense_gemm_skinny(x, w, bias=None, out_dtype=None, pdl=False):
+    if _lib.host is not None:
+        y = _lib.host.dense_gemm_skinny(x, w, bias, _CODES.get(out_dtype, -1), pdl)
+        if y is not None:
+            return _done(y)
     m, k = x.shape
     n = w.shape[0]
     od = x.dtype if out_dtype is None else out_dtype
@@ -257,6 +275,10 @@ def w8a8_gemm(xq, x_scale, w, w_scale, out_dtype, kind=W8_INT8, bias=None, pdl=F
 
 def int8_linear(x, w_q, w_scale, bias=None, pdl=False):
     """Int8Linear::forward (linear.cpp:560-636) in two launches instead of three."""
+    if _lib.host is not None:
+        y = _lib.host.w8_linear(x, w_q, w_scale, bias, W8_INT8, pdl)
+        if y is not None:
+            return _done(y)
     q, s = int8_quant_per_token(x, pdl)
     # the launch before is the quantisation, itself behind everything earlier: the GEMM may start on its weights during it
     return w8a8_gemm(q, s, w_q, w_scale, x.dtype, W8_INT8, bias, True)
@@ -264,6 +286,10 @@ def int8_linear(x, w_q, w_scale, bias=None, pdl=False):
 
 def fp8_linear(x, w_fp8, w_scale, bias=None, pdl=False):
     """Fp8Linear::forward (linear.cpp:1660-1695)."""
+    if _lib.host is not None:
+        y = _lib.host.w8_linear(x, w_fp8, w_scale, bias, W8_FP8, pdl)
+        if y is not None:
+            return _done(y)
     q, s = fp8_quant_per_tensor(x, pdl)
     return w8a8_gemm(q, s, w_fp8, w_scale, x.dtype, W8_FP8, bias, True)
 
@@ -384,6 +410,10 @@ def qkv_rope_append(cos, sin, qkv, token_batch, placement, k_bufs, v_bufs, num_h
 
 def decode_attention(q, buf_lens, k_bufs, v_bufs, mask, scale, max_len_buf, num_kv_heads, bshd=True, pdl=False):
     """nn::multi_query_attention_rag_buffer: q (B, len_q, H_q, d); k_bufs/v_bufs lists of per-task tensors."""
+    if _lib.host is not None:
+        out = _lib.host.decode_attention(q, buf_lens, k_bufs, v_bufs, mask, scale, max_len_buf, num_kv_heads, bshd, pdl)
+        if out is not None:
+            return _done(out)
     b, len_q, hq, d = q.shape
     out = torch.empty_like(q)
     ws_bytes = _lib.load().zl_decode_attention_workspace_bytes(b, len_q, hq, d, max_len_buf)
