@@ -268,6 +268,9 @@ int zl_qkv_rope_append(const float* cos, const float* sin, const void* qkv, void
 /* one-shot hint: the NEXT zl_decode_attention call on this thread also prefetches [ptr, ptr+bytes) into L2
  * (weights of a later GEMM; attention leaves HBM idle at small batch). */
 int zl_decode_attention_set_prefetch(const void* ptr, size_t bytes);
+/* one-shot hint: the NEXT zl_decode_attention call on this thread has the mask, lengths, sizes, workspace and stream of the call before, which
+ * nothing has written to since (the layers of a prompt's portion): what that call derived from the mask is used again. */
+int zl_decode_attention_same_mask(void);
 size_t zl_decode_attention_workspace_bytes(int B, int len_q, int num_heads, int dim_head, int max_len_buf);
 /* q (B, len_q, H_q, d); buf_lens (B); k_addrs/v_addrs (B) device arrays of device pointers;
  * mask int8 ragged concat of (len_q, len_buf_b); out (B, len_q, H_q, d).  bshd: (len_buf, H_kv, d) else

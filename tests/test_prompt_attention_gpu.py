@@ -130,3 +130,30 @@ def test_blocks_of_rows_and_clusters_of_splits(lib, cuda, hq, hkv, d, len_q, ctx
         for scale in (d ** -0.5, -d ** -0.5, 0.0):
             out = ops.decode_attention(qd, lens, [k.to(cuda)], [v.to(cuda)], mask.to(cuda), scale, ctx, hkv)[0]
             assert rel_l2(out.double().cpu().numpy(), _exact(q, k, v, mask, scale).numpy()) <= TOL[torch.bfloat16][1], (qd is shifted, scale)
+
+
+@pytest.mark.parametrize("d,len_q,ctx", [(128, 200, 333), (64, 100, 1100), (128, 3, 40)])
+def test_layers_that_share_a_mask(lib, cuda, d, len_q, ctx):
+    """The second call uses the bits that the first one left (also where the decode kernels serve it, which have none), the third derives them again."""
+    from zhilight_b200 import _lib, ops
+    g = torch.Generator(device="cuda").manual_seed(5)
+    hq, hkv = 8, 2
+    q = torch.randn(1, len_q, hq, d, generator=g, device=cuda).half()
+    k, v = (torch.randn(ctx, hkv, d, generator=g, device=cuda).half() for _ in range(2))
+    lens = torch.tensor([ctx], dtype=torch.int32, device=cuda)
+    mask, other = _causal(len_q, ctx).to(cuda), (torch.rand(len_q, ctx, generator=g, device=cuda) < 0.5).to(torch.int8)
+    table = torch.tensor([k.data_ptr(), v.data_ptr()], dtype=torch.int64, device=cuda)
+    size = lib.zl_decode_attention_workspace_bytes(1, len_q, hq, d, ctx)
+    ws = torch.empty(size, dtype=torch.uint8, device=cuda)
+
+    def call(m):
+        out = torch.empty_like(q)
+        _lib.call("zl_decode_attention", q.data_ptr(), lens.data_ptr(), table.data_ptr(), table.data_ptr() + 8, m.data_ptr(), d ** -0.5, ctx, out.data_ptr(), 1,
+                  len_q, hq, hkv, d, 1, ws.data_ptr(), size, ops.F16, 0, torch.cuda.current_stream().cuda_stream)
+        return out
+    first = call(mask)
+    lib.zl_decode_attention_same_mask()
+    assert torch.equal(call(mask), first)
+    third = call(other)
+    assert not torch.equal(third, first)
+    assert torch.equal(third, ops.decode_attention(q, lens, [k], [v], other, d ** -0.5, ctx, hkv))

@@ -360,6 +360,12 @@ extern "C" int zl_decode_attention_set_prefetch(const void* ptr, size_t bytes) {
     g_attn_pf_bytes = bytes;
     return ZL_OK;
 }
+// one-shot as well: the layers of a prompt's portion share its mask, whose bits the first one's call has left in the workspace
+static thread_local bool g_attn_mask_ready = false;
+extern "C" int zl_decode_attention_same_mask(void) {
+    g_attn_mask_ready = true;
+    return ZL_OK;
+}
 
 extern "C" size_t zl_decode_attention_workspace_bytes(int B, int len_q, int num_heads, int dim_head,
                                                       int max_len_buf) {
@@ -395,7 +401,7 @@ static bool prompt_route(int len_q, int m_query, int dim_head, int B, int num_kv
 template <typename T, int D>
 static int prompt_attention(const void* q, const int32_t* buf_lens, void* const* k_addrs, void* const* v_addrs, const int8_t* mask, float scale,
                             int max_len_buf, void* out, int B, int len_q, int num_heads, int num_kv_heads, int bshd, void* workspace,
-                            size_t workspace_bytes, int pdl, zl_stream_t stream) {
+                            size_t workspace_bytes, int pdl, bool mask_ready, zl_stream_t stream) {
     const int m_query = num_heads / num_kv_heads;
     const int blocks = cdiv(len_q * m_query, kPaRows), tiles = cdiv(max_len_buf, kPaKeys);
     const int splits = prompt_attn_splits((long long)blocks * num_kv_heads * B, tiles);
@@ -412,11 +418,12 @@ static int prompt_attention(const void* q, const int32_t* buf_lens, void* const*
         ZL_CHECK_CUDA(cudaFuncSetAttribute(k_attn_prompt<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, PaCfg<D>::kBytes));
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
-    if (mask)
+    const bool mask_pass = mask && !mask_ready;
+    if (mask_pass)
         ZL_CHECK_CUDA(launch(k_mask_bits, dim3(len_q, B), dim3(256), 0, stream, pdl != 0, mask, buf_lens, bits, last, len_q, tiles));
     const int aligned = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
     // behind the mask's kernel the attention may start early whatever the caller's chain allows: it waits for that kernel to end
-    ZL_CHECK_CUDA((launch_attn_prompt<T, D>(dim3(blocks, num_kv_heads, B * splits), splits, stream, pdl != 0 || mask, (const T*)q, buf_lens,
+    ZL_CHECK_CUDA((launch_attn_prompt<T, D>(dim3(blocks, num_kv_heads, B * splits), splits, stream, pdl != 0 || mask_pass, (const T*)q, buf_lens,
                                             (T* const*)k_addrs, (T* const*)v_addrs, (const uint64_t*)bits, (const int32_t*)last, tiles, scale,
                                             (T*)out, len_q, num_heads, num_kv_heads, m_query, splits, bshd, aligned, words + kWaitAttnPrompt)));
     g_attn_pf_ptr = nullptr;
@@ -429,6 +436,8 @@ extern "C" int zl_decode_attention(const void* q, const int32_t* buf_lens, void*
                                    void* out, int B, int len_q, int num_heads, int num_kv_heads, int dim_head,
                                    int bshd, void* workspace, size_t workspace_bytes, int dtype, int pdl,
                                    zl_stream_t stream) {
+    const bool mask_ready = g_attn_mask_ready;
+    g_attn_mask_ready = false;
     ZL_CHECK_ARG(q && buf_lens && k_addrs && v_addrs && out && B > 0 && len_q > 0 && max_len_buf > 0);
     ZL_CHECK_ARG(num_heads > 0 && num_kv_heads > 0 && num_heads % num_kv_heads == 0);
     ZL_CHECK_SUPPORTED(dim_head == 64 || dim_head == 128);
@@ -437,13 +446,13 @@ extern "C" int zl_decode_attention(const void* q, const int32_t* buf_lens, void*
     if (prompt_route(len_q, m_query, dim_head, B, num_kv_heads, mask, max_len_buf, out, workspace, workspace_bytes)) {
         if (dtype == ZL_F16)
             return dim_head == 128 ? prompt_attention<__half, 128>(q, buf_lens, k_addrs, v_addrs, mask, scale, max_len_buf, out, B, len_q, num_heads,
-                                                                   num_kv_heads, bshd, workspace, workspace_bytes, pdl, stream)
+                                                                   num_kv_heads, bshd, workspace, workspace_bytes, pdl, mask_ready, stream)
                                    : prompt_attention<__half, 64>(q, buf_lens, k_addrs, v_addrs, mask, scale, max_len_buf, out, B, len_q, num_heads,
-                                                                  num_kv_heads, bshd, workspace, workspace_bytes, pdl, stream);
+                                                                  num_kv_heads, bshd, workspace, workspace_bytes, pdl, mask_ready, stream);
         return dim_head == 128 ? prompt_attention<__nv_bfloat16, 128>(q, buf_lens, k_addrs, v_addrs, mask, scale, max_len_buf, out, B, len_q,
-                                                                      num_heads, num_kv_heads, bshd, workspace, workspace_bytes, pdl, stream)
+                                                                      num_heads, num_kv_heads, bshd, workspace, workspace_bytes, pdl, mask_ready, stream)
                                : prompt_attention<__nv_bfloat16, 64>(q, buf_lens, k_addrs, v_addrs, mask, scale, max_len_buf, out, B, len_q,
-                                                                     num_heads, num_kv_heads, bshd, workspace, workspace_bytes, pdl, stream);
+                                                                     num_heads, num_kv_heads, bshd, workspace, workspace_bytes, pdl, mask_ready, stream);
     }
     int splits = attn_num_splits(B, len_q, num_kv_heads, m_query, max_len_buf);
     // latency regime: few CTAs of work -> 256-key CTAs that issue all their loads up front

@@ -132,12 +132,27 @@ __global__ void k_advance(int32_t* __restrict__ tokens, int32_t* __restrict__ po
 }
 // prefill chunk setup: positions pos0.., token -> task map, the task's buffer length, and the causal mask
 // mask[i][j] = j <= pos0 + i over len_buf = pos0 + n keys (attention_kernel.cu:434-489 mask contract, int8)
-__global__ void k_prefill_setup(int32_t* __restrict__ pos, int32_t* __restrict__ tb, int32_t* __restrict__ lens,
-                                int8_t* __restrict__ mask, int task, int pos0, int n) {
+// Bound by the mask's stores: 16 bytes of it per thread, whatever rows they belong to (512 x 1024: 17 us with a byte per thread and turn -> 3)
+__global__ void __launch_bounds__(256) k_prefill_setup(int32_t* __restrict__ pos, int32_t* __restrict__ tb, int32_t* __restrict__ lens,
+                                                       int8_t* __restrict__ mask, int task, int pos0, int n) {
     const int len_buf = pos0 + n;
-    for (int i = threadIdx.x + blockIdx.x * blockDim.x; i < n * len_buf; i += blockDim.x * gridDim.x) {
-        const int qi = i / len_buf, j = i % len_buf;
-        mask[i] = j <= pos0 + qi ? 1 : 0;
+    const long long all = (long long)n * len_buf;
+    for (long long i = (threadIdx.x + (long long)blockIdx.x * blockDim.x) * 16; i < all; i += (long long)blockDim.x * gridDim.x * 16) {
+        int qi = (int)(i / len_buf), j = (int)(i % len_buf);
+        uint32_t w[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+            if (j <= pos0 + qi) w[e >> 2] |= 1u << (8 * (e & 3));
+            if (++j == len_buf) {
+                j = 0;
+                ++qi;
+            }
+        }
+        if (i + 16 <= all) {
+            *reinterpret_cast<uint4*>(mask + i) = make_uint4(w[0], w[1], w[2], w[3]);   // the buffer is the allocator's: aligned
+        } else {
+            for (int e = 0; i + e < all; ++e) mask[i + e] = (int8_t)((w[e >> 2] >> (8 * (e & 3))) & 1u);
+        }
     }
     if (blockIdx.x == 0) {
         for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -550,7 +565,7 @@ int alloc_runtime(zl_llama* m) {
     }
     if (c.prefill_chunk > 0) {
         RCHECK(dmalloc((void**)&m->d_tb, T * 4));
-        RCHECK(dmalloc((void**)&m->d_pf_tokens, T * 4));
+        RCHECK(dmalloc((void**)&m->d_pf_tokens, (size_t)c.max_seq * 4));
         RCHECK(dmalloc((void**)&m->d_pf_pos, T * 4));
         RCHECK(dmalloc((void**)&m->d_mask, (size_t)c.prefill_chunk * c.max_seq));
     }
@@ -561,7 +576,7 @@ int alloc_runtime(zl_llama* m) {
     m->attn_ws_bytes = zl_decode_attention_workspace_bytes(T, 1, m->hq, d, c.max_seq);
     RCHECK(dmalloc(&m->attn_ws, m->attn_ws_bytes));
     RCHECK(dmalloc(&m->argmax_ws, zl_argmax_workspace_bytes(B)));
-    ZL_CHECK_CUDA(cudaMallocHost((void**)&m->h_stage, sizeof(int32_t) * (4 * B + 4 + T)));
+    ZL_CHECK_CUDA(cudaMallocHost((void**)&m->h_stage, sizeof(int32_t) * (4 * B + 4 + (c.prefill_chunk > 0 ? c.max_seq : 0))));
     ZL_CHECK_CUDA(cudaMallocHost((void**)&m->h_ring, sizeof(int32_t) * zl_llama::kStageSlots * 2 * B));
     for (int i = 0; i < zl_llama::kStageSlots; ++i)
         ZL_CHECK_CUDA(cudaEventCreateWithFlags(&m->ring_ev[i], cudaEventDisableTiming));
@@ -726,6 +741,7 @@ int dense_or_w8(zl_llama* m, const void* x, const DenseLin& L, void* y, int B, i
 struct PrefillChunk {
     int task, pos0, n;
     bool last;   // run final norm + lm_head + pick on the chunk's last token
+    int first;   // its place in d_pf_tokens
 };
 
 // ------------------------------------------------------------------------------------------------------------------
@@ -834,7 +850,8 @@ int enqueue_step(zl_llama* m, int n_tasks, int len_bucket, const PrefillChunk* p
     const float scale = 1.0f / sqrtf((float)d);   // attention.cpp:89
 
     if (pf) {
-        k_prefill_setup<<<8, 256, 0, st>>>(m->d_pf_pos, m->d_tb, m->d_lens, m->d_mask, pf->task, pf->pos0, pf->n);
+        const long long mask_bytes = (long long)pf->n * (pf->pos0 + pf->n);
+        k_prefill_setup<<<(unsigned)std::min<long long>((mask_bytes + 4095) / 4096, 1024), 256, 0, st>>>(m->d_pf_pos, m->d_tb, m->d_lens, m->d_mask, pf->task, pf->pos0, pf->n);
         ZL_CHECK_LAUNCH();
     } else {
         ZL_CHECK_CUDA(launch(k_lens_from_pos, dim3(cdiv(B, 64)), dim3(64), 0, st, false, (const int32_t*)m->d_pos,
@@ -842,7 +859,7 @@ int enqueue_step(zl_llama* m, int n_tasks, int len_bucket, const PrefillChunk* p
     }
     m->cur_tb = pf ? m->d_tb : m->d_iota;
     m->cur_pos = pf ? m->d_pf_pos : m->d_pos;
-    m->cur_tokens = pf ? m->d_pf_tokens : m->d_tokens;
+    m->cur_tokens = pf ? m->d_pf_tokens + pf->first : m->d_tokens;
     RCHECK(zl_rope_cos_sin(m->cur_pos, m->cosb, m->sinb, B, d, c.rope_theta, c.rope_llama3_factor,
                            c.rope_low_freq_factor, c.rope_high_freq_factor, c.rope_orig_ctx, 1, st));
     RCHECK(zl_embedding(m->cur_tokens, m->emb, m->h, B, D, c.vocab_size, dt, 0, st));
@@ -905,6 +922,7 @@ int enqueue_step(zl_llama* m, int n_tasks, int len_bucket, const PrefillChunk* p
         }
         if (pf) {
             // one task, len_q = chunk, causal int8 mask (Attention::dynamic_batch_forward with len_q > 1, attention.cpp:846-964)
+            if (l > 0) zl_decode_attention_same_mask();
             RCHECK(zl_decode_attention(m->q, m->d_lens + pf->task, L.k_addrs + pf->task, L.v_addrs + pf->task, m->d_mask,
                                        scale, pf->pos0 + pf->n, m->ao, 1, pf->n, m->hq, m->hkv, d, 1, m->attn_ws,
                                        m->attn_ws_bytes, dt, pdl, st));
@@ -1374,16 +1392,16 @@ extern "C" int zl_llama_prefill(zl_llama_t* m, int task, const int32_t* tokens_h
         zl_set_last_error(__FILE__, __LINE__, "prompt does not fit the KV buffers (max_seq)");
         return ZL_ERR_STATE;
     }
-    int32_t* h_tok = m->h_stage + 4 * m->cfg.max_batch + 4;   // pinned staging for one chunk of token ids
+    // All tokens go over at once, so that the chunks follow each other without the host waiting for one of them (a gap of 25 - 50 us each)
+    int32_t* h_tok = m->h_stage + 4 * m->cfg.max_batch + 4;   // pinned
+    for (int i = 0; i < n; ++i) {
+        ZL_CHECK_ARG(tokens_host[i] >= 0 && tokens_host[i] < m->cfg.vocab_size);
+        h_tok[i] = tokens_host[i];
+    }
+    ZL_CHECK_CUDA(cudaMemcpyAsync(m->d_pf_tokens, h_tok, (size_t)n * 4, cudaMemcpyHostToDevice, m->stream));
     for (int c0 = 0; c0 < n; c0 += chunk) {
         const int cn = (n - c0) < chunk ? (n - c0) : chunk;
-        if (c0 > 0) ZL_SYNC(m->stream);   // staging buffer reuse
-        for (int i = 0; i < cn; ++i) {
-            ZL_CHECK_ARG(tokens_host[c0 + i] >= 0 && tokens_host[c0 + i] < m->cfg.vocab_size);
-            h_tok[i] = tokens_host[c0 + i];
-        }
-        ZL_CHECK_CUDA(cudaMemcpyAsync(m->d_pf_tokens, h_tok, cn * 4, cudaMemcpyHostToDevice, m->stream));
-        PrefillChunk pc{task, pos0 + c0, cn, c0 + cn == n};
+        PrefillChunk pc{task, pos0 + c0, cn, c0 + cn == n, c0};
         RCHECK(enqueue_step(m, 1, 0, &pc));
     }
     ZL_CHECK_CUDA(cudaMemcpyAsync(m->h_stage + 3 * m->cfg.max_batch, m->d_next, 4, cudaMemcpyDeviceToHost, m->stream));
