@@ -409,8 +409,9 @@ static T2Pick t2_pick(int M, int row_tiles, int G) {
 }
 
 // Whether M tokens are this kernel's.  Beyond 256 w4a16_tc.cu would need several passes; below, tiles on few pairs stand against its ranges
-// over all SMs and their exchange: 10 us + 4.2 ns per token and million weights.  Measured, N x K, there / here, us: 4096 x 14336 at M = 64 / 96 /
-// 128 / 256 24.7 / 36 / 39 / 55 and 24.2 / 24.7 / 26.7 / 33; 6144 x 4096 at M = 96 / 256 22.3 / 24.7 and 18.4 / 22.6; 28672 x 4096 at M = 32 / 64
+// over all SMs and their exchange: 10 us + 4.2 ns per token and million weights, a quarter more where it works on 128 or 256 tokens for fewer.
+// Measured, N x K, there / here, us: 4096 x 14336 at M = 64 / 76 / 128 / 256 24.7 / 30.9 / 39 / 55 and 24.2 / 24.7 / 26.7 / 33; 6144 x 4096 at M = 76
+// 25.0 and 18.4; 4096 x 4096 18.9 and 16.5; 28672 x 4096 at M = 32 / 64
 // 32.9 / 36.7 and 30.4 / 31.2, of which a pair of feed-forward calls at M = 32 keeps nothing (54.0 and 54.9); 512 x 14336 at M = 32 13 and 23.
 // Where its ranges are down to eight groups every tile is cut, and what is exchanged grows with M (2304 x 1152 at M = 40 / 256: 18 / 51 there,
 // 12 / 12.4 here; 1664 x 2176: 17 / 50 and 12.4 / 14.5; 3328 x 5248 at M = 128: 31 and 17.5).
@@ -418,7 +419,7 @@ bool w4_tc2_route(int M, int N, int K) {
     if (M <= 16 || N % kTcRows || K % kW4GroupK) return false;
     if (M > 256) return true;
     const int G = K / kW4GroupK;
-    const double there = 10.0 + 4.2e-9 * M * (double)N * K;
+    const double there = (10.0 + 4.2e-9 * M * (double)N * K) * (M > 64 && N >= 4096 ? 1.25 : 1.0);
     const bool cut = M > 32 && (long long)(N / kTcRows) * G < 8 * device_sm_count();
     return t2_pick(M, cdiv(N, kTc2Rows), G).us < there + (!cut ? 0.0 : K < 4096 ? 0.1 * M : N >= 1024 ? 0.015 * M : 0.0);
 }
