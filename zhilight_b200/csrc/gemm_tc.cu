@@ -56,6 +56,7 @@ struct alignas(64) GemmTcP {
     const void* sw;             // 8-bit: scales of the rows of w, or one
     int sw_mode;                // 0: per row in y's type, 1 / 2: per row fp32, 3: one fp32
     unsigned* err;              // wait_words()[kWaitGemmTc]
+    int behind;                 // dependents may start once everything before this kernel has ended
 };
 
 struct GtTile {
@@ -208,8 +209,9 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
         mbar_fence_init();
     }
     if (warp == 2) tc2_alloc(s_tmem);
-    pdl_trigger();
+    if (!p.behind) pdl_trigger();
     if (KIND == kGt16) pdl_wait();   // 8-bit: below; the weights do not wait for the rows' quantisation (8192 x 8192, 24 rows: 1 us)
+    if (p.behind) pdl_trigger();
     if (GROUPED && warp == 3) {   // tiles before each group: a running sum over the groups' sizes
         int base = 0;
         for (int g0 = 0; g0 < p.groups; g0 += 32) {
@@ -624,6 +626,12 @@ cudaError_t launch_gemm_tc(const GemmP& p, int batch, int in_dtype, int out_dtyp
     q.epi = epilogue;
     const int pairs = gt_plan(q, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, batch, out_dtype == ZL_F32 ? 4 : 2);
     if (pairs <= 0) return cudaErrorNotSupported;
+    // The 16-bit kernel touches nothing of its predecessor's before it has waited for it, so its allocation, barriers and cluster launch run under the
+    // predecessor's end whatever the caller's chain allows.  A caller that did not ask for that may have a dependent which reads what was written
+    // before this kernel without waiting: it starts behind the wait.  In a row of calls: bf16 8192 x 2048, 777 rows 32.8 -> 30.6 us; 1280 -> 8288,
+    // 164 rows 12.4 -> 10.0; both products of 16 experts 129 -> 123.
+    q.behind = !pdl;
+    pdl = true;
     if (bf16) return out_dtype == ZL_F32 ? launch_gt16<__nv_bfloat16, float>(q, grouped, pairs, pdl, stream)
                                          : launch_gt16<__nv_bfloat16, __nv_bfloat16>(q, grouped, pairs, pdl, stream);
     return out_dtype == ZL_F32 ? launch_gt16<__half, float>(q, grouped, pairs, pdl, stream) : launch_gt16<__half, __half>(q, grouped, pairs, pdl, stream);

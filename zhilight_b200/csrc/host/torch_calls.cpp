@@ -186,7 +186,8 @@ PyObject* decode_attention(PyObject*, PyObject* const* a, Py_ssize_t na) {
             PyErr_Clear();
             throw NotPlain{};
         }
-        const int max_len = to_int(a[6]), kv_heads = to_int(a[7]), bshd = truth(a[8]), pdl = truth(a[9]), dt = dtype_of(q);
+        const int max_len = to_int(a[6]), kv_heads = to_int(a[7]), bshd = truth(a[8]), dt = dtype_of(q);
+        truth(a[9]);
         const int b = (int)q.size(0), len_q = (int)q.size(1), heads = (int)q.size(2), dim = (int)q.size(3);
         // every tensor whose memory the launches below use; what torch cannot resize belongs to another owner and has to be waited for
         std::vector<const at::Tensor*> used{&q, &lens};
@@ -217,9 +218,10 @@ PyObject* decode_attention(PyObject*, PyObject* const* a, Py_ssize_t na) {
         const c10::cuda::CUDAStream cs = c10::cuda::getCurrentCUDAStream();
         const int rc = unlocked([&] {
             const int e = zl.write_pointers(table, at_.data(), 2 * b, (zl_stream_t)cs.stream());
+            // the table is written behind everything earlier: the attention may start under that launch's end, whatever the caller's chain allows
             return e ? e
                      : zl.attn(q.data_ptr(), static_cast<const int32_t*>(lens.data_ptr()), table, table + b, static_cast<const int8_t*>(mask), (float)scale,
-                               max_len, out.data_ptr(), b, len_q, heads, kv_heads, dim, bshd, ws, ws_bytes, dt, pdl, (zl_stream_t)cs.stream());
+                               max_len, out.data_ptr(), b, len_q, heads, kv_heads, dim, bshd, ws, ws_bytes, dt, 1, (zl_stream_t)cs.stream());
         });
         if (rc == 0)
             for (const c10::Storage& s : storages) c10::cuda::CUDACachingAllocator::recordStream(s.data_ptr(), cs);

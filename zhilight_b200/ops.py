@@ -420,7 +420,7 @@ def decode_attention(q, buf_lens, k_bufs, v_bufs, mask, scale, max_len_buf, num_
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
     (ka, va), _table = _ptr_tables(q.device, k_bufs, v_bufs)
     _lib.call("zl_decode_attention", _p(q), _p(buf_lens), ka, va, _p(mask), float(scale), max_len_buf,
-              _p(out), b, len_q, hq, num_kv_heads, d, int(bshd), _p(ws), ws_bytes, _dt(q), int(pdl), _stream())
+              _p(out), b, len_q, hq, num_kv_heads, d, int(bshd), _p(ws), ws_bytes, _dt(q), 1, _stream())   # behind the table's launch
     _in_use(q, buf_lens, mask, *k_bufs, *v_bufs)
     return out
 
