@@ -237,3 +237,44 @@ def test_row_limit_of_the_few_rows_kernel(cuda, limit, want):
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", _FEW_ROWS, root], env=env, capture_output=True, text=True, timeout=300)
     assert r.stdout.split() == [want], r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_starts_under_its_predecessors_end(lib, cuda, captured):
+    """Inputs that the launch before is still writing, on this stream and behind another one's event; and a dependent that reads its weights ahead of its
+    own wait: they were written before this kernel, whose early start must not let the dependent overtake the writer."""
+    from zhilight_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(0)
+    m, n, k = 100, 512, 1024
+    src = [torch.randn(*s, generator=g, device=cuda).bfloat16() for s in ((m, k), (n, k), (256, n))]
+    x, w, w2 = (torch.zeros_like(t) for t in src)
+    ref = src[0].float() @ src[1].float().T
+    side = torch.cuda.Stream()
+
+    def step():
+        torch.cuda._sleep(200_000)
+        for d, s in zip((w2, x), (src[2], src[0])):
+            d.copy_(s)
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(200_000)
+            w.copy_(src[1])
+        torch.cuda.current_stream().wait_stream(side)
+        y = ops.dense_gemm_skinny(x, w)
+        return y, ops.dense_gemm_skinny(y[:16], w2, pdl=True)
+    ops.dense_gemm_skinny(src[0], src[1])                             # prepared outside of the capture
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            y, z = step()
+    for _ in range(3):
+        for t in (x, w, w2):
+            t.zero_()
+        if captured:
+            graph.replay()
+        else:
+            y, z = step()
+        torch.cuda.synchronize()
+        assert ((y.float() - ref).norm() / ref.norm()).item() <= 4e-3    # bf16's rounding is at most 2^-9 of a value, fp32 sums are far below
+        want = y[:16].float() @ src[2].float().T
+        assert ((z.float() - want).norm() / want.norm()).item() <= 4e-3
