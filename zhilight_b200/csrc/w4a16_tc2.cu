@@ -54,6 +54,25 @@ struct T2Cfg {
     static_assert(t2_slots(256) * 64 + 256 <= 512 && t2_slots(128) * 64 + 128 <= 512, "TMEM columns");
     static_assert(kBytes <= 232448, "shared memory");
 };
+// A weight slot is held while its group converts and is then a round trip to L2 from being full again: more than two per group
+__host__ __device__ constexpr int t2_raw_slots(int ntok) {
+    const int fit = (T2Cfg::kRing - t2_slots(ntok) * t2_x_bytes(ntok)) / (T2Cfg::kNib + T2Cfg::kTr);
+    return fit < T2Cfg::kMaxRaw ? fit : T2Cfg::kMaxRaw;
+}
+// A wait by parity takes the landing (or the release) before the last one for the one it is meant for, so whoever waits or looks has to know that the
+// last but one has been.  The four groups and the two issuing warps run free of each other; what orders them is that group s gets its slot of A once
+// group s - slots has been multiplied, and with it all before.
+//   A's slot, looked at ahead of group s:   s - 4 had its slot, so s - 4 - slots is multiplied, which has to cover s - 2 slots
+//   weights of s + 4, looked at behind the wait for A's slot of s: s - slots is multiplied, which has to cover s + 4 - raw (ahead of that wait only s - 4 -
+//                                           slots is: 256 tokens, four slots and 11 weight slots, are one short of it)
+//   release of weights s + 2, looked at while s is loaded: s - raw is released, so s - raw - slots is multiplied, which has to cover s + 2 - 2 raw
+__host__ __device__ constexpr bool t2_rings_hold(int ntok) {
+    return t2_slots(ntok) >= T2Cfg::kGroups && t2_raw_slots(ntok) >= t2_slots(ntok) + T2Cfg::kGroups &&
+           t2_raw_slots(ntok) >= t2_slots(ntok) + T2Cfg::kRawWarps;
+}
+static_assert(t2_rings_hold(32) && t2_rings_hold(64) && t2_rings_hold(96) && t2_rings_hold(128) && t2_rings_hold(160) && t2_rings_hold(192) &&
+                  t2_rings_hold(224) && t2_rings_hold(256),
+              "a wait by parity could take an earlier phase for its own");
 
 struct T2Tile {
     int n0, t0, ntok;   // first row of w of the pair, first token, tokens (a multiple of 32)
@@ -87,8 +106,7 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
     const int stages_all = (p.K / kW4GroupK + SUB - 1) / SUB, g_first = stages_all * part / splits * SUB;
     const int G = stages_all * (part + 1) / splits * SUB - g_first;
     const int slots = t2_slots(p.ntok), nacc = t2_accs(p.ntok), xstage = t2_x_bytes(p.ntok), acol0 = 512 - slots * 64;
-    // a weight slot is held while its group converts and is then a round trip to L2 from being full again: more than two per group
-    const int rslots = min(C::kMaxRaw, (C::kRing - slots * xstage) / (C::kNib + C::kTr));
+    const int rslots = t2_raw_slots(p.ntok);
     uint8_t* const nibs = smem + slots * xstage;
     uint8_t* const trs = nibs + rslots * C::kNib;
 
@@ -239,7 +257,7 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
                 rs -= rslots;
                 rph ^= 1u;
             }
-            const bool next = mbar_test(&raw_full[rs], rph);
+            bool next = false;
             const __half2 sc2 = *reinterpret_cast<const __half2*>(tr + (tt * 8 + g8) * 4);
             const int zz = tr[64 + tt * 8 + g8];
             const __half2 cz = __float2half2_rn(hi ? (float)(64 + (zz >> 4)) : (float)(1024 + (zz & 0xF)));
@@ -276,6 +294,7 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
                 if (ks == 0) {
                     if (!__all_sync(0xffffffffu, free) && !(ok = tc2_wait(&ax_empty[as / SUB], ph ^ 1u, s_abort, p.err, 0x3700 + as))) break;
                     tc_fence_after();
+                    next = mbar_test(&raw_full[rs], rph);   // not before this wait: see t2_rings_hold
                 }
                 tc_st16(taddr + (uint32_t)(ks * 32), r[0]);
                 tc_st16(taddr + (uint32_t)(ks * 32 + 16), r[1]);
@@ -448,6 +467,13 @@ cudaError_t launch_w4_tc2(const W4Params& p, bool pdl, cudaStream_t stream) {
 }
 
 }  // namespace zl
+
+extern "C" int zl_w4_pairs_rings(int ntok, int* slots, int* raw_slots) {
+    ZL_CHECK_ARG(ntok >= 32 && ntok <= 256 && ntok % 32 == 0 && slots && raw_slots);
+    *slots = zl::t2_slots(ntok);
+    *raw_slots = zl::t2_raw_slots(ntok);
+    return ZL_OK;
+}
 
 extern "C" int zl_w4_pairs_splits(int M, int N, int K) {
     return zl_w4_pairs_route(M, N, K) ? zl::t2_pick(M, zl::cdiv(N, zl::kTc2Rows), K / zl::kW4GroupK).splits : 0;
