@@ -375,6 +375,10 @@ extern "C" size_t zl_decode_attention_workspace_bytes(int B, int len_q, int num_
     return (size_t)B * len_q * num_heads * splits * (dim_head + 2) * sizeof(float);
 }
 
+extern "C" int zl_prompt_attention_smem_bytes(int dim_head) {
+    return dim_head == 64 ? PaCfg<64>::kBytes : dim_head == 128 ? PaCfg<128>::kBytes : 0;
+}
+
 // Workspace of the prompt kernel ahead of the splits' partial results: the mask's bits, then the last visible keys.
 static size_t prompt_head_bytes(int B, int len_q, int max_len_buf, const int8_t* mask) {
     const size_t q_rows = (size_t)B * len_q;

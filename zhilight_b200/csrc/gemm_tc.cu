@@ -38,7 +38,7 @@ constexpr int kGtMiscOff = kGtBarOff + (3 * kGtMaxStages + 4) * 8;
 constexpr int kGtMaxGroups = 1024;
 constexpr int kGtCumOff = kGtMiscOff + 16;                       // grouped: tiles before each group
 constexpr int kGtBytes = kGtCumOff + (kGtMaxGroups + 1) * 4 + 1024;   // + slack for the manual 1024-byte alignment
-static_assert(kGtBytes <= 232448, "shared memory");
+static_assert(kGtBytes <= 232448 && tmem_alone(kGtBytes), "shared memory");
 enum { kGt16 = 0, kGtInt8 = 1, kGtFp8 = 2 };
 
 struct alignas(64) GemmTcP {

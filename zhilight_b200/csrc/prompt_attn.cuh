@@ -163,7 +163,9 @@ struct PaCfg {
     static constexpr int kRow = D + 4;                           // merge: floats per row, 16-byte chunks of eight lanes on eight bank groups
     static constexpr int kMl = kPaRows * kRow * 4;               // {maximum, sum} of a row behind the accumulators
     static constexpr int kMerge = kMl + kPaRows * 8;
-    static constexpr int kBytes = (kStaged > kMerge ? kStaged : kMerge) + 1024;   // + slack for the manual 1024-byte alignment
+    static constexpr int kUsed = (kStaged > kMerge ? kStaged : kMerge) + 1024;    // + slack for the manual 1024-byte alignment
+    static constexpr int kBytes = kHalfTmemSmem;                 // more than it uses, for the sake of tensor memory
+    static_assert(kUsed <= kBytes, "shared memory");
     static constexpr int kS = 128;                               // TMEM columns: O 0 .. D - 1, S / P 128 .. 255 (two buffers of 64)
 };
 

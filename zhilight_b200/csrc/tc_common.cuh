@@ -9,6 +9,15 @@ namespace zl {
 
 constexpr int kTcRows = 128;   // rows per tile = UMMA M = TMEM lanes
 
+// Tensor memory is given out by an instruction that waits, without a bound, until columns are free.  A CTA that waits there can be one that its
+// cluster, or the CTA with the other pieces of its tile, waits for in turn, so an SM must never take more CTAs than its 512 columns serve.  Shared
+// memory sees to that, whatever registers the compiler gives a kernel: one that takes half of the columns asks for so much that two of it fit, but
+// neither a third nor one that takes them all.
+constexpr int kSmSmem = 228 * 1024, kCtaSmem = 1024;   // of an SM; what the system takes of it for a CTA
+constexpr int kHalfTmemSmem = 112 * 1024;
+static_assert(2 * (kHalfTmemSmem + 1024 + kCtaSmem) <= kSmSmem && 3 * kHalfTmemSmem > kSmSmem, "two of them, with up to 1 KB of static shared memory each");
+__host__ __device__ constexpr bool tmem_alone(int smem) { return 2 * smem > kSmSmem && smem + kHalfTmemSmem + 2 * kCtaSmem > kSmSmem; }
+
 // ---- PTX wrappers -------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");

@@ -87,7 +87,7 @@ struct TsCfg {
     static constexpr int kMiscOff = kBarOff + kNumBars * 8;
     static constexpr int kBytes = kMiscOff + 16 + 1024;                 // + slack for the manual 1024-byte alignment
     static_assert(kACol0 + AS * KG * 64 <= 512, "TMEM columns");
-    static_assert(kBytes <= 232448, "shared memory");
+    static_assert(kBytes <= 232448 && tmem_alone(kBytes), "shared memory");
 };
 
 // ---- stream-k schedule ------------------------------------------------------------------------------------------------

@@ -52,7 +52,7 @@ struct T2Cfg {
     static constexpr int kMiscOff = kBarOff + (2 * kMaxRaw + 2 * kMaxSlots + 4) * 8;
     static constexpr int kBytes = kMiscOff + 16 + 1024;                // + slack for the manual 1024-byte alignment
     static_assert(t2_slots(256) * 64 + 256 <= 512 && t2_slots(128) * 64 + 128 <= 512, "TMEM columns");
-    static_assert(kBytes <= 232448, "shared memory");
+    static_assert(kBytes <= 232448 && tmem_alone(kBytes), "shared memory");
 };
 // A weight slot is held while its group converts and is then a round trip to L2 from being full again: more than two per group
 __host__ __device__ constexpr int t2_raw_slots(int ntok) {
