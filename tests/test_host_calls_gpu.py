@@ -113,3 +113,29 @@ def test_memory_of_another_stream_outlives_its_tensors(lib, cuda):
     assert not at & {t.data_ptr() for t in new}
     torch.cuda.synchronize()
     assert torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("call", ["w4", "dense", "int8", "attention"])
+@pytest.mark.parametrize("native", [True, False])
+def test_out_of_memory_is_torchs_own_error(lib, cuda, monkeypatch, call, native):
+    """A program that frees memory and tries again knows it by its type.  No kernel is launched: the result cannot be allocated."""
+    from zhilight_b200 import _lib, ops
+    assert _lib.host is not None
+    m, n, k = 2048, 32768, 128
+    x, w = torch.zeros(m, k, device=cuda).half(), torch.zeros(n, k, device=cuda, dtype=torch.int8)
+    packed = torch.zeros(int(lib.zl_w4_packed_bytes(n, k, 128)), dtype=torch.uint8, device=cuda)
+    wh, one = torch.zeros(n, k, device=cuda).half(), torch.ones(n, device=cuda)
+    q, kv = torch.zeros(1, 4096, 128, 128, device=cuda).half(), torch.zeros(4096, 1, 128, device=cuda).half()
+    lens = torch.tensor([4096], dtype=torch.int32, device=cuda)
+    run = {"w4": lambda: ops.w4a16_gemm_fused(x, packed, n, k, variant=1), "dense": lambda: ops.dense_gemm_skinny(x, wh),
+           "int8": lambda: ops.int8_linear(x, w, one), "attention": lambda: ops.decode_attention(q, lens, [kv], [kv], None, 0.09, 4096, 1)}[call]
+    if not native:
+        monkeypatch.setattr(_lib, "host", None)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    torch.cuda.set_per_process_memory_fraction(1e-6)
+    try:
+        with pytest.raises(torch.OutOfMemoryError):
+            run()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)

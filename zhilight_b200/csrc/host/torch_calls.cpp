@@ -12,9 +12,9 @@
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
-#include <exception>
 #include <vector>
 
 #include "../../../include/zhilight_b200.h"
@@ -89,14 +89,13 @@ PyObject* result(int rc, const at::Tensor& out) { return rc ? PyLong_FromLong(rc
 
 template <typename F>
 PyObject* guarded(F&& f) {
+    HANDLE_TH_ERRORS   // what torch throws here becomes what its own calls raise, torch.OutOfMemoryError for one
     try {
         return f();
     } catch (const NotPlain&) {
-        Py_RETURN_NONE;
-    } catch (const std::exception& e) {
-        PyErr_SetString(PyExc_RuntimeError, e.what());
-        return nullptr;
     }
+    Py_RETURN_NONE;
+    END_HANDLE_TH_ERRORS
 }
 
 // x, packed, n, k, group_size, bias, residual, epilogue, pdl, out, variant
