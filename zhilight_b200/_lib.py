@@ -116,7 +116,10 @@ def parse_header(path=HEADER):
 
 _lib = None
 _protos = None
-host = None   # once loaded: the native module of the calls that are made per layer and token (csrc/host/torch_calls.cpp)
+# The native module of the calls that are made per layer and token (csrc/host/torch_calls.cpp), once the library is loaded and ops.py, the only one to
+# use it, is imported.  It needs torch, which nothing else here does.  None: ops.py's general path serves every call.
+host = None
+_host_wanted = False
 
 
 _path = None
@@ -133,7 +136,7 @@ def use(path):
 
 def load():
     """Load the library (building nothing).  Raises if the .so is absent."""
-    global _lib, _protos, host
+    global _lib, _protos
     if _lib is not None:
         return _lib
     path = _path or LIB_PATH
@@ -150,10 +153,28 @@ def load():
         fn = getattr(lib, name)          # AttributeError if the symbol is missing
         fn.restype = ctypes.c_char_p if ret.replace("const", "").strip() == "char*" else _ctype(ret)
         fn.argtypes = [_ctype(t) for t, _ in params]
-    from . import _host              # built with the library; ImportError if it is missing
-    _host.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in _protos})
-    _lib, host = lib, _host
+    _lib = lib
+    if _host_wanted:
+        _bind_host()
     return lib
+
+
+def _bind_host():
+    global host
+    try:
+        from . import _host
+    except ImportError:              # not built here, or against another torch
+        return
+    _host.bind({name: ctypes.cast(getattr(_lib, name), ctypes.c_void_p).value for name in _protos})
+    host = _host
+
+
+def want_host():
+    """Torch is imported: the native module may be loaded with the library, or now if that is loaded already."""
+    global _host_wanted
+    _host_wanted = True
+    if _lib is not None and host is None:
+        _bind_host()
 
 
 def protos():

@@ -5,7 +5,8 @@
 `build()` makes the whole library.  `build(family=...)` serves a program that runs one model family in a checkout
 without built files: when the whole library is present and current it is returned, otherwise only the sources that
 family's step needs are compiled and linked into libzhilight_b200_<family>.so (the binding skips the entry points such
-a library does not have).  Either way the host module _host.so (csrc/host) is built beside it, against this interpreter and torch.
+a library does not have).  Either way the host module _host.so (csrc/host) is built beside it, against this interpreter and torch, where that
+can be done: the library does not need it.
 """
 import hashlib
 import os
@@ -74,28 +75,43 @@ def _digest(paths):
 
 
 def build_host(force=False):
-    """The native module behind the calls that are made once per layer and token."""
+    """The native module behind the calls that are made once per layer and token.  None where it cannot be built (no torch, no compiler, no
+    Python headers): ops.py serves every call without it.  Torch itself is only imported to build it."""
+    import importlib.metadata
+    import importlib.util
     import sysconfig
+    import warnings
 
-    import torch
+    if importlib.util.find_spec("torch") is None:
+        return None
     src = os.path.join(CSRC, "host", "torch_calls.cpp")
     header = os.path.join(HERE, "..", "include", "zhilight_b200.h")
     out = os.path.join(HERE, "_host.so")
-    tag = " ".join([_digest([src, header]), torch.__version__, sys.version])
+    tag = " ".join([_digest([src, header]), importlib.metadata.version("torch"), sys.version])
     dig_path = out + ".digest"
     if not force and os.path.exists(out) and os.path.exists(dig_path) and open(dig_path).read() == tag:
         return out
-    troot = os.path.dirname(torch.__file__)
-    cuda = os.path.dirname(os.path.dirname(_nvcc()))
-    includes = [sysconfig.get_paths()["include"], os.path.join(troot, "include"), os.path.join(troot, "include", "torch", "csrc", "api", "include"),
-                os.path.join(cuda, "include")]
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI, "-o", out, src]
-    cmd += ["-I" + i for i in includes] + ["-L" + os.path.join(troot, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode != 0:
-        raise RuntimeError("host module failed:\n" + r.stdout + r.stderr)
-    with open(dig_path, "w") as f:
-        f.write(tag)
+    part = "%s.%d" % (out, os.getpid())
+    try:
+        import torch
+        for old in (dig_path, out):      # rather none than one of other sources
+            if os.path.exists(old):
+                os.remove(old)
+        troot = os.path.dirname(torch.__file__)
+        cuda = os.path.dirname(os.path.dirname(_nvcc()))
+        includes = [sysconfig.get_paths()["include"], os.path.join(troot, "include"),
+                    os.path.join(troot, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include")]
+        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI, "-o", part, src]
+        cmd += ["-I" + i for i in includes] + ["-L" + os.path.join(troot, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(r.stdout + r.stderr)
+        os.replace(part, out)            # whole at any time, whoever else builds or loads it
+        with open(dig_path, "w") as f:
+            f.write(tag)
+    except (ImportError, OSError, RuntimeError) as e:
+        warnings.warn("the native host module was not built, every call takes ops.py's general path:\n%s" % e)
+        return None
     return out
 
 

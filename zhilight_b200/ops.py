@@ -10,6 +10,8 @@ import torch
 
 from . import _lib
 
+_lib.want_host()
+
 F16, BF16, F32 = 0, 1, 2
 EPI_NONE, EPI_SWIGLU, EPI_RESIDUAL, EPI_QKV_ROPE = 0, 1, 2, 3
 
