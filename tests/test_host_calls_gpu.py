@@ -36,29 +36,48 @@ FORMS = {"plain": lambda t: t, "strided": lambda t: torch.cat([t, t], 1)[:, :t.s
          "subclass": lambda t: t.as_subclass(_Own), "flat": lambda t: t[0], "float": lambda t: t.float(), "narrow": lambda t: t[:, :64]}
 
 
+def _linear(k, n, quant, dtype, seed):
+    from zhilight_b200 import layers
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    w = torch.randn(n, k, generator=g, device="cuda")
+    sd = {"bias": torch.randn(n, generator=g, device="cuda")}
+    if quant == 1:
+        sd.update(weight=torch.randint(-127, 128, (n, k), generator=g, device="cuda", dtype=torch.int8), weight_scale=torch.rand(n, generator=g, device="cuda") * 0.01)
+    elif quant == 7:
+        sd.update(weight=w.clamp(-4, 4).to(torch.float8_e4m3fn).view(torch.uint8), weight_scale=torch.tensor([0.1], device="cuda"))
+    elif quant == 5:
+        sd.update(qweight=torch.randint(-2 ** 31, 2 ** 31 - 1, (k // 8, n), generator=g, device="cuda", dtype=torch.int64).int(),
+                  qzeros=torch.full((k // 128, n // 8), 0x77777777, dtype=torch.int32, device="cuda"), scales=torch.rand(k // 128, n, generator=g, device="cuda").half() * 0.01)
+    else:
+        sd["weight"] = w * 0.05
+    lin = layers.Linear(k, n, "", quant, dtype)
+    lin.load_state_dict(sd)
+    return lin, g
+
+
 @pytest.mark.parametrize("form", sorted(FORMS))
 @pytest.mark.parametrize("m", [1, 40])
 def test_linears(lib, cuda, monkeypatch, form, m):
-    from zhilight_b200 import layers
-    g = torch.Generator(device="cuda").manual_seed(m)
-    k, n = 512, 384
     for quant, dtype in ((0, "bfloat"), (0, "half"), (1, "half"), (7, "bfloat"), (5, "half")):
-        w = torch.randn(n, k, generator=g, device=cuda)
-        sd = {"bias": torch.randn(n, generator=g, device=cuda)}
-        if quant == 1:
-            sd.update(weight=torch.randint(-127, 128, (n, k), generator=g, device=cuda, dtype=torch.int8), weight_scale=torch.rand(n, generator=g, device=cuda) * 0.01)
-        elif quant == 7:
-            sd.update(weight=w.clamp(-4, 4).to(torch.float8_e4m3fn).view(torch.uint8), weight_scale=torch.tensor([0.1], device=cuda))
-        elif quant == 5:
-            sd.update(qweight=torch.randint(-2 ** 31, 2 ** 31 - 1, (k // 8, n), generator=g, device=cuda, dtype=torch.int64).int(),
-                      qzeros=torch.full((k // 128, n // 8), 0x77777777, dtype=torch.int32, device=cuda), scales=torch.rand(k // 128, n, generator=g, device=cuda).half() * 0.01)
-        else:
-            sd["weight"] = w * 0.05
-        lin = layers.Linear(k, n, "", quant, dtype)
-        lin.load_state_dict(sd)
-        x = torch.randn(m, k, generator=g, device=cuda).to(lin.dtype)
+        lin, g = _linear(512, 384, quant, dtype, m)
+        x = torch.randn(m, 512, generator=g, device=cuda).to(lin.dtype)
         _same(_both(monkeypatch, lambda: lin(FORMS[form](x))))
         _same(_both(monkeypatch, lambda: lin(x[None])))
+
+
+ONE_ROW = {"odd pitch": lambda x: torch.cat([x, x[:, :13]], 1).expand(2, -1).contiguous()[:1, :x.shape[1]], "pitch of one": lambda x: x.flatten().as_strided(x.shape, (1, 1)),
+           "short pitch": lambda x: x.flatten().as_strided(x.shape, (8, 1)), "broadcast": lambda x: x.expand(1, -1).as_strided(x.shape, (0, 1))}
+
+
+@pytest.mark.parametrize("form", sorted(ONE_ROW))
+@pytest.mark.parametrize("quant,dtype", [(0, "bfloat"), (0, "half"), (1, "half"), (7, "bfloat"), (5, "half")])
+def test_one_row_of_any_pitch(lib, cuda, form, quant, dtype):
+    """A single row is contiguous whatever lies between it and a next one that is not there."""
+    lin, g = _linear(512, 384, quant, dtype, 3)
+    x = torch.randn(1, 512, generator=g, device=cuda).to(lin.dtype)
+    given = ONE_ROW[form](x)
+    assert given.stride(0) != 512 and torch.equal(given, x)
+    assert torch.equal(lin(given), lin(x))
 
 
 def test_entry_points(lib, cuda, monkeypatch):

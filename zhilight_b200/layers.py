@@ -81,7 +81,8 @@ class Linear:
             raise _lib.ZLError(-1, "Input size mismatch")
         if x.dtype != self.dtype:
             raise _lib.ZLError(-1, "Input data type mismatch")
-        x2 = (x if x.dim() == 2 else x.reshape(-1, self.dim_in)).contiguous()
+        # one row counts as contiguous whatever its pitch, which the kernels would take for their alignment: reshape gives it its own length
+        x2 = (x if x.dim() == 2 and x.stride(0) == self.dim_in else x.reshape(-1, self.dim_in)).contiguous()
         q, n, k = self.quant, self.dim_out, self.dim_in
         if q == QUANT_NONE:
             y = ops.dense_gemm_skinny(x2, self._p["weight"], self.bias)
