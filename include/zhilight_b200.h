@@ -141,11 +141,14 @@ typedef struct zl_w4_fused_args {
 int zl_w4a16_gemm_fused(const zl_w4_fused_args_t* args, zl_stream_t stream);
 /* 1 if the exact-integer kernel (variant 1, M <= 16) can run this shape: its staged activations must fit shared memory. */
 int zl_w4_int_kernel_fits(int M, int N, int K);
-/* which kernel serves (M, N, K) on the ZLW4I layout (variant 1): 3 = exact-integer mma.sync kernel (from 9 rows on only with the fused
- * RMSNorm or the exchange, else the fp16 mma.sync kernel), 4 = tcgen05 / TMEM / TMA kernels, up to 16 rows (32 of small matrices) the fp16 mma.sync kernel (any M,
- * N % 128 == 0, no fused RMSNorm prologue), 0 = neither (pack variant 0 and use the fp16 mma.sync kernel). */
+/* what (M, N, K) may ask for on the ZLW4I layout (variant 1): 3 = everything, the fused RMSNorm prologue and the exchange among it (up to 16 rows that
+ * the exact-integer kernel can stage), 4 = everything but these two (any M, N % 128 == 0), 0 = nothing (pack variant 0).  Which kernel serves a call:
+ * behind 3 the exact-integer mma.sync kernel, unless the next query names another; behind 4 what the next two queries name, else the stream-k kernel. */
 int zl_w4_int_layout_route(int M, int N, int K);
-/* whether, of the two kernels behind answer 4, the one over pairs of SMs serves the shape (1) or the stream-k kernel (0) */
+/* 1 if a call without RMSNorm prologue and exchange runs on the fp16 mma.sync kernel: 9 to 16 rows, fewer that the integer kernel has no room for, and
+ * up to 32 rows of small matrices */
+int zl_w4_few_rows_route(int M, int N, int K);
+/* 1 if (M, N, K) runs on the tcgen05 kernel over pairs of SMs */
 int zl_w4_pairs_route(int M, int N, int K);
 /* pairs of a cluster that share the K of a tile there (1: none do), 0 where that kernel does not serve the shape */
 int zl_w4_pairs_splits(int M, int N, int K);

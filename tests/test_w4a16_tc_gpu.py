@@ -1,5 +1,5 @@
 """GPU parity: the tcgen05 W4A16 kernels of the ZLW4I layout vs the CPU oracle: stream-k (k_w4a16_ts) and pairs of SMs (k_w4a16_tc2).  Which one serves
-a shape is zl_w4_pairs_route's answer; the tests named stream_k assert that it is the first.
+a shape is the answer of the route queries; the tests named stream_k, and those that force its splits, assert that it is the first.
 
 Each rounds w = (q - z) * s to fp16 once (what the reference's M > 40 dequant + cuBLASLt route does,
 q_gemm_k_major.cu:843-905, 1083-1100), multiplies fp16 x fp16 exactly and accumulates all of K in fp32 in TMEM.
@@ -35,6 +35,10 @@ def splits(lib):
     lib.zl_w4_tc_set_splits(0)
 
 
+def _stream_k(lib, m, n, k):
+    return (lib.zl_w4_int_layout_route(m, n, k), lib.zl_w4_few_rows_route(m, n, k), lib.zl_w4_pairs_route(m, n, k)) == (4, 0, 0)
+
+
 def _check_watchdog(lib):
     assert lib.zl_w4_tc_watchdog() == 0 and lib.zl_w4_tc2_watchdog() == 0
 
@@ -49,6 +53,22 @@ def test_route_selects_tcgen05(lib):
     assert lib.zl_w4_int_layout_route(8, 4096, 14336) == 4      # staged activations of the integer kernel do not fit
     assert lib.zl_w4_int_layout_route(2048, 6144, 4096) == 4
     assert lib.zl_w4_int_layout_route(32, 96, 4096) == 0        # N % 128 != 0: the fp16 mma.sync kernel (variant 0)
+
+
+def test_every_shape_has_one_kernel(lib, cuda):
+    """The queries name at most one kernel for a shape, and the fp16 mma.sync kernel where a call runs on it."""
+    for m in (1, 4, 8, 9, 16, 17, 32, 33, 64, 128, 256, 300):
+        for k, n in ((1024, 512), (2048, 9472), (2048, 9600), (4096, 4096), (4096, 6144), (8192, 4736), (8320, 384), (14336, 512), (14336, 4096), (4096, 28672)):
+            route, few, pairs = lib.zl_w4_int_layout_route(m, n, k), lib.zl_w4_few_rows_route(m, n, k), lib.zl_w4_pairs_route(m, n, k)
+            assert route in (3, 4) and few + pairs <= 1 and (lib.zl_w4_pairs_splits(m, n, k) > 0) == (pairs == 1)
+            if route == 3:
+                assert pairs == 0 and few == (m > 8)
+            elif m <= 16:
+                assert few == 1
+            elif m <= 32:
+                assert few == (k <= 8192 if n <= 4736 else k <= 2048 if n <= 9472 else False)
+            else:
+                assert few == 0 and (m <= 256 or pairs == 1)
 
 
 @pytest.mark.parametrize("m", [17, 32, 33, 64, 65, 128, 200, 256, 300])
@@ -83,7 +103,8 @@ def test_model_shapes(lib, cuda, k, n, m, sym):
 @pytest.mark.parametrize("s", [1, 2, 3, 4])
 def test_split_k_is_deterministic_and_exact_enough(lib, cuda, splits, s):
     from zhilight_b200 import ops
-    k, n, m = 2048, 256, 40
+    k, n, m = 8320, 256, 40
+    assert _stream_k(lib, m, n, k)
     w, packed = _setup(cuda, k, n, False, 8)
     x = torch.randn(m, k, generator=torch.Generator().manual_seed(2)).half().to(cuda)
     splits(s)
@@ -97,7 +118,8 @@ def test_split_k_is_deterministic_and_exact_enough(lib, cuda, splits, s):
 @pytest.mark.parametrize("m,s", [(20, 1), (40, 2)])
 def test_bias_residual_swiglu(lib, cuda, splits, m, s):
     from zhilight_b200 import ops
-    k, f = 1024, 1280
+    k, f = 8320, 1280
+    assert _stream_k(lib, m, 2 * f, k) and _stream_k(lib, m, 512, k)
     rm = ops.swiglu_row_map(f, cuda)
     w, packed = _setup(cuda, k, 2 * f, False, 7, rm)
     g = torch.Generator().manual_seed(9)
@@ -123,11 +145,12 @@ def test_bias_residual_swiglu(lib, cuda, splits, m, s):
 
 
 @pytest.mark.parametrize("d,hq,hkv,k,t,s", [(128, 4, 2, 512, 24, 0), (64, 4, 2, 256, 40, 0), (128, 8, 1, 1024, 130, 0),
-                                           (128, 32, 8, 4096, 32, 0), (128, 32, 8, 4096, 20, 3), (128, 8, 2, 2048, 32, 2)])
+                                           (128, 32, 8, 4096, 32, 0), (128, 32, 8, 4096, 20, 3), (128, 32, 8, 4096, 32, 2)])
 def test_qkv_rope_epilogue(lib, cuda, splits, d, hq, hkv, k, t, s):
     """fused qkv split + RoPE + KV append vs the stand-alone rope/append operator on the plain GEMM output"""
     from zhilight_b200 import ops
     n = (hq + 2 * hkv) * d
+    assert s == 0 or _stream_k(lib, t, n, k)
     rm = ops.qkv_rope_row_map(hq + 2 * hkv, d, cuda)
     _, packed = _setup(cuda, k, n, False, 14, rm)
     _, packed_plain = _setup(cuda, k, n, False, 14)
@@ -170,11 +193,11 @@ def test_strided_activations_and_fused_norm_is_rejected(lib, cuda):
 
 
 @pytest.mark.parametrize("m", [17, 32, 33, 64, 65, 128, 129, 200, 256])
-@pytest.mark.parametrize("k,n", [(8192, 384), (14336, 512)])
+@pytest.mark.parametrize("k,n", [(8320, 384), (14336, 512)])
 def test_stream_k_token_counts(lib, cuda, m, k, n):
     """every NTOK instantiation (32 / 64 / 128 / 256), ragged last 16-token chunk; every tile is cut"""
     from zhilight_b200 import ops
-    assert lib.zl_w4_int_layout_route(m, n, k) == 4 and lib.zl_w4_pairs_route(m, n, k) == 0
+    assert _stream_k(lib, m, n, k)
     w, packed = _setup(cuda, k, n, False, 5)
     x = torch.randn(m, k, generator=torch.Generator().manual_seed(m)).half()
     y = ops.w4a16_gemm_fused(x.to(cuda), packed, n, k, variant=1)
@@ -186,12 +209,12 @@ def test_stream_k_token_counts(lib, cuda, m, k, n):
         assert rel_l2(y[i], ref[i]) <= 2 * TOL, i
 
 
-@pytest.mark.parametrize("m,k,f,n", [(20, 4096, 1280, 640), (40, 4096, 1344, 640), (100, 4096, 1280, 512), (33, 4096, 14336, 28672)])
+@pytest.mark.parametrize("m,k,f,n", [(20, 8320, 1280, 640), (40, 4096, 1344, 640), (100, 4096, 1280, 512), (33, 4096, 14336, 28672)])
 def test_stream_k_bias_residual_swiglu(lib, cuda, m, k, f, n):
     """Epilogues behind the exchange of partial tiles, and (the last shape, more tiles than blocks) of whole tiles with the residual
     fetched ahead; the residual's stores of two columns and, from an odd address, of one."""
     from zhilight_b200 import ops
-    assert [lib.zl_w4_pairs_route(m, i, k) for i in (2 * f, n)] == [0, 0]
+    assert _stream_k(lib, m, 2 * f, k) and _stream_k(lib, m, n, k)
     g = torch.Generator().manual_seed(9)
     x = torch.randn(m, k, generator=g).half()
     w, packed = _setup(cuda, k, 2 * f, False, 7, ops.swiglu_row_map(f, cuda))
@@ -220,16 +243,16 @@ def test_stream_k_bias_residual_swiglu(lib, cuda, m, k, f, n):
 def test_stream_k_qkv_rope_epilogue(lib, cuda, t):
     from zhilight_b200 import ops
     hq, hkv, d, k = 32, 8, 128, 4096
-    assert lib.zl_w4_pairs_route(t, (hq + 2 * hkv) * d, k) == 0
+    assert _stream_k(lib, t, (hq + 2 * hkv) * d, k)
     test_qkv_rope_epilogue(lib, cuda, lib.zl_w4_tc_set_splits, d, hq, hkv, k, t, 0)
 
 
-@pytest.mark.parametrize("m,k,n", [(4, 14336, 512), (32, 4096, 6144), (100, 8192, 384), (200, 8192, 384)])
+@pytest.mark.parametrize("m,k,n", [(20, 14336, 512), (32, 4096, 6144), (100, 8192, 384), (200, 8192, 384)])
 def test_stream_k_starts_ahead_of_its_predecessor(lib, cuda, m, k, n):
     """Weights are fetched and converted while the predecessor still runs; the result is that of a launch behind it."""
     from tests.test_w4a16_tc2_gpu import behind_slow_predecessors
     from zhilight_b200 import ops
-    assert lib.zl_w4_int_layout_route(m, n, k) == 4 and lib.zl_w4_pairs_route(m, n, k) == 0
+    assert _stream_k(lib, m, n, k)
     _, packed = _setup(cuda, k, n, False, 5)
     x = torch.randn(m, k, generator=torch.Generator().manual_seed(m)).half().to(cuda)
     want = ops.w4a16_gemm_fused(x, packed, n, k, variant=1)

@@ -2,8 +2,10 @@
 //
 // Stands in for nn::gptq::gptq_gemm_k_major's router (reference src/nn/quant/gptq/q_gemm_k_major.cu:957-1116:
 // M <= 40 GEMV, else dequant + cuBLASLt) and for GPTQMarlin::forward (src/nn/linear/linear.cpp:1247-1451):
-//   M <= 16 and the staged activations fit shared memory -> k_w4a16_v3  (exact-integer mma.sync kernel, ZLW4I layout)
-//   M <= 16 otherwise, N % 128 == 0, and M <= 32 of small matrices -> k_w4a16_v2 (fp16 mma.sync kernel, on the ZLW4I layout)
+//   M <= 8 (16 with the fused RMSNorm or the exchange) and the staged activations fit shared memory
+//                                                        -> k_w4a16_v3  (exact-integer mma.sync kernel, ZLW4I layout)
+//   M <= 16 otherwise, and M <= 32 of small matrices with N % 128 == 0 (few_rows)
+//                                                        -> k_w4a16_v2  (fp16 mma.sync kernel, on the ZLW4I layout)
 //   otherwise, N % 128 == 0                              -> k_w4a16_tc2 (tcgen05 over pairs of SMs, ZLW4I layout) where w4_tc2_route has it
 //                                                           faster, always above 256 rows; else
 //                                                           k_w4a16_ts  (tcgen05 kernel, stream-k, A operand in TMEM, ZLW4I layout)
@@ -41,6 +43,20 @@ static int int_layout_route(int M, int N, int K) {
     return 0;
 }
 
+// Up to 16 rows that the integer kernel has no room for, and 9 to 16 rows that are its to choose (not the norm's or the exchange's): the fp16
+// mma.sync kernel.  Against the tcgen05 kernel, us: 4096 x 14336 17.6 -> 10.7 (4 rows), 18.8 -> 13.5 (16); 28672 x 4096 26.1 -> 19.2 (8),
+// 26.3 -> 24.4 (16); 8192 x 3584 12.8 -> 9.0.  Against the integer kernel: 16384 x 2048, 12 rows 13.8 -> 9.3; up to 8 rows that one is the
+// faster (28672 x 4096, 5 rows: 16.8 against 19.2).
+// 17 to 32 rows of small matrices, whose time in the tcgen05 kernels is the 9 us that one launch of them takes: one wave of 32-row super-tiles up
+// to K = 8192, two up to 2048.  Here against there, us, N x K, 17 / 32 rows: 2304 x 1152 6.2 / 6.3 against 14.5 / 15.1; 4096 x 4096 10.3 / 10.4
+// against 14.5; 4096 x 8192 16.1 / 16.5 against 18.7 / 19.7; 8192 x 2048 12.1 / 12.4 against 13.5.  Not 4096 x 14336 24.6 / 25.0 against 24.7 / 26.3;
+// 6144 x 4096 16.5 / 18.3 against 16.5; 14336 x 1024 12.4 / 14.5 against 12.1.
+static bool few_rows(int M, int N, int K, int route, bool norm_or_exchange) {
+    const int super_tiles = N / 32, sms = device_sm_count();
+    const bool small = M <= 32 && route == 4 && K <= (super_tiles <= sms ? 8192 : super_tiles <= 2 * sms ? 2048 : 0);
+    return small || (M <= 16 && (route == 4 || (route == 3 && M > 8 && !norm_or_exchange)));
+}
+
 namespace zl {
 __global__ void k_qkv_rope_row_map(int32_t* map, int n_rows, int d) {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -74,8 +90,12 @@ extern "C" int zl_w4_int_layout_route(int M, int N, int K) {
     return int_layout_route(M, N, K);
 }
 
+extern "C" int zl_w4_few_rows_route(int M, int N, int K) {
+    return few_rows(M, N, K, zl_w4_int_layout_route(M, N, K), false) ? 1 : 0;
+}
+
 extern "C" int zl_w4_pairs_route(int M, int N, int K) {
-    return zl_w4_int_layout_route(M, N, K) == 4 && w4_tc2_route(M, N, K) ? 1 : 0;
+    return zl_w4_int_layout_route(M, N, K) == 4 && !zl_w4_few_rows_route(M, N, K) && w4_tc2_route(M, N, K) ? 1 : 0;
 }
 
 extern "C" int zl_qkv_rope_row_map(int32_t* row_map, int n_heads_total, int dim_head, zl_stream_t stream) {
@@ -146,17 +166,7 @@ extern "C" int zl_w4a16_gemm_fused(const zl_w4_fused_args_t* a, zl_stream_t stre
     const int route = a->variant == kW4VariantInt ? int_layout_route(a->M, a->N, a->K) : 2;
     ZL_CHECK_SUPPORTED(route != 0 && "ZLW4I layout: M > 16 (or staged activations too large) and N % 128 != 0: use variant 0");
     ZL_CHECK_SUPPORTED(!(route == 4 && a->ln_weight) && "the tcgen05 kernel has no fused RMSNorm prologue: run zl_rmsnorm first");
-    // Up to 16 rows that the integer kernel has no room for, and 9 to 16 rows that are its to choose (not the norm's or the exchange's): the fp16
-    // mma.sync kernel.  Against the tcgen05 kernel, us: 4096 x 14336 17.6 -> 10.7 (4 rows), 18.8 -> 13.5 (16); 28672 x 4096 26.1 -> 19.2 (8),
-    // 26.3 -> 24.4 (16); 8192 x 3584 12.8 -> 9.0.  Against the integer kernel: 16384 x 2048, 12 rows 13.8 -> 9.3; up to 8 rows that one is the
-    // faster (28672 x 4096, 5 rows: 16.8 against 19.2).
-    // 17 to 32 rows of small matrices, whose time in the tcgen05 kernels is the 9 us that one launch of them takes: one wave of 32-row super-tiles up
-    // to K = 8192, two up to 2048.  Here against there, us, N x K, 17 / 32 rows: 2304 x 1152 6.2 / 6.3 against 14.5 / 15.1; 4096 x 4096 10.3 / 10.4
-    // against 14.5; 4096 x 8192 16.1 / 16.5 against 18.7 / 19.7; 8192 x 2048 12.1 / 12.4 against 13.5.  Not 4096 x 14336 24.6 / 25.0 against 24.7 / 26.3;
-    // 6144 x 4096 16.5 / 18.3 against 16.5; 14336 x 1024 12.4 / 14.5 against 12.1.
-    const int super_tiles = a->N / 32, sms = device_sm_count();
-    const bool small = a->M <= 32 && route == 4 && a->K <= (super_tiles <= sms ? 8192 : super_tiles <= 2 * sms ? 2048 : 0);
-    const bool few = small || (a->M <= 16 && (route == 4 || (route == 3 && a->M > 8 && !a->ln_weight && !a->tp_mode)));
+    const bool few = few_rows(a->M, a->N, a->K, route, a->ln_weight || a->tp_mode);
     const bool pairs = !few && route == 4 && w4_tc2_route(a->M, a->N, a->K);
     const int step = pairs ? a->M : route == 4 ? 256 : 32;
     for (int m0 = 0; m0 < a->M; m0 += step) {
