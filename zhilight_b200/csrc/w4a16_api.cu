@@ -202,7 +202,7 @@ extern "C" int zl_w4a16_gemm_fused(const zl_w4_fused_args_t* a, zl_stream_t stre
             p.dbg = dbg;
         }
         p.trace = g_w4_trace;
-        if (p.dbg & 32) p.ln_w = nullptr;   // timing probe: drop the fused RMSNorm (results are wrong)
+        if ((p.dbg & 32) && a->M <= 8) p.ln_w = nullptr;   // timing probe: drop the fused RMSNorm (results are wrong)
         p.tp_cd = tp_cd;
         p.tp_mode = a->tp_mode;
         p.tp_index = a->tp_index;

@@ -710,8 +710,11 @@ static cudaError_t launch_v3_t(const W4Params& p, int smem, bool pdl, cudaStream
             return cudaErrorNotSupported;
         }
     }
-    return launch(k_w4a16_v3<NT, NORM, WARPS, SUBS, STAGES, RT, PACK>, dim3(grid), dim3(WARPS * SUBS * 32), (size_t)smem, stream,
-                  pdl, p);
+    if constexpr (NT == 2 && !NORM)
+        return cudaErrorNotSupported;   // 9 to 16 rows with neither norm nor exchange are the fp16 kernel's (w4a16_api.cu)
+    else
+        return launch(k_w4a16_v3<NT, NORM, WARPS, SUBS, STAGES, RT, PACK>, dim3(grid), dim3(WARPS * SUBS * 32), (size_t)smem, stream,
+                      pdl, p);
 }
 
 template <int NT, int WARPS, int SUBS, int STAGES, int RT = NT * 8>
@@ -819,7 +822,7 @@ cudaError_t prepare_w4_v3() {
 #undef ZL_SET2
     ZL_SET(1, false, 8, 2, 5) ZL_SET(1, true, 8, 2, 5) ZL_SET(1, false, 8, 2, 4) ZL_SET(1, true, 8, 2, 4)
     ZL_SET(1, false, 16, 1, 4) ZL_SET(1, true, 16, 1, 4)
-    ZL_SET(2, false, 8, 2, 4) ZL_SET(2, true, 8, 2, 4) ZL_SET(2, false, 16, 1, 4) ZL_SET(2, true, 16, 1, 4)
+    ZL_SET(2, true, 8, 2, 4) ZL_SET(2, true, 16, 1, 4)
 #undef ZL_SET
 #define ZL_SETX(NT, NORM, W, SB, PK)                                                                            \
     e = cudaFuncSetAttribute(k_w4a16_v3<NT, NORM, W, SB, 4, NT * 8, PK, 1>,                                     \
