@@ -162,11 +162,12 @@ unsigned zl_w4_tc_watchdog(void);
  * the current device since it was last reported; zl_last_error names it.  The decoders ask at the end of every step, the GEMMs
  * and zl_decode_attention with prompt portions at each call. */
 int zl_check_waits(void);
-/* the unreported code of the general tensor-core GEMM (zl_gemm_nt*, zl_dense_gemm_skinny* and zl_w8a8_gemm with prompt-sized M) and of
- * the 4-bit GEMM over pairs of SMs, after a synchronisation of the device; 0 = none */
+/* the unreported code of the general tensor-core GEMM (zl_gemm_nt*, zl_dense_gemm_skinny* and zl_w8a8_gemm with prompt-sized M), of the 4-bit GEMM
+ * over pairs of SMs and of the attention of prompt portions, after a synchronisation of the device; 0 = none */
 unsigned zl_gemm_tc_watchdog(void);
 unsigned zl_w4_tc2_watchdog(void);
-/* tests: the codes of the current device, these two and that of the attention (host memory; NULL: none could be had) */
+unsigned zl_prompt_attention_watchdog(void);
+/* tests: the three codes of the current device, in this order (host memory; NULL: none could be had) */
 void* zl_wait_words(void);
 /* debug / tests: at least `splits` pieces per weight-row tile in the tcgen05 kernel's stream-k schedule (0 = automatic; also
  * ZL_TC_SPLITS). */

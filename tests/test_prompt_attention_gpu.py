@@ -13,6 +13,12 @@ pytestmark = pytest.mark.gpu
 TOL = {torch.float16: ("f16", 1e-3), torch.bfloat16: ("bf16", 6e-3)}
 
 
+@pytest.fixture(autouse=True)
+def no_wait_gave_up(lib):
+    yield
+    assert lib.zl_prompt_attention_watchdog() == 0
+
+
 def _run(cuda, dtype, lens, len_q, hq, hkv, d, masks, bshd=True, seed=0):
     from zhilight_b200 import ops
     g = torch.Generator().manual_seed(seed)

@@ -13,29 +13,32 @@ pytestmark = pytest.mark.gpu
 def words(lib, cuda):
     torch.cuda.synchronize()
     w = ctypes.cast(lib.zl_wait_words(), ctypes.POINTER(ctypes.c_uint))
-    assert w and (w[0], w[1]) == (0, 0)
+    assert w and (w[0], w[1], w[2]) == (0, 0, 0)
     yield w
-    w[0] = w[1] = 0
+    w[0] = w[1] = w[2] = 0
 
 
-@pytest.mark.parametrize("which,name", [(0, "general tensor-core GEMM"), (1, "4-bit GEMM")])
-@pytest.mark.parametrize("call", ["w4", "nt", "dense", "w8", "check"])
+@pytest.mark.parametrize("which,name", [(0, "general tensor-core GEMM"), (1, "4-bit GEMM"), (2, "attention of prompt portions")])
+@pytest.mark.parametrize("call", ["w4", "nt", "dense", "w8", "attention", "check"])
 def test_next_call_raises_once(lib, cuda, words, which, name, call):
     from zhilight_b200 import _lib, ops
     x, w = torch.ones(40, 128, dtype=torch.float16, device=cuda), torch.ones(128, 128, dtype=torch.float16, device=cuda)
     packed = torch.zeros(int(lib.zl_w4_packed_bytes(128, 128, 128)), dtype=torch.uint8, device=cuda)
     x8, one = torch.ones(40, 128, dtype=torch.int8, device=cuda), torch.ones(128, device=cuda)
+    q, kv = torch.ones(1, 64, 32, 128, dtype=torch.float16, device=cuda), torch.ones(512, 8, 128, dtype=torch.float16, device=cuda)
+    lens = torch.tensor([512], dtype=torch.int32, device=cuda)
     run = {"w4": lambda: ops.w4a16_gemm_fused(x, packed, 128, 128, variant=1), "nt": lambda: ops.gemm_nt(x, w),
            "dense": lambda: ops.dense_gemm_skinny(x, w), "w8": lambda: ops.w8a8_gemm(x8, one[:40], x8.new_ones(128, 128), one, torch.float16),
-           "check": ops.check_waits}[call]
+           "attention": lambda: ops.decode_attention(q, lens, [kv], [kv], None, 0.09, 512, 8), "check": ops.check_waits}[call]
     run()
     words[which] = 0x3401
-    assert (lib.zl_gemm_tc_watchdog(), lib.zl_w4_tc2_watchdog())[which] == 0x3401
+    codes = [lib.zl_gemm_tc_watchdog(), lib.zl_w4_tc2_watchdog(), lib.zl_prompt_attention_watchdog()]
+    assert codes == [0x3401 if i == which else 0 for i in range(3)]
     with pytest.raises(_lib.ZLError, match=name + ".*0x3401"):
         run()
     run()
     torch.cuda.synchronize()
-    assert (words[0], words[1]) == (0, 0)
+    assert (words[0], words[1], words[2]) == (0, 0, 0)
 
 
 def test_decoder_raises_at_the_end_of_its_step(lib, cuda, words):
@@ -58,9 +61,10 @@ def test_decoder_raises_at_the_end_of_its_step(lib, cuda, words):
     with pytest.raises(_lib.ZLError, match="0x2403"):
         step()
     np.testing.assert_array_equal(step(), want)
-    words[1] = 0x3403
-    with pytest.raises(_lib.ZLError, match="0x3403"):
-        dec.prefill(0, np.arange(5, dtype=np.int32), 0)
+    for i, code in ((1, 0x3403), (2, 0x4403)):
+        words[i] = code
+        with pytest.raises(_lib.ZLError, match=hex(code)):
+            dec.prefill(0, np.arange(5, dtype=np.int32), 0)
 
 
 _CAPTURE_FIRST = """

@@ -375,6 +375,12 @@ extern "C" size_t zl_decode_attention_workspace_bytes(int B, int len_q, int num_
     return (size_t)B * len_q * num_heads * splits * (dim_head + 2) * sizeof(float);
 }
 
+extern "C" unsigned zl_prompt_attention_watchdog(void) {
+    cudaDeviceSynchronize();
+    const unsigned* words = wait_words();
+    return words ? words[kWaitAttnPrompt] : 0u;
+}
+
 extern "C" int zl_prompt_attention_smem_bytes(int dim_head) {
     return dim_head == 64 ? PaCfg<64>::kBytes : dim_head == 128 ? PaCfg<128>::kBytes : 0;
 }
