@@ -101,9 +101,9 @@ def test_attention(lib, cuda, monkeypatch, b, len_q):
     length = torch.tensor(lens, dtype=torch.int32, device=cuda)
     mask = torch.ones(len_q, lens[0], device=cuda).tril(lens[0] - len_q).to(torch.int8) if len_q > 1 else None
 
-    def call(k=ks, v=vs, m=mask, scale=0.09, query=q):
-        return ops.decode_attention(query, length, k, v, m, scale, max(lens), 2)
-    for f in (call, lambda: call(tuple(ks), tuple(vs)), lambda: call(iter(ks), list(vs)), lambda: call(scale=1), lambda: call(query=torch.cat([q, q], 3)[..., :128]),
+    def call(k=ks, v=vs, m=mask, scale=0.09, query=q, pdl=False):
+        return ops.decode_attention(query, length, k, v, m, scale, max(lens), 2, pdl=pdl)
+    for f in (call, lambda: call(tuple(ks), tuple(vs)), lambda: call(iter(ks), list(vs)), lambda: call(scale=1), lambda: call(pdl=True), lambda: call(query=torch.cat([q, q], 3)[..., :128]),
               lambda: call([t.as_subclass(_Own) for t in ks]), lambda: call([torch.from_dlpack(t) for t in ks]), lambda: call(query=q.double()),
               lambda: call(query=q[0])):
         _same(_both(monkeypatch, f))
