@@ -6,23 +6,37 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def _both(monkeypatch, f):
-    """f() through the native module (which has to serve it unless it says otherwise) and through the general path."""
-    from zhilight_b200 import ZLError, _lib
-    outs = []
-    for host in (_lib.host, None):
+class _Asked:
+    """The native module, with a note of whether it served each call (a refusal of the library's is an answer too) or left it to the general path."""
+
+    def __init__(self, host):
+        self.host, self.served = host, []
+
+    def __getattr__(self, name):
+        def call(*args):
+            y = getattr(self.host, name)(*args)
+            self.served.append(y is not None)
+            return y
+        return call
+
+
+def _same(monkeypatch, f, served=True, raises=None):
+    """f() with the native module and without: the same result, or the same error where one is named.  served: whether the module serves the call;
+    None: it is not asked."""
+    from zhilight_b200 import _lib
+    asked, outs = _Asked(_lib.host), []
+    for host in (asked, None):
         with monkeypatch.context() as m:
             m.setattr(_lib, "host", host)
-            try:
+            if raises is None:
                 outs.append(f())
-            except (ZLError, RuntimeError, ValueError, IndexError, TypeError) as e:
-                outs.append((type(e), getattr(e, "code", None)))
-    return outs
-
-
-def _same(outs):
+            else:
+                with pytest.raises(raises) as e:
+                    f()
+                outs.append((type(e.value), getattr(e.value, "code", None)))
+    assert asked.served == ([] if served is None else [served])
     a, b = outs
-    if isinstance(a, tuple) or isinstance(b, tuple):
+    if raises is not None:
         assert a == b
     else:
         assert a.dtype == b.dtype and a.shape == b.shape and a.stride() == b.stride() and torch.equal(a, b)
@@ -32,8 +46,10 @@ class _Own(torch.Tensor):
     pass
 
 
-FORMS = {"plain": lambda t: t, "strided": lambda t: torch.cat([t, t], 1)[:, :t.shape[1]], "parameter": lambda t: torch.nn.Parameter(t, requires_grad=False),
-         "subclass": lambda t: t.as_subclass(_Own), "flat": lambda t: t[0], "float": lambda t: t.float(), "narrow": lambda t: t[:, :64]}
+# a form of x, whether the native module serves it (None: layers.Linear has refused it before)
+FORMS = {"plain": (lambda t: t, True), "strided": (lambda t: torch.cat([t, t], 1)[:, :t.shape[1]], True),
+         "parameter": (lambda t: torch.nn.Parameter(t, requires_grad=False), True), "subclass": (lambda t: t.as_subclass(_Own), False),
+         "flat": (lambda t: t[0], None), "float": (lambda t: t.float(), None), "narrow": (lambda t: t[:, :64], None)}
 
 
 def _linear(k, n, quant, dtype, seed):
@@ -58,11 +74,13 @@ def _linear(k, n, quant, dtype, seed):
 @pytest.mark.parametrize("form", sorted(FORMS))
 @pytest.mark.parametrize("m", [1, 40])
 def test_linears(lib, cuda, monkeypatch, form, m):
+    from zhilight_b200 import ZLError
+    make, served = FORMS[form]
     for quant, dtype in ((0, "bfloat"), (0, "half"), (1, "half"), (7, "bfloat"), (5, "half")):
         lin, g = _linear(512, 384, quant, dtype, m)
         x = torch.randn(m, 512, generator=g, device=cuda).to(lin.dtype)
-        _same(_both(monkeypatch, lambda: lin(FORMS[form](x))))
-        _same(_both(monkeypatch, lambda: lin(x[None])))
+        _same(monkeypatch, lambda: lin(make(x)), served, ZLError if served is None else None)
+        _same(monkeypatch, lambda: lin(x[None]))
 
 
 ONE_ROW = {"odd pitch": lambda x: torch.cat([x, x[:, :13]], 1).expand(2, -1).contiguous()[:1, :x.shape[1]], "pitch of one": lambda x: x.flatten().as_strided(x.shape, (1, 1)),
@@ -81,19 +99,31 @@ def test_one_row_of_any_pitch(lib, cuda, form, quant, dtype):
 
 
 def test_entry_points(lib, cuda, monkeypatch):
-    from zhilight_b200 import ops
+    from zhilight_b200 import ZLError, ops
     g = torch.Generator(device="cuda").manual_seed(0)
     x, w = torch.randn(3, 256, generator=g, device=cuda).half(), torch.randn(512, 256, generator=g, device=cuda).half()
-    for f in (lambda: ops.dense_gemm_skinny(x, w, out_dtype=torch.float32), lambda: ops.dense_gemm_skinny(x, w, out_dtype=torch.float64),
-              lambda: ops.dense_gemm_skinny(x, w.t()), lambda: ops.dense_gemm_skinny(x[:, :7].contiguous(), w[:, :7].contiguous()), lambda: ops.dense_gemm_skinny(x.cpu(), w),
-              lambda: ops.int8_linear(x, w.to(torch.int8), torch.rand(512, device=cuda, generator=torch.Generator(device="cuda").manual_seed(1))),
-              lambda: ops.int8_linear(x[:0], w.to(torch.int8), torch.ones(512, device=cuda)), lambda: ops.fp8_linear(x, w.to(torch.int8), torch.ones(1, device=cuda).double())):
-        _same(_both(monkeypatch, f))
+    scale = torch.rand(512, device=cuda, generator=g)
+    packed = torch.zeros(int(lib.zl_w4_packed_bytes(512, 256, 128)), dtype=torch.uint8, device=cuda)
+    given = torch.empty(3, 512, device=cuda).half()
+    _same(monkeypatch, lambda: ops.w4a16_gemm_fused(x, packed, 512, 256, variant=1))
+    _same(monkeypatch, lambda: ops.w4a16_gemm_fused(x, packed, 512, 256, variant=1, out=given))
+    _same(monkeypatch, lambda: ops.w4a16_gemm_fused(x, packed, 512, 256, epilogue=ops.EPI_SWIGLU, variant=1, pdl=True))
+    _same(monkeypatch, lambda: ops.w4a16_gemm_fused(x, packed, 512, 256, epilogue=ops.EPI_RESIDUAL, variant=1), raises=ZLError)
+    _same(monkeypatch, lambda: ops.w4a16_gemm_fused(x.float(), packed, 512, 256, variant=1), False, ZLError)
+    _same(monkeypatch, lambda: ops.dense_gemm_skinny(x, w, out_dtype=torch.float32))
+    _same(monkeypatch, lambda: ops.dense_gemm_skinny(x, w, out_dtype=torch.float64), False, ZLError)
+    _same(monkeypatch, lambda: ops.dense_gemm_skinny(x, w.t()), False, ZLError)
+    _same(monkeypatch, lambda: ops.dense_gemm_skinny(x[:, :7].contiguous(), w[:, :7].contiguous()), raises=ZLError)
+    _same(monkeypatch, lambda: ops.dense_gemm_skinny(x.cpu(), w), False, ZLError)
+    _same(monkeypatch, lambda: ops.int8_linear(x, w.to(torch.int8), scale))
+    _same(monkeypatch, lambda: ops.int8_linear(x[:0], w.to(torch.int8), scale), raises=ZLError)
+    _same(monkeypatch, lambda: ops.fp8_linear(x, w.to(torch.float8_e4m3fn).view(torch.uint8), torch.ones(1, device=cuda)))
+    _same(monkeypatch, lambda: ops.fp8_linear(x, w.to(torch.int8), torch.ones(1, device=cuda).double()), False, ZLError)
 
 
 @pytest.mark.parametrize("b,len_q", [(1, 1), (5, 1), (1, 40)])
 def test_attention(lib, cuda, monkeypatch, b, len_q):
-    from zhilight_b200 import ops
+    from zhilight_b200 import ZLError, ops
     g = torch.Generator(device="cuda").manual_seed(b)
     lens = [300 - 17 * i for i in range(b)]
     q = torch.randn(b, len_q, 8, 128, generator=g, device=cuda).half()
@@ -103,10 +133,14 @@ def test_attention(lib, cuda, monkeypatch, b, len_q):
 
     def call(k=ks, v=vs, m=mask, scale=0.09, query=q, pdl=False):
         return ops.decode_attention(query, length, k, v, m, scale, max(lens), 2, pdl=pdl)
-    for f in (call, lambda: call(tuple(ks), tuple(vs)), lambda: call(iter(ks), list(vs)), lambda: call(scale=1), lambda: call(pdl=True), lambda: call(query=torch.cat([q, q], 3)[..., :128]),
-              lambda: call([t.as_subclass(_Own) for t in ks]), lambda: call([torch.from_dlpack(t) for t in ks]), lambda: call(query=q.double()),
-              lambda: call(query=q[0])):
-        _same(_both(monkeypatch, f))
+    for f in (call, lambda: call(tuple(ks), tuple(vs)), lambda: call(scale=1), lambda: call(pdl=True)):
+        _same(monkeypatch, f)
+    for f in (lambda: call([t.as_subclass(_Own) for t in ks]), lambda: call([torch.from_dlpack(t) for t in ks])):
+        _same(monkeypatch, f, False)
+    _same(monkeypatch, lambda: call(iter(ks), list(vs)), False, TypeError)
+    _same(monkeypatch, lambda: call(query=torch.cat([q, q], 3)[..., :128]), False, ZLError)
+    _same(monkeypatch, lambda: call(query=q.double()), False, ZLError)
+    _same(monkeypatch, lambda: call(query=q[0]), False, ValueError)
 
 
 def test_memory_of_another_stream_outlives_its_tensors(lib, cuda):
