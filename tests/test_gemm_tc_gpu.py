@@ -114,6 +114,18 @@ def test_long_sums_of_few_tiles(lib, cuda, dtype, out, m, n, k, splits):
     _close(ops.gemm_nt(xb, wb, out_dtype=out), prod(xb.double(), wb.double()), prod(xb.double().abs(), wb.double().abs()), k, out)
 
 
+@pytest.mark.parametrize("b,m,n,k,pairs", [(1, 33, 128, 200, 0), (1, 33, 128, 216, 1), (1, 200, 256, 256, 1), (1, 384, 2050, 256, 1), (16, 33, 512, 136, 0), (16, 256, 128, 64, 0),
+                                            (48, 200, 250, 128, 1), (48, 33, 1024, 256, 1), (4, 384, 512, 72, 0)])
+def test_line_to_the_tile_kernel(lib, cuda, b, m, n, k, pairs):
+    """Both sides of the line of short sums, at one to forty-eight matrices."""
+    from zhilight_b200 import ops
+    assert lib.zl_gemm_nt_pairs_route(m, n, k, b) == pairs
+    g = torch.Generator().manual_seed(k)
+    x, w = _rand(g, b, m, k, dtype=BF), _rand(g, b, n, k, dtype=BF)
+    prod = lambda a, c: torch.einsum("bmk,bnk->bmn", a, c)  # noqa: E731
+    _close(ops.gemm_nt(x, w, out_dtype=torch.float32), prod(x.double(), w.double()), prod(x.double().abs(), w.double().abs()), k, torch.float32)
+
+
 @pytest.mark.parametrize("dtype", [BF, HF])
 @pytest.mark.parametrize("sizes", [[0, 9, 1, 0, 31], [32, 33, 0, 64, 1], [1] * 150, [256, 0, 257, 3], [700, 12]])
 @pytest.mark.parametrize("n,k", [(128, 64), (300, 200), (512, 520)])

@@ -479,23 +479,6 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
     }
 }
 
-// Rows of x per tile for M rows, `rows` row tiles (times the batch) and `pairs` pairs of CTAs: the waves times a tile's cost per
-// 64-k stage, which is its loads (16 KB of w and 64 B per row of x, about 50 B a cycle) rather than its MMAs (2 cycles per row)
-static int gt_pick_ntok(int M, long long rows, int pairs) {
-    int best = 32;
-    double best_cost = 1e30;
-    for (int n = 32; n <= 256; n += 32) {
-        const long long tiles = rows * cdiv(M, n), waves = (tiles + pairs - 1) / pairs;
-        const double cost = (double)waves * (330.0 + 1.3 * n);
-        if (cost < best_cost - 1e-9) {
-            best_cost = cost;
-            best = n;
-        }
-        if (n >= M) break;
-    }
-    return best;
-}
-
 // Rows of x per tile, and how many pairs share a tile's K, for `blocks` 128-byte blocks of k: with few tiles the pairs of a cluster (the device holds
 // fit[0] clusters of two pairs at a time, fit[1] of four) take a part each and exchange their sums.  In cycles, fitted to the times below: a block
 // 190 + 1.4 per row of x, the exchange 2850 + 42 per row.  Measured, one pair / two, us, N x K: bf16 4096 x 14336, 65 rows 39.3 / 31.2, 256 rows
@@ -523,21 +506,23 @@ static GtPick gt_pick(int M, long long rows, int pairs, int blocks, const int (&
 }
 
 // A short K and few tiles are the tile kernel's: a launch of it costs 2.9 us and 1 us per 100 of k, here the pair's allocation, barriers and
-// hand-overs cost 5 us and k a quarter of that.  Both times in us, fitted to 566 measured shapes (M = 33 .. 512, N = 128 .. 4096, K = 64 .. 8192,
-// 1 .. 64 matrices; above K = 512 this kernel was the faster one at all of them): the tile kernel's first wave of 64 x 64 blocks and what
-// each further block's rows cost; here the tile's rows and what a further wave of pairs costs.  Measured, tile kernel / here, M x N x K: 33 x 128 x 64
-// 2.7 / 5.3; 256 x 2048 x 256 5.7 / 6.5; 128 x 512 x 384 7.0 / 6.5; 16 matrices of 33 x 512 x 128 3.8 / 6.0, of 300 x 512 x 128 11.1 / 9.1; 48 of
-// 64 x 1024 x 128 12.7 / 10.7, of 33 x 1024 x 128 9.2 / 9.9.  At no measured shape does the choice cost more than 3 % of the tile kernel's time.
+// hand-overs cost 4 us and k a sixth of that.  Both times in us per call of a row of calls in a graph, where this kernel starts under the end of the one
+// before it, fitted to 1488 measured shapes (M = 33 .. 512, N = 128 .. 4096, K = 64 .. 1024, 1 .. 48 matrices; above K = 256 this kernel was the
+// faster one at all of them): the tile kernel's first wave of 64 x 64 blocks and what each further block's rows cost; here the tile's rows and what a
+// further wave of pairs costs.  Measured, tile kernel / here, M x N x K: 33 x 128 x 64 2.8 / 4.0; 256 x 512 x 256 5.5 / 4.4; 384 x 2048 x 256 7.8 / 5.6;
+// 16 matrices of 33 x 512 x 128 3.7 / 4.8, of 256 x 128 x 64 3.6 / 5.6; 48 of 200 x 256 x 128 12.4 / 8.9, of 33 x 4096 x 256 37.8 / 25.6.  The estimates err by 6 and 5 %
+// on average, so half a microsecond counts as even and stays there: at no measured shape does this kernel serve what the other one would serve faster
+// (without, up to 14 % there), and what stays costs up to 25 %, 1 % on average over all shapes.
 bool gemm_tile_faster(int M, int N, int K, int batch) {
-    if (K > 512) return false;
+    if (K > 256) return false;
     const int sms = device_sm_count(), pairs = sms / 2;
     const long long blocks = (long long)batch * cdiv(M, 64) * cdiv(N, 64), rows = (long long)batch * cdiv(N, kTc2Rows);
     const double further = blocks > sms ? (double)(blocks - sms) * M / (64.0 * cdiv(M, 64)) : 0.0;
-    const int n = gt_pick_ntok(M, rows, pairs);
+    const int n = gt_pick(M, rows, pairs, cdiv(K, 64), {0, 0}).ntok;   // too short a K for any pairs to share
     const double waves = (double)((rows * cdiv(M, n) + pairs - 1) / pairs - 1);
-    const double tile = 2.93 + 0.01046 * K + further * (0.00902 + 2.84e-5 * K);
-    const double here = 4.84 + 0.00246 * K + 0.025 * n + waves * (0.205 + 0.0232 * n + 0.001 * K);
-    return tile < here;
+    const double tile = 2.9 + 0.0102 * K + further * (0.0086 + 3.1e-5 * K);
+    const double here = 3.3 + 0.0017 * K + 0.028 * n + waves * (0.2 + 0.0204 * n + 0.003 * K);
+    return tile < here + 0.45;
 }
 
 bool gemm_tc_route(const GemmP& p, int batch, int in_dtype) {
