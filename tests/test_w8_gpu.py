@@ -207,3 +207,29 @@ def test_long_sums_of_few_tiles(lib, cuda, m, n, k, splits):
     y = ops.w8a8_gemm(xf.view(torch.uint8), one, wf.view(torch.uint8), one, torch.bfloat16, ops.W8_FP8)
     ref = xf.double() @ wf.double().T / 16
     assert float((y.double() - ref).norm() / ref.norm()) <= 2.0 ** -8
+
+
+@pytest.mark.parametrize("m,n,k,kind,pairs", [(8, 9472, 4480, 0, 1), (8, 9464, 4480, 0, 0), (1, 9472, 4416, 0, 0), (3, 3584, 19328, 0, 1), (3, 3576, 19328, 0, 0), (9, 5120, 4928, 0, 1),
+                                              (16, 5112, 4992, 0, 0), (9, 4096, 11008, 0, 1), (16, 5120, 4864, 0, 0), (17, 512, 8192, 0, 1), (17, 2560, 8128, 0, 0),
+                                              (32, 2576, 8192, 0, 1), (32, 5124, 4096, 0, 1), (32, 5116, 4096, 0, 0), (8, 5120, 8192, 1, 0), (8, 9472, 4480, 1, 1), (9, 3072, 4096, 1, 1),
+                                              (16, 3064, 4224, 1, 0), (16, 3072, 4032, 1, 0), (17, 1544, 8192, 1, 1), (32, 1528, 8192, 1, 0)])
+def test_line_between_the_kernels(lib, cuda, m, n, k, kind, pairs):
+    """Both sides of each line of up to 32 rows: int8 exact, e4m3 within what an fp32 accumulator may drop and the output's rounding."""
+    from zhilight_b200 import ops
+    assert lib.zl_w8_pairs_route(m, n, k, kind) == pairs
+    g = torch.Generator(device="cuda").manual_seed(n)
+    sw, b = torch.rand(n, generator=g, device="cuda") * 0.01, torch.randn(n, generator=g, device="cuda").half()
+    if kind == ops.W8_INT8:
+        x, w = (torch.randint(-128, 128, s, generator=g, device="cuda", dtype=torch.int8) for s in ((m, k), (n, k)))
+        sx = torch.rand(m, generator=g, device="cuda") * 0.01
+        want = (((x.double() @ w.double().T).float() * sx[:, None]) * sw).half()
+        assert torch.equal(ops.w8a8_gemm(x, sx, w, sw, torch.float16, bias=b), (want.float() + b.float()).half())
+        return
+    x, w = (torch.randn(*s, generator=g, device="cuda").to(torch.float8_e4m3fn) for s in ((m, k), (n, k)))
+    one = torch.rand(1, generator=g, device="cuda") * 0.01
+    y = ops.w8a8_gemm(x.view(torch.uint8), one, w.view(torch.uint8), sw[:1], torch.float16, ops.W8_FP8, bias=b)
+    scale = one.double() * sw[:1].double()
+    ref, mag = (x.double() @ w.double().T) * scale + b.double(), (x.double().abs() @ w.double().abs().T) * scale
+    # the sum rounds once to fp16 ahead of the bias's addition and once behind it
+    lim = (k / 32 + 4) * 2.0 ** -23 * mag + 2.0 ** -11 * (ref.abs() + (ref - b.double()).abs()) + 2.0 ** -24
+    assert not ((y.double() - ref).abs() > lim).any()

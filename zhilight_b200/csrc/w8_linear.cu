@@ -499,19 +499,28 @@ extern "C" int zl_int8_scale_back(const int32_t* acc, const float* x_scale, cons
     return ZL_OK;
 }
 
-// Whether M rows go to the kernel on pairs of SMs (gemm_tc.cu), which costs the same from 1 row to 128; the mma.sync kernel reads the
-// weights once per 32 rows and its activations once per 16 weight rows.  us, here against mma.sync (int8 / fp8):
-//   M = 64      4096 x 4096 19 against 24; 4096 x 14336 26 / 31
-//   M = 33      no slower than the split-k kernel that served it before, from 1088 x 512 (6.0 against 6.7 / 6.0) and 256 x 1024 (6.7
-//               against 7.9 / 7.0) up to 14336 x 1024 (9.5 / 9.0 against 9.7 / 9.0)
-//   M = 32      8192 x 8192 23 against 34 / 46; 14336 x 4096 19 / 33 / 44; 4096 x 14336 27 / 29 / 37; 4096 x 4096 19 / 15 / 17
-//   M = 16      8192 x 8192 23 / 25 / 35; 14336 x 4096 19 / 25 / 33; 4096 x 14336 27 / 21 / 29
-//   M = 8       8192 x 8192 23 / 20 / 21; 28672 x 8192 48 / 60 / 62
-static bool w8_tc_route(int M, int N, int K) {
-    if (M > 32) return true;
+// Whether M rows go to the kernel on pairs of SMs (gemm_tc.cu), which costs the same from 1 row to 32 and has few, large tiles, whose K up to four
+// pairs share; the mma.sync kernel reads its activations once per 16 weight rows and takes half as long again from 8 rows to 9 and from 16 to 17, fp8
+// more than int8.  So the lines are weights per step of rows, and below 17 rows N as well: few tiles read the weights through few SMs.  us of a whole
+// Linear in a row of calls, quantisation included, mma.sync / here; of 1112 measured points (46 sizes from 1024 x 1024 to 28672 x 8192) none is sent here
+// that takes longer here, and what stays costs 1.7 % on average:
+//   int8, 32 rows   4096 x 4096 11.9 / 11.8; 6144 x 4096 20.0 / 12.6; 8192 x 8192 36.0 / 19.3; 1024 x 8192 17.0 / 11.5
+//         16        4096 x 4096 8.9 / 11.8; 6144 x 4096 14.5 / 12.5; 4096 x 8192 13.9 / 14.8; 4096 x 14336 21.7 / 19.1
+//          8        8192 x 8192 19.1 / 18.8; 8192 x 5120 14.7 / 15.0; 10240 x 4096 17.1 / 14.2; 28672 x 8192 59.9 / 43.8
+//   fp8,  32 rows   2048 x 4096 14.4 / 15.8; 4096 x 4096 20.5 / 17.8; 8192 x 8192 49.9 / 24.8
+//         16        2048 x 8192 16.4 / 18.4; 4096 x 4096 14.8 / 12.3; 8192 x 8192 39.6 / 25.0
+//          8        8192 x 5120 16.7 / 14.7; 14336 x 4096 20.7 / 16.4; 4096 x 14336 22.7 / 24.6
+// From 33 rows on it is here at every size (1088 x 512 6.0 against 6.7 / 6.0 for the kernel that served it before).
+static bool w8_tc_route(int M, int N, int K, bool fp8) {
+    constexpr long long kMi = 1 << 20;
     const long long weights = (long long)N * K;
-    if (weights < (48ll << 20)) return false;
-    return weights >= (128ll << 20) || M > (N >= 8192 ? 8 : 24);
+    if (M > 32 || weights >= 128 * kMi) return true;
+    if (M > 16) return fp8 ? weights >= 12 * kMi : weights >= 20 * kMi || (K >= 8192 && weights >= 4 * kMi);
+    if (M > 8) return fp8 ? weights >= 12 * kMi && N >= 3072 : weights >= 24 * kMi && (N >= 5120 || weights >= 43 * kMi);
+    return weights >= 40 * kMi && (N >= 9472 || (weights >= 66 * kMi && N >= 3584));
+}
+extern "C" int zl_w8_pairs_route(int M, int N, int K, int kind) {
+    return M > 0 && N > 0 && K > 0 && w8_tc_route(M, N, K, kind != ZL_W8_INT8) ? 1 : 0;
 }
 
 extern "C" int zl_w8a8_gemm(const void* xq, const float* x_scale, const void* w, const void* w_scale,
@@ -528,8 +537,8 @@ extern "C" int zl_w8a8_gemm(const void* xq, const float* x_scale, const void* w,
     const uint8_t* xq8 = static_cast<const uint8_t*>(xq);
     const uint8_t* w8 = static_cast<const uint8_t*>(w);
     const int sw_f32 = kind == ZL_W8_FP8_ROWS ? 2 : (w_scale_dtype == ZL_F32 ? 1 : 0);
-    if (w8_tc_route(M, N, K)) {
-        const bool fp8 = kind != ZL_W8_INT8;
+    const bool fp8 = kind != ZL_W8_INT8;
+    if (w8_tc_route(M, N, K, fp8)) {
         const int sw_mode = fp8 ? (kind == ZL_W8_FP8_ROWS ? 2 : 3) : sw_f32;
         cudaError_t e;
 #define ZL_W8_TC(TT, F8)                                                                                                              \
