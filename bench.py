@@ -1284,7 +1284,7 @@ def main():
                           "requests": args.requests, "prompt_tokens": plen, "new_tokens": n_out, "batch": 1,
                           "prefill": "chunked, %d tokens per pass (tcgen05 GEMMs)" % args.prefill_chunk}
 
-    # ---- extras of the N = 1 line: BASELINE config 3 batch sizes and config 2, through the same harness ----
+    # ---- extras of the N = 1 line: batch sizes of the 8B model and the 1B bf16 model, through the same harness ----
     if sweep:
         out["batch_sweep"] = {}
         for b in sweep:
@@ -1310,7 +1310,7 @@ def main():
         "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind,
         "bytes_per_launch": g_bytes / g_launches, "us_per_launch": g_ms * 1e3 / iters / g_launches,
         "traffic": None,
-        "traffic_note": "dram bytes are not observable from inside the run; ncu --set full captures: profiles/r01_w4a16_traffic.json (integer kernel: dram reads = algorithmic bytes within 0.1 %), profiles/r02_w4a16_ts_ncu_full.txt (tcgen05 kernel: 61.4 MB read for 61.0 MB algorithmic)",
+        "traffic_note": "dram bytes are not observable from inside the run; ncu --set full captures: profiles/first_w4a16_traffic.json (integer kernel: dram reads = algorithmic bytes within 0.1 %), profiles/w4a16_ts_ncu_full.txt (tcgen05 kernel: 61.4 MB read for 61.0 MB algorithmic)",
     }
 
     if extras:

@@ -60,7 +60,7 @@ def test_awq_decode_matches_oracle(lib, cuda):
 
 @pytest.mark.parametrize("dtype,tol", [("f16", 2e-3), ("bf16", 2e-2)])
 def test_dense_decode_matches_oracle(lib, cuda, dtype, tol):
-    """BASELINE config 2 path (Llama-3.2-1B bf16: no quant, tied lm_head, d=64 attention)."""
+    """The path of Llama-3.2-1B bf16 (no quant, tied lm_head, d=64 attention)."""
     for nxt, logits, ref in _run(TINY, 0, dtype, tied=True):
         assert rel_l2(logits, ref) <= tol
 

@@ -49,7 +49,7 @@ def test_awq_pipeline_bit_exact_vs_reference(lib, ref, cuda):
 @pytest.mark.parametrize("sym", [False, True])
 @pytest.mark.parametrize("m", [1, 4, 16, 33])
 def test_w4a16_vs_reference_gemv(lib, ref, cuda, sym, m):
-    """BASELINE config 1 shape.  The reference accumulates 8 products in fp16, we accumulate in fp32: the two
+    """One row, 4096 x 4096.  The reference accumulates 8 products in fp16, we accumulate in fp32: the two
     must agree to ~1e-3 (L2) and ours must be the closer one to the exact result."""
     from zhilight_b200 import ops
     k = n = 4096

@@ -3,7 +3,7 @@
 // Why: on B200 a decode GEMM must consume ~23 weight bytes per cycle per SM to keep up with HBM.  The classic
 // "dequantise int4 -> fp16 on the CUDA cores, then fp16 MMA" recipe (our v1/v2 kernels, Marlin, the reference's
 // GEMV) costs ~10 issue slots per packed word, which makes the kernel ISSUE-bound before it is HBM-bound
-// (profiles/r01b_w4a16_v2.txt: 48 % issue utilisation at 32 % of HBM peak).  Here the int4 weights never
+// (profiles/first_w4a16_v2_ncu_full.txt: 48 % issue utilisation at 32 % of HBM peak).  Here the int4 weights never
 // become floating point:
 //   * activations are decomposed once per CTA into a block-floating-point integer  x_k = 2^e_g * m_k,
 //     m_k a 16-bit integer per 128-group (error <= 2^-16 of the group maximum, far below fp16's own 2^-11),

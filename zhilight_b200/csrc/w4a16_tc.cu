@@ -23,7 +23,7 @@
 //                      MMA issuer   : one thread, 8 x tcgen05.mma 128 x NTOK x 16 per stage (A from TMEM, B from smem),
 //                                     tcgen05.commit frees the stage; also owns the TMEM allocation
 //
-// Why A in TMEM (measured on the first version, which wrote a swizzled fp16 A tile to shared memory; profiles/r02_w4a16_tc_*):
+// Why A in TMEM (measured on the first version, which wrote a swizzled fp16 A tile to shared memory; profiles/w4a16_tc_*):
 // a 128 x 128 fp16 A stage is 32 KB written and read back through shared memory per 8.5 KB of HBM traffic, plus a
 // generic->async proxy fence per hand-over and ~10 address / store instructions per converted word.  With TMEM lane =
 // weight row and 32-bit column = two consecutive k the conversion stays in registers.
@@ -66,7 +66,7 @@ struct TsCfg {
     static constexpr int kWarpDq0 = 4, kWarpRaw = 4 + DQ, kWarpX = kWarpRaw + 1, kWarpMma = kWarpRaw + 2;
     static constexpr int kThreads = (kWarpMma + 1) * 32;
     // A pipeline stage is KG quantisation groups (KG x 128 k): every hand-over (mbarrier wait, fence, commit) costs the
-    // single MMA-issuing warp 60-150 cycles, ~700 per stage (measured with the clock64 trace, profiles/r02_tc_trace_*),
+    // single MMA-issuing warp 60-150 cycles, ~700 per stage (measured with the clock64 trace, profiles/tc_trace_*),
     // against 128 cycles of tensor work per group at 32 tokens -- two groups per stage halve that overhead per byte.
     static constexpr int KG = NTOK <= 128 ? 2 : 1;
     static constexpr int AS = NTOK <= 64 ? 3 : (NTOK <= 128 ? 2 : 3);   // A (TMEM) / x (smem) stages
