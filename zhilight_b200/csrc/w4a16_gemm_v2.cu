@@ -71,16 +71,19 @@ __device__ __forceinline__ void load_bfrag_v2(uint4 (&b)[NT][4], const W4Params&
         if (tok < p.mc) {
             const __half* src = p.x + (size_t)tok * p.ldx + kbase;
             uint4 in[4];
-            if (INTL && p.x32) {
-                ld_cg_u8(src + t * 32, in[0], in[1]);
-                ld_cg_u8(src + t * 32 + 16, in[2], in[3]);
-            } else {
+            if (INTL) {
+                if (p.x32) {
+                    ld_cg_u8(src + t * 32, in[0], in[1]);
+                    ld_cg_u8(src + t * 32 + 16, in[2], in[3]);
+                } else {
 #pragma unroll
-                for (int ii = 0; ii < 4; ++ii) in[ii] = ld_cg_u4(src + v2_k<INTL>(ii, t));
+                    for (int ii = 0; ii < 4; ++ii) in[ii] = ld_cg_u4(src + v2_k<true>(ii, t));
+                }
             }
 #pragma unroll
             for (int ii = 0; ii < 4; ++ii) {
-                uint4 v = in[ii];
+                // ZLW4: each where it is used (all four first: 105 rows of 6528 -> 2880, four passes, 47.6 -> 48.7 us)
+                uint4 v = INTL ? in[ii] : ld_cg_u4(src + v2_k<false>(ii, t));
                 if (NORM) {
                     __half2* hv = reinterpret_cast<__half2*>(&v);
                     const __half2* hw = reinterpret_cast<const __half2*>(&wl[ii]);
