@@ -385,7 +385,7 @@ extern "C" int zl_prompt_attention_smem_bytes(int dim_head) {
     return dim_head == 64 ? PaCfg<64>::kBytes : dim_head == 128 ? PaCfg<128>::kBytes : 0;
 }
 
-// Workspace of the prompt kernel ahead of the splits' partial results: the mask's bits, then the last visible keys.
+// Workspace of the prompt kernel: the mask's bits, then the last visible keys.
 static size_t prompt_head_bytes(int B, int len_q, int max_len_buf, const int8_t* mask) {
     const size_t q_rows = (size_t)B * len_q;
     return mask ? (q_rows * cdiv(max_len_buf, kPaKeys) * 8 + 15) / 16 * 16 + (q_rows * 4 + 15) / 16 * 16 : 0;

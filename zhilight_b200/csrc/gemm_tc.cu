@@ -7,8 +7,8 @@
 // cycles' worth.  Operands through tensor-TMA in six stages of 128-byte swizzled rows, two accumulators in TMEM so that a tile's
 // epilogue runs under the next tile's MMAs, persistent pairs of CTAs that take the tiles in turn.  bf16, 14336 x 4096: M = 2048
 // 970 -> 171 us (1410 TFLOP/s), M = 512 268 -> 55 us, M = 64 69 -> 30 us; 8192 x 2048, M = 1024: 154 -> 34 us.  Bound by the tensor
-// cores from about 1000 rows on, below by the loads of w (and by too few tiles: 4096 x 14336 keeps 16 of 74 pairs busy at M <= 256,
-// 52 us against 200).
+// cores from about 1000 rows on, below by the loads of w and by tiles that do not fill the pairs: 4096 x 14336 has 16 of them for 74 pairs at M <= 256
+// (200 us on mma.sync, 42.6 with a pair each, 37.2 where two share one).
 //
 //   warp 0       producer  : w and x boxes, one lane
 //   warp 1       MMA       : of the leader, one lane, 4 x 256 x ntok x 16 per 64-k block

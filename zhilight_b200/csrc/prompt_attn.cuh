@@ -13,12 +13,15 @@
 //   warps 6-7  K and V tiles by 16-byte cp.async into the swizzled layout (the buffers' addresses are known to the device only), K a tile ahead
 //
 // Probabilities are carried as a 16-bit value and the rest of it as another (two MMAs), fp16 models' times 2^10.  A row's reference maximum only
-// follows the true one once that has grown by 2^5 (fp16) or 2^8, so that O is seldom rescaled; with one fp16 value that would cost precision (the
-// largest probability is no power of two any more: 2.8e-4 from 64 bits against 2.55e-4), with two it is 2.1e-4, all of it the output's rounding.  Two
-// CTAs share an SM (256 columns each): one's MMAs run under the other's softmax.  Bound by the MMAs (a tile: 450 cycles of S, whose operands
-// come at 128 bytes a cycle, and 580 of P V) and, for short prompts, by a chain of about 10 us (launch, mask, first loads, merge).  500 rows
-// behind 1000 positions, bf16, 32 heads on 8: 65 us on mma.sync with 64-row blocks, 29 here; 512 x 1500 with 64 heads on 8, all launches of the
-// call: 120 -> 50.
+// follows the true one once that has grown by 2^5 (fp16) or 2^8, so that O is seldom rescaled (the conditional rescaling published with
+// FlashAttention-4); with one fp16 value that would cost precision (the largest probability is no power of two any more: 2.8e-4 from 64 bits against
+// 2.55e-4), with two it is 2.1e-4, all of it the output's rounding.
+//
+// Two CTAs share an SM (256 columns each): one's MMAs run under the other's softmax.  Bound by the chain S -> softmax -> P of a tile: 512 rows over 4096
+// keys, 64 heads on 8, take 114 us alone, 3700 cycles for a tile of each of the SM's two CTAs, whose MMAs take 2060 (each: 450 of S, whose operands come
+// at 128 bytes a cycle, and 580 of P V); at 500 rows behind 1000 positions, 32 on 8, 33 us, the tensor pipe is busy for 20 % of the time and 30 % of the
+// issue slots are taken.  Short prompts are a chain of about 10 us besides (launch, mask, first loads, merge).  500 rows behind 1000 positions, bf16, all launches
+// of the call: 65 us on mma.sync with 64-row blocks, 34 here; 512 x 1500 with 64 heads on 8: 120 -> 49.
 //
 // An int8 mask is turned into bits first (k_mask_bits), once for all kv heads, together with each row's last visible key: tiles behind the last
 // key any row of the block sees are never loaded, which halves a causal prompt's work.  Few blocks are cut along their keys: the CTAs of a

@@ -43,7 +43,7 @@ struct W4Params {
 };
 
 cudaError_t launch_w4_v2(const W4Params& p, bool pdl, cudaStream_t stream);
-// the same on the ZLW4I layout, up to 16 rows, no fused RMSNorm prologue
+// the same on the ZLW4I layout, up to 32 rows, no fused RMSNorm prologue
 cudaError_t launch_w4_v2_int_layout(const W4Params& p, bool pdl, cudaStream_t stream);
 cudaError_t prepare_w4_v2();
 // exact-integer kernel on the ZLW4I layout; false = staged activations do not fit shared memory

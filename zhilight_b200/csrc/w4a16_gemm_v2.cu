@@ -13,7 +13,7 @@
 //   * 2 CTAs per SM leave room for the next kernel's CTAs to become resident under programmatic dependent
 //     launch and pre-fill their rings.
 //
-// INTL: the same kernel on the ZLW4I layout (w4_layout.cuh), for up to 16 rows that the integer kernel has no room for.  A word there is four
+// INTL: the same kernel on the ZLW4I layout (w4_layout.cuh), for up to 32 rows: which ones is few_rows' in w4a16_api.cu.  A word there is four
 // consecutive k of rows g and g + 8, which is one MMA's A fragment once the order of k within the group is the layout's; a lane's x then is 64
 // consecutive bytes.  10 instructions per word where ZLW4 takes 9, and no second copy of the weights.  Bound by these conversions and by x, which
 // every CTA reads whole.

@@ -10,7 +10,7 @@
 //   * up to 64 tokens there are two accumulators; with one, eight epilogue warps shorten the gap.
 // 28672 x 4096 with SwiGLU: 1000 tokens 499 -> 190 us, 256 tokens 128 -> 60; 4096 x 14336 with the residual: 1000 tokens 408 -> 88 us
 // (1360 TFLOP/s).  Bound by the tensor cores at 256 tokens (1084 cycles per 128-k group, at the clock that the power limit leaves); below 130
-// tokens by the conversion (650 cycles of a group, 340 of them when nothing else runs on the SM).
+// tokens by the conversion (0.31 us of a group, about 600 cycles; 340 when nothing else runs on the SM).
 //
 // What a stage costs one thread is what bounded small tiles before that (830 cycles): looking at a barrier takes it 120 - 200 cycles even when the
 // phase has ended, two TMA instructions and their votes 400.  So the issuing threads are single lanes that run their warp's loop alone and look at
@@ -429,11 +429,13 @@ static T2Pick t2_pick(int M, int row_tiles, int G) {
 
 // Whether M tokens are this kernel's.  Beyond 256 w4a16_tc.cu would need several passes; below, tiles on few pairs stand against its ranges
 // over all SMs and their exchange: 10 us + 4.2 ns per token and million weights, a quarter more where it works on 128 or 256 tokens for fewer.
-// Measured, N x K, there / here, us: 4096 x 14336 at M = 64 / 76 / 128 / 256 24.7 / 30.9 / 39 / 55 and 24.2 / 24.7 / 26.7 / 33; 6144 x 4096 at M = 76
-// 25.0 and 18.4; 4096 x 4096 18.9 and 16.5; 28672 x 4096 at M = 32 / 64
-// 32.9 / 36.7 and 30.4 / 31.2, of which a pair of feed-forward calls at M = 32 keeps nothing (54.0 and 54.9); 512 x 14336 at M = 32 13 and 23.
-// Where its ranges are down to eight groups every tile is cut, and what is exchanged grows with M (2304 x 1152 at M = 40 / 256: 18 / 51 there,
-// 12 / 12.4 here; 1664 x 2176: 17 / 50 and 12.4 / 14.5; 3328 x 5248 at M = 128: 31 and 17.5).
+// Where its ranges are down to eight groups every tile is cut, and what is exchanged grows with M.
+// Measured in a row of calls, N x K, there / here, us: 4096 x 14336 at M = 32 / 64 / 128 / 256 21 / 23 / 36 / 59 and 21 / 22 / 25 / 31; 28672 x 4096 31 / 37 /
+// 54 / 105 and 28 / 29 / 37 / 61; 6144 x 4096 15 / 19 / 28 / 49 and 14 / 15 / 17 / 20; 2304 x 1152 at M = 33 / 256 16 / 49 and 10 / 10; 512 x 14336 18 / 34 and
+// 18 / 18; 4096 x 4096 at M = 33 / 64 13.1 / 13.7 and 14.1 / 14.3; 10240 x 8192 at M = 17 / 48 24 / 27 and 27 / 28.  The estimates are older than that: of 19 sizes this
+// kernel was the faster one at every one from 65 rows on and the other at three below, by 12 % at most, while calls stay there
+// that take up to 29 % (82 % at 256 rows of 512 x 14336) longer.  In a feed-forward of 4096 and 14336 at 32 rows both products there take 55.6 us,
+// both here 54.6, one of each 55.4 to 57.4; as programmatic dependents in a graph 47.2, 43.8, and 45.0 to 48.1.
 bool w4_tc2_route(int M, int N, int K) {
     if (M <= 16 || N % kTcRows || K % kW4GroupK) return false;
     if (M > 256) return true;
