@@ -152,6 +152,8 @@ int zl_w4_few_rows_route(int M, int N, int K);
 int zl_w4_pairs_route(int M, int N, int K);
 /* pairs of a cluster that share the K of a tile there (1: none do), 0 where that kernel does not serve the shape */
 int zl_w4_pairs_splits(int M, int N, int K);
+/* pieces that the tiles of its last wave come in (2: halves along the tokens); 0: another kernel's */
+int zl_w4_pairs_pieces(int M, int N, int K);
 /* tests: its pipeline's slots of converted and of packed weights (128-k groups) with `ntok` rows of x per tile (32, 64 .. 256) */
 int zl_w4_pairs_rings(int ntok, int* slots, int* raw_slots);
 /* last watchdog code published by the 4-bit stream-k kernel on the current device (0 = none); a bounded mbarrier wait that expires

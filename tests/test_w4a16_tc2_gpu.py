@@ -170,3 +170,28 @@ def test_shared_tiles_with_swiglu(lib, cuda):
     y = ops.w4a16_gemm_fused(x.to(cuda), packed, 2 * f, k, epilogue=ops.EPI_SWIGLU, variant=1).float().cpu().numpy()
     gu = oops._t(gptq.gemm_f32(x.numpy(), w), "f16")
     assert rel_l2(y, gu[:, :f] / (1.0 + np.exp(-gu[:, :f])) * gu[:, f:]) <= 2e-3
+
+
+@pytest.mark.parametrize("m,k,n,pieces", [(322, 1024, 12800, 2), (387, 1024, 13568, 2), (360, 1024, 12672, 2), (385, 1024, 13568, 2), (512, 1024, 18944, 1)])
+def test_last_wave_in_halves(lib, cuda, m, k, n, pieces):
+    """Tiles of the last wave in halves: one row behind the first half, an odd number of 128-row tiles, a last wave that is full (whole tiles); every epilogue
+    (all warps take part in it), every row."""
+    from zhilight_b200 import ops
+    assert lib.zl_w4_pairs_pieces(m, n, k) == pieces
+    w, packed = _setup(cuda, k, n, False, 6)
+    x = _x(m, k, m)
+    ref = gptq.gemm_f32(x.numpy(), w)
+    y = ops.w4a16_gemm_fused(x.to(cuda), packed, n, k, variant=1).float().cpu().numpy()
+    assert max(rel_l2(y[i], ref[i]) for i in range(m)) <= TOL
+    res = torch.randn(m, n, generator=torch.Generator().manual_seed(3)).half()
+    h = res.to(cuda)
+    ops.w4a16_gemm_fused(x.to(cuda), packed, n, k, residual=h, epilogue=ops.EPI_RESIDUAL, variant=1, out=h)
+    want = oops._t(oops._t(ref, "f16") + res.float().numpy(), "f16")
+    got = h.float().cpu().numpy()
+    assert max(rel_l2(got[i], want[i]) for i in range(m)) <= TOL
+    if n % 256 == 0:
+        _, packed2 = _setup(cuda, k, n, False, 6, ops.swiglu_row_map(n // 2, cuda))
+        act = ops.w4a16_gemm_fused(x.to(cuda), packed2, n, k, epilogue=ops.EPI_SWIGLU, variant=1).float().cpu().numpy()
+        gu = oops._t(ref, "f16")
+        want = gu[:, :n // 2] / (1.0 + np.exp(-gu[:, :n // 2])) * gu[:, n // 2:]
+        assert max(rel_l2(act[i], want[i]) for i in range(m)) <= 2e-3

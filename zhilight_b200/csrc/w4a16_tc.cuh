@@ -30,6 +30,7 @@ struct alignas(64) W4TcParams {
     __half* const* v_addrs;
     int num_heads, num_kv_heads, dim_head;
     int ntok, tok_tiles;        // w4a16_tc2.cu: rows of x per tile, tiles along them
+    int whole, cut;             // w4a16_tc2.cu: tiles from the `whole`-th on come in `cut` pieces of their rows of x
     int splits;                 // w4a16_tc2.cu: pairs of a cluster that share a tile's K (then a tile per cluster)
     int wide;                   // two neighbouring values of y may be stored together
 };
@@ -55,11 +56,13 @@ __device__ __forceinline__ void tc_fetch_residual(const W4TcParams& p, int prow,
 }
 __device__ __forceinline__ uint32_t tc_bits(float x) { return (uint32_t)__half_as_ushort(__float2half_rn(x)); }
 
-__device__ __forceinline__ void tc_epilogue16(const W4TcParams& p, int prow, int lane, int c0, float (&v)[16],
-                                              const uint32_t* rpre = nullptr) {   // rpre: what tc_fetch_residual got
+// EPI: the epilogue, or -1: p.epi's.  rpre: what tc_fetch_residual got
+template <int EPI = -1>
+__device__ __forceinline__ void tc_epilogue16(const W4TcParams& p, int prow, int lane, int c0, float (&v)[16], const uint32_t* rpre = nullptr) {
+    const int epi = EPI < 0 ? p.epi : EPI;
     const float b = p.bias ? __half2float(p.bias[prow]) : 0.f;
     const bool odd = lane & 1, up = lane & 8;
-    if (p.epi == ZL_EPI_SWIGLU) {
+    if (epi == ZL_EPI_SWIGLU) {
         const int n_out = p.N / 2;
         const int col = (prow >> 5) * 16 + ((lane >> 4) << 3) + (lane & 7);
         uint32_t h[8];   // token 2 j of the gate's lane, 2 j + 1 of the up lane
@@ -84,7 +87,7 @@ __device__ __forceinline__ void tc_epilogue16(const W4TcParams& p, int prow, int
                 if (tok < p.M) p.y[(size_t)tok * n_out + col] = __ushort_as_half((unsigned short)h[j]);
             }
         }
-    } else if (p.epi == ZL_EPI_QKV_ROPE) {
+    } else if (epi == ZL_EPI_QKV_ROPE) {
         const int d = p.dim_head, half_dim = d / 2, tiles_per_head = d / 32;
         const int st = prow >> 5, head = st / tiles_per_head, jt = st % tiles_per_head;
         const int c = jt * 16 + ((lane >> 4) << 3) + (lane & 7);
@@ -127,7 +130,7 @@ __device__ __forceinline__ void tc_epilogue16(const W4TcParams& p, int prow, int
         uint32_t h[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) h[i] = tc_bits(v[i] + b);
-        const bool res = p.epi == ZL_EPI_RESIDUAL;
+        const bool res = epi == ZL_EPI_RESIDUAL;
         if (p.wide) {
             uint32_t rw[8];
             if (res && !rpre) tc_fetch_residual(p, prow, lane, c0, rw);

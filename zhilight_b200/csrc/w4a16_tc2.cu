@@ -78,14 +78,160 @@ struct T2Tile {
     int n0, t0, ntok;   // first row of w of the pair, first token, tokens (a multiple of 32)
 };
 __device__ __forceinline__ bool t2_tile(const W4TcParams& p, int i, T2Tile& t) {
+    int piece = 0, n = p.ntok;
+    if (i >= p.whole) {   // of the last wave
+        const int j = i - p.whole;
+        i = p.whole + j / p.cut;
+        piece = j % p.cut;
+        n /= p.cut;
+    }
     const int rt = i / p.tok_tiles;
     t.n0 = rt * kTc2Rows;
-    t.t0 = (i - rt * p.tok_tiles) * p.ntok;
-    t.ntok = min(p.ntok, (p.M - t.t0 + 31) & ~31);
+    t.t0 = (i - rt * p.tok_tiles) * p.ntok + piece * n;
+    t.ntok = min(n, (p.M - t.t0 + 31) & ~31);
     return t.n0 < p.N;
 }
 
-template <int SUB>
+__device__ __forceinline__ void t2_ld8(uint32_t taddr, float (&v)[8]) {
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// The residual epilogue of tc_epilogue16, eight tokens at a time: what sixteen hold beside the conversion's state does not fit its registers
+__device__ __forceinline__ void t2_residual16(const W4TcParams& p, uint32_t taddr, int prow, int lane, int c0) {
+    const float b = p.bias ? __half2float(p.bias[prow]) : 0.f;
+    const bool odd = lane & 1;
+#pragma unroll
+    for (int half = 0; half < 2; ++half, c0 += 8, taddr += 8) {
+        uint32_t h[8], r[4];
+        if (p.wide) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int tok = c0 + 2 * j + odd;
+                r[j] = tok < p.M ? *reinterpret_cast<const uint32_t*>(p.residual + (size_t)tok * p.N + (prow & ~1)) : 0u;
+            }
+        }
+        float v[8];
+        t2_ld8(taddr, v);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) h[i] = tc_bits(v[i] + b);
+        if (p.wide) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t other = __shfl_xor_sync(0xffffffffu, odd ? h[2 * j] : h[2 * j + 1], 1);
+                const int tok = c0 + 2 * j + odd;
+                const uint32_t w = odd ? (other | (h[2 * j + 1] << 16)) : (h[2 * j] | (other << 16));
+                const float2 x = __half22float2(*reinterpret_cast<const __half2*>(&w)), y = __half22float2(*reinterpret_cast<const __half2*>(&r[j]));
+                if (tok < p.M) *reinterpret_cast<__half2*>(p.y + (size_t)tok * p.N + (prow & ~1)) = __floats2half2_rn(x.x + y.x, x.y + y.y);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (c0 + i >= p.M) continue;
+                const size_t at = (size_t)(c0 + i) * p.N + prow;
+                p.y[at] = __float2half_rn(__half2float(__ushort_as_half((unsigned short)h[i])) + __half2float(p.residual[at]));
+            }
+        }
+    }
+}
+
+// The qkv epilogue, eight tokens at a time as well, its loads in the order that hides them: what places a token's row came with the chunk before, the
+// rows' addresses, cosines and sines come together ahead of the sums.  at: placement and batch of token c0 + (lane & 15).
+__device__ __forceinline__ int2 t2_rope_place(const W4TcParams& p, int tok) {
+    return tok < p.M ? make_int2(p.placement[tok], p.token_batch[tok]) : make_int2(-1, 0);
+}
+__device__ __forceinline__ void t2_rope16(const W4TcParams& p, uint32_t taddr, int prow, int lane, int c0, int2 at) {
+    const float b = p.bias ? __half2float(p.bias[prow]) : 0.f;
+    const bool up = lane & 8;
+    const int d = p.dim_head, half_dim = d / 2, tiles_per_head = d / 32;
+    const int st = prow >> 5, head = st / tiles_per_head, jt = st % tiles_per_head;
+    const int c = jt * 16 + ((lane >> 4) << 3) + (lane & 7);
+    const bool is_v = head >= p.num_heads + p.num_kv_heads, is_q = head < p.num_heads;
+    __half* mine = nullptr;   // output row of token c0 + (lane & 15)
+    if (is_q) {
+        if (c0 + (lane & 15) < p.M) mine = p.q_out + ((size_t)(c0 + (lane & 15)) * p.num_heads + head) * d;
+    } else if (at.x >= 0) {
+        mine = (is_v ? p.v_addrs : p.k_addrs)[at.y] + ((size_t)at.x * p.num_kv_heads + (is_v ? head - p.num_heads - p.num_kv_heads : head - p.num_heads)) * d;
+    }
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        float cl[4], ch[4], sl[4], sh[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int tok = c0 + half * 8 + 2 * j + (up ? 1 : 0);
+            const bool turn = !is_v && tok < p.M;
+            const float *cs = p.cos + (size_t)tok * d + c, *sn = p.sin + (size_t)tok * d + c;
+            cl[j] = turn ? cs[0] : 1.f, sl[j] = turn ? sn[0] : 0.f;
+            ch[j] = turn ? cs[half_dim] : 1.f, sh[j] = turn ? sn[half_dim] : 0.f;
+        }
+        float v[8];
+        t2_ld8(taddr + half * 8, v);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float m0 = __half2float(__float2half_rn(v[2 * j] + b)), m1 = __half2float(__float2half_rn(v[2 * j + 1] + b));
+            const float other = __shfl_xor_sync(0xffffffffu, up ? m0 : m1, 8);
+            const float lo = up ? other : m0, hi = up ? m1 : other;
+            v[2 * j] = is_v ? lo : lo * cl[j] - hi * sl[j];
+            v[2 * j + 1] = is_v ? hi : hi * ch[j] + lo * sh[j];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            __half* dst = reinterpret_cast<__half*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(mine), half * 8 + 2 * j + (up ? 1 : 0)));
+            if (!dst) continue;
+            dst[c] = __float2half_rn(v[2 * j]);
+            dst[c + half_dim] = __float2half_rn(v[2 * j + 1]);
+        }
+    }
+}
+
+// This warp's part of a finished tile's epilogue, 32 rows of w (TMEM lanes) by the chunks of 16 tokens that are its set's, and its arrival.  Sets 0, 1
+// are the epilogue warps, 2 .. 5 the dequant groups.  shared: these help, with a chunk of eight each, the epilogue warps take two (they start
+// earlier: a group converts its first stage of the next tile before).
+template <int EPI>
+__device__ __forceinline__ bool t2_finish(const W4TcParams& p, uint8_t* smem, uint32_t tmem, int tile, int acc, uint32_t phase, bool shared) {
+    uint64_t* const acc_full = reinterpret_cast<uint64_t*>(smem + T2Cfg::kBarOff) + 2 * T2Cfg::kMaxRaw + 2 * T2Cfg::kMaxSlots + acc;
+    volatile int* const s_abort = reinterpret_cast<volatile int*>(smem + T2Cfg::kMiscOff) + 1;
+    const int lane = threadIdx.x & 31, q = (threadIdx.x >> 5) & 3, set = threadIdx.x >> 7;
+    const uint32_t rank = cluster_rank();
+    T2Tile t;
+    t2_tile(p, tile, t);
+    const int prow = t.n0 + (int)(rank & 1) * 128 + q * 32 + lane;
+    const bool rows = prow < p.N;               // N % 128 == 0: all of the CTA's rows or none
+    const int chunks = min(t.ntok, p.M - t.t0 + 15) >> 4;
+    int c = set < 2 ? set : set + 2;
+    int2 place = EPI == ZL_EPI_QKV_ROPE ? t2_rope_place(p, t.t0 + c * 16 + (lane & 15)) : make_int2(0, 0);
+    if (!tc2_wait(acc_full, phase, s_abort, p.err, 0x3800 + acc)) return false;
+    tc_fence_after();
+    if (rows) {
+        while (c < chunks) {
+            const int at = c * 16;
+            c += !shared || (set < 2 && !(c & 2)) ? 2 : set < 2 ? 6 : 8;
+            const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * 64 + at);
+            if (EPI == ZL_EPI_RESIDUAL) {
+                t2_residual16(p, taddr, prow, lane, t.t0 + at);
+            } else if (EPI == ZL_EPI_QKV_ROPE) {
+                const int2 now = place;
+                place = t2_rope_place(p, t.t0 + c * 16 + (lane & 15));
+                t2_rope16(p, taddr, prow, lane, t.t0 + at, now);
+            } else {
+                float v[16];
+                tc_ld16(taddr, v);
+                tc_epilogue16<EPI>(p, prow, lane, t.t0 + at, v);
+            }
+        }
+    }
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive_at(cluster_map(smem_u32(acc_full + 2), rank & ~1u));   // the leader's acc_empty
+    return true;
+}
+
+template <int SUB, int EPI>
 __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_constant__ W4TcParams p) {
     using C = T2Cfg;
     extern __shared__ uint8_t smem_dyn[];
@@ -107,6 +253,7 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
     const int G = stages_all * (part + 1) / splits * SUB - g_first;
     const int slots = t2_slots(p.ntok), nacc = t2_accs(p.ntok), xstage = t2_x_bytes(p.ntok), acol0 = 512 - slots * 64;
     const int rslots = t2_raw_slots(p.ntok);
+    const bool shared = nacc == 1 && splits == 1;   // a tile's epilogue is everybody's: nothing is multiplied until it has ended
     uint8_t* const nibs = smem + slots * xstage;
     uint8_t* const trs = nibs + rslots * C::kNib;
 
@@ -121,7 +268,7 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&acc_full[i], 1);
-            mbar_init(&acc_empty[i], 2 * C::kEpiWarps);
+            mbar_init(&acc_empty[i], 2 * (C::kEpiWarps + (shared ? C::kDqWarps : 0)));
         }
         *s_abort = 0;
         mbar_fence_init();
@@ -133,7 +280,7 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
     cluster_sync_all();   // both CTAs' barriers and allocations are in place
     tc_fence_after();
     const uint32_t tmem = *s_tmem;
-    const int q = warp & 3, set = warp >> 2;   // epilogue warps; with K split a tile's only chunks come behind the exchange below
+    const int q = warp & 3, set = warp >> 2;   // epilogue and dequant warps; with K split a tile's only chunks come behind the exchange below
     T2Tile t;
 
     if (warp >= C::kWarpRaw && warp < C::kWarpX) {
@@ -243,9 +390,19 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
         for (int i = pair; t2_tile(p, i, t); i += pairs) stages += G;
         int as = group, rs = group;
         uint32_t ph = 0, rph = 0;
-        bool raw_ready = false;
+        bool raw_ready = false, ok = true;
+        // Once a tile is multiplied a group has nothing to convert but what finds a slot beside it (slots stages of the next one): then it takes its
+        // part of the epilogue.  28672 x 4096 with SwiGLU, 256 tokens 59.3 -> 55.0 us, 1000 tokens 199 -> 184; 6144 x 4096, 1000
+        // tokens 49.2 -> 45.1; 4096 x 4096 with the residual 36.2 -> 32.8.
+        int finished = 0;
+        auto finish = [&]() {
+            const int n = finished++;
+            return t2_finish<EPI>(p, smem, tmem, pair + n * pairs, 0, (uint32_t)n & 1u, true);
+        };
         for (int st = group; st < stages; st += C::kGroups) {
             if (st >= slots && st < slots + C::kGroups) pdl_wait();
+            while (shared && ok && st >= (finished + 1) * G + slots) ok = finish();
+            if (!ok) break;
             if (!raw_ready && !tc2_wait(&raw_full[rs], rph, s_abort, p.err, 0x3600 + rs)) break;
             // looking at a barrier takes 200 cycles: they pass under the conversion
             const bool free = mbar_test(&ax_empty[as / SUB], ph ^ 1u);
@@ -263,7 +420,6 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
             const __half2 cz = __float2half2_rn(hi ? (float)(64 + (zz >> 4)) : (float)(1024 + (zz & 0xF)));
             const __half2 s2 = hi ? __half2half2(__high2half(sc2)) : __half2half2(__low2half(sc2));
             const uint32_t taddr = tlane + (uint32_t)(as * 64);
-            bool ok = true;
 #pragma unroll
             for (int ks = 0; ks < 2; ++ks) {    // 64 k at a time: 32 columns
                 uint4 wv[4];
@@ -310,37 +466,17 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
                 ph ^= 1u;
             }
         }
+        if (shared) {
+            pdl_wait();
+            while (ok && finished * G < stages) ok = finish();
+        }
     } else {
         int acc = 0;
         uint32_t acc_ph = 0;
         pdl_wait();
-        for (int i = pair; t2_tile(p, i, t); i += pairs) {
-            const int prow = t.n0 + (int)rank * 128 + q * 32 + lane;
-            const bool res = p.epi == ZL_EPI_RESIDUAL && p.wide && prow < p.N && splits == 1;
-            uint32_t rnext[8];
-            if (res) tc_fetch_residual(p, prow, lane, t.t0 + set * 16, rnext);
-            if (!tc2_wait(&acc_full[acc], acc_ph, s_abort, p.err, 0x3800 + acc)) break;
-            tc_fence_after();
-            if (splits > 1) break;
-            const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * 64);
-            if (prow < p.N) {               // N % 128 == 0: all of the CTA's rows or none
-                for (int c0 = set * 16; c0 < t.ntok && t.t0 + c0 < p.M; c0 += 32) {
-                    float v[16];
-                    tc_ld16(taddr + (uint32_t)c0, v);
-                    if (res) {
-                        uint32_t rcur[8];
-#pragma unroll
-                        for (int u = 0; u < 8; ++u) rcur[u] = rnext[u];
-                        if (c0 + 32 < t.ntok) tc_fetch_residual(p, prow, lane, t.t0 + c0 + 32, rnext);
-                        tc_epilogue16(p, prow, lane, t.t0 + c0, v, rcur);
-                    } else {
-                        tc_epilogue16(p, prow, lane, t.t0 + c0, v);
-                    }
-                }
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_at(cluster_map(smem_u32(&acc_empty[acc]), lead));
+        if (splits > 1 && t2_tile(p, pair, t)) tc2_wait(&acc_full[0], 0, s_abort, p.err, 0x3800);   // the rest comes behind the exchange
+        for (int i = pair; splits == 1 && t2_tile(p, i, t); i += pairs) {
+            if (!t2_finish<EPI>(p, smem, tmem, i, acc, acc_ph, shared)) break;
             if (++acc == nacc) {
                 acc = 0;
                 acc_ph ^= 1u;
@@ -356,11 +492,12 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
         tc_fence_after();
         const bool any = t2_tile(p, pair, t);
         const int row = q * 32 + lane, prow = t.n0 + (int)rank * 128 + row;
-        const bool epilogue = warp < C::kEpiWarps && any && prow < p.N;
+        const bool epilogue = warp < C::kWarpRaw && any && prow < p.N;   // the dequant warps too
+        constexpr int kSets = C::kWarpRaw / 4;
         const int chunks = min(t.ntok, p.M - t.t0 + 15) / 16;
         const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16);
         if (epilogue)
-            for (int c = set; c < chunks; c += 2) {
+            for (int c = set; c < chunks; c += kSets) {
                 if (c % splits == part) continue;
                 float v[16];
                 tc_ld16(taddr + (uint32_t)(c * 16), v);
@@ -368,11 +505,11 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
             }
         cluster_sync_all();
         if (epilogue)
-            for (int c = part + set * splits; c < chunks; c += 2 * splits) {
+            for (int c = part + set * splits; c < chunks; c += kSets * splits) {
                 float v[16];
                 tc_ld16(taddr + (uint32_t)(c * 16), v);
                 tc2_split_sum<false>(smem, part, c, splits, chunks, row, v);
-                tc_epilogue16(p, prow, lane, t.t0 + c * 16, v);
+                tc_epilogue16<EPI>(p, prow, lane, t.t0 + c * 16, v);
             }
         tc_fence_before();
         __syncthreads();
@@ -384,9 +521,22 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
 }
 
 // ---- host side --------------------------------------------------------------------------------------------------------
+// One instance per epilogue: all of them in one kernel, and the epilogue twice in it, cost instruction fetches that the conversion waits for
+typedef void (*T2Kernel)(W4TcParams);
+static T2Kernel t2_kernel(int sub, int epi) {
+    switch (epi) {
+        case ZL_EPI_SWIGLU: return sub == 2 ? k_w4a16_tc2<2, ZL_EPI_SWIGLU> : k_w4a16_tc2<1, ZL_EPI_SWIGLU>;
+        case ZL_EPI_RESIDUAL: return sub == 2 ? k_w4a16_tc2<2, ZL_EPI_RESIDUAL> : k_w4a16_tc2<1, ZL_EPI_RESIDUAL>;
+        case ZL_EPI_QKV_ROPE: return sub == 2 ? k_w4a16_tc2<2, ZL_EPI_QKV_ROPE> : k_w4a16_tc2<1, ZL_EPI_QKV_ROPE>;
+        default: return sub == 2 ? k_w4a16_tc2<2, ZL_EPI_NONE> : k_w4a16_tc2<1, ZL_EPI_NONE>;
+    }
+}
 cudaError_t prepare_w4_tc2() {
-    const cudaError_t e = cudaFuncSetAttribute(k_w4a16_tc2<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, T2Cfg::kBytes);
-    return e != cudaSuccess ? e : cudaFuncSetAttribute(k_w4a16_tc2<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, T2Cfg::kBytes);
+    cudaError_t e = cudaSuccess;
+    for (int epi = ZL_EPI_NONE; epi <= ZL_EPI_QKV_ROPE && e == cudaSuccess; ++epi)
+        for (int sub = 1; sub <= 2 && e == cudaSuccess; ++sub)
+            e = cudaFuncSetAttribute(t2_kernel(sub, epi), cudaFuncAttributeMaxDynamicSharedMemorySize, T2Cfg::kBytes);
+    return e;
 }
 
 // 128-k groups of a stage.  Handing a stage over costs the MMA warp 460 cycles whatever is in it, which is what bounded up to 128 tokens; of
@@ -400,27 +550,44 @@ static int t2_sub(int ntok) { return ntok <= 128 ? 2 : 1; }
 // token, a further wave less than that, since two accumulators (up to 64 tokens) or only the next tile's first groups hide the epilogue.
 // Measured, one pair / two / three, N x K, us: 4096 x 14336, 32 tokens 43 / 27 / 22.7, 96 tokens 45 / 31 / 24.7, 256 tokens 46.5 / 33 / -;
 // 4096 x 4096, 96 tokens 18.8 / 16.5 / 16.5, 128 tokens 19.7 / 16.5 / 18.2; 6144 x 4096, 64 tokens 19.0 / 16.5 / -; 8192 x 3584, 128 tokens
-// 19.7 / 18.6 / -.
+// 19.7 / 18.6 / -.  These are the times from before every warp helped with the epilogue; up to 256 rows they stand, since the line to the stream-k kernel
+// rests on them.  Beyond, fitted again to 56 sizes and their tiles (M = 320 .. 1000 of eight matrices; within 5 % where power is no limit): a group 0.35, or 0.08 +
+// 0.0021 per token above 128, start and end 9 + 0.01 per token, a further wave's end 1.5 + 0.01 per token (hidden up to 64).  There a last wave of few tiles
+// may also be cut in halves along its tokens: 28672 x 4096 is 448 tiles of 256 tokens at M = 1000, six waves and four tiles: 192 -> 184 us; M = 512 110 -> 103 (224
+// tiles, three waves and two); 16384 x 2048, M = 1000 67.8 -> 61.7.  Quarters: 184, 102 and 73, the conversion (0.4 a group) is the same for 64 tokens.
 struct T2Pick {
-    int ntok, splits;
+    int ntok, splits, cut;   // cut: 2: tiles of the last wave come in halves
     double us;
 };
 static int t2_clusters(int splits) {
     static PairsFit fit;
-    return pairs_clusters(k_w4a16_tc2<1>, T2Cfg::kThreads, T2Cfg::kBytes, splits, fit);
+    return pairs_clusters(k_w4a16_tc2<1, ZL_EPI_NONE>, T2Cfg::kThreads, T2Cfg::kBytes, splits, fit);
 }
 static T2Pick t2_pick(int M, int row_tiles, int G) {
     const int pairs = device_sm_count() / 2;
-    T2Pick best{32, 1, 1e30};
+    T2Pick best{32, 1, 1, 1e30};
     for (int n = 32; n <= 256; n += 32) {
         const long long tiles = (long long)row_tiles * cdiv(M, n), waves = (tiles + pairs - 1) / pairs;
-        const double group = n <= 128 ? fmax(0.31, 0.0022 * n) : fmax(0.00223 * n, 0.21 + 0.00137 * n);
-        const double further = (double)(waves - 1) * (n <= 64 ? 0.3 : n <= 128 ? 3.0 + 0.03 * n : 0.0074 * n);
         for (int s = 1; s <= 4; ++s) {
             const int sub = t2_sub(n), mine = cdiv(cdiv(G, sub), s) * sub;
             if (s > 1 && (cdiv(G, sub) < 2 * s || tiles * s > pairs || tiles > t2_clusters(s))) break;
-            const double us = 8.8 + 0.03 * n + (double)waves * mine * group + further + (s > 1 ? 1.2 + 0.01 * n : 0.0);
-            if (us < best.us - 1e-9) best = T2Pick{n, s, us};
+            const double exchange = s > 1 ? 1.2 + 0.01 * n : 0.0;
+            if (M <= 256) {
+                const double group = n <= 128 ? fmax(0.31, 0.0022 * n) : fmax(0.00223 * n, 0.21 + 0.00137 * n);
+                const double further = (double)(waves - 1) * (n <= 64 ? 0.3 : n <= 128 ? 3.0 + 0.03 * n : 0.0074 * n);
+                const double us = 8.8 + 0.03 * n + (double)waves * mine * group + further + exchange;
+                if (us < best.us - 1e-9) best = T2Pick{n, s, 1, us};
+                continue;
+            }
+            const long long whole = tiles / pairs, left = tiles % pairs;
+            auto group = [](int n) { return n <= 128 ? 0.35 : 0.08 + 0.0021 * n; };
+            const double wave = mine * group(n), end = n <= 64 ? 0.0 : 1.5 + 0.01 * n, us = 9.0 + 0.01 * n + exchange + (double)waves * wave + (double)(waves - 1) * end;
+            if (us < best.us - 1e-9) best = T2Pick{n, s, 1, us};
+            // the last wave's tiles in halves: one wave of them as well, none of them empty
+            if (s == 1 && whole > 0 && left > 0 && left * 2 <= pairs && n % 64 == 0 && (M - 1) % n + 1 > n / 2) {
+                const double shorter = us - wave + mine * fmax(0.4, group(n / 2));
+                if (shorter < best.us - 1e-9) best = T2Pick{n, 1, 2, shorter};
+            }
         }
         if (n >= M) break;
     }
@@ -458,13 +625,16 @@ cudaError_t launch_w4_tc2(const W4Params& p, bool pdl, cudaStream_t stream) {
     q.ntok = pick.ntok;
     q.splits = pick.splits;
     q.tok_tiles = cdiv(p.mc, q.ntok);
+    int tiles = row_tiles * q.tok_tiles;
+    q.cut = pick.cut;
+    q.whole = pick.cut > 1 ? tiles / max_pairs * max_pairs : tiles;
+    tiles = q.whole + (tiles - q.whole) * q.cut;
     {   // x as [K / 64][M][64]: a stage's atoms of half the tokens are one box
         const uint64_t dims[3] = {64, (uint64_t)p.mc, (uint64_t)p.K / 64}, strides[2] = {(uint64_t)p.ldx * 2, 128};
         const uint32_t box[3] = {64, (uint32_t)q.ntok / 2, (uint32_t)(2 * sub)};
         if (!tc_make_map_nd(&q.xmap, p.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B)) return cudaErrorInvalidValue;
     }
-    const int tiles = row_tiles * q.tok_tiles;
-    return launch_pairs(sub == 2 ? k_w4a16_tc2<2> : k_w4a16_tc2<1>, (tiles < max_pairs ? tiles : max_pairs) * q.splits, q.splits, dim3(T2Cfg::kThreads),
+    return launch_pairs(t2_kernel(sub, p.epi), (tiles < max_pairs ? tiles : max_pairs) * q.splits, q.splits, dim3(T2Cfg::kThreads),
                         (size_t)T2Cfg::kBytes, stream, pdl, q);
 }
 
@@ -479,6 +649,10 @@ extern "C" int zl_w4_pairs_rings(int ntok, int* slots, int* raw_slots) {
 
 extern "C" int zl_w4_pairs_splits(int M, int N, int K) {
     return zl_w4_pairs_route(M, N, K) ? zl::t2_pick(M, zl::cdiv(N, zl::kTc2Rows), K / zl::kW4GroupK).splits : 0;
+}
+
+extern "C" int zl_w4_pairs_pieces(int M, int N, int K) {
+    return zl_w4_pairs_route(M, N, K) ? zl::t2_pick(M, zl::cdiv(N, zl::kTc2Rows), K / zl::kW4GroupK).cut : 0;
 }
 
 extern "C" unsigned zl_w4_tc2_watchdog(void) {
