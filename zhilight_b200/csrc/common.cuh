@@ -87,6 +87,14 @@ __device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// A kernel that waits before it touches anything at all can always be launched as a programmatic dependent: its launch, barriers and allocations
+// run under the predecessor's end.  early: the caller's chain asks for more, what is constant is read ahead of the wait and dependents may start at
+// once.  Without, a dependent of that kind could read ahead of what this kernel's predecessors write: it starts behind the wait.
+__device__ __forceinline__ void pdl_start(bool early) {
+    if (!early) pdl_wait();
+    pdl_trigger();
+}
+
 // Launch helper: sets the PDL attribute when `pdl` is non-zero.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,

@@ -39,6 +39,7 @@ struct W4Params {
     int tp_mode = 0;
     int tp_index = 0;              // exchange index within the step (< 512): parity of the slot + part of the word tag
     __half* tp_h_out = nullptr;
+    int early = 0;                 // the caller's chain: see pdl_start
     int x32 = 0;                   // rows of x start on 32 bytes (set by launch_w4_v2_int_layout)
 };
 

@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(TsCfg<NTOK>::kThreads, 1) k_w4a16_ts(const __g
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "n"(512));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
-    pdl_trigger();
+    pdl_start(p.early);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -683,6 +683,7 @@ bool w4_tc_params(W4TcParams& q, const W4Params& p) {
     q.err = nullptr;
     q.ntok = q.tok_tiles = 0;
     q.splits = 1;
+    q.early = p.early;
     q.wide = ((reinterpret_cast<uintptr_t>(p.y) | reinterpret_cast<uintptr_t>(p.residual)) & 3) == 0;
     return true;
 }

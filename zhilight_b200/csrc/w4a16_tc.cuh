@@ -31,6 +31,7 @@ struct alignas(64) W4TcParams {
     int num_heads, num_kv_heads, dim_head;
     int ntok, tok_tiles;        // w4a16_tc2.cu: rows of x per tile, tiles along them
     int whole, cut;             // w4a16_tc2.cu: tiles from the `whole`-th on come in `cut` pieces of their rows of x
+    int early;                  // see pdl_start
     int splits;                 // w4a16_tc2.cu: pairs of a cluster that share a tile's K (then a tile per cluster)
     int wide;                   // two neighbouring values of y may be stored together
 };

@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(T2Cfg::kThreads, 1) k_w4a16_tc2(const __grid_c
         mbar_fence_init();
     }
     if (warp == C::kWarpMma) tc2_alloc(s_tmem);
-    pdl_trigger();
+    pdl_start(p.early);
     tc_fence_before();
     __syncthreads();
     cluster_sync_all();   // both CTAs' barriers and allocations are in place
