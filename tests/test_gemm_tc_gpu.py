@@ -152,6 +152,30 @@ def test_grouped(lib, cuda, dtype, sizes, n, k):
     _close(ops.gemm_nt_grouped(x, w, off, total, x_rows=rows), ref, mag, k, dtype)
 
 
+@pytest.mark.parametrize("dtype", [BF, HF])
+@pytest.mark.parametrize("sizes,n", [([40], 132), ([47], 130), ([257, 0, 300, 1], 516), ([16, 33, 500], 1026)])
+def test_gated_units_of_16_bits(lib, cuda, dtype, sizes, n):
+    """Two columns of a gated unit per store (n % 4 == 0) and one (n % 4 == 2); chunks of 16 rows with 1 to 16 in them, groups of several tiles.  Half a unit of the
+    output's last place, 2^-9 (2^-12) of a value on average, and what fp32 sums of values of about 1 lose."""
+    from zhilight_b200 import ops
+    g = torch.Generator().manual_seed(n)
+    total, k = sum(sizes), 576
+    x, w = _rand(g, total, k, dtype=dtype) / 8, _rand(g, len(sizes), n, k, dtype=dtype)
+    off = torch.tensor(np.concatenate([[0], np.cumsum(sizes)]), dtype=torch.int32, device="cuda")
+    back = torch.randperm(total, generator=g).to(torch.int32).cuda()
+    owner = torch.repeat_interleave(torch.arange(len(sizes)), torch.tensor(sizes)).cuda()
+    ref = torch.cat([x[owner == i].double() @ w[i].double().T for i in range(len(sizes))])
+    a, u = ref[:, 0::2].clamp(max=1.5), ref[:, 1::2].clamp(-1.5, 1.5)
+    want = a * torch.sigmoid(1.7 * a) * (u + 0.5)
+    tol = 2.0 ** (-8 if dtype == BF else -11)
+    rel = lambda y, want: float(((y.double() - want).norm(dim=1) / want.norm(dim=1)).max())  # noqa: E731
+    y = ops.gemm_nt_grouped(x, w, off, total, y_rows=back, epilogue=ops.GEMM_EPI_GLU_CLAMP, limit=1.5, alpha=1.7, beta=0.5)
+    assert rel(y[back.long()], want) < tol
+    if len(sizes) == 1:
+        assert rel(ops.gemm_nt_glu_clamp(x, w[0], None, dtype, 1.5, 1.7, 0.5), want) < tol
+        assert rel(ops.gemm_nt_fused(x, w[0], None, dtype, ops.GEMM_EPI_GEGLU_TANH), F.gelu(ref[:, 0::2], approximate="tanh") * ref[:, 1::2]) < tol
+
+
 @pytest.mark.parametrize("k", [128, 640])
 def test_infinities_stay_in_their_rows_and_columns(lib, cuda, k):
     from zhilight_b200 import ops

@@ -13,7 +13,7 @@
 //   warp 0       producer  : w and x boxes, one lane
 //   warp 1       MMA       : of the leader, one lane, 4 x 256 x ntok x 16 per 64-k block
 //   warp 2       TMEM allocation
-//   warps 4-11   epilogue  : quadrant = warp % 4, 16-row chunks of x in turns; lane = row of w = column of y
+//   warps 4-11   epilogue  : quadrant = warp % 4, 16-row chunks of x in turns; lane = row of w = column of y; of the last tile all warps
 //   warps 12-15  grouped   : rows of x through their index lists, by 16-byte cp.async into the swizzled layout that the boxes have;
 //                            a stage's barrier counts the copies as they land, warp 3 hands the stage to the MMAs
 //
@@ -30,11 +30,11 @@
 
 namespace zl {
 
-constexpr int kGtThreads = 12 * 32, kGtRowWarps = 4, kGtGroupThreads = kGtThreads + kGtRowWarps * 32, kGtEpiWarps = 8;
+constexpr int kGtThreads = 16 * 32, kGtRowWarps = 4, kGtEpiWarps = 8, kGtSets = 4;   // sets of four warps, one per quadrant of TMEM lanes
 // The ring is cut into as many stages as fit, of blocks of 16 KB of w and 128 bytes per row of a CTA's half tile of x.
 constexpr int kGtRing = 204800, kGtMaxStages = 12, kGtAStage = 128 * 128;
 constexpr int kGtBarOff = kGtRing;
-constexpr int kGtMiscOff = kGtBarOff + (3 * kGtMaxStages + 4) * 8;
+constexpr int kGtMiscOff = kGtBarOff + (3 * kGtMaxStages + 5) * 8;
 constexpr int kGtMaxGroups = 1024;
 constexpr int kGtCumOff = kGtMiscOff + 16;                       // grouped: tiles before each group
 constexpr int kGtBytes = kGtCumOff + (kGtMaxGroups + 1) * 4 + 1024;   // + slack for the manual 1024-byte alignment
@@ -91,12 +91,55 @@ __device__ __forceinline__ bool gt_tile(const GemmTcP& p, const int* s_cum, int 
     return true;
 }
 
-// 16 rows of y, column n of this lane; mine: row of y of token c0 + lane (grouped)
+// two values of a 16-bit type, the first one below
+template <typename TO>
+__device__ __forceinline__ uint32_t gt_pack2(float a, float b) {
+    if constexpr (std::is_same<TO, __half>::value) {
+        const __half2 h = __floats2half2_rn(a, b);
+        return *reinterpret_cast<const uint32_t*>(&h);
+    } else {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+        return *reinterpret_cast<const uint32_t*>(&h);
+    }
+}
+// own: two rows of y of this lane's column, other: of the neighbour's; the first row of both for the lane of the lower column, the second for the other's
+__device__ __forceinline__ uint32_t gt_trade(uint32_t own, uint32_t other, bool upper) { return __byte_perm(own, other, upper ? 0x3276 : 0x5410); }
+
+// 16 rows of y, column n of this lane; mine: row of y of token c0 + lane (grouped).  Two columns of every other token per lane (wide): half the stores, twice
+// as wide.  16-bit values travel in pairs and the last rows alone are looked at one by one: the instructions are what a tile's end takes, 1250 cycles a
+// chunk with a look, a conversion and a product of addresses for each value.
 template <typename TO>
 __device__ __forceinline__ void gt_put16(const GemmTcP& p, const GtTile& t, TO* y, int mine, int n, int c0, const float (&v)[16], int lane) {
     const GemmP& g = p.g;
     const int odd = lane & 1;
-    if (p.wide) {   // two columns of every other token per lane: half the stores, twice as wide
+    if (sizeof(TO) == 2 && p.wide) {
+        uint32_t w[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t own = gt_pack2<TO>(v[2 * j], v[2 * j + 1]);
+            w[j] = gt_trade(own, __shfl_xor_sync(0xffffffffu, own, 1), odd);
+        }
+        const int first = t.t0 + c0 + odd, left = n < g.N ? t.M - first : 0;   // N is even
+        TO* at = y + (n & ~1);
+        if (g.grp_off) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int row = __shfl_sync(0xffffffffu, mine, 2 * j + odd);
+                if (2 * j < left) *reinterpret_cast<uint32_t*>(at + (size_t)row * g.ldy) = w[j];
+            }
+        } else {
+            at += (size_t)first * g.ldy;
+            const size_t step = 2 * (size_t)g.ldy;
+            if (left >= 15) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j, at += step) *reinterpret_cast<uint32_t*>(at) = w[j];
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j, at += step)
+                    if (2 * j < left) *reinterpret_cast<uint32_t*>(at) = w[j];
+            }
+        }
+    } else if (p.wide) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const float other = __shfl_xor_sync(0xffffffffu, odd ? v[2 * j] : v[2 * j + 1], 1);
@@ -135,18 +178,30 @@ __device__ __forceinline__ void gt_store16(const GemmTcP& p, const GtTile& t, in
             const float other = __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, 1);
             v[j] = pair_unit<EPI>(odd ? other : a0, odd ? a1 : other, g);
         }
+        if (sizeof(TO) == 2 && p.wide) {   // two columns of every other one of its tokens per lane
+            const bool up = lane & 2;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int m = t.t0 + c0 + 2 * j + odd;
-            const int row = g.grp_off ? __shfl_sync(0xffffffffu, mine, 2 * j + odd) : m;
-            if ((n | 1) < g.N && m < t.M) y[(size_t)row * g.ldy + (n >> 1)] = from_f32<TO>(v[j]);
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t own = gt_pack2<TO>(v[2 * i], v[2 * i + 1]), w = gt_trade(own, __shfl_xor_sync(0xffffffffu, own, 2), up);
+                const int at = 4 * i + 2 * up + odd, m = t.t0 + c0 + at;
+                const int row = g.grp_off ? __shfl_sync(0xffffffffu, mine, at) : m;
+                if (n < g.N && m < t.M) *reinterpret_cast<uint32_t*>(y + (size_t)row * g.ldy + ((n >> 1) & ~1)) = w;   // N % 4 == 0
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int m = t.t0 + c0 + 2 * j + odd;
+                const int row = g.grp_off ? __shfl_sync(0xffffffffu, mine, 2 * j + odd) : m;
+                if ((n | 1) < g.N && m < t.M) y[(size_t)row * g.ldy + (n >> 1)] = from_f32<TO>(v[j]);
+            }
         }
     } else {
         // results first, stores behind them: the compiler cannot tell y from the gate's values
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const int m = t.t0 + c0 + i;
-            v[i] = m < t.M && n < g.N ? gemm_epilogue<EPI>(v[i] + bias, g, t.b, m, n) : 0.f;
+            constexpr bool kReads = EPI == ZL_GEMM_EPI_SIGMOID_GATE || EPI == ZL_GEMM_EPI_GELU_TANH_MUL;
+            v[i] = !kReads || (m < t.M && n < g.N) ? gemm_epilogue<EPI>(v[i] + bias, g, t.b, m, n) : 0.f;
         }
         gt_put16<TO>(p, t, y, mine, n, c0, v, lane);
     }
@@ -173,14 +228,15 @@ __device__ __forceinline__ void gt_store16_8bit(const GemmTcP& p, const GtTile& 
 }
 
 template <typename T, typename TO, bool GROUPED, int KIND, int SUB>
-__global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_gemm_tc(const __grid_constant__ GemmTcP p) {
+__global__ void __launch_bounds__(kGtThreads, 1) k_gemm_tc(const __grid_constant__ GemmTcP p) {
     extern __shared__ uint8_t smem_dyn[];
     uint8_t* smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + kGtBarOff);
     uint64_t* empty = full + kGtMaxStages;
     uint64_t* acc_full = empty + kGtMaxStages;
     uint64_t* acc_empty = acc_full + 2;
-    uint64_t* rows_full = acc_empty + 2;       // grouped: this CTA's rows of a stage have landed
+    uint64_t* last_full = acc_empty + 2;       // the pair's last tile
+    uint64_t* rows_full = last_full + 1;       // grouped: this CTA's rows of a stage have landed
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(smem + kGtMiscOff);
     volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
     int* s_cum = reinterpret_cast<int*>(smem + kGtCumOff);
@@ -205,6 +261,7 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
             mbar_init(&acc_full[i], 1);
             mbar_init(&acc_empty[i], 2 * kGtEpiWarps);
         }
+        mbar_init(last_full, 1);
         *s_abort = 0;
         mbar_fence_init();
     }
@@ -233,6 +290,7 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
     cluster_sync_all();   // both CTAs' barriers and allocations are in place
     tc_fence_after();
     const uint32_t tmem = *s_tmem;
+    const int total = GROUPED ? s_cum[p.groups] : p.row_tiles * p.tok_tiles * p.groups;
 
     // The three loops below are one lane's each: a vote or a look at a barrier costs the warp 100 - 200 cycles a stage, so each looks at its next
     // barrier while this stage's copies or MMAs are on their way
@@ -311,7 +369,7 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
                         }
                     }
                     tc2_commit(used, lead);
-                    if (k == ks - 1) tc2_commit(&acc_full[acc], lead);
+                    if (k == ks - 1) tc2_commit(i + pairs < total ? &acc_full[acc] : last_full, lead);
                 }
                 if (++acc == 2) {
                     acc = 0;
@@ -341,7 +399,7 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
                 }
         }
         __syncwarp();
-    } else if (GROUPED && warp >= 12) {
+    } else if (GROUPED && warp >= 4 + kGtEpiWarps) {
         // thread: 16-byte chunk c of rows j, j + 16, ... of the CTA's half
         const int tid = threadIdx.x - 12 * 32, c = tid & 7, j = tid >> 3;
         const uint32_t sm = smem_u32(smem) + kGtAStage + (uint32_t)(j * 128 + ((c ^ (j & 7)) << 4));
@@ -382,8 +440,10 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
     }
-    // epilogue warps; with K split a tile's only chunks come behind the exchange below
-    const int q = warp & 3, set = (warp - 4) >> 2;
+    // The epilogue warps' tiles.  The last one is everybody's: nothing is left to hide its end, and the other warps have nothing else to do.  With the shorter
+    // chunks of gt_put16, in a row of calls: bf16 8192 x 2048, 777 rows 31.3 -> 29.0 us; 16 experts of 2048 x 2048, 512 rows in four each: 127.5 -> 121.8;
+    // fp8 14336 x 4096, 500 rows 41.1 -> 39.6.  With K split a tile's only chunks come behind the exchange below.
+    const int q = warp & 3, set = ((warp >> 2) + kGtSets - 1) % kGtSets;   // 0, 1: the epilogue warps
     float bias = 0.f, s_w = 0.f;
     auto row_values = [&](const GtTile& t, int n) {
         bias = s_w = 0.f;
@@ -413,31 +473,29 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
             }
         }
     };
-    const bool epilogue = warp >= 4 && warp < 4 + kGtEpiWarps;
-    if (epilogue) {
+    {
         if (KIND != kGt16) pdl_wait();
-        int acc = 0, hint = 0;
-        uint32_t acc_ph = 0;
+        const int tiles = pair < total ? (total - pair + pairs - 1) / pairs : 0;
+        int hint = 0;
         GtTile t;
-        for (int i = pair; gt_tile<GROUPED>(p, s_cum, i, hint, t); i += pairs) {
-            if (!tc2_wait(&acc_full[acc], acc_ph, s_abort, p.err, 0x2800 + acc)) break;
+        for (int j = set < 2 ? 0 : tiles - 1; j >= 0 && j < tiles; ++j) {
+            const int acc = j & 1;
+            const bool last = j == tiles - 1;
+            gt_tile<GROUPED>(p, s_cum, pair + j * pairs, hint, t);
+            if (!tc2_wait(last ? last_full : &acc_full[acc], last ? 0u : (uint32_t)(j >> 1) & 1u, s_abort, p.err, 0x2800 + acc)) break;
             tc_fence_after();
             if (splits > 1) break;
-            const int n = t.n0 + (int)rank * 128 + q * 32 + lane;
+            const int n = t.n0 + (int)rank * 128 + q * 32 + lane, step = last ? 16 * kGtSets : 32;
             row_values(t, n);
             const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * 256);
-            for (int c0 = set * 16; c0 < t.ntok && t.t0 + c0 < t.M; c0 += 32) {
+            for (int c0 = set * 16; c0 < t.ntok && t.t0 + c0 < t.M; c0 += step) {
                 float v[16];
                 tc_ld16(taddr + (uint32_t)c0, v);
                 put(t, n, c0, v);
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_at(cluster_map(smem_u32(&acc_empty[acc]), lead));
-            if (++acc == 2) {
-                acc = 0;
-                acc_ph ^= 1u;
-            }
+            if (lane == 0 && !last) mbar_arrive_at(cluster_map(smem_u32(&acc_empty[acc]), lead));
         }
     }
     __syncwarp();
@@ -453,22 +511,19 @@ __global__ void __launch_bounds__(GROUPED ? kGtGroupThreads : kGtThreads, 1) k_g
         const int row = q * 32 + lane, n = t.n0 + (int)rank * 128 + row;
         const int chunks = any ? min(t.ntok, t.M - t.t0 + 15) / 16 : 0;
         const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16);
-        if (epilogue)
-            for (int c = set; c < chunks; c += 2) {
-                if (c % splits == part) continue;
-                float v[16];
-                tc_ld16(taddr + (uint32_t)(c * 16), v);
-                tc2_split_push(smem_u32(smem), (int)rank, part, c, splits, chunks, row, v);
-            }
+        for (int c = set; c < chunks; c += kGtSets) {
+            if (c % splits == part) continue;
+            float v[16];
+            tc_ld16(taddr + (uint32_t)(c * 16), v);
+            tc2_split_push(smem_u32(smem), (int)rank, part, c, splits, chunks, row, v);
+        }
         cluster_sync_all();
-        if (epilogue) {
-            row_values(t, n);
-            for (int c = part + set * splits; c < chunks; c += 2 * splits) {
-                float v[16];
-                tc_ld16(taddr + (uint32_t)(c * 16), v);
-                tc2_split_sum<KIND == kGtInt8>(smem, part, c, splits, chunks, row, v);
-                put(t, n, c * 16, v);
-            }
+        row_values(t, n);
+        for (int c = part + set * splits; c < chunks; c += kGtSets * splits) {
+            float v[16];
+            tc_ld16(taddr + (uint32_t)(c * 16), v);
+            tc2_split_sum<KIND == kGtInt8>(smem, part, c, splits, chunks, row, v);
+            put(t, n, c * 16, v);
         }
         tc_fence_before();
         __syncthreads();
@@ -548,7 +603,7 @@ static cudaError_t launch_gt_sub(const GemmTcP& q, int pairs, bool pdl, cudaStre
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) set[dev] = true;
     }
-    return launch_pairs(k_gemm_tc<T, TO, GROUPED, KIND, SUB>, pairs, q.splits, dim3(GROUPED ? kGtGroupThreads : kGtThreads), (size_t)kGtBytes, stream, pdl, q);
+    return launch_pairs(k_gemm_tc<T, TO, GROUPED, KIND, SUB>, pairs, q.splits, dim3(kGtThreads), (size_t)kGtBytes, stream, pdl, q);
 }
 template <typename T, typename TO, bool GROUPED, int KIND>
 static cudaError_t launch_gt(const GemmTcP& q, int pairs, bool pdl, cudaStream_t stream) {
@@ -580,7 +635,7 @@ static int gt_plan(GemmTcP& q, CUtensorMapDataType dt, int batch, int out_bytes)
     q.tok_tiles = 0;
     q.ntok = 256;
     q.splits = 1;
-    q.wide = p.N % 2 == 0 && p.ldy % 2 == 0 && p.yb % 2 == 0 && reinterpret_cast<uintptr_t>(p.y) % (2 * out_bytes) == 0;
+    q.wide = p.N % (epi_pairs(q.epi) ? 4 : 2) == 0 && p.ldy % 2 == 0 && p.yb % 2 == 0 && reinterpret_cast<uintptr_t>(p.y) % (2 * out_bytes) == 0;
     if (!tc2_map_3d(&q.wmap, p.w, dt, p.K, p.N, batch, p.ldw, p.wb, 128)) return 0;
     if (!grouped) {
         int fit[2];
