@@ -163,12 +163,11 @@ struct PaCfg {
     static constexpr int kTile = kAtoms * kPaKeys * 128;         // K or V: [64 of d][64 keys][128 B]
     static constexpr int kKOff = kQ, kVOff = kQ + 2 * kTile;
     static constexpr int kStaged = kQ + 4 * kTile;
-    static constexpr int kRow = D + 4;                           // merge: floats per row, 16-byte chunks of eight lanes on eight bank groups
-    static constexpr int kMl = kPaRows * kRow * 4;               // {maximum, sum} of a row behind the accumulators
-    static constexpr int kMerge = kMl + kPaRows * 8;
-    static constexpr int kUsed = (kStaged > kMerge ? kStaged : kMerge) + 1024;    // + slack for the manual 1024-byte alignment
+    static constexpr int kMl = kStaged;                          // merge: {maximum, sum}, then weight, of the rows of up to 8 key ranges
+    static constexpr int kUsed = kMl + 8 * kPaRows * 8 + 1024;   // + slack for the manual 1024-byte alignment
     static constexpr int kBytes = kHalfTmemSmem;                 // more than it uses, for the sake of tensor memory
     static_assert(kUsed <= kBytes, "shared memory");
+    static_assert(kPaRows * (D + 8 * 4) * 4 <= kStaged, "merge: [key range][row][D / ranges + 4] floats, where Q, K and V were");
     static constexpr int kS = 128;                               // TMEM columns: O 0 .. D - 1, S / P 128 .. 255 (two buffers of 64)
 };
 
@@ -452,73 +451,85 @@ k_attn_prompt(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* 
     }
     __syncwarp();
     tc2_drain(s_abort);
-    const int share = kPaRows / splits;   // rows that each CTA of the cluster finishes
     if (splits > 1) {
-        cluster_sync_all();               // nobody's Q, K and V are needed any more: their place takes the rows' results
+        // Each CTA of the cluster finishes its columns of all rows, thread = row as before: 128 threads each add what they hold in tensor memory to what the
+        // others sent.  Rows shared out instead, all columns through shared memory, took 10000 cycles behind the first barrier: 500 rows behind 1000 positions 36.8 us,
+        // 35.0 so.
+        const int cols = D / splits, pitch = cols + 4;           // pitch: 16-byte chunks of eight lanes on eight bank groups
+        const uint32_t ml = smem_u32(smem) + C::kMl + tid * 8;
+        if (warp < kPaWarpS)
+            for (int s = 0; s < splits; ++s) pa_st_cluster2(cluster_map(ml + split * (kPaRows * 8), s), make_float2(m_ref, l));
+        cluster_sync_all();               // nobody's Q, K and V are needed any more: their place takes the sums
+        const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
+        float2* const mine = reinterpret_cast<float2*>(smem + C::kMl) + tid;
         if (warp < kPaWarpS) {
-            const uint32_t at = smem_u32(smem) + (uint32_t)((split * share + tid % share) * C::kRow * 4);
-            const uint32_t dst = cluster_map(at, tid / share);
-            const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
             tc_fence_after();
 #pragma unroll
-            for (int d0 = 0; d0 < D; d0 += 64) {
-                uint32_t v[64];
+            for (int d0 = 0; d0 < D; d0 += 32) {
+                if (cols >= 32 && d0 / cols == split) continue;
+                uint32_t v[32];
                 pa_ld32(taddr + (uint32_t)d0, v);
-                pa_ld32(taddr + (uint32_t)(d0 + 32), v + 32);
                 pa_wait_ld();
 #pragma unroll
-                for (int i = 0; i < 64; i += 4)
-                    pa_st_cluster4(dst + (d0 + i) * 4, count > 0 ? make_uint4(v[i], v[i + 1], v[i + 2], v[i + 3]) : make_uint4(0u, 0u, 0u, 0u));
+                for (int i = 0; i < 32; i += 4) {
+                    const int to = (d0 + i) / cols, c = (d0 + i) % cols;
+                    if (to != split)
+                        pa_st_cluster4(cluster_map(smem_u32(smem) + ((split * kPaRows + tid) * pitch + c) * 4, to),
+                                       count > 0 ? make_uint4(v[i], v[i + 1], v[i + 2], v[i + 3]) : make_uint4(0u, 0u, 0u, 0u));
+                }
             }
-            pa_st_cluster2(cluster_map(smem_u32(smem) + C::kMl + (split * share + tid % share) * 8, tid / share), make_float2(m_ref, l));
+            // weights of the row's parts, in place of their maxima
+            float m = -INFINITY, sum = 0.f;
+            for (int s = 0; s < splits; ++s) m = fmaxf(m, mine[s * kPaRows].x);
+            for (int s = 0; s < splits; ++s) {
+                const float f = pa_exp2(mine[s * kPaRows].x - m);
+                sum = fmaf(mine[s * kPaRows].y, f, sum);
+                mine[s * kPaRows].x = f;
+            }
+            const float inv = 1.f / sum;
+            for (int s = 0; s < splits; ++s) mine[s * kPaRows].x *= inv;
         }
-        tc_fence_before();
         cluster_sync_all();
-    } else {
-        tc_fence_before();
-        __syncthreads();
+        if (warp < kPaWarpS) {
+            const int r = row0 + tid;
+            T* dst = out + (((size_t)b * len_q + r / m_query) * num_heads + hk * m_query + r % m_query) * D + split * cols;
+            for (int c0 = 0; c0 < cols; c0 += 16) {
+                float own[16], o[16] = {};
+                tc_ld16(taddr + (uint32_t)(split * cols + c0), own);   // of 8 columns the first half
+                for (int s = 0; s < splits; ++s) {
+                    const float f = mine[s * kPaRows].x;
+                    const float4* from = reinterpret_cast<const float4*>(smem + ((s * kPaRows + tid) * pitch + c0) * 4);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const float4 v = s != split ? from[u] : count > 0 ? make_float4(own[4 * u], own[4 * u + 1], own[4 * u + 2], own[4 * u + 3]) : float4{};
+                        o[4 * u] = fmaf(v.x, f, o[4 * u]), o[4 * u + 1] = fmaf(v.y, f, o[4 * u + 1]);
+                        o[4 * u + 2] = fmaf(v.z, f, o[4 * u + 2]), o[4 * u + 3] = fmaf(v.w, f, o[4 * u + 3]);
+                    }
+                }
+#pragma unroll
+                for (int h = 0; h < 16; h += 8) {
+                    if (r >= rows || c0 + h >= cols) continue;
+                    uint32_t w[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        T two[2] = {from_f32<T>(o[h + 2 * i]), from_f32<T>(o[h + 2 * i + 1])};
+                        w[i] = *reinterpret_cast<const uint32_t*>(two);
+                    }
+                    if (aligned) {
+                        *reinterpret_cast<uint4*>(dst + c0 + h) = make_uint4(w[0], w[1], w[2], w[3]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) reinterpret_cast<uint32_t*>(dst + c0 + h)[i] = w[i];
+                    }
+                }
+            }
+        }
     }
+    tc_fence_before();
+    __syncthreads();
     if (warp == kPaWarpO) {
         tc_fence_after();
         pa_dealloc(tmem);
-    }
-    if (splits > 1) {
-        if (tid < share) {                // weights of a row's parts, in place of their maxima and sums
-            float2* ml = reinterpret_cast<float2*>(smem + C::kMl) + tid;
-            float m = -INFINITY, sum = 0.f;
-            for (int s = 0; s < splits; ++s) m = fmaxf(m, ml[s * share].x);
-            for (int s = 0; s < splits; ++s) {
-                const float f = pa_exp2(ml[s * share].x - m);
-                sum = fmaf(ml[s * share].y, f, sum);
-                ml[s * share].x = f;
-            }
-            const float inv = 1.f / sum;
-            for (int s = 0; s < splits; ++s) ml[s * share].x *= inv;
-        }
-        __syncthreads();
-        constexpr int kLanes = D / 4, kPer = kPaThreads / kLanes;   // threads of a row, rows at a time
-        const int d0 = (tid % kLanes) * 4;
-        const unsigned first = row0 + split * share;
-#pragma unroll 4
-        for (int rr = tid / kLanes; rr < share; rr += kPer) {
-            float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int s = 0; s < splits; ++s) {
-                const float4 v = *reinterpret_cast<const float4*>(smem + ((s * share + rr) * C::kRow + d0) * 4);
-                const float f = *reinterpret_cast<const float*>(smem + C::kMl + (s * share + rr) * 8);
-                o.x = fmaf(v.x, f, o.x), o.y = fmaf(v.y, f, o.y), o.z = fmaf(v.z, f, o.z), o.w = fmaf(v.w, f, o.w);
-            }
-            const unsigned r = first + rr, qi = r / (unsigned)m_query;
-            if (r >= (unsigned)rows) continue;
-            T w[4] = {from_f32<T>(o.x), from_f32<T>(o.y), from_f32<T>(o.z), from_f32<T>(o.w)};
-            T* dst = out + (((size_t)b * len_q + qi) * num_heads + hk * m_query + (r - qi * m_query)) * D + d0;
-            const uint2 two = make_uint2(reinterpret_cast<const uint32_t*>(w)[0], reinterpret_cast<const uint32_t*>(w)[1]);
-            if (aligned) {
-                *reinterpret_cast<uint2*>(dst) = two;
-            } else {
-                reinterpret_cast<uint32_t*>(dst)[0] = two.x;
-                reinterpret_cast<uint32_t*>(dst)[1] = two.y;
-            }
-        }
     }
 }
 
