@@ -479,6 +479,8 @@ int zl_gemm_nt_grouped(const void* x, long long ldx, const int32_t* x_rows, cons
                        long long w_group_stride, void* y, long long ldy, const int32_t* y_rows, const int32_t* group_offsets,
                        int groups, int max_rows, int N, int K, int in_dtype, int out_dtype, int epilogue, float limit,
                        float alpha, float beta, int pdl, zl_stream_t stream);
+/* zeroes the rows of y (rows x row_bytes, contiguous) that no entry of that list lands on; y_rows null: entry e lands on row e */
+int zl_clear_unlisted_rows(void* y, long long row_bytes, int rows, const int32_t* y_rows, const int32_t* group_offsets, int groups, int pdl, zl_stream_t stream);
 /* One problem with the clamped gated unit over column pairs and a per-column fp32 bias (NULL: none; 2 entries per output
  * column, added before the unit): y (M, N / 2) = g sigmoid(alpha g) (u + beta), g = min(gate, limit), u = clamp(up, +-limit). */
 int zl_gemm_nt_glu_clamp(const void* x, long long ldx, const void* w, long long ldw, const float* bias, void* y, long long ldy,

@@ -176,6 +176,26 @@ def test_gated_units_of_16_bits(lib, cuda, dtype, sizes, n):
         assert rel(ops.gemm_nt_fused(x, w[0], None, dtype, ops.GEMM_EPI_GEGLU_TANH), F.gelu(ref[:, 0::2], approximate="tanh") * ref[:, 1::2]) < tol
 
 
+@pytest.mark.parametrize("rows_out,listed,n,out", [(33, 20, 512, BF), (4000, 3990, 512, torch.float32), (4111, 0, 256, torch.float32), (4100, 4100, 520, HF), (2600, 30, 1030, BF)])
+def test_rows_that_no_entry_lands_on(lib, cuda, rows_out, listed, n, out):
+    """They are zeros, whatever the memory held: few, most, none and all rows listed, slices of the last partial one, rows of no multiple of 16 bytes, an output
+    so small that it is written whole first; with and without a list of y's rows."""
+    from zhilight_b200 import ops
+    g = torch.Generator().manual_seed(rows_out)
+    k = 128
+    dtype = BF if out == torch.float32 else out
+    x, w = _rand(g, max(listed, 1), k, dtype=dtype), _rand(g, 3, n, k, dtype=dtype)
+    off = torch.tensor([0, listed // 3, listed // 2, listed], dtype=torch.int32, device="cuda")
+    rows = torch.arange(max(listed, 1), dtype=torch.int32, device="cuda")
+    for back in (None, torch.randperm(rows_out, generator=g)[:max(listed, 1)].to(torch.int32).cuda()):
+        junk = torch.full((rows_out, n), float("nan"), dtype=out, device=cuda)
+        del junk                                        # the allocator's next block of this size
+        y = ops.gemm_nt_grouped(x, w, off, rows_out, x_rows=rows, y_rows=back, out_dtype=out)
+        free = torch.ones(rows_out, dtype=torch.bool, device=cuda)
+        free[(rows if back is None else back.long())[:listed]] = False
+        assert int(free.sum()) == rows_out - listed and not y[free].any() and (listed == 0 or bool((y[~free].abs().sum(1) > 0).all()))
+
+
 @pytest.mark.parametrize("k", [128, 640])
 def test_infinities_stay_in_their_rows_and_columns(lib, cuda, k):
     from zhilight_b200 import ops

@@ -643,3 +643,49 @@ extern "C" int zl_gemm_nt_grouped(const void* x, long long ldx, const int32_t* x
     p.beta = beta;
     return gemm_dispatch(p, groups, in_dtype, out_dtype, epilogue, pdl, stream);
 }
+
+// Rows of y that no entry of a grouped product's list lands on become zeros; the others are left to the product.  A block finds the rows of its slice in the
+// list, so it is bound by that walk.  Against writing all of y, us in a row of calls: 2048 rows of 4 KB 1.9 / 2.8, of 8 KB 2.0 / 4.9, of 1 KB 2.0 / 1.4; 32768 of
+// 1 KB 4.7 / 9.1; 64 of 4 KB 1.4 / 1.1; and the product behind it starts under its end.
+namespace zl {
+constexpr int kClearRows = 4096, kClearThreads = 1024;
+__global__ void __launch_bounds__(kClearThreads) k_clear_unlisted(uint8_t* y, long long row_bytes, int rows, int slice, const int32_t* __restrict__ y_rows,
+                                                                  const int32_t* __restrict__ group_offsets, int groups, int early) {
+    __shared__ uint32_t listed[kClearRows / 32];
+    pdl_start(early);
+    pdl_wait();
+    const int r0 = blockIdx.x * slice, n = min(slice, rows - r0);
+    const int first = group_offsets[0], last = group_offsets[groups];
+    for (int i = threadIdx.x; i < (n + 31) / 32; i += kClearThreads) listed[i] = 0;
+    __syncthreads();
+    if (y_rows) {
+#pragma unroll 4
+        for (int e = first + (int)threadIdx.x; e < last; e += kClearThreads) {
+            const int r = y_rows[e] - r0;
+            if (r >= 0 && r < n) atomicOr(&listed[r >> 5], 1u << (r & 31));
+        }
+        __syncthreads();
+    }
+    for (int w = threadIdx.x >> 5; w < n; w += kClearThreads / 32) {
+        if (y_rows ? (listed[w >> 5] >> (w & 31)) & 1 : r0 + w >= first && r0 + w < last) continue;
+        uint8_t* row = y + (size_t)(r0 + w) * row_bytes;
+        const int lane = threadIdx.x & 31;
+        if ((reinterpret_cast<uintptr_t>(row) | row_bytes) & 15)
+            for (long long i = lane; i < row_bytes / 2; i += 32) reinterpret_cast<uint16_t*>(row)[i] = 0;
+        else
+            for (long long i = lane; i < row_bytes / 16; i += 32) reinterpret_cast<uint4*>(row)[i] = make_uint4(0, 0, 0, 0);
+    }
+}
+}  // namespace zl
+
+extern "C" int zl_clear_unlisted_rows(void* y, long long row_bytes, int rows, const int32_t* y_rows, const int32_t* group_offsets, int groups, int pdl,
+                                      zl_stream_t stream) {
+    ZL_CHECK_ARG(y && row_bytes > 0 && row_bytes % 2 == 0 && rows > 0 && group_offsets && groups > 0);
+    ZL_CHECK_ARG((reinterpret_cast<uintptr_t>(y) & 1) == 0);
+    const int sms = device_sm_count();
+    int slice = cdiv(rows, sms) < 32 ? 32 : cdiv(rows, sms);
+    if (slice > kClearRows) slice = kClearRows;
+    ZL_CHECK_CUDA(launch(k_clear_unlisted, dim3(cdiv(rows, slice)), dim3(kClearThreads), 0, stream, true, static_cast<uint8_t*>(y), row_bytes, rows, slice, y_rows,
+                         group_offsets, groups, pdl));
+    return ZL_OK;
+}

@@ -572,8 +572,12 @@ def gemm_nt_grouped(x, w, group_offsets, rows_out, x_rows=None, y_rows=None, out
     sorted by group; y has `rows_out` rows of N (N / 2 with the gated-unit epilogue) columns, zero where nothing lands."""
     g, n, k = w.shape
     n_out = n // 2 if epilogue == GEMM_EPI_GLU_CLAMP else n
-    y = torch.zeros((rows_out, n_out), dtype=out_dtype or x.dtype, device=x.device)
+    row_bytes = n_out * (out_dtype or x.dtype).itemsize
+    scan = row_bytes >= 1024 and row_bytes * rows_out >= 4 << 20      # below, writing every row is as fast as looking them up (k_clear_unlisted)
+    y = (torch.empty if scan else torch.zeros)((rows_out, n_out), dtype=out_dtype or x.dtype, device=x.device)
     total = (x_rows if x_rows is not None else y_rows if y_rows is not None else x).shape[0]
+    if scan:
+        _lib.call("zl_clear_unlisted_rows", _p(y), row_bytes, rows_out, _p(y_rows), _p(group_offsets), g, 0, _stream())
     _lib.call("zl_gemm_nt_grouped", _p(x), x.shape[1], _p(x_rows), _p(w), k, n * k, _p(y), n_out, _p(y_rows), _p(group_offsets),
               g, total, n, k, _dt(x), _dt(y), epilogue, limit, alpha, beta, 0, _stream())
     return y
