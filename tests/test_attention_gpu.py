@@ -76,3 +76,17 @@ def test_fully_masked_row_is_zero_not_nan(lib, cuda):
     mask = torch.zeros(32, dtype=torch.int8, device=cuda)
     out = ops.decode_attention(q, torch.tensor([32], dtype=torch.int32, device=cuda), k, v, mask, 0.125, 32, 1)
     assert torch.isfinite(out).all() and out.abs().max() < 1e-6     # sum seeded with 1e-20 (attention_kernel.cu:466)
+
+
+@pytest.mark.parametrize("dtype,name,tol", [(torch.float16, "f16", 1e-3), (torch.bfloat16, "bf16", 6e-3)])
+@pytest.mark.parametrize("hq,hkv,d,longest,tasks", [(8, 2, 128, 700, 3), (4, 4, 64, 257, 2), (8, 1, 128, 2048, 2), (16, 8, 128, 2000, 2), (16, 2, 128, 1000, 4),   # 256-key CTAs: 3, 2, 8, 8, 4 splits
+                                                    (8, 4, 128, 4096, 32), (8, 4, 128, 4096, 40), (16, 8, 128, 1100, 40), (8, 8, 64, 1030, 40),
+                                                    (16, 16, 64, 2900, 24)])                                             # 1024-key CTAs: 4, 4, 2, 2, 3
+def test_splits_that_merge_in_a_cluster(lib, cuda, dtype, name, tol, hq, hkv, d, longest, tasks):
+    """Both sides of the lines to the merge in a launch of its own and to three CTAs per SM; splits without a key, heads of a partial group."""
+    lens = ([longest, 1, 17, longest // 4 + 1] + [40 + i for i in range(tasks)])[:tasks]
+    for masked in (True, False):
+        out, ref = _case(cuda, dtype, name, hq, hkv, d, lens, masked=masked, seed=6)
+        for b in range(min(tasks, 6)):
+            assert rel_l2(out[b], ref[b]) <= 2 * tol, b
+        assert rel_l2(out, ref) <= tol

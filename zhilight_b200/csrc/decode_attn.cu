@@ -26,8 +26,9 @@ constexpr int kAttnMaxRange = 1024;            // keys per CTA; logits live in s
 constexpr int kAttnRowStride = kAttnMaxRange + 4;
 constexpr int kAttnMaxSplits = 64;
 
-template <typename T, int D, bool PV_FP32>
-__global__ void __launch_bounds__(kAttnThreads)
+// PER_SM: CTAs of an SM at least; up to 168 (3) or 128 registers (4)
+template <typename T, int D, bool PV_FP32, int PER_SM>
+__global__ void __launch_bounds__(kAttnThreads, PER_SM)
 k_decode_attn(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* const* __restrict__ k_addrs,
               T* const* __restrict__ v_addrs, const int8_t* __restrict__ mask, float scale,
               T* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_m,
@@ -264,6 +265,8 @@ k_decode_attn(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* 
         }
     }
     __syncthreads();
+    float* s_all = s_red + kAttnWarps * 8 * D;   // the CTA's results, for the others of a cluster
+    static_assert((kAttnWarps + 1) * 8 * D <= 8 * kAttnRowStride, "shared memory");
     for (int e = tid; e < mq * D; e += kAttnThreads) {
         const int h = e / D, d = e % D;
         float v = 0.f;
@@ -273,6 +276,8 @@ k_decode_attn(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* 
         const size_t vh = (size_t)bq * num_heads + head0 + h;
         if (num_splits == 1) {
             out[vh * D + d] = from_f32<T>(v);
+        } else if (!part_o) {
+            s_all[e] = v;
         } else {
             part_o[(vh * num_splits + split) * D + d] = v;
             if (d == 0) {
@@ -281,6 +286,8 @@ k_decode_attn(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* 
             }
         }
     }
+    if (num_splits > 1 && !part_o)   // the splits are a cluster
+        attn_merge_cluster<T, D, kAttnThreads>(s_all, s_m, s_l, num_splits, split, mq, out + ((size_t)bq * num_heads + head0) * D);
 }
 
 
@@ -333,6 +340,27 @@ __global__ void k_attn_combine(const float* __restrict__ part_o, const float* __
         res += part_o[((size_t)vh * num_splits + i) * D + d] * w;
     }
     out[(size_t)vh * D + d] = from_f32<T>(res);
+}
+
+// grid.x, the key splits of a head group, as a cluster or not
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_splits(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool pdl, bool cluster, Args... args) {
+    if (!cluster) return launch(kernel, grid, block, smem, stream, pdl, args...);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = grid.x;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 2 : 1;
+    zl_count_launch();
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
 static int attn_num_splits(int B, int len_q, int num_kv_heads, int m_query, int max_len_buf) {
@@ -478,6 +506,21 @@ extern "C" int zl_decode_attention(const void* q, const int32_t* buf_lens, void*
     if (splits > 1) {
         const size_t need = vheads * splits * (dim_head + 2) * sizeof(float);
         ZL_CHECK_ARG(workspace != nullptr && workspace_bytes >= need);
+    }
+    static const bool old_short = getenv("ZL_ATTN_OLD_SHORT") != nullptr;
+    static const bool pv_fp32 = getenv("ZL_ATTN_PV_FP32") != nullptr;
+    // The splits of a head group as a cluster, which merges their results (attn_merge_cluster), or through the workspace and a second launch.  us, launch / cluster,
+    // 32 heads on 8, D = 128, fp16: 256-key CTAs on an SM each 8 x 300 10.0 / 8.4, 4 x 1000 11.3 / 9.0, 1 x 2000 12.1 / 9.4; more of them than SMs come and go
+    // by whole clusters: 12 x 300 14.5 / 14.7, 32 x 300 26.0 / 28.9, 8 x 2000 29.0 / 40.6; 16 clusters of eight find no room at once: 2 x 2000 12.7 / 16.4.  1024-key CTAs: 16 x 4096 43.9 / 40.9, 32 x 1500 34.5 / 32.0,
+    // 32 x 4096 66.0 / 64.6; against it three splits 51.5 / 52.3 (32 x 3000), eight 20.5 / 27.2 (32 x 2048, 8 heads on 1), 2048 CTAs 73.6 / 75.4 (32 x 4096, 16 on 16, D = 64).
+    const int sms = device_sm_count();
+    const long long ctas = (long long)splits * num_kv_heads * hg0 * B * len_q;
+    const bool cluster = splits > 1 && !(use_short && old_short) &&
+                         (use_short ? splits <= kAttnClusterSplits && ctas <= (splits <= 4 ? sms : sms / 2) : (splits == 2 || splits == 4) && ctas <= 8ll * sms);
+    // What four CTAs per SM hold in one wave goes three at a time: the places of short sequences are taken again.  us, four / three: 16 x 4096 40.8 / 40.4 (bf16 43.8 /
+    // 41.9), 32 x 2048 40.9 / 38.3, 16 x 1500 17.9 / 17.0; against it 32 x 4096 (1024 CTAs) 64.6 / 74.9, and 32 x 700 14.7 / 18.6, whose keys come from L2.
+    const bool three = dim_head == 128 && ctas <= 4ll * sms && max_len_buf >= 400 * splits;
+    if (splits > 1 && !cluster) {
         part_o = static_cast<float*>(workspace);
         part_m = part_o + vheads * splits * dim_head;
         part_l = part_m + vheads * splits;
@@ -486,13 +529,11 @@ extern "C" int zl_decode_attention(const void* q, const int32_t* buf_lens, void*
     dim3 grid(splits, num_kv_heads * hgroups, B * len_q), block(kAttnThreads);
     // default for the latency regime: the warp-per-32-keys kernel (one __syncthreads per CTA); ZL_ATTN_OLD_SHORT=1 keeps the
     // previous 512-thread short kernel for A/B measurements
-    static const bool old_short = getenv("ZL_ATTN_OLD_SHORT") != nullptr;
-    static const bool pv_fp32 = getenv("ZL_ATTN_PV_FP32") != nullptr;
     const bool use_warp = use_short && !old_short;
 #define ZL_ATTN_LAUNCH(TT, DD)                                                                                  \
     if (use_warp) {                                                                                             \
-        ZL_CHECK_CUDA(launch(k_decode_attn_warp<TT, DD>, grid, dim3(kWarpAttnWarps * 32),                       \
-                             (size_t)warp_attn_smem_floats<DD>() * sizeof(float), stream, pdl != 0, (const TT*)q, \
+        ZL_CHECK_CUDA(launch_splits(k_decode_attn_warp<TT, DD>, grid, dim3(kWarpAttnWarps * 32),                \
+                             (size_t)warp_attn_smem_floats<DD>() * sizeof(float), stream, pdl != 0, cluster, (const TT*)q, \
                              buf_lens, (TT* const*)k_addrs, (TT* const*)v_addrs, mask, scale, (TT*)out, part_o, \
                              part_m, part_l, len_q, num_heads, num_kv_heads, m_query, splits, bshd));            \
     } else if (use_short) {                                                                                     \
@@ -509,15 +550,15 @@ extern "C" int zl_decode_attention(const void* q, const int32_t* buf_lens, void*
                              num_heads, num_kv_heads, m_query, splits, bshd, g_attn_pf_ptr, g_attn_pf_bytes));                                  \
     } else                                                                                                      \
     if (pv_fp32) {                                                                                              \
-        ZL_CHECK_CUDA(launch(k_decode_attn<TT, DD, true>, grid, block, 0, stream, pdl != 0, (const TT*)q, buf_lens, \
+        ZL_CHECK_CUDA(launch_splits(k_decode_attn<TT, DD, true, 4>, grid, block, 0, stream, pdl != 0, cluster, (const TT*)q, buf_lens, \
                              (TT* const*)k_addrs, (TT* const*)v_addrs, mask, scale, (TT*)out, part_o, part_m,   \
                              part_l, len_q, num_heads, num_kv_heads, m_query, splits, bshd, g_attn_pf_ptr,      \
                              g_attn_pf_bytes));                                                                 \
     } else                                                                                                      \
-    ZL_CHECK_CUDA(launch(k_decode_attn<TT, DD, false>, grid, block, 0, stream, pdl != 0, (const TT*)q, buf_lens, \
+    ZL_CHECK_CUDA(launch_splits(three ? k_decode_attn<TT, DD, false, DD == 128 ? 3 : 4> : k_decode_attn<TT, DD, false, 4>, grid, block, 0, stream, pdl != 0, cluster, (const TT*)q, buf_lens, \
                          (TT* const*)k_addrs, (TT* const*)v_addrs, mask, scale, (TT*)out, part_o, part_m,       \
                          part_l, len_q, num_heads, num_kv_heads, m_query, splits, bshd, g_attn_pf_ptr, g_attn_pf_bytes)); \
-    if (splits > 1)                                                                                             \
+    if (part_o)                                                                                                 \
         ZL_CHECK_CUDA(launch(k_attn_combine<TT>, dim3((unsigned)vheads), dim3(DD), 0, stream, pdl != 0,         \
                              (const float*)part_o, (const float*)part_m, (const float*)part_l, (TT*)out, splits));
     if (dtype == ZL_F16) {

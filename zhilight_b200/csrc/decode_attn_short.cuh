@@ -3,6 +3,7 @@
 // 512 threads; every global load of the item is issued before the first dependent instruction.
 #pragma once
 #include "common.cuh"
+#include "tc2_common.cuh"
 
 namespace zl {
 
@@ -204,6 +205,43 @@ __device__ __forceinline__ void attn_short_item(const T* __restrict__ q, const i
             }
         }
     }
+}
+
+// Up to this many key splits of a head group are one cluster and merge their results themselves; the portable size of a cluster.
+constexpr int kAttnClusterSplits = 8;
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
+// The splits' results, o (mq, D) and the heads' maxima and sums at the same places of every CTA's shared memory, merged by the rule of k_attn_combine: each
+// CTA takes every splits-th THREADS values.  out: the group's first row.  It stands in for a second launch where that is the slower (zl_decode_attention).
+template <typename T, int D, int THREADS>
+__device__ __forceinline__ void attn_merge_cluster(const float* o, const float* m, const float* l, int splits, int split, int mq, T* out) {
+    cluster_sync_all();   // every CTA's results are in place
+    const uint32_t o_at = smem_u32(o), m_at = smem_u32(m), l_at = smem_u32(l);
+    for (int e = (int)threadIdx.x + split * THREADS; e < mq * D; e += splits * THREADS) {
+        const int h = e / D;
+        float pm[kAttnClusterSplits], pl[kAttnClusterSplits], po[kAttnClusterSplits], gm = -1e20f, gs = 0.f, res = 0.f;
+#pragma unroll
+        for (int i = 0; i < kAttnClusterSplits; ++i) {
+            if (i >= splits) continue;
+            pm[i] = ld_cluster_f32(cluster_map(m_at + h * 4, i));
+            pl[i] = ld_cluster_f32(cluster_map(l_at + h * 4, i));
+            po[i] = ld_cluster_f32(cluster_map(o_at + e * 4, i));
+        }
+#pragma unroll
+        for (int i = 0; i < kAttnClusterSplits; ++i)
+            if (i < splits) gm = fmaxf(gm, pm[i]);
+#pragma unroll
+        for (int i = 0; i < kAttnClusterSplits; ++i)
+            if (i < splits) gs += pl[i] * expf(pm[i] - gm);
+#pragma unroll
+        for (int i = 0; i < kAttnClusterSplits; ++i)
+            if (i < splits) res += po[i] * (pl[i] / gs * expf(pm[i] - gm));
+        out[e] = from_f32<T>(res);
+    }
+    cluster_sync_all();   // nobody's shared memory goes while another CTA may still read it
 }
 
 }  // namespace zl

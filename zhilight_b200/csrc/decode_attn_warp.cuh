@@ -17,7 +17,7 @@ constexpr int kWarpAttnWarps = 8;
 constexpr int kWarpAttnRange = kWarpAttnWarps * 32;   // keys per CTA
 
 template <int D>
-constexpr int warp_attn_smem_floats() { return kWarpAttnWarps * (32 * 8 + 8 * D + 16); }   // per warp: P[32][8], o[8][D], m[8], l[8]
+constexpr int warp_attn_smem_floats() { return kWarpAttnWarps * (32 * 8 + 8 * D + 16) + 8 * D + 16; }   // per warp: P[32][8], o[8][D], m[8], l[8]; the CTA's o, m, l
 
 template <typename T, int D>
 __global__ void __launch_bounds__(kWarpAttnWarps * 32)
@@ -193,6 +193,7 @@ k_decode_attn_warp(const T* __restrict__ q, const int32_t* __restrict__ buf_lens
     __syncthreads();
     // ---- merge the warps (KERNEL_mqa_combine rule) ----
     constexpr int WS = 32 * 8 + 8 * D + 16;
+    float* s_all = s_dyn + kWarpAttnWarps * WS;
     for (int e = tid; e < mq * D; e += kWarpAttnWarps * 32) {
         const int h = e / D, d = e % D;
         float gm = -1e20f;
@@ -209,6 +210,9 @@ k_decode_attn_warp(const T* __restrict__ q, const int32_t* __restrict__ buf_lens
         const size_t vh = (size_t)bq * num_heads + head0 + h;
         if (num_splits == 1) {
             out[vh * D + d] = from_f32<T>(v);
+        } else if (!part_o) {
+            s_all[e] = v;
+            if (d == 0) s_all[8 * D + h] = gm, s_all[8 * D + 8 + h] = gl;
         } else {
             part_o[(vh * num_splits + split) * D + d] = v;
             if (d == 0) {
@@ -217,6 +221,8 @@ k_decode_attn_warp(const T* __restrict__ q, const int32_t* __restrict__ buf_lens
             }
         }
     }
+    if (num_splits > 1 && !part_o)   // the splits are a cluster
+        attn_merge_cluster<T, D, kWarpAttnWarps * 32>(s_all, s_all + 8 * D, s_all + 8 * D + 8, num_splits, split, mq, out + ((size_t)bq * num_heads + head0) * D);
 }
 
 }  // namespace zl

@@ -95,6 +95,8 @@ struct Words256 {
     unsigned long long w[256];
 };
 __global__ void k_write_words(const __grid_constant__ Words256 words, unsigned long long* dst, int n) {
+    pdl_start(false);
+    pdl_wait();
     if (threadIdx.x < n) dst[threadIdx.x] = words.w[threadIdx.x];
 }
 
@@ -246,7 +248,7 @@ extern "C" int zl_write_pointers(void* dst, const void* pointers, int n, zl_stre
         Words256 w;
         memcpy(w.w, static_cast<const unsigned long long*>(pointers) + i, (size_t)c * 8);
         memset(w.w + c, 0, (size_t)(256 - c) * 8);
-        ZL_CHECK_CUDA(launch(k_write_words, dim3(1), dim3(256), 0, stream, false, w, static_cast<unsigned long long*>(dst) + i, c));
+        ZL_CHECK_CUDA(launch(k_write_words, dim3(1), dim3(256), 0, stream, true, w, static_cast<unsigned long long*>(dst) + i, c));
     }
     return ZL_OK;
 }
