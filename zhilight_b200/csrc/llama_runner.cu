@@ -82,6 +82,11 @@ struct zl_llama {
     cudaEvent_t ring_ev[kStageSlots] = {};
     bool ring_used[kStageSlots] = {};
     int ring_next = 0;
+    // logits on their way to the caller's memory: a ring of pinned pieces
+    static constexpr int kOutPieces = 4;
+    static constexpr size_t kOutPiece = 256 << 10;
+    char* h_out = nullptr;        // pinned [kOutPieces][kOutPiece]
+    cudaEvent_t out_ev[kOutPieces] = {};
     // prefill keeps its own (token, position) arrays: the decode-state arrays d_tokens / d_pos of tasks 0..B-1 survive a
     // prefill that happens between two zl_llama_step_device calls (continuous batching)
     int32_t *d_pf_tokens = nullptr, *d_pf_pos = nullptr;
@@ -580,6 +585,8 @@ int alloc_runtime(zl_llama* m) {
     ZL_CHECK_CUDA(cudaMallocHost((void**)&m->h_ring, sizeof(int32_t) * zl_llama::kStageSlots * 2 * B));
     for (int i = 0; i < zl_llama::kStageSlots; ++i)
         ZL_CHECK_CUDA(cudaEventCreateWithFlags(&m->ring_ev[i], cudaEventDisableTiming));
+    ZL_CHECK_CUDA(cudaMallocHost((void**)&m->h_out, zl_llama::kOutPieces * zl_llama::kOutPiece));
+    for (int i = 0; i < zl_llama::kOutPieces; ++i) ZL_CHECK_CUDA(cudaEventCreateWithFlags(&m->out_ev[i], cudaEventDisableTiming));
     ZL_SYNC(m->stream);
     return ZL_OK;
 }
@@ -1119,7 +1126,10 @@ extern "C" void zl_llama_destroy(zl_llama_t* m) {
     }
     if (m->h_stage) cudaFreeHost(m->h_stage);
     if (m->h_ring) cudaFreeHost(m->h_ring);
+    if (m->h_out) cudaFreeHost(m->h_out);
     for (cudaEvent_t e : m->ring_ev)
+        if (e) cudaEventDestroy(e);
+    for (cudaEvent_t e : m->out_ev)
         if (e) cudaEventDestroy(e);
     for (void* p : {(void*)m->d_pf_tokens, (void*)m->d_pf_pos})
         if (p) cudaFree(p);
@@ -1282,15 +1292,41 @@ extern "C" int zl_llama_step_device(zl_llama_t* m, int B) {
     return ZL_OK;
 }
 
+// The step's logits to the caller's memory.  Pageable memory is filled piece by piece behind copies to pinned pieces: 512 KB take 40 us beside the step so, 47 when the
+// runtime stages the copy (a step of four users over 32000 words: 233.2 -> 227.8 us).
+static int read_logits(zl_llama* m, float* dst, size_t count) {
+    cudaPointerAttributes at = {};
+    const bool pinned = cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type != cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    const size_t bytes = count * sizeof(float), piece = zl_llama::kOutPiece;
+    if (pinned) {
+        ZL_CHECK_CUDA(cudaMemcpyAsync(dst, m->logits, bytes, cudaMemcpyDeviceToHost, m->stream));
+        return ZL_OK;
+    }
+    const int n = (int)((bytes + piece - 1) / piece);
+    auto part = [&](int i) { return i + 1 < n ? piece : bytes - (size_t)i * piece; };
+    for (int i = 0; i < n + zl_llama::kOutPieces; ++i) {
+        const int slot = i % zl_llama::kOutPieces, done = i - zl_llama::kOutPieces;
+        char* const at_host = m->h_out + slot * piece;
+        if (done >= 0 && done < n) {
+            ZL_CHECK_CUDA(cudaEventSynchronize(m->out_ev[slot]));
+            memcpy(reinterpret_cast<char*>(dst) + (size_t)done * piece, at_host, part(done));
+        }
+        if (i < n) {
+            ZL_CHECK_CUDA(cudaMemcpyAsync(at_host, reinterpret_cast<const char*>(m->logits) + (size_t)i * piece, part(i), cudaMemcpyDeviceToHost, m->stream));
+            ZL_CHECK_CUDA(cudaEventRecord(m->out_ev[slot], m->stream));
+        }
+    }
+    return ZL_OK;
+}
+
 extern "C" int zl_llama_decode(zl_llama_t* m, const int32_t* tokens_host, const int32_t* positions_host, int B,
                                int32_t* next_tokens_host, float* logits_host) {
     ZL_CHECK_ARG(next_tokens_host != nullptr);
     RCHECK(zl_llama_set_state(m, tokens_host, positions_host, B));
     RCHECK(run_step(m, B));
     ZL_CHECK_CUDA(cudaMemcpyAsync(m->h_stage + 3 * B, m->d_next, B * 4, cudaMemcpyDeviceToHost, m->stream));
-    if (logits_host)   // (B, vocab/tp) of this rank's shard
-        ZL_CHECK_CUDA(cudaMemcpyAsync(logits_host, m->logits, (size_t)B * m->vshard * 4, cudaMemcpyDeviceToHost,
-                                      m->stream));
+    if (logits_host) RCHECK(read_logits(m, logits_host, (size_t)B * m->vshard));   // (B, vocab/tp) of this rank's shard
     ZL_SYNC(m->stream);
     for (int i = 0; i < B; ++i) next_tokens_host[i] = m->h_stage[3 * B + i];
     return ZL_OK;
@@ -1405,8 +1441,7 @@ extern "C" int zl_llama_prefill(zl_llama_t* m, int task, const int32_t* tokens_h
         RCHECK(enqueue_step(m, 1, 0, &pc));
     }
     ZL_CHECK_CUDA(cudaMemcpyAsync(m->h_stage + 3 * m->cfg.max_batch, m->d_next, 4, cudaMemcpyDeviceToHost, m->stream));
-    if (logits_host)
-        ZL_CHECK_CUDA(cudaMemcpyAsync(logits_host, m->logits, (size_t)m->vshard * 4, cudaMemcpyDeviceToHost, m->stream));
+    if (logits_host) RCHECK(read_logits(m, logits_host, m->vshard));
     ZL_SYNC(m->stream);
     *next_token_host = m->h_stage[3 * m->cfg.max_batch];
     if (pos0 + n > m->cur_max_len) m->cur_max_len = pos0 + n;

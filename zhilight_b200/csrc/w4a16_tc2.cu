@@ -607,6 +607,18 @@ bool w4_tc2_route(int M, int N, int K) {
     if (M <= 16 || N % kTcRows || K % kW4GroupK) return false;
     if (M > 256) return true;
     const int G = K / kW4GroupK;
+    // Both as they are since each starts under its predecessor's end: here 5.8 us, 0.34 a group of a wave and 1.5 for sums that meet; there 10 us and 0.156 (up to
+    // 32 rows) or 11.5 and 0.17 per million weights.  Measured in a row of calls, there / here, 32 and 40 rows, N x K: 14336 x 4096 19.6 / 16.7 and 21.8 / 17.4; 8192 x 8192
+    // 19.7 / 18.2 and 23.1 / 18.7; 8192 x 4096 14.8 / 12.9 and 18.0 / 13.4; 5120 x 5120 16.7 / 14.2 and 17.8 / 14.8; 16384 x 2048 15.8 / 11.5 and 17.7 / 12.1; a feed-forward of
+    // 2048 and 8192 35.5 / 28.4 and 35.4 / 27.7; not 10240 x 8192 23.4 / 28.0 and 25.9 / 28.8 (40 pairs of 74 work), 22016 x 4096 24.2 / 27.3 and 27.0 / 28.1 (a second
+    // wave of 12).  Where they are closer, and below 26 million weights, the older estimates below decide.
+    const double weights = 1e-6 * N * K;
+    if (M <= 64 && weights >= 26.0) {
+        const T2Pick pick = t2_pick(M, cdiv(N, kTc2Rows), G);
+        const int pairs = device_sm_count() / 2, sub = t2_sub(pick.ntok), mine = cdiv(cdiv(G, sub), pick.splits) * sub;
+        const double here = 5.8 + 0.34 * mine * cdiv(cdiv(N, kTc2Rows) * cdiv(M, pick.ntok), pairs) + (pick.splits > 1 ? 1.5 : 0.0);
+        if (M <= 32 ? here < 0.9 * (10.0 + 0.156 * weights) : here < 0.85 * (11.5 + 0.17 * weights)) return true;
+    }
     const double there = (10.0 + 4.2e-9 * M * (double)N * K) * (M > 64 && N >= 4096 ? 1.25 : 1.0);
     const bool cut = M > 32 && (long long)(N / kTcRows) * G < 8 * device_sm_count();
     return t2_pick(M, cdiv(N, kTc2Rows), G).us < there + (!cut ? 0.0 : K < 4096 ? 0.1 * M : N >= 1024 ? 0.015 * M : 0.0);
