@@ -454,29 +454,33 @@ k_attn_prompt(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* 
     if (splits > 1) {
         // Each CTA of the cluster finishes its columns of all rows, thread = row as before: 128 threads each add what they hold in tensor memory to what the
         // others sent.  Rows shared out instead, all columns through shared memory, took 10000 cycles behind the first barrier: 500 rows behind 1000 positions 36.8 us,
-        // 35.0 so.
-        const int cols = D / splits, pitch = cols + 4;           // pitch: 16-byte chunks of eight lanes on eight bank groups
+        // 35.0 so; and with each CTA beginning at another one of the cluster 76 x 1100 (four ranges) 19.6 -> 17.7.
+        const int cols = D / splits, sh = 31 - __clz(cols), pitch = cols + 4;   // splits: a power of two; pitch: 16-byte chunks of eight lanes on eight bank groups
         const uint32_t ml = smem_u32(smem) + C::kMl + tid * 8;
         if (warp < kPaWarpS)
             for (int s = 0; s < splits; ++s) pa_st_cluster2(cluster_map(ml + split * (kPaRows * 8), s), make_float2(m_ref, l));
         cluster_sync_all();               // nobody's Q, K and V are needed any more: their place takes the sums
         const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
         float2* const mine = reinterpret_cast<float2*>(smem + C::kMl) + tid;
+        const uint32_t place = smem_u32(smem) + (split * kPaRows + tid) * pitch * 4;
         if (warp < kPaWarpS) {
             tc_fence_after();
-#pragma unroll
-            for (int d0 = 0; d0 < D; d0 += 32) {
-                if (cols >= 32 && d0 / cols == split) continue;
-                uint32_t v[32];
-                pa_ld32(taddr + (uint32_t)d0, v);
+            const int first = ((split + 1) << sh) & ~31;          // each CTA begins with another one's columns
+#pragma unroll 1
+            for (int d = 0; d < D; d += 64) {
+                uint32_t v[64];
+                const int d1 = (first + d) & (D - 1), d2 = (first + d + 32) & (D - 1);
+                pa_ld32(taddr + (uint32_t)d1, v);
+                pa_ld32(taddr + (uint32_t)d2, v + 32);
                 pa_wait_ld();
 #pragma unroll
-                for (int i = 0; i < 32; i += 4) {
-                    const int to = (d0 + i) / cols, c = (d0 + i) % cols;
+                for (int i = 0; i < 64; i += 4) {
+                    const int at = (i < 32 ? d1 : d2) + (i & 31), to = at >> sh;
                     if (to != split)
-                        pa_st_cluster4(cluster_map(smem_u32(smem) + ((split * kPaRows + tid) * pitch + c) * 4, to),
+                        pa_st_cluster4(cluster_map(place + (at & (cols - 1)) * 4, to),
                                        count > 0 ? make_uint4(v[i], v[i + 1], v[i + 2], v[i + 3]) : make_uint4(0u, 0u, 0u, 0u));
                 }
+                if (cols == 64 && D == 128) break;               // of two CTAs the other half is this one's own
             }
             // weights of the row's parts, in place of their maxima
             float m = -INFINITY, sum = 0.f;
@@ -496,6 +500,7 @@ k_attn_prompt(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* 
             for (int c0 = 0; c0 < cols; c0 += 16) {
                 float own[16], o[16] = {};
                 tc_ld16(taddr + (uint32_t)(split * cols + c0), own);   // of 8 columns the first half
+#pragma unroll 2
                 for (int s = 0; s < splits; ++s) {
                     const float f = mine[s * kPaRows].x;
                     const float4* from = reinterpret_cast<const float4*>(smem + ((s * kPaRows + tid) * pitch + c0) * 4);
@@ -534,14 +539,15 @@ k_attn_prompt(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* 
 }
 
 // Key splits (CTAs of a cluster) of a launch of `ctas` row blocks over up to `tiles` key tiles.  A tile is about 1 us of a CTA's chain, being a
-// cluster 3 us, so four tiles stay whole (256 x 256, 32 heads on 8: 12.6 against 14.5 us in two) and further ones are cut down to two a CTA:
-// 32 x 1100 15.8 us in eight, 18.2 in four.  Two CTAs share an SM, but larger clusters then wait for room: beyond one CTA per SM only pairs
-// (256 x 1300, 16 heads on 4: 19.9 us in four, 23.9 in eight; 128 x 600, 64 on 8: 19.0 in two, 21.0 in four).
+// cluster 2 us, so few tiles stay whole (256 x 256, 32 heads on 8: 12.1 against 12.5 us in two), more of them where two CTAs would share an SM (512 x 512 17.2 / 18.9,
+// against it 512 x 1024 27.3 / 25.4), and further ones are cut down to two a CTA: 76 x 1100 28.7 us whole, 21.3 in two, 17.7 in four; 200 x 900, 8 on 1, 15.6 in four,
+// 14.1 in eight.  Larger clusters wait for room (16 of eight: 100 x 800, 16 on 4, 17.5 us, in four 15.2): beyond one CTA per SM only pairs (256 x 1300, 16 heads on 4: 18.3 us in four, 23.3 in eight; 128 x 600, 64 on 8:
+// 16.8 in two, 20.7 in four).
 inline int prompt_attn_splits(long long ctas, int tiles) {
     const int sms = device_sm_count();
     int s = 1;
-    if (tiles >= 8 && ctas * 2 <= 2ll * sms) s = 2;
-    while (s > 1 && s < 8 && tiles >= 4 * s && ctas * s * 2 <= sms) s *= 2;
+    if (tiles >= (ctas * 2 <= sms ? 8 : 12) && ctas * 2 <= 2ll * sms) s = 2;
+    while (s > 1 && s < 8 && tiles >= (s == 2 ? 8 : 12) && ctas * s * 2 <= (s == 2 ? sms : sms * 3 / 4)) s *= 2;
     return s;
 }
 
