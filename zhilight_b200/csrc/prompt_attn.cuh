@@ -20,12 +20,13 @@
 // Two CTAs share an SM (256 columns each): one's MMAs run under the other's softmax.  Bound by the chain S -> softmax -> P of a tile: 512 rows over 4096
 // keys, 64 heads on 8, take 114 us alone, 3700 cycles for a tile of each of the SM's two CTAs, whose MMAs take 2060 (each: 450 of S, whose operands come
 // at 128 bytes a cycle, and 580 of P V); at 500 rows behind 1000 positions, 32 on 8, 33 us, the tensor pipe is busy for 20 % of the time and 30 % of the
-// issue slots are taken.  Short prompts are a chain of about 10 us besides (launch, mask, first loads, merge).  500 rows behind 1000 positions, bf16, all launches
-// of the call: 65 us on mma.sync with 64-row blocks, 34 here; 512 x 1500 with 64 heads on 8: 120 -> 49.
+// issue slots are taken: of 52000 cycles 5000 until the first tile, 31000 of tiles, 15500 of the merge before its columns were shared out.  One buffer of scores and
+// one of probabilities, so that the next scores come under the softmax, is slower (34.7 against 33.5 us): P V then waits behind them.  500 rows behind 1000
+// positions, bf16, all launches of the call: 65 us on mma.sync with 64-row blocks, 33 here; 512 x 1500 with 64 heads on 8: 120 -> 48.
 //
 // An int8 mask is turned into bits first (k_mask_bits), once for all kv heads, together with each row's last visible key: tiles behind the last
 // key any row of the block sees are never loaded, which halves a causal prompt's work.  Few blocks are cut along their keys: the CTAs of a
-// cluster take a range each and push their rows' O, maximum and sum into the shared memory of the CTA that finishes the row.
+// cluster take a range each and push their O, maximum and sum into the shared memory of the CTAs that finish these columns.
 //
 // Nothing waits for ever: see tc2_common.cuh.  The waits begin behind the launch dependency.
 #pragma once

@@ -6,10 +6,10 @@
 // cutting the tiles into one range per CTA makes two of a CTA's two or three pieces partial ones that travel through L2 as tagged
 // words.  Here
 //   * a tile is 256 rows of w by up to 256 tokens over two SMs: each converts its own 128 rows and loads half of the tokens;
-//   * tiles are taken whole, in turn by persistent pairs; the token tile's size is chosen so that the last wave is full;
-//   * up to 64 tokens there are two accumulators; with one, eight epilogue warps shorten the gap.
-// 28672 x 4096 with SwiGLU: 1000 tokens 499 -> 190 us, 256 tokens 128 -> 60; 4096 x 14336 with the residual: 1000 tokens 408 -> 88 us
-// (1360 TFLOP/s).  Bound by the tensor cores at 256 tokens (1084 cycles per 128-k group, at the clock that the power limit leaves); below 130
+//   * tiles are taken whole, in turn by persistent pairs; the token tile's size is chosen so that the last wave is full, or its tiles come in halves;
+//   * up to 64 tokens there are two accumulators; with one, the epilogue and the dequant warps shorten the gap together (t2_finish).
+// 28672 x 4096 with SwiGLU: 1000 tokens 499 -> 180 us (cuBLAS fp16 170), 256 tokens 128 -> 55; 4096 x 14336 with the residual: 1000 tokens 408 -> 90 us
+// (1300 TFLOP/s).  Bound by the tensor cores at 256 tokens (1084 cycles per 128-k group, at the clock that the power limit leaves); below 130
 // tokens by the conversion (0.31 us of a group, about 600 cycles; 340 when nothing else runs on the SM).
 //
 // What a stage costs one thread is what bounded small tiles before that (830 cycles): looking at a barrier takes it 120 - 200 cycles even when the
@@ -19,7 +19,7 @@
 // 4096 x 14336, 256 rows 53.9 -> 45.4 us, 512 rows 55.9 -> 49.2; 28672 x 4096, 64 rows 36 -> 32; 6144 x 4096, 96 rows 22.4 -> 18.9.
 // Few tiles: the pairs of a cluster share a tile's K (t2_pick).
 //
-//   warps 0-7    epilogue : quadrant = warp % 4, 16-token chunks in turns
+//   warps 0-7    epilogue : quadrant = warp % 4, 16-token chunks in turns, above 64 tokens shared with the dequant warps
 //   warps 8-23   dequant  : four groups of four warps take the 128-k groups in turn, one per slot of A; lane = weight row, quadrant =
 //                           warp % 4; their arrivals of both CTAs for a stage meet on the leader's barrier
 //   warps 24, 25 weights  : tensor-TMA of the 4 ZLW4I records of a stage and their trailers, this CTA's 128 rows, stages in turn
