@@ -290,6 +290,10 @@ int zl_decode_attention(const void* q, const int32_t* buf_lens, void* const* k_a
                         const int8_t* mask, float scale, int max_len_buf, void* out, int B, int len_q,
                         int num_heads, int num_kv_heads, int dim_head, int bshd, void* workspace,
                         size_t workspace_bytes, int dtype, int pdl, zl_stream_t stream);
+/* the same behind everything earlier on the stream, with the addresses in host memory, B of K and B of V; table: device, room for them */
+int zl_decode_attention_host(const void* q, const int32_t* buf_lens, const void* addrs, void* table, const int8_t* mask, float scale, int max_len_buf, void* out,
+                             int B, int len_q, int num_heads, int num_kv_heads, int dim_head, int bshd, void* workspace, size_t workspace_bytes, int dtype,
+                             zl_stream_t stream);
 
 /* int8 KV cache (KV_CACHE_DTYPE=int8 of the reference): KERNEL_mqa_rag_buffer_split_kv_quant
  * (src/nn/attention/attention_kernel.cu:804-880, src/nn/attention/quant_attention.cuh:10-123).  K / V buffers per task are

@@ -90,3 +90,36 @@ def test_splits_that_merge_in_a_cluster(lib, cuda, dtype, name, tol, hq, hkv, d,
         for b in range(min(tasks, 6)):
             assert rel_l2(out[b], ref[b]) <= 2 * tol, b
         assert rel_l2(out, ref) <= tol
+
+
+@pytest.mark.parametrize("tasks,len_q,hq,hkv,longest", [(1, 1, 8, 2, 300), (2, 20, 8, 2, 200), (1, 150, 8, 2, 150), (1, 40, 32, 4, 700), (32, 1, 4, 1, 40), (33, 1, 4, 1, 40),
+                                                        (20, 1, 8, 8, 900)])
+@pytest.mark.parametrize("masked", [True, False])
+def test_addresses_from_the_host(lib, cuda, tasks, len_q, hq, hkv, longest, masked):
+    """With the call's first kernel (up to 32 tasks and a CTA per SM) and through a table the call writes: the same bits as through a table of the caller's, in a
+    row of calls on changing buffers."""
+    from zhilight_b200 import _lib, ops
+    d = 128
+    g = torch.Generator().manual_seed(tasks)
+    lens = [max(len_q, longest - 7 * i) for i in range(tasks)]
+    n = torch.tensor(lens, dtype=torch.int32, device=cuda)
+    mask = torch.cat([(torch.rand(len_q, m, generator=g) < 0.7).to(torch.int8).reshape(-1) for m in lens]).to(cuda) if masked else None
+    ws_bytes = lib.zl_decode_attention_workspace_bytes(tasks, len_q, hq, d, longest)
+    ws = torch.empty(ws_bytes + 16, dtype=torch.uint8, device=cuda)
+    stream = torch.cuda.current_stream().cuda_stream
+    got, want = [], []
+    for turn in range(3):
+        q = torch.randn(tasks, len_q, hq, d, generator=g).half().to(cuda)
+        kv = [torch.randn(m, hkv, d, generator=g).half().to(cuda) for m in lens + lens]
+        addrs = torch.tensor([t.data_ptr() for t in kv], dtype=torch.int64)
+        for own in (False, True):
+            out, table = torch.full_like(q, float("nan")), torch.empty(2 * tasks, dtype=torch.int64, device=cuda)
+            args = (mask.data_ptr() if masked else None, d ** -0.5, longest, out.data_ptr(), tasks, len_q, hq, hkv, d, 1, ws.data_ptr(), ws_bytes, ops.F16)
+            if own:
+                table.copy_(addrs)
+                _lib.call("zl_decode_attention", q.data_ptr(), n.data_ptr(), table.data_ptr(), table.data_ptr() + 8 * tasks, *args, 0, stream)
+            else:
+                _lib.call("zl_decode_attention_host", q.data_ptr(), n.data_ptr(), addrs.data_ptr(), table.data_ptr(), *args, stream)
+            (want if own else got).append(out)
+        torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(got, want)) and not any(torch.isnan(a).any() for a in got)

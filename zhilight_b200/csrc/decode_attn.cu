@@ -33,7 +33,7 @@ k_decode_attn(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* 
               T* const* __restrict__ v_addrs, const int8_t* __restrict__ mask, float scale,
               T* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_m,
               float* __restrict__ part_l, int len_q, int num_heads, int num_kv_heads, int m_query,
-              int num_splits, int bshd, const uint8_t* __restrict__ pf_ptr, unsigned long long pf_bytes) {
+              int num_splits, int bshd, const uint8_t* __restrict__ pf_ptr, unsigned long long pf_bytes, const __grid_constant__ AttnAddrs inl) {
     constexpr int NI = D / 32;                 // 16-byte chunks per lane per key row
     constexpr int DC = D / 8;                  // threads covering one V row
     constexpr int NSUB = kAttnThreads / DC;    // key subsets in the PV phase
@@ -50,7 +50,7 @@ k_decode_attn(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* 
     const int mq = min(8, m_query - mq0);
     const int head0 = hk * m_query + mq0;
 
-    pdl_trigger();
+    pdl_start(!inl.behind);
     // attention barely touches HBM at small batch: use the time to pull a later GEMM's weights into L2
     if (pf_ptr) {
         const int n_cta = gridDim.x * gridDim.y * gridDim.z;
@@ -68,8 +68,8 @@ k_decode_attn(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* 
 
     const size_t stride = bshd ? (size_t)num_kv_heads * D : (size_t)D;
     const size_t base = bshd ? (size_t)hk * D : (size_t)hk * len_buf * D;
-    const T* kbase = k_addrs[b] + base;
-    const T* vbase = v_addrs[b] + base;
+    const T* kbase = attn_addr(inl, k_addrs, b, false) + base;
+    const T* vbase = attn_addr(inl, v_addrs, b, true) + base;
 
     const int8_t* mrow = nullptr;
     if (mask) {
@@ -436,10 +436,34 @@ static bool prompt_route(int len_q, int m_query, int dim_head, int B, int num_kv
     return !mask || (workspace && prompt_head_bytes(B, len_q, max_len_buf, mask) <= workspace_bytes && len_q <= 65535);
 }
 
+// Addresses of the caches that a caller holds on the host: B of K, then B of V; table: room for them on the device.
+struct HostAddrs {
+    const void* addrs;   // null: the tables are the caller's
+    void* table;
+};
+// They travel with the call's first kernel, `ctas` of them, which is then a programmatic dependent behind everything earlier, or a launch before it writes the table,
+// behind everything earlier as well, so that the attention may start under its end.  Up to one CTA per SM the launch of 1.3 us is saved: us in a row of calls, table /
+// inline, 32 heads on 8: 4 x 300 9.2 / 8.3, 2 x 17 8.2 / 6.1, a portion of 33 behind 567 14.4 / 13.7 (in a graph).  More CTAs come while the kernel before ends are placed where it
+// ends first, several on an SM, and stay there: 16 x 4096 with heads of 64 21.6 / 27.2, 500 behind 1000 32.9 / 33.5; as plain launches 32.9 / 34.6.
+static int attn_addresses(const HostAddrs& host, int B, long long ctas, bool only_tables, AttnAddrs& inl, void* const*& k_addrs, void* const*& v_addrs, int& pdl,
+                          zl_stream_t stream) {
+    if (!host.addrs) return ZL_OK;
+    pdl = 1;
+    if (B <= kAttnInline && ctas <= device_sm_count() && !only_tables) {
+        for (int i = 0; i < 2 * B; ++i) inl.p[i] = static_cast<const void* const*>(host.addrs)[i];
+        inl.n = B;
+        inl.behind = 1;
+        return ZL_OK;
+    }
+    k_addrs = static_cast<void* const*>(host.table);
+    v_addrs = k_addrs + B;
+    return zl_write_pointers(host.table, host.addrs, 2 * B, stream);
+}
+
 template <typename T, int D>
 static int prompt_attention(const void* q, const int32_t* buf_lens, void* const* k_addrs, void* const* v_addrs, const int8_t* mask, float scale,
                             int max_len_buf, void* out, int B, int len_q, int num_heads, int num_kv_heads, int bshd, void* workspace,
-                            size_t workspace_bytes, int pdl, bool mask_ready, zl_stream_t stream) {
+                            size_t workspace_bytes, int pdl, bool mask_ready, const HostAddrs& host, zl_stream_t stream) {
     const int m_query = num_heads / num_kv_heads;
     const int blocks = cdiv(len_q * m_query, kPaRows), tiles = cdiv(max_len_buf, kPaKeys);
     const int splits = prompt_attn_splits((long long)blocks * num_kv_heads * B, tiles);
@@ -457,26 +481,29 @@ static int prompt_attention(const void* q, const int32_t* buf_lens, void* const*
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
     const bool mask_pass = mask && !mask_ready;
+    AttnAddrs inl = {};
+    const int rc = attn_addresses(host, B, mask_pass ? (long long)len_q * B : (long long)blocks * num_kv_heads * B * splits, false, inl, k_addrs, v_addrs, pdl, stream);
+    if (rc) return rc;
     if (mask_pass)
-        ZL_CHECK_CUDA(launch(k_mask_bits, dim3(len_q, B), dim3(256), 0, stream, pdl != 0, mask, buf_lens, bits, last, len_q, tiles));
+        ZL_CHECK_CUDA(launch(k_mask_bits, dim3(len_q, B), dim3(256), 0, stream, pdl != 0, mask, buf_lens, bits, last, len_q, tiles, inl.behind));
+    AttnAddrs own = inl;
+    own.behind = inl.behind && !mask_pass;
     const int aligned = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
     // behind the mask's kernel the attention may start early whatever the caller's chain allows: it waits for that kernel to end
     ZL_CHECK_CUDA((launch_attn_prompt<T, D>(dim3(blocks, num_kv_heads, B * splits), splits, stream, pdl != 0 || mask_pass, (const T*)q, buf_lens,
                                             (T* const*)k_addrs, (T* const*)v_addrs, (const uint64_t*)bits, (const int32_t*)last, tiles, scale,
-                                            (T*)out, len_q, num_heads, num_kv_heads, m_query, splits, bshd, aligned, words + kWaitAttnPrompt)));
+                                            (T*)out, len_q, num_heads, num_kv_heads, m_query, splits, bshd, aligned, words + kWaitAttnPrompt, own)));
     g_attn_pf_ptr = nullptr;
     g_attn_pf_bytes = 0;
     return ZL_OK;
 }
 
-extern "C" int zl_decode_attention(const void* q, const int32_t* buf_lens, void* const* k_addrs,
-                                   void* const* v_addrs, const int8_t* mask, float scale, int max_len_buf,
-                                   void* out, int B, int len_q, int num_heads, int num_kv_heads, int dim_head,
-                                   int bshd, void* workspace, size_t workspace_bytes, int dtype, int pdl,
-                                   zl_stream_t stream) {
+static int attention(const void* q, const int32_t* buf_lens, void* const* k_addrs, void* const* v_addrs, const HostAddrs& host, const int8_t* mask, float scale,
+                     int max_len_buf, void* out, int B, int len_q, int num_heads, int num_kv_heads, int dim_head, int bshd, void* workspace,
+                     size_t workspace_bytes, int dtype, int pdl, zl_stream_t stream) {
     const bool mask_ready = g_attn_mask_ready;
     g_attn_mask_ready = false;
-    ZL_CHECK_ARG(q && buf_lens && k_addrs && v_addrs && out && B > 0 && len_q > 0 && max_len_buf > 0);
+    ZL_CHECK_ARG(q && buf_lens && (host.addrs || (k_addrs && v_addrs)) && out && B > 0 && len_q > 0 && max_len_buf > 0);
     ZL_CHECK_ARG(num_heads > 0 && num_kv_heads > 0 && num_heads % num_kv_heads == 0);
     ZL_CHECK_SUPPORTED(dim_head == 64 || dim_head == 128);
     ZL_CHECK_SUPPORTED(dtype == ZL_F16 || dtype == ZL_BF16);
@@ -484,13 +511,13 @@ extern "C" int zl_decode_attention(const void* q, const int32_t* buf_lens, void*
     if (prompt_route(len_q, m_query, dim_head, B, num_kv_heads, mask, max_len_buf, out, workspace, workspace_bytes)) {
         if (dtype == ZL_F16)
             return dim_head == 128 ? prompt_attention<__half, 128>(q, buf_lens, k_addrs, v_addrs, mask, scale, max_len_buf, out, B, len_q, num_heads,
-                                                                   num_kv_heads, bshd, workspace, workspace_bytes, pdl, mask_ready, stream)
+                                                                   num_kv_heads, bshd, workspace, workspace_bytes, pdl, mask_ready, host, stream)
                                    : prompt_attention<__half, 64>(q, buf_lens, k_addrs, v_addrs, mask, scale, max_len_buf, out, B, len_q, num_heads,
-                                                                  num_kv_heads, bshd, workspace, workspace_bytes, pdl, mask_ready, stream);
+                                                                  num_kv_heads, bshd, workspace, workspace_bytes, pdl, mask_ready, host, stream);
         return dim_head == 128 ? prompt_attention<__nv_bfloat16, 128>(q, buf_lens, k_addrs, v_addrs, mask, scale, max_len_buf, out, B, len_q,
-                                                                      num_heads, num_kv_heads, bshd, workspace, workspace_bytes, pdl, mask_ready, stream)
+                                                                      num_heads, num_kv_heads, bshd, workspace, workspace_bytes, pdl, mask_ready, host, stream)
                                : prompt_attention<__nv_bfloat16, 64>(q, buf_lens, k_addrs, v_addrs, mask, scale, max_len_buf, out, B, len_q,
-                                                                     num_heads, num_kv_heads, bshd, workspace, workspace_bytes, pdl, mask_ready, stream);
+                                                                     num_heads, num_kv_heads, bshd, workspace, workspace_bytes, pdl, mask_ready, host, stream);
     }
     int splits = attn_num_splits(B, len_q, num_kv_heads, m_query, max_len_buf);
     // latency regime: few CTAs of work -> 256-key CTAs that issue all their loads up front
@@ -519,6 +546,9 @@ extern "C" int zl_decode_attention(const void* q, const int32_t* buf_lens, void*
                          (use_short ? splits <= kAttnClusterSplits && ctas <= (splits <= 4 ? sms : sms / 2) : (splits == 2 || splits == 4) && ctas <= 8ll * sms);
     // What four CTAs per SM hold in one wave goes three at a time: the places of short sequences are taken again.  us, four / three: 16 x 4096 40.8 / 40.4 (bf16 43.8 /
     // 41.9), 32 x 2048 40.9 / 38.3, 16 x 1500 17.9 / 17.0; against it 32 x 4096 (1024 CTAs) 64.6 / 74.9, and 32 x 700 14.7 / 18.6, whose keys come from L2.
+    AttnAddrs inl = {};
+    const int rc = attn_addresses(host, B, ctas, use_short && old_short, inl, k_addrs, v_addrs, pdl, stream);
+    if (rc) return rc;
     const bool three = dim_head == 128 && ctas <= 4ll * sms && max_len_buf >= 400 * splits;
     if (splits > 1 && !cluster) {
         part_o = static_cast<float*>(workspace);
@@ -535,7 +565,7 @@ extern "C" int zl_decode_attention(const void* q, const int32_t* buf_lens, void*
         ZL_CHECK_CUDA(launch_splits(k_decode_attn_warp<TT, DD>, grid, dim3(kWarpAttnWarps * 32),                \
                              (size_t)warp_attn_smem_floats<DD>() * sizeof(float), stream, pdl != 0, cluster, (const TT*)q, \
                              buf_lens, (TT* const*)k_addrs, (TT* const*)v_addrs, mask, scale, (TT*)out, part_o, \
-                             part_m, part_l, len_q, num_heads, num_kv_heads, m_query, splits, bshd));            \
+                             part_m, part_l, len_q, num_heads, num_kv_heads, m_query, splits, bshd, inl));       \
     } else if (use_short) {                                                                                     \
         static bool attr_set = false;                                                                           \
         if (!attr_set) {                                                                                        \
@@ -553,11 +583,11 @@ extern "C" int zl_decode_attention(const void* q, const int32_t* buf_lens, void*
         ZL_CHECK_CUDA(launch_splits(k_decode_attn<TT, DD, true, 4>, grid, block, 0, stream, pdl != 0, cluster, (const TT*)q, buf_lens, \
                              (TT* const*)k_addrs, (TT* const*)v_addrs, mask, scale, (TT*)out, part_o, part_m,   \
                              part_l, len_q, num_heads, num_kv_heads, m_query, splits, bshd, g_attn_pf_ptr,      \
-                             g_attn_pf_bytes));                                                                 \
+                             g_attn_pf_bytes, inl));                                                            \
     } else                                                                                                      \
     ZL_CHECK_CUDA(launch_splits(three ? k_decode_attn<TT, DD, false, DD == 128 ? 3 : 4> : k_decode_attn<TT, DD, false, 4>, grid, block, 0, stream, pdl != 0, cluster, (const TT*)q, buf_lens, \
                          (TT* const*)k_addrs, (TT* const*)v_addrs, mask, scale, (TT*)out, part_o, part_m,       \
-                         part_l, len_q, num_heads, num_kv_heads, m_query, splits, bshd, g_attn_pf_ptr, g_attn_pf_bytes)); \
+                         part_l, len_q, num_heads, num_kv_heads, m_query, splits, bshd, g_attn_pf_ptr, g_attn_pf_bytes, inl)); \
     if (part_o)                                                                                                 \
         ZL_CHECK_CUDA(launch(k_attn_combine<TT>, dim3((unsigned)vheads), dim3(DD), 0, stream, pdl != 0,         \
                              (const float*)part_o, (const float*)part_m, (const float*)part_l, (TT*)out, splits));
@@ -570,4 +600,19 @@ extern "C" int zl_decode_attention(const void* q, const int32_t* buf_lens, void*
     g_attn_pf_ptr = nullptr;
     g_attn_pf_bytes = 0;
     return ZL_OK;
+}
+
+extern "C" int zl_decode_attention(const void* q, const int32_t* buf_lens, void* const* k_addrs, void* const* v_addrs, const int8_t* mask, float scale,
+                                   int max_len_buf, void* out, int B, int len_q, int num_heads, int num_kv_heads, int dim_head, int bshd,
+                                   void* workspace, size_t workspace_bytes, int dtype, int pdl, zl_stream_t stream) {
+    return attention(q, buf_lens, k_addrs, v_addrs, HostAddrs{}, mask, scale, max_len_buf, out, B, len_q, num_heads, num_kv_heads, dim_head, bshd, workspace,
+                     workspace_bytes, dtype, pdl, stream);
+}
+
+extern "C" int zl_decode_attention_host(const void* q, const int32_t* buf_lens, const void* addrs, void* table, const int8_t* mask, float scale, int max_len_buf,
+                                        void* out, int B, int len_q, int num_heads, int num_kv_heads, int dim_head, int bshd, void* workspace,
+                                        size_t workspace_bytes, int dtype, zl_stream_t stream) {
+    ZL_CHECK_ARG(addrs && table);
+    return attention(q, buf_lens, nullptr, nullptr, HostAddrs{addrs, table}, mask, scale, max_len_buf, out, B, len_q, num_heads, num_kv_heads, dim_head, bshd,
+                     workspace, workspace_bytes, dtype, 1, stream);
 }

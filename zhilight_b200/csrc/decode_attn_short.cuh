@@ -207,6 +207,18 @@ __device__ __forceinline__ void attn_short_item(const T* __restrict__ q, const i
     }
 }
 
+// Addresses of the tasks' caches as a kernel's parameter, in place of tables on the device, and whether the kernel is the first one of its call: it then waits for
+// everything earlier before it lets dependents start, as the launch that writes a table would.
+constexpr int kAttnInline = 32;
+struct AttnAddrs {
+    const void* p[2 * kAttnInline];   // of K, then of V
+    int n, behind;                    // tasks, 0: the tables
+};
+template <typename T>
+__device__ __forceinline__ const T* attn_addr(const AttnAddrs& a, T* const* table, int b, bool v) {
+    return a.n ? static_cast<const T*>(a.p[(v ? a.n : 0) + b]) : table[b];
+}
+
 // Up to this many key splits of a head group are one cluster and merge their results themselves; the portable size of a cluster.
 constexpr int kAttnClusterSplits = 8;
 __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {

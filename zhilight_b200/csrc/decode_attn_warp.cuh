@@ -24,7 +24,7 @@ __global__ void __launch_bounds__(kWarpAttnWarps * 32)
 k_decode_attn_warp(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* const* __restrict__ k_addrs,
                    T* const* __restrict__ v_addrs, const int8_t* __restrict__ mask, float scale, T* __restrict__ out,
                    float* __restrict__ part_o, float* __restrict__ part_m, float* __restrict__ part_l, int len_q,
-                   int num_heads, int num_kv_heads, int m_query, int num_splits, int bshd) {
+                   int num_heads, int num_kv_heads, int m_query, int num_splits, int bshd, const __grid_constant__ AttnAddrs inl) {
     constexpr int NI = D / 32;
     constexpr int DC = D / 8;            // lanes covering one V row (16 bytes each)
     constexpr int RPI = 32 / DC;         // V rows per load instruction of the warp: 2 (D = 128) or 4 (D = 64)
@@ -44,7 +44,7 @@ k_decode_attn_warp(const T* __restrict__ q, const int32_t* __restrict__ buf_lens
     const int mq = min(8, m_query - mq0);
     const int head0 = hk * m_query + mq0;
 
-    pdl_trigger();
+    pdl_start(!inl.behind);
     pdl_wait();
 
     const int len_buf = buf_lens[b];
@@ -57,8 +57,8 @@ k_decode_attn_warp(const T* __restrict__ q, const int32_t* __restrict__ buf_lens
 
     const size_t stride = bshd ? (size_t)num_kv_heads * D : (size_t)D;
     const size_t base = bshd ? (size_t)hk * D : (size_t)hk * len_buf * D;
-    const T* kbase = k_addrs[b] + base;
-    const T* vbase = v_addrs[b] + base;
+    const T* kbase = attn_addr(inl, k_addrs, b, false) + base;
+    const T* vbase = attn_addr(inl, v_addrs, b, true) + base;
     const int8_t* mrow = nullptr;
     if (mask) {
         size_t len_off = 0;

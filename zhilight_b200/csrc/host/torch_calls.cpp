@@ -29,8 +29,7 @@ struct {
     decltype(&zl_fp8_quant_per_tensor) fp8_quant;
     decltype(&zl_w8a8_gemm) w8;
     decltype(&zl_decode_attention_workspace_bytes) attn_bytes;
-    decltype(&zl_write_pointers) write_pointers;
-    decltype(&zl_decode_attention) attn;
+    decltype(&zl_decode_attention_host) attn;
 } zl;
 
 struct NotPlain {};   // the general path's
@@ -176,7 +175,7 @@ PyObject* w8_linear(PyObject*, PyObject* const* a, Py_ssize_t na) {
 PyObject* decode_attention(PyObject*, PyObject* const* a, Py_ssize_t na) {
     return guarded([&]() -> PyObject* {
         args(na, 10);
-        if (!zl.attn || !zl.attn_bytes || !zl.write_pointers) throw NotPlain{};
+        if (!zl.attn || !zl.attn_bytes) throw NotPlain{};
         const at::Tensor &q = plain(a[0], true), &lens = plain(a[1], true);
         if (q.dim() != 4) throw NotPlain{};
         void* const mask = optional(a[4], true);
@@ -213,14 +212,11 @@ PyObject* decode_attention(PyObject*, PyObject* const* a, Py_ssize_t na) {
         const size_t ws_bytes = zl.attn_bytes(b, len_q, heads, dim, max_len), table_at = (ws_bytes + 15) / 16 * 16;
         const at::Tensor room = empty(q, {(int64_t)(table_at + 16 * b)}, at::kByte);   // the kernels' workspace, then the table of addresses
         uint8_t* const ws = static_cast<uint8_t*>(room.data_ptr());
-        void** const table = reinterpret_cast<void**>(ws + table_at);
+        void* const table = ws + table_at;
         const c10::cuda::CUDAStream cs = c10::cuda::getCurrentCUDAStream();
         const int rc = unlocked([&] {
-            const int e = zl.write_pointers(table, at_.data(), 2 * b, (zl_stream_t)cs.stream());
-            // the table is written behind everything earlier: the attention may start under that launch's end, whatever the caller's chain allows
-            return e ? e
-                     : zl.attn(q.data_ptr(), static_cast<const int32_t*>(lens.data_ptr()), table, table + b, static_cast<const int8_t*>(mask), (float)scale,
-                               max_len, out.data_ptr(), b, len_q, heads, kv_heads, dim, bshd, ws, ws_bytes, dt, 1, (zl_stream_t)cs.stream());
+            return zl.attn(q.data_ptr(), static_cast<const int32_t*>(lens.data_ptr()), at_.data(), table, static_cast<const int8_t*>(mask), (float)scale, max_len,
+                           out.data_ptr(), b, len_q, heads, kv_heads, dim, bshd, ws, ws_bytes, dt, (zl_stream_t)cs.stream());
         });
         if (rc == 0)
             for (const c10::Storage& s : storages) c10::cuda::CUDACachingAllocator::recordStream(s.data_ptr(), cs);
@@ -244,8 +240,7 @@ PyObject* bind(PyObject*, PyObject* d) {
     set(zl.fp8_quant, "zl_fp8_quant_per_tensor");
     set(zl.w8, "zl_w8a8_gemm");
     set(zl.attn_bytes, "zl_decode_attention_workspace_bytes");
-    set(zl.write_pointers, "zl_write_pointers");
-    set(zl.attn, "zl_decode_attention");
+    set(zl.attn, "zl_decode_attention_host");
     if (PyErr_Occurred()) return nullptr;
     Py_RETURN_NONE;
 }

@@ -30,6 +30,7 @@
 //
 // Nothing waits for ever: see tc2_common.cuh.  The waits begin behind the launch dependency.
 #pragma once
+#include "decode_attn_short.cuh"
 #include "tc2_common.cuh"
 
 #include <type_traits>
@@ -42,9 +43,9 @@ constexpr int kPaWarpS = 4, kPaWarpO = 5, kPaWarpLoad = 6, kPaLoaders = 64, kPaT
 // mask rows -> bits.  grid (len_q, B), 256 threads; bits [B][len_q][pitch64] with zero words behind len_buf, last [B][len_q]: index
 // of the last visible key, -1 for none
 __global__ void __launch_bounds__(256) k_mask_bits(const int8_t* __restrict__ mask, const int32_t* __restrict__ buf_lens, uint64_t* bits,
-                                                   int32_t* last, int len_q, int pitch64) {
+                                                   int32_t* last, int len_q, int pitch64, int behind) {
     __shared__ int s_last[8];
-    pdl_trigger();
+    pdl_start(!behind);
     pdl_wait();
     const int qi = blockIdx.x, b = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     size_t off = 0;
@@ -178,7 +179,7 @@ template <typename T, int D>
 __global__ void __launch_bounds__(kPaThreads, 2)
 k_attn_prompt(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* const* __restrict__ k_addrs, T* const* __restrict__ v_addrs,
               const uint64_t* __restrict__ bits, const int32_t* __restrict__ last, int pitch64, float scale, T* __restrict__ out, int len_q,
-              int num_heads, int num_kv_heads, int m_query, int splits, int bshd, int aligned, unsigned* err) {
+              int num_heads, int num_kv_heads, int m_query, int splits, int bshd, int aligned, unsigned* err, const __grid_constant__ AttnAddrs inl) {
     using C = PaCfg<D>;
     constexpr bool kHalf = std::is_same<T, __half>::value;
     constexpr int CH = D / 8;                                    // 16-byte chunks per row
@@ -209,11 +210,11 @@ k_attn_prompt(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* 
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    pdl_trigger();   // behind the allocation: a dependent that takes all of TMEM cannot keep this block waiting for it
+    pdl_start(!inl.behind);   // behind the allocation: a dependent that takes all of TMEM cannot keep this block waiting for it
     pdl_wait();
     const uint32_t tmem = s_tmem;
     const int len_buf = buf_lens[b];
-    const T *kp = k_addrs[b], *vp = v_addrs[b];
+    const T *kp = attn_addr(inl, k_addrs, b, false), *vp = attn_addr(inl, v_addrs, b, true);
 
     // keys this block can see; every warp finds out by itself, the loaders go ahead of the rows of q
     int n = len_buf;
