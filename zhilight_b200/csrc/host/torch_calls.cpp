@@ -171,7 +171,7 @@ PyObject* w8_linear(PyObject*, PyObject* const* a, Py_ssize_t na) {
     });
 }
 
-// q, buf_lens, k_bufs, v_bufs, mask, scale, max_len_buf, num_kv_heads, bshd, pdl (which changes nothing, see below)
+// q, buf_lens, k_bufs, v_bufs, mask, scale, max_len_buf, num_kv_heads, bshd, pdl (which changes nothing: the call is behind everything earlier)
 PyObject* decode_attention(PyObject*, PyObject* const* a, Py_ssize_t na) {
     return guarded([&]() -> PyObject* {
         args(na, 10);
