@@ -138,6 +138,34 @@ def test_blocks_of_rows_and_clusters_of_splits(lib, cuda, hq, hkv, d, len_q, ctx
             assert rel_l2(out.double().cpu().numpy(), _exact(q, k, v, mask, scale).numpy()) <= TOL[torch.bfloat16][1], (qd is shifted, scale)
 
 
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("hkv", [1, 4, 16])
+@pytest.mark.parametrize("masked", [True, False])
+def test_ranges_without_a_key(lib, cuda, d, hkv, masked):
+    """Clusters of eight, four and two key ranges of which some have no tile: their CTAs come to the merge as soon as they run, whatever the others do.  Calls in a
+    row on changing inputs, each against the same call alone, the last one against 64 bits."""
+    from zhilight_b200 import ops
+    g = torch.Generator().manual_seed(8)
+    lens, len_q = [1500, 1, 64, 130], 33
+    n = torch.tensor(lens, dtype=torch.int32, device=cuda)
+    masks = [(torch.arange(m)[None, :] <= torch.arange(len_q)[:, None]).to(torch.int8) if i % 2 == 0 else torch.ones(len_q, m, dtype=torch.int8) for i, m in enumerate(lens)]
+    flat = torch.cat([m.reshape(-1) for m in masks]).to(cuda) if masked else None
+    sets = [(torch.randn(4, len_q, 4 * hkv, d, generator=g).half(), *([torch.randn(m, hkv, d, generator=g).half() for m in lens] for _ in range(2))) for _ in range(3)]
+    on = [(q.to(cuda), [t.to(cuda) for t in k], [t.to(cuda) for t in v]) for q, k, v in sets]
+    call = lambda q, k, v: ops.decode_attention(q, n, k, v, flat, d ** -0.5, max(lens), hkv)  # noqa: E731
+    torch.cuda.synchronize()
+    row = [call(*a) for a in on for _ in range(4)]
+    torch.cuda.synchronize()
+    for i, a in enumerate(on):
+        alone = call(*a)
+        torch.cuda.synchronize()
+        assert all(torch.equal(o, alone) for o in row[4 * i:4 * i + 4])
+    q, k, v = sets[-1]
+    for i in range(4):
+        ref = _exact(q[i], k[i], v[i], masks[i] if masked else torch.ones(len_q, lens[i]), d ** -0.5)
+        assert rel_l2(row[-1][i].double().cpu().numpy(), ref.numpy()) <= 1e-3, i
+
+
 @pytest.mark.parametrize("d,len_q,ctx", [(128, 200, 333), (64, 100, 1100), (128, 3, 40)])
 def test_layers_that_share_a_mask(lib, cuda, d, len_q, ctx):
     """The second call uses the bits that the first one left (also where the decode kernels serve it, which have none), the third derives them again."""

@@ -210,6 +210,7 @@ k_attn_prompt(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* 
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (splits > 1) cluster_arrive();   // waited for ahead of the merge's first store into another CTA, which must have started by then
     pdl_start(!inl.behind);   // behind the allocation: a dependent that takes all of TMEM cannot keep this block waiting for it
     pdl_wait();
     const uint32_t tmem = s_tmem;
@@ -454,6 +455,7 @@ k_attn_prompt(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* 
     __syncwarp();
     tc2_drain(s_abort);
     if (splits > 1) {
+        cluster_wait();   // every CTA of the cluster runs: one without a key to look at is here before another one has started
         // Each CTA of the cluster finishes its columns of all rows, thread = row as before: 128 threads each add what they hold in tensor memory to what the
         // others sent.  Rows shared out instead, all columns through shared memory, took 10000 cycles behind the first barrier: 500 rows behind 1000 positions 36.8 us,
         // 35.0 so; and with each CTA beginning at another one of the cluster 76 x 1100 (four ranges) 19.6 -> 17.7.
