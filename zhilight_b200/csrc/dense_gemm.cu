@@ -170,6 +170,12 @@ k_dense_skinny(const T* __restrict__ x, int ldx, const T* __restrict__ w, const 
     }
 }
 
+// ZL_DENSE_NO_PDL (experiments): ordinary launches, whatever the caller's chain allows
+static bool dense_no_pdl() {
+    static const bool v = getenv("ZL_DENSE_NO_PDL") != nullptr;
+    return v;
+}
+
 template <typename T, typename TO, int NT>
 static cudaError_t launch_dense_ks(const T* x, int ldx, const T* w, const T* bias, TO* y, int mc, int N, int K,
                                    bool pdl, cudaStream_t stream, int act, const float* mul, int ld_mul) {
@@ -193,7 +199,7 @@ static cudaError_t launch_dense_ks(const T* x, int ldx, const T* w, const T* bia
     // Up to 80 MB a programmatic dependent always, the weights ahead of the wait only where the caller's chain allows it: launch and block scheduling run under the
     // predecessor's end.  In a row of calls, bf16, 4 rows, us: 3072 x 3072 8.2 -> 5.8, 4096 x 4096 8.0 -> 7.0, 5120 x 2560 8.4 -> 6.8, 14336 x 1024 10.3 -> 9.3; against it
     // 11008 x 4096 (90 MB, most of it in L2 from call to call), 24 rows 39.1 -> 40.7.
-    const bool dependent = pdl || (long long)N * K <= (40ll << 20);
+    const bool dependent = pdl || (!dense_no_pdl() && (long long)N * K <= (40ll << 20));
 #define ZL_DENSE_LAUNCH(KS_)                                                                                           \
     {                                                                                                                  \
         const int groups = cdiv(tiles, kDenseWarps / KS_);                                                             \
@@ -250,8 +256,7 @@ extern "C" int zl_dense_gemm_skinny_mul(const void* x, int ldx, const void* w, c
     ZL_CHECK_SUPPORTED(K % 32 == 0);
     ZL_CHECK_ARG(ldx >= K && ldx % 8 == 0);
     ZL_CHECK_ARG((reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0);
-    static const bool no_pdl = getenv("ZL_DENSE_NO_PDL") != nullptr;   // experiment knob
-    if (no_pdl) pdl = 0;
+    if (dense_no_pdl()) pdl = 0;
     // Prompt-sized M: the tensor-core kernel (gemm_tc.cu) reads the weights once instead of once per 32 rows.  bf16, M = 777,
     // 8192 x 2048: 443 -> 33 us; M = 33, 14336 x 4096: 72 -> 28 us.  Two passes over a matrix that fits the caches cost what its
     // launch costs (M = 33, 2048 x 2048: 17.4 against 19.0 us).
