@@ -174,8 +174,8 @@ def test_shared_tiles_with_swiglu(lib, cuda):
 
 @pytest.mark.parametrize("m,k,n,pieces", [(322, 1024, 12800, 2), (387, 1024, 13568, 2), (360, 1024, 12672, 2), (385, 1024, 13568, 2), (512, 1024, 18944, 1)])
 def test_last_wave_in_halves(lib, cuda, m, k, n, pieces):
-    """Tiles of the last wave in halves: one row behind the first half, an odd number of 128-row tiles, a last wave that is full (whole tiles); every epilogue
-    (all warps take part in it), every row."""
+    """Tiles of the last wave in halves: one row behind the first half, an odd number of 128-row tiles, a last wave that is full (whole tiles); every row.  All
+    warps take part in the epilogues: none, the residual's and SwiGLU's here, qkv's below."""
     from zhilight_b200 import ops
     assert lib.zl_w4_pairs_pieces(m, n, k) == pieces
     w, packed = _setup(cuda, k, n, False, 6)
@@ -195,3 +195,59 @@ def test_last_wave_in_halves(lib, cuda, m, k, n, pieces):
         gu = oops._t(ref, "f16")
         want = gu[:, :n // 2] / (1.0 + np.exp(-gu[:, :n // 2])) * gu[:, n // 2:]
         assert max(rel_l2(act[i], want[i]) for i in range(m)) <= 2e-3
+
+
+@pytest.mark.parametrize("d,hq,hkv,k,t,pieces", [(128, 92, 4, 1024, 322, 2), (64, 160, 20, 1024, 450, 2), (128, 102, 2, 1024, 387, 2), (128, 32, 8, 1024, 1000, 1),
+                                                 (64, 288, 8, 512, 40, 1), (128, 144, 4, 1024, 100, 1)])
+def test_qkv_rope_epilogue_over_several_tiles(lib, cuda, d, hq, hkv, k, t, pieces):
+    """More tiles than pairs: a chunk's placement comes with the chunk before, and the warps that convert the next tile help; whole and halved last waves, one
+    accumulator and two (40 rows).  Against the oracle's matrix turned in 64 bits: every row of q and of the caches, and nothing else written."""
+    from zhilight_b200 import ops
+    heads, n = hq + 2 * hkv, (hq + 2 * hkv) * d
+    assert lib.zl_w4_pairs_pieces(t, n, k) == pieces and lib.zl_w4_pairs_splits(t, n, k) == 1
+    rows = ops.qkv_rope_row_map(heads, d, cuda)
+    w, packed = _setup(cuda, k, n, False, 14, rows)
+    x, bias = _x(t, k, 8), (torch.randn(n, generator=torch.Generator().manual_seed(2)) * 0.5).half()
+    pos = torch.tensor([(5 * i) % 61 for i in range(t)], dtype=torch.int32, device=cuda)
+    cos, sin = ops.rope_cos_sin(pos, d, 10000.0)
+    tb = [i % 3 for i in range(t)]
+    pl = [-1 if i in (7, t - 1) else i // 3 for i in range(t)]      # two tokens that are not cached
+    bufs = [[torch.zeros(t // 3 + 2, hkv, d, dtype=torch.float16, device=cuda) for _ in range(3)] for _ in range(2)]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)  # noqa: E731
+    q = ops.w4a16_gemm_fused(x.to(cuda), packed, n, k, bias=bias.to(cuda)[rows.long()], epilogue=ops.EPI_QKV_ROPE, variant=1,
+                             rope=dict(cos=cos, sin=sin, token_batch=i32(tb), placement=i32(pl), k_bufs=bufs[0], v_bufs=bufs[1], num_heads=hq,
+                                       num_kv_heads=hkv, dim_head=d))
+    lin = torch.from_numpy(oops._t(gptq.gemm_f32(x.numpy(), w) + bias.float().numpy(), "f16")).double().view(t, heads, d)
+    turned = torch.cat([-lin[..., d // 2:], lin[..., :d // 2]], -1)
+    want = lin * cos.cpu().double()[:, None] + turned * sin.cpu().double()[:, None]
+    want[:, hq + hkv:] = lin[:, hq + hkv:]
+    got = q.cpu().double().view(t, hq, d)
+    for i in range(t):
+        assert rel_l2(got[i].numpy(), want[i, :hq].numpy()) <= TOL, i
+    for kind in range(2):
+        ref = [torch.zeros(t // 3 + 2, hkv, d, dtype=torch.float64) for _ in range(3)]
+        for i in range(t):
+            if pl[i] >= 0:
+                ref[tb[i]][pl[i]] = want[i, hq + kind * hkv:hq + (kind + 1) * hkv]
+        for b in range(3):
+            have = bufs[kind][b].cpu().double()
+            for i in range(t // 3 + 2):
+                assert rel_l2(have[i].numpy(), ref[b][i].numpy()) <= 2 * TOL if ref[b][i].any() else not have[i].any(), (kind, b, i)
+
+
+@pytest.mark.parametrize("m,k,n", [(150, 512, 384), (322, 1024, 12800), (100, 1024, 19456), (97, 2304, 2304)])
+def test_outputs_on_an_odd_address(lib, cuda, m, k, n):
+    """One value per store, with one tile a pair, several, halves, and tiles that pairs share: the bits of the stores of two, and nothing beside them."""
+    from zhilight_b200 import ops
+    assert lib.zl_w4_pairs_route(m, n, k) == 1
+    _, packed = _setup(cuda, k, n, False, 4)
+    g = torch.Generator().manual_seed(2)
+    x, bias, res = _x(m, k, 9).to(cuda), (torch.randn(n, generator=g) * 0.5).half().to(cuda), torch.randn(m, n, generator=g).half().to(cuda)
+    call = lambda r, out, **kw: ops.w4a16_gemm_fused(x, packed, n, k, bias=bias, residual=r, variant=1, out=out, **kw)  # noqa: E731
+    for kw in (dict(epilogue=ops.EPI_RESIDUAL), {}):
+        want = call(res if kw else None, torch.empty_like(res), **kw)
+        room = torch.full((m * n + 2,), 7.0, dtype=torch.float16, device=cuda)
+        odd = room[1:-1].view(m, n)
+        odd.copy_(res)
+        call(odd if kw else None, odd, **kw)
+        assert torch.equal(odd, want) and float(room[0]) == float(room[-1]) == 7.0
