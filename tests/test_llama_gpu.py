@@ -1,10 +1,12 @@
 """GPU parity: the whole decode step (driver + every kernel) against the CPU oracle model on small
 synthetic checkpoints -- the round trip a user of zhilight.LLaMA / DynamicBatchGenerator sees:
 state_dict in (HF-GPTQ layout), (token, position) per task in, logits / greedy tokens out."""
+import ctypes
 import os
 
 import numpy as np
 import pytest
+import torch
 
 from oracle import model as omodel
 from tests.helpers import rel_l2
@@ -296,3 +298,36 @@ def test_large_batch_decode_on_8b_shapes_matches_batch_1(lib, cuda, b, graph, pd
         assert np.isfinite(lb).all(), step
         for t in (0, b // 2, b - 1):
             assert rel_l2(lb[t], l1[0]) <= 5e-3, (step, t)
+
+
+@pytest.mark.parametrize("vocab,batches", [(8192, [8, 9, 32]), (9008, [7, 8, 29, 30]), (70016, [1, 3, 4])])
+def test_logits_reach_any_kind_of_host_memory(lib, cuda, vocab, batches):
+    """One to four pinned pieces of 256 KB with a last one that is full, partial or the only one, and the runtime's copy above 1 MB: pageable memory gets the bits
+    that page-locked and registered memory get, over steps of other tokens (a stale piece would show), nothing behind them; a prompt's logits likewise."""
+    from zhilight_b200.llama import LlamaDecoder
+    dec = LlamaDecoder(quant_type=5, group_size=128, max_batch=max(batches), max_seq=64, prefill_chunk=16, **dict(TINY, vocab_size=vocab))
+    dec.init_synthetic(seed=1)
+    rng = np.random.default_rng(vocab)
+    size = max(batches) * vocab
+    registered = np.empty(size + 1, dtype=np.float32)
+    assert int(torch.cuda.cudart().cudaHostRegister(registered.ctypes.data, registered.nbytes, 0)) == 0
+    places = [np.empty(size + 1, dtype=np.float32), torch.empty(size + 1, pin_memory=True).numpy(), registered]
+    ptr = lambda a: a.ctypes.data_as(ctypes.c_void_p)  # noqa: E731
+    try:
+        for b in batches:
+            for step in range(3):
+                tok, pos, nxt = rng.integers(0, vocab, b).astype(np.int32), np.full(b, step, dtype=np.int32), np.empty(b, dtype=np.int32)
+                for place in places:
+                    place.fill(np.nan)
+                    assert lib.zl_llama_decode(dec.h, ptr(tok), ptr(pos), b, ptr(nxt), ptr(place)) == 0
+                    logits = place[:b * vocab].reshape(b, vocab)
+                    assert np.isfinite(logits).all() and np.isnan(place[b * vocab:]).all() and np.array_equal(logits.argmax(1), nxt)
+                    assert np.array_equal(place, places[0], equal_nan=True)
+        tok, nxt = rng.integers(0, vocab, 20).astype(np.int32), np.empty(1, dtype=np.int32)
+        for place in places:
+            place.fill(np.nan)
+            assert lib.zl_llama_prefill(dec.h, 0, ptr(tok), 20, 0, ptr(nxt), ptr(place)) == 0
+            assert np.isfinite(place[:vocab]).all() and np.isnan(place[vocab:]).all() and np.array_equal(place, places[0], equal_nan=True)
+    finally:
+        torch.cuda.cudart().cudaHostUnregister(registered.ctypes.data)
+        dec.close()
