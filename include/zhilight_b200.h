@@ -290,6 +290,9 @@ int zl_decode_attention(const void* q, const int32_t* buf_lens, void* const* k_a
                         const int8_t* mask, float scale, int max_len_buf, void* out, int B, int len_q,
                         int num_heads, int num_kv_heads, int dim_head, int bshd, void* workspace,
                         size_t workspace_bytes, int dtype, int pdl, zl_stream_t stream);
+/* tests: how one query row per task runs: its key splits, and the CTAs of an SM that the kernel of 1024-key CTAs is compiled for, 0: 256-key CTAs; returns whether the
+ * splits of a head group merge in a cluster */
+int zl_decode_attention_plan(int B, int num_heads, int num_kv_heads, int dim_head, int max_len_buf, int dtype, int* splits, int* per_sm);
 /* the same behind everything earlier on the stream, with the addresses in host memory, B of K and B of V; table: device, room for them */
 int zl_decode_attention_host(const void* q, const int32_t* buf_lens, const void* addrs, void* table, const int8_t* mask, float scale, int max_len_buf, void* out,
                              int B, int len_q, int num_heads, int num_kv_heads, int dim_head, int bshd, void* workspace, size_t workspace_bytes, int dtype,

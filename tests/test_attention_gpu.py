@@ -1,5 +1,7 @@
 """GPU parity: batch decode attention over per-task ragged KV buffers vs the oracle
 (reference semantics attention_kernel.cu:434-489, 674-725, 730-923)."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -123,3 +125,21 @@ def test_addresses_from_the_host(lib, cuda, tasks, len_q, hq, hkv, longest, mask
             (want if own else got).append(out)
         torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(got, want)) and not any(torch.isnan(a).any() for a in got)
+
+
+@pytest.mark.parametrize("dtype,name,tol", [(torch.float16, "f16", 1e-3), (torch.bfloat16, "bf16", 6e-3)])
+@pytest.mark.parametrize("tasks,hq,hkv,d,longest,splits,per_sm,merged", [
+    (21, 8, 2, 128, 760, 3, 0, True), (24, 8, 2, 128, 760, 3, 0, False), (16, 8, 2, 128, 1000, 4, 0, True), (18, 8, 2, 128, 1000, 4, 0, False),      # 126 and 144 CTAs, 128 and 144
+    (12, 4, 1, 128, 2000, 8, 0, True), (16, 4, 1, 64, 2000, 8, 0, False), (12, 8, 2, 64, 1200, 5, 0, True),                                         # 96, 128, 120
+    (56, 8, 8, 128, 300, 1, 4, False), (64, 8, 4, 128, 900, 2, 4, True), (40, 8, 8, 128, 300, 1, 3, False), (96, 8, 8, 64, 300, 1, 5, False)])      # 448, 512, 320, 768
+def test_places_of_the_splits(lib, cuda, dtype, name, tol, tasks, hq, hkv, d, longest, splits, per_sm, merged):
+    """Both sides of the lines where clusters of 256-key CTAs find no room at once, and where an SM takes three, four or five CTAs; sequences of one length, and one
+    in four whole beside short ones."""
+    if name == "bf16" and per_sm == 4:
+        per_sm, merged = 3, False                                                                                      # beyond its wave of three nothing is a cluster
+    got = [ctypes.c_int(), ctypes.c_int()]
+    assert lib.zl_decode_attention_plan(tasks, hq, hkv, d, longest, 0 if name == "f16" else 1, *map(ctypes.byref, got)) == int(merged)
+    assert [v.value for v in got] == [splits, per_sm]
+    for lens in ([longest] * tasks, [longest if i % 4 == 0 else longest // 8 + 1 for i in range(tasks)]):
+        out, ref = _case(cuda, dtype, name, hq, hkv, d, lens, masked=False, seed=7)
+        assert rel_l2(out, ref) <= tol

@@ -26,7 +26,7 @@ constexpr int kAttnMaxRange = 1024;            // keys per CTA; logits live in s
 constexpr int kAttnRowStride = kAttnMaxRange + 4;
 constexpr int kAttnMaxSplits = 64;
 
-// PER_SM: CTAs of an SM at least; up to 168 (3) or 128 registers (4)
+// PER_SM: CTAs of an SM at least, by registers: for D = 128 3 or 4, for D = 64 4 or 5 (attn_per_sm)
 template <typename T, int D, bool PV_FP32, int PER_SM>
 __global__ void __launch_bounds__(kAttnThreads, PER_SM)
 k_decode_attn(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* const* __restrict__ k_addrs,
@@ -363,6 +363,39 @@ static cudaError_t launch_splits(void (*kernel)(KArgs...), dim3 grid, dim3 block
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// CTAs of an SM.  The lengths of the sequences are on the device, so a choice has to hold for all of them.  us, caches all of one length, random ones from half of it on, an
+// even spread down to a quarter, every fourth one whole beside eighths; 32 heads on 8, in a graph.
+//   D = 128, up to three CTAs per SM: three, whose registers hold more loads.  fp16, four / three: 24 x 2048 42.8 / 41.1, 38.7 / 37.1, 36.7 / 35.6, 21.2 / 20.3.
+//   fp16, more: four, 128 registers; a wave of four is two of three: 16 x 4096 50.7 / 69.9, 45.8 / 60.9, 41.1 / 40.7, 31.7 / 30.0; 64 x 1000 50.7 / 67.6, 43.3 / 52.2, 40.0 / 36.4,
+//   26.1 / 28.6: only the spread gains by three, where the places of short sequences are taken again.
+//   bf16, more: four have too few registers (24 bytes are spilled), so three, unless that is a wave more, beyond the first one of four: 32 x 4096 108 / 114, 93.4 / 95.8,
+//   71.9 / 75.8, 59.5 / 58.4; against it 40 x 4096 138 / 126, 111 / 108, 92.8 / 87.5, 73.3 / 68.3; 24 x 4096 90.2 / 84.0, 74.1 / 71.0, 57.1 / 55.8, 54.5 / 49.1.  Within the first one
+//   what the lengths are decides, 64 x 1000 55.7 / 71.0, 47.6 / 54.8, 43.2 / 37.6, 27.8 / 29.6, and it stays at three.
+//   D = 64: five (96 registers), for bf16 four (100) where these are all: 16 x 4096, five / four, 36.3 / 34.0, 33.2 / 31.6, 22.5 / 21.2, 19.5 / 19.0.  Six hold a fifth more CTAs in a
+//   wave, but spill: fp16 24 x 4096, five / six, 61.5 / 60.2, 46.9 / 52.7, 33.4 / 43.8, 19.6 / 21.5.
+static int attn_per_sm(int dim_head, bool fp16, long long ctas) {
+    const long long sms = device_sm_count();
+    auto waves = [&](int per) { return (ctas + per * sms - 1) / (per * sms); };
+    if (dim_head == 64) return fp16 || ctas > 4 * sms ? 5 : 4;
+    if (ctas <= 3 * sms) return 3;
+    return fp16 || (ctas > 4 * sms && waves(4) < waves(3)) ? 4 : 3;
+}
+// The splits of a head group as a cluster, which merges their results (attn_merge_cluster), or through the workspace and a second launch.  us, launch / cluster, fp16, D = 128.
+// 256-key CTAs are a cluster where the device has room for all clusters with one CTA per SM: 8 x 500 9.9 / 8.7, 4 x 1000 10.6 / 8.8, 2 x 1500 11.1 / 8.9 (96 CTAs by six), 13 x 2000, 8 heads on 1,
+// 11.5 / 9.1 (104 by eight); where it has not, some SMs work twice as long: 6 x 760 10.9 / 15.9 (144 CTAs by three), 18 x 1000, 8 on 2, 11.0 / 16.0 (144 by four), 2 x 2000 11.8 / 16.9 (128
+// by eight).
+// 1024-key CTAs: two or four splits in one wave, 16 x 4096 55.1 / 50.7, 20 x 1500 32.4 / 31.0; in more where each split is long, 32 x 4096 101 / 97.9, against it 32 x 1100 (16 heads on
+// 16, every fourth one whole) 29.4 / 30.6.  Three find their places badly: 18 x 3000 46.7 / 67.8; 2048 CTAs gain nothing: 32 x 4096 (16 on 16, D = 64) 108 / 109.
+static bool attn_cluster(bool use_short, int splits, long long ctas, int max_len_buf, int dim_head, int per_sm) {
+    const long long sms = device_sm_count();
+    if (use_short) {
+        static ClustersFit fit;
+        return splits <= kAttnClusterSplits && ctas / splits <= clusters_at_once(k_decode_attn_warp<__half, 128>, kWarpAttnWarps * 32, 160 * 1024, splits, fit);
+    }
+    if (splits != 2 && splits != 4) return false;
+    return ctas <= per_sm * sms || (!(dim_head == 128 && per_sm == 3) && ctas <= 8 * sms && max_len_buf >= 800 * splits);
+}
+
 static int attn_num_splits(int B, int len_q, int num_kv_heads, int m_query, int max_len_buf) {
     const int hgroups = (m_query + 7) / 8;
     const int base = B * len_q * num_kv_heads * hgroups;
@@ -401,6 +434,28 @@ extern "C" size_t zl_decode_attention_workspace_bytes(int B, int len_q, int num_
     int splits = cdiv(max_len_buf > 0 ? max_len_buf : 1, kAttnMaxRange);
     if (splits < kAttnMaxSplits) splits = kAttnMaxSplits;
     return (size_t)B * len_q * num_heads * splits * (dim_head + 2) * sizeof(float);
+}
+
+// Splits of a call on len_q = 1 and how they run: the kernel of 256-key CTAs, or that of 1024-key ones and its CTAs of an SM.
+struct AttnPlan {
+    int splits, per_sm;   // per_sm 0: 256-key CTAs
+    long long ctas;
+};
+static AttnPlan attn_plan(int B, int len_q, int num_kv_heads, int m_query, int dim_head, int max_len_buf, bool fp16) {
+    const long long groups = (long long)B * len_q * num_kv_heads * cdiv(m_query, 8);
+    // latency regime: few CTAs of work -> 256-key CTAs that issue all their loads up front
+    const int short_splits = cdiv(max_len_buf, kShortRange);
+    if (short_splits <= kAttnMaxSplits && groups * short_splits <= 4 * 148) return AttnPlan{short_splits, 0, groups * short_splits};
+    const int splits = attn_num_splits(B, len_q, num_kv_heads, m_query, max_len_buf);
+    return AttnPlan{splits, attn_per_sm(dim_head, fp16, groups * splits), groups * splits};
+}
+extern "C" int zl_decode_attention_plan(int B, int num_heads, int num_kv_heads, int dim_head, int max_len_buf, int dtype, int* splits, int* per_sm) {
+    ZL_CHECK_ARG(B > 0 && num_heads > 0 && num_kv_heads > 0 && num_heads % num_kv_heads == 0 && max_len_buf > 0 && splits && per_sm);
+    ZL_CHECK_SUPPORTED((dim_head == 64 || dim_head == 128) && (dtype == ZL_F16 || dtype == ZL_BF16));
+    const AttnPlan plan = attn_plan(B, 1, num_kv_heads, num_heads / num_kv_heads, dim_head, max_len_buf, dtype == ZL_F16);
+    *splits = plan.splits;
+    *per_sm = plan.per_sm;
+    return plan.splits > 1 && attn_cluster(plan.per_sm == 0, plan.splits, plan.ctas, max_len_buf, dim_head, plan.per_sm) ? 1 : 0;
 }
 
 extern "C" unsigned zl_prompt_attention_watchdog(void) {
@@ -519,13 +574,9 @@ static int attention(const void* q, const int32_t* buf_lens, void* const* k_addr
                                : prompt_attention<__nv_bfloat16, 64>(q, buf_lens, k_addrs, v_addrs, mask, scale, max_len_buf, out, B, len_q,
                                                                      num_heads, num_kv_heads, bshd, workspace, workspace_bytes, pdl, mask_ready, host, stream);
     }
-    int splits = attn_num_splits(B, len_q, num_kv_heads, m_query, max_len_buf);
-    // latency regime: few CTAs of work -> 256-key CTAs that issue all their loads up front
-    const int hg0 = (m_query + 7) / 8;
-    const int short_splits = cdiv(max_len_buf, kShortRange);
-    const bool use_short = short_splits <= kAttnMaxSplits &&
-                           (long long)B * len_q * num_kv_heads * hg0 * short_splits <= 4 * 148;
-    if (use_short) splits = short_splits;
+    const AttnPlan plan = attn_plan(B, len_q, num_kv_heads, m_query, dim_head, max_len_buf, dtype == ZL_F16);
+    const int splits = plan.splits, per_sm = plan.per_sm;
+    const bool use_short = per_sm == 0;
     const size_t vheads = (size_t)B * len_q * num_heads;
     float* part_o = nullptr;
     float* part_m = nullptr;
@@ -536,20 +587,10 @@ static int attention(const void* q, const int32_t* buf_lens, void* const* k_addr
     }
     static const bool old_short = getenv("ZL_ATTN_OLD_SHORT") != nullptr;
     static const bool pv_fp32 = getenv("ZL_ATTN_PV_FP32") != nullptr;
-    // The splits of a head group as a cluster, which merges their results (attn_merge_cluster), or through the workspace and a second launch.  us, launch / cluster,
-    // 32 heads on 8, D = 128, fp16: 256-key CTAs on an SM each 8 x 300 10.0 / 8.4, 4 x 1000 11.3 / 9.0, 1 x 2000 12.1 / 9.4; more of them than SMs come and go
-    // by whole clusters: 12 x 300 14.5 / 14.7, 32 x 300 26.0 / 28.9, 8 x 2000 29.0 / 40.6; 16 clusters of eight find no room at once: 2 x 2000 12.7 / 16.4.  1024-key CTAs: 16 x 4096 43.9 / 40.9, 32 x 1500 34.5 / 32.0,
-    // 32 x 4096 66.0 / 64.6; against it three splits 51.5 / 52.3 (32 x 3000), eight 20.5 / 27.2 (32 x 2048, 8 heads on 1), 2048 CTAs 73.6 / 75.4 (32 x 4096, 16 on 16, D = 64).
-    const int sms = device_sm_count();
-    const long long ctas = (long long)splits * num_kv_heads * hg0 * B * len_q;
-    const bool cluster = splits > 1 && !(use_short && old_short) &&
-                         (use_short ? splits <= kAttnClusterSplits && ctas <= (splits <= 4 ? sms : sms / 2) : (splits == 2 || splits == 4) && ctas <= 8ll * sms);
-    // What four CTAs per SM hold in one wave goes three at a time: the places of short sequences are taken again.  us, four / three: 16 x 4096 40.8 / 40.4 (bf16 43.8 /
-    // 41.9), 32 x 2048 40.9 / 38.3, 16 x 1500 17.9 / 17.0; against it 32 x 4096 (1024 CTAs) 64.6 / 74.9, and 32 x 700 14.7 / 18.6, whose keys come from L2.
+    const bool cluster = splits > 1 && !(use_short && old_short) && attn_cluster(use_short, splits, plan.ctas, max_len_buf, dim_head, per_sm);
     AttnAddrs inl = {};
-    const int rc = attn_addresses(host, B, ctas, use_short && old_short, inl, k_addrs, v_addrs, pdl, stream);
+    const int rc = attn_addresses(host, B, plan.ctas, use_short && old_short, inl, k_addrs, v_addrs, pdl, stream);
     if (rc) return rc;
-    const bool three = dim_head == 128 && ctas <= 4ll * sms && max_len_buf >= 400 * splits;
     if (splits > 1 && !cluster) {
         part_o = static_cast<float*>(workspace);
         part_m = part_o + vheads * splits * dim_head;
@@ -585,7 +626,7 @@ static int attention(const void* q, const int32_t* buf_lens, void* const* k_addr
                              part_l, len_q, num_heads, num_kv_heads, m_query, splits, bshd, g_attn_pf_ptr,      \
                              g_attn_pf_bytes, inl));                                                            \
     } else                                                                                                      \
-    ZL_CHECK_CUDA(launch_splits(three ? k_decode_attn<TT, DD, false, DD == 128 ? 3 : 4> : k_decode_attn<TT, DD, false, 4>, grid, block, 0, stream, pdl != 0, cluster, (const TT*)q, buf_lens, \
+    ZL_CHECK_CUDA(launch_splits(per_sm == 4 ? k_decode_attn<TT, DD, false, 4> : k_decode_attn<TT, DD, false, DD == 128 ? 3 : 5>, grid, block, 0, stream, pdl != 0, cluster, (const TT*)q, buf_lens, \
                          (TT* const*)k_addrs, (TT* const*)v_addrs, mask, scale, (TT*)out, part_o, part_m,       \
                          part_l, len_q, num_heads, num_kv_heads, m_query, splits, bshd, g_attn_pf_ptr, g_attn_pf_bytes, inl)); \
     if (part_o)                                                                                                 \

@@ -199,24 +199,24 @@ inline cudaError_t launch_pairs(void (*kernel)(KArgs...), int pairs, int splits,
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-// clusters of `splits` pairs of a kernel (one CTA per SM) that the current device holds at a time, 0: none; the caller keeps what was asked before
-struct PairsFit {
-    std::atomic<int> known[64][5] = {};   // count + 1
+// clusters of `size` CTAs of a kernel, one CTA per SM by shared memory, that the current device holds at a time, 0: none; the caller keeps what was asked before
+struct ClustersFit {
+    std::atomic<int> known[64][9] = {};   // count + 1
 };
 template <typename... KArgs>
-inline int pairs_clusters(void (*kernel)(KArgs...), int threads, int smem, int splits, PairsFit& fit) {
+inline int clusters_at_once(void (*kernel)(KArgs...), int threads, int smem, int size, ClustersFit& fit) {
     int dev = 0;
     cudaGetDevice(&dev);
-    const bool cached = dev >= 0 && dev < 64 && splits < 5;
-    int n = cached ? fit.known[dev][splits].load(std::memory_order_relaxed) - 1 : -1;
+    const bool cached = dev >= 0 && dev < 64 && size < 9;
+    int n = cached ? fit.known[dev][size].load(std::memory_order_relaxed) - 1 : -1;
     if (n >= 0) return n;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((device_sm_count() / (2 * splits) + 1) * 2 * splits);
+    cfg.gridDim = dim3((device_sm_count() / size + 1) * size);
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2 * splits;
+    attr.val.clusterDim.x = size;
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
@@ -225,8 +225,14 @@ inline int pairs_clusters(void (*kernel)(KArgs...), int threads, int smem, int s
         cudaGetLastError();
         n = 0;
     }
-    if (cached) fit.known[dev][splits].store(n + 1, std::memory_order_relaxed);
+    if (cached) fit.known[dev][size].store(n + 1, std::memory_order_relaxed);
     return n;
+}
+// clusters of `splits` pairs
+typedef ClustersFit PairsFit;
+template <typename... KArgs>
+inline int pairs_clusters(void (*kernel)(KArgs...), int threads, int smem, int splits, PairsFit& fit) {
+    return clusters_at_once(kernel, threads, smem, 2 * splits, fit);
 }
 
 // (K, rows, batch) tensor, row pitch ld and batch pitch in elements; box = 128 bytes of k x box_rows rows, 128-byte swizzle
