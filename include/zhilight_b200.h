@@ -282,6 +282,8 @@ int zl_decode_attention_set_prefetch(const void* ptr, size_t bytes);
 int zl_decode_attention_same_mask(void);
 /* tests: dynamic shared memory of a CTA of the kernel behind prompt portions; two CTAs of an SM share its tensor memory */
 int zl_prompt_attention_smem_bytes(int dim_head);
+/* tests: parts that it cuts the keys into, a cluster of CTAs each */
+int zl_prompt_attention_ranges(int B, int len_q, int num_heads, int num_kv_heads, int max_len_buf);
 size_t zl_decode_attention_workspace_bytes(int B, int len_q, int num_heads, int dim_head, int max_len_buf);
 /* q (B, len_q, H_q, d); buf_lens (B); k_addrs/v_addrs (B) device arrays of device pointers;
  * mask int8 ragged concat of (len_q, len_buf_b); out (B, len_q, H_q, d).  bshd: (len_buf, H_kv, d) else

@@ -138,6 +138,21 @@ def test_blocks_of_rows_and_clusters_of_splits(lib, cuda, hq, hkv, d, len_q, ctx
             assert rel_l2(out.double().cpu().numpy(), _exact(q, k, v, mask, scale).numpy()) <= TOL[torch.bfloat16][1], (qd is shifted, scale)
 
 
+@pytest.mark.parametrize("d,len_q,ctx,hq,hkv,ranges", [(128, 107, 2600, 16, 2, 8), (64, 110, 4090, 16, 2, 8), (128, 100, 800, 16, 4, 4), (64, 217, 1500, 8, 8, 4), (128, 268, 4070, 8, 1, 8),
+                                                       (128, 107, 2600, 8, 1, 8), (64, 91, 2600, 64, 8, 2), (128, 512, 512, 4, 4, 4)])
+def test_ranges_and_places(lib, cuda, d, len_q, ctx, hq, hkv, ranges):
+    """Both sides of the line to eight ranges: 14 groups, of which each CTA has an SM for itself, and 16 or 17 of many and of few keys; clusters that fill half of the SMs,
+    behind the mask's kernel."""
+    from zhilight_b200 import ops
+    assert lib.zl_prompt_attention_ranges(1, len_q, hq, hkv, ctx) == ranges
+    g = torch.Generator().manual_seed(len_q)
+    q, k, v = (torch.randn(*s, generator=g).half() for s in ((len_q, hq, d), (ctx, hkv, d), (ctx, hkv, d)))
+    mask, lens = _causal(len_q, ctx), torch.tensor([ctx], dtype=torch.int32, device=cuda)
+    outs = [ops.decode_attention(q[None].to(cuda), lens, [k.to(cuda)], [v.to(cuda)], mask.to(cuda), d ** -0.5, ctx, hkv)[0] for _ in range(3)]
+    assert rel_l2(outs[0].double().cpu().numpy(), _exact(q, k, v, mask, d ** -0.5).numpy()) <= TOL[torch.float16][1]
+    assert all(torch.equal(o, outs[0]) for o in outs)
+
+
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("hkv", [1, 4, 16])
 @pytest.mark.parametrize("masked", [True, False])

@@ -464,6 +464,11 @@ extern "C" unsigned zl_prompt_attention_watchdog(void) {
     return words ? words[kWaitAttnPrompt] : 0u;
 }
 
+extern "C" int zl_prompt_attention_ranges(int B, int len_q, int num_heads, int num_kv_heads, int max_len_buf) {
+    if (B <= 0 || len_q <= 0 || num_heads <= 0 || num_kv_heads <= 0 || num_heads % num_kv_heads || max_len_buf <= 0) return 0;
+    const long long groups = (long long)cdiv(len_q * (num_heads / num_kv_heads), kPaRows) * num_kv_heads * B;
+    return prompt_attn_splits(groups, cdiv(max_len_buf, kPaKeys), prompt_attn_fit(8));
+}
 extern "C" int zl_prompt_attention_smem_bytes(int dim_head) {
     return dim_head == 64 ? PaCfg<64>::kBytes : dim_head == 128 ? PaCfg<128>::kBytes : 0;
 }
@@ -521,7 +526,8 @@ static int prompt_attention(const void* q, const int32_t* buf_lens, void* const*
                             size_t workspace_bytes, int pdl, bool mask_ready, const HostAddrs& host, zl_stream_t stream) {
     const int m_query = num_heads / num_kv_heads;
     const int blocks = cdiv(len_q * m_query, kPaRows), tiles = cdiv(max_len_buf, kPaKeys);
-    const int splits = prompt_attn_splits((long long)blocks * num_kv_heads * B, tiles);
+    const long long groups = (long long)blocks * num_kv_heads * B;
+    const int splits = prompt_attn_splits(groups, tiles, prompt_attn_fit(8));
     const size_t q_rows = (size_t)B * len_q;
     uint64_t* bits = mask ? static_cast<uint64_t*>(workspace) : nullptr;
     int32_t* last = mask ? reinterpret_cast<int32_t*>(static_cast<uint8_t*>(workspace) + (q_rows * tiles * 8 + 15) / 16 * 16) : nullptr;
@@ -532,12 +538,12 @@ static int prompt_attention(const void* q, const int32_t* buf_lens, void* const*
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-        ZL_CHECK_CUDA(cudaFuncSetAttribute(k_attn_prompt<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, PaCfg<D>::kBytes));
+        ZL_CHECK_CUDA(cudaFuncSetAttribute(k_attn_prompt<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, PaCfg<D>::kAloneBytes));
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
     const bool mask_pass = mask && !mask_ready;
     AttnAddrs inl = {};
-    const int rc = attn_addresses(host, B, mask_pass ? (long long)len_q * B : (long long)blocks * num_kv_heads * B * splits, false, inl, k_addrs, v_addrs, pdl, stream);
+    const int rc = attn_addresses(host, B, mask_pass ? (long long)len_q * B : groups * splits, false, inl, k_addrs, v_addrs, pdl, stream);
     if (rc) return rc;
     if (mask_pass)
         ZL_CHECK_CUDA(launch(k_mask_bits, dim3(len_q, B), dim3(256), 0, stream, pdl != 0, mask, buf_lens, bits, last, len_q, tiles, inl.behind));
@@ -545,7 +551,7 @@ static int prompt_attention(const void* q, const int32_t* buf_lens, void* const*
     own.behind = inl.behind && !mask_pass;
     const int aligned = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
     // behind the mask's kernel the attention may start early whatever the caller's chain allows: it waits for that kernel to end
-    ZL_CHECK_CUDA((launch_attn_prompt<T, D>(dim3(blocks, num_kv_heads, B * splits), splits, stream, pdl != 0 || mask_pass, (const T*)q, buf_lens,
+    ZL_CHECK_CUDA((launch_attn_prompt<T, D>(dim3(blocks, num_kv_heads, B * splits), splits, groups <= prompt_attn_fit(splits), stream, pdl != 0 || mask_pass, (const T*)q, buf_lens,
                                             (T* const*)k_addrs, (T* const*)v_addrs, (const uint64_t*)bits, (const int32_t*)last, tiles, scale,
                                             (T*)out, len_q, num_heads, num_kv_heads, m_query, splits, bshd, aligned, words + kWaitAttnPrompt, own)));
     g_attn_pf_ptr = nullptr;

@@ -168,6 +168,8 @@ struct PaCfg {
     static constexpr int kMl = kStaged;                          // merge: {maximum, sum}, then weight, of the rows of up to 8 key ranges
     static constexpr int kUsed = kMl + 8 * kPaRows * 8 + 1024;   // + slack for the manual 1024-byte alignment
     static constexpr int kBytes = kHalfTmemSmem;                 // more than it uses, for the sake of tensor memory
+    static constexpr int kAloneBytes = 120 * 1024;               // no SM takes two of them
+    static_assert(2 * kAloneBytes > kSmSmem, "an SM each");
     static_assert(kUsed <= kBytes, "shared memory");
     static_assert(kPaRows * (D + 8 * 4) * 4 <= kStaged, "merge: [key range][row][D / ranges + 4] floats, where Q, K and V were");
     static constexpr int kS = 128;                               // TMEM columns: O 0 .. D - 1, S / P 128 .. 255 (two buffers of 64)
@@ -545,22 +547,32 @@ k_attn_prompt(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* 
 // Key splits (CTAs of a cluster) of a launch of `ctas` row blocks over up to `tiles` key tiles.  A tile is about 1 us of a CTA's chain, being a
 // cluster 2 us, so few tiles stay whole (256 x 256, 32 heads on 8: 12.1 against 12.5 us in two), more of them where two CTAs would share an SM (512 x 512 17.2 / 18.9,
 // against it 512 x 1024 27.3 / 25.4), and further ones are cut down to two a CTA: 76 x 1100 28.7 us whole, 21.3 in two, 17.7 in four; 200 x 900, 8 on 1, 15.6 in four,
-// 14.1 in eight.  Larger clusters wait for room (16 of eight: 100 x 800, 16 on 4, 17.5 us, in four 15.2): beyond one CTA per SM only pairs (256 x 1300, 16 heads on 4: 18.3 us in four, 23.3 in eight; 128 x 600, 64 on 8:
-// 16.8 in two, 20.7 in four).
-inline int prompt_attn_splits(long long ctas, int tiles) {
+// 14.1 in eight.  Beyond one CTA per SM only pairs (256 x 1300, 16 heads on 4: 18.3 us in four, 23.3 in eight; 128 x 600, 64 on 8: 16.8 in two, 20.7 in four).
+// Where some SM has to take two of clusters of eight, they have to save that: us, four / eight, 14 clusters, which find an SM per CTA, 16 tiles 16.4 / 15.0, 64 tiles 38.6 / 28.5 (22.9 as below); 16, which
+// do not, 16 tiles 15.2 / 18.1, 41 tiles 29.2 / 25.4; 18 of 41 tiles 27.5 / 26.6, of 24 20.3 / 21.4.
+// fit: of clusters of eight, see prompt_attn_fit
+inline int prompt_attn_splits(long long ctas, int tiles, int fit) {
     const int sms = device_sm_count();
     int s = 1;
     if (tiles >= (ctas * 2 <= sms ? 8 : 12) && ctas * 2 <= 2ll * sms) s = 2;
-    while (s > 1 && s < 8 && tiles >= (s == 2 ? 8 : 12) && ctas * s * 2 <= (s == 2 ? sms : sms * 3 / 4)) s *= 2;
+    if (s == 2 && tiles >= 8 && ctas * 4 <= sms) s = 4;
+    if (s == 4 && (ctas <= fit ? tiles >= 12 : tiles >= 40 && ctas * 8 <= sms)) s = 8;
     return s;
 }
 
+// Clusters of `splits` CTAs that find an SM for every CTA at once.  Such a launch takes the shared memory that keeps its CTAs on an SM each: some came in twos on the SMs that the
+// mask's kernel had left empty.  107 rows on 2600 keys, 8 heads on 1, 23.8 -> 18.1 us; 91 on 2600, 64 on 8, 45.6 -> 36.6.
+inline int prompt_attn_fit(int splits) {
+    static ClustersFit fit;
+    return splits == 1 ? device_sm_count() : clusters_at_once(k_attn_prompt<__half, 128>, kPaThreads, PaCfg<128>::kAloneBytes, splits, fit);
+}
+
 template <typename T, int D, typename... Args>
-inline cudaError_t launch_attn_prompt(dim3 grid, int splits, cudaStream_t stream, bool pdl, Args... args) {
+inline cudaError_t launch_attn_prompt(dim3 grid, int splits, bool alone, cudaStream_t stream, bool pdl, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(kPaThreads);
-    cfg.dynamicSmemBytes = PaCfg<D>::kBytes;
+    cfg.dynamicSmemBytes = alone ? PaCfg<D>::kAloneBytes : PaCfg<D>::kBytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     int n = 0;
