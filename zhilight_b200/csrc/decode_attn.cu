@@ -26,7 +26,7 @@ constexpr int kAttnMaxRange = 1024;            // keys per CTA; logits live in s
 constexpr int kAttnRowStride = kAttnMaxRange + 4;
 constexpr int kAttnMaxSplits = 64;
 
-// PER_SM: CTAs of an SM at least, by registers: for D = 128 3 or 4, for D = 64 4 or 5 (attn_per_sm)
+// PER_SM: CTAs of an SM at least, by registers: for D = 128 3 or 4, for D = 64 4, 5 or 0 (attn_per_sm)
 template <typename T, int D, bool PV_FP32, int PER_SM>
 __global__ void __launch_bounds__(kAttnThreads, PER_SM)
 k_decode_attn(const T* __restrict__ q, const int32_t* __restrict__ buf_lens, T* const* __restrict__ k_addrs,
@@ -373,10 +373,11 @@ static cudaError_t launch_splits(void (*kernel)(KArgs...), dim3 grid, dim3 block
 //   what the lengths are decides, 64 x 1000 55.7 / 71.0, 47.6 / 54.8, 43.2 / 37.6, 27.8 / 29.6, and it stays at three.
 //   D = 64: five (96 registers), for bf16 four (100) where these are all: 16 x 4096, five / four, 36.3 / 34.0, 33.2 / 31.6, 22.5 / 21.2, 19.5 / 19.0.  Six hold a fifth more CTAs in a
 //   wave, but spill: fp16 24 x 4096, five / six, 61.5 / 60.2, 46.9 / 52.7, 33.4 / 43.8, 19.6 / 21.5.
-static int attn_per_sm(int dim_head, bool fp16, long long ctas) {
+//   Six without a word to the compiler, 80 registers and no spill, where the rows of a prompt, all of one length, are one wave of them: 48 rows on 148 keys, 16 heads on 16, fp16 9.8 -> 7.9.
+static int attn_per_sm(int dim_head, bool fp16, bool one_length, long long ctas) {
     const long long sms = device_sm_count();
     auto waves = [&](int per) { return (ctas + per * sms - 1) / (per * sms); };
-    if (dim_head == 64) return fp16 || ctas > 4 * sms ? 5 : 4;
+    if (dim_head == 64) return one_length && waves(6) < waves(5) ? 6 : fp16 || ctas > 4 * sms ? 5 : 4;
     if (ctas <= 3 * sms) return 3;
     return fp16 || (ctas > 4 * sms && waves(4) < waves(3)) ? 4 : 3;
 }
@@ -447,7 +448,7 @@ static AttnPlan attn_plan(int B, int len_q, int num_kv_heads, int m_query, int d
     const int short_splits = cdiv(max_len_buf, kShortRange);
     if (short_splits <= kAttnMaxSplits && groups * short_splits <= 4 * 148) return AttnPlan{short_splits, 0, groups * short_splits};
     const int splits = attn_num_splits(B, len_q, num_kv_heads, m_query, max_len_buf);
-    return AttnPlan{splits, attn_per_sm(dim_head, fp16, groups * splits), groups * splits};
+    return AttnPlan{splits, attn_per_sm(dim_head, fp16, B == 1 && len_q > 1, groups * splits), groups * splits};
 }
 extern "C" int zl_decode_attention_plan(int B, int num_heads, int num_kv_heads, int dim_head, int max_len_buf, int dtype, int* splits, int* per_sm) {
     ZL_CHECK_ARG(B > 0 && num_heads > 0 && num_kv_heads > 0 && num_heads % num_kv_heads == 0 && max_len_buf > 0 && splits && per_sm);
@@ -632,7 +633,7 @@ static int attention(const void* q, const int32_t* buf_lens, void* const* k_addr
                              part_l, len_q, num_heads, num_kv_heads, m_query, splits, bshd, g_attn_pf_ptr,      \
                              g_attn_pf_bytes, inl));                                                            \
     } else                                                                                                      \
-    ZL_CHECK_CUDA(launch_splits(per_sm == 4 ? k_decode_attn<TT, DD, false, 4> : k_decode_attn<TT, DD, false, DD == 128 ? 3 : 5>, grid, block, 0, stream, pdl != 0, cluster, (const TT*)q, buf_lens, \
+    ZL_CHECK_CUDA(launch_splits(per_sm == 6 ? k_decode_attn<TT, DD, false, DD == 64 ? 0 : 4> : per_sm == 4 ? k_decode_attn<TT, DD, false, 4> : k_decode_attn<TT, DD, false, DD == 128 ? 3 : 5>, grid, block, 0, stream, pdl != 0, cluster, (const TT*)q, buf_lens, \
                          (TT* const*)k_addrs, (TT* const*)v_addrs, mask, scale, (TT*)out, part_o, part_m,       \
                          part_l, len_q, num_heads, num_kv_heads, m_query, splits, bshd, g_attn_pf_ptr, g_attn_pf_bytes, inl)); \
     if (part_o)                                                                                                 \
