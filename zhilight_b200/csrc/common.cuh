@@ -76,9 +76,11 @@ inline int device_sm_count() {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Programmatic dependent launch (PDL).  Every kernel in the decode chain calls pdl_trigger() as
-// early as possible (its dependents only prefetch read-only weights before their own pdl_wait())
-// and pdl_wait() before touching anything a predecessor produced.
+// Programmatic dependent launch (PDL).  Every kernel in the decode chain calls pdl_wait() before
+// touching anything a predecessor produced.  Where the caller's chain allows early reads it calls
+// pdl_trigger() as early as possible (its dependents only prefetch read-only weights before their
+// own pdl_wait()); kernels that are launched as dependents without that permission trigger behind
+// their wait (pdl_start).
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void pdl_trigger() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -93,6 +95,13 @@ __device__ __forceinline__ void pdl_wait() {
 __device__ __forceinline__ void pdl_start(bool early) {
     if (!early) pdl_wait();
     pdl_trigger();
+}
+// The same for a kernel of up to two CTAs per SM.  once: no CTA has more than one share of the work.  If some have, dependents begin when the last CTA leaves: CTAs that come before are
+// placed in twos on the SMs that end first, neighbours together, which have the longer shares; as an ordinary launch puts them these are on an SM each.
+// In graphs, ordinary / early / so: 4-bit 22016 x 4096, 16 rows (2.3 tiles a CTA) 18.9 / 21.8 / 18.5 us, 12800 x 1024 5.2 / 5.5 / 4.9; dense 6000 x 6144, 32 rows, 31.0 / 34.0 / 30.8.
+__device__ __forceinline__ void pdl_start_shares(bool early, bool once) {
+    if (!early) pdl_wait();
+    if (early || once) pdl_trigger();
 }
 
 // Launch helper: sets the PDL attribute when `pdl` is non-zero.

@@ -51,7 +51,7 @@ k_dense_skinny(const T* __restrict__ x, int ldx, const T* __restrict__ w, const 
         tr[0] = globaltimer_ns();
         tr[15] = 0xDull;
     }
-    pdl_start(early);
+    pdl_start_shares(early, false);   // even of one share each: 4096 x 4096, 8 rows, in a graph 6.5 us as ordinary launches, 7.4 with the early start, 6.2 so
     const int all_steps = K / 32;
     const int s_lo = (int)((long long)all_steps * ks / KS), steps = (int)((long long)all_steps * (ks + 1) / KS);
 
@@ -197,8 +197,8 @@ static cudaError_t launch_dense_ks(const T* x, int ldx, const T* w, const T* bia
         ks *= 2;
     dim3 block(kDenseWarps * 32);
     // Up to 80 MB a programmatic dependent always, the weights ahead of the wait only where the caller's chain allows it: launch and block scheduling run under the
-    // predecessor's end.  In a row of calls, bf16, 4 rows, us: 3072 x 3072 8.2 -> 5.8, 4096 x 4096 8.0 -> 7.0, 5120 x 2560 8.4 -> 6.8, 14336 x 1024 10.3 -> 9.3; against it
-    // 11008 x 4096 (90 MB, most of it in L2 from call to call), 24 rows 39.1 -> 40.7.
+    // predecessor's end, but see pdl_start_shares.  In a row of calls on weights that come from HBM, bf16, 4 rows, us: 3072 x 3072 10.1 -> 7.7, 4096 x 4096 10.3 -> 8.2, 5120 x 5120
+    // 16.5 -> 13.7, 14336 x 2048 16.5 -> 13.9; in a graph 7.6 -> 7.3, 8.2 -> 7.9, 13.5 -> 13.2, 13.8 -> 13.5.
     const bool dependent = pdl || (!dense_no_pdl() && (long long)N * K <= (40ll << 20));
 #define ZL_DENSE_LAUNCH(KS_)                                                                                           \
     {                                                                                                                  \

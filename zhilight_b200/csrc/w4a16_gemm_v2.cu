@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(WARPS * 32, ((NT <= 2 && WARPS == 8) ? 2 : 1))
         return p.packed + ((size_t)tile * G + gi) * kW4BlockBytes;
     };
 
-    pdl_start(p.early);
+    pdl_start_shares(p.early, n_tiles <= (int)gridDim.x);
     if (lane == 0) {
 #pragma unroll
         for (int s = 0; s < kV2Stages; ++s) mbar_init(&bars[s], 1);

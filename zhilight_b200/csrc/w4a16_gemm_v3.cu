@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(WARPS * SUBS * 32, 1) k_w4a16_v3(const W4Param
         if (tr && threadIdx.x == 0 && tr_n < 16) tr[tr_n++] = globaltimer_ns();
     };
     stamp();
-    pdl_start(p.early);
+    pdl_start_shares(p.early, n_tiles <= tile_stride);
     if (lane == 0) {
 #pragma unroll
         for (int s = 0; s < STAGES; ++s) mbar_init(&bars[s], 1);
