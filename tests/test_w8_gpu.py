@@ -36,6 +36,20 @@ def test_int8_quant_per_token_bit_exact(lib, cuda, tag, m, k):
     np.testing.assert_array_equal(s.cpu().numpy(), os_)
 
 
+@pytest.mark.parametrize("m,k", [(1, 2048), (148, 2048), (149, 2056), (296, 4096), (297, 4104), (888, 8200), (889, 512), (444, 16392)])
+def test_int8_quant_of_one_to_six_rows_per_sm(lib, cuda, m, k):
+    """Its CTAs ask for shared memory by how many an SM shall take; every kernel instance, calls in a row on changing rows."""
+    from zhilight_b200 import ops
+    xs = [_x(m, k, "f16", seed=m + i) for i in range(3)]
+    on = [_dev(x, "f16", cuda) for x in xs]
+    torch.cuda.synchronize()
+    got = [ops.int8_quant_per_token(x) for x in on]
+    for x, (q, s) in zip(xs, got):
+        oq, os_ = oracle.int8_quant_per_token(x)
+        np.testing.assert_array_equal(q.cpu().numpy(), oq)
+        np.testing.assert_array_equal(s.cpu().numpy(), os_)
+
+
 @pytest.mark.parametrize("tag", ["f16", "bf16"])
 @pytest.mark.parametrize("m,n,k,f32_scale,with_bias", [
     (1, 4096, 4096, False, False), (3, 1000, 512, True, False), (8, 6144, 4096, False, True),

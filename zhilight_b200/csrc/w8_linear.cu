@@ -435,12 +435,28 @@ static cudaError_t launch_w8(const uint8_t* xq, const float* sx, const uint8_t* 
     return launch_w8_ks<T, FP8, 4>(xq, sx, w, sw, sw_f32, bias, y, mc, N, K, pdl, st);
 }
 
+constexpr int kSmBytes = 228 * 1024;   // shared memory of an SM
 template <typename T>
 static cudaError_t launch_int8_quant(const T* x, int ldx, int8_t* q, float* scale, int M, int K, bool pdl, cudaStream_t stream) {
     const int chunks = cdiv(K, 256 * 8);
     auto kernel = chunks <= 1 ? k_int8_quant_per_token<T, 1> : chunks <= 2 ? k_int8_quant_per_token<T, 2>
                   : chunks <= 4 ? k_int8_quant_per_token<T, 4> : chunks <= 8 ? k_int8_quant_per_token<T, 8> : k_int8_quant_per_token<T, 0>;
-    return launch(kernel, dim3(M), dim3(256), 0, stream, true, x, ldx, q, scale, K, (int)pdl);
+    // Where it comes under the end of whatever was before, its CTAs ask for the shared memory that spreads them over the SMs: beside a GEMM that still runs they were placed in
+    // sixes.  With the GEMM behind it, in a graph, ordinary launches / dependents / dependents so: 100 rows of 4096 x 4096 11.5 / 12.7 / 11.5 us, 64 of 8192 x 8192 14.6 / 16.1 / 14.3, 160 of
+    // 6144 x 4096 13.2 / 14.7 / 12.7, 32 of 28672 x 4096 26.3 / 28.6 / 26.2.
+    const int per_sm = cdiv(M, device_sm_count()), smem = pdl || per_sm > 6 ? 0 : kSmBytes / (per_sm + 1);
+    if (smem > 48 * 1024) {
+        static bool set[64][5] = {};
+        const int at = chunks <= 1 ? 0 : chunks <= 2 ? 1 : chunks <= 4 ? 2 : chunks <= 8 ? 3 : 4;
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (dev < 0 || dev >= 64 || !set[dev][at]) {
+            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmBytes / 2);
+            if (e != cudaSuccess) return e;
+            if (dev >= 0 && dev < 64) set[dev][at] = true;
+        }
+    }
+    return launch(kernel, dim3(M), dim3(256), (size_t)smem, stream, true, x, ldx, q, scale, K, (int)pdl);
 }
 
 }  // namespace zl
