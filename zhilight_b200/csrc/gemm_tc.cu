@@ -483,11 +483,21 @@ __global__ void __launch_bounds__(kGtThreads, 1) k_gemm_tc(const __grid_constant
         bool told = false;
         int hint = 0;
         GtTile t;
-        if (helps && meet) asm volatile("bar.sync 2, %0;" ::"n"(kMeet) : "memory");
         for (int j = helps ? tiles - 1 : 0; j >= 0 && j < tiles && !(helps && !meet); ++j) {
             const int acc = j & 1;
             const bool last = j == tiles - 1;
+            // which tile, its bias and its scales ahead of the wait
+            if (GROUPED && helps) {   // whose group lies anywhere: a walk from the first of 64 groups on took as long as the tile's end, 1.2 us
+                int end = p.groups;
+                while (end - hint > 1) {
+                    const int mid = (hint + end) >> 1;
+                    (s_cum[mid] <= pair + j * pairs ? hint : end) = mid;
+                }
+            }
             gt_tile<GROUPED>(p, s_cum, pair + j * pairs, hint, t);
+            const int n = t.n0 + (int)rank * 128 + q * 32 + lane, step = last ? 16 * kGtSets : 32;
+            if (splits == 1) row_values(t, n);
+            if (helps) asm volatile("bar.sync 2, %0;" ::"n"(kMeet) : "memory");
             const bool ok = helps ? !*s_abort : tc2_wait(last ? last_full : &acc_full[acc], last ? 0u : (uint32_t)(j >> 1) & 1u, s_abort, p.err, 0x2800 + acc);
             if (last && set == 0 && meet) {
                 asm volatile("bar.arrive 2, %0;" ::"n"(kMeet) : "memory");
@@ -496,8 +506,6 @@ __global__ void __launch_bounds__(kGtThreads, 1) k_gemm_tc(const __grid_constant
             if (!ok) break;
             tc_fence_after();
             if (splits > 1) break;
-            const int n = t.n0 + (int)rank * 128 + q * 32 + lane, step = last ? 16 * kGtSets : 32;
-            row_values(t, n);
             const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * 256);
             for (int c0 = set * 16; c0 < t.ntok && t.t0 + c0 < t.M; c0 += step) {
                 float v[16];
