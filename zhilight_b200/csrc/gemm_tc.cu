@@ -140,15 +140,30 @@ __device__ __forceinline__ void gt_put16(const GemmTcP& p, const GtTile& t, TO* 
             }
         }
     } else if (p.wide) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        const int first = t.t0 + c0 + odd, left = n < g.N ? t.M - first : 0;   // N is even
+        struct alignas(2 * sizeof(TO)) Two {
+            TO a, b;
+        };
+        auto two = [&](int j) {
             const float other = __shfl_xor_sync(0xffffffffu, odd ? v[2 * j] : v[2 * j + 1], 1);
-            const int m = t.t0 + c0 + 2 * j + odd;
-            const int row = g.grp_off ? __shfl_sync(0xffffffffu, mine, 2 * j + odd) : m;
-            struct alignas(2 * sizeof(TO)) Two {
-                TO a, b;
-            } two = {from_f32<TO>(odd ? other : v[2 * j]), from_f32<TO>(odd ? v[2 * j + 1] : other)};
-            if (n < g.N && m < t.M) *reinterpret_cast<Two*>(y + (size_t)row * g.ldy + (n & ~1)) = two;   // N is even
+            return Two{from_f32<TO>(odd ? other : v[2 * j]), from_f32<TO>(odd ? v[2 * j + 1] : other)};
+        };
+        TO* at = y + (n & ~1);
+        if (g.grp_off) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const Two w = two(j);
+                const int row = __shfl_sync(0xffffffffu, mine, 2 * j + odd);
+                if (2 * j < left) *reinterpret_cast<Two*>(at + (size_t)row * g.ldy) = w;
+            }
+        } else {
+            at += (size_t)first * g.ldy;
+            const size_t step = 2 * (size_t)g.ldy;
+#pragma unroll
+            for (int j = 0; j < 8; ++j, at += step) {
+                const Two w = two(j);
+                if (2 * j < left) *reinterpret_cast<Two*>(at) = w;
+            }
         }
     } else {
 #pragma unroll
