@@ -103,7 +103,10 @@ int zl_w4_unpack(const void* packed, uint32_t* qweight_km, uint8_t* qzeros_km, v
  * (src/nn/quant/gptq/q_gemm_k_major.cu:957-1116, 176-237, 529-578):
  * y[m,n] = sum_k x[m,k] * (q[n,k]-z[n,k/g]) * s[n,k/g] (+bias[n]), fp16 in/out, fp32 accumulate.
  * x (M, K) f16 row stride ldx; y (M, N_out) f16 where N_out = N (NONE/RESIDUAL) or N/2 (SWIGLU).
- * Any M >= 1 (weights are re-streamed per 32-token chunk).  pdl != 0 -> programmatic dependent launch. */
+ * Any M >= 1 (weights are re-streamed per 32-token chunk).
+ * pdl, here, of the activations' 8-bit quantisation and of zl_dense_gemm_skinny*: 0 an ordinary launch; 1 a programmatic dependent launch in a chain that
+ * allows early reads: the weights are read ahead of the wait for the launch before, and dependents may begin at once; 2 a programmatic dependent that
+ * waits for the launch before ahead of everything it reads or writes (dense GEMMs of more than 80 MB of weights: an ordinary launch). */
 int zl_w4a16_gemm(const void* x, int ldx, const void* packed, const void* bias, const void* residual,
                   void* y, int M, int N, int K, int group_size, int epilogue, int pdl, zl_stream_t stream);
 

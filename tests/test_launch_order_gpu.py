@@ -1,5 +1,6 @@
 """GPU: launches that start under the end of the one before them.  Whatever the callers' `pdl` says, a row of calls gives the bits of the same calls one by one,
 and the switch for ordinary launches gives these."""
+import ctypes
 import os
 import subprocess
 import sys
@@ -61,22 +62,69 @@ def test_a_row_of_calls_gives_the_bits_of_single_calls(lib, cuda, m):
             assert all(torch.isfinite(y).all() for y in a) and all(torch.equal(y, z) for y, z in zip(a, b)), turn
 
 
-_EDGES = """
-import ctypes
+def _programmatic_edges(call):
+    """Programmatic edges between the launches of two calls in a captured graph, and all of them"""
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        call()
+        call()
+    n = ctypes.c_size_t(32)
+    nodes = [(ctypes.c_void_p * 32)() for _ in range(2)]
+    edges = (ctypes.c_uint8 * 256)()       # eight bytes an edge: two ports, the type, reserved ones
+    assert ctypes.CDLL("libcudart.so.12").cudaGraphGetEdges_v2(ctypes.c_void_p(graph.raw_cuda_graph()), *nodes, edges, ctypes.byref(n)) == 0
+    return sum(edges[8 * i + 2] for i in range(n.value)), n.value
+
+
+@pytest.mark.parametrize("what", ["dense", "w4-1", "w4-12", "w4-48", "w4-300", "int8", "fp8", "fp8-large"])
+def test_three_kinds_of_launches(lib, cuda, what):
+    """pdl 0: ordinary launches, 1 and 2: programmatic dependents, of one or several kernels; the same bits, and what the Python calls ask for."""
+    from oracle import gptq
+    from zhilight_b200 import _lib, ops
+    m = int(what.split("-")[1]) if what.startswith("w4") else 80 if what == "fp8-large" else 4
+    x = torch.randn(m, K, generator=torch.Generator().manual_seed(1)).half().to(cuda)
+    stream = lambda: torch.cuda.current_stream().cuda_stream  # noqa: E731
+    if what == "dense":
+        w, y = torch.randn(K, K, device=cuda).half(), torch.empty(m, K, dtype=torch.float16, device=cuda)
+        run = lambda pdl: _lib.call("zl_dense_gemm_skinny", x.data_ptr(), K, w.data_ptr(), None, y.data_ptr(), m, K, K, ops.F16, ops.F16, pdl, stream())  # noqa: E731
+        python = lambda: ops.dense_gemm_skinny(x, w)  # noqa: E731
+    elif what.startswith("w4"):
+        qw, qz, sc, gi = gptq.make_gptq_checkpoint(K, K, 128, False, seed=3)
+        km = [torch.from_numpy(a.view(d) if d else a).to(cuda) for a, d in zip(gptq.to_k_major(qw, qz, sc, gi, 128)[:3], ("int32", None, None))]
+        packed, y = ops.w4_pack(*km, 128, variant=1), torch.empty(m, K, dtype=torch.float16, device=cuda)
+
+        def run(pdl):
+            a = _lib.W4FusedArgs(x.data_ptr(), K, packed.data_ptr(), None, None, y.data_ptr(), m, K, K, 128, 0, pdl, None, 1e-5)
+            a.variant = 1
+            _lib.call("zl_w4a16_gemm_fused", ctypes.byref(a), stream())
+        python = lambda: ops.w4a16_gemm_fused(x, packed, K, K, variant=1)  # noqa: E731
+    else:
+        y, s = torch.empty(m, K, dtype=torch.uint8, device=cuda), torch.empty(m, device=cuda)
+        if what == "int8":
+            run = lambda pdl: _lib.call("zl_int8_quant_per_token", x.data_ptr(), K, y.data_ptr(), s.data_ptr(), m, K, ops.F16, pdl, stream())  # noqa: E731
+            python = lambda: ops.int8_quant_per_token(x)[0].view(torch.uint8)  # noqa: E731
+        else:
+            run = lambda pdl: _lib.call("zl_fp8_quant_per_tensor", x.data_ptr(), y.data_ptr(), s.data_ptr(), x.numel(), ops.F16, pdl, stream())  # noqa: E731
+            python = lambda: ops.fp8_quant_per_tensor(x)[0]  # noqa: E731
+    want = python().clone()
+    torch.cuda.synchronize()
+    kernels = 3 if what == "fp8-large" else 1
+    for pdl in (0, 1, 2):
+        y.zero_()
+        run(pdl)
+        torch.cuda.synchronize()
+        assert torch.equal(y, want), pdl
+        assert _programmatic_edges(lambda: run(pdl)) == ((2 * kernels - 1) * (pdl != 0), 2 * kernels - 1), pdl
+    assert _programmatic_edges(python)[0] == 2 * kernels - 1
+
+
+_SWITCH = """
 import torch
+from tests.test_launch_order_gpu import _programmatic_edges
 from zhilight_b200 import ops
 x, w = torch.randn(4, 1024, device="cuda").half(), torch.randn(1024, 1024, device="cuda").half()
-run = lambda: ops.dense_gemm_skinny(ops.dense_gemm_skinny(x, w), w)
-run()
+ops.dense_gemm_skinny(x, w)
 torch.cuda.synchronize()
-graph = torch.cuda.CUDAGraph(keep_graph=True)
-with torch.cuda.graph(graph):
-    run()
-n = ctypes.c_size_t(8)
-nodes = [(ctypes.c_void_p * 8)() for _ in range(2)]
-edges = (ctypes.c_uint8 * 64)()       # eight bytes an edge: two ports, the type, reserved ones
-rc = ctypes.CDLL("libcudart.so.12").cudaGraphGetEdges_v2(ctypes.c_void_p(graph.raw_cuda_graph()), *nodes, edges, ctypes.byref(n))
-print("edges", rc, n.value, edges[2])
+print("edges", *_programmatic_edges(lambda: ops.dense_gemm_skinny(x, w)))
 """
 
 
@@ -87,6 +135,6 @@ def test_switch_for_ordinary_launches(lib, cuda, switch, programmatic):
     env.pop("ZL_DENSE_NO_PDL", None)
     if switch:
         env["ZL_DENSE_NO_PDL"] = "1"
-    r = subprocess.run([sys.executable, "-c", _EDGES], env=env, capture_output=True, text=True, timeout=300)
+    r = subprocess.run([sys.executable, "-c", _SWITCH], env=env, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
-    assert r.stdout.split()[-4:] == ["edges", "0", "1", str(programmatic)]
+    assert r.stdout.split()[-3:] == ["edges", str(programmatic), "1"]

@@ -89,9 +89,11 @@ __device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// A kernel that waits before it touches anything at all can always be launched as a programmatic dependent: its launch, barriers and allocations
-// run under the predecessor's end.  early: the caller's chain asks for more, what is constant is read ahead of the wait and dependents may start at
-// once.  Without, a dependent of that kind could read ahead of what this kernel's predecessors write: it starts behind the wait.
+// `pdl` of the 4-bit GEMMs, of the activations' 8-bit quantisation and of the dense GEMM of few rows: an ordinary launch; a programmatic dependent in a caller's
+// chain that allows early reads, what is constant comes ahead of the wait and dependents may start at once; a dependent that waits before it touches anything
+// at all, whose launch, barriers and allocations alone run under the predecessor's end.
+constexpr int kPdlNone = 0, kPdlEarly = 1, kPdlBehind = 2;
+// early: false for the last kind.  A dependent of the second one could read ahead of what this kernel's predecessors write: it starts behind the wait.
 __device__ __forceinline__ void pdl_start(bool early) {
     if (!early) pdl_wait();
     pdl_trigger();

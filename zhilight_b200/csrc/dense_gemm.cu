@@ -178,7 +178,7 @@ static bool dense_no_pdl() {
 
 template <typename T, typename TO, int NT>
 static cudaError_t launch_dense_ks(const T* x, int ldx, const T* w, const T* bias, TO* y, int mc, int N, int K,
-                                   bool pdl, cudaStream_t stream, int act, const float* mul, int ld_mul) {
+                                   int pdl, cudaStream_t stream, int act, const float* mul, int ld_mul) {
     const int tiles = cdiv(N, 16);
     static int sms = 0;
     if (sms == 0) {
@@ -196,16 +196,15 @@ static cudaError_t launch_dense_ks(const T* x, int ldx, const T* w, const T* bia
            (tiles * ks < slots || (tiles * ks) % slots > 0 && (tiles * ks) / slots < 4 && ks < 2))
         ks *= 2;
     dim3 block(kDenseWarps * 32);
-    // Up to 80 MB a programmatic dependent always, the weights ahead of the wait only where the caller's chain allows it: launch and block scheduling run under the
-    // predecessor's end, but see pdl_start_shares.  In a row of calls on weights that come from HBM, bf16, 4 rows, us: 3072 x 3072 10.1 -> 7.7, 4096 x 4096 10.3 -> 8.2, 5120 x 5120
-    // 16.5 -> 13.7, 14336 x 2048 16.5 -> 13.9; in a graph 7.6 -> 7.3, 8.2 -> 7.9, 13.5 -> 13.2, 13.8 -> 13.5.
-    const bool dependent = pdl || (!dense_no_pdl() && (long long)N * K <= (40ll << 20));
+    // kPdlBehind: up to 80 MB a programmatic dependent, whose launch and block scheduling run under the predecessor's end, but see pdl_start_shares.  In a row of calls on
+    // weights that come from HBM, bf16, 4 rows, us: 3072 x 3072 10.1 -> 7.7, 4096 x 4096 10.3 -> 8.2, 5120 x 5120 16.5 -> 13.7, 14336 x 2048 16.5 -> 13.9; in a graph 7.6 -> 7.3, 8.2 -> 7.9, 13.5 -> 13.2, 13.8 -> 13.5.
+    const bool dependent = pdl == kPdlBehind ? (long long)N * K <= (40ll << 20) : pdl != kPdlNone, early = pdl != kPdlBehind;
 #define ZL_DENSE_LAUNCH(KS_)                                                                                           \
     {                                                                                                                  \
         const int groups = cdiv(tiles, kDenseWarps / KS_);                                                             \
         const int grid = groups < sms * 2 ? groups : sms * 2;                                                          \
         return launch(k_dense_skinny<T, TO, NT, KS_, UNROLL>, dim3(grid), block, 0, stream, dependent, x, ldx, w, bias, y, mc, \
-                      N, K, g_w4_trace, act, mul, ld_mul, (int)pdl);                                                                          \
+                      N, K, g_w4_trace, act, mul, ld_mul, (int)early);                                                                          \
     }
     if (ks == 1) ZL_DENSE_LAUNCH(1);
     if (ks == 2) ZL_DENSE_LAUNCH(2);
@@ -216,7 +215,7 @@ static cudaError_t launch_dense_ks(const T* x, int ldx, const T* w, const T* bia
 
 template <typename T, typename TO>
 static cudaError_t launch_dense(const T* x, int ldx, const T* w, const T* bias, TO* y, int mc, int N, int K,
-                                bool pdl, cudaStream_t stream, int act, const float* mul, int ld_mul) {
+                                int pdl, cudaStream_t stream, int act, const float* mul, int ld_mul) {
     if (mc <= 8) return launch_dense_ks<T, TO, 1>(x, ldx, w, bias, y, mc, N, K, pdl, stream, act, mul, ld_mul);
     if (mc <= 16) return launch_dense_ks<T, TO, 2>(x, ldx, w, bias, y, mc, N, K, pdl, stream, act, mul, ld_mul);
     return launch_dense_ks<T, TO, 4>(x, ldx, w, bias, y, mc, N, K, pdl, stream, act, mul, ld_mul);
@@ -224,7 +223,7 @@ static cudaError_t launch_dense(const T* x, int ldx, const T* w, const T* bias, 
 
 template <typename T>
 static cudaError_t dispatch_out(const T* x, int ldx, const T* w, const T* bias, void* y, int mc, int N, int K,
-                                int out_dtype, bool pdl, cudaStream_t stream, size_t y_off, int act, const float* mul, int ld_mul) {
+                                int out_dtype, int pdl, cudaStream_t stream, size_t y_off, int act, const float* mul, int ld_mul) {
     if (out_dtype == ZL_F32)
         return launch_dense<T, float>(x, ldx, w, bias, static_cast<float*>(y) + y_off, mc, N, K, pdl, stream, act, mul, ld_mul);
     return launch_dense<T, T>(x, ldx, w, bias, static_cast<T*>(y) + y_off, mc, N, K, pdl, stream, act, mul, ld_mul);
@@ -256,7 +255,7 @@ extern "C" int zl_dense_gemm_skinny_mul(const void* x, int ldx, const void* w, c
     ZL_CHECK_SUPPORTED(K % 32 == 0);
     ZL_CHECK_ARG(ldx >= K && ldx % 8 == 0);
     ZL_CHECK_ARG((reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0);
-    if (dense_no_pdl()) pdl = 0;
+    if (dense_no_pdl()) pdl = kPdlNone;
     // Prompt-sized M: the tensor-core kernel (gemm_tc.cu) reads the weights once instead of once per 32 rows.  bf16, M = 777,
     // 8192 x 2048: 443 -> 33 us; M = 33, 14336 x 4096: 72 -> 28 us.  Two passes over a matrix that fits the caches cost what its
     // launch costs (M = 33, 2048 x 2048: 17.4 against 19.0 us).
@@ -264,7 +263,7 @@ extern "C" int zl_dense_gemm_skinny_mul(const void* x, int ldx, const void* w, c
         GemmP p{x, w, y, mul_all, ldx, 0, K, 0, N, 0, ld_mul, 0, M, N, K};
         p.bias_t = bias;
         const int epi = act == 1 ? ZL_GEMM_EPI_RELU2 : act == 2 ? ZL_GEMM_EPI_TANH : act == 3 ? ZL_GEMM_EPI_GELU_TANH_MUL : ZL_GEMM_EPI_NONE;
-        const cudaError_t e = gemm_tc_route(p, 1, dtype) ? launch_gemm_tc(p, 1, dtype, out_dtype, epi, pdl != 0, stream) : cudaErrorNotSupported;
+        const cudaError_t e = gemm_tc_route(p, 1, dtype) ? launch_gemm_tc(p, 1, dtype, out_dtype, epi, pdl != kPdlNone && pdl != kPdlBehind, stream) : cudaErrorNotSupported;
         if (e != cudaErrorNotSupported) {
             ZL_CHECK_CUDA(e);
             return ZL_OK;
@@ -272,7 +271,7 @@ extern "C" int zl_dense_gemm_skinny_mul(const void* x, int ldx, const void* w, c
     }
     for (int m0 = 0; m0 < M; m0 += 32) {
         const int mc = (M - m0) < 32 ? (M - m0) : 32;
-        const bool use_pdl = pdl != 0 && m0 == 0;
+        const int use_pdl = pdl == kPdlNone || m0 == 0 ? pdl : kPdlBehind;
         const float* mul = mul_all ? mul_all + (size_t)m0 * ld_mul : nullptr;
         cudaError_t e;
         if (dtype == ZL_F16)

@@ -84,6 +84,8 @@ int unlocked(F&& f) {
     Unlocked u;
     return f();
 }
+// pdl of a call: early reads, or a dependent that waits for everything earlier first
+int launched(PyObject* pdl) { return truth(pdl) ? 1 : 2; }
 PyObject* result(int rc, const at::Tensor& out) { return rc ? PyLong_FromLong(rc) : THPVariable_Wrap(out); }
 
 template <typename F>
@@ -115,7 +117,7 @@ PyObject* w4a16_gemm_fused(PyObject*, PyObject* const* a, Py_ssize_t na) {
         p.bias = optional(a[5], false);
         p.residual = optional(a[6], false);
         p.epilogue = to_int(a[7]);
-        p.pdl = truth(a[8]);
+        p.pdl = launched(a[8]);
         p.variant = to_int(a[10]);
         if (p.epilogue == ZL_EPI_QKV_ROPE || p.N < 0) throw NotPlain{};
         const at::Tensor y = a[9] == Py_None ? empty(x, {x.size(0), p.epilogue == ZL_EPI_SWIGLU ? p.N / 2 : p.N}, at::kHalf) : plain(a[9], false);
@@ -133,7 +135,7 @@ PyObject* dense_gemm_skinny(PyObject*, PyObject* const* a, Py_ssize_t na) {
         const at::Tensor &x = plain(a[0], true), &w = plain(a[1], true);
         if (x.dim() != 2 || w.dim() < 1) throw NotPlain{};
         void* const bias = optional(a[2], true);
-        const int dt = dtype_of(x), od = a[3] == Py_None ? dt : to_int(a[3]), pdl = truth(a[4]);
+        const int dt = dtype_of(x), od = a[3] == Py_None ? dt : to_int(a[3]), pdl = launched(a[4]);
         if (od != ZL_F16 && od != ZL_BF16 && od != ZL_F32) throw NotPlain{};
         const at::Tensor y = empty(x, {x.size(0), w.size(0)}, od == ZL_F16 ? at::kHalf : od == ZL_BF16 ? at::kBFloat16 : at::kFloat);
         const zl_stream_t s = stream();
@@ -153,7 +155,7 @@ PyObject* w8_linear(PyObject*, PyObject* const* a, Py_ssize_t na) {
         const at::Tensor &x = plain(a[0], true), &w = plain(a[1], true), &ws = plain(a[2], true);
         if (x.dim() != 2 || w.dim() < 1) throw NotPlain{};
         void* const bias = optional(a[3], true);
-        const int kind = to_int(a[4]), pdl = truth(a[5]), dt = dtype_of(x), ws_dt = dtype_of(ws);
+        const int kind = to_int(a[4]), pdl = launched(a[5]), dt = dtype_of(x), ws_dt = dtype_of(ws);
         const int64_t m = x.size(0), k = x.size(1), scale_at = (m * k + 15) / 16 * 16;
         const at::Tensor y = empty(x, {m, w.size(0)}, x.scalar_type());
         const at::Tensor room = empty(x, {scale_at + 4 * m}, at::kByte);   // the 8-bit rows, then their scales

@@ -638,13 +638,14 @@ static void prefetch_target(zl_llama* m, int l, int slot, int B, const void** pt
 // ZL_NO_PDL_MASK (experiments): launch these kernels with a full dependency instead of a programmatic one.
 // 1 qkv GEMM, 2 attention, 4 o GEMM, 8 gate_up GEMM, 16 down GEMM, 32 final norm, 64 lm_head, 128 argmax.
 // Default 70 = lm_head + o GEMM + attention: a PDL-launched lm_head measured 128 us slower per step than a normally
-// launched one; early-launched o GEMM / attention CTAs cost another ~1 % each.
+// launched one; early-launched o GEMM / attention CTAs cost another ~1 % each.  By default the 4-bit o GEMM is a dependent that
+// waits first (kPdlBehind), which costs nothing: 692.5 / 692.6 against 693.1 / 692.8 tok/s.
+static const char* no_pdl_asked() {
+    static const char* const v = getenv("ZL_NO_PDL_MASK");
+    return v;
+}
 static int no_pdl_mask(bool tensor_parallel = false) {
-    static int v = -2;
-    if (v == -2) {
-        const char* e = getenv("ZL_NO_PDL_MASK");
-        v = e ? atoi(e) : -1;
-    }
+    static const int v = no_pdl_asked() ? atoi(no_pdl_asked()) : -1;
     if (v >= 0) return v;
     // single GPU: lm_head, o GEMM, attention with full dependencies measured best (640 -> 710 tok/s);
     // tensor parallel (exchange inside the GEMMs): a PDL-launched attention kernel wins (N = 2: 783 vs 754 tok/s)
@@ -690,7 +691,7 @@ int w4_gemm(zl_llama* m, const void* x, int ldx, const W4Lin& w, const void* res
     a.epilogue = epi;
     {
         const int bit = slot == 0 ? 1 : slot == 2 ? 4 : slot == 3 ? 8 : slot == 4 ? 16 : 0;
-        a.pdl = (no_pdl_mask(c.tp_size > 1) & bit) ? 0 : c.use_pdl;
+        a.pdl = (no_pdl_mask(c.tp_size > 1) & bit) ? (c.use_pdl && !no_pdl_asked() ? kPdlBehind : kPdlNone) : c.use_pdl;
     }
     a.ln_weight = ln_w;
     a.eps = c.eps;

@@ -207,24 +207,25 @@ extern "C" int zl_w4a16_gemm_fused(const zl_w4_fused_args_t* a, zl_stream_t stre
         p.tp_mode = a->tp_mode;
         p.tp_index = a->tp_index;
         p.tp_h_out = static_cast<__half*>(a->tp_h_out);
-        // Always a programmatic dependent; the weights ahead of the wait only where the caller's chain allows it.  In a row of calls without that: a feed-forward of
-        // 4096 and 14336 at 32 rows 53.9 -> 49.2 us, one row of 4096 x 4096 6.15 -> 5.18 (what the host needs for a call).
-        p.early = a->pdl != 0 && m0 == 0;
+        // kPdlBehind against ordinary launches, in a row of calls: a feed-forward of 4096 and 14336 at 32 rows 53.9 -> 49.2 us, one row of 4096 x 4096 6.15 -> 5.18 (what the
+        // host needs for a call).
+        const bool dependent = a->pdl != kPdlNone;
+        p.early = !dependent || (a->pdl != kPdlBehind && m0 == 0);
         p.pf_ptr = static_cast<const uint8_t*>(a->prefetch_ptr);
         p.pf_bytes = a->prefetch_bytes;
         if (pairs) {
-            ZL_CHECK_CUDA(launch_w4_tc2(p, true, stream));
+            ZL_CHECK_CUDA(launch_w4_tc2(p, dependent, stream));
         } else if (few) {
-            ZL_CHECK_CUDA(launch_w4_v2_int_layout(p, true, stream));
+            ZL_CHECK_CUDA(launch_w4_v2_int_layout(p, dependent, stream));
         } else if (route == 4) {
-            ZL_CHECK_CUDA(launch_w4_tc(p, true, stream));
+            ZL_CHECK_CUDA(launch_w4_tc(p, dependent, stream));
         } else if (route == 3) {
             cudaError_t ce = cudaSuccess;
-            const bool ok = launch_w4_v3(p, true, stream, &ce);
+            const bool ok = launch_w4_v3(p, dependent, stream, &ce);
             ZL_CHECK_SUPPORTED(ok && "ZLW4I kernel: staged activations do not fit shared memory (use variant 0)");
             ZL_CHECK_CUDA(ce);
         } else {
-            ZL_CHECK_CUDA(launch_w4_v2(p, true, stream));
+            ZL_CHECK_CUDA(launch_w4_v2(p, dependent, stream));
         }
     }
     return ZL_OK;

@@ -246,22 +246,23 @@ __global__ void __launch_bounds__(256) k_fp8_convert(const T* __restrict__ x, ui
         fp8_convert8(x + i, q + i, inv);
 }
 
-// Above this many values (eight rounds of a 1024-thread CTA) the walk of the whole input by every CTA costs more than two more launches.  All
-// of them, and k_int8_quant_per_token, are programmatic dependents always (pdl_start), the word is zeroed by a kernel and not by a memset so that the chain holds:
-// a whole fp8 Linear of 500 x 4096 -> 14336 43.2 -> 41.1 us in a row of calls, an int8 one of 24 x 8192 -> 8192 20.6 -> 19.9.
+// Above this many values (eight rounds of a 1024-thread CTA) the walk of the whole input by every CTA costs more than two more launches.  The
+// word is zeroed by a kernel and not by a memset so that a chain of dependents holds.  kPdlBehind against ordinary launches, k_int8_quant_per_token too: a whole fp8 Linear of 500 x 4096 -> 14336 43.2 -> 41.1 us in a row of calls, an int8 one of 24 x 8192 -> 8192 20.6 -> 19.9.
 constexpr size_t kFp8OneLaunchMax = 65536;
 
 template <typename T>
-static cudaError_t launch_fp8_quant(const T* x, uint8_t* q, float* scale, size_t n, bool pdl, cudaStream_t st) {
+static cudaError_t launch_fp8_quant(const T* x, uint8_t* q, float* scale, size_t n, int pdl, cudaStream_t st) {
     const size_t vecs = n / 8;
+    const bool dependent = pdl != kPdlNone;
+    const int early = pdl != kPdlBehind;
     if (n <= kFp8OneLaunchMax)
         return launch(k_fp8_quant_per_tensor<T>, dim3((unsigned)((vecs + kFp8SmallThreads - 1) / kFp8SmallThreads)), dim3(kFp8SmallThreads), 0,
-                      st, true, x, q, scale, n, (int)pdl);
+                      st, dependent, x, q, scale, n, early);
     const size_t most = 8 * (size_t)device_sm_count();
     const unsigned ctas = (unsigned)((vecs + 255) / 256 < most ? (vecs + 255) / 256 : most);
-    cudaError_t e = launch(k_fp8_zero, dim3(1), dim3(32), 0, st, true, scale, (int)pdl);
-    if (e == cudaSuccess) e = launch(k_fp8_scale<T>, dim3(ctas), dim3(256), 0, st, true, x, scale, n);
-    if (e == cudaSuccess) e = launch(k_fp8_convert<T>, dim3(ctas), dim3(256), 0, st, true, x, q, (const float*)scale, n);
+    cudaError_t e = launch(k_fp8_zero, dim3(1), dim3(32), 0, st, dependent, scale, early);
+    if (e == cudaSuccess) e = launch(k_fp8_scale<T>, dim3(ctas), dim3(256), 0, st, dependent, x, scale, n);
+    if (e == cudaSuccess) e = launch(k_fp8_convert<T>, dim3(ctas), dim3(256), 0, st, dependent, x, q, (const float*)scale, n);
     return e;
 }
 
@@ -437,14 +438,14 @@ static cudaError_t launch_w8(const uint8_t* xq, const float* sx, const uint8_t* 
 
 constexpr int kSmBytes = 228 * 1024;   // shared memory of an SM
 template <typename T>
-static cudaError_t launch_int8_quant(const T* x, int ldx, int8_t* q, float* scale, int M, int K, bool pdl, cudaStream_t stream) {
+static cudaError_t launch_int8_quant(const T* x, int ldx, int8_t* q, float* scale, int M, int K, int pdl, cudaStream_t stream) {
     const int chunks = cdiv(K, 256 * 8);
     auto kernel = chunks <= 1 ? k_int8_quant_per_token<T, 1> : chunks <= 2 ? k_int8_quant_per_token<T, 2>
                   : chunks <= 4 ? k_int8_quant_per_token<T, 4> : chunks <= 8 ? k_int8_quant_per_token<T, 8> : k_int8_quant_per_token<T, 0>;
     // Where it comes under the end of whatever was before, its CTAs ask for the shared memory that spreads them over the SMs: beside a GEMM that still runs they were placed in
     // sixes.  With the GEMM behind it, in a graph, ordinary launches / dependents / dependents so: 100 rows of 4096 x 4096 11.5 / 12.7 / 11.5 us, 64 of 8192 x 8192 14.6 / 16.1 / 14.3, 160 of
     // 6144 x 4096 13.2 / 14.7 / 12.7, 32 of 28672 x 4096 26.3 / 28.6 / 26.2.
-    const int per_sm = cdiv(M, device_sm_count()), smem = pdl || per_sm > 6 ? 0 : kSmBytes / (per_sm + 1);
+    const int per_sm = cdiv(M, device_sm_count()), smem = pdl != kPdlBehind || per_sm > 6 ? 0 : kSmBytes / (per_sm + 1);
     if (smem > 48 * 1024) {
         static bool set[64][5] = {};
         const int at = chunks <= 1 ? 0 : chunks <= 2 ? 1 : chunks <= 4 ? 2 : chunks <= 8 ? 3 : 4;
@@ -456,7 +457,7 @@ static cudaError_t launch_int8_quant(const T* x, int ldx, int8_t* q, float* scal
             if (dev >= 0 && dev < 64) set[dev][at] = true;
         }
     }
-    return launch(kernel, dim3(M), dim3(256), (size_t)smem, stream, true, x, ldx, q, scale, K, (int)pdl);
+    return launch(kernel, dim3(M), dim3(256), (size_t)smem, stream, pdl != kPdlNone, x, ldx, q, scale, K, (int)(pdl != kPdlBehind));
 }
 
 }  // namespace zl
@@ -469,8 +470,8 @@ extern "C" int zl_int8_quant_per_token(const void* x, int ldx, void* q, float* s
     ZL_CHECK_ARG(dtype == ZL_F16 || dtype == ZL_BF16);
     ZL_CHECK_SUPPORTED(K % 8 == 0 && ldx % 8 == 0 && ldx >= K);
     ZL_CHECK_ARG((reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(q) & 7) == 0);
-    const cudaError_t e = dtype == ZL_F16 ? launch_int8_quant(static_cast<const __half*>(x), ldx, static_cast<int8_t*>(q), scale, M, K, pdl != 0, stream)
-                                          : launch_int8_quant(static_cast<const __nv_bfloat16*>(x), ldx, static_cast<int8_t*>(q), scale, M, K, pdl != 0, stream);
+    const cudaError_t e = dtype == ZL_F16 ? launch_int8_quant(static_cast<const __half*>(x), ldx, static_cast<int8_t*>(q), scale, M, K, pdl, stream)
+                                          : launch_int8_quant(static_cast<const __nv_bfloat16*>(x), ldx, static_cast<int8_t*>(q), scale, M, K, pdl, stream);
     ZL_CHECK_CUDA(e);
     return ZL_OK;
 }
@@ -499,8 +500,8 @@ extern "C" int zl_fp8_quant_per_tensor(const void* x, void* q, float* scale, siz
     ZL_CHECK_ARG(dtype == ZL_F16 || dtype == ZL_BF16);
     ZL_CHECK_SUPPORTED(n % 8 == 0);
     ZL_CHECK_SUPPORTED(n <= ((size_t)1 << 22));   // the range this entry point has always had; the kernels below know no such limit
-    const cudaError_t e = dtype == ZL_F16 ? launch_fp8_quant(static_cast<const __half*>(x), static_cast<uint8_t*>(q), scale, n, pdl != 0, stream)
-                                          : launch_fp8_quant(static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), scale, n, pdl != 0, stream);
+    const cudaError_t e = dtype == ZL_F16 ? launch_fp8_quant(static_cast<const __half*>(x), static_cast<uint8_t*>(q), scale, n, pdl, stream)
+                                          : launch_fp8_quant(static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), scale, n, pdl, stream);
     ZL_CHECK_CUDA(e);
     return ZL_OK;
 }

@@ -153,6 +153,11 @@ def swiglu_row_map(f, device):
 
 
 # ------------------------------------------------------------------ compute
+def _launched(pdl):
+    """`pdl` of the calls that know three launches: early reads (True), or a dependent that waits for everything earlier first.  0, an ordinary launch, is not used here."""
+    return 1 if pdl else 2
+
+
 def w4a16_gemm(x, packed, n, k, group_size=128, bias=None, residual=None, epilogue=EPI_NONE, pdl=False, out=None):
     """nn::gptq::gptq_gemm_k_major (GEMV path) on the ZLW4 layout."""
     if x.dtype != torch.float16:
@@ -162,7 +167,7 @@ def w4a16_gemm(x, packed, n, k, group_size=128, bias=None, residual=None, epilog
     if out is None:
         out = torch.empty((m, n_out), dtype=torch.float16, device=x.device)
     _lib.call("zl_w4a16_gemm", _p(x), x.stride(0), _p(packed), _p(bias), _p(residual), _p(out), m, n, k, group_size,
-              epilogue, int(pdl), _stream())
+              epilogue, _launched(pdl), _stream())
     return out
 
 
@@ -195,7 +200,7 @@ def w4a16_gemm_fused(x, packed, n, k, group_size=128, bias=None, residual=None, 
     m = x.shape[0]
     # in the structure's order: one call, not an assignment for each of its members
     a = _lib.W4FusedArgs(x.data_ptr(), x.stride(0), packed.data_ptr(), _dp(bias), _dp(residual), None, m, n, k, group_size, epilogue,
-                         int(pdl), _dp(ln_weight), eps)
+                         _launched(pdl), _dp(ln_weight), eps)
     if variant:
         a.variant = int(variant)
     table = None
@@ -230,7 +235,7 @@ def dense_gemm_skinny(x, w, bias=None, out_dtype=None, pdl=False):
     od = x.dtype if out_dtype is None else out_dtype
     out = torch.empty((m, n), dtype=od, device=x.device)
     _lib.call("zl_dense_gemm_skinny", _p(x), x.stride(0), _p(w), _p(bias), _p(out), m, n, k, _dt(x), _dt(out),
-              int(pdl), _stream())
+              _launched(pdl), _stream())
     return out
 
 
@@ -242,7 +247,7 @@ def int8_quant_per_token(x, pdl=False):
     m, k = x.shape
     q = torch.empty((m, k), dtype=torch.int8, device=x.device)
     scale = torch.empty((m,), dtype=torch.float32, device=x.device)
-    _lib.call("zl_int8_quant_per_token", _p(x), x.stride(0), _p(q), _p(scale), m, k, _dt(x), int(pdl), _stream())
+    _lib.call("zl_int8_quant_per_token", _p(x), x.stride(0), _p(q), _p(scale), m, k, _dt(x), _launched(pdl), _stream())
     return q, scale
 
 
@@ -261,7 +266,7 @@ def fp8_quant_per_tensor(x, pdl=False):
     """nn::fp8::dynamic_scaled_quant: returns (q uint8 holding e4m3 bits, scale f32 (1))."""
     q = torch.empty(x.shape, dtype=torch.uint8, device=x.device)
     scale = torch.empty((1,), dtype=torch.float32, device=x.device)
-    _lib.call("zl_fp8_quant_per_tensor", _p(x), _p(q), _p(scale), x.numel(), _dt(x), int(pdl), _stream())
+    _lib.call("zl_fp8_quant_per_tensor", _p(x), _p(q), _p(scale), x.numel(), _dt(x), _launched(pdl), _stream())
     return q, scale
 
 
@@ -692,7 +697,7 @@ def dense_gemm_skinny_mul(x, w, act, mul=None, out_dtype=None):
     n = w.shape[0]
     y = torch.empty((m, n), dtype=out_dtype or x.dtype, device=x.device)
     _lib.call("zl_dense_gemm_skinny_mul", _p(x), k, _p(w), None, _p(y), m, n, k, _dt(x), _dt(y), act, _p(mul),
-              mul.shape[1] if mul is not None else 0, 0, _stream())
+              mul.shape[1] if mul is not None else 0, _launched(False), _stream())
     return y
 
 
