@@ -570,8 +570,8 @@ __global__ void __launch_bounds__(kGtThreads, 1) k_gemm_tc(const __grid_constant
 }
 
 // Rows of x per tile, and how many pairs share a tile's K, for `blocks` 128-byte blocks of k: with few tiles the pairs of a cluster (the device holds
-// fit[0] clusters of two pairs at a time, fit[1] of four) take a part each and exchange their sums.  In cycles, fitted to the times below: a block
-// 190 + 1.4 per row of x, the exchange 2850 + 42 per row.  Measured, one pair / two, us, N x K: bf16 4096 x 14336, 65 rows 39.3 / 31.2, 256 rows
+// fit[0] clusters of two pairs at a time, fit[1] of four) take a part each and exchange their sums.  In cycles, fitted to the times below, which are from before all
+// warps took part in the exchange and in the last tile's end: a block 190 + 1.4 per row of x, the exchange 2850 + 42 per row.  Measured, one pair / two, us, N x K: bf16 4096 x 14336, 65 rows 39.3 / 31.2, 256 rows
 // 42.6 / 37.2; 1024 x 8192, 65 rows 23.3 / 17.2 and 14.9 with four; int8 8192 x 8192, 24 rows 20.3 / 18.9; against it bf16 4096 x 4096, 512 rows
 // 22.5 / 25.4; 8192 x 2048, 256 rows 16.9 / 20.9.
 struct GtPick {
@@ -601,8 +601,9 @@ static GtPick gt_pick(int M, long long rows, int pairs, int blocks, const int (&
 // faster one at all of them): the tile kernel's first wave of 64 x 64 blocks and what each further block's rows cost; here the tile's rows and what a
 // further wave of pairs costs.  Measured, tile kernel / here, M x N x K: 33 x 128 x 64 2.8 / 4.0; 256 x 512 x 256 5.5 / 4.4; 384 x 2048 x 256 7.8 / 5.6;
 // 16 matrices of 33 x 512 x 128 3.7 / 4.8, of 256 x 128 x 64 3.6 / 5.6; 48 of 200 x 256 x 128 12.4 / 8.9, of 33 x 4096 x 256 37.8 / 25.6.  The estimates err by 6 and 5 %
-// on average, so half a microsecond counts as even and stays there: at no measured shape does this kernel serve what the other one would serve faster
-// (without, up to 14 % there), and what stays costs up to 25 %, 1 % on average over all shapes.
+// on average, so half a microsecond counts as even and stays there.  This kernel has become faster since, the estimates are those of then.  With both as they are now, 768 shapes
+// (M = 33 .. 512, N = 128 .. 4096, K = 64 .. 256, 1 .. 48 matrices): this kernel still serves none that the other one would serve faster by more than 2 %, and what stays
+// costs up to 94 %, 4 % on average over all: 48 matrices of 200 x 512 x 64 8.0 / 15.6 us (here / there), of 33 x 2048 x 192 10.8 / 17.7, one of 512 x 4096 x 64 5.8 / 8.4.
 bool gemm_tile_faster(int M, int N, int K, int batch) {
     if (K > 256) return false;
     const int sms = device_sm_count(), pairs = sms / 2;

@@ -1293,9 +1293,9 @@ extern "C" int zl_llama_step_device(zl_llama_t* m, int B) {
     return ZL_OK;
 }
 
-// The step's logits to the caller's memory.  Up to 1 MB reach pageable memory through pinned pieces, each copied out while the next one is on its way: 512 KB take 38 us
-// beside the step so, 46 when the runtime stages the copy (a step of four users over 32000 words: 231 -> 216 us, of eight 294 -> 280); of 2 MB the runtime's copy takes
-// 146 us, one in pieces 165.
+// The step's logits to the caller's memory.  Up to 1 MB reach pageable memory through pinned pieces, each copied out while the next one is on its way: 512 KB make a
+// step 36 us longer so, 49 when the runtime stages the copy, 1 MB 64 and 83 (steps of four and eight users over 32000 words in a row, two layers: 177 us and 210
+// without logits, 213 and 274 with them; 191 and 233 into page-locked memory); of 2 MB the runtime's copy takes 146 us, one in pieces 165.
 static int read_logits(zl_llama* m, float* dst, size_t count) {
     const size_t bytes = count * sizeof(float), piece = zl_llama::kOutPiece;
     bool direct = bytes > zl_llama::kOutPieces * piece;

@@ -8,8 +8,8 @@
 //   * a tile is 256 rows of w by up to 256 tokens over two SMs: each converts its own 128 rows and loads half of the tokens;
 //   * tiles are taken whole, in turn by persistent pairs; the token tile's size is chosen so that the last wave is full, or its tiles come in halves;
 //   * up to 64 tokens there are two accumulators; with one, the epilogue and the dequant warps shorten the gap together (t2_finish).
-// 28672 x 4096 with SwiGLU: 1000 tokens 499 -> 180 us (cuBLAS fp16 170), 256 tokens 128 -> 55; 4096 x 14336 with the residual: 1000 tokens 408 -> 90 us
-// (1300 TFLOP/s).  Bound by the tensor cores at 256 tokens (1084 cycles per 128-k group, at the clock that the power limit leaves); below 130
+// 28672 x 4096 with SwiGLU: 1000 tokens 499 -> 182 us (cuBLAS fp16 178), 256 tokens 128 -> 55; 4096 x 14336 with the residual: 1000 tokens 408 -> 92 us
+// (88; 1280 TFLOP/s).  These are 200 calls in a row on a rested GPU; after half a second of them the power limit makes it 211 and 103 (cuBLAS 204 and 100).  Bound by the tensor cores at 256 tokens (1084 cycles per 128-k group, at the clock that the power limit leaves); below 130
 // tokens by the conversion (0.31 us of a group, about 600 cycles; 340 when nothing else runs on the SM).
 //
 // What a stage costs one thread is what bounded small tiles before that (830 cycles): looking at a barrier takes it 120 - 200 cycles even when the
@@ -551,7 +551,7 @@ static int t2_sub(int ntok) { return ntok <= 128 ? 2 : 1; }
 // Measured, one pair / two / three, N x K, us: 4096 x 14336, 32 tokens 43 / 27 / 22.7, 96 tokens 45 / 31 / 24.7, 256 tokens 46.5 / 33 / -;
 // 4096 x 4096, 96 tokens 18.8 / 16.5 / 16.5, 128 tokens 19.7 / 16.5 / 18.2; 6144 x 4096, 64 tokens 19.0 / 16.5 / -; 8192 x 3584, 128 tokens
 // 19.7 / 18.6 / -.  These are the times from before every warp helped with the epilogue; up to 256 rows they stand, since the line to the stream-k kernel
-// rests on them.  Beyond, fitted again to 56 sizes and their tiles (M = 320 .. 1000 of eight matrices; within 5 % where power is no limit): a group 0.35, or 0.08 +
+// rests on them (see w4_tc2_route for what that costs).  Beyond, fitted again to 56 sizes and their tiles (M = 320 .. 1000 of eight matrices; within 5 % where power is no limit): a group 0.35, or 0.08 +
 // 0.0021 per token above 128, start and end 9 + 0.01 per token, a further wave's end 1.5 + 0.01 per token (hidden up to 64).  There a last wave of few tiles
 // may also be cut in halves along its tokens: 28672 x 4096 is 448 tiles of 256 tokens at M = 1000, six waves and four tiles: 192 -> 184 us; M = 512 110 -> 103 (224
 // tiles, three waves and two); 16384 x 2048, M = 1000 67.8 -> 61.7.  Quarters: 184, 102 and 73, the conversion (0.4 a group) is the same for 64 tokens.
@@ -599,9 +599,10 @@ static T2Pick t2_pick(int M, int row_tiles, int G) {
 // Where its ranges are down to eight groups every tile is cut, and what is exchanged grows with M.
 // Measured in a row of calls, N x K, there / here, us: 4096 x 14336 at M = 32 / 64 / 128 / 256 21 / 23 / 36 / 59 and 21 / 22 / 25 / 31; 28672 x 4096 31 / 37 /
 // 54 / 105 and 28 / 29 / 37 / 61; 6144 x 4096 15 / 19 / 28 / 49 and 14 / 15 / 17 / 20; 2304 x 1152 at M = 33 / 256 16 / 49 and 10 / 10; 512 x 14336 18 / 34 and
-// 18 / 18; 4096 x 4096 at M = 33 / 64 13.1 / 13.7 and 14.1 / 14.3; 10240 x 8192 at M = 17 / 48 24 / 27 and 27 / 28.  The estimates are older than that: of 19 sizes this
-// kernel was the faster one at every one from 65 rows on and the other at three below, by 12 % at most, while calls stay there
-// that take up to 29 % (82 % at 256 rows of 512 x 14336) longer.  In a feed-forward of 4096 and 14336 at 32 rows both products there take 55.6 us,
+// 18 / 18; 4096 x 4096 at M = 33 / 64 13.1 / 13.7 and 14.1 / 14.3; 10240 x 8192 at M = 17 / 48 24 / 27 and 27 / 28.  The estimates are older than that.  With
+// both kernels as they are now, 284 points in graphs (22 sizes from 2048 x 2048 to 27648 x 5120, 17 .. 256 rows): none is sent here that takes longer here (among 95 further points 64 rows of
+// 9472 x 8192 are, 27.8 / 22.5, half of the pairs work, and 17 of 18944 x 4096 where the weights come from HBM, 18.8 / 18.4); of the 77 that stay 52 would be the faster ones here by more than 2 %, 10 % on average over the 77: 64 rows of 6144 x 4096 12.7 / 17.8 (here / there), 96 of 2048 x 4096
+// 12.0 / 16.3, 128 of 1024 x 8192 12.6 / 16.7 (and 256 of 512 x 14336 18 / 34).  In a feed-forward of 4096 and 14336 at 32 rows both products there take 55.6 us,
 // both here 54.6, one of each 55.4 to 57.4; as programmatic dependents in a graph 47.2, 43.8, and 45.0 to 48.1.
 bool w4_tc2_route(int M, int N, int K) {
     if (M <= 16 || N % kTcRows || K % kW4GroupK) return false;

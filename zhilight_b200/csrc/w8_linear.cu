@@ -247,7 +247,8 @@ __global__ void __launch_bounds__(256) k_fp8_convert(const T* __restrict__ x, ui
 }
 
 // Above this many values (eight rounds of a 1024-thread CTA) the walk of the whole input by every CTA costs more than two more launches.  The
-// word is zeroed by a kernel and not by a memset so that a chain of dependents holds.  kPdlBehind against ordinary launches, k_int8_quant_per_token too: a whole fp8 Linear of 500 x 4096 -> 14336 43.2 -> 41.1 us in a row of calls, an int8 one of 24 x 8192 -> 8192 20.6 -> 19.9.
+// word is zeroed by a kernel and not by a memset so that a chain of dependents holds.  kPdlBehind against ordinary launches,
+// k_int8_quant_per_token too: a whole fp8 Linear of 500 x 4096 -> 14336 43.2 -> 41.1 us in a row of calls, an int8 one of 24 x 8192 -> 8192 20.6 -> 19.9.
 constexpr size_t kFp8OneLaunchMax = 65536;
 
 template <typename T>
@@ -525,8 +526,8 @@ extern "C" int zl_int8_scale_back(const int32_t* acc, const float* x_scale, cons
 // Whether M rows go to the kernel on pairs of SMs (gemm_tc.cu), which costs the same from 1 row to 32 and has few, large tiles, whose K up to four
 // pairs share; the mma.sync kernel reads its activations once per 16 weight rows and takes half as long again from 8 rows to 9 and from 16 to 17, fp8
 // more than int8.  So the lines are weights per step of rows, and below 17 rows N as well: few tiles read the weights through few SMs.  us of a whole
-// Linear in a row of calls, quantisation included, mma.sync / here; of 1112 measured points (46 sizes from 1024 x 1024 to 28672 x 8192) none is sent here
-// that takes longer here, and what stays costs 1.7 % on average:
+// Linear in a row of calls, quantisation included, mma.sync / here, when the lines were drawn; of 1112 measured points (46 sizes from 1024 x 1024 to 28672 x 8192) none was sent here
+// that took longer here, and what stayed cost 1.7 % on average:
 //   int8, 32 rows   4096 x 4096 11.9 / 11.8; 6144 x 4096 20.0 / 12.6; 8192 x 8192 36.0 / 19.3; 1024 x 8192 17.0 / 11.5
 //         16        4096 x 4096 8.9 / 11.8; 6144 x 4096 14.5 / 12.5; 4096 x 8192 13.9 / 14.8; 4096 x 14336 21.7 / 19.1
 //          8        8192 x 8192 19.1 / 18.8; 8192 x 5120 14.7 / 15.0; 10240 x 4096 17.1 / 14.2; 28672 x 8192 59.9 / 43.8
@@ -534,6 +535,8 @@ extern "C" int zl_int8_scale_back(const int32_t* acc, const float* x_scale, cons
 //         16        2048 x 8192 16.4 / 18.4; 4096 x 4096 14.8 / 12.3; 8192 x 8192 39.6 / 25.0
 //          8        8192 x 5120 16.7 / 14.7; 14336 x 4096 20.7 / 16.4; 4096 x 14336 22.7 / 24.6
 // From 33 rows on it is here at every size (1088 x 512 6.0 against 6.7 / 6.0 for the kernel that served it before).
+// This kernel has become faster since.  With both as they are now, 450 points in graphs (25 sizes, 1 .. 32 rows): still none is sent here that takes longer here, and the 180
+// that stay cost 4.4 % on average, up to 49 %: fp8, 32 rows of 3072 x 3072 14.4 / 9.7, 8 rows of 8192 x 8192 19.0 / 13.6; int8, 32 rows of 4096 x 4096 11.0 / 9.6.
 static bool w8_tc_route(int M, int N, int K, bool fp8) {
     constexpr long long kMi = 1 << 20;
     const long long weights = (long long)N * K;

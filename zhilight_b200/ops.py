@@ -417,7 +417,8 @@ def qkv_rope_append(cos, sin, qkv, token_batch, placement, k_bufs, v_bufs, num_h
 
 def decode_attention(q, buf_lens, k_bufs, v_bufs, mask, scale, max_len_buf, num_kv_heads, bshd=True, pdl=False):
     """nn::multi_query_attention_rag_buffer: q (B, len_q, H_q, d); k_bufs/v_bufs lists of per-task tensors.  pdl is taken as for the other calls and
-    changes nothing: the table of addresses is written by a launch behind everything earlier, and the attention may always start under its end."""
+    changes nothing: the call's first kernel waits for everything earlier.  For up to 32 tasks and one CTA per SM it takes the caches' addresses along as a parameter, else
+    it writes them to a table and the attention starts under its end."""
     if _lib.host is not None:
         out = _lib.host.decode_attention(q, buf_lens, k_bufs, v_bufs, mask, scale, max_len_buf, num_kv_heads, bshd, pdl)
         if out is not None:
