@@ -211,8 +211,8 @@ __device__ __forceinline__ void attn_short_item(const T* __restrict__ q, const i
 // everything earlier before it lets dependents start, as the launch that writes a table would.
 constexpr int kAttnInline = 32;
 struct AttnAddrs {
+    int n, behind;                    // tasks, 0: the tables; beside the other parameters: a line of them further back is fetched when a kernel starts
     const void* p[2 * kAttnInline];   // of K, then of V
-    int n, behind;                    // tasks, 0: the tables
 };
 template <typename T>
 __device__ __forceinline__ const T* attn_addr(const AttnAddrs& a, T* const* table, int b, bool v) {

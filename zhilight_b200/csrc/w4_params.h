@@ -9,6 +9,7 @@ namespace zl {
 struct W4Params {
     const __half* x;
     int ldx;
+    int early = 0;            // the caller's chain: see pdl_start; the first thing a kernel asks for, so beside what it reads next
     const uint8_t* packed;
     const __half* bias;       // indexed by PACKED row
     const __half* residual;
@@ -39,7 +40,6 @@ struct W4Params {
     int tp_mode = 0;
     int tp_index = 0;              // exchange index within the step (< 512): parity of the slot + part of the word tag
     __half* tp_h_out = nullptr;
-    int early = 0;                 // the caller's chain: see pdl_start
     int x32 = 0;                   // rows of x start on 32 bytes (set by launch_w4_v2_int_layout)
 };
 
