@@ -138,3 +138,38 @@ def test_switch_for_ordinary_launches(lib, cuda, switch, programmatic):
     r = subprocess.run([sys.executable, "-c", _SWITCH], env=env, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
     assert r.stdout.split()[-3:] == ["edges", str(programmatic), "1"]
+
+
+_CAPTURED_FIRST = """
+import torch
+from zhilight_b200 import ops
+what = %r
+g = torch.Generator().manual_seed(1)
+x = torch.randn(149, 2056, generator=g).half().cuda()
+kv = [torch.randn(2600, 8, 128, generator=g).half().cuda() for _ in range(8)]
+q = torch.randn(4, 1, 32, 128, generator=g).half().cuda()
+lens = torch.tensor([1000, 900, 800, 700], dtype=torch.int32, device="cuda")
+rows = torch.randn(1, 107, 16, 128, generator=g).half().cuda()
+long = torch.tensor([2600], dtype=torch.int32, device="cuda")
+run = {"int8": lambda: ops.int8_quant_per_token(x)[0], "one row": lambda: ops.decode_attention(q, lens, [t[:n] for t, n in zip(kv, lens_)], [t[:n] for t, n in zip(kv[4:], lens_)], None,
+                                                                                              0.1, 1000, 8),
+       "rows": lambda: ops.decode_attention(rows, long, kv[:1], kv[1:2], None, 0.1, 2600, 8)}[what]
+lens_ = [1000, 900, 800, 700]
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    y = run()
+graph.replay()
+torch.cuda.synchronize()
+got = y.clone()
+print("same", torch.equal(got, run()), float(got.float().abs().sum()) > 0)
+"""
+
+
+@pytest.mark.parametrize("what", ["int8", "one row", "rows"])
+def test_first_call_of_a_process_may_be_captured(cuda, what):
+    """The device is asked how many clusters it holds, and a kernel is given its shared memory, inside the capture."""
+    env = dict(os.environ, PYTHONPATH=os.path.join(os.path.dirname(__file__), ".."))
+    r = subprocess.run([sys.executable, "-c", _CAPTURED_FIRST % what], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    assert r.stdout.split() == ["same", "True", "True"]
